@@ -1,123 +1,53 @@
 // Fused decode attention over GAAC-compressed K/V (sm_100a): slot layout and paged layout in one kernel template.
 //
-// CTA = (batch row, kv head, context split), ATT_WARPS warps, one CTA per SM.  Every warp streams its own 16-token tiles
-// through a private two-stage shared-memory ring filled by bulk asynchronous copies (the TMA engine without a tensor map,
-// completion counted in bytes on an mbarrier), rebuilds BF16 K/V fragments in registers (byte-SWAR, gaac_tile.h) and feeds
-// mma.sync m16n8k16:
-//   S^T[16 tok x 8 heads] = K[16 x 128] . Q^T        O^T[128 dims x 8 heads] += V^T[128 x 16 tok] . P^T
+// CTA = (batch row, kv head, context split), ATT_WARPS warps, one CTA per SM.  The CTA streams its 16-token tiles through one ring of
+// shared-memory stages, each holding TPS consecutive tiles of K and V, filled by bulk asynchronous copies (the TMA engine without a
+// tensor map, completion counted in bytes on the stage's mbarrier).  Warps take tiles from a shared counter, rebuild BF16 K/V fragments
+// in registers (byte-SWAR) and feed mma.sync m16n8k16:
+//   S^T[16 tok x 8 columns] = K[16 x 128] . Q^T        O^T[channel pairs x 8 columns] += V^T . P^T      (gaac_attn_tile.cuh)
 // with an fp32 online softmax in the exp2 domain whose maximum is raised lazily.  Raw BF16 tiles (the slot layout's tail, the
-// paged layout's filling block and raw-fallback tiles) are read straight from global memory into the same fragments.  Tiles
-// are handed to the warps of a CTA from a shared counter.  The warps of a CTA are merged in shared memory, the CTA writes
-// one partial (m, l, acc[128]) per query head, and the last CTA of a (row, kv head) to finish merges the splits and writes
-// the output, so one launch does the whole layer.
+// paged layout's filling block and raw-fallback tiles) are read straight from global memory into the same fragments.  The warps of a
+// CTA are merged in shared memory, the CTA writes one partial (m, l, acc[128]) per query head, and the last CTA of a (row, kv head) to
+// finish merges the splits and writes the output, so one launch does the whole layer.
 //
 // What the measurements on B200 say (they shaped the code below):
-//  * per-lane cp.async copies (18 instructions per tile pair and warp) kept the load/store unit 60 % busy, and it is shared
-//    with the fragment reads: the L1-bypassing form sends one sector request per lane and writes shared memory one lane
-//    chunk per wavefront, the caching form coalesces but still costs ~22 cycles per instruction.  Bulk copies take that
-//    work off the SM; they want few large copies (one 128-byte copy per row, which would allow a conflict-free skewed
-//    layout, was 15 % slower), so shared memory holds the storage order and the 16-byte fragment reads accept a 2-way (K) /
-//    4-way (V) bank conflict (worth 0.7 us of 74).
-//  * the kernel is bound by instruction issue (ALU pipe) and by the shared-memory pipe, not by HBM: spreading the 3-bit
-//    codes through a 4096-entry table costs one load with ~3.5-way bank conflicts, by arithmetic two multiply-adds and
-//    three logic instructions.  Which is faster moved with the rest of the kernel (table while the copies loaded the
-//    load/store unit less than the integer pipe, half and half after the bulk copies brought the storage-order conflicts);
-//    in the final kernel arithmetic only is fastest by 1 %, table only slowest by 4 % (GAAC_LUTC = 0 / 2 / 1).
+//  * the kernel is bound by instruction issue and by the ALU pipe, not by HBM.  With a private two-stage ring per warp every warp issued
+//    eight copies per tile pair, about 200 of 1354 instructions; one copy of four tiles, issued by the warp that is last to leave a
+//    stage, takes that to about 25 per tile pair.
+//  * bulk copies want few large copies (one 128-byte copy per row, which would allow a conflict-free skewed layout, was 15 % slower), so
+//    shared memory holds the storage order and the 16-byte fragment reads accept a 2-way (K) / 4-way (V) bank conflict.
 //
 // Fragment conventions follow the reference kernel (gaac/kernel.py:62-66,160-194), whose storage order they mirror.
-#include <cuda_bf16.h>
-#include <math_constants.h>
 #include <algorithm>
 #include "gaac_api.cuh"
-#include "gaac_tile.h"
+#include "gaac_attn_tile.cuh"
 
 namespace gaac {
 
-#ifndef GAAC_LUTC
-#define GAAC_LUTC 0
-#endif
-// Softmax weights enter the PV product as BF16 (tensor-core operand).  GAAC_SPLIT_P = 1: each weight goes in as the sum of two
-// BF16 numbers, its rounded value and the rounded remainder (two MMAs on the same V fragments), which brings the relative error
-// of a weight from 2^-8 down to 2^-16; = 0: the rounded value only, as the reference kernel does (gaac/kernel.py:178).
-#ifndef GAAC_SPLIT_P
-#define GAAC_SPLIT_P 1
-#endif
-// Build-time knobs of the experiments that shaped the kernel (the defaults are what ships):
-//   GAAC_WARPS    warps per CTA (one CTA per SM; the register budget per thread follows from it).  Only 16 is tested for results;
-//                 12 and 18 were timing experiments, 8 is known to give wrong output
-//   GAAC_ESC_WIN  escape bytes staged per tile and kind
-//   GAAC_QSMEM    1: the query fragments live in a shared-memory table read once per K group instead of 16 registers per lane
-#ifndef GAAC_WARPS
-#define GAAC_WARPS 16
-#endif
-#ifndef GAAC_ESC_WIN
-#define GAAC_ESC_WIN 256
-#endif
-#ifndef GAAC_QSMEM
-#define GAAC_QSMEM 0
-#endif
-//   GAAC_ALU2FMA  bit mask of integer operations of the group decoder written as multiply-adds, which issue on the FMA pipe
-//                 instead of the half-rate ALU pipe: 1 = the >> 12 of the code word as a high multiply, 2 = the three-term
-//                 exponent sum as two multiply-adds by 1, 4 = the escape position advance as a multiply-add by 1
-#ifndef GAAC_ALU2FMA
-#define GAAC_ALU2FMA 0
-#endif
-//   GAAC_ABLATE   timing-only builds that compute WRONG results, to see where the time goes: 1 = no rebuild at all (fragments
-//                 taken from the staged bytes as they are), 2 = every group decoded as tier 0 (no tags, no escape bytes),
-//                 3 = raw tier compiled out
-#ifndef GAAC_ABLATE
-#define GAAC_ABLATE 0
-#endif
-//   GAAC_RAWPATCH 1: raw-tier groups are resolved by a short pass per tile that turns each of them into a table entry, after
-//                 which the group decoder has no branch at all; 0: the decoder branches on the raw tag of every group
-#ifndef GAAC_RAWPATCH
-#define GAAC_RAWPATCH 1
-#endif
-//   GAAC_DEEP     1: a warp's copies run a whole tile ahead: the stage it has just consumed is refilled at once with the tile after
-//                 the next one; 0: the next tile's copies are issued in the middle of the current tile (half a tile ahead).
-//                 Measured 2 % SLOWER at 1 (with and without the rebuild): the copies already arrive in time, the kernel waits
-//                 for instruction issue, not for memory
-#ifndef GAAC_DEEP
-#define GAAC_DEEP 0
-#endif
-constexpr int ATT_WARPS = GAAC_WARPS;
-constexpr int ATT_THREADS = ATT_WARPS * 32;
-constexpr int NSTAGE = 2;
-constexpr int ESC_WIN = GAAC_ESC_WIN;                       // escape bytes staged per tile and kind; longer tiles read theirs from global memory
-// ---- stage layout (bytes)
-// Stage = 16 bytes (mbarrier, then 8 bytes that stay zero) + a block per side:
-//   sign/mantissa (2048, storage order) | codes (768) | tag words (64) | escape window (ESC_WIN + 16: it starts at the
-//   16-byte boundary below the tile's first escape byte).  Every piece is ONE bulk copy: copies of 128 bytes (one per
-//   row, skewed to avoid the bank conflicts of the storage order) were measured 15 % slower, the copy engine wants few large
-//   copies, so the fragment reads accept a 2-way (K) / 4-way (V) conflict.
-// A side block is laid out as the paged tile slot is, so the paged layout fetches a whole slot with one copy.
-constexpr int ESC_COPY = ESC_WIN + 16;
-constexpr int SM_ROW = 128;
-constexpr int SB_SM = 0, SB_CD = SB_SM + 16 * SM_ROW, SB_FL = SB_CD + 768, SB_ESC = SB_FL + 64, SIDE_BYTES = SB_ESC + ESC_COPY;
-constexpr int ST_MBAR = 0, ST_ZERO = 8, ST_K = 16, ST_V = ST_K + SIDE_BYTES;
-constexpr int ST_KSM = ST_K + SB_SM, ST_KCD = ST_K + SB_CD, ST_KFL = ST_K + SB_FL, ST_KESC = ST_K + SB_ESC;
-constexpr int ST_VSM = ST_V + SB_SM, ST_VCD = ST_V + SB_CD, ST_VFL = ST_V + SB_FL, ST_VESC = ST_V + SB_ESC;
-constexpr int STAGE_BYTES = ST_V + SIDE_BYTES;
-static_assert(SB_CD - SB_SM == SLOT_CD_OFF && SB_FL - SB_SM == SLOT_FL_OFF && SB_ESC - SB_SM == SLOT_OVF_OFF, "side block laid out as the paged tile slot");
-constexpr int META_TILES = 512;                      // tiles of a CTA's range whose metadata is staged (longer ranges read the rest from global)
-// CTA tables: escape-byte table (2 KiB), K / V base words, per-tile metadata, and the code table: four 3-bit codes -> four bytes
-// for all 4096 values of a 12-bit field (16 KiB).  The table turns four logic instructions per lookup into one shared-memory load.
-constexpr int TB_LUTX = 0, TB_KB = 2048, TB_VB = TB_KB + 256, TB_META = TB_VB + 256, TB_LUTC = TB_META + 2 * META_TILES * 4;
-constexpr int TB_Q = TB_LUTC + (GAAC_LUTC ? 4096 * 4 : 0);          // query fragments: [4 K groups][32 lanes] x 16 bytes
-constexpr int TABLE_BYTES = TB_Q + (GAAC_QSMEM ? 4 * 32 * 16 : 0);
-// Raw-tier patch table of a warp: per side PATCH_MAX entries of 8 bytes = the two exponent addends of a raw group with the
-// 4-bit-window base already taken off (the decoder adds that base to every promoted group).  Tiles with more raw groups on a
-// side (random bit patterns) take the decoder that branches.
-constexpr int PATCH_MAX = 32, PATCH_BYTES = 2 * PATCH_MAX * 8;
-constexpr int WARP_SMEM = NSTAGE * STAGE_BYTES + PATCH_BYTES;
-constexpr int ATT_SMEM = TABLE_BYTES + ATT_WARPS * WARP_SMEM;
-static_assert(TABLE_BYTES % 16 == 0 && STAGE_BYTES % 16 == 0 && ST_KSM % 16 == 0 && ST_KCD % 16 == 0 && ST_KFL % 16 == 0 && ST_KESC % 16 == 0 &&
-              ST_VSM % 16 == 0 && ST_VCD % 16 == 0 && ST_VFL % 16 == 0 && ST_VESC % 16 == 0 && ESC_COPY % 16 == 0 && ST_MBAR % 8 == 0 && SM_ROW % 16 == 0,
+// Warps per CTA (20 warps at 96 registers measured 3 % slower: the kernel is short of issue slots, not of warps, and what they work on takes ring space).
+constexpr int ATT_WARPS = 16, ATT_THREADS = ATT_WARPS * 32;
+// ---- ring of stages.  A stage holds TPS consecutive tiles.
+//   slot layout:  per side  sign/mantissa of the tiles (TPS x 2048) | codes (TPS x 768) | tag words (TPS x 64) | the tiles' escape bytes, which are
+//                 contiguous in memory: one window of at most SIDE_ESC bytes that starts at the 16-byte boundary below the first
+//   paged layout: TPS x {K slot, V slot}, each as it lies in the block buffer (one copy per slot, at most PSLOT bytes of it)
+// Four tiles per stage: eight copies of 256 B .. 8 KB per four tile pairs; eight stages keep sixteen tiles in flight behind the sixteen in use.
+constexpr int TPS = 4, NSTG = 8;
+constexpr int SIDE_ESC = TPS * (ESC_WIN + 16);
+constexpr int SB_CD = TPS * TILE_SM, SB_FL = SB_CD + TPS * TILE_CD, SB_ESC = SB_FL + TPS * 4 * T, SIDE_BYTES = SB_ESC + SIDE_ESC;
+constexpr int STAGE_BYTES = 2 * SIDE_BYTES;
+static_assert(SIDE_BYTES == TPS * PSLOT, "both layouts use stages of the same size");
+constexpr int META_TILES = 1024;                   // tiles of a CTA's range whose metadata is staged (longer ranges read the rest from global)
+// CTA tables: escape-byte table, K / V base words, zero bytes, the stages' mbarriers, use counts
+// and escape windows {K start, K bytes, V start, V bytes}, the per-tile metadata of the range, the warps' scratch
+constexpr int TB_LUTX = 0, TB_BASES = LUTX_BYTES, TB_ZERO = TB_BASES + BASES_BYTES, TB_FULL = TB_ZERO + 16, TB_DONE = TB_FULL + 8 * NSTG, TB_WIN = TB_DONE + 4 * NSTG, TB_META = TB_WIN + 16 * NSTG,
+              TB_RING = TB_META + 2 * META_TILES * 4, TB_SCRATCH = TB_RING + NSTG * STAGE_BYTES;
+constexpr int ATT_SMEM = TB_SCRATCH + ATT_WARPS * WARP_SCRATCH;
+static_assert(TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_WIN % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
               "bulk copies need 16-byte aligned shared-memory destinations and sizes");
 static_assert(ATT_SMEM + 64 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
 static_assert(ATT_THREADS / 128 * 2 >= 8, "the fused exchange keeps at most two merged heads per thread");
-constexpr unsigned FULLM = 0xffffffffu;
-constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+static_assert((TPS & (TPS - 1)) == 0 && (NSTG & (NSTG - 1)) == 0, "");
+constexpr int ACC_LD = D + 8;                        // row stride of the staged accumulators: 8j + r banks, conflict-free stores
 
 struct AttnParams {
   // slot layout
@@ -140,463 +70,6 @@ struct AttnParams {
   // debug instantiation only: the rebuilt BF16 K / V rows are written to [B*n_kv, dump_S, 128] (row = token of the head)
   uint16_t* dump_k; uint16_t* dump_v; long dump_S;
 };
-
-#ifndef GAAC_MMA_VOLATILE
-#define GAAC_MMA_VOLATILE 1
-#endif
-#if GAAC_MMA_VOLATILE
-#define GAAC_MMA_ASM asm volatile
-#else
-#define GAAC_MMA_ASM asm
-#endif
-__device__ __forceinline__ void mma16816(float* c, const u32* a, u32 b0, u32 b1) {
-  GAAC_MMA_ASM("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// ---- bulk asynchronous copies (TMA engine, no tensor map): global -> shared, completion counted in bytes on an mbarrier.
-// Both addresses are 16-byte aligned and the size is a multiple of 16 at every call site.
-__device__ __forceinline__ void mbar_init(u32 mbar, u32 count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(count)); }
-__device__ __forceinline__ void mbar_expect_tx(u32 mbar, u32 bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_add_tx(u32 mbar, u32 bytes) { asm volatile("mbarrier.expect_tx.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory"); }
-__device__ __forceinline__ void mbar_arrive(u32 mbar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory"); }
-__device__ __forceinline__ void bulk_g2s(u32 dst, const void* src, u32 bytes, u32 mbar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
-}
-// Bounded wait for a phase of the barrier: false when it gave up (the copies of a stage normally land within microseconds;
-// the bound is there so that a lost copy can never hang the GPU).
-constexpr int MBAR_WAIT_LIMIT = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(u32 mbar, u32 parity) {
-  for (int it = 0; it < MBAR_WAIT_LIMIT; it++) {
-    u32 ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ float fast_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
-// What a warp remembers of a tile between issuing its copies and consuming it.  Slot layout: offsets of the tile's escape
-// bytes inside the head's escape bytes.  Paged layout: the mode-table entries (>= 0: compressed slot, < 0: bit-complement
-// of a raw tile of the pool).
-struct TileMeta { int mk, mv; };
-
-// Per-head values of the slot layout that the copy addressing needs.
-struct LaneAddr {
-  int ohk, ohv;                  // first escape byte of the head inside ovf
-  int availk, availv;            // bytes from there to the end of the allocation (clamped to int)
-};
-
-// Running state of one warp.
-struct WarpAcc {
-  float acc[8][4];       // m-tile mt: c0 = O[dim 16mt+r][head 2j], c1 = [..][2j+1], c2 = O[16mt+r+8][2j], c3 = [..][2j+1]
-  float m0, m1, l0, l1;  // heads 2j, 2j+1 (exp2 domain); l summed over this lane's tokens only
-};
-
-// Online softmax on the score fragment + P^T B-fragments for the PV product.
-// The running maximum is only raised (and the accumulators rescaled) when some score of the tile exceeds it by more than
-// RESCALE_TAU in the exp2 domain; otherwise the tile is weighted against the stale maximum, so P stays below 2^RESCALE_TAU.
-// Sums and accumulators are fp32 and P keeps its relative BF16 rounding, so the result is as exact as with the true
-// maximum, and the common tile needs no cross-lane reduction, no rescale factor and no accumulator multiply.
-constexpr float RESCALE_TAU = 16.f;
-// P^T B-fragments of one tile for the PV product: hi = the weights rounded to BF16, lo = the BF16-rounded remainders.
-struct PFrag { u32 hi0, hi1, lo0, lo1; };
-template <bool FULL_TILE>
-__device__ __forceinline__ void softmax_step(WarpAcc& A, const float* sc, float scale_log2, int nvalid, int lane, PFrag& P) {
-  const int j = lane & 3, r = lane >> 2;
-  const bool v0 = FULL_TILE || r < nvalid, v8 = FULL_TILE || r + 8 < nvalid;     // a full tile needs no token masks
-  const float s00 = v0 ? sc[0] * scale_log2 : -CUDART_INF_F, s01 = v0 ? sc[1] * scale_log2 : -CUDART_INF_F;
-  const float s80 = v8 ? sc[2] * scale_log2 : -CUDART_INF_F, s81 = v8 ? sc[3] * scale_log2 : -CUDART_INF_F;
-  float mt0 = fmaxf(s00, s80), mt1 = fmaxf(s01, s81);
-  if (__any_sync(FULLM, mt0 > A.m0 + RESCALE_TAU || mt1 > A.m1 + RESCALE_TAU)) {
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) { mt0 = fmaxf(mt0, __shfl_xor_sync(FULLM, mt0, o)); mt1 = fmaxf(mt1, __shfl_xor_sync(FULLM, mt1, o)); }
-    const float mn0 = fmaxf(A.m0, mt0), mn1 = fmaxf(A.m1, mt1);
-    const float al0 = (mn0 == -CUDART_INF_F) ? 0.f : fast_exp2(A.m0 - mn0), al1 = (mn1 == -CUDART_INF_F) ? 0.f : fast_exp2(A.m1 - mn1);
-    A.l0 *= al0; A.l1 *= al1; A.m0 = mn0; A.m1 = mn1;
-#pragma unroll
-    for (int n = 0; n < 8; n++) { A.acc[n][0] *= al0; A.acc[n][2] *= al0; A.acc[n][1] *= al1; A.acc[n][3] *= al1; }
-  }
-  const float mu0 = fmaxf(A.m0, -1e30f), mu1 = fmaxf(A.m1, -1e30f);       // a maximum of -inf (nothing seen yet) must not produce inf - inf
-  const float p00 = fast_exp2(s00 - mu0), p80 = fast_exp2(s80 - mu0), p01 = fast_exp2(s01 - mu1), p81 = fast_exp2(s81 - mu1);
-  A.l0 += p00 + p80; A.l1 += p01 + p81;
-  // this lane publishes W0 = (P[tok r][2j], P[tok r][2j+1]), W8 = (P[tok r+8][2j], P[tok r+8][2j+1]);
-  // it needs b0 = (P[tok 2j][head r], P[tok 2j+1][head r]), b1 = the same for tokens 2j+8, 2j+9
-  __nv_bfloat162 x = __floats2bfloat162_rn(p00, p01), y = __floats2bfloat162_rn(p80, p81);
-  const u32 W0 = *reinterpret_cast<u32*>(&x), W8 = *reinterpret_cast<u32*>(&y);
-  const int srcA = 8 * j + (r >> 1), srcB = srcA + 4;
-  const u32 a0 = __shfl_sync(FULLM, W0, srcA), a8 = __shfl_sync(FULLM, W8, srcA), b0w = __shfl_sync(FULLM, W0, srcB), b8w = __shfl_sync(FULLM, W8, srcB);
-  const u32 sel = (r & 1) ? 0x7632u : 0x5410u;
-  P.hi0 = prmt(a0, b0w, sel); P.hi1 = prmt(a8, b8w, sel);
-#if GAAC_SPLIT_P
-  // what the rounding dropped, exactly (p - bf16(p) is representable in fp32), rounded to BF16 in turn and routed the same way
-  __nv_bfloat162 xl = __floats2bfloat162_rn(p00 - __uint_as_float(W0 << 16), p01 - __uint_as_float(W0 & 0xFFFF0000u));
-  __nv_bfloat162 yl = __floats2bfloat162_rn(p80 - __uint_as_float(W8 << 16), p81 - __uint_as_float(W8 & 0xFFFF0000u));
-  const u32 L0 = *reinterpret_cast<u32*>(&xl), L8 = *reinterpret_cast<u32*>(&yl);
-  const u32 c0 = __shfl_sync(FULLM, L0, srcA), c8 = __shfl_sync(FULLM, L8, srcA), d0w = __shfl_sync(FULLM, L0, srcB), d8w = __shfl_sync(FULLM, L8, srcB);
-  P.lo0 = prmt(c0, d0w, sel); P.lo1 = prmt(c8, d8w, sel);
-#else
-  P.lo0 = P.lo1 = 0u;
-#endif
-}
-
-// PV for one pair of V words: tokens (2j, 2j+1, 2j+8, 2j+9) x elements (4w .. 4w+3).
-__device__ __forceinline__ void pv_words(WarpAcc& A, int w, const u32 (&u01)[4], const u32 (&u23)[4], const PFrag& P) {
-#if GAAC_SPLIT_P && defined(GAAC_PV_INTERLEAVE)
-  // the two MMAs into one accumulator depend on each other: issue the two independent ones in between
-  u32 a[4], c[4];
-  a[0] = prmt(u01[0], u01[1], 0x5410); a[2] = prmt(u01[2], u01[3], 0x5410);     // dim 8(4w)+r
-  a[1] = prmt(u01[0], u01[1], 0x7632); a[3] = prmt(u01[2], u01[3], 0x7632);     // dim 8(4w+1)+r
-  c[0] = prmt(u23[0], u23[1], 0x5410); c[2] = prmt(u23[2], u23[3], 0x5410);     // dim 8(4w+2)+r
-  c[1] = prmt(u23[0], u23[1], 0x7632); c[3] = prmt(u23[2], u23[3], 0x7632);     // dim 8(4w+3)+r
-  mma16816(A.acc[2 * w], a, P.hi0, P.hi1);
-  mma16816(A.acc[2 * w + 1], c, P.hi0, P.hi1);
-  mma16816(A.acc[2 * w], a, P.lo0, P.lo1);
-  mma16816(A.acc[2 * w + 1], c, P.lo0, P.lo1);
-#else
-  u32 a[4];
-  a[0] = prmt(u01[0], u01[1], 0x5410); a[2] = prmt(u01[2], u01[3], 0x5410);     // dim 8(4w)+r
-  a[1] = prmt(u01[0], u01[1], 0x7632); a[3] = prmt(u01[2], u01[3], 0x7632);     // dim 8(4w+1)+r
-  mma16816(A.acc[2 * w], a, P.hi0, P.hi1);
-#if GAAC_SPLIT_P
-  mma16816(A.acc[2 * w], a, P.lo0, P.lo1);
-#endif
-  a[0] = prmt(u23[0], u23[1], 0x5410); a[2] = prmt(u23[2], u23[3], 0x5410);     // dim 8(4w+2)+r
-  a[1] = prmt(u23[0], u23[1], 0x7632); a[3] = prmt(u23[2], u23[3], 0x7632);     // dim 8(4w+3)+r
-  mma16816(A.acc[2 * w + 1], a, P.hi0, P.hi1);
-#if GAAC_SPLIT_P
-  mma16816(A.acc[2 * w + 1], a, P.lo0, P.lo1);
-#endif
-#endif
-}
-
-// rowoff / total as scan_rows leaves them: escape bytes (low half) and raw groups (high half) before the row, or of the tile
-__device__ __forceinline__ int esc_part(int v) { return v & 0xFFFF; }
-__device__ __forceinline__ int raw_part(int v) { return v >> 16; }
-
-// Q^T B-fragments of the score product.  Lane (j, r) holds, for k-step s, the words q[head r][16s + 2j, +1] and
-// q[head r][16s + 2j + 8, +9]; K group g of a lane uses k-steps 2g and 2g + 1.
-#if GAAC_QSMEM
-struct QFrag {
-  const uint4* tab;                                   // [4][32] in shared memory, built once per CTA
-  __device__ __forceinline__ void group(int g, int lane, u32 (&b)[4]) const { const uint4 v = tab[g * 32 + lane]; b[0] = v.x; b[1] = v.y; b[2] = v.z; b[3] = v.w; }
-};
-#else
-struct QFrag {
-  u32 qa[8][2];
-  __device__ __forceinline__ void group(int g, int, u32 (&b)[4]) const { b[0] = qa[2 * g][0]; b[1] = qa[2 * g][1]; b[2] = qa[2 * g + 1][0]; b[3] = qa[2 * g + 1][1]; }
-};
-#endif
-
-// Escape bytes of one tile as read by the group decoder.
-//   staged window (WIN): zp = shared-memory address of a zero byte below the tile's first escape byte; a group without an
-//     escape byte reads zp[0] and a 4-bit-window group reads zp[off + pos]: one multiply-add, no branch.
-//   global memory (!WIN, tiles whose escapes exceed the window): plain loads at glob[pos].
-//   off = distance from zp to the tile's first escape byte (the zero byte a group without escapes reads sits at zp[0]).
-template <bool WIN> struct EscSrc { const uint8_t* zp; const uint8_t* glob; int off; };
-
-// ---- byte-SWAR pieces written for the pipes of the SM: logic ops (LOP3 / PRMT / SHF) run on the ALU pipe, whose rate is half
-// the issue rate, so shifts that can be merged with an add are written as multiply-adds (FMA pipe) and the 3-bit -> byte
-// spreading of the codes is a table lookup (load/store pipe).
-template <u32 K> __device__ __forceinline__ u32 mad_k(u32 a, u32 c) {
-  u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "n"(K), "r"(c)); return d;
-}
-__device__ __forceinline__ void bf16x4_dev(u32 sm4, u32 e4, u32& p01, u32& p23) {
-  const u32 eh = __umulhi(e4, 0x80000000u);                          // e4 >> 1
-  const u32 el = mad_k<128u>(e4, 0u);                                // e4 << 7
-  const u32 h4 = (sm4 & 0x80808080u) | (eh & 0x7F7F7F7Fu);
-  const u32 l4 = (el & 0x80808080u) | (sm4 & 0x7F7F7F7Fu);
-  p01 = prmt(l4, h4, 0x5140); p23 = prmt(l4, h4, 0x7362);
-}
-// four 5-bit fields at bits 0..19 of u -> field << 3 per byte (raw-tier exponent high bits); same result as spread_hi5
-__device__ __forceinline__ u32 spread_hi5_dev(u32 u) {
-  const u32 y = mad_k<64u>(u & 0xFFC00u, u & 0x3FFu);               // fields 0,1 at bits 0-9, fields 2,3 at bits 16-25
-  return mad_k<64u>(y & 0x03E003E0u, (y & 0x001F001Fu) << 3);       // odd fields up 3 more bits, everything << 3
-}
-
-// Rebuild one group (two sign/mantissa words) into four bf16x2 words.  Same results as decode_group_lut (gaac_tile.h);
-// pos16 = es.off + escape position of the group, advanced past it on return; lutc = the 4096-entry code table.
-// RT (only with WIN): raw groups were turned into patch-table entries by build_raw_patches, which also left each entry's number in
-// the first payload byte of its group: the addends of EVERY group then come from one load, out of the escape-byte table
-// (byte = the 4-bit-window escape byte, or the zero byte) or out of the patch table (byte = entry number), chosen by address
-// arithmetic, and the decoder has no branch.  patch_rel = patch table address - escape-byte table address (shared memory).
-template <bool WIN, bool RT>
-__device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 c24, u32 tg, int& pos16, const EscSrc<WIN>& es,
-                                                 const u32x2* lutx, const uint8_t* lutc, const u32x4& bw, u32 out[4], u32 patch_rel = 0u) {
-  static_assert(WIN || !RT, "the patch table goes with the staged escape window");
-  const u32 m1 = tg & 1u;                             // promoted (tags are 0, 1 or 3)
-  u32 xe;
-  if (WIN) xe = es.zp[m1 * (u32)pos16];               // raw groups read a payload byte here; their addends are replaced below
-  else xe = m1 ? es.glob[pos16 - es.off] : 0u;
-  u32 x0, x1;
-  if (RT) {
-    const u32 r2 = tg & 2u;                           // 2 for a raw group
-    const u32x2 x = *reinterpret_cast<const u32x2*>(reinterpret_cast<const uint8_t*>(lutx) + (8u * xe + r2 * (patch_rel >> 1)));
-    x0 = x.x; x1 = x.y;
-    pos16 += (int)(2u * r2);                          // a raw payload is five bytes: four here, one below with every promoted group
-  } else {
-    const u32x2 x = lutx[xe];
-    x0 = x.x; x1 = x.y;
-  }
-#if GAAC_LUTC == 1
-  const u32 c_lo = *reinterpret_cast<const u32*>(lutc + ((c24 << 2) & 0x3FFCu));
-  const u32 c_hi = *reinterpret_cast<const u32*>(lutc + ((c24 >> 10) & 0x3FFCu));
-#elif GAAC_LUTC == 2
-  // one half through the table (load/store pipe), the other half by arithmetic (ALU + FMA pipes): balances the pipes
-  const u32 c_lo = *reinterpret_cast<const u32*>(lutc + ((c24 << 2) & 0x3FFCu));
-  const u32 th = (c24 >> 12) & 0xFFFu;
-  const u32 xh = mad_k<1023u>((c24 >> 12) & 0xFC0u, th);
-  const u32 c_hi = mad_k<31u>(xh & 0x00380038u, xh);
-#else
-  // four 3-bit codes -> four bytes in two steps; each step moves the upper fields with a multiply-add: (t & M) * (2^k - 1) + t
-#if GAAC_ALU2FMA & 1
-  const u32 c12 = __umulhi(c24, 1u << 20);            // c24 >> 12
-#else
-  const u32 c12 = c24 >> 12;
-#endif
-  const u32 tl = c24 & 0xFFFu, th = c12 & 0xFFFu;
-  const u32 xl = mad_k<1023u>(c24 & 0xFC0u, tl), xh = mad_k<1023u>(c12 & 0xFC0u, th);
-  const u32 c_lo = mad_k<31u>(xl & 0x00380038u, xl), c_hi = mad_k<31u>(xh & 0x00380038u, xh);
-#endif
-  const u32 blo = bw.x + m1 * bw.z, bhi = bw.y + m1 * bw.w;
-#if GAAC_ABLATE == 3
-  if (false) {
-#else
-  if (!RT && (tg & 2u)) {                             // raw exponents: e = code | hi5 << 3 (the base must not contribute)
-#endif
-    u32 w0, w1; int sh;
-    if (WIN) {
-      const u32 a = (u32)__cvta_generic_to_shared(es.zp) + (u32)pos16;
-      sh = 8 * (int)(a & 3u);
-      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(a & ~3u) : "memory");
-      asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(a & ~3u) : "memory");
-    } else {
-      const uint8_t* p = es.glob + (pos16 - es.off);
-      sh = 8 * (int)(reinterpret_cast<uintptr_t>(p) & 3);
-      const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-      w0 = a[0]; w1 = a[1];
-    }
-    const u32 lo = funnel_r(w0, w1, sh), hi = w1 >> sh;              // bytes 0-3 and byte 4 of the payload
-    x0 = spread_hi5_dev(lo & 0xFFFFFu) - blo;
-    x1 = spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - bhi;
-    pos16 += 4;
-  }
-#if GAAC_ALU2FMA & 4
-  pos16 = (int)mad_k<1u>(m1, (u32)pos16);
-#else
-  pos16 += (int)m1;
-#endif
-#if GAAC_ALU2FMA & 2
-  bf16x4_dev(sm_lo, mad_k<1u>(c_lo, mad_k<1u>(blo, x0)), out[0], out[1]);
-  bf16x4_dev(sm_hi, mad_k<1u>(c_hi, mad_k<1u>(bhi, x1)), out[2], out[3]);
-#else
-  bf16x4_dev(sm_lo, c_lo + blo + x0, out[0], out[1]);
-  bf16x4_dev(sm_hi, c_hi + bhi + x1, out[2], out[3]);
-#endif
-}
-
-// Scores of one compressed K tile: sc += K . Q^T.  flrow / rowoff: tag word and escape offset of row (lane & 15) held by
-// lanes 0-15.
-// dump (debug instantiation only): where token 0 of this tile goes in the [token][128] dump of the head; every lane writes the
-// fragment words it rebuilt at the (token, channel) pairs they stand for, rows >= nvalid are left alone.
-template <bool WIN, bool DUMP, bool RT = false>
-__device__ __forceinline__ void k_scores(float* sc, const uint8_t* stage, const uint8_t* tables, const EscSrc<WIN>& es, u32 flrow, int rowoff,
-                                         int lane, const QFrag& Q, uint16_t* dump = nullptr, int nvalid = T, u32 patch_rel = 0u) {
-  const int j = lane & 3, r = lane >> 2;
-  const u32x2* lutx = reinterpret_cast<const u32x2*>(tables + TB_LUTX);
-  u32 t8[2]; int pos[2]; uint4 s0[2], s1[2]; u32 cd[2][3];
-  float s2[4] = {0.f, 0.f, 0.f, 0.f};                  // second accumulator: two dependent MMA chains of four instead of one of eight
-#pragma unroll
-  for (int o = 0; o < 2; o++) {
-    const u32 fl = __shfl_sync(FULLM, flrow, 8 * o + r);
-    pos[o] = esc_part(__shfl_sync(FULLM, rowoff, 8 * o + r)) + esc_prefix(fl, 8 * j) + es.off;
-    t8[o] = fl >> (8 * j);
-    s0[o] = *reinterpret_cast<const uint4*>(stage + ST_KSM + (8 * o + (lane >> 2)) * SM_ROW + 32 * (lane & 3));   // storage order, skewed rows
-    s1[o] = *reinterpret_cast<const uint4*>(stage + ST_KSM + (8 * o + (lane >> 2)) * SM_ROW + 32 * (lane & 3) + 16);
-    const u32* c = reinterpret_cast<const u32*>(stage + ST_KCD + o * 384 + 12 * lane);
-    cd[o][0] = c[0]; cd[o][1] = c[1]; cd[o][2] = c[2];
-  }
-#pragma unroll
-  for (int g = 0; g < 4; g++) {
-    const u32x4 bw = *reinterpret_cast<const u32x4*>(tables + TB_KB + 16 * (4 * j + g));
-    u32 f[2][4];
-#pragma unroll
-    for (int o = 0; o < 2; o++) {
-      const u32 smlo = g == 0 ? s0[o].x : g == 1 ? s0[o].z : g == 2 ? s1[o].x : s1[o].z;
-      const u32 smhi = g == 0 ? s0[o].y : g == 1 ? s0[o].w : g == 2 ? s1[o].y : s1[o].w;
-#if GAAC_ABLATE == 1
-      f[o][0] = smlo; f[o][1] = smhi; f[o][2] = smlo ^ cd[o][0]; f[o][3] = smhi ^ cd[o][g % 3];
-#elif GAAC_ABLATE == 2
-      decode_group_dev<WIN, RT>(smlo, smhi, k_group_codes(cd[o], g), 0u, pos[o], es, lutx, tables + TB_LUTC, bw, f[o], patch_rel);
-#else
-      decode_group_dev<WIN, RT>(smlo, smhi, k_group_codes(cd[o], g), t8[o] >> (2 * g), pos[o], es, lutx, tables + TB_LUTC, bw, f[o], patch_rel);
-#endif
-    }
-    if (DUMP) {
-#pragma unroll
-      for (int o = 0; o < 2; o++)
-        if (8 * o + r < nvalid) {
-          u32* row = reinterpret_cast<u32*>(dump + (8 * o + r) * D);
-          row[(32 * g + 2 * j) >> 1] = f[o][0]; row[(32 * g + 2 * j + 8) >> 1] = f[o][1];
-          row[(32 * g + 16 + 2 * j) >> 1] = f[o][2]; row[(32 * g + 16 + 2 * j + 8) >> 1] = f[o][3];
-        }
-    }
-    u32 qb[4];
-    Q.group(g, lane, qb);
-    { const u32 a[4] = {f[0][0], f[1][0], f[0][1], f[1][1]}; mma16816(sc, a, qb[0], qb[1]); }
-    { const u32 a[4] = {f[0][2], f[1][2], f[0][3], f[1][3]}; mma16816(s2, a, qb[2], qb[3]); }
-  }
-  sc[0] += s2[0]; sc[1] += s2[1]; sc[2] += s2[2]; sc[3] += s2[3];
-}
-
-// O^T += V^T . P^T for one compressed V tile.  flrow / rowoff of V row (lane & 15) are held by lanes 16-31.
-template <bool WIN, bool DUMP, bool RT = false>
-__device__ __forceinline__ void v_accum(WarpAcc& A, const uint8_t* stage, const uint8_t* tables, const EscSrc<WIN>& es, u32 flrow, int rowoff,
-                                        int lane, const PFrag& P, uint16_t* dump = nullptr, int nvalid = T, u32 patch_rel = 0u) {
-  const int j = lane & 3, r = lane >> 2;
-  const u32x2* lutx = reinterpret_cast<const u32x2*>(tables + TB_LUTX);
-  u32 t4[4]; int pos[4]; uint4 sm[4]; u32 cd[6];
-#pragma unroll
-  for (int t = 0; t < 4; t++) {
-    const int tok = 2 * j + (t & 1) + 8 * (t >> 1);
-    const u32 fl = __shfl_sync(FULLM, flrow, 16 + tok);
-    pos[t] = esc_part(__shfl_sync(FULLM, rowoff, 16 + tok)) + esc_prefix(fl, 4 * r) + es.off;
-    t4[t] = fl >> (4 * r);
-    sm[t] = *reinterpret_cast<const uint4*>(stage + ST_VSM + (lane >> 1) * SM_ROW + 64 * (lane & 1) + 16 * t);
-  }
-  {
-    const uint2* c2 = reinterpret_cast<const uint2*>(stage + ST_VCD + 24 * lane);
-    uint2 ca = c2[0], cb = c2[1], cc = c2[2];
-    cd[0] = ca.x; cd[1] = ca.y; cd[2] = cb.x; cd[3] = cb.y; cd[4] = cc.x; cd[5] = cc.y;
-  }
-#pragma unroll
-  for (int g = 0; g < 2; g++) {
-    const u32x4 bw = *reinterpret_cast<const u32x4*>(tables + TB_VB + 16 * (2 * r + g));
-    u32 f[4][4];
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const u32 smlo = g == 0 ? sm[t].x : sm[t].z, smhi = g == 0 ? sm[t].y : sm[t].w;
-#if GAAC_ABLATE == 1
-      f[t][0] = smlo; f[t][1] = smhi; f[t][2] = smlo ^ cd[g]; f[t][3] = smhi ^ cd[g + 3];
-#elif GAAC_ABLATE == 2
-      decode_group_dev<WIN, RT>(smlo, smhi, v_group_codes(cd, t, g), 0u, pos[t], es, lutx, tables + TB_LUTC, bw, f[t], patch_rel + PATCH_MAX * 8);
-#else
-      decode_group_dev<WIN, RT>(smlo, smhi, v_group_codes(cd, t, g), t4[t] >> (2 * g), pos[t], es, lutx, tables + TB_LUTC, bw, f[t], patch_rel + PATCH_MAX * 8);
-#endif
-    }
-    if (DUMP) {
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int tok = 2 * j + (t & 1) + 8 * (t >> 1);
-        if (tok < nvalid) {
-#pragma unroll
-          for (int i = 0; i < 4; i++) {                // word i = stored positions 16r + 8g + 2i, +1  <->  channels 8(8g + 2i) + r, 8(8g + 2i + 1) + r
-            dump[tok * D + 8 * (8 * g + 2 * i) + r] = (uint16_t)(f[t][i] & 0xFFFFu);
-            dump[tok * D + 8 * (8 * g + 2 * i + 1) + r] = (uint16_t)(f[t][i] >> 16);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const u32 u01[4] = {f[0][2 * h], f[1][2 * h], f[2][2 * h], f[3][2 * h]};
-      const u32 u23[4] = {f[0][2 * h + 1], f[1][2 * h + 1], f[2][2 * h + 1], f[3][2 * h + 1]};
-      pv_words(A, 2 * g + h, u01, u23, P);
-    }
-  }
-}
-
-// Escape-byte offsets of the rows of a staged tile: lanes 0-15 scan the K rows, lanes 16-31 the V rows.  flrow = tag word of
-// row (lane & 15) of the lane's side (0 when that side is raw), rowoff = escape bytes of the rows before it, total = rowoff
-// of the row after it (lane 15 / 31 hold the tile's totals).
-__device__ __forceinline__ void scan_rows(const uint8_t* stage, bool rawk, bool rawv, int lane, u32& flrow, int& rowoff, int& total) {
-  const int row = lane & 15;
-  const bool isv = lane >= 16;
-  flrow = (isv ? rawv : rawk) ? 0u : *reinterpret_cast<const u32*>(stage + (isv ? ST_VFL : ST_KFL) + 4 * row);
-  // one scan for two prefixes: escape bytes in the low half, raw groups in the high half (a tile has at most 1280 and 256 of them)
-  const int sz = row_esc_bytes(flrow) + (popc(flrow & 0xAAAAAAAAu) << 16);
-  int inc = sz;
-#pragma unroll
-  for (int d = 1; d < 16; d <<= 1) { int v = __shfl_up_sync(FULLM, inc, d, 16); if (row >= d) inc += v; }
-  rowoff = inc - sz; total = inc;
-}
-
-// Turn the raw-tier groups of a staged tile into patch-table entries, so that the group decoder needs no branch.  Lanes 0-15
-// own the K rows, lanes 16-31 the V rows (as in scan_rows); a lane walks the raw groups of its row.  For each one: read the
-// five payload bytes from the staged escape window, spread the 5-bit fields to byte positions, take off the 4-bit-window base
-// words (the decoder adds them to every promoted group), store the two words as entry k of the side's patch table, and write k
-// over the first payload byte, which is where the decoder looks for a promoted group's escape byte.  k = number of raw
-// groups before this one on the tile side (rows in order, groups ascending).  side_on[0/1]: whether the K / V side takes part.
-__device__ __forceinline__ void build_raw_patches(uint8_t* stage, const uint8_t* tables, uint8_t* patch, int off_k, int off_v, bool on_k, bool on_v,
-                                                  u32 flrow, int rowoff, int lane) {
-  const bool isv = lane >= 16;
-  u32 rb = (isv ? on_v : on_k) ? (flrow & 0xAAAAAAAAu) : 0u;
-  uint8_t* win = stage + ST_ZERO + (isv ? off_v : off_k);           // the tile side's first escape byte
-  const uint8_t* bws = tables + (isv ? TB_VB : TB_KB);
-  u32x2* ptab = reinterpret_cast<u32x2*>(patch + (isv ? PATCH_MAX * 8 : 0));
-  while (__any_sync(FULLM, rb != 0u)) {
-    if (rb) {
-      const int bit = __ffs(rb) - 1, g = bit >> 1;                  // raw bit of group g is bit 2g + 1
-      rb &= rb - 1u;
-      const u32 below = flrow & ((1u << (bit - 1)) - 1u);            // tag bits of the groups before g
-      const int pos = esc_part(rowoff) + popc(below & 0x55555555u) + 4 * popc(below & 0xAAAAAAAAu);
-      const int k = raw_part(rowoff) + popc(below & 0xAAAAAAAAu);
-      uint8_t* pl = win + pos;
-      const u32 a = (u32)__cvta_generic_to_shared(pl);
-      const int sh = 8 * (int)(a & 3u);
-      const u32 w0 = *reinterpret_cast<const u32*>(pl - (a & 3u)), w1 = *reinterpret_cast<const u32*>(pl - (a & 3u) + 4);
-      const u32 lo = funnel_r(w0, w1, sh), hi = w1 >> sh;            // bytes 0-3 and byte 4 of the payload
-      const u32x4 bw = *reinterpret_cast<const u32x4*>(bws + 16 * g);
-      ptab[k] = u32x2{spread_hi5_dev(lo & 0xFFFFFu) - (bw.x + bw.z), spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - (bw.y + bw.w)};
-      *pl = (uint8_t)k;
-    }
-  }
-  __syncwarp();
-}
-
-// Scores of a raw BF16 tile [16][128] in global memory (rows >= nvalid are not read).
-template <bool DUMP>
-__device__ __forceinline__ void raw_scores(float* sc, const uint16_t* kraw, int nvalid, int lane, const QFrag& Q, uint16_t* dump = nullptr) {
-  const int j = lane & 3, r = lane >> 2;
-  u32 qb[4];
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    u32 a[4];
-    if ((s & 1) == 0) Q.group(s >> 1, lane, qb);
-    const uint16_t* k0 = kraw + r * D + 16 * s + 2 * j;
-    const uint16_t* k8 = k0 + 8 * D;
-    a[0] = r < nvalid ? *reinterpret_cast<const u32*>(k0) : 0u; a[2] = r < nvalid ? *reinterpret_cast<const u32*>(k0 + 8) : 0u;
-    a[1] = r + 8 < nvalid ? *reinterpret_cast<const u32*>(k8) : 0u; a[3] = r + 8 < nvalid ? *reinterpret_cast<const u32*>(k8 + 8) : 0u;
-    if (DUMP) {
-      if (r < nvalid) { u32* row = reinterpret_cast<u32*>(dump + r * D); row[(16 * s + 2 * j) >> 1] = a[0]; row[(16 * s + 2 * j + 8) >> 1] = a[2]; }
-      if (r + 8 < nvalid) { u32* row = reinterpret_cast<u32*>(dump + (r + 8) * D); row[(16 * s + 2 * j) >> 1] = a[1]; row[(16 * s + 2 * j + 8) >> 1] = a[3]; }
-    }
-    mma16816(sc, a, qb[2 * (s & 1)], qb[2 * (s & 1) + 1]);
-  }
-}
-// O^T += V^T . P^T for a raw BF16 tile.
-template <bool DUMP>
-__device__ __forceinline__ void raw_accum(WarpAcc& A, const uint16_t* vraw, int nvalid, int lane, const PFrag& P, uint16_t* dump = nullptr) {
-  const int j = lane & 3, r = lane >> 2;
-#pragma unroll
-  for (int w = 0; w < 4; w++) {
-    u32 u01[4], u23[4];
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const int tok = 2 * j + (t & 1) + 8 * (t >> 1);
-      const uint16_t* vr = vraw + tok * D + 8 * (4 * w) + r;
-      const bool ok = tok < nvalid;
-      const u32 e0 = ok ? vr[0] : 0u, e1 = ok ? vr[8] : 0u, e2 = ok ? vr[16] : 0u, e3 = ok ? vr[24] : 0u;
-      u01[t] = e0 | (e1 << 16); u23[t] = e2 | (e3 << 16);
-      if (DUMP && ok) {
-        uint16_t* o = dump + tok * D + 8 * (4 * w) + r;
-        o[0] = (uint16_t)e0; o[8] = (uint16_t)e1; o[16] = (uint16_t)e2; o[24] = (uint16_t)e3;
-      }
-    }
-    pv_words(A, w, u01, u23, P);
-  }
-}
 
 // ---- cross-GPU exchange helpers.  A receive buffer holds 8-byte entries: the low word is an fp32 value, the high word the
 // number of the exchange it belongs to.  An entry is written with ONE 64-bit store and read with one 64-bit load, so a reader
@@ -637,17 +110,101 @@ __device__ __forceinline__ bool x_merge_rows(const unsigned long long* base, int
   return ok;
 }
 
-template <bool PAGED, bool DUMP>
+// ---- merge of the splits.  The ticket is taken with an acquire-release atomic at GPU scope by one thread between two CTA barriers: the
+// barrier before it orders every thread's partial stores before the release, the barrier after it orders the acquire before every
+// thread's loads of the other CTAs' partials - no per-thread fence is needed.
+__device__ __forceinline__ bool last_split(int* counter, int NS, int* s_last) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ticket;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
+    *s_last = (ticket == NS - 1);
+    if (ticket == NS - 1) *counter = 0;               // leave the counter ready for the next call
+  }
+  __syncthreads();
+  return *s_last != 0;
+}
+// Partials of rows row0 .. row0 + heads - 1 (heads <= HMAX <= 8) -> deliver(head, M, L, acc[threadIdx.x & 127]).  All loads are independent of one
+// another (no per-split dependent chain): scale factors first, then the weighted sum with one warp per split and 16-byte loads, then a
+// cross-warp sum in shared memory.
+template <int HMAX, class F>
+__device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area, long row0, int heads, const F& deliver) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, NS = p.nsplit;
+  float* c_f = reinterpret_cast<float*>(area);        // [heads][NS]  m, then exp2(m - M)
+  float* c_l = c_f + 8 * NS;                          // [heads][NS]  l
+  float* c_ML = c_l + 8 * NS;                         // [8][2]       M, L per head
+  float* c_red = c_ML + 16;                           // [W][8][128]  (NS <= 1024 keeps this inside the ring area)
+  for (int i = tid; i < heads * NS; i += ATT_THREADS) { c_f[i] = __ldcg(p.pm + row0 * NS + i); c_l[i] = __ldcg(p.pl + row0 * NS + i); }
+  float4 acc[HMAX];                                   // split `warp` of every head, in flight while M and L are computed
+#pragma unroll
+  for (int g = 0; g < HMAX; g++)
+    acc[g] = (g < heads && warp < NS) ? __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * NS + warp) * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  if (warp < heads) {
+    float M = -CUDART_INF_F;
+    for (int s2 = lane; s2 < NS; s2 += 32) M = fmaxf(M, c_f[warp * NS + s2]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(FULLM, M, o));
+    float L = 0.f;
+    for (int s2 = lane; s2 < NS; s2 += 32) {
+      const float ms = c_f[warp * NS + s2];
+      const float f = (ms == -CUDART_INF_F) ? 0.f : fast_exp2(ms - M);
+      c_f[warp * NS + s2] = f; L += c_l[warp * NS + s2] * f;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(FULLM, L, o);
+    if (lane == 0) { c_ML[2 * warp] = M; c_ML[2 * warp + 1] = L; }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int g = 0; g < HMAX; g++) {
+    const float f = (g < heads && warp < NS) ? c_f[g * NS + warp] : 0.f;
+    acc[g] = make_float4(acc[g].x * f, acc[g].y * f, acc[g].z * f, acc[g].w * f);
+  }
+  for (int s2 = warp + ATT_WARPS; s2 < NS; s2 += ATT_WARPS) {
+#pragma unroll
+    for (int g = 0; g < HMAX; g++) {
+      if (g < heads) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * NS + s2) * D) + lane);
+        const float f = c_f[g * NS + s2];
+        acc[g].x += v.x * f; acc[g].y += v.y * f; acc[g].z += v.z * f; acc[g].w += v.w * f;
+      }
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < HMAX; g++)
+    if (g < heads) *reinterpret_cast<float4*>(c_red + ((warp * 8 + g) * D) + 4 * lane) = acc[g];
+  __syncthreads();
+  for (int g = tid >> 7; g < heads; g += ATT_THREADS / 128) {
+    float Ac = 0.f;
+    const int d = tid & 127;
+#pragma unroll
+    for (int w = 0; w < ATT_WARPS; w++) Ac += c_red[(w * 8 + g) * D + d];
+    deliver(g, c_ML[2 * g], c_ML[2 * g + 1], Ac);
+  }
+}
+
+template <bool PAGED, bool DUMP, int NSET>
 __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last;
   const int tid = threadIdx.x, lane = tid & 31, j = lane & 3, r = lane >> 2;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
+  const u32 smem_s = (u32)__cvta_generic_to_shared(smem);
+  int* const done = reinterpret_cast<int*>(smem + TB_DONE);
   // ---- programmatic dependent launch: the grid is launched with stream serialisation relaxed, so its CTAs can be made
-  // resident while the previous kernel of the stream is still finishing (its split merge runs on a few SMs only).  Nothing
-  // is read before that kernel has completed; the next kernel of the stream may be staged behind this one right away (it
-  // cannot become resident before this grid's CTAs leave their SMs).  Both instructions are no-ops in a plain launch.
+  // resident while the previous kernel of the stream is still finishing (its split merge runs on a few SMs only).  What does not
+  // depend on memory is set up before the wait; nothing is read before that kernel has completed; the next kernel of the stream may be
+  // staged behind this one right away (it cannot become resident before this grid's CTAs leave their SMs).  Both instructions are no-ops
+  // in a plain launch.
+  if (tid < 256) fill_lutx(reinterpret_cast<u32x2*>(smem + TB_LUTX), tid);
+  if (tid >= 256 && tid < 260) reinterpret_cast<u32*>(smem + TB_ZERO)[tid - 256] = 0u;
+  if (lane == 0 && warp < NSTG) {
+    mbar_init(smem_s + TB_FULL + 8 * warp, 1);
+    done[warp] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
 
@@ -670,7 +227,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   }
   const int b = bh / p.n_kv, kvh = bh % p.n_kv;
 
-  // ---- which cache head, how many tokens, this CTA's tile range [tlo, thi)
+  // ---- which cache head, how many tokens, this CTA's tile range [tlo, tlo + n)
   // (without a slot map row b reads slot b; without a length table every head holds S_uniform tokens: the two dependent
   // loads at the head of the prologue disappear for callers whose heads are all alike, which is what two Pages are)
   int S, ch = 0, TL = 0, ohk = 0, ohv = 0;
@@ -685,415 +242,284 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     TL = sl < 0 ? 0 : t_ld;
   }
   // These values are the same in every thread, but they were loaded from memory: passing them through a shuffle tells the
-  // compiler so, and the address arithmetic built on them (one lane issues the copies) stays in uniform registers.
+  // compiler so, and the address arithmetic built on them stays in uniform registers.
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
   const int ntiles = (S + 15) >> 4, chunk = (ntiles + p.nsplit - 1) / p.nsplit;
-  const int tlo = min(split * chunk, ntiles), thi = min(tlo + chunk, ntiles);
+  const int tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo), nstages = (n + TPS - 1) / TPS;
   const long smh = (long)ch * p.S_pad * D, cdh = (long)ch * p.S_pad * CB, rowb = (long)ch * p.S_pad, tileb = (long)ch * (p.S_pad >> 4);
   ohk = __shfl_sync(FULLM, ohk, 0); ohv = __shfl_sync(FULLM, ohv, 0);
 
-  // ---- addressing of this lane, and the copies of the warp's first tile: they are put in flight before the CTA builds its
-  // tables so that the first tile arrives while the tables are written
-  uint8_t* ring = smem + TABLE_BYTES + warp * WARP_SMEM;
-  const u32 ring_s = (u32)__cvta_generic_to_shared(ring);
-  LaneAddr L;
-  L.ohk = ohk; L.ohv = ohv;
-  L.availk = PAGED ? 0 : (int)min((long)(1 << 30), p.K.ovf_bytes - ohk); L.availv = PAGED ? 0 : (int)min((long)(1 << 30), p.V.ovf_bytes - ohv);
   const int* metak = reinterpret_cast<const int*>(smem + TB_META);
   const int* metav = metak + META_TILES;
-  auto global_meta = [&](int tile) -> TileMeta {
+  auto global_meta = [&](int i) -> TileMeta {         // i counts from the first tile of the CTA's range
+    const int tile = tlo + i;
     if (PAGED) { const int pc = p.bt[(long)b * p.bt_stride + tile] * (2 * p.n_kv) + 2 * kvh; return TileMeta{p.mt[pc], p.mt[pc + 1]}; }
     return TileMeta{p.K.tile_off[tileb + tile], p.V.tile_off[tileb + tile]};
   };
-  auto meta_of = [&](int tile) -> TileMeta {          // valid after the CTA has staged its metadata
-    if (tile - tlo < META_TILES) return TileMeta{metak[tile - tlo], metav[tile - tlo]};
-    return global_meta(tile);
+  auto meta_of = [&](int i) -> TileMeta {             // valid after the CTA has staged its metadata
+    if (i < META_TILES) return TileMeta{metak[i], metav[i]};
+    return global_meta(i);
   };
-  // Slot layout, escape window of a tile whose escapes start `m` bytes into the head's escape bytes, in 32-bit arithmetic:
-  // w16 = its first byte's offset inside a 16-byte unit, n = bytes of the copy from the unit's start (a multiple of 16, at most
-  // ESC_COPY, inside the allocation; 0 when the unit starts before the allocation).
-  const int a16k = PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.K.ovf) + (unsigned)ohk) & 15), a16v = PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.V.ovf) + (unsigned)ohv) & 15);
-  auto esc_win = [&](bool vside, int m, int& w16, int& n) {
-    w16 = ((vside ? a16v : a16k) + m) & 15;
-    const int to_end = (vside ? L.availv : L.availk) - m + w16;                 // bytes from the unit's start to the end of the allocation
-    n = ((vside ? L.ohv : L.ohk) + m < w16) ? 0 : max(0, min(ESC_COPY, to_end & ~15));
+  // ---- filling a stage, in two parts: what needs no metadata (slot layout only), and what does.  Executed by one lane.
+  auto issue_payload = [&](int st) {
+    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES;
+    const int first = st * TPS;
+    const u32 cnt = (u32)min(TPS, n - first);
+    const long tile = tlo + first;
+    mbar_add_tx(mb, 2 * cnt * (TILE_SM + TILE_CD + 4 * T));
+    bulk_g2s(dst, p.K.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb); bulk_g2s(dst + SIDE_BYTES, p.V.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb);
+    bulk_g2s(dst + SB_CD, p.K.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb); bulk_g2s(dst + SIDE_BYTES + SB_CD, p.V.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb);
+    bulk_g2s(dst + SB_FL, reinterpret_cast<const uint8_t*>(p.K.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
+    bulk_g2s(dst + SIDE_BYTES + SB_FL, reinterpret_cast<const uint8_t*>(p.V.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
   };
-  auto bulk_issue = [&](u32 st, int tile, const TileMeta& m) {                  // executed by lane 0
-    const u32 mb = st + ST_MBAR;
-    // the stage may have been written through ordinary stores (patch numbers in its escape window): order those before the
-    // copy engine's writes to the same bytes
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (PAGED) {
-      const u32 n = (u32)min(p.TS, SLOT_OVF_OFF + ESC_COPY);                    // a slot is one contiguous piece, escapes included
-      mbar_expect_tx(mb, (m.mk >= 0 ? n : 0u) + (m.mv >= 0 ? n : 0u));
-      if (m.mk >= 0) bulk_g2s(st + ST_KSM, p.buf + (long)m.mk * p.TS, n, mb);
-      if (m.mv >= 0) bulk_g2s(st + ST_VSM, p.buf + (long)m.mv * p.TS, n, mb);
-    } else {
-      int wk, nk, wv, nv;
-      esc_win(false, m.mk, wk, nk); esc_win(true, m.mv, wv, nv);
-      mbar_expect_tx(mb, (u32)(2 * (TILE_SM + TILE_CD + 4 * T) + nk + nv));
-      const long so = smh + (long)tile * TILE_SM, co = cdh + (long)tile * TILE_CD, fo = (rowb + (long)tile * T) * 4;
-      bulk_g2s(st + ST_KSM, p.K.sm + so, TILE_SM, mb); bulk_g2s(st + ST_VSM, p.V.sm + so, TILE_SM, mb);
-      bulk_g2s(st + ST_KCD, p.K.codes + co, TILE_CD, mb); bulk_g2s(st + ST_VCD, p.V.codes + co, TILE_CD, mb);
-      bulk_g2s(st + ST_KFL, reinterpret_cast<const uint8_t*>(p.K.flags) + fo, 4 * T, mb);
-      bulk_g2s(st + ST_VFL, reinterpret_cast<const uint8_t*>(p.V.flags) + fo, 4 * T, mb);
-      if (nk > 0) bulk_g2s(st + ST_KESC, p.K.ovf + ((long)L.ohk + m.mk - wk), (u32)nk, mb);
-      if (nv > 0) bulk_g2s(st + ST_VESC, p.V.ovf + ((long)L.ohv + m.mv - wv), (u32)nv, mb);
-    }
+  // Escape window of a side for tiles whose escape bytes are [m0, m1) of the head's: from the 16-byte boundary at or below the first byte, a
+  // multiple of 16 bytes, at most SIDE_ESC, inside the allocation (no bytes when the boundary lies before it).
+  auto esc_window = [&](const gaac_side& sd, int oh, int m0, int m1, int& start, u32& bytes) {
+    const int w16 = (int)((reinterpret_cast<uintptr_t>(sd.ovf) + (unsigned)oh + (unsigned)m0) & 15);
+    const long to_end = (long)sd.ovf_bytes - oh - m0 + w16;
+    start = m0 - w16;
+    bytes = (long)oh + m0 < w16 || to_end <= 0 ? 0u : (u32)max(0L, min((long)min(SIDE_ESC, (m1 - m0 + w16 + 15) & ~15), to_end & ~15L));
   };
-  // Escape bytes of a staged side as the group decoder reads them: first escape byte in global memory, offset from the stage's
-  // zero byte to the first escape byte, staged bytes counted from the first escape byte
-  auto staged_escapes = [&](bool vside, int m, int& off, int& avail) {
-    const int base = (vside ? ST_VESC : ST_KESC) - ST_ZERO;
-    if (PAGED) { off = base; avail = min(p.ovf_slot, min(p.TS, SLOT_OVF_OFF + ESC_COPY) - SLOT_OVF_OFF); }
-    else { int w16, n; esc_win(vside, m, w16, n); off = base + w16; avail = n - w16; }
+  auto issue_rest = [&](int st, const TileMeta& m0, const TileMeta& m1) {        // m0: metadata of the stage's first tile, m1: of the first one behind it (slot layout)
+    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES;
+    int4 w; u32 nk, nv;
+    esc_window(p.K, ohk, m0.mk, m1.mk, w.x, nk); esc_window(p.V, ohv, m0.mv, m1.mv, w.z, nv);
+    w.y = (int)nk; w.w = (int)nv;
+    *reinterpret_cast<int4*>(smem + TB_WIN + 16 * (st % NSTG)) = w;
+    mbar_expect_tx(mb, nk + nv);
+    if (nk > 0) bulk_g2s(dst + SB_ESC, p.K.ovf + ((long)ohk + w.x), nk, mb);
+    if (nv > 0) bulk_g2s(dst + SIDE_BYTES + SB_ESC, p.V.ovf + ((long)ohv + w.z), nv, mb);
   };
-  auto global_escapes = [&](bool vside, int m) -> const uint8_t* {            // only tiles whose escapes exceed the window get here
-    if (PAGED) return p.buf + (long)m * p.TS + SLOT_OVF_OFF;
-    return (vside ? p.V.ovf : p.K.ovf) + ((long)(vside ? L.ohv : L.ohk) + m);
-  };
-  // ---- prologue.  Everything that reads global memory is put in flight first and consumed afterwards: the payload of the
-  // warp's first tile (needs no metadata in the slot layout), the tile's metadata, the metadata of the CTA's range, the
-  // query rows; then the tables are built while those loads travel.
-  int tile = tlo + warp;
-  TileMeta cur{0, 0};
-  if (lane == 0) {                                    // one barrier per stage, one arrival (this lane's) per phase; 8 zero bytes beside it
-    mbar_init(ring_s + ST_MBAR, 1); mbar_init(ring_s + STAGE_BYTES + ST_MBAR, 1);
-    *reinterpret_cast<unsigned long long*>(ring + ST_ZERO) = 0ull; *reinterpret_cast<unsigned long long*>(ring + STAGE_BYTES + ST_ZERO) = 0ull;
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncwarp();
-  if (tile < thi) {
-    if (PAGED) { cur = global_meta(tile); if (lane == 0) bulk_issue(ring_s, tile, cur); }
-    else {
-      // slot layout: the six payload copies need no metadata and leave at once; the escape windows (and the barrier's arrival)
-      // follow further down, when the tile's escape offsets have come back from global memory
-      if (lane == 0) {
-        const u32 mb = ring_s + ST_MBAR;
-        const long so = smh + (long)tile * TILE_SM, co = cdh + (long)tile * TILE_CD, fo = (rowb + (long)tile * T) * 4;
-        mbar_add_tx(mb, 2 * (TILE_SM + TILE_CD + 4 * T));
-        bulk_g2s(ring_s + ST_KSM, p.K.sm + so, TILE_SM, mb); bulk_g2s(ring_s + ST_VSM, p.V.sm + so, TILE_SM, mb);
-        bulk_g2s(ring_s + ST_KCD, p.K.codes + co, TILE_CD, mb); bulk_g2s(ring_s + ST_VCD, p.V.codes + co, TILE_CD, mb);
-        bulk_g2s(ring_s + ST_KFL, reinterpret_cast<const uint8_t*>(p.K.flags) + fo, 4 * T, mb);
-        bulk_g2s(ring_s + ST_VFL, reinterpret_cast<const uint8_t*>(p.V.flags) + fo, 4 * T, mb);
-      }
-      cur = global_meta(tile);
-    }
-  }
-  int* mk_s = reinterpret_cast<int*>(smem + TB_META);
-  int* mv_s = mk_s + META_TILES;
-  const int nstaged = min(thi - tlo, META_TILES);
-  TileMeta m_first{0, 0};
-  if (tid < nstaged) m_first = global_meta(tlo + tid);
-  QFrag Q;
-#if GAAC_QSMEM
-  Q.tab = reinterpret_cast<const uint4*>(smem + TB_Q);
-  uint4 q_mine = make_uint4(0u, 0u, 0u, 0u);            // threads 0..127 load one table entry each: K group tid >> 5 of lane tid & 31
-  if (tid < 128) {
-    const int gg = tid >> 5, jj = tid & 3, rr = (tid & 31) >> 2;
-    if (rr < G) {
-      const uint16_t* qp = p.q + ((long)b * p.n_q + kvh * G + rr) * D + 32 * gg + 2 * jj;
-      q_mine = make_uint4(*reinterpret_cast<const u32*>(qp), *reinterpret_cast<const u32*>(qp + 8), *reinterpret_cast<const u32*>(qp + 16), *reinterpret_cast<const u32*>(qp + 24));
-    }
-  }
-#else
-  {
-    const bool ok = r < G;
-    const uint16_t* qp = p.q + ((long)b * p.n_q + kvh * G + (ok ? r : 0)) * D;
+  auto behind = [&](int st, const TileMeta& none) { const int i = (st + 1) * TPS; return i < n || tlo + i < ntiles ? global_meta(i) : none; };
+  const u32 slot_bytes = PAGED ? (u32)min(p.TS, PSLOT) : 0u;                   // a paged slot is one contiguous piece, escapes included
+  auto issue_paged = [&](int st, const TileMeta (&m)[TPS]) {
+    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES;
+    const int cnt = min(TPS, n - st * TPS);
+    u32 pieces = 0;
 #pragma unroll
-    for (int s = 0; s < 8; s++) {
-      Q.qa[s][0] = ok ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j) : 0u;
-      Q.qa[s][1] = ok ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j + 8) : 0u;
+    for (int t = 0; t < TPS; t++) pieces += t < cnt ? (m[t].mk >= 0 ? 1u : 0u) + (m[t].mv >= 0 ? 1u : 0u) : 0u;
+    mbar_expect_tx(mb, pieces * slot_bytes);
+#pragma unroll
+    for (int t = 0; t < TPS; t++) {
+      if (t < cnt && m[t].mk >= 0) bulk_g2s(dst + 2 * t * PSLOT, p.buf + (long)m[t].mk * p.TS, slot_bytes, mb);
+      if (t < cnt && m[t].mv >= 0) bulk_g2s(dst + (2 * t + 1) * PSLOT, p.buf + (long)m[t].mv * p.TS, slot_bytes, mb);
     }
+  };
+  constexpr int FAR = 1 << 28;                        // "until the end of the allocation", as an escape offset
+
+  // ---- prologue.  Everything that reads global memory is put in flight first and consumed afterwards: the first stages' payload (needs
+  // no metadata in the slot layout), their metadata, the metadata of the CTA's range, the query rows; then the tables are built while
+  // those loads travel.
+  // HBM is idle when the grid starts and every CTA asks at once: the stages that the first tiles are in go first, the others follow once
+  // the small loads are back (filling all eight at once held those loads, and with them the first tile, back for 5 us).
+  constexpr int FIRST = (ATT_WARPS + TPS - 1) / TPS;
+  const bool filler = lane == 0 && warp < min(NSTG, nstages);                  // warp w fills stage w
+  TileMeta f0{0, 0}, f1{0, 0};
+  auto fill_paged = [&](int st) {
+    TileMeta m[TPS];
+#pragma unroll
+    for (int t = 0; t < TPS; t++) m[t] = st * TPS + t < n ? global_meta(st * TPS + t) : TileMeta{-1, -1};
+    issue_paged(st, m);
+  };
+  if (filler) {
+    if (!PAGED) { f0 = global_meta(warp * TPS); f1 = behind(warp, TileMeta{FAR, FAR}); }
+    if (warp < FIRST) { if (PAGED) fill_paged(warp); else issue_payload(warp); }
   }
-#endif
-  // ---- CTA tables: escape-byte table, code table, per-lane-class base words {b3lo, b3hi, b4lo-b3lo, b4hi-b3hi} per group,
-  // zero pads, per-tile metadata of the range (escape offsets or mode-table entries, so that the main loop never waits on a
-  // dependent global load)
+  const int nstaged = min(n, META_TILES);
+  TileMeta m_first{0, 0};
+  if (tid < nstaged) m_first = global_meta(tid);
+  QFrag Q;
+  load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * D, D, G, lane);
   {
     const int brow = PAGED ? kvh : ch % p.n_base_rows;
-    const uint8_t* b3k = (PAGED ? p.b3k : p.K.base3) + brow * D; const uint8_t* b4k = (PAGED ? p.b4k : p.K.base4) + brow * D;
-    const uint8_t* b3v = (PAGED ? p.b3v : p.V.base3) + brow * D; const uint8_t* b4v = (PAGED ? p.b4v : p.V.base4) + brow * D;
-    constexpr int KB_T0 = ATT_THREADS >= 320 ? 256 : 0, VB_T0 = KB_T0 + 32;       // which threads build the base words (beside the escape-byte table when the CTA is small)
-    if (tid >= KB_T0 && tid < KB_T0 + 16) {           // K: lane class jj, group gg -> words 2gg, 2gg+1
-      const int t = tid - KB_T0, jj = t >> 2, gg = t & 3; u32 w3[8], w4[8];
-      k_base_words(b3k, jj, w3); k_base_words(b4k, jj, w4);
-      *reinterpret_cast<u32x4*>(smem + TB_KB + 16 * t) = u32x4{w3[2 * gg], w3[2 * gg + 1], w4[2 * gg] - w3[2 * gg], w4[2 * gg + 1] - w3[2 * gg + 1]};
-    } else if (tid >= VB_T0 && tid < VB_T0 + 16) {    // V: lane class rr, group gg
-      const int t = tid - VB_T0, rr = t >> 1, gg = t & 1; u32 w3[4], w4[4];
-      v_base_words(b3v, rr, w3); v_base_words(b4v, rr, w4);
-      *reinterpret_cast<u32x4*>(smem + TB_VB + 16 * t) = u32x4{w3[2 * gg], w3[2 * gg + 1], w4[2 * gg] - w3[2 * gg], w4[2 * gg + 1] - w3[2 * gg + 1]};
-    }
-    if (tid < 256) fill_lutx(reinterpret_cast<u32x2*>(smem + TB_LUTX), tid);
-#if GAAC_QSMEM
-    if (tid < 128) reinterpret_cast<uint4*>(smem + TB_Q)[tid] = q_mine;
-#endif
-#if GAAC_LUTC
-    for (int i = tid; i < 4096; i += ATT_THREADS) reinterpret_cast<u32*>(smem + TB_LUTC)[i] = spread_codes4((u32)i);
-#endif
-    if (tid == 0) s_next = tlo + ATT_WARPS;           // tiles tlo .. tlo+W-1 go to warps 0..W-1, the rest is handed out on demand
+    if (warp == ATT_WARPS - 2) fill_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
+    if (warp == ATT_WARPS - 1) fill_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
+    if (tid == 0) s_next = ATT_WARPS;                        // tiles 0 .. W-1 of the range go to warps 0 .. W-1, the rest is handed out on demand
+    int* mk_s = reinterpret_cast<int*>(smem + TB_META);
+    int* mv_s = mk_s + META_TILES;
     if (tid < nstaged) { mk_s[tid] = m_first.mk; mv_s[tid] = m_first.mv; }
-    for (int i = tid + ATT_THREADS; i < nstaged; i += ATT_THREADS) { const TileMeta m = global_meta(tlo + i); mk_s[i] = m.mk; mv_s[i] = m.mv; }
+    for (int i = tid + ATT_THREADS; i < nstaged; i += ATT_THREADS) { const TileMeta m = global_meta(i); mk_s[i] = m.mk; mv_s[i] = m.mv; }
   }
-  if (!PAGED && tile < thi && lane == 0) {
-    const u32 mb = ring_s + ST_MBAR;
-    int wk, nk, wv, nv;
-    esc_win(false, cur.mk, wk, nk); esc_win(true, cur.mv, wv, nv);
-    if (nk + nv > 0) mbar_add_tx(mb, (u32)(nk + nv));
-    if (nk > 0) bulk_g2s(ring_s + ST_KESC, p.K.ovf + ((long)L.ohk + cur.mk - wk), (u32)nk, mb);
-    if (nv > 0) bulk_g2s(ring_s + ST_VESC, p.V.ovf + ((long)L.ohv + cur.mv - wv), (u32)nv, mb);
-    mbar_arrive(mb);
-  }
-  WarpAcc A;
-#pragma unroll
-  for (int n = 0; n < 8; n++) A.acc[n][0] = A.acc[n][1] = A.acc[n][2] = A.acc[n][3] = 0.f;
-  A.m0 = A.m1 = -CUDART_INF_F; A.l0 = A.l1 = 0.f;
+  if (!PAGED && filler && warp < FIRST) issue_rest(warp, f0, f1);
+  WarpAcc<NSET> A;
+  A.clear();
   __syncthreads();
+  if (filler && warp >= FIRST) { if (PAGED) fill_paged(warp); else { issue_payload(warp); issue_rest(warp, f0, f1); } }
 
   uint16_t* const dump_k = DUMP ? p.dump_k + (long)bh * p.dump_S * D : nullptr;
   uint16_t* const dump_v = DUMP ? p.dump_v + (long)bh * p.dump_S * D : nullptr;
-  // ---- main loop.  The warp's first tile is tlo + warp; every further tile is taken from the CTA's counter while the
-  // current one is being consumed, one tile ahead of its use, so fast and slow warps finish within about one tile of each
-  // other.  The counter is read at the top of the iteration and its value used after the K half, which hides the latency
-  // of the shared-memory atomic; the copies of the next tile are issued between the K half and the V half.
-  int stg = 0;
-  u32 phase = 0;                                       // bit s: parity of the phase of stage s that is waited for next
-#if GAAC_DEEP
-  // the warp's second tile goes into the other stage right away; from then on the stage a tile leaves is refilled, as soon as the
-  // tile is done, with the tile after the next one, so the copies of a tile have a whole tile's time to arrive
-  int tile_b = thi; TileMeta meta_b{0, 0};
-  if (tile < thi) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&s_next, 1);
-    tile_b = __shfl_sync(FULLM, t, 0);
-    if (tile_b < thi) { meta_b = meta_of(tile_b); if (lane == 0) bulk_issue(ring_s + STAGE_BYTES, tile_b, meta_b); }
-  }
-#endif
-  while (tile < thi) {
-    int t1 = 0;
-    if (lane == 0) t1 = atomicAdd(&s_next, 1);
-    if (!__all_sync(FULLM, mbar_wait(ring_s + stg * STAGE_BYTES + ST_MBAR, (phase >> stg) & 1u))) {     // the whole warp gives up together
+  const WarpView W{smem_s + TB_LUTX, smem_s + TB_BASES, smem_s + TB_ZERO, smem_s + TB_SCRATCH + warp * WARP_SCRATCH};
+  const int paged_avail = PAGED ? min(p.ovf_slot, (int)slot_bytes - SLOT_OVF_OFF) : 0;
+  // ---- main loop.  The warp's first tile is tile `warp` of the range; every further one is taken from the CTA's counter at the top of the
+  // iteration, one tile ahead of its use, so fast and slow warps finish within about one tile of each other.  The warp that is the
+  // last to leave a stage fills it again with the tiles NSTG stages on.
+  int it = warp;
+  while (it < n) {
+    int nx = 0;
+    if (lane == 0) nx = atomicAdd(&s_next, 1);
+    const int st = it / TPS, ti = it % TPS, slot = st % NSTG;
+    const TileMeta cur = meta_of(it);
+    // A parity says one thing about two phases: the stage's wait is only right once its slot's previous use is over, that is, once all its tiles
+    // were counted out (a warp can be handed a tile whose slot still waits for its previous copies).
+    if (!__all_sync(FULLM, wait_count(smem_s + TB_DONE + 4 * slot, TPS * (st / NSTG)) && mbar_wait(smem_s + TB_FULL + 8 * slot, (u32)(st / NSTG) & 1u))) {     // the whole warp gives up together
       if (lane == 0) atomicExch(p.err, 1);
       break;
     }
-    phase ^= 1u << stg;
-    const uint8_t* stage = ring + stg * STAGE_BYTES;
+    const int sb = TB_RING + slot * STAGE_BYTES, tile = tlo + it;
     const int nvalid = min(T, S - tile * T);
     const bool rawk = PAGED && cur.mk < 0, rawv = PAGED && cur.mv < 0;
-    u32 flrow; int rowoff, total;
-    scan_rows(stage, rawk, rawv, lane, flrow, rowoff, total);
-    // which decoder each side takes: the staged window (branch-free, raw groups through the patch table) when the side's escape
-    // bytes all fit the window and it has at most PATCH_MAX raw groups; else the one that reads escapes from global memory
-    int off_k = 0, off_v = 0, avail_k = 0, avail_v = 0;
-    if (!rawk) staged_escapes(false, cur.mk, off_k, avail_k);
-    if (!rawv) staged_escapes(true, cur.mv, off_v, avail_v);
-    const int tot_k = __shfl_sync(FULLM, total, 15), tot_v = __shfl_sync(FULLM, total, 31);
-    const bool win_k = !rawk && esc_part(tot_k) + 8 <= avail_k && (!GAAC_RAWPATCH || raw_part(tot_k) <= PATCH_MAX);     // +8: a raw payload is read as two aligned words
-    const bool win_v = !rawv && esc_part(tot_v) + 8 <= avail_v && (!GAAC_RAWPATCH || raw_part(tot_v) <= PATCH_MAX);
-    uint8_t* const patch = ring + NSTAGE * STAGE_BYTES;
-    const u32 patch_rel = (u32)(patch - (smem + TB_LUTX));
-#if GAAC_RAWPATCH
-    if ((win_k && raw_part(tot_k) > 0) || (win_v && raw_part(tot_v) > 0))
-      build_raw_patches(ring + stg * STAGE_BYTES, smem, patch, off_k, off_v, win_k, win_v, flrow, rowoff, lane);
-#endif
+    SideView ks, vs;
+    if (PAGED) {
+      const uint8_t* t0 = smem + sb + 2 * ti * PSLOT;
+      const u32 esc = smem_s + sb + 2 * ti * PSLOT + SLOT_OVF_OFF;
+      ks = SideView{t0, t0 + SLOT_CD_OFF, t0 + SLOT_FL_OFF, esc, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF, paged_avail};
+      vs = SideView{t0 + PSLOT, t0 + PSLOT + SLOT_CD_OFF, t0 + PSLOT + SLOT_FL_OFF, esc + PSLOT, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, paged_avail};
+    } else {
+      const int4 w = *reinterpret_cast<const int4*>(smem + TB_WIN + 16 * slot);
+      const uint8_t* t0 = smem + sb + ti * TILE_SM;
+      const uint8_t* c0 = smem + sb + SB_CD + ti * TILE_CD;
+      const uint8_t* f0 = smem + sb + SB_FL + ti * 4 * T;
+      const int ok = cur.mk - w.x, ov = cur.mv - w.z;
+      ks = SideView{t0, c0, f0, smem_s + sb + SB_ESC + ok, p.K.ovf + ((long)ohk + cur.mk), w.y - ok};
+      vs = SideView{t0 + SIDE_BYTES, c0 + SIDE_BYTES, f0 + SIDE_BYTES, smem_s + sb + SIDE_BYTES + SB_ESC + ov, p.V.ovf + ((long)ohv + cur.mv), w.w - ov};
+    }
+    const TilePlan plan = plan_tile(ks, vs, rawk, rawv, W, lane);
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (!rawk) {
-      if (win_k)
-        k_scores<true, DUMP, GAAC_RAWPATCH != 0>(sc, stage, smem, EscSrc<true>{stage + ST_ZERO, nullptr, off_k}, flrow, rowoff, lane, Q, dump_k + (long)tile * T * D, nvalid, patch_rel);
-      else
-        k_scores<false, DUMP>(sc, stage, smem, EscSrc<false>{nullptr, global_escapes(false, cur.mk), 0}, flrow, rowoff, lane, Q, dump_k + (long)tile * T * D, nvalid);
-    } else {
-      raw_scores<DUMP>(sc, p.raw + (long)(~cur.mk) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
+    if (!rawk) k_tile<DUMP>(sc, ks, plan, W, lane, Q, dump_k + (long)tile * T * D, nvalid);
+    else raw_scores<DUMP>(sc, p.raw + (long)(~cur.mk) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
+    nx = __shfl_sync(FULLM, nx, 0);
+    PFrag<NSET> P;
+    if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
+    else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
+    if (!rawv) v_tile<DUMP, NSET>(A, vs, plan, W, lane, P, dump_v + (long)tile * T * D, nvalid);
+    else raw_accum<DUMP, NSET>(A, p.raw + (long)(~cur.mv) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
+    // the stage's bytes may have been written through ordinary stores (patch numbers): order those before the copy engine's next
+    // writes to the same bytes, then count this warp out of the stage
+    if (st + NSTG < nstages) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        int left;
+        asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(left) : "r"(smem_s + TB_DONE + 4 * slot) : "memory");
+        if ((left & (TPS - 1)) == TPS - 1) {
+          const int ns = st + NSTG, i0 = ns * TPS;
+          if (PAGED) {
+            TileMeta m[TPS];
+#pragma unroll
+            for (int t = 0; t < TPS; t++) m[t] = i0 + t < n ? meta_of(i0 + t) : TileMeta{-1, -1};
+            issue_paged(ns, m);
+          } else {
+            const TileMeta m0 = meta_of(i0), m1 = i0 + TPS < n ? meta_of(i0 + TPS) : TileMeta{FAR, FAR};
+            issue_payload(ns);
+            issue_rest(ns, m0, m1);
+          }
+        }
+      }
     }
-    t1 = __shfl_sync(FULLM, t1, 0);
-    TileMeta nxt{0, 0};
-#if !GAAC_DEEP
-    if (t1 < thi) {
-      nxt = meta_of(t1);
-      const u32 st = ring_s + (stg ^ 1) * STAGE_BYTES;
-      if (lane == 0) bulk_issue(st, t1, nxt);
-    }
-#endif
-    PFrag P;
-    if (nvalid == T) softmax_step<true>(A, sc, p.scale_log2, nvalid, lane, P);
-    else softmax_step<false>(A, sc, p.scale_log2, nvalid, lane, P);
-    if (!rawv) {
-      if (win_v)
-        v_accum<true, DUMP, GAAC_RAWPATCH != 0>(A, stage, smem, EscSrc<true>{stage + ST_ZERO, nullptr, off_v}, flrow, rowoff, lane, P, dump_v + (long)tile * T * D, nvalid, patch_rel);
-      else
-        v_accum<false, DUMP>(A, stage, smem, EscSrc<false>{nullptr, global_escapes(true, cur.mv), 0}, flrow, rowoff, lane, P, dump_v + (long)tile * T * D, nvalid);
-    } else {
-      raw_accum<DUMP>(A, p.raw + (long)(~cur.mv) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
-    }
-#if GAAC_DEEP
-    __syncwarp();                                      // every lane has read what it needs of this stage
-    if (t1 < thi) { nxt = meta_of(t1); if (lane == 0) bulk_issue(ring_s + stg * STAGE_BYTES, t1, nxt); }
-    cur = meta_b; tile = tile_b; meta_b = nxt; tile_b = t1; stg ^= 1;
-#else
-    cur = nxt; stg ^= 1; tile = t1;
-#endif
+    it = nx;
   }
-  // ---- slot layout: the raw BF16 tail belongs to the last split's warp 0
-  if (!PAGED && TL > 0 && split == p.nsplit - 1 && warp == 0) {
+  // ---- slot layout: the raw BF16 tail belongs to the last split's last warp
+  if (!PAGED && TL > 0 && split == p.nsplit - 1 && warp == ATT_WARPS - 1) {
     const uint16_t* kraw = reinterpret_cast<const uint16_t*>(p.K.tail) + (long)ch * p.tail_cap * D;
     const uint16_t* vraw = reinterpret_cast<const uint16_t*>(p.V.tail) + (long)ch * p.tail_cap * D;
     for (int t0 = 0; t0 < TL; t0 += T) {
       const int nvalid = min(T, TL - t0);
       float sc[4] = {0.f, 0.f, 0.f, 0.f};
       raw_scores<DUMP>(sc, kraw, nvalid, lane, Q, dump_k + ((long)S + t0) * D);
-      PFrag P;
-      softmax_step<false>(A, sc, p.scale_log2, nvalid, lane, P);
-      raw_accum<DUMP>(A, vraw, nvalid, lane, P, dump_v + ((long)S + t0) * D);
+      PFrag<NSET> P;
+      softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
+      raw_accum<DUMP, NSET>(A, vraw, nvalid, lane, P, dump_v + ((long)S + t0) * D);
       kraw += T * D; vraw += T * D;
     }
   }
 
-  // ---- merge the warps of the CTA (the rings are free now)
+  // ---- merge the warps of the CTA (the ring is free now)
   __syncthreads();
-  constexpr int ACC_LD = D + 4;                                  // row stride of the staged accumulators: 4j + r banks, conflict-free stores
-  float* sh_m = reinterpret_cast<float*>(smem + TABLE_BYTES);    // [W][8]
+  float* sh_m = reinterpret_cast<float*>(smem + TB_RING);        // [W][8]
   float* sh_l = sh_m + ATT_WARPS * 8;                            // [W][8]
   float* sh_acc = sh_l + ATT_WARPS * 8;                          // [W][8][ACC_LD]
 #pragma unroll
-  for (int o = 4; o < 32; o <<= 1) { A.l0 += __shfl_xor_sync(FULLM, A.l0, o); A.l1 += __shfl_xor_sync(FULLM, A.l1, o); }
-  if (r == 0) { sh_m[warp * 8 + 2 * j] = A.m0; sh_l[warp * 8 + 2 * j] = A.l0; sh_m[warp * 8 + 2 * j + 1] = A.m1; sh_l[warp * 8 + 2 * j + 1] = A.l1; }
-  if (2 * j < G) {                                               // heads 2j, 2j+1 (the second may be a padding head: stored, never read)
+  for (int s = 0; s < NSET; s++) {
+    const int h = 4 * s + j;
+    float l = A.l[s];
 #pragma unroll
-    for (int n = 0; n < 8; n++) {
-      float* a0 = sh_acc + ((warp * 8 + 2 * j) * ACC_LD) + 16 * n + r;
-      a0[0] = A.acc[n][0]; a0[ACC_LD] = A.acc[n][1]; a0[8] = A.acc[n][2]; a0[ACC_LD + 8] = A.acc[n][3];
+    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(FULLM, l, o);
+    if (r == 0) { sh_m[warp * 8 + h] = A.m[s]; sh_l[warp * 8 + h] = l; }
+    if (h < G) {
+      float* a0 = sh_acc + (warp * 8 + h) * ACC_LD + r;
+#pragma unroll
+      for (int i = 0; i < 16; i++) a0[8 * i] = A.acc[s][i >> 2][i & 3];
     }
   }
   __syncthreads();
   const int NS = p.nsplit;
-  {
-    const int d = tid & 127;
-    for (int g = tid >> 7; g < G; g += ATT_THREADS / 128) {
-      float M = -CUDART_INF_F;
-#pragma unroll
-      for (int w = 0; w < ATT_WARPS; w++) M = fmaxf(M, sh_m[w * 8 + g]);
-      float Lc = 0.f, Ac = 0.f;
-#pragma unroll
-      for (int w = 0; w < ATT_WARPS; w++) {
-        const float mw = sh_m[w * 8 + g];
-        const float f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
-        Lc += sh_l[w * 8 + g] * f; Ac += sh_acc[(w * 8 + g) * ACC_LD + d] * f;
+  const long qh0 = (long)b * p.n_q + kvh * G;
+  const int d = tid & 127;
+  // where a query head's merged (M, L, acc) goes when this is the last word of this GPU on it
+  const int x_ep = p.x_recv ? __ldcg(p.x_epoch) : 0;             // number of this exchange - 1; advanced only after every group has read it
+  auto deliver = [&](int g, float M, float L, float Ac) {
+    const long qh = qh0 + g;
+    if (p.x_recv) {                                  // the partial, pushed to every rank's receive buffer over NVLink
+      const long row = ((long)((x_ep & 1) * p.x_world + p.x_rank) * p.x_rows_cap + qh) * 130;
+      for (int rk = 0; rk < p.x_world; rk++) {
+        unsigned long long* o = p.x_recv[rk] + row;
+        if (d == 0) { x_store(o, M * LN2, (u32)x_ep + 1u); x_store(o + 1, L, (u32)x_ep + 1u); }
+        x_store(o + 2 + d, Ac, (u32)x_ep + 1u);
       }
-      const long qh = (long)b * p.n_q + kvh * G + g, pidx = qh * NS + split;
+    } else if (p.part) {                             // un-normalised partial for a cross-GPU merge: m in natural-log units
+      float* o = p.part + qh * 130;
+      if (d == 0) { o[0] = M * LN2; o[1] = L; }
+      o[2 + d] = Ac;
+    } else {
+      const float v = L > 0.f ? Ac / L : 0.f;
+      p.out[qh * D + d] = __bfloat16_as_ushort(__float2bfloat16(v));
+      if (p.out_f32) p.out_f32[qh * D + d] = v;
+    }
+  };
+  for (int g = tid >> 7; g < G; g += ATT_THREADS / 128) {
+    float M = -CUDART_INF_F;
+#pragma unroll
+    for (int w = 0; w < ATT_WARPS; w++) M = fmaxf(M, sh_m[w * 8 + g]);
+    float Lc = 0.f, Ac = 0.f;
+#pragma unroll
+    for (int w = 0; w < ATT_WARPS; w++) {
+      const float mw = sh_m[w * 8 + g];
+      const float f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
+      Lc += sh_l[w * 8 + g] * f; Ac += sh_acc[(w * 8 + g) * ACC_LD + d] * f;
+    }
+    if (NS == 1) deliver(g, M, Lc, Ac);              // nothing to merge with
+    else {
+      const long pidx = (qh0 + g) * NS + split;
       if (d == 0) { p.pm[pidx] = M; p.pl[pidx] = Lc; }
       p.pa[pidx * D + d] = Ac;
     }
   }
-  // ---- the last CTA of this (row, kv head) merges the splits.  The ticket is taken with an acquire-release atomic at GPU scope
-  // by one thread between two CTA barriers: the barrier before it orders every thread's partial stores before the release, the
-  // barrier after it orders the acquire before every thread's loads of the other CTAs' partials - no per-thread fence is needed.
-  __syncthreads();
-  if (tid == 0) {
-    int ticket;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(p.counters + bh) : "memory");
-    s_last = (ticket == NS - 1);
-    if (s_last) p.counters[bh] = 0;                 // leave the counter ready for the next call
+  if (NS > 1) {
+    if (!last_split(p.counters + bh, NS, &s_last)) return;
+    merge_splits<4 * NSET>(p, smem + TB_RING, qh0, G, deliver);
   }
-  __syncthreads();
-  if (!s_last) return;
-  // All loads below are independent of one another (no per-split dependent chain): scale factors first, then the weighted sum
-  // with one warp per split and 16-byte loads, then a cross-warp sum in shared memory.
-  {
-    float* c_f = reinterpret_cast<float*>(smem + TABLE_BYTES);           // [G][NS]  m, then exp2(m - M)
-    float* c_l = c_f + 8 * NS;                                            // [G][NS]  l
-    float* c_ML = c_l + 8 * NS;                                           // [8][2]   M, L per head
-    float* c_red = c_ML + 16;                                             // [W][G][128] (NS <= 1024 keeps this inside the ring area)
-    const long qh0 = (long)b * p.n_q + kvh * G;
-    for (int i = tid; i < G * NS; i += ATT_THREADS) { c_f[i] = __ldcg(p.pm + qh0 * NS + i); c_l[i] = __ldcg(p.pl + qh0 * NS + i); }
-    float4 pre[8];                                                        // split `warp` of every head, in flight while M and L are computed
-#pragma unroll
-    for (int g = 0; g < 8; g++)
-      pre[g] = (g < G && warp < NS) ? __ldcg(reinterpret_cast<const float4*>(p.pa + ((qh0 + g) * NS + warp) * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    if (warp < G) {
-      float M = -CUDART_INF_F;
-      for (int s2 = lane; s2 < NS; s2 += 32) M = fmaxf(M, c_f[warp * NS + s2]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(FULLM, M, o));
-      float L = 0.f;
-      for (int s2 = lane; s2 < NS; s2 += 32) {
-        const float ms = c_f[warp * NS + s2];
-        const float f = (ms == -CUDART_INF_F) ? 0.f : fast_exp2(ms - M);
-        c_f[warp * NS + s2] = f; L += c_l[warp * NS + s2] * f;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(FULLM, L, o);
-      if (lane == 0) { c_ML[2 * warp] = M; c_ML[2 * warp + 1] = L; }
-    }
-    __syncthreads();
-    float4 acc4[8];
-#pragma unroll
-    for (int g = 0; g < 8; g++) {
-      const float f = (g < G && warp < NS) ? c_f[g * NS + warp] : 0.f;
-      acc4[g] = make_float4(pre[g].x * f, pre[g].y * f, pre[g].z * f, pre[g].w * f);
-    }
-    for (int s2 = warp + ATT_WARPS; s2 < NS; s2 += ATT_WARPS) {
-#pragma unroll
-      for (int g = 0; g < 8; g++) {
-        if (g < G) {
-          const float4 v = __ldcg(reinterpret_cast<const float4*>(p.pa + ((qh0 + g) * NS + s2) * D) + lane);
-          const float f = c_f[g * NS + s2];
-          acc4[g].x += v.x * f; acc4[g].y += v.y * f; acc4[g].z += v.z * f; acc4[g].w += v.w * f;
-        }
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < 8; g++)
-      if (g < G) *reinterpret_cast<float4*>(c_red + ((warp * 8 + g) * D) + 4 * lane) = acc4[g];
-    __syncthreads();
-    const int d = tid & 127;
-    const int x_ep = p.x_recv ? __ldcg(p.x_epoch) : 0;         // number of this exchange - 1; advanced only after every group has read it
-    for (int g = tid >> 7; g < G; g += ATT_THREADS / 128) {
-      float Ac = 0.f;
-#pragma unroll
-      for (int w = 0; w < ATT_WARPS; w++) Ac += c_red[(w * 8 + g) * D + d];
-      const float M = c_ML[2 * g], L = c_ML[2 * g + 1];
+  if (p.x_recv) {
+    // Every entry carries the exchange number, so nothing else announces the rows (see x_store / x_load).
+    if (!p.x_fused) return;                          // the wait-and-merge runs as its own launch (gaac_exchange_merge)
+    // ---- fused: wait (bounded) for the rows of this group from every rank, merge them, write the output
+    const unsigned long long* base = p.x_recv[p.x_rank] + (long)(x_ep & 1) * p.x_world * p.x_rows_cap * 130;
+    float v[2] = {0.f, 0.f};
+    int bad = 0;
+    for (int g = tid >> 7, i = 0; g < G; g += ATT_THREADS / 128, i++)
+      bad |= !x_merge_rows(base, p.x_world, p.x_rows_cap, qh0 + g, d, (u32)x_ep + 1u, v[i]);
+    const int any_bad = __syncthreads_or(bad);       // a group whose rows did not all arrive is reported and comes back as zeros
+    if (any_bad && tid == 0) atomicExch(p.x_err, 1);
+    for (int g = tid >> 7, i = 0; g < G; g += ATT_THREADS / 128, i++) {
       const long qh = qh0 + g;
-      if (p.x_recv) {                                // the same partial, pushed to every rank's receive buffer over NVLink
-        const long row = ((long)((x_ep & 1) * p.x_world + p.x_rank) * p.x_rows_cap + qh) * 130;
-        for (int rk = 0; rk < p.x_world; rk++) {
-          unsigned long long* o = p.x_recv[rk] + row;
-          if (d == 0) { x_store(o, M * LN2, (u32)x_ep + 1u); x_store(o + 1, L, (u32)x_ep + 1u); }
-          x_store(o + 2 + d, Ac, (u32)x_ep + 1u);
-        }
-      } else if (p.part) {                           // un-normalised partial for a cross-GPU merge: m in natural-log units
-        float* o = p.part + qh * 130;
-        if (d == 0) { o[0] = M * LN2; o[1] = L; }
-        o[2 + d] = Ac;
-      } else {
-        const float v = L > 0.f ? Ac / L : 0.f;
-        p.out[qh * D + d] = __bfloat16_as_ushort(__float2bfloat16(v));
-        if (p.out_f32) p.out_f32[qh * D + d] = v;
-      }
+      const float o = any_bad ? 0.f : v[i];
+      if (p.out) p.out[qh * D + d] = __bfloat16_as_ushort(__float2bfloat16(o));
+      if (p.out_f32) p.out_f32[qh * D + d] = o;
     }
-    if (p.x_recv) {
-      // Every entry carries the exchange number, so nothing else announces the rows (see x_store / x_load).
-      if (!p.x_fused) return;                        // the wait-and-merge runs as its own launch (gaac_exchange_merge)
-      // ---- fused: wait (bounded) for the rows of this group from every rank, merge them, write the output
-      const unsigned long long* base = p.x_recv[p.x_rank] + (long)(x_ep & 1) * p.x_world * p.x_rows_cap * 130;
-      float v[2] = {0.f, 0.f};
-      int bad = 0;
-      for (int g = tid >> 7, i = 0; g < G; g += ATT_THREADS / 128, i++)
-        bad |= !x_merge_rows(base, p.x_world, p.x_rows_cap, qh0 + g, d, (u32)x_ep + 1u, v[i]);
-      const int any_bad = __syncthreads_or(bad);     // a group whose rows did not all arrive is reported and comes back as zeros
-      if (any_bad && tid == 0) atomicExch(p.x_err, 1);
-      for (int g = tid >> 7, i = 0; g < G; g += ATT_THREADS / 128, i++) {
-        const long qh = qh0 + g;
-        const float o = any_bad ? 0.f : v[i];
-        if (p.out) p.out[qh * D + d] = __bfloat16_as_ushort(__float2bfloat16(o));
-        if (p.out_f32) p.out_f32[qh * D + d] = o;
-      }
-      // the exchange number advances when every group of this launch is through (each has read it by then)
-      __syncthreads();
-      if (tid == 0) {
-        __threadfence();
-        if (atomicAdd(p.x_ticket, 1) == (int)gridDim.x - 1) { *p.x_ticket = 0; __threadfence(); atomicAdd(p.x_epoch, 1); }
-      }
+    // the exchange number advances when every group of this launch is through (each has read it by then)
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      if (atomicAdd(p.x_ticket, 1) == (int)gridDim.x - 1) { *p.x_ticket = 0; __threadfence(); atomicAdd(p.x_epoch, 1); }
     }
   }
 }
@@ -1107,107 +533,96 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 // both warps run the same softmax step on the same numbers.  Tiles are handed to PAIRS from the CTA's counter; the even warp
 // takes the number and passes it through the exchange slot.  A warp whose bounded wait on its copies runs out says so in
 // the same slot, so that both warps of the pair leave the loop together and nobody is left at the barrier.
-// Output: un-normalised partials of "virtual heads" vq = 2 * query head + half, i.e. exactly the layout gaac_combine turns into
-// out [B, n_q, 256].
-static_assert(GAAC_LUTC == 0 && ATT_WARPS % 2 == 0, "the 256-dim kernel uses the arithmetic code spreading and warp pairs");
-constexpr int T256_HALF = 2048 + 256 + 256;                       // per half: escape-byte table, K base words, V base words (same offsets as the CTA tables above)
-constexpr int XCH_PAR_BYTES = 2 * 32 * 16 + 16;                    // one parity: two halves x 32 lanes x float4, then {next tile, fail flag of half 0, of half 1, -}
-constexpr int T256_XCH = 2 * T256_HALF;
-constexpr int TABLE256_BYTES = T256_XCH + (ATT_WARPS / 2) * 2 * XCH_PAR_BYTES;
-constexpr int ATT256_SMEM = TABLE256_BYTES + ATT_WARPS * WARP_SMEM;
-static_assert(TB_KB == 2048 && TB_VB == 2048 + 256 && TABLE256_BYTES % 16 == 0 && ATT256_SMEM + 64 <= 232448, "table layout shared with the 128-dim kernel; one CTA per SM");
+// Output: partials of "virtual heads" vq = 2 * query head + half, which the last CTA of a (row, kv head) merges into out [B, n_q, 256].
 
+constexpr int META256_TILES = 128;
+constexpr int PSLOT256 = SLOT_OVF_OFF + 144;                       // staged bytes of a tile slot, at most (what shared memory has room for)
+constexpr int XCH_PAR_BYTES = 2 * 32 * 16 + 16;                    // one parity: two halves x 32 lanes x float4, then {next tile, fail flag of half 0, of half 1, -}
+constexpr int T256_BASES = LUTX_BYTES, T256_ZERO = T256_BASES + 2 * BASES_BYTES, T256_META = T256_ZERO + 16, T256_XCH = T256_META + META256_TILES * 16;
+constexpr int T256_SCRATCH = T256_XCH + (ATT_WARPS / 2) * 2 * XCH_PAR_BYTES, T256_RING = T256_SCRATCH + ATT_WARPS * WARP_SCRATCH;
+constexpr int STAGE256_BYTES = 16 + 2 * PSLOT256, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
+constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES;
+static_assert(T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_XCH % 16 == 0 && ATT256_SMEM + 64 <= 232448, "one CTA per SM");
+
+template <int NSET>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int s_next;
+  __shared__ int s_next, s_last;
   const int bh = blockIdx.x, split = blockIdx.y, tid = threadIdx.x, lane = tid & 31, j = lane & 3, r = lane >> 2;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);
   const int hf = warp & 1, pair = warp >> 1;
-  const int b = bh / p.n_kv, kvh = bh % p.n_kv, G = p.G, hh = 2 * kvh + hf, NT = 4 * p.n_kv;    // p.n_kv = 256-dim kv heads; NT tile slots per block
+  const int b = bh / p.n_kv, kvh = bh % p.n_kv, G = p.G, NT = 4 * p.n_kv;    // p.n_kv = 256-dim kv heads; NT tile slots per block
+  const int ring = T256_RING + warp * WARP256_BYTES;
+  const u32 smem_s = (u32)__cvta_generic_to_shared(smem), ring_s = smem_s + ring;
+  if (tid < 256) fill_lutx(reinterpret_cast<u32x2*>(smem), tid);
+  if (tid >= 256 && tid < 260) reinterpret_cast<u32*>(smem + T256_ZERO)[tid - 256] = 0u;
+  for (int i = tid; i < (ATT_WARPS / 2) * 2 * XCH_PAR_BYTES / 4; i += ATT_THREADS) reinterpret_cast<u32*>(smem + T256_XCH)[i] = 0u;      // exchange slots start out zero
+  if (lane == 0) {
+    mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
   const int S = __shfl_sync(FULLM, p.seq_len[b], 0);
   const int ntiles = (S + 15) >> 4, chunk = (ntiles + p.nsplit - 1) / p.nsplit;
-  const int tlo = min(split * chunk, ntiles), thi = min(tlo + chunk, ntiles);
-  uint8_t* ring = smem + TABLE256_BYTES + warp * WARP_SMEM;
-  const u32 ring_s = (u32)__cvta_generic_to_shared(ring);
-  const uint8_t* tables = smem + hf * T256_HALF;
+  const int tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo);
   uint8_t* xch = smem + T256_XCH + pair * (2 * XCH_PAR_BYTES);
-  auto meta = [&](int tile) -> TileMeta { const int pc = p.bt[(long)b * p.bt_stride + tile] * NT + 2 * hh; return TileMeta{p.mt[pc], p.mt[pc + 1]}; };
-  auto issue = [&](u32 st, const TileMeta& m) {                                // executed by lane 0
-    const u32 mb = st + ST_MBAR, n = (u32)min(p.TS, SLOT_OVF_OFF + ESC_COPY);
-    mbar_expect_tx(mb, (m.mk >= 0 ? n : 0u) + (m.mv >= 0 ? n : 0u));
-    if (m.mk >= 0) bulk_g2s(st + ST_KSM, p.buf + (long)m.mk * p.TS, n, mb);
-    if (m.mv >= 0) bulk_g2s(st + ST_VSM, p.buf + (long)m.mv * p.TS, n, mb);
+  const int4* meta_s = reinterpret_cast<const int4*>(smem + T256_META);        // per tile: mode-table entries of {K, V} of half 0, of half 1
+  auto slot_of = [&](int i) { return p.bt[(long)b * p.bt_stride + tlo + i] * NT + 4 * kvh; };
+  auto meta_of = [&](int i) -> TileMeta {
+    if (i < META256_TILES) { const int2 m = reinterpret_cast<const int2*>(meta_s + i)[hf]; return TileMeta{m.x, m.y}; }
+    const int pc = slot_of(i) + 2 * hf;
+    return TileMeta{p.mt[pc], p.mt[pc + 1]};
   };
-  if (lane == 0) {
-    mbar_init(ring_s + ST_MBAR, 1); mbar_init(ring_s + STAGE_BYTES + ST_MBAR, 1);
-    *reinterpret_cast<unsigned long long*>(ring + ST_ZERO) = 0ull; *reinterpret_cast<unsigned long long*>(ring + STAGE_BYTES + ST_ZERO) = 0ull;
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncwarp();
-  int tile = tlo + pair;
+  const u32 slot_bytes = (u32)min(p.TS, PSLOT256);
+  auto issue = [&](u32 st, const TileMeta& m) {                                // executed by lane 0
+    // the stage may have been written through ordinary stores (patch numbers): order those before the copy engine's writes
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(st, (m.mk >= 0 ? slot_bytes : 0u) + (m.mv >= 0 ? slot_bytes : 0u));
+    if (m.mk >= 0) bulk_g2s(st + 16, p.buf + (long)m.mk * p.TS, slot_bytes, st);
+    if (m.mv >= 0) bulk_g2s(st + 16 + PSLOT256, p.buf + (long)m.mv * p.TS, slot_bytes, st);
+  };
+  int it = pair;
   TileMeta cur{0, 0};
-  if (tile < thi) { cur = meta(tile); if (lane == 0) issue(ring_s, cur); }
+  if (it < n) {
+    const int pc = slot_of(it) + 2 * hf;
+    cur = TileMeta{p.mt[pc], p.mt[pc + 1]};
+    if (lane == 0) issue(ring_s, cur);
+  }
   QFrag Q;
-#if GAAC_QSMEM
-#error "the 256-dim kernel keeps the query fragments in registers"
-#else
-  {
-    const bool ok = r < G;
-    const uint16_t* qp = p.q + ((long)b * p.n_q + kvh * G + (ok ? r : 0)) * (2 * D) + hf * D;
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-      Q.qa[s][0] = ok ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j) : 0u;
-      Q.qa[s][1] = ok ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j + 8) : 0u;
-    }
+  load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * (2 * D) + hf * D, 2 * D, G, lane);
+  if (warp >= 8 && warp < 12) {
+    const int h2 = warp & 1, row = (2 * kvh + h2) * D;
+    uint8_t* o = smem + T256_BASES + h2 * BASES_BYTES;
+    if (warp < 10) fill_bases<false>(o, p.b3k + row, p.b4k + row, lane); else fill_bases<true>(o, p.b3v + row, p.b4v + row, lane);
   }
-#endif
-  {   // tables of both halves; exchange slots start out zero
-    if (tid < 256) { fill_lutx(reinterpret_cast<u32x2*>(smem + TB_LUTX), tid); fill_lutx(reinterpret_cast<u32x2*>(smem + T256_HALF + TB_LUTX), tid); }
-    constexpr int KB_T0 = ATT_THREADS >= 320 ? 256 : 0, VB_T0 = KB_T0 + 32;
-    if (tid >= KB_T0 && tid < KB_T0 + 32) {           // K: half, lane class jj, group gg
-      const int t = tid - KB_T0, h2 = t >> 4, jj = (t >> 2) & 3, gg = t & 3; u32 w3[8], w4[8];
-      const int row = 2 * kvh + h2;
-      k_base_words(p.b3k + row * D, jj, w3); k_base_words(p.b4k + row * D, jj, w4);
-      *reinterpret_cast<u32x4*>(smem + h2 * T256_HALF + TB_KB + 16 * (t & 15)) = u32x4{w3[2 * gg], w3[2 * gg + 1], w4[2 * gg] - w3[2 * gg], w4[2 * gg + 1] - w3[2 * gg + 1]};
-    } else if (tid >= VB_T0 && tid < VB_T0 + 32) {    // V: half, lane class rr, group gg
-      const int t = tid - VB_T0, h2 = t >> 4, rr = (t >> 1) & 7, gg = t & 1; u32 w3[4], w4[4];
-      const int row = 2 * kvh + h2;
-      v_base_words(p.b3v + row * D, rr, w3); v_base_words(p.b4v + row * D, rr, w4);
-      *reinterpret_cast<u32x4*>(smem + h2 * T256_HALF + TB_VB + 16 * (t & 15)) = u32x4{w3[2 * gg], w3[2 * gg + 1], w4[2 * gg] - w3[2 * gg], w4[2 * gg + 1] - w3[2 * gg + 1]};
-    }
-    for (int i = tid; i < (ATT_WARPS / 2) * 2 * XCH_PAR_BYTES / 4; i += ATT_THREADS) reinterpret_cast<u32*>(smem + T256_XCH)[i] = 0u;
-    if (tid == 0) s_next = tlo + ATT_WARPS / 2;       // tiles tlo .. tlo + pairs - 1 go to the pairs in order, the rest is handed out on demand
-  }
-  WarpAcc A;
-#pragma unroll
-  for (int n = 0; n < 8; n++) A.acc[n][0] = A.acc[n][1] = A.acc[n][2] = A.acc[n][3] = 0.f;
-  A.m0 = A.m1 = -CUDART_INF_F; A.l0 = A.l1 = 0.f;
+  if (tid < min(n, META256_TILES)) { const int pc = slot_of(tid); reinterpret_cast<int4*>(smem + T256_META)[tid] = make_int4(p.mt[pc], p.mt[pc + 1], p.mt[pc + 2], p.mt[pc + 3]); }
+  if (tid == 0) s_next = ATT_WARPS / 2;               // tiles 0 .. pairs - 1 of the range go to the pairs in order, the rest is handed out on demand
+  WarpAcc<NSET> A;
+  A.clear();
   __syncthreads();
 
+  const WarpView W{smem_s, smem_s + T256_BASES + hf * BASES_BYTES, smem_s + T256_ZERO, smem_s + T256_SCRATCH + warp * WARP_SCRATCH};
   int stg = 0, par = 0;
   u32 phase = 0;
-  const int esc_off = ST_KESC - ST_ZERO, esc_off_v = ST_VESC - ST_ZERO;
-  const int esc_avail = min(p.ovf_slot, min(p.TS, SLOT_OVF_OFF + ESC_COPY) - SLOT_OVF_OFF);
-  while (tile < thi) {
+  const int avail = min(p.ovf_slot, (int)slot_bytes - SLOT_OVF_OFF);
+  while (it < n) {
     int t1 = 0;
     if (hf == 0 && lane == 0) t1 = atomicAdd(&s_next, 1);
-    const bool ok = __all_sync(FULLM, mbar_wait(ring_s + stg * STAGE_BYTES + ST_MBAR, (phase >> stg) & 1u));
+    const bool ok = __all_sync(FULLM, mbar_wait(ring_s + stg * STAGE256_BYTES, (phase >> stg) & 1u));
     phase ^= 1u << stg;
-    const uint8_t* stage = ring + stg * STAGE_BYTES;
-    const int nvalid = min(T, S - tile * T);
-    const bool rawk = cur.mk < 0, rawv = cur.mv < 0;
-    u32 flrow = 0; int rowoff = 0, total = 0;
+    const int so = ring + stg * STAGE256_BYTES + 16;
+    const uint8_t* stage = smem + so;
+    const int nvalid = min(T, S - (tlo + it) * T);
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
+    const u32 esc = smem_s + so + SLOT_OVF_OFF;
+    const SideView ks{stage, stage + SLOT_CD_OFF, stage + SLOT_FL_OFF, esc, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF, avail};
+    const SideView vs{stage + PSLOT256, stage + PSLOT256 + SLOT_CD_OFF, stage + PSLOT256 + SLOT_FL_OFF, esc + PSLOT256, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, avail};
+    TilePlan plan{};
     if (ok) {
-      scan_rows(stage, rawk, rawv, lane, flrow, rowoff, total);
-      if (!rawk) {
-        if (esc_part(__shfl_sync(FULLM, total, 15)) + 8 <= esc_avail)
-          k_scores<true, false>(sc, stage, tables, EscSrc<true>{stage + ST_ZERO, nullptr, esc_off}, flrow, rowoff, lane, Q);
-        else
-          k_scores<false, false>(sc, stage, tables, EscSrc<false>{nullptr, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF, 0}, flrow, rowoff, lane, Q);
-      } else raw_scores<false>(sc, p.raw + (long)(~cur.mk) * (T * D), nvalid, lane, Q);
+      plan = plan_tile(ks, vs, cur.mk < 0, cur.mv < 0, W, lane);
+      if (cur.mk >= 0) k_tile<false>(sc, ks, plan, W, lane, Q, nullptr, nvalid);
+      else raw_scores<false>(sc, p.raw + (long)(~cur.mk) * (T * D), nvalid, lane, Q, nullptr);
     }
     // ---- the two halves' partial scores meet; the next tile's number and a failed wait travel with them
     uint8_t* slot = xch + par * XCH_PAR_BYTES;
@@ -1222,36 +637,41 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     par ^= 1;
     if (failed) { if (lane == 0) atomicExch(p.err, 1); break; }                 // both warps of the pair see the same flags and leave together
     TileMeta nxt{0, 0};
-    if (t1 < thi) { nxt = meta(t1); if (lane == 0) issue(ring_s + (stg ^ 1) * STAGE_BYTES, nxt); }
-    PFrag P;
-    if (nvalid == T) softmax_step<true>(A, sc, p.scale_log2, nvalid, lane, P);
-    else softmax_step<false>(A, sc, p.scale_log2, nvalid, lane, P);
-    if (!rawv) {
-      if (esc_part(__shfl_sync(FULLM, total, 31)) + 8 <= esc_avail)
-        v_accum<true, false>(A, stage, tables, EscSrc<true>{stage + ST_ZERO, nullptr, esc_off_v}, flrow, rowoff, lane, P);
-      else
-        v_accum<false, false>(A, stage, tables, EscSrc<false>{nullptr, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, 0}, flrow, rowoff, lane, P);
-    } else raw_accum<false>(A, p.raw + (long)(~cur.mv) * (T * D), nvalid, lane, P);
-    cur = nxt; stg ^= 1; tile = t1;
+    if (t1 < n) { nxt = meta_of(t1); if (lane == 0) issue(ring_s + (stg ^ 1) * STAGE256_BYTES, nxt); }
+    PFrag<NSET> P;
+    if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
+    else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
+    if (cur.mv >= 0) v_tile<false, NSET>(A, vs, plan, W, lane, P, nullptr, nvalid);
+    else raw_accum<false, NSET>(A, p.raw + (long)(~cur.mv) * (T * D), nvalid, lane, P, nullptr);
+    cur = nxt; stg ^= 1; it = t1;
+    __syncwarp();                                      // every lane has read this stage before its next copies are issued
   }
-  // ---- merge the warps of the CTA, half by half, and write one partial per virtual head (2 * query head + half)
+  // ---- merge the warps of the CTA, half by half: one partial per virtual head (2 * query head + half)
   __syncthreads();
-  constexpr int ACC_LD = D + 4;
-  float* sh_m = reinterpret_cast<float*>(smem + TABLE256_BYTES);
+  float* sh_m = reinterpret_cast<float*>(smem + T256_RING);
   float* sh_l = sh_m + ATT_WARPS * 8;
   float* sh_acc = sh_l + ATT_WARPS * 8;
 #pragma unroll
-  for (int o = 4; o < 32; o <<= 1) { A.l0 += __shfl_xor_sync(FULLM, A.l0, o); A.l1 += __shfl_xor_sync(FULLM, A.l1, o); }
-  if (r == 0) { sh_m[warp * 8 + 2 * j] = A.m0; sh_l[warp * 8 + 2 * j] = A.l0; sh_m[warp * 8 + 2 * j + 1] = A.m1; sh_l[warp * 8 + 2 * j + 1] = A.l1; }
-  if (2 * j < G) {
+  for (int s = 0; s < NSET; s++) {
+    const int h = 4 * s + j;
+    float l = A.l[s];
 #pragma unroll
-    for (int n = 0; n < 8; n++) {
-      float* a0 = sh_acc + ((warp * 8 + 2 * j) * ACC_LD) + 16 * n + r;
-      a0[0] = A.acc[n][0]; a0[ACC_LD] = A.acc[n][1]; a0[8] = A.acc[n][2]; a0[ACC_LD + 8] = A.acc[n][3];
+    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(FULLM, l, o);
+    if (r == 0) { sh_m[warp * 8 + h] = A.m[s]; sh_l[warp * 8 + h] = l; }
+    if (h < G) {
+      float* a0 = sh_acc + (warp * 8 + h) * ACC_LD + r;
+#pragma unroll
+      for (int i = 0; i < 16; i++) a0[8 * i] = A.acc[s][i >> 2][i & 3];
     }
   }
   __syncthreads();
-  const int d = tid & 127;
+  const int d = tid & 127, NS = p.nsplit;
+  const long row0 = 2 * ((long)b * p.n_q + kvh * G);
+  auto deliver = [&](long row, float L, float Ac) {
+    const float v = L > 0.f ? Ac / L : 0.f;
+    p.out[row * D + d] = __bfloat16_as_ushort(__float2bfloat16(v));
+    if (p.out_f32) p.out_f32[row * D + d] = v;
+  };
   for (int vg = tid >> 7; vg < 2 * G; vg += ATT_THREADS / 128) {
     const int g = vg >> 1, h2 = vg & 1;
     float M = -CUDART_INF_F;
@@ -1265,9 +685,17 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
       const float f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
       Lc += sh_l[ww * 8 + g] * f; Ac += sh_acc[(ww * 8 + g) * ACC_LD + d] * f;
     }
-    const long vq = ((long)b * p.n_q + kvh * G + g) * 2 + h2, pidx = vq * p.nsplit + split;
-    if (d == 0) { p.pm[pidx] = M * LN2; p.pl[pidx] = Lc; }                      // m in natural-log units, as gaac_combine expects
-    p.pa[pidx * D + d] = Ac;
+    if (NS == 1) deliver(row0 + vg, Lc, Ac);
+    else {
+      const long pidx = (row0 + vg) * NS + split;
+      if (d == 0) { p.pm[pidx] = M; p.pl[pidx] = Lc; }
+      p.pa[pidx * D + d] = Ac;
+    }
+  }
+  if (NS == 1 || !last_split(p.counters + bh, NS, &s_last)) return;
+  for (int first = 0; first < 2 * G; first += 8) {
+    __syncthreads();                                   // the area is used again
+    merge_splits<8>(p, smem + T256_RING, row0 + first, min(8, 2 * G - first), [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
   }
 }
 
@@ -1392,17 +820,33 @@ static void launch_row_order(const int* seq_lens, const int* slot, int n_kv, int
   if (cudaLaunchKernelEx(&cfg, row_order_kernel, seq_lens, slot, n_kv, B, order) != cudaSuccess) cudaGetLastError();     // the attention launch that follows reports
 }
 
-template <bool PAGED, bool DUMP>
-static int launch_attn(const AttnParams& p, cudaStream_t st) {
-  cudaFuncSetAttribute(decode_attn_kernel<PAGED, DUMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM);
+template <bool PAGED, bool DUMP, int NSET>
+static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
+  cudaFuncSetAttribute(decode_attn_kernel<PAGED, DUMP, NSET>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit); cfg.blockDim = dim3(ATT_THREADS);
   cfg.dynamicSmemBytes = ATT_SMEM; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, decode_attn_kernel<PAGED, DUMP>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
+  if (cudaLaunchKernelEx(&cfg, decode_attn_kernel<PAGED, DUMP, NSET>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
   return launch_status();
+}
+template <int NSET>
+static int launch_attn256(const AttnParams& p, cudaStream_t st) {
+  cudaFuncSetAttribute(paged256_attn_kernel<NSET>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT256_SMEM);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit); cfg.blockDim = dim3(ATT_THREADS);
+  cfg.dynamicSmemBytes = ATT256_SMEM; cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, paged256_attn_kernel<NSET>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
+  return launch_status();
+}
+template <bool PAGED, bool DUMP>
+static int launch_attn(const AttnParams& p, cudaStream_t st) {
+  return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1>(p, st) : launch_attn_as<PAGED, DUMP, 2>(p, st);
 }
 
 static int sm_count_of_current_device() {
@@ -1588,18 +1032,9 @@ extern "C" int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt
   p.buf = st->buf; p.raw = (const uint16_t*)st->raw; p.mt = st->mt; p.bt = bt; p.bt_stride = bt_stride; p.TS = st->TS; p.ovf_slot = st->ovf_slot;
   p.b3k = st->b3k; p.b4k = st->b4k; p.b3v = st->b3v; p.b4v = st->b4v; p.seq_len = seq_lens;
   p.q = (const uint16_t*)q_bf16; p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.G = n_q / n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
+  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32;
   if (int e = carve_workspace(workspace, workspace_bytes, B, 2 * n_q, nsplit, p)) return e;     // one partial per (query head, half)
-  cudaFuncSetAttribute(paged256_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT256_SMEM);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(B * n_kv), (unsigned)nsplit); cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = ATT256_SMEM; cfg.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, paged256_attn_kernel, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
-  // the halves' partials are laid out as 2 * B * n_q heads of 128 dims, which is out [B, n_q, 256] after the merge
-  combine_kernel<<<(unsigned)(2 * B * n_q), 128, 0, (cudaStream_t)stream>>>(p.pm, p.pl, p.pa, nsplit, (uint16_t*)out_bf16, out_f32);
-  return launch_status();
+  return p.G <= 4 ? launch_attn256<1>(p, (cudaStream_t)stream) : launch_attn256<2>(p, (cudaStream_t)stream);
 }
 
 // ---- test hooks: the same kernels, instantiated so that every rebuilt BF16 fragment is also written to memory

@@ -1,0 +1,483 @@
+// Warp-level pieces of the fused decode attention: asynchronous copies, the rebuild of a compressed 16-token tile into tensor-core
+// fragments, the score and value products and the online softmax step.  Used by the kernels of gaac_attn.cu.
+//
+// What bounds them: instruction issue and the integer (ALU) pipe, whose rate is half the issue rate, not HBM.  Measured on a B200
+// at batch 1, 32 query / 8 kv heads, 65536 tokens: 1354 warp instructions per (K tile + V tile) at 67 % issue slots used before the
+// forms below, of which the group decoder itself is about 530; the rest was copy issue per warp, escape offsets through two
+// lookups per row, a transpose of the V fragments and softmax work for padding heads.
+//
+// Head columns.  The tensor-core tile has 8 columns.  Query heads are handled in sets of four (NSET = 1 for a GQA group of up to
+// 4, 2 for 5..8); lane j of a quad works for head 4 * set + j throughout:
+//   scores  S^T[16 tok x 8] = K[16 x 128] . Q^T : column 2j = head j of set 0, column 2j + 1 = head j of set 1 (zero without it)
+//   values  O^T += V^T . P^T : a rebuilt word holds TWO channels of one token, so the contraction runs over (token, channel parity)
+//           and column 2j + parity takes (P, 0) or (0, P): the words go into the product as they were decoded, with no transpose
+//           (32 byte permutes per tile before), and each lane gets both channels of its own head.
+#pragma once
+#include <cuda_bf16.h>
+#include <math_constants.h>
+#include "gaac_tile.h"
+
+namespace gaac {
+
+constexpr unsigned FULLM = 0xffffffffu;
+constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+
+__device__ __forceinline__ void mma16816(float* c, u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// ---- bulk asynchronous copies (TMA engine, no tensor map): global -> shared, completion counted in bytes on an mbarrier.
+// Both addresses are 16-byte aligned and the size is a multiple of 16 at every call site.
+__device__ __forceinline__ void mbar_init(u32 mbar, u32 count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(count)); }
+__device__ __forceinline__ void mbar_expect_tx(u32 mbar, u32 bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_add_tx(u32 mbar, u32 bytes) { asm volatile("mbarrier.expect_tx.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(u32 mbar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory"); }
+__device__ __forceinline__ void bulk_g2s(u32 dst, const void* src, u32 bytes, u32 mbar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
+}
+// Bounded wait for a phase of the barrier: false when it gave up (the copies of a stage normally land within microseconds;
+// the bound is there so that a lost copy can never hang the GPU).
+constexpr int MBAR_WAIT_LIMIT = 1 << 22;
+__device__ __forceinline__ bool mbar_wait(u32 mbar, u32 parity) {
+  for (int it = 0; it < MBAR_WAIT_LIMIT; it++) {
+    u32 ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// The same for a count in shared memory that other warps raise: waits until it is at least `least`.
+__device__ __forceinline__ bool wait_count(u32 addr, int least) {
+  for (int it = 0; it < MBAR_WAIT_LIMIT; it++) {
+    int v;
+    asm volatile("ld.relaxed.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    if (v >= least) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ float fast_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+// one step of an inclusive scan over a warp: v += v of the lane `d` below, where there is one
+__device__ __forceinline__ void scan_step(u32& v, int d) {
+  asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
+}
+
+// What a warp needs to know of a tile besides its staged bytes.  Slot layout: offsets of the tile's escape bytes inside the head's
+// escape bytes.  Paged layout: the mode-table entries (>= 0: compressed slot, < 0: bit-complement of a raw tile of the pool).
+struct TileMeta { int mk, mv; };
+
+// ---- running state of one warp.  acc[set][mt][c] = O[head 4 * set + j][channel 8 * (4 * mt + c) + r]; m, l in the exp2 domain, l summed over
+// this lane's tokens only
+template <int NSET> struct WarpAcc {
+  float acc[NSET][4][4];
+  float m[NSET], l[NSET];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int s = 0; s < NSET; s++) {
+      m[s] = -CUDART_INF_F; l[s] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[s][i][0] = acc[s][i][1] = acc[s][i][2] = acc[s][i][3] = 0.f;
+    }
+  }
+};
+
+// Q^T B-fragments of the score product.  Lane (j, r) provides column r = head 4 * (r & 1) + (r >> 1): for k-step s the words
+// q[16s + 2j, +1] and q[16s + 2j + 8, +9] of that head (zero where the group has no such head).
+struct QFrag { u32 qa[8][2]; };
+__device__ __forceinline__ int q_head(int r) { return 4 * (r & 1) + (r >> 1); }
+__device__ __forceinline__ void load_q(QFrag& Q, const uint16_t* q0, long head_stride, int G, int lane) {
+  const int j = lane & 3, h = q_head(lane >> 2);
+  const uint16_t* qp = q0 + (h < G ? h : 0) * head_stride;
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    Q.qa[s][0] = h < G ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j) : 0u;
+    Q.qa[s][1] = h < G ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j + 8) : 0u;
+  }
+}
+
+// Weights of one tile as B-fragments of the value product: [0]: tokens 2j (b0) and 2j + 1 (b1), [1]: tokens 2j + 8 and 2j + 9.  A weight enters as the
+// sum of two BF16 numbers, its rounded value (hi) and the rounded remainder (lo), which brings its relative error to 2^-16.
+template <int NSET> struct PFrag { u32 hi[NSET][2][2], lo[NSET][2][2]; };
+
+// Online softmax on the score fragment.  The running maximum is only raised (and the accumulators rescaled) when some score of the
+// tile exceeds it by more than RESCALE_TAU in the exp2 domain; otherwise the tile is weighted against the stale maximum, so P stays
+// below 2^RESCALE_TAU.  Sums and accumulators are fp32 and P keeps its relative rounding, so the result is as exact as with the true
+// maximum, and the common tile needs no cross-lane reduction, no rescale factor and no accumulator multiply.
+constexpr float RESCALE_TAU = 16.f;
+template <int NSET, bool FULL_TILE>
+__device__ __forceinline__ void softmax_step(WarpAcc<NSET>& A, const float* sc, float scale_log2, int nvalid, int lane, PFrag<NSET>& P) {
+  const int j = lane & 3, r = lane >> 2;
+  float s0[NSET], s8[NSET];
+  bool over = false;
+#pragma unroll
+  for (int s = 0; s < NSET; s++) {
+    s0[s] = FULL_TILE || r < nvalid ? sc[s] * scale_log2 : -CUDART_INF_F;             // a full tile needs no token masks
+    s8[s] = FULL_TILE || r + 8 < nvalid ? sc[2 + s] * scale_log2 : -CUDART_INF_F;
+    over |= fmaxf(s0[s], s8[s]) > A.m[s] + RESCALE_TAU;
+  }
+  if (__any_sync(FULLM, over)) {
+#pragma unroll
+    for (int s = 0; s < NSET; s++) {
+      float mt = fmaxf(s0[s], s8[s]);
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) mt = fmaxf(mt, __shfl_xor_sync(FULLM, mt, o));
+      const float mn = fmaxf(A.m[s], mt), al = (mn == -CUDART_INF_F) ? 0.f : fast_exp2(A.m[s] - mn);
+      A.l[s] *= al; A.m[s] = mn;
+#pragma unroll
+      for (int i = 0; i < 4; i++) { A.acc[s][i][0] *= al; A.acc[s][i][1] *= al; A.acc[s][i][2] *= al; A.acc[s][i][3] *= al; }
+    }
+  }
+  // this lane has the weights of tokens r and r + 8 for head j; as column r of the value product it needs those of head r >> 1 for tokens
+  // 2j, 2j + 1, 2j + 8, 2j + 9, in the low (parity 0) or high (parity 1) half of a word whose other half is zero
+  const int src = 8 * j + (r >> 1);
+  const u32 sel0 = (r & 1) ? 0x1044u : 0x4410u, sel8 = (r & 1) ? 0x3244u : 0x4432u;
+#pragma unroll
+  for (int s = 0; s < NSET; s++) {
+    const float mu = fmaxf(A.m[s], -1e30f);                                          // a maximum of -inf (nothing seen yet) must not produce inf - inf
+    const float p0 = fast_exp2(s0[s] - mu), p8 = fast_exp2(s8[s] - mu);
+    A.l[s] += p0 + p8;
+    __nv_bfloat162 h = __floats2bfloat162_rn(p0, p8);
+    const u32 H = *reinterpret_cast<u32*>(&h);
+    __nv_bfloat162 l = __floats2bfloat162_rn(p0 - __uint_as_float(H << 16), p8 - __uint_as_float(H & 0xFFFF0000u));      // the remainders are exact in fp32
+    const u32 L = *reinterpret_cast<u32*>(&l);
+    const u32 ha = __shfl_sync(FULLM, H, src), hb = __shfl_sync(FULLM, H, src + 4), la = __shfl_sync(FULLM, L, src), lb = __shfl_sync(FULLM, L, src + 4);
+    P.hi[s][0][0] = prmt(ha, 0u, sel0); P.hi[s][0][1] = prmt(hb, 0u, sel0); P.hi[s][1][0] = prmt(ha, 0u, sel8); P.hi[s][1][1] = prmt(hb, 0u, sel8);
+    P.lo[s][0][0] = prmt(la, 0u, sel0); P.lo[s][0][1] = prmt(lb, 0u, sel0); P.lo[s][1][0] = prmt(la, 0u, sel8); P.lo[s][1][1] = prmt(lb, 0u, sel8);
+  }
+}
+
+// Value product of words i, i + 1 (i = 2 * mt) of the lane's four tokens (2j, 2j + 1, 2j + 8, 2j + 9).
+template <int NSET>
+__device__ __forceinline__ void pv_words(WarpAcc<NSET>& A, int mt, const u32 (&w0)[4], const u32 (&w1)[4], const PFrag<NSET>& P) {
+#pragma unroll
+  for (int s = 0; s < NSET; s++) {
+    mma16816(A.acc[s][mt], w0[0], w1[0], w0[1], w1[1], P.hi[s][0][0], P.hi[s][0][1]);
+    mma16816(A.acc[s][mt], w0[0], w1[0], w0[1], w1[1], P.lo[s][0][0], P.lo[s][0][1]);
+    mma16816(A.acc[s][mt], w0[2], w1[2], w0[3], w1[3], P.hi[s][1][0], P.hi[s][1][1]);
+    mma16816(A.acc[s][mt], w0[2], w1[2], w0[3], w1[3], P.lo[s][1][0], P.lo[s][1][1]);
+  }
+}
+
+// ---- CTA tables and the stage layout
+constexpr int ESC_WIN = 192;                                // escape bytes staged per tile and kind in the paged layout; longer tiles read theirs from global memory
+constexpr int PSLOT = SLOT_OVF_OFF + ESC_WIN + 16;          // staged bytes of a paged tile slot, at most
+constexpr int PATCH_MAX = 64;                               // raw groups of a tile (K and V together) that the patch table holds
+constexpr int PATCH_BYTES = PATCH_MAX * 8, WALK_BYTES = 32 * 16;
+constexpr int WARP_SCRATCH = PATCH_BYTES + WALK_BYTES;      // shared memory of a warp besides its stages: patch table, segment positions per lane
+constexpr int LUTX_BYTES = 2048, BASES_V = 256, BASES_BYTES = 512;      // escape-byte table; base words of K, of V behind them
+
+// One side (K or V) of a staged tile.  esc = shared-memory address of its first escape byte, glob = the same bytes in global memory, avail = staged escape
+// bytes.
+struct SideView { const uint8_t *sm, *cd, *fl; u32 esc; const uint8_t* glob; int avail; };
+// What does not change from tile to tile, as shared-memory addresses: the escape-byte table, the base words (K, then V), a zero byte, the warp's
+// scratch.
+struct WarpView { u32 lutx, bases, zero, scratch; };
+
+__device__ __forceinline__ u32 lds_u8(u32 a) { u32 v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ u32 lds_u16(u32 a) { u32 v; asm volatile("{\n .reg .u16 t;\n ld.shared.u16 t, [%1];\n cvt.u32.u16 %0, t;\n}" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ u32 lds_u32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ u32x2 lds_u64(u32 a) { u32x2 v; asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
+__device__ __forceinline__ u32x4 lds_u128(u32 a) { u32x4 v; asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
+__device__ __forceinline__ void sts_u8(u32 a, u32 v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_u64(u32 a, u32 x, u32 y) { asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
+__device__ __forceinline__ void sts_u128(u32 a, u32 x, u32 y, u32 z, u32 w) { asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory"); }
+
+// ---- byte-SWAR pieces written for the pipes of the SM: logic ops (LOP3 / PRMT / SHF) run on the ALU pipe, whose rate is half
+// the issue rate, so shifts that can be merged with an add are written as multiply-adds (FMA pipe)
+template <u32 K> __device__ __forceinline__ u32 mad_k(u32 a, u32 c) {
+  u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "n"(K), "r"(c)); return d;
+}
+__device__ __forceinline__ u32 mad(u32 a, u32 b, u32 c) { u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
+// the bits of a where the mask has ones, those of b elsewhere (one instruction; the compiler needs two for the and/and/or form)
+__device__ __forceinline__ u32 bit_select(u32 a, u32 b, u32 mask) { u32 d; asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(a), "r"(b), "r"(mask)); return d; }
+__device__ __forceinline__ void bf16x4_dev(u32 sm4, u32 e4, u32& p01, u32& p23) {
+  const u32 eh = __umulhi(e4, 0x80000000u);                          // e4 >> 1
+  const u32 el = mad_k<128u>(e4, 0u);                                // e4 << 7
+  const u32 h4 = bit_select(sm4, eh, 0x80808080u), l4 = bit_select(el, sm4, 0x80808080u);
+  p01 = prmt(l4, h4, 0x5140); p23 = prmt(l4, h4, 0x7362);
+}
+// four 5-bit fields at bits 0..19 of u -> field << 3 per byte (raw-tier exponent high bits); same result as spread_hi5
+__device__ __forceinline__ u32 spread_hi5_dev(u32 u) {
+  const u32 y = mad_k<64u>(u & 0xFFC00u, u & 0x3FFu);               // fields 0,1 at bits 0-9, fields 2,3 at bits 16-25
+  return mad_k<64u>(y & 0x03E003E0u, (y & 0x001F001Fu) << 3);       // odd fields up 3 more bits, everything << 3
+}
+// Escape bytes of up to four groups whose tags are t (upper bits clear): one for a promoted group (tag 01), five for a raw one (11), which
+// is one bit per tag bit and three more copies of every upper bit.
+__device__ __forceinline__ u32 seg_esc(u32 t) { return (u32)popc((t & 0xAAu) * 0x01010100u + t); }
+
+// The 24 code bits of a group, picked out of two neighbouring words by one byte permute that already puts codes 4..7 at the top:
+// bits 0..11 = codes 0..3, bits 20..31 = codes 4..7 (B = byte offset of the group in the lane's code string).
+template <int B> __device__ __forceinline__ u32 group_codes(const u32* cd) {
+  constexpr int i = B & 3;
+  constexpr u32 sel = (u32)i | (u32)(i + 1) << 4 | (u32)(i + 1) << 8 | (u32)(i + 2) << 12;
+  return prmt(cd[B >> 2], i >= 2 ? cd[(B >> 2) + 1] : 0u, sel);
+}
+
+// Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, pos =
+// position of the group's escape bytes, advanced past them.
+// WIN: the escape bytes are staged; pos counts from the zero byte (a group without an escape byte reads that), and raw groups were turned
+//   into patch-table entries by build_raw_patches, which also left each entry's number in the first payload byte of its group: the addends
+//   of EVERY group come from one load, out of the escape-byte table (byte = the 4-bit-window escape byte, or the zero byte) or out of the
+//   patch table (byte = entry number), chosen by address arithmetic, and the decoder has no branch (a branch per group cost 13 % of the
+//   kernel although 0.75 % of the groups took it).
+// !WIN (tiles whose escape bytes are not all staged, or with more raw groups than the patch table holds): plain loads at glob[pos].
+template <bool WIN>
+__device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& pos, const uint8_t* glob, const WarpView& w, const u32x4& bw, u32 out[4]) {
+  const u32 m1 = tg & 1u;                             // promoted (tags are 0, 1 or 3)
+  const u32 blo = mad(m1, bw.z, bw.x), bhi = mad(m1, bw.w, bw.y);
+  u32 x0, x1;
+  if (WIN) {
+    const u32 r2 = tg & 2u;                           // 2 for a raw group: its table is the patch table
+    const u32 xe = lds_u8(mad(m1, pos, w.zero));
+    const u32x2 x = lds_u64(mad_k<8u>(xe, mad(r2, (w.scratch - w.lutx) >> 1, w.lutx)));
+    x0 = x.x; x1 = x.y;
+    pos = mad_k<2u>(r2, pos);                         // a raw payload is five bytes: four here, one below with every promoted group
+  } else {
+    const u32x2 x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
+    x0 = x.x; x1 = x.y;
+    if (tg & 2u) {                                    // raw exponents: e = code | hi5 << 3 (the base must not contribute)
+      const uint8_t* p = glob + pos;
+      const int sh = 8 * (int)(reinterpret_cast<uintptr_t>(p) & 3);
+      const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+      const u32 w0 = a[0], w1 = a[1];
+      const u32 lo = funnel_r(w0, w1, sh), hi = w1 >> sh;              // bytes 0-3 and byte 4 of the payload
+      x0 = spread_hi5_dev(lo & 0xFFFFFu) - blo;
+      x1 = spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - bhi;
+      pos += 4;
+    }
+  }
+  pos += m1;
+  // four 3-bit codes -> four bytes in two steps; each step moves the upper fields with a multiply-add: (t & M) * (2^k - 1) + t
+  const u32 th = z >> 20;
+  const u32 xl = mad_k<1023u>(z & 0xFC0u, z & 0xFFFu), xh = mad_k<1023u>(th & 0xFC0u, th);
+  bf16x4_dev(sm_lo, mad_k<31u>(xl & 0x00380038u, xl) + blo + x0, out[0], out[1]);
+  bf16x4_dev(sm_hi, mad_k<31u>(xh & 0x00380038u, xh) + bhi + x1, out[2], out[3]);
+}
+
+// ---- where a lane's escape bytes are.  A lane owns 8 groups of a K tile (tokens r and r + 8, groups 4j .. 4j + 3 of each) and 8 of a V tile
+// (groups 2r, 2r + 1 of tokens 2j, 2j + 1, 2j + 8, 2j + 9).
+//   tags  2 bits per group: K segments (8 bits) at bits 0 and 8, V segments (4 bits) at bits 16, 20, 24, 28
+//   k, v  position of each segment's first escape byte inside the tile side, two per word
+//   win   bit 0 / 1: the K / V side takes the decoder with staged escape bytes
+struct TilePlan { u32 tags, k, v[2]; int win; };
+
+// Turn the raw-tier groups of a staged tile (K and V in one pass) into patch-table entries, so that the group decoder needs no branch.  A lane
+// walks its own raw groups: read the five payload bytes, spread the 5-bit fields to byte positions, take off the 4-bit-window base words (the
+// decoder adds them to every promoted group), store the two words as entry k, and write k over the first payload byte, which is where the
+// decoder looks.  Returns false when there are more than PATCH_MAX (the caller then takes the decoder that reads global memory, so the bytes
+// written over do not matter).  At a raw share of 0.75 % a tile pair has 3.8 raw groups, hardly ever two in one lane: one trip.
+__device__ __forceinline__ bool build_raw_patches(u32 raw_bits, const TilePlan& t, u32 esc_k, u32 esc_v, const WarpView& w, int lane) {
+  u32 some = __ballot_sync(FULLM, raw_bits != 0u);
+  if (!some) return true;
+  const u32 mine = w.scratch + PATCH_BYTES + 16 * lane, j = lane & 3, r = lane >> 2;
+  sts_u128(mine, prmt(t.k, 0u, 0x1010), prmt(t.k, 0u, 0x3232), t.v[0], t.v[1]);        // position by quarter of the tag word: the walk picks one at run time
+  u32 base = 0;
+  do {
+    const u32 n = base + (u32)popc(some);
+    if (n > PATCH_MAX) return false;
+    if (raw_bits) {
+      const u32 bit = (u32)__ffs((int)raw_bits) - 1u;                // upper tag bit of the group
+      raw_bits &= raw_bits - 1u;
+      const bool isv = bit >= 16u;
+      const u32 first = bit & (isv ? ~3u : ~7u);                     // first tag bit of its segment
+      const u32 below = (t.tags >> first) & ((1u << (bit - 1u - first)) - 1u);
+      const u32 pl = (isv ? esc_v : esc_k) + lds_u16(mine + ((bit >> 2) << 1)) + seg_esc(below);
+      const u32 k = base + (u32)popc(some & ((1u << lane) - 1u));
+      const u32 sh = 8u * (pl & 3u), w0 = lds_u32(pl & ~3u), w1 = lds_u32((pl & ~3u) + 4u);
+      const u32 lo = funnel_r(w0, w1, (int)sh), hi = w1 >> sh;         // bytes 0-3 and byte 4 of the payload
+      const u32x4 bw = lds_u128(w.bases + (isv ? BASES_V + 32u * r + 8u * (bit & 2u) : 64u * j + 8u * (bit & 6u)));
+      sts_u64(w.scratch + 8u * k, spread_hi5_dev(lo & 0xFFFFFu) - (bw.x + bw.z), spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - (bw.y + bw.w));
+      sts_u8(pl, k);
+    }
+    base = n;
+    some = __ballot_sync(FULLM, raw_bits != 0u);
+  } while (some);
+  __syncwarp();
+  return true;
+}
+
+// K: the lanes of an octet are in the order of the tile's escape bytes, so ONE warp scan over both octets' segment sizes (packed in a word) gives
+// every lane its two positions.  V: a scan over the lanes of equal j (one byte per token: a row has at most 80 escape bytes) places a lane
+// inside its four rows, then a scan over j (two 16-bit sums: tokens 0..7 and 8..15) places the rows inside the tile.
+__device__ __forceinline__ TilePlan plan_tile(const SideView& ks, const SideView& vs, bool rawk, bool rawv, const WarpView& w, int lane) {
+  const int j = lane & 3, r = lane >> 2;
+  TilePlan t;
+  u32 k0 = 0, k1 = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+  if (!rawk) { k0 = ks.fl[lane]; k1 = ks.fl[32 + lane]; }                                     // byte j of row r's tag word is byte `lane` of the octet's 32
+  if (!rawv) {
+    const uint2 a = *reinterpret_cast<const uint2*>(vs.fl + 8 * j), b = *reinterpret_cast<const uint2*>(vs.fl + 32 + 8 * j);      // tag words of the four tokens
+    v0 = (a.x >> (4 * r)) & 15u; v1 = (a.y >> (4 * r)) & 15u; v2 = (b.x >> (4 * r)) & 15u; v3 = (b.y >> (4 * r)) & 15u;
+  }
+  const u32 kown = mad_k<65536u>(seg_esc(k1), seg_esc(k0));
+  const u32 vown = mad_k<16777216u>(seg_esc(v3), mad_k<65536u>(seg_esc(v2), mad_k<256u>(seg_esc(v1), seg_esc(v0))));
+  u32 kinc = kown, vinc = vown;
+  scan_step(kinc, 1); scan_step(kinc, 2);
+  scan_step(kinc, 4); scan_step(vinc, 4); scan_step(kinc, 8); scan_step(vinc, 8); scan_step(kinc, 16); scan_step(vinc, 16);
+  const u32 ktot = __shfl_sync(FULLM, kinc, 31), rows = __shfl_sync(FULLM, vinc, 28 + j), before = vinc - vown;      // row totals; this lane's share starts `before` into its rows
+  t.k = kinc - kown + (ktot << 16);                                                          // the second octet's escape bytes follow the first's
+  const u32 sum = (rows & 0x00FF00FFu) + ((rows >> 8) & 0x00FF00FFu);                       // tokens 2j, 2j + 1 | tokens 2j + 8, 2j + 9
+  u32 js = sum;
+  { const u32 v = __shfl_up_sync(FULLM, js, 1, 4); if (j >= 1) js += v; }
+  { const u32 v = __shfl_up_sync(FULLM, js, 2, 4); if (j >= 2) js += v; }
+  const u32 vtot = __shfl_sync(FULLM, js, 3, 4), jb = js - sum + (vtot << 16);              // where rows 2j and 2j + 8 start
+  const u32 even = prmt(jb, 0u, 0x1010) + prmt(before, 0u, 0x4140) + ((rows & 0xFFu) << 16);
+  const u32 odd = prmt(jb, 0u, 0x3232) + prmt(before, 0u, 0x4342) + (rows & 0x00FF0000u);
+  t.v[0] = even; t.v[1] = odd;
+  t.tags = mad_k<256u>(k1, k0) + mad_k<65536u>(v0, mad_k<1048576u>(v1, mad_k<16777216u>(v2, mad_k<268435456u>(v3, 0u))));
+  const int total_k = (int)((ktot & 0xFFFFu) + (ktot >> 16)), total_v = (int)((vtot & 0xFFFFu) + (vtot >> 16));
+  t.win = (total_k <= ks.avail ? 1 : 0) | (total_v <= vs.avail ? 2 : 0);
+  const u32 sides = ((t.win & 1) ? 0xAAAAu : 0u) | ((t.win & 2) ? 0xAAAA0000u : 0u);
+  if (!build_raw_patches(t.tags & sides, t, ks.esc, vs.esc, w, lane)) t.win = 0;
+  return t;
+}
+
+// ---- score product of one compressed K tile: sc += K . Q^T.  dump (debug instantiation only): where token 0 of this tile goes in the
+// [token][128] dump of the head; rows >= nvalid are left alone.
+template <bool WIN, bool DUMP>
+__device__ __forceinline__ void k_decode(float* sc, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const QFrag& Q, uint16_t* dump, int nvalid) {
+  const int j = lane & 3, r = lane >> 2;
+  const u32 from = WIN ? s.esc - w.zero : 0u;
+  u32 pos[2] = {(t.k & 0xFFFFu) + from, (t.k >> 16) + from};
+  uint4 s0[2], s1[2]; u32 cd[2][3];
+  float s2[4] = {0.f, 0.f, 0.f, 0.f};                  // second accumulator: two dependent MMA chains of four instead of one of eight
+#pragma unroll
+  for (int o = 0; o < 2; o++) {
+    const uint8_t* m = s.sm + o * 1024 + 32 * lane;
+    s0[o] = *reinterpret_cast<const uint4*>(m); s1[o] = *reinterpret_cast<const uint4*>(m + 16);
+    const u32* c = reinterpret_cast<const u32*>(s.cd + o * 384 + 12 * lane);
+    cd[o][0] = c[0]; cd[o][1] = c[1]; cd[o][2] = c[2];
+  }
+#pragma unroll
+  for (int g = 0; g < 4; g++) {
+    const u32x4 bw = lds_u128(w.bases + 64 * j + 16 * g);
+    u32 f[2][4];
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      const u32 smlo = g == 0 ? s0[o].x : g == 1 ? s0[o].z : g == 2 ? s1[o].x : s1[o].z;
+      const u32 smhi = g == 0 ? s0[o].y : g == 1 ? s0[o].w : g == 2 ? s1[o].y : s1[o].w;
+      const u32 z = g == 0 ? group_codes<0>(cd[o]) : g == 1 ? group_codes<3>(cd[o]) : g == 2 ? group_codes<6>(cd[o]) : group_codes<9>(cd[o]);
+      decode_group_dev<WIN>(smlo, smhi, z, t.tags >> (8 * o + 2 * g), pos[o], s.glob, w, bw, f[o]);
+    }
+    if (DUMP) {
+#pragma unroll
+      for (int o = 0; o < 2; o++)
+        if (8 * o + r < nvalid) {
+          u32* row = reinterpret_cast<u32*>(dump + (8 * o + r) * D);
+          row[(32 * g + 2 * j) >> 1] = f[o][0]; row[(32 * g + 2 * j + 8) >> 1] = f[o][1];
+          row[(32 * g + 16 + 2 * j) >> 1] = f[o][2]; row[(32 * g + 16 + 2 * j + 8) >> 1] = f[o][3];
+        }
+    }
+    mma16816(sc, f[0][0], f[1][0], f[0][1], f[1][1], Q.qa[2 * g][0], Q.qa[2 * g][1]);
+    mma16816(s2, f[0][2], f[1][2], f[0][3], f[1][3], Q.qa[2 * g + 1][0], Q.qa[2 * g + 1][1]);
+  }
+  sc[0] += s2[0]; sc[1] += s2[1]; sc[2] += s2[2]; sc[3] += s2[3];
+}
+template <bool DUMP>
+__device__ __forceinline__ void k_tile(float* sc, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const QFrag& Q, uint16_t* dump, int nvalid) {
+  if (t.win & 1) k_decode<true, DUMP>(sc, s, t, w, lane, Q, dump, nvalid);
+  else k_decode<false, DUMP>(sc, s, t, w, lane, Q, dump, nvalid);
+}
+
+// ---- value product of one compressed V tile
+template <bool WIN, bool DUMP, int NSET>
+__device__ __forceinline__ void v_decode(WarpAcc<NSET>& A, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const PFrag<NSET>& P, uint16_t* dump, int nvalid) {
+  const int j = lane & 3, r = lane >> 2;
+  const u32 from = WIN ? s.esc - w.zero : 0u;
+  u32 pos[4] = {(t.v[0] & 0xFFFFu) + from, (t.v[0] >> 16) + from, (t.v[1] & 0xFFFFu) + from, (t.v[1] >> 16) + from};
+  uint4 sm[4]; u32 cd[6];
+#pragma unroll
+  for (int i = 0; i < 4; i++) sm[i] = *reinterpret_cast<const uint4*>(s.sm + 64 * lane + 16 * i);
+  {
+    const uint2* c2 = reinterpret_cast<const uint2*>(s.cd + 24 * lane);
+    const uint2 ca = c2[0], cb = c2[1], cc = c2[2];
+    cd[0] = ca.x; cd[1] = ca.y; cd[2] = cb.x; cd[3] = cb.y; cd[4] = cc.x; cd[5] = cc.y;
+  }
+#pragma unroll
+  for (int g = 0; g < 2; g++) {
+    const u32x4 bw = lds_u128(w.bases + BASES_V + 32 * r + 16 * g);
+    u32 f[4][4];
+    decode_group_dev<WIN>(g ? sm[0].z : sm[0].x, g ? sm[0].w : sm[0].y, g ? group_codes<3>(cd) : group_codes<0>(cd), t.tags >> (16 + 2 * g), pos[0], s.glob, w, bw, f[0]);
+    decode_group_dev<WIN>(g ? sm[1].z : sm[1].x, g ? sm[1].w : sm[1].y, g ? group_codes<9>(cd) : group_codes<6>(cd), t.tags >> (20 + 2 * g), pos[1], s.glob, w, bw, f[1]);
+    decode_group_dev<WIN>(g ? sm[2].z : sm[2].x, g ? sm[2].w : sm[2].y, g ? group_codes<15>(cd) : group_codes<12>(cd), t.tags >> (24 + 2 * g), pos[2], s.glob, w, bw, f[2]);
+    decode_group_dev<WIN>(g ? sm[3].z : sm[3].x, g ? sm[3].w : sm[3].y, g ? group_codes<21>(cd) : group_codes<18>(cd), t.tags >> (28 + 2 * g), pos[3], s.glob, w, bw, f[3]);
+    if (DUMP) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int tok = 2 * j + (i & 1) + 8 * (i >> 1);
+        if (tok < nvalid) {
+#pragma unroll
+          for (int q = 0; q < 4; q++) {                // word q = stored positions 16r + 8g + 2q, +1  <->  channels 8(8g + 2q) + r, 8(8g + 2q + 1) + r
+            dump[tok * D + 8 * (8 * g + 2 * q) + r] = (uint16_t)(f[i][q] & 0xFFFFu);
+            dump[tok * D + 8 * (8 * g + 2 * q + 1) + r] = (uint16_t)(f[i][q] >> 16);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const u32 w0[4] = {f[0][2 * h], f[1][2 * h], f[2][2 * h], f[3][2 * h]};
+      const u32 w1[4] = {f[0][2 * h + 1], f[1][2 * h + 1], f[2][2 * h + 1], f[3][2 * h + 1]};
+      pv_words<NSET>(A, 2 * g + h, w0, w1, P);
+    }
+  }
+}
+template <bool DUMP, int NSET>
+__device__ __forceinline__ void v_tile(WarpAcc<NSET>& A, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const PFrag<NSET>& P, uint16_t* dump, int nvalid) {
+  if (t.win & 2) v_decode<true, DUMP, NSET>(A, s, t, w, lane, P, dump, nvalid);
+  else v_decode<false, DUMP, NSET>(A, s, t, w, lane, P, dump, nvalid);
+}
+
+// ---- raw BF16 tiles [16][128] in global memory (rows >= nvalid are not read): the slot layout's tail, the paged layout's filling block
+// and its tiles that stayed raw
+template <bool DUMP>
+__device__ __forceinline__ void raw_scores(float* sc, const uint16_t* kraw, int nvalid, int lane, const QFrag& Q, uint16_t* dump) {
+  const int j = lane & 3, r = lane >> 2;
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    const uint16_t* k0 = kraw + r * D + 16 * s + 2 * j;
+    const uint16_t* k8 = k0 + 8 * D;
+    const u32 a0 = r < nvalid ? *reinterpret_cast<const u32*>(k0) : 0u, a2 = r < nvalid ? *reinterpret_cast<const u32*>(k0 + 8) : 0u;
+    const u32 a1 = r + 8 < nvalid ? *reinterpret_cast<const u32*>(k8) : 0u, a3 = r + 8 < nvalid ? *reinterpret_cast<const u32*>(k8 + 8) : 0u;
+    if (DUMP) {
+      if (r < nvalid) { u32* row = reinterpret_cast<u32*>(dump + r * D); row[(16 * s + 2 * j) >> 1] = a0; row[(16 * s + 2 * j + 8) >> 1] = a2; }
+      if (r + 8 < nvalid) { u32* row = reinterpret_cast<u32*>(dump + (r + 8) * D); row[(16 * s + 2 * j) >> 1] = a1; row[(16 * s + 2 * j + 8) >> 1] = a3; }
+    }
+    mma16816(sc, a0, a1, a2, a3, Q.qa[s][0], Q.qa[s][1]);
+  }
+}
+template <bool DUMP, int NSET>
+__device__ __forceinline__ void raw_accum(WarpAcc<NSET>& A, const uint16_t* vraw, int nvalid, int lane, const PFrag<NSET>& P, uint16_t* dump) {
+  const int j = lane & 3, r = lane >> 2;
+#pragma unroll
+  for (int mt = 0; mt < 4; mt++) {
+    u32 w0[4], w1[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const int tok = 2 * j + (t & 1) + 8 * (t >> 1);
+      const uint16_t* vr = vraw + tok * D + 8 * (4 * mt) + r;
+      const bool ok = tok < nvalid;
+      const u32 e0 = ok ? vr[0] : 0u, e1 = ok ? vr[8] : 0u, e2 = ok ? vr[16] : 0u, e3 = ok ? vr[24] : 0u;
+      w0[t] = e0 | (e1 << 16); w1[t] = e2 | (e3 << 16);
+      if (DUMP && ok) {
+        uint16_t* o = dump + tok * D + 8 * (4 * mt) + r;
+        o[0] = (uint16_t)e0; o[8] = (uint16_t)e1; o[16] = (uint16_t)e2; o[24] = (uint16_t)e3;
+      }
+    }
+    pv_words<NSET>(A, mt, w0, w1, P);
+  }
+}
+
+// ---- base words of a side, {b3lo, b3hi, b4lo - b3lo, b4hi - b3hi} per group (16 bytes; K: lane class jj, group gg at 64 * jj + 16 * gg; V: lane class rr,
+// group gg at 32 * rr + 16 * gg).  Thread t < 32 makes word t of the 32 half groups: eight byte loads that do not wait for one another.
+template <bool VSIDE>
+__device__ __forceinline__ void fill_bases(uint8_t* bases, const uint8_t* b3, const uint8_t* b4, int t) {
+  int d0, d1, d2, d3;                                // channels of the half group (see k_base_words, v_base_words)
+  if (VSIDE) { d0 = 32 * (t & 3) + (t >> 2); d1 = d0 + 8; d2 = d0 + 16; d3 = d0 + 24; }
+  else { d0 = 16 * (t & 7) + 2 * (t >> 3); d1 = d0 + 1; d2 = d0 + 8; d3 = d0 + 9; }
+  const u32 w3 = (u32)b3[d0] | (u32)b3[d1] << 8 | (u32)b3[d2] << 16 | (u32)b3[d3] << 24, w4 = (u32)b4[d0] | (u32)b4[d1] << 8 | (u32)b4[d2] << 16 | (u32)b4[d3] << 24;
+  u32* o = reinterpret_cast<u32*>(bases + (VSIDE ? BASES_V : 0) + 16 * (t >> 1)) + (t & 1);
+  o[0] = w3; o[2] = w4 - w3;
+}
+
+}  // namespace gaac
