@@ -15,11 +15,10 @@
 #pragma once
 #include <cuda_bf16.h>
 #include <math_constants.h>
-#include "gaac_tile.h"
+#include "gaac_lane.cuh"
 
 namespace gaac {
 
-constexpr unsigned FULLM = 0xffffffffu;
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
 __device__ __forceinline__ void mma16816(float* c, u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
@@ -58,10 +57,6 @@ __device__ __forceinline__ bool wait_count(u32 addr, int least) {
   return false;
 }
 __device__ __forceinline__ float fast_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-// one step of an inclusive scan over a warp: v += v of the lane `d` below, where there is one
-__device__ __forceinline__ void scan_step(u32& v, int d) {
-  asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
-}
 
 // What a warp needs to know of a tile besides its staged bytes.  Slot layout: offsets of the tile's escape bytes inside the head's
 // escape bytes.  Paged layout: the mode-table entries (>= 0: compressed slot, < 0: bit-complement of a raw tile of the pool).
@@ -165,96 +160,10 @@ constexpr int PSLOT = SLOT_OVF_OFF + ESC_WIN + 16;          // staged bytes of a
 constexpr int PATCH_MAX = 64;                               // raw groups of a tile (K and V together) that the patch table holds
 constexpr int PATCH_BYTES = PATCH_MAX * 8, WALK_BYTES = 32 * 16;
 constexpr int WARP_SCRATCH = PATCH_BYTES + WALK_BYTES;      // shared memory of a warp besides its stages: patch table, segment positions per lane
-constexpr int LUTX_BYTES = 2048, BASES_V = 256, BASES_BYTES = 512;      // escape-byte table; base words of K, of V behind them
 
 // One side (K or V) of a staged tile.  esc = shared-memory address of its first escape byte, glob = the same bytes in global memory, avail = staged escape
 // bytes.
 struct SideView { const uint8_t *sm, *cd, *fl; u32 esc; const uint8_t* glob; int avail; };
-// What does not change from tile to tile, as shared-memory addresses: the escape-byte table, the base words (K, then V), a zero byte, the warp's
-// scratch.
-struct WarpView { u32 lutx, bases, zero, scratch; };
-
-__device__ __forceinline__ u32 lds_u8(u32 a) { u32 v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ u32 lds_u16(u32 a) { u32 v; asm volatile("{\n .reg .u16 t;\n ld.shared.u16 t, [%1];\n cvt.u32.u16 %0, t;\n}" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ u32 lds_u32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ u32x2 lds_u64(u32 a) { u32x2 v; asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
-__device__ __forceinline__ u32x4 lds_u128(u32 a) { u32x4 v; asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
-__device__ __forceinline__ void sts_u8(u32 a, u32 v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
-__device__ __forceinline__ void sts_u64(u32 a, u32 x, u32 y) { asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
-__device__ __forceinline__ void sts_u128(u32 a, u32 x, u32 y, u32 z, u32 w) { asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory"); }
-
-// ---- byte-SWAR pieces written for the pipes of the SM: logic ops (LOP3 / PRMT / SHF) run on the ALU pipe, whose rate is half
-// the issue rate, so shifts that can be merged with an add are written as multiply-adds (FMA pipe)
-template <u32 K> __device__ __forceinline__ u32 mad_k(u32 a, u32 c) {
-  u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "n"(K), "r"(c)); return d;
-}
-__device__ __forceinline__ u32 mad(u32 a, u32 b, u32 c) { u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
-// the bits of a where the mask has ones, those of b elsewhere (one instruction; the compiler needs two for the and/and/or form)
-__device__ __forceinline__ u32 bit_select(u32 a, u32 b, u32 mask) { u32 d; asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(a), "r"(b), "r"(mask)); return d; }
-__device__ __forceinline__ void bf16x4_dev(u32 sm4, u32 e4, u32& p01, u32& p23) {
-  const u32 eh = __umulhi(e4, 0x80000000u);                          // e4 >> 1
-  const u32 el = mad_k<128u>(e4, 0u);                                // e4 << 7
-  const u32 h4 = bit_select(sm4, eh, 0x80808080u), l4 = bit_select(el, sm4, 0x80808080u);
-  p01 = prmt(l4, h4, 0x5140); p23 = prmt(l4, h4, 0x7362);
-}
-// four 5-bit fields at bits 0..19 of u -> field << 3 per byte (raw-tier exponent high bits); same result as spread_hi5
-__device__ __forceinline__ u32 spread_hi5_dev(u32 u) {
-  const u32 y = mad_k<64u>(u & 0xFFC00u, u & 0x3FFu);               // fields 0,1 at bits 0-9, fields 2,3 at bits 16-25
-  return mad_k<64u>(y & 0x03E003E0u, (y & 0x001F001Fu) << 3);       // odd fields up 3 more bits, everything << 3
-}
-// Escape bytes of up to four groups whose tags are t (upper bits clear): one for a promoted group (tag 01), five for a raw one (11), which
-// is one bit per tag bit and three more copies of every upper bit.
-__device__ __forceinline__ u32 seg_esc(u32 t) { return (u32)popc((t & 0xAAu) * 0x01010100u + t); }
-
-// The 24 code bits of a group, picked out of two neighbouring words by one byte permute that already puts codes 4..7 at the top:
-// bits 0..11 = codes 0..3, bits 20..31 = codes 4..7 (B = byte offset of the group in the lane's code string).
-template <int B> __device__ __forceinline__ u32 group_codes(const u32* cd) {
-  constexpr int i = B & 3;
-  constexpr u32 sel = (u32)i | (u32)(i + 1) << 4 | (u32)(i + 1) << 8 | (u32)(i + 2) << 12;
-  return prmt(cd[B >> 2], i >= 2 ? cd[(B >> 2) + 1] : 0u, sel);
-}
-
-// Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, pos =
-// position of the group's escape bytes, advanced past them.
-// WIN: the escape bytes are staged; pos counts from the zero byte (a group without an escape byte reads that), and raw groups were turned
-//   into patch-table entries by build_raw_patches, which also left each entry's number in the first payload byte of its group: the addends
-//   of EVERY group come from one load, out of the escape-byte table (byte = the 4-bit-window escape byte, or the zero byte) or out of the
-//   patch table (byte = entry number), chosen by address arithmetic, and the decoder has no branch (a branch per group cost 13 % of the
-//   kernel although 0.75 % of the groups took it).
-// !WIN (tiles whose escape bytes are not all staged, or with more raw groups than the patch table holds): plain loads at glob[pos].
-template <bool WIN>
-__device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& pos, const uint8_t* glob, const WarpView& w, const u32x4& bw, u32 out[4]) {
-  const u32 m1 = tg & 1u;                             // promoted (tags are 0, 1 or 3)
-  const u32 blo = mad(m1, bw.z, bw.x), bhi = mad(m1, bw.w, bw.y);
-  u32 x0, x1;
-  if (WIN) {
-    const u32 r2 = tg & 2u;                           // 2 for a raw group: its table is the patch table
-    const u32 xe = lds_u8(mad(m1, pos, w.zero));
-    const u32x2 x = lds_u64(mad_k<8u>(xe, mad(r2, (w.scratch - w.lutx) >> 1, w.lutx)));
-    x0 = x.x; x1 = x.y;
-    pos = mad_k<2u>(r2, pos);                         // a raw payload is five bytes: four here, one below with every promoted group
-  } else {
-    const u32x2 x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
-    x0 = x.x; x1 = x.y;
-    if (tg & 2u) {                                    // raw exponents: e = code | hi5 << 3 (the base must not contribute)
-      const uint8_t* p = glob + pos;
-      const int sh = 8 * (int)(reinterpret_cast<uintptr_t>(p) & 3);
-      const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-      const u32 w0 = a[0], w1 = a[1];
-      const u32 lo = funnel_r(w0, w1, sh), hi = w1 >> sh;              // bytes 0-3 and byte 4 of the payload
-      x0 = spread_hi5_dev(lo & 0xFFFFFu) - blo;
-      x1 = spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - bhi;
-      pos += 4;
-    }
-  }
-  pos += m1;
-  // four 3-bit codes -> four bytes in two steps; each step moves the upper fields with a multiply-add: (t & M) * (2^k - 1) + t
-  const u32 th = z >> 20;
-  const u32 xl = mad_k<1023u>(z & 0xFC0u, z & 0xFFFu), xh = mad_k<1023u>(th & 0xFC0u, th);
-  bf16x4_dev(sm_lo, mad_k<31u>(xl & 0x00380038u, xl) + blo + x0, out[0], out[1]);
-  bf16x4_dev(sm_hi, mad_k<31u>(xh & 0x00380038u, xh) + bhi + x1, out[2], out[3]);
-}
-
 // ---- where a lane's escape bytes are.  A lane owns 8 groups of a K tile (tokens r and r + 8, groups 4j .. 4j + 3 of each) and 8 of a V tile
 // (groups 2r, 2r + 1 of tokens 2j, 2j + 1, 2j + 8, 2j + 9).
 //   tags  2 bits per group: K segments (8 bits) at bits 0 and 8, V segments (4 bits) at bits 16, 20, 24, 28
@@ -297,9 +206,6 @@ __device__ __forceinline__ bool build_raw_patches(u32 raw_bits, const TilePlan& 
   return true;
 }
 
-// K: the lanes of an octet are in the order of the tile's escape bytes, so ONE warp scan over both octets' segment sizes (packed in a word) gives
-// every lane its two positions.  V: a scan over the lanes of equal j (one byte per token: a row has at most 80 escape bytes) places a lane
-// inside its four rows, then a scan over j (two 16-bit sums: tokens 0..7 and 8..15) places the rows inside the tile.
 __device__ __forceinline__ TilePlan plan_tile(const SideView& ks, const SideView& vs, bool rawk, bool rawv, const WarpView& w, int lane) {
   const int j = lane & 3, r = lane >> 2;
   TilePlan t;
@@ -309,21 +215,8 @@ __device__ __forceinline__ TilePlan plan_tile(const SideView& ks, const SideView
     const uint2 a = *reinterpret_cast<const uint2*>(vs.fl + 8 * j), b = *reinterpret_cast<const uint2*>(vs.fl + 32 + 8 * j);      // tag words of the four tokens
     v0 = (a.x >> (4 * r)) & 15u; v1 = (a.y >> (4 * r)) & 15u; v2 = (b.x >> (4 * r)) & 15u; v3 = (b.y >> (4 * r)) & 15u;
   }
-  const u32 kown = mad_k<65536u>(seg_esc(k1), seg_esc(k0));
-  const u32 vown = mad_k<16777216u>(seg_esc(v3), mad_k<65536u>(seg_esc(v2), mad_k<256u>(seg_esc(v1), seg_esc(v0))));
-  u32 kinc = kown, vinc = vown;
-  scan_step(kinc, 1); scan_step(kinc, 2);
-  scan_step(kinc, 4); scan_step(vinc, 4); scan_step(kinc, 8); scan_step(vinc, 8); scan_step(kinc, 16); scan_step(vinc, 16);
-  const u32 ktot = __shfl_sync(FULLM, kinc, 31), rows = __shfl_sync(FULLM, vinc, 28 + j), before = vinc - vown;      // row totals; this lane's share starts `before` into its rows
-  t.k = kinc - kown + (ktot << 16);                                                          // the second octet's escape bytes follow the first's
-  const u32 sum = (rows & 0x00FF00FFu) + ((rows >> 8) & 0x00FF00FFu);                       // tokens 2j, 2j + 1 | tokens 2j + 8, 2j + 9
-  u32 js = sum;
-  { const u32 v = __shfl_up_sync(FULLM, js, 1, 4); if (j >= 1) js += v; }
-  { const u32 v = __shfl_up_sync(FULLM, js, 2, 4); if (j >= 2) js += v; }
-  const u32 vtot = __shfl_sync(FULLM, js, 3, 4), jb = js - sum + (vtot << 16);              // where rows 2j and 2j + 8 start
-  const u32 even = prmt(jb, 0u, 0x1010) + prmt(before, 0u, 0x4140) + ((rows & 0xFFu) << 16);
-  const u32 odd = prmt(jb, 0u, 0x3232) + prmt(before, 0u, 0x4342) + (rows & 0x00FF0000u);
-  t.v[0] = even; t.v[1] = odd;
+  u32 ktot, vtot;
+  tile_positions<true, true>(k0, k1, v0, v1, v2, v3, j, t.k, ktot, t.v, vtot);
   t.tags = mad_k<256u>(k1, k0) + mad_k<65536u>(v0, mad_k<1048576u>(v1, mad_k<16777216u>(v2, mad_k<268435456u>(v3, 0u))));
   const int total_k = (int)((ktot & 0xFFFFu) + (ktot >> 16)), total_v = (int)((vtot & 0xFFFFu) + (vtot >> 16));
   t.win = (total_k <= ks.avail ? 1 : 0) | (total_v <= vs.avail ? 2 : 0);
@@ -466,18 +359,6 @@ __device__ __forceinline__ void raw_accum(WarpAcc<NSET>& A, const uint16_t* vraw
     }
     pv_words<NSET>(A, mt, w0, w1, P);
   }
-}
-
-// ---- base words of a side, {b3lo, b3hi, b4lo - b3lo, b4hi - b3hi} per group (16 bytes; K: lane class jj, group gg at 64 * jj + 16 * gg; V: lane class rr,
-// group gg at 32 * rr + 16 * gg).  Thread t < 32 makes word t of the 32 half groups: eight byte loads that do not wait for one another.
-template <bool VSIDE>
-__device__ __forceinline__ void fill_bases(uint8_t* bases, const uint8_t* b3, const uint8_t* b4, int t) {
-  int d0, d1, d2, d3;                                // channels of the half group (see k_base_words, v_base_words)
-  if (VSIDE) { d0 = 32 * (t & 3) + (t >> 2); d1 = d0 + 8; d2 = d0 + 16; d3 = d0 + 24; }
-  else { d0 = 16 * (t & 7) + 2 * (t >> 3); d1 = d0 + 1; d2 = d0 + 8; d3 = d0 + 9; }
-  const u32 w3 = (u32)b3[d0] | (u32)b3[d1] << 8 | (u32)b3[d2] << 16 | (u32)b3[d3] << 24, w4 = (u32)b4[d0] | (u32)b4[d1] << 8 | (u32)b4[d2] << 16 | (u32)b4[d3] << 24;
-  u32* o = reinterpret_cast<u32*>(bases + (VSIDE ? BASES_V : 0) + 16 * (t >> 1)) + (t & 1);
-  o[0] = w3; o[2] = w4 - w3;
 }
 
 }  // namespace gaac

@@ -36,8 +36,7 @@ __device__ __forceinline__ int append_encode(WarpScratch& ws, const gaac_store& 
 template <int KIND_V>
 __device__ __forceinline__ void append_store(WarpScratch& ws, const gaac_store& st, const LaneTile& lt, long h, int tile, int total, long S_cap, long ovf_cap, int lane) {
   const long trow = h * S_cap + (long)tile * T;
-  store_tile_payload<KIND_V>(lt, st.sm + trow * D, st.codes + trow * CB, lane);
-  if (lane < T) st.flags[trow + lane] = (int)ws.fl[lane];
+  store_tile_payload<KIND_V>(lt, st.sm + trow * D, st.codes + trow * CB, reinterpret_cast<uint8_t*>(st.flags + trow), lane);
   const int used = st.ovf_used[h];
   store_tile_escapes<KIND_V>(ws, lt, st.ovf + h * ovf_cap + used, lane);
   __syncwarp();
@@ -122,8 +121,7 @@ __device__ __forceinline__ void store_one(WarpScratch& ws, const PagedParams& p,
     fits = total <= st.ovf_slot;
     if (fits) {
       uint8_t* base = st.buf + pt * st.TS;
-      store_tile_payload<KIND_V>(lt, base, base + SLOT_CD_OFF, lane);
-      if (lane < T) reinterpret_cast<u32*>(base + SLOT_FL_OFF)[lane] = ws.fl[lane];
+      store_tile_payload<KIND_V>(lt, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, lane);
       store_tile_escapes<KIND_V>(ws, lt, base + SLOT_OVF_OFF, lane);
     }
   }

@@ -41,8 +41,7 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(
     LaneTile lt;
     const int total = encode_tile_warp<KIND_V>(ws, nvalid, b3w, b4w, lane, lt);
     const long trow = h * S_pad + row0;
-    store_tile_payload<KIND_V>(lt, sm + trow * D, codes + trow * CB, lane);
-    if (lane < T) flags[trow + lane] = (int)ws.fl[lane];
+    store_tile_payload<KIND_V>(lt, sm + trow * D, codes + trow * CB, reinterpret_cast<uint8_t*>(flags + trow), lane);
     // escape bytes: gathered in shared memory with byte stores (every lane at its own positions), then written to the tile's
     // scratch slot as whole words by neighbouring lanes, so the slot costs one or two coalesced stores instead of ~50 byte stores
     store_tile_escapes<KIND_V>(ws, lt, esc_stage[warp], lane);

@@ -45,6 +45,14 @@ GAAC_HD u32 funnel_r(u32 lo, u32 hi, int sh) {          // (hi:lo) >> sh, 0 <= s
   return sh ? (u32)((((u64)hi << 32) | lo) >> sh) : lo;
 #endif
 }
+// the bits of a where the mask has ones, those of b elsewhere (one instruction; the compiler needs two for the and/and/or form)
+GAAC_HD u32 bits_of(u32 a, u32 b, u32 mask) {
+#if defined(__CUDA_ARCH__)
+  u32 d; asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(a), "r"(b), "r"(mask)); return d;
+#else
+  return (a & mask) | (b & ~mask);
+#endif
+}
 GAAC_HD int popc(u32 x) {
 #if defined(__CUDA_ARCH__)
   return __popc(x);
@@ -93,43 +101,49 @@ GAAC_HD u32 code_field12(const u32* c, int s) {
 }
 
 // ---- encode side -----------------------------------------------------------------------------------------------
+// low bytes (l4) and high bytes (h4) of four bf16 values -> sign/mantissa bytes and exponent bytes
+GAAC_HD void split_bytes4(u32 l4, u32 h4, u32& sm4, u32& e4) {
+  sm4 = bits_of(h4, l4, 0x80808080u);
+  e4 = bits_of(h4 * 2u, l4 >> 7, 0xFEFEFEFEu);
+}
 // two bf16 pairs (elements 0,1) (2,3) -> sign/mantissa bytes and exponent bytes
-GAAC_HD void split_bf16x4(u32 p01, u32 p23, u32& sm4, u32& e4) {
-  u32 l4 = prmt(p01, p23, 0x6420), h4 = prmt(p01, p23, 0x7531);
-  sm4 = (h4 & 0x80808080u) | (l4 & 0x7F7F7F7Fu);
-  e4 = ((h4 << 1) & 0xFEFEFEFEu) | ((l4 >> 7) & 0x01010101u);
-}
-// per-byte a - b (mod 256), no borrow across bytes
-GAAC_HD u32 sub_bytes(u32 a, u32 b) {
-  return ((a | 0x80808080u) - (b & 0x7F7F7F7Fu)) ^ ((a ^ ~b) & 0x80808080u);
-}
-// four codes (one per byte, < 8) -> 12 bits
-GAAC_HD u32 pack_codes4(u32 c4) { return (c4 & 7u) | ((c4 >> 5) & 0x38u) | ((c4 >> 10) & 0x1C0u) | ((c4 >> 15) & 0xE00u); }
-// bit 3 of each byte -> 4 bits
-GAAC_HD u32 pack_bit4(u32 d4) { return (((d4 >> 3) & 0x01010101u) * 0x10204080u) >> 28; }
+GAAC_HD void split_bf16x4(u32 p01, u32 p23, u32& sm4, u32& e4) { split_bytes4(prmt(p01, p23, 0x6420), prmt(p01, p23, 0x7531), sm4, e4); }
+// bit 3 of each byte of lo (bits 0-3 of the result) and of hi (bits 4-7): the fields are 8 bits apart, so one multiply brings them side by side
+GAAC_HD u32 pack_bit4x2(u32 lo, u32 hi) { return (((hi & 0x08080808u) * 16u + (lo & 0x08080808u)) * 0x00204081u) >> 24; }
 // (byte >> 3) of each byte -> 20 bits
 GAAC_HD u32 pack_hi5(u32 e4) {
   u32 f = (e4 >> 3) & 0x1F1F1F1Fu;
   return (f & 0x1Fu) | ((f >> 3) & 0x3E0u) | ((f >> 6) & 0x7C00u) | ((f >> 9) & 0xF8000u);
 }
+// the low three bits of every byte of lo (elements 0-3) and hi (4-7) -> 24 bits, element i at bit 3i; higher bits of the bytes are ignored
+GAAC_HD u32 pack_codes8(u32 lo, u32 hi) {
+  const u32 yl = bits_of(lo, lo >> 5, 0x00070007u), yh = bits_of(hi, hi >> 5, 0x00070007u);      // two codes at bits 0-5 of bytes 0 and 2
+  u32 v = prmt(yl, yh, 0x6420) & 0x3F3F3F3Fu;
+  v = bits_of(v, v >> 2, 0x003F003Fu) & 0x0FFF0FFFu;
+  return bits_of(v, v >> 4, 0x00000FFFu);
+}
 
 // Encode one group of 8 stored positions given its exponent bytes (elements 0-3 in e_lo, 4-7 in e_hi) and the bases.
-// Returns the tier tag (0, 1, 3); codes24 = 8 x 3-bit codes; esc = escape payload (1 byte for tier 1, 40 bits for tier 2).
+// Returns the tier tag (0, 1, 3); codes24 = 8 x 3-bit codes; esc1 = the escape byte of tier 1 (any value for the other tiers).
+// A window is tried with ONE 32-bit subtraction per half group: base tables leave room for their window (3-bit base <= 248, 4-bit base <=
+// 240), so "every byte of e - b is below the window" as a plain word difference means that no byte borrowed, which is the same as
+// "every exponent lies in its window".  Both windows are tried up front and everything is picked with selects: in a warp some lane
+// nearly always needs the 4-bit window.
+GAAC_HD u32 encode_group_codes(u32 e_lo, u32 e_hi, u32 b3_lo, u32 b3_hi, u32 b4_lo, u32 b4_hi, u32& codes24, u32& esc1) {
+  const u32 d3l = e_lo - b3_lo, d3h = e_hi - b3_hi, d4l = e_lo - b4_lo, d4h = e_hi - b4_hi;
+  const bool t0 = ((d3l | d3h) & 0xF8F8F8F8u) == 0, t1 = ((d4l | d4h) & 0xF0F0F0F0u) == 0;
+  codes24 = pack_codes8(t0 ? d3l : (t1 ? d4l : e_lo), t0 ? d3h : (t1 ? d4h : e_hi));
+  esc1 = pack_bit4x2(d4l, d4h);
+  return t0 ? 0u : (t1 ? 1u : 3u);
+}
+// Escape payload of a raw group: the upper five bits of its eight exponents, 40 bits.
+GAAC_HD u64 raw_payload(u32 e_lo, u32 e_hi) { return (u64)pack_hi5(e_lo) | ((u64)pack_hi5(e_hi) << 20); }
+// The same with the payload of whatever tier came out (0 / one byte / 40 bits).
 GAAC_HD u32 encode_group(u32 e_lo, u32 e_hi, u32 b3_lo, u32 b3_hi, u32 b4_lo, u32 b4_hi, u32& codes24, u64& esc) {
-  // Both windows are tried up front and the tier is picked with selects: in a warp some lane nearly always needs the 4-bit
-  // window, so a branch per tier would run both paths one after the other.  Only the raw tier (under 1 %) branches.
-  const u32 d3l = sub_bytes(e_lo, b3_lo), d3h = sub_bytes(e_hi, b3_hi);
-  const u32 d4l = sub_bytes(e_lo, b4_lo), d4h = sub_bytes(e_hi, b4_hi);
-  const bool t0 = ((d3l | d3h) & 0xF8F8F8F8u) == 0;
-  const bool t1 = ((d4l | d4h) & 0xF0F0F0F0u) == 0;
-  if (t0 | t1) {
-    const u32 cl = t0 ? d3l : (d4l & 0x07070707u), ch = t0 ? d3h : (d4h & 0x07070707u);
-    codes24 = pack_codes4(cl) | (pack_codes4(ch) << 12);
-    esc = t0 ? 0u : (pack_bit4(d4l) | (pack_bit4(d4h) << 4));
-    return t0 ? 0u : 1u;
-  }
-  codes24 = pack_codes4(e_lo & 0x07070707u) | (pack_codes4(e_hi & 0x07070707u) << 12);
-  esc = (u64)pack_hi5(e_lo) | ((u64)pack_hi5(e_hi) << 20); return 3u;
+  u32 esc1;
+  const u32 tag = encode_group_codes(e_lo, e_hi, b3_lo, b3_hi, b4_lo, b4_hi, codes24, esc1);
+  esc = tag == 0u ? 0u : (tag == 1u ? (u64)esc1 : raw_payload(e_lo, e_hi));
+  return tag;
 }
 
 // Rebuild the exponent bytes of one half group (4 stored positions).

@@ -2,7 +2,7 @@
 // One warp owns one 16-token tile.  Shared by the page encoder, the slot-cache append and the paged store kernels.
 #pragma once
 #include <cuda_runtime.h>
-#include "gaac_tile.h"
+#include "gaac_lane.cuh"
 
 namespace gaac {
 
@@ -26,19 +26,17 @@ struct PtrEsc {
   }
 };
 
-// Encoded tile held in registers, one lane's share.  8 groups per lane for both kinds:
+// Encoded tile held in registers, one lane's share.  8 groups per lane for both kinds, in runs of consecutive groups of one row (segments):
 //   K: idx = 4*o + g  -> row 8o + (lane>>2), group 4*(lane&3) + g          V: idx = 2*t + g -> row tok(t), group 2*(lane>>2) + g
 struct LaneTile {
   u32 sm[16];        // K: [o][8] words;  V: [t][4] words
   u32 cd[6];         // K: [o][3] words;  V: 192 code bits (4 token slots x 48)
-  u64 esc[8];
+  u32 esc1[8];       // the escape byte of a tier 1 group
   u32 tags;          // 2 bits per idx
+  u32 pos[2];        // where the segments' escape bytes begin inside the tile: K: pos[0] = {octet 0, octet 1};  V: pos[t >> 1] = {t & ~1, t | 1} (16 bits each)
 };
 
 __device__ __forceinline__ int v_tok(int j, int t) { return 2 * j + (t & 1) + 8 * (t >> 1); }
-__device__ __forceinline__ int lane_row(int kind_v, int lane, int idx) { return kind_v ? v_tok(lane & 3, idx >> 1) : 8 * (idx >> 2) + (lane >> 2); }
-__device__ __forceinline__ int lane_group(int kind_v, int lane, int idx) { return kind_v ? 2 * (lane >> 2) + (idx & 1) : 4 * (lane & 3) + (idx & 3); }
-
 // Stage rows [row0, row0+16) of a [*, 128] bf16 matrix into ws.xs; rows >= nvalid are zero-filled.
 __device__ __forceinline__ void stage_rows(WarpScratch& ws, const uint16_t* src, long row_stride, int nvalid, int lane) {
 #pragma unroll
@@ -74,118 +72,164 @@ __device__ __forceinline__ void stage_rows_async(WarpScratch& ws, const uint16_t
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Encode the staged tile.  Rows >= nvalid become empty rows (sm = 0, codes = 0, tag word 0).  On return every lane holds
-// its share in `lt`, ws.fl / ws.rowoff are filled and the tile's escape byte count is returned (same in all lanes).
+// Four 8 x 8 matrices of 16-bit values out of the staged tile: channels 16s .. 16s + 7 and 16s + 8 .. 16s + 15 of tokens 0..7 (w[0], w[1]) and of
+// tokens 8..15 (w[2], w[3]).  `at`: the lane's row address, &xs[(8 * (lane >> 4) + (lane & 7)) * XS_STRIDE + 8 * ((lane >> 3) & 1)].  Rows are 68
+// words apart, so the eight rows of a matrix lie in different banks.
+//   plain:      lane (j, r) gets channels 2j, 2j + 1 of token r, which is how a lane owns a K tile
+//   transposed: lane (j, r) gets channel r of tokens 2j, 2j + 1, which is how it owns a V tile
+template <bool TRANS> __device__ __forceinline__ void load_matrices(u32 (&w)[4], u32 at, int s) {
+  if (!TRANS) asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(at + 32 * s) : "memory");
+  else asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(at + 32 * s) : "memory");
+}
+__device__ __forceinline__ u32 matrix_row_address(const WarpScratch& ws, int lane) {
+  return (u32)__cvta_generic_to_shared(&ws.xs[(8 * (lane >> 4) + (lane & 7)) * XS_STRIDE + 8 * ((lane >> 3) & 1)]);
+}
+// Four groups of 24 code bits (bits 24..31 ignored) -> 96 bits
+__device__ __forceinline__ void join_codes(u32 c0, u32 c1, u32 c2, u32 c3, u32* cd) {
+  cd[0] = prmt(c0, c1, 0x4210); cd[1] = prmt(c1, c2, 0x5421); cd[2] = prmt(c2, c3, 0x6542);
+}
+
+// Encode the staged tile.  Rows >= nvalid become empty rows (sm = 0, codes = 0, tag word 0); they must have been staged as zeros.  On return
+// every lane holds its share in `lt` and the tile's escape byte count is returned (same in all lanes).
+// Bound by instruction issue: 16-bit loads one by one, a byte-exact subtraction per window, a table of tags in shared memory and a branch per
+// escape byte made 1205 warp instructions per tile; now the fragments come in by ldmatrix, a window is one subtraction per word and the
+// positions of the escape bytes come from one warp scan.
 template <int KIND_V>
 __device__ __forceinline__ int encode_tile_warp(WarpScratch& ws, int nvalid, const u32* b3w, const u32* b4w, int lane, LaneTile& lt) {
   const int j = lane & 3, r = lane >> 2;
+  const u32 at = matrix_row_address(ws, lane);
   lt.tags = 0;
-  __syncwarp();                                      // staged rows visible; previous tile's scratch no longer in use
-  if (!KIND_V) {
+  __syncwarp();                                      // staged rows visible
+  u32 c24[8];
 #pragma unroll
-    for (int o = 0; o < 2; o++) {
-      int row = 8 * o + r; u32 t8 = 0;
-      if (row < nvalid) encode_k_lane(&ws.xs[row * XS_STRIDE], j, b3w, b4w, &lt.sm[8 * o], &lt.cd[3 * o], t8, &lt.esc[4 * o]);
-      else {
+  for (int g = 0; g < (KIND_V ? 2 : 4); g++) {
+    if (!KIND_V) {
+      u32 e[2][2];                                   // [octet][half group]
 #pragma unroll
-        for (int i = 0; i < 8; i++) lt.sm[8 * o + i] = 0;
-        lt.cd[3 * o] = lt.cd[3 * o + 1] = lt.cd[3 * o + 2] = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) lt.esc[4 * o + i] = 0;
+      for (int h = 0; h < 2; h++) {
+        u32 w[4];
+        load_matrices<false>(w, at, 2 * g + h);
+        split_bf16x4(w[0], w[1], lt.sm[2 * g + h], e[0][h]);
+        split_bf16x4(w[2], w[3], lt.sm[8 + 2 * g + h], e[1][h]);
       }
-      lt.tags |= t8 << (8 * o);
-    }
-  } else {
-    u64 c48[4];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      int row = v_tok(j, t); u32 t4 = 0; c48[t] = 0;
-      if (row < nvalid) encode_v_lane(&ws.xs[row * XS_STRIDE], r, b3w, b4w, &lt.sm[4 * t], c48[t], t4, &lt.esc[2 * t]);
-      else {
+      for (int o = 0; o < 2; o++)
+        lt.tags |= encode_group_codes(e[o][0], e[o][1], b3w[2 * g], b3w[2 * g + 1], b4w[2 * g], b4w[2 * g + 1], c24[4 * o + g], lt.esc1[4 * o + g]) << (8 * o + 2 * g);
+    } else {
+      u32 e[4][2];                                   // [token slot][half group]
 #pragma unroll
-        for (int i = 0; i < 4; i++) lt.sm[4 * t + i] = 0;
-        lt.esc[2 * t] = lt.esc[2 * t + 1] = 0;
+      for (int h = 0; h < 2; h++) {
+        const int i = 2 * g + h;                     // channels 32i .. 32i + 31: four matrices of each token half
+        u32 a[4], b[4];
+        load_matrices<true>(a, at, 2 * i); load_matrices<true>(b, at, 2 * i + 1);
+#pragma unroll
+        for (int th = 0; th < 2; th++) {             // tokens 2j, 2j + 1 (+ 8): a byte transpose sorts the pairs by token and by low / high byte
+          const u32 x0 = a[2 * th], x1 = a[2 * th + 1], x2 = b[2 * th], x3 = b[2 * th + 1];
+          const u32 p = prmt(x0, x1, 0x5140), q = prmt(x2, x3, 0x5140), p2 = prmt(x0, x1, 0x7362), q2 = prmt(x2, x3, 0x7362);
+          split_bytes4(prmt(p, q, 0x5410), prmt(p, q, 0x7632), lt.sm[8 * th + i], e[2 * th][h]);
+          split_bytes4(prmt(p2, q2, 0x5410), prmt(p2, q2, 0x7632), lt.sm[8 * th + 4 + i], e[2 * th + 1][h]);
+        }
       }
-      lt.tags |= t4 << (4 * t);
+#pragma unroll
+      for (int t = 0; t < 4; t++)
+        lt.tags |= encode_group_codes(e[t][0], e[t][1], b3w[2 * g], b3w[2 * g + 1], b4w[2 * g], b4w[2 * g + 1], c24[2 * t + g], lt.esc1[2 * t + g]) << (4 * t + 2 * g);
     }
-    lt.cd[0] = (u32)c48[0];
-    lt.cd[1] = (u32)(c48[0] >> 32) | ((u32)c48[1] << 16);
-    lt.cd[2] = (u32)(c48[1] >> 16);
-    lt.cd[3] = (u32)c48[2];
-    lt.cd[4] = (u32)(c48[2] >> 32) | ((u32)c48[3] << 16);
-    lt.cd[5] = (u32)(c48[3] >> 16);
   }
-  __syncwarp();                                      // xs fully read before the scratch tables are reused by a later tile
+  if (nvalid < T) {                                  // empty rows: zeros as values, which the windows above may have coded as anything
 #pragma unroll
-  for (int idx = 0; idx < 8; idx++) ws.tag[lane_row(KIND_V, lane, idx)][lane_group(KIND_V, lane, idx)] = (uint8_t)((lt.tags >> (2 * idx)) & 3u);
-  __syncwarp();
-  int total;
-  {
-    u32 fl = 0; int sz = 0;
-    if (lane < T) {
-      const u32* tw = reinterpret_cast<const u32*>(ws.tag[lane]);
+    for (int t = 0; t < (KIND_V ? 4 : 2); t++) {
+      if ((KIND_V ? v_tok(j, t) : 8 * t + r) >= nvalid) {
+        lt.tags &= KIND_V ? ~(0xFu << (4 * t)) : ~(0xFFu << (8 * t));
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        u32 w = tw[q];                               // four tags, one per byte
-        fl |= ((w & 3u) | ((w >> 6) & 0xCu) | ((w >> 12) & 0x30u) | ((w >> 18) & 0xC0u)) << (8 * q);
+        for (int i = 0; i < (KIND_V ? 2 : 4); i++) c24[(KIND_V ? 2 : 4) * t + i] = 0u;
       }
-      sz = row_esc_bytes(fl);
     }
-    int inc = sz;
-#pragma unroll
-    for (int d = 1; d < T; d <<= 1) { int v = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += v; }
-    if (lane < T) { ws.fl[lane] = fl; ws.rowoff[lane] = inc - sz; }
-    total = __shfl_sync(FULL, inc, T - 1);
   }
-  __syncwarp();
-  return total;
+  join_codes(c24[0], c24[1], c24[2], c24[3], lt.cd);
+  join_codes(c24[4], c24[5], c24[6], c24[7], lt.cd + 3);
+  u32 total, none;
+  if (!KIND_V) tile_positions<true, false>(lt.tags & 0xFFu, lt.tags >> 8, 0u, 0u, 0u, 0u, j, lt.pos[0], total, lt.pos, none);
+  else tile_positions<false, true>(0u, 0u, lt.tags & 15u, (lt.tags >> 4) & 15u, (lt.tags >> 8) & 15u, lt.tags >> 12, j, none, none, lt.pos, total);
+  return (int)((total & 0xFFFFu) + (total >> 16));
 }
 
-// Write one lane's sign/mantissa and code bytes of the tile (tile-relative destinations).
+// 32 bytes in one store (the address is a multiple of 32)
+__device__ __forceinline__ void store_32(void* p, const u32* w) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+}
+// Write one lane's sign/mantissa bytes, code bytes and tags of the tile (tile-relative destinations in global memory; fl_dst: 16 tag words).
+// A lane's sign/mantissa bytes are 32 (K) or 64 (V) contiguous ones: whole sectors where the destination is 32-byte aligned, which only a
+// paged slot whose stride is an odd multiple of 16 is not.
 template <int KIND_V>
-__device__ __forceinline__ void store_tile_payload(const LaneTile& lt, uint8_t* sm_dst, uint8_t* cd_dst, int lane) {
+__device__ __forceinline__ void store_tile_payload(const LaneTile& lt, uint8_t* sm_dst, uint8_t* cd_dst, uint8_t* fl_dst, int lane) {
+  constexpr int STEP = KIND_V ? 32 : 1024;
+  uint8_t* s0 = sm_dst + (KIND_V ? 64 : 32) * lane;
+  if ((reinterpret_cast<uintptr_t>(sm_dst) & 31) == 0) { store_32(s0, lt.sm); store_32(s0 + STEP, lt.sm + 8); }
+  else {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint4* s = reinterpret_cast<uint4*>(s0 + h * STEP);
+      s[0] = make_uint4(lt.sm[8 * h], lt.sm[8 * h + 1], lt.sm[8 * h + 2], lt.sm[8 * h + 3]);
+      s[1] = make_uint4(lt.sm[8 * h + 4], lt.sm[8 * h + 5], lt.sm[8 * h + 6], lt.sm[8 * h + 7]);
+    }
+  }
   if (!KIND_V) {
 #pragma unroll
     for (int o = 0; o < 2; o++) {
-      uint4* s = reinterpret_cast<uint4*>(sm_dst + o * 1024 + 32 * lane);
-      s[0] = make_uint4(lt.sm[8 * o], lt.sm[8 * o + 1], lt.sm[8 * o + 2], lt.sm[8 * o + 3]);
-      s[1] = make_uint4(lt.sm[8 * o + 4], lt.sm[8 * o + 5], lt.sm[8 * o + 6], lt.sm[8 * o + 7]);
       u32* c = reinterpret_cast<u32*>(cd_dst + o * 384 + 12 * lane);
       c[0] = lt.cd[3 * o]; c[1] = lt.cd[3 * o + 1]; c[2] = lt.cd[3 * o + 2];
     }
+    fl_dst[lane] = (uint8_t)lt.tags;                 // byte j of row r's tag word is byte `lane` of the octet's 32
+    fl_dst[32 + lane] = (uint8_t)(lt.tags >> 8);
   } else {
-#pragma unroll
-    for (int t = 0; t < 4; t++)
-      *reinterpret_cast<uint4*>(sm_dst + 64 * lane + 16 * t) = make_uint4(lt.sm[4 * t], lt.sm[4 * t + 1], lt.sm[4 * t + 2], lt.sm[4 * t + 3]);
     uint2* c = reinterpret_cast<uint2*>(cd_dst + 24 * lane);
     c[0] = make_uint2(lt.cd[0], lt.cd[1]); c[1] = make_uint2(lt.cd[2], lt.cd[3]); c[2] = make_uint2(lt.cd[4], lt.cd[5]);
+    // byte r >> 1 of a row's tag word: the even lane's two groups below the odd one's; the even lane writes tokens 2j, 2j + 1, the odd one the others
+    const int j = lane & 3, r = lane >> 2;
+    const u32 other = __shfl_xor_sync(FULLM, lt.tags, 4);
+    const u32 lo = (r & 1) ? other : lt.tags, hi = (r & 1) ? lt.tags : other;
+    const int sh = (r & 1) ? 8 : 0;
+    uint8_t* f = fl_dst + 4 * (2 * j + ((r & 1) ? 8 : 0)) + (r >> 1);
+    f[0] = (uint8_t)(((lo >> sh) & 15u) | (((hi >> sh) & 15u) << 4));
+    f[4] = (uint8_t)(((lo >> (sh + 4)) & 15u) | (((hi >> (sh + 4)) & 15u) << 4));
   }
 }
 
-// Write the tile's escape bytes at esc_dst + (tile-relative position), rows in token order, groups ascending.
+// Write the tile's escape bytes at esc_dst + (tile-relative position), rows in token order, groups ascending.  The tile is still staged in
+// ws.xs: a raw group's payload is made from there, in a loop that most lanes never enter (under 1 % of the groups are raw).
 template <int KIND_V>
 __device__ __forceinline__ void store_tile_escapes(const WarpScratch& ws, const LaneTile& lt, uint8_t* esc_dst, int lane) {
-  if (lt.tags == 0) return;
-  // A lane's groups come in runs of consecutive groups of one row (K: 2 rows x 4 groups, V: 4 rows x 2 groups): the position of a
-  // run's first escape byte is computed once, the groups of the run then follow one another in the row's escape bytes.
-  constexpr int RUN = KIND_V ? 2 : 4;
+  constexpr int RUN = KIND_V ? 2 : 4;                // groups of a segment
+  const int j = lane & 3, r = lane >> 2;
 #pragma unroll
-  for (int base = 0; base < 8; base += RUN) {
-    const u32 tr = (lt.tags >> (2 * base)) & ((1u << (2 * RUN)) - 1u);
-    if (tr) {
-      const int row = lane_row(KIND_V, lane, base), g0 = lane_group(KIND_V, lane, base);
-      uint8_t* d = esc_dst + ws.rowoff[row] + esc_prefix(ws.fl[row], 2 * g0);
+  for (int s = 0; s < 8 / RUN; s++) {
+    const u32 pw = KIND_V ? lt.pos[s >> 1] : lt.pos[0];
+    uint8_t* d = esc_dst + ((s & 1) ? pw >> 16 : pw & 0xFFFFu);
 #pragma unroll
-      for (int i = 0; i < RUN; i++) {
-        const u32 tag = (tr >> (2 * i)) & 3u;
-        if (tag) {
-          const u64 e = lt.esc[base + i];
-          d[0] = (uint8_t)e;
-          if (tag & 2u) { d[1] = (uint8_t)(e >> 8); d[2] = (uint8_t)(e >> 16); d[3] = (uint8_t)(e >> 24); d[4] = (uint8_t)(e >> 32); }
-          d += tag_esc_bytes(tag);
-        }
+    for (int i = 0; i < RUN; i++) {
+      const u32 tag = (lt.tags >> (2 * (s * RUN + i))) & 3u;
+      if (tag & 1u) *d = (uint8_t)lt.esc1[s * RUN + i];                                      // a raw group's first byte is set right below
+      d += tag_esc_bytes(tag);
+    }
+  }
+  for (u32 raw = lt.tags & 0xAAAAu; raw; raw &= raw - 1u) {
+    const int bit = __ffs((int)raw) - 1, idx = bit >> 1, s = idx / RUN, g = idx % RUN;
+    const u32 below = (lt.tags >> (2 * s * RUN)) & ((1u << (2 * g)) - 1u);
+    const u32 pw = KIND_V && (s & 2) ? lt.pos[1] : lt.pos[0];
+    uint8_t* d = esc_dst + ((s & 1) ? pw >> 16 : pw & 0xFFFFu) + seg_esc(below);
+    u32 sm, e[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      if (!KIND_V) {
+        const u32* p = reinterpret_cast<const u32*>(&ws.xs[(8 * s + r) * XS_STRIDE + 16 * (2 * g + h) + 2 * j]);
+        split_bf16x4(p[0], p[4], sm, e[h]);
+      } else {
+        const uint16_t* p = &ws.xs[v_tok(j, s) * XS_STRIDE + 32 * (2 * g + h) + r];
+        split_bf16x4((u32)p[0] | ((u32)p[8] << 16), (u32)p[16] | ((u32)p[24] << 16), sm, e[h]);
       }
     }
+    const u64 w = raw_payload(e[0], e[1]);
+    d[0] = (uint8_t)w; d[1] = (uint8_t)(w >> 8); d[2] = (uint8_t)(w >> 16); d[3] = (uint8_t)(w >> 24); d[4] = (uint8_t)(w >> 32);
   }
 }
 
