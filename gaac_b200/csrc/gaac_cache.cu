@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restric
   }
 }
 
-struct PagedDecodeParams { gaac_paged st; const int* pairs; uint16_t *sk, *sv; long row_stride; };
+struct PagedDecodeParams { gaac_paged st; const int* pairs; int P; uint16_t *sk, *sv; long row_stride; };
 
 template <int KIND_V>
-__device__ __forceinline__ void decode_block_one(WarpScratch& ws, const PagedDecodeParams& p, int e, int t, int lane) {
+__device__ __forceinline__ void decode_block_one(DecodeScratch& ws, const PagedDecodeParams& p, const WarpView& w, int e, int t, int lane) {
   const gaac_paged& st = p.st;
   const int kvh = t >> 1, NT = 2 * st.n_kv;
   const int blk = p.pairs[3 * e], row0 = p.pairs[3 * e + 1], nvalid = p.pairs[3 * e + 2];
@@ -180,17 +180,25 @@ __device__ __forceinline__ void decode_block_one(WarpScratch& ws, const PagedDec
     return;
   }
   const uint8_t* base = st.buf + pt * st.TS;
-  u32 b3w[8], dw[8];
-  load_base_deltas<KIND_V>((KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D, lane, b3w, dw);
-  PtrEsc esc{base + SLOT_OVF_OFF};
-  decode_tile_warp<KIND_V>(ws, base, base + SLOT_CD_OFF, reinterpret_cast<const u32*>(base + SLOT_FL_OFF), esc, b3w, dw, lane);
+  decode_tile_warp<KIND_V>(ws, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, base + SLOT_OVF_OFF, w, lane);
   unstage_rows(ws, dst, p.row_stride, nvalid, lane);
 }
 
-__global__ void __launch_bounds__(32) paged_decode_blocks_kernel(const __grid_constant__ PagedDecodeParams p) {
-  __shared__ __align__(16) WarpScratch ws;
-  const int e = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
-  if (t & 1) decode_block_one<1>(ws, p, e, t, lane); else decode_block_one<0>(ws, p, e, t, lane);
+// One warp per (entry, tile slot); the CTA's four entries have the slot index t = 2*kvh + kind in common, and with it the tables.
+// grid = (ceil(P / 4), 2*n_kv).
+constexpr int PDEC_WARPS = 4;
+template <int KIND_V>
+__device__ __forceinline__ void decode_blocks_cta(DecodeScratch* scratch, DecodeTables& tables, const PagedDecodeParams& p, int t) {
+  const int kvh = t >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x * PDEC_WARPS + warp;
+  const WarpView w = fill_decode_tables<KIND_V>(tables, (KIND_V ? p.st.b3v : p.st.b3k) + kvh * D, (KIND_V ? p.st.b4v : p.st.b4k) + kvh * D);
+  __syncthreads();
+  if (e < p.P) decode_block_one<KIND_V>(scratch[warp], p, w, e, t, lane);
+}
+__global__ void __launch_bounds__(PDEC_WARPS * 32) paged_decode_blocks_kernel(const __grid_constant__ PagedDecodeParams p) {
+  __shared__ __align__(16) DecodeScratch scratch[PDEC_WARPS];
+  __shared__ __align__(16) DecodeTables tables;
+  const int t = blockIdx.y;
+  if (t & 1) decode_blocks_cta<1>(scratch, tables, p, t); else decode_blocks_cta<0>(scratch, tables, p, t);
 }
 
 static int check_paged(const gaac_paged* st) {
@@ -246,8 +254,8 @@ extern "C" int gaac_paged_decode_blocks(const gaac_paged* st, const int32_t* pai
   if (!pairs || !sk || !sv || P < 0 || row_stride < (int64_t)st->n_kv * D) return GAAC_E_ARG;
   if (!aligned16(sk) || !aligned16(sv) || row_stride % 8) return GAAC_E_ALIGN;
   if (P == 0) return GAAC_OK;
-  PagedDecodeParams p{*st, pairs, (uint16_t*)sk, (uint16_t*)sv, row_stride};
-  paged_decode_blocks_kernel<<<dim3((unsigned)P, (unsigned)(2 * st->n_kv)), 32, 0, (cudaStream_t)stream>>>(p);
+  PagedDecodeParams p{*st, pairs, P, (uint16_t*)sk, (uint16_t*)sv, row_stride};
+  paged_decode_blocks_kernel<<<dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)), PDEC_WARPS * 32, 0, (cudaStream_t)stream>>>(p);
   return launch_status();
 }
 

@@ -165,21 +165,21 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) decode_page_kernel(
     const uint8_t* __restrict__ sm, const uint8_t* __restrict__ codes, const int* __restrict__ flags, const int* __restrict__ tile_off,
     long tile_off_stride, const uint8_t* __restrict__ ovf, const int* __restrict__ head_start, const uint8_t* __restrict__ base3,
     const uint8_t* __restrict__ base4, const int* __restrict__ bidx, int n_kv, long S, long S_pad, uint16_t* __restrict__ out, int ntiles) {
-  __shared__ __align__(16) WarpScratch scratch[ENC_WARPS];
+  __shared__ __align__(16) DecodeScratch scratch[ENC_WARPS];
+  __shared__ __align__(16) DecodeTables tables;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long h = blockIdx.y;
-  WarpScratch& ws = scratch[warp];
+  DecodeScratch& ws = scratch[warp];
   const int brow = bidx ? bidx[h] : (int)(h % n_kv);
-  u32 b3w[8], b4w[8];
-  load_base_deltas<KIND_V>(base3 + (long)brow * D, base4 + (long)brow * D, lane, b3w, b4w);
+  const WarpView w = fill_decode_tables<KIND_V>(tables, base3 + (long)brow * D, base4 + (long)brow * D);
+  const uint8_t* esc_head = ovf + (long)head_start[h];
+  __syncthreads();
   const int tile0 = blockIdx.x * (ENC_WARPS * ENC_TILES_PER_WARP);
   for (int i = 0; i < ENC_TILES_PER_WARP; i++) {
     const int tile = tile0 + i * ENC_WARPS + warp;
     if (tile >= ntiles) break;
     const long row0 = (long)tile * T, trow = h * S_pad + row0;
-    PtrEsc esc{ovf + (long)head_start[h] + tile_off[h * tile_off_stride + tile]};
-    __syncwarp();
-    decode_tile_warp<KIND_V>(ws, sm + trow * D, codes + trow * CB, reinterpret_cast<const u32*>(flags + trow), esc, b3w, b4w, lane);
+    decode_tile_warp<KIND_V>(ws, sm + trow * D, codes + trow * CB, reinterpret_cast<const uint8_t*>(flags + trow), esc_head + tile_off[h * tile_off_stride + tile], w, lane);
     unstage_rows(ws, out + (h * S + row0) * D, D, (int)min((long)T, S - row0), lane);
   }
 }

@@ -9,21 +9,19 @@ namespace gaac {
 constexpr int XS_STRIDE = 136;                      // u16 per staged row: 272 B keeps 16-byte alignment and spreads banks
 constexpr unsigned FULL = 0xffffffffu;
 
+constexpr int ESC_STAGE = 256;                      // escape bytes of a tile that the decoder stages; longer tiles read theirs where they are
+
 // Per-warp scratch in shared memory.
 struct WarpScratch {
   uint16_t xs[T * XS_STRIDE];                        // staged tile, natural channel order
-  uint8_t tag[T][16];                                // tier tag per (row, group)
-  u32 fl[T];                                         // tag word per row
-  int rowoff[T];                                     // escape offset of each row inside the tile
 };
-
-// Escape byte reader over plain memory (global or shared).
-struct PtrEsc {
-  const uint8_t* p;
-  __host__ __device__ u32 byte(int pos) const { return p[pos]; }
-  __host__ __device__ u64 bytes5(int pos) const {
-    return (u64)p[pos] | ((u64)p[pos + 1] << 8) | ((u64)p[pos + 2] << 16) | ((u64)p[pos + 3] << 24) | ((u64)p[pos + 4] << 32);
-  }
+struct DecodeScratch : WarpScratch {
+  u32 esc[ESC_STAGE / 4 + 4];                        // the tile's escape bytes, from the 4-byte boundary at or below the first; the raw decoder may read one word behind them
+};
+// What the warps of a CTA that decodes tiles of one (kind, head) share: the escape-byte table and the base words.
+struct DecodeTables {
+  u32x2 lutx[256];
+  uint8_t bases[BASES_BYTES];
 };
 
 // Encoded tile held in registers, one lane's share.  8 groups per lane for both kinds, in runs of consecutive groups of one row (segments):
@@ -239,75 +237,94 @@ __device__ __forceinline__ void load_base_words(const uint8_t* b3row, const uint
   if (!KIND_V) { k_base_words(b3row, lane & 3, b3w); k_base_words(b4row, lane & 3, b4w); }
   else { v_base_words(b3row, lane >> 2, b3w); v_base_words(b4row, lane >> 2, b4w); }
 }
-// Same, but the second table is returned as the difference (4-bit base word - 3-bit base word) that decode_group wants.
+// Fill the tables of a decoding CTA (any number of threads); the caller synchronises.
 template <int KIND_V>
-__device__ __forceinline__ void load_base_deltas(const uint8_t* b3row, const uint8_t* b4row, int lane, u32* b3w, u32* dw) {
-  load_base_words<KIND_V>(b3row, b4row, lane, b3w, dw);
-#pragma unroll
-  for (int i = 0; i < (KIND_V ? 4 : 8); i++) dw[i] -= b3w[i];
+__device__ __forceinline__ WarpView fill_decode_tables(DecodeTables& t, const uint8_t* b3row, const uint8_t* b4row) {
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) fill_lutx(t.lutx, i);
+  if (threadIdx.x < 32) fill_bases<KIND_V != 0>(t.bases, b3row, b4row, threadIdx.x);
+  return WarpView{(u32)__cvta_generic_to_shared(t.lutx), (u32)__cvta_generic_to_shared(t.bases), 0u, 0u};
+}
+template <bool TRANS> __device__ __forceinline__ void store_matrices(u32 at, int s, u32 w0, u32 w1, u32 w2, u32 w3) {       // the opposite of load_matrices
+  if (!TRANS) asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(at + 32 * s), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+  else asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(at + 32 * s), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+}
+// 32 bytes in one load (the address is a multiple of 32)
+__device__ __forceinline__ void load_32(u32* w, const void* p) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
 }
 
-// Rebuild a compressed tile into ws.xs (natural channel order, bf16 bits).  sm/cd/fl: tile-relative sources;
-// esc: reader positioned at the tile's first escape byte.
-template <int KIND_V, class Esc>
-__device__ __forceinline__ void decode_tile_warp(WarpScratch& ws, const uint8_t* sm_src, const uint8_t* cd_src, const u32* fl_src,
-                                                 const Esc& esc, const u32* b3w, const u32* dw, int lane) {
+// Rebuild a compressed tile into ws.xs (natural channel order, bf16 bits).  sm / cd / fl: tile-relative sources in global memory; esc: the tile's first
+// escape byte in global memory.  Everything but the escape bytes is asked for at once; those are fetched with one coalesced load as soon as the tags
+// say how many there are (a load per group waited for the one before it at every raw group's branch).  The group decoder is the attention
+// kernels'; the fragments go to shared memory by stmatrix.
+template <int KIND_V>
+__device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, const uint8_t* sm_src, const uint8_t* cd_src, const uint8_t* fl_src, const uint8_t* esc_src,
+                                                 const WarpView& w, int lane) {
   const int j = lane & 3, r = lane >> 2;
-  {
-    u32 fl = lane < T ? fl_src[lane] : 0u; int sz = row_esc_bytes(fl), inc = sz;
+  constexpr int STEP = KIND_V ? 32 : 1024, SEGS = KIND_V ? 4 : 2;
+  u32 sm[16], cd[6], tags, total, none, pos[SEGS];
+  const uint8_t* s0 = sm_src + (KIND_V ? 64 : 32) * lane;
+  u32 fl[SEGS];
+  if (!KIND_V) { fl[0] = fl_src[lane]; fl[1] = fl_src[32 + lane]; }                            // byte j of row r's tag word is byte `lane` of the octet's 32
+  else {
+    const u32* f = reinterpret_cast<const u32*>(fl_src);
 #pragma unroll
-    for (int d = 1; d < T; d <<= 1) { int v = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += v; }
-    if (lane < T) { ws.fl[lane] = fl; ws.rowoff[lane] = inc - sz; }
+    for (int t = 0; t < SEGS; t++) fl[t] = f[v_tok(j, t)];
   }
-  __syncwarp();
+  if ((reinterpret_cast<uintptr_t>(sm_src) & 31) == 0) { load_32(sm, s0); load_32(sm + 8, s0 + STEP); }
+  else {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint4 a = *reinterpret_cast<const uint4*>(s0 + h * STEP), b = *reinterpret_cast<const uint4*>(s0 + h * STEP + 16);
+      sm[8 * h] = a.x; sm[8 * h + 1] = a.y; sm[8 * h + 2] = a.z; sm[8 * h + 3] = a.w; sm[8 * h + 4] = b.x; sm[8 * h + 5] = b.y; sm[8 * h + 6] = b.z; sm[8 * h + 7] = b.w;
+    }
+  }
   if (!KIND_V) {
 #pragma unroll
-    for (int o = 0; o < 2; o++) {
-      const int row = 8 * o + r;
-      const uint4* s = reinterpret_cast<const uint4*>(sm_src + o * 1024 + 32 * lane);
-      uint4 s0 = s[0], s1 = s[1];
-      const u32 sm[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-      const u32* c = reinterpret_cast<const u32*>(cd_src + o * 384 + 12 * lane);
-      const u32 cd[3] = {c[0], c[1], c[2]};
-      const u32 fl = ws.fl[row];
-      int pos = ws.rowoff[row] + esc_prefix(fl, 8 * j);
-#pragma unroll
-      for (int g = 0; g < 4; g++) {
-        u32 out[4];
-        decode_group(sm[2 * g], sm[2 * g + 1], k_group_codes(cd, g), (fl >> (8 * j + 2 * g)) & 3u, pos, esc,
-                     b3w[2 * g], b3w[2 * g + 1], dw[2 * g], dw[2 * g + 1], out);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          int s_ = 2 * g + h;
-          u32* x = reinterpret_cast<u32*>(&ws.xs[row * XS_STRIDE + 16 * s_ + 2 * j]);
-          x[0] = out[2 * h]; x[4] = out[2 * h + 1];
-        }
-      }
-    }
+    for (int i = 0; i < 6; i++) cd[i] = reinterpret_cast<const u32*>(cd_src + (i / 3) * 384 + 12 * lane)[i % 3];
+    u32 kp, nv[2];
+    tile_positions<true, false>(fl[0], fl[1], 0u, 0u, 0u, 0u, j, kp, total, nv, none);
+    tags = fl[0] | (fl[1] << 8); pos[0] = kp & 0xFFFFu; pos[1] = kp >> 16;
   } else {
-    const uint2* c2 = reinterpret_cast<const uint2*>(cd_src + 24 * lane);
-    uint2 ca = c2[0], cb = c2[1], cc = c2[2];
-    const u32 cd[6] = {ca.x, ca.y, cb.x, cb.y, cc.x, cc.y};
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const int row = v_tok(j, t);
-      uint4 s = *reinterpret_cast<const uint4*>(sm_src + 64 * lane + 16 * t);
-      const u32 sm[4] = {s.x, s.y, s.z, s.w};
-      const u32 fl = ws.fl[row];
-      int pos = ws.rowoff[row] + esc_prefix(fl, 4 * r);
+    for (int i = 0; i < 3; i++) { const uint2 c = reinterpret_cast<const uint2*>(cd_src + 24 * lane)[i]; cd[2 * i] = c.x; cd[2 * i + 1] = c.y; }
 #pragma unroll
-      for (int g = 0; g < 2; g++) {
-        u32 out[4];
-        decode_group(sm[2 * g], sm[2 * g + 1], v_group_codes(cd, t, g), (fl >> (4 * r + 2 * g)) & 3u, pos, esc,
-                     b3w[2 * g], b3w[2 * g + 1], dw[2 * g], dw[2 * g + 1], out);
+    for (int t = 0; t < SEGS; t++) fl[t] = (fl[t] >> (4 * r)) & 15u;
+    u32 vp[2];
+    tile_positions<false, true>(0u, 0u, fl[0], fl[1], fl[SEGS - 2], fl[SEGS - 1], j, none, none, vp, total);
+    tags = fl[0] | (fl[1] << 4) | (fl[SEGS - 2] << 8) | (fl[SEGS - 1] << 12);
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          int w = 2 * g + h;
-          uint16_t* x = &ws.xs[row * XS_STRIDE + r];
-          x[8 * (4 * w)] = (uint16_t)out[2 * h]; x[8 * (4 * w + 1)] = (uint16_t)(out[2 * h] >> 16);
-          x[8 * (4 * w + 2)] = (uint16_t)out[2 * h + 1]; x[8 * (4 * w + 3)] = (uint16_t)(out[2 * h + 1] >> 16);
-        }
-      }
+    for (int t = 0; t < SEGS; t++) pos[t] = t & 1 ? vp[t >> 1] >> 16 : vp[t >> 1] & 0xFFFFu;
+  }
+  const int n = (int)((total & 0xFFFFu) + (total >> 16)), ofs = (int)(reinterpret_cast<uintptr_t>(esc_src) & 3);
+  const uint8_t* esc = esc_src;
+  __syncwarp();                                      // the scratch is no longer in use
+  if (n <= ESC_STAGE) {
+    const u32* g = reinterpret_cast<const u32*>(esc_src - ofs);
+    for (int i = lane; 4 * i < (n > 0 ? n + ofs : 0); i += 32) ws.esc[i] = g[i];
+    esc = reinterpret_cast<const uint8_t*>(ws.esc) + ofs;
+  }
+  __syncwarp();
+  const u32 at = matrix_row_address(ws, lane);
+#pragma unroll
+  for (int g = 0; g < (KIND_V ? 2 : 4); g++) {
+    u32 f[SEGS][4];
+    const u32x4 bw = lds_u128(w.bases + (KIND_V ? BASES_V + 32 * r : 64 * j) + 16 * g);
+#pragma unroll
+    for (int i = 0; i < SEGS; i++) {
+      constexpr int PER = 8 / SEGS;                  // groups of a segment
+      const int b = 3 * (PER * i + g);               // byte of the group's codes in the lane's 24
+      const u32 z = b == 0 ? group_codes<0>(cd) : b == 3 ? group_codes<3>(cd) : b == 6 ? group_codes<6>(cd) : b == 9 ? group_codes<9>(cd) :
+                    b == 12 ? group_codes<12>(cd) : b == 15 ? group_codes<15>(cd) : b == 18 ? group_codes<18>(cd) : group_codes<21>(cd);
+      decode_group_dev<false>(sm[2 * (PER * i + g)], sm[2 * (PER * i + g) + 1], z, tags >> (2 * (PER * i + g)), pos[i], esc, w, bw, f[i]);
+    }
+    if (!KIND_V) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) store_matrices<false>(at, 2 * g + h, f[0][2 * h], f[0][2 * h + 1], f[1][2 * h], f[1][2 * h + 1]);
+    } else {                                         // word q of a token: channels 8(8g + 2q) + r and 8(8g + 2q + 1) + r; a transposed matrix wants one channel of tokens 2j and 2j + 1
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        store_matrices<true>(at, 4 * g + q, prmt(f[0][q], f[1][q], 0x5410), prmt(f[0][q], f[1][q], 0x7632), prmt(f[SEGS - 2][q], f[SEGS - 1][q], 0x5410), prmt(f[SEGS - 2][q], f[SEGS - 1][q], 0x7632));
     }
   }
   __syncwarp();
