@@ -7,25 +7,29 @@ namespace gaac {
 constexpr int ENC_WARPS = 4;          // warps per CTA
 constexpr int ENC_TILES_PER_WARP = 4; // consecutive work items of one warp share the head's base words
 
-// One warp per (head, tile).  grid = (ceil(ntiles / (ENC_WARPS*ENC_TILES_PER_WARP)), H).  Token t of head h is read at
-// x + h * x_head_stride + t * x_row_stride (bf16 elements): head-major [H, S_in, 128] or token-major [L, n_kv, 128] input.
+// What one kind's encode reads and writes.
+struct EncodeSide {
+  const uint16_t* x; const uint8_t *base3, *base4;
+  uint8_t *sm, *codes; int* flags; uint8_t* slots; int* tile_bytes;
+  int* clear;                     // optional: a word that the first block sets to zero (the ticket of the scan, a status word)
+};
+struct EncodeParams { EncodeSide side[2]; long S, x_head_stride, x_row_stride, S_pad; const int* bidx; int n_kv, ntiles; };
+
+// One warp per (head, tile).  Token t of head h is read at x + h * x_head_stride + t * x_row_stride (bf16 elements): head-major [H, S_in, 128] or
+// token-major [L, n_kv, 128] input.
 template <int KIND_V>
-__global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(
-    const uint16_t* __restrict__ x, long S, long x_head_stride, long x_row_stride, long S_pad, const uint8_t* __restrict__ base3,
-    const uint8_t* __restrict__ base4, const int* __restrict__ bidx, int n_kv, uint8_t* __restrict__ sm, uint8_t* __restrict__ codes,
-    int* __restrict__ flags, uint8_t* __restrict__ slots, int* __restrict__ tile_bytes, int ntiles) {
-  __shared__ __align__(16) WarpScratch scratch[2][ENC_WARPS];       // two per warp: the next tile's rows arrive while this one is encoded
-  __shared__ __align__(16) uint8_t esc_stage[ENC_WARPS][TILE_MAX_ESC];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+__device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const EncodeSide& s, WarpScratch (*scratch)[ENC_WARPS], uint8_t* esc) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ntiles = p.ntiles;
   const long h = blockIdx.y;
-  const int brow = bidx ? bidx[h] : (int)(h % n_kv);
+  if (s.clear && blockIdx.x == 0 && h == 0 && threadIdx.x == 0) *s.clear = 0;
+  const int brow = p.bidx ? p.bidx[h] : (int)(h % p.n_kv);
   u32 b3w[8], b4w[8];
-  load_base_words<KIND_V>(base3 + (long)brow * D, base4 + (long)brow * D, lane, b3w, b4w);
+  load_base_words<KIND_V>(s.base3 + (long)brow * D, s.base4 + (long)brow * D, lane, b3w, b4w);
   const int tile0 = blockIdx.x * (ENC_WARPS * ENC_TILES_PER_WARP) + warp;
-  const uint16_t* xh = x + h * x_head_stride;
+  const uint16_t* xh = s.x + h * p.x_head_stride;
   auto fetch = [&](int i) {                           // rows of the warp's i-th tile into scratch[i & 1]
     const long row0 = (long)(tile0 + i * ENC_WARPS) * T;
-    stage_rows_async(scratch[i & 1][warp], xh + row0 * x_row_stride, x_row_stride, (int)min((long)T, S - row0), lane);
+    stage_rows_async(scratch[i & 1][warp], xh + row0 * p.x_row_stride, p.x_row_stride, (int)min((long)T, p.S - row0), lane);
     async_commit();
   };
   if (tile0 < ntiles) fetch(0);
@@ -37,29 +41,71 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(
     if (more) { fetch(i + 1); async_wait<1>(); } else async_wait<0>();
     WarpScratch& ws = scratch[i & 1][warp];
     const long row0 = (long)tile * T;
-    const int nvalid = (int)min((long)T, S - row0);
+    const int nvalid = (int)min((long)T, p.S - row0);
     LaneTile lt;
     const int total = encode_tile_warp<KIND_V>(ws, nvalid, b3w, b4w, lane, lt);
-    const long trow = h * S_pad + row0;
-    store_tile_payload<KIND_V>(lt, sm + trow * D, codes + trow * CB, reinterpret_cast<uint8_t*>(flags + trow), lane);
+    const long trow = h * p.S_pad + row0;
+    store_tile_payload<KIND_V>(lt, s.sm + trow * D, s.codes + trow * CB, reinterpret_cast<uint8_t*>(s.flags + trow), lane);
     // escape bytes: gathered in shared memory with byte stores (every lane at its own positions), then written to the tile's
     // scratch slot as whole words by neighbouring lanes, so the slot costs one or two coalesced stores instead of ~50 byte stores
-    store_tile_escapes<KIND_V>(ws, lt, esc_stage[warp], lane);
+    store_tile_escapes<KIND_V>(ws, lt, esc, lane);
     __syncwarp();
     {
-      u32* dst = reinterpret_cast<u32*>(slots + (h * ntiles + tile) * (long)TILE_MAX_ESC);
-      const u32* src = reinterpret_cast<const u32*>(esc_stage[warp]);
+      u32* dst = reinterpret_cast<u32*>(s.slots + (h * ntiles + tile) * (long)TILE_MAX_ESC);
+      const u32* src = reinterpret_cast<const u32*>(esc);
       for (int k = lane; 4 * k < total; k += 32) dst[k] = src[k];
     }
-    if (lane == 0) tile_bytes[h * ntiles + tile] = total;
+    if (lane == 0) s.tile_bytes[h * ntiles + tile] = total;
+  }
+}
+// KIND 0 / 1: K or V alone, grid = (ceil(ntiles / 16), H).  2: both, grid z = kind (a prompt's K and V: one launch, and short prompts leave
+// half as much of the GPU idle).
+template <int KIND>
+__global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(const __grid_constant__ EncodeParams p) {
+  __shared__ __align__(16) WarpScratch scratch[2][ENC_WARPS];       // two per warp: the next tile's rows arrive while this one is encoded
+  __shared__ __align__(16) uint8_t esc_stage[ENC_WARPS][TILE_MAX_ESC];
+  const bool v = KIND == 2 ? blockIdx.z != 0 : KIND == 1;
+  if (KIND != 0 && v) encode_tiles_cta<1>(p, p.side[KIND == 2 ? 1 : 0], scratch, esc_stage[threadIdx.x >> 5]);
+  if (KIND != 1 && !v) encode_tiles_cta<0>(p, p.side[0], scratch, esc_stage[threadIdx.x >> 5]);
+}
+static dim3 encode_grid(int ntiles, int64_t H, int kinds) { return dim3((ntiles + ENC_WARPS * ENC_TILES_PER_WARP - 1) / (ENC_WARPS * ENC_TILES_PER_WARP), (unsigned)H, (unsigned)kinds); }
+
+// head_start[0..H] = exclusive prefix of head_bytes, by one CTA of SCAN_THREADS threads (H is the number of cache heads).
+__device__ __forceinline__ void head_prefix(const int* head_bytes, int H, int* head_start) {
+  __shared__ int hsum[32];
+  __shared__ int hcarry;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) { hcarry = 0; head_start[0] = 0; }
+  __syncthreads();
+  for (int base = 0; base < H; base += blockDim.x) {
+    const int i = base + tid;
+    int inc = i < H ? __ldcg(head_bytes + i) : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { int u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
+    if (lane == 31) hsum[warp] = inc;
+    __syncthreads();
+    int before = hcarry;
+    for (int w = 0; w < warp; w++) before += hsum[w];
+    if (i < H) head_start[i + 1] = before + inc;
+    __syncthreads();
+    if (tid == (int)blockDim.x - 1) hcarry = before + inc;
+    __syncthreads();
   }
 }
 
-// Exclusive prefix of tile_bytes per head.  One CTA of 1024 threads per head, four tiles per thread and pass: a 64K-token
-// head (4096 tiles) is one pass of two warp scans.
+// Exclusive prefix of tile_bytes per head.  One CTA of 1024 threads per (head, kind), four tiles per thread and pass: a 64K-token
+// head (4096 tiles) is one pass of two warp scans.  With head_start (one kind) the CTA that finishes last also makes the prefix over the
+// heads, head_start[0..H], and hands head_start[H] to the host through `total` (pinned memory, may be NULL): a launch and a copy less than
+// doing it behind this kernel.  head_start[H] is the ticket until then and must be zero on entry.
+struct ScanSide { const int* tile_bytes; int *tile_off, *head_bytes; };
+struct ScanParams { ScanSide side[2]; int ntiles; long tile_off_stride; int* head_start; int* total; };
 constexpr int SCAN_THREADS = 1024;
-__global__ void __launch_bounds__(SCAN_THREADS) tile_scan_kernel(const int* __restrict__ tile_bytes, int ntiles, int* __restrict__ tile_off,
-                                                                  long tile_off_stride, int* __restrict__ head_bytes) {
+__global__ void __launch_bounds__(SCAN_THREADS) tile_scan_kernel(const __grid_constant__ ScanParams p) {
+  const int* tile_bytes = p.side[blockIdx.y].tile_bytes;
+  int* tile_off = p.side[blockIdx.y].tile_off;
+  int* head_bytes = p.side[blockIdx.y].head_bytes;
+  const int ntiles = p.ntiles;
+  const long tile_off_stride = p.tile_off_stride;
   __shared__ int wsum[32];
   __shared__ int carry_s, pass_total;
   const long h = blockIdx.x;
@@ -97,67 +143,76 @@ __global__ void __launch_bounds__(SCAN_THREADS) tile_scan_kernel(const int* __re
     __syncthreads();
   }
   if (tid == 0 && head_bytes) head_bytes[h] = carry_s;
-}
-
-// head_start[0..H] = exclusive prefix of head_bytes (one small CTA; H is the number of cache heads).
-__global__ void __launch_bounds__(256) head_prefix_kernel(const int* __restrict__ head_bytes, int H, int* __restrict__ head_start) {
-  __shared__ int wsum[8];
-  __shared__ int carry_s;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) { carry_s = 0; head_start[0] = 0; }
+  if (!p.head_start) return;
+  __shared__ int last;
+  const int H = gridDim.x;
+  if (tid == 0) { __threadfence(); last = atomicAdd(p.head_start + H, 1) == H - 1; }
   __syncthreads();
-  for (int base = 0; base < H; base += 256) {
-    const int i = base + tid;
-    const int v = i < H ? head_bytes[i] : 0;
-    int inc = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { int u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
-    if (lane == 31) wsum[warp] = inc;
-    __syncthreads();
-    int woff = 0;
-    for (int w = 0; w < warp; w++) woff += wsum[w];
-    const int carry = carry_s;
-    if (i < H) head_start[i + 1] = carry + woff + inc;
-    __syncthreads();
-    if (tid == 255) carry_s = carry + woff + inc;
-    __syncthreads();
+  if (!last) return;
+  __threadfence();
+  head_prefix(head_bytes, H, p.head_start);
+  if (tid == 0 && p.total) {
+    *(volatile int*)p.total = p.head_start[H];
+    __threadfence_system();
   }
 }
 
-// One warp per (head, tile): slot -> ovf[head_start[h] + tile_off[h, tile]]; optionally the per-row escape offsets
+__global__ void __launch_bounds__(SCAN_THREADS) head_prefix_kernel(const int* __restrict__ head_bytes, int H, int* __restrict__ head_start) { head_prefix(head_bytes, H, head_start); }
+
+// What one kind's compaction reads and writes.
+struct CompactSide { const uint8_t* slots; const int *tile_bytes, *tile_off, *head_start; uint8_t* ovf; const int* flags; int* ovf_off; int* status; };
+struct FinishParams {              // the end of a prompt's prefill, see prefill_finish
+  const uint16_t *k_tok, *v_tok; long row_stride, L; int n_kv; long h0; uint16_t *ktail, *vtail; int *seq_len, *tail_len, *used_k, *used_v, *status;
+};
+struct CompactParams {
+  CompactSide side[2]; int ntiles; unsigned n_items; long tile_off_stride, head_stride, S, S_pad; int zero_pad; long ovf_cap, head_cap;
+  int finish; FinishParams fin;
+};
+__device__ void prefill_finish(const FinishParams& p);
+
+// Escape bytes of every tile: slot -> ovf[head_start[h] + tile_off[h, tile]]; optionally the per-row escape offsets
 // ovf_off[h, row] = tile_off[h, tile] + (escape bytes of the tile's earlier rows), recomputed from the tag words.
-__global__ void __launch_bounds__(128) compact_copy_kernel(const uint8_t* __restrict__ slots, const int* __restrict__ tile_bytes, int ntiles,
-                                                            const int* __restrict__ tile_off, long tile_off_stride,
-                                                            const int* __restrict__ head_start, long head_stride, uint8_t* __restrict__ ovf, long n_items,
-                                                            const int* __restrict__ flags, long S, long S_pad, int* __restrict__ ovf_off, int zero_pad,
-                                                            long ovf_cap, long head_cap, int* __restrict__ status) {
-  const long item = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (item >= n_items) return;
-  const int lane = threadIdx.x & 31;
-  const long h = item / ntiles, t = item % ntiles;
-  const int n = tile_bytes[item];
-  const int toff = tile_off[h * tile_off_stride + t];
-  const uint8_t* src = slots + item * (long)TILE_MAX_ESC;
+// Eight lanes per tile: a tile has some 55 escape bytes and 16 tag words, and what the kernel waits for are its loads (sizes and offsets, then the
+// bytes), so a warp keeps four tiles in flight.  grid y = kind.
+__global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant__ CompactParams p) {
+  if (p.finish && blockIdx.x == gridDim.x - 1) {     // one more block: the rest of a prompt's prefill
+    if (blockIdx.y == 0) prefill_finish(p.fin);
+    return;
+  }
+  const CompactSide& s = p.side[blockIdx.y];
+  const int lane = threadIdx.x & 31, q = lane & 7;
+  const unsigned first = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 4, item = first + (lane >> 3);
+  const bool live = item < p.n_items;
+  const unsigned h = live ? item / (unsigned)p.ntiles : 0u, t = live ? item - h * (unsigned)p.ntiles : 0u;
+  const int n = live ? s.tile_bytes[item] : 0;
+  const int toff = live ? s.tile_off[h * p.tile_off_stride + t] : 0;
+  const uint8_t* src = s.slots + (long)item * TILE_MAX_ESC;
   // bounds: the whole stream must fit ovf_cap bytes (ovf_cap > 0), a head's part head_cap bytes (head_cap > 0), read padding
   // included; a tile that does not fit is not written and bit 0 of *status is set
-  const long at = (head_start ? (long)head_start[h] : h * head_stride) + toff;        // no table: head h's stream starts at h * head_stride
-  const bool fits = (ovf_cap <= 0 || at + n + zero_pad <= ovf_cap) && (head_cap <= 0 || (long)toff + n + zero_pad <= head_cap);
-  if (fits) { uint8_t* dst = ovf + at; for (int i = lane; i < n; i += 32) dst[i] = src[i]; }
-  else if (lane == 0 && status) atomicOr(status, 1);
-  if (zero_pad && head_cap <= 0 && head_start && item == 0 && lane < zero_pad) {                                    // over-read padding behind the last head (packed stream)
-    const long end = (long)head_start[n_items / ntiles];
-    if (ovf_cap <= 0 || end + zero_pad <= ovf_cap) ovf[end + lane] = 0;
-    else if (lane == 0 && status) atomicOr(status, 1);
+  const long at = (s.head_start ? (long)s.head_start[h] : (long)h * p.head_stride) + toff;        // no table: head h's stream starts at h * head_stride
+  const bool fits = (p.ovf_cap <= 0 || at + n + p.zero_pad <= p.ovf_cap) && (p.head_cap <= 0 || (long)toff + n + p.zero_pad <= p.head_cap);
+  if (fits) {
+    uint8_t* dst = s.ovf + at;
+#pragma unroll 4
+    for (int i = q; i < n; i += 8) dst[i] = src[i];
+  } else if (live && q == 0 && s.status) atomicOr(s.status, 1);
+  if (p.zero_pad && p.head_cap <= 0 && s.head_start && first == 0 && lane < p.zero_pad) {                              // over-read padding behind the last head (packed stream)
+    const long end = (long)s.head_start[p.n_items / (unsigned)p.ntiles];
+    if (p.ovf_cap <= 0 || end + p.zero_pad <= p.ovf_cap) s.ovf[end + lane] = 0;
+    else if (lane == 0 && s.status) atomicOr(s.status, 1);
   }
-  if (ovf_off) {
-    const long row = t * T + (lane & 15);
-    const int sz = (lane < T && row < S) ? row_esc_bytes((u32)flags[h * S_pad + row]) : 0;
-    int inc = sz;
+  if (s.ovf_off) {
+    const long row = (long)t * T + 2 * q;
+    const int s0 = live && row < p.S ? row_esc_bytes((u32)s.flags[h * p.S_pad + row]) : 0, s1 = live && row + 1 < p.S ? row_esc_bytes((u32)s.flags[h * p.S_pad + row + 1]) : 0;
+    int inc = s0 + s1;
 #pragma unroll
-    for (int d = 1; d < T; d <<= 1) { int v = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += v; }
-    if (lane < T && row < S) ovf_off[h * S + row] = toff + inc - sz;
+    for (int d = 1; d < 8; d <<= 1) { const int v = __shfl_up_sync(FULL, inc, d, 8); if (q >= d) inc += v; }
+    int* o = s.ovf_off + (long)h * p.S + row;
+    if (live && row < p.S) o[0] = toff + inc - s0 - s1;
+    if (live && row + 1 < p.S) o[1] = toff + inc - s1;
   }
 }
+static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_items + 15) / 16 + (p.finish ? 1 : 0), (unsigned)kinds); }
 
 // One warp per (head, tile): compressed tile -> bf16 rows.
 template <int KIND_V>
@@ -244,50 +299,52 @@ __global__ void __launch_bounds__(128) bases_from_hist_kernel(const long long* _
 // Last step of a slot's prefill (one CTA): the prompt's remainder (L mod 16 rows) goes into the raw tails of the slot's heads,
 // the heads' token counters are set, and the largest escape stream of the slot per kind is reported for the host's capacity
 // check.  k_tok / v_tok: token-major rows, head h of token t at t * row_stride + h * 128 (bf16 elements).
-__global__ void __launch_bounds__(256) prefill_finish_kernel(const uint16_t* __restrict__ k_tok, const uint16_t* __restrict__ v_tok, long row_stride, long L,
-                                                              int n_kv, long h0, uint16_t* __restrict__ ktail, uint16_t* __restrict__ vtail,
-                                                              int* __restrict__ seq_len, int* __restrict__ tail_len, int* __restrict__ used_k,
-                                                              int* __restrict__ used_v, int* __restrict__ status) {
-  const long n_full = L / T * T;
-  const int rem = (int)(L - n_full), tid = threadIdx.x;
-  const int per_kind = rem * n_kv * 16;                              // 16-byte pieces
+__device__ void prefill_finish(const FinishParams& p) {
+  const long n_full = p.L / T * T;
+  const int rem = (int)(p.L - n_full), tid = threadIdx.x;
+  const int per_kind = rem * p.n_kv * 16;                            // 16-byte pieces
   for (int i = tid; i < 2 * per_kind; i += blockDim.x) {
     const int kind = i >= per_kind, j = i - kind * per_kind;
-    const int r = j / (n_kv * 16), h = (j >> 4) % n_kv, c = j & 15;
-    const uint16_t* src = (kind ? v_tok : k_tok) + (n_full + r) * row_stride + h * D + c * 8;
-    uint16_t* dst = (kind ? vtail : ktail) + ((h0 + h) * T + r) * D + c * 8;
+    const int r = j / (p.n_kv * 16), h = (j >> 4) % p.n_kv, c = j & 15;
+    const uint16_t* src = (kind ? p.v_tok : p.k_tok) + (n_full + r) * p.row_stride + h * D + c * 8;
+    uint16_t* dst = (kind ? p.vtail : p.ktail) + ((p.h0 + h) * T + r) * D + c * 8;
     *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
   }
-  if (tid < n_kv) {
-    seq_len[h0 + tid] = (int)n_full; tail_len[h0 + tid] = rem;
-    if (n_full == 0) { used_k[h0 + tid] = 0; used_v[h0 + tid] = 0; }
+  for (int h = tid; h < p.n_kv; h += blockDim.x) {
+    p.seq_len[p.h0 + h] = (int)n_full; p.tail_len[p.h0 + h] = rem;
+    if (n_full == 0) { p.used_k[p.h0 + h] = 0; p.used_v[p.h0 + h] = 0; }
   }
-  __syncthreads();
   if (tid == 0) {
     int mk = 0, mv = 0;
-    for (int h = 0; h < n_kv; h++) { mk = max(mk, used_k[h0 + h]); mv = max(mv, used_v[h0 + h]); }
-    status[1] = mk; status[3] = mv;
+    if (n_full) for (int h = 0; h < p.n_kv; h++) { mk = max(mk, p.used_k[p.h0 + h]); mv = max(mv, p.used_v[p.h0 + h]); }
+    p.status[1] = mk; p.status[3] = mv;
+    if (n_full == 0) { p.status[0] = 0; p.status[2] = 0; }           // no copy in front of this step
   }
 }
+__global__ void __launch_bounds__(128) prefill_finish_kernel(const __grid_constant__ FinishParams p) { prefill_finish(p); }
 
 }  // namespace gaac
 
 using namespace gaac;
 
-extern "C" int gaac_encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
-                                 const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
-                                 uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes, void* stream) {
+// gaac_encode_tiles with a word that the kernel clears
+static int encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad, const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
+                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes, int32_t* clear, void* stream) {
   if (!x_bf16 || !base3 || !base4 || !sm || !codes || !flags || !slots || !tile_bytes) return GAAC_E_ARG;
   if (H <= 0 || S <= 0 || S_in < S || S_pad < (S + T - 1) / T * T || S_pad % T || n_kv <= 0 || H > 65535 || (kind != GAAC_KIND_K && kind != GAAC_KIND_V)) return GAAC_E_ARG;
   if (!aligned16(x_bf16) || !aligned16(sm) || !aligned16(codes)) return GAAC_E_ALIGN;
   const int ntiles = (int)((S + T - 1) / T);
-  dim3 grid((ntiles + ENC_WARPS * ENC_TILES_PER_WARP - 1) / (ENC_WARPS * ENC_TILES_PER_WARP), (unsigned)H);
+  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles};
   cudaStream_t st = (cudaStream_t)stream;
-  if (kind == GAAC_KIND_K)
-    encode_tiles_kernel<0><<<grid, ENC_WARPS * 32, 0, st>>>((const uint16_t*)x_bf16, S, S_in * D, D, S_pad, base3, base4, bidx, n_kv, sm, codes, flags, slots, tile_bytes, ntiles);
-  else
-    encode_tiles_kernel<1><<<grid, ENC_WARPS * 32, 0, st>>>((const uint16_t*)x_bf16, S, S_in * D, D, S_pad, base3, base4, bidx, n_kv, sm, codes, flags, slots, tile_bytes, ntiles);
+  if (kind == GAAC_KIND_K) encode_tiles_kernel<0><<<encode_grid(ntiles, H, 1), ENC_WARPS * 32, 0, st>>>(p);
+  else encode_tiles_kernel<1><<<encode_grid(ntiles, H, 1), ENC_WARPS * 32, 0, st>>>(p);
   return launch_status();
+}
+
+extern "C" int gaac_encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
+                                 const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
+                                 uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes, void* stream) {
+  return encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, nullptr, stream);
 }
 
 extern "C" int gaac_compact(const uint8_t* slots, const int32_t* tile_bytes, int64_t H, int64_t ntiles, const int32_t* head_start,
@@ -296,13 +353,20 @@ extern "C" int gaac_compact(const uint8_t* slots, const int32_t* tile_bytes, int
   if (!tile_bytes || !tile_off || H <= 0 || ntiles <= 0 || tile_off_stride < ntiles) return GAAC_E_ARG;
   if (head_start && (!ovf || !slots)) return GAAC_E_ARG;
   if (ovf_off && (!head_start || !flags || S <= 0 || S_pad < S)) return GAAC_E_ARG;
-  cudaStream_t st = (cudaStream_t)stream;
-  tile_scan_kernel<<<(unsigned)H, SCAN_THREADS, 0, st>>>(tile_bytes, (int)ntiles, tile_off, tile_off_stride, head_bytes);
-  if (head_start) {
-    const long n_items = H * ntiles;
-    compact_copy_kernel<<<(unsigned)((n_items + 3) / 4), 128, 0, st>>>(slots, tile_bytes, (int)ntiles, tile_off, tile_off_stride, head_start, 0, ovf, n_items,
-                                                                    flags, S, S_pad, ovf_off, 0, 0, 0, nullptr);
-  }
+  const ScanParams sp{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, tile_off_stride, nullptr, nullptr};
+  tile_scan_kernel<<<(unsigned)H, SCAN_THREADS, 0, (cudaStream_t)stream>>>(sp);
+  if (head_start) return gaac_compact_copy(slots, tile_bytes, H, ntiles, head_start, ovf, tile_off, tile_off_stride, flags, S, S_pad, ovf_off, 0, 0, 0, nullptr, stream);
+  return launch_status();
+}
+
+static int encode_begin(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad, const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
+                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes, int32_t* tile_off, int32_t* head_bytes, int32_t* head_start,
+                        int32_t* total, void* stream) {
+  if (!tile_off || !head_bytes || !head_start) return GAAC_E_ARG;
+  if (int e = encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, head_start + H, stream)) return e;
+  const int64_t ntiles = (S + T - 1) / T;
+  const ScanParams sp{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, total};
+  tile_scan_kernel<<<(unsigned)H, SCAN_THREADS, 0, (cudaStream_t)stream>>>(sp);
   return launch_status();
 }
 
@@ -310,28 +374,35 @@ extern "C" int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64
                                  const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                                  uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
                                  int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, void* stream) {
-  if (!tile_off || !head_bytes || !head_start) return GAAC_E_ARG;
-  if (int e = gaac_encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, stream)) return e;
-  const int64_t ntiles = (S + T - 1) / T;
-  if (int e = gaac_compact(nullptr, tile_bytes, H, ntiles, nullptr, nullptr, tile_off, ntiles, head_bytes, nullptr, 0, 0, nullptr, stream)) return e;
-  return gaac_head_prefix(head_bytes, H, head_start, stream);
+  return encode_begin(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, tile_off, head_bytes, head_start, nullptr, stream);
+}
+
+extern "C" int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
+                                 const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
+                                 uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
+                                 int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream) {
+  if (!total_pinned) return GAAC_E_ARG;
+  if (int e = encode_begin(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, tile_off, head_bytes, head_start, total_pinned, stream)) return e;
+  return cudaStreamSynchronize((cudaStream_t)stream) == cudaSuccess ? GAAC_OK : GAAC_E_LAUNCH;
 }
 
 extern "C" int gaac_compact_copy(const uint8_t* slots, const int32_t* tile_bytes, int64_t H, int64_t ntiles, const int32_t* head_start, uint8_t* ovf,
                                  const int32_t* tile_off, int64_t tile_off_stride, const int32_t* flags, int64_t S, int64_t S_pad, int32_t* ovf_off,
                                  int zero_pad, int64_t ovf_cap, int64_t head_cap, int32_t* status, void* stream) {
   if (!slots || !tile_bytes || !head_start || !ovf || !tile_off || H <= 0 || ntiles <= 0 || tile_off_stride < ntiles || zero_pad < 0 || zero_pad > 32) return GAAC_E_ARG;
-  if (ovf_cap < 0 || head_cap < 0) return GAAC_E_ARG;
+  if (ovf_cap < 0 || head_cap < 0 || H * ntiles > 0x7FFFFFF0LL) return GAAC_E_ARG;
   if (ovf_off && (!flags || S <= 0 || S_pad < S)) return GAAC_E_ARG;
-  const long n_items = H * ntiles;
-  compact_copy_kernel<<<(unsigned)((n_items + 3) / 4), 128, 0, (cudaStream_t)stream>>>(slots, tile_bytes, (int)ntiles, tile_off, tile_off_stride, head_start, 0, ovf,
-                                                                                       n_items, flags, S, S_pad, ovf_off, zero_pad, ovf_cap, head_cap, status);
+  CompactParams p{};
+  p.side[0] = CompactSide{slots, tile_bytes, tile_off, head_start, ovf, flags, ovf_off, status};
+  p.ntiles = (int)ntiles; p.n_items = (unsigned)(H * ntiles); p.tile_off_stride = tile_off_stride; p.S = S; p.S_pad = S_pad;
+  p.zero_pad = zero_pad; p.ovf_cap = ovf_cap; p.head_cap = head_cap;
+  compact_copy_kernel<<<compact_grid(p, 1), 128, 0, (cudaStream_t)stream>>>(p);
   return launch_status();
 }
 
 extern "C" int gaac_head_prefix(const int32_t* head_bytes, int64_t H, int32_t* head_start, void* stream) {
   if (!head_bytes || !head_start || H <= 0) return GAAC_E_ARG;
-  head_prefix_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(head_bytes, (int)H, head_start);
+  head_prefix_kernel<<<1, SCAN_THREADS, 0, (cudaStream_t)stream>>>(head_bytes, (int)H, head_start);
   return launch_status();
 }
 
@@ -390,32 +461,37 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   const long h0 = (long)slot * n_kv;
   const int ntiles = (int)(L / T);
   const long S = (long)ntiles * T, tiles_cap = S_cap / T, n_items = (long)n_kv * ntiles;
-  // scratch: escape slots of K, of V, then the tile sizes of K, of V
-  uint8_t* slots[2] = {scratch, scratch + n_items * TILE_MAX_ESC};
-  int32_t* tbytes[2] = {reinterpret_cast<int32_t*>(scratch + 2 * n_items * TILE_MAX_ESC), reinterpret_cast<int32_t*>(scratch + 2 * n_items * TILE_MAX_ESC) + n_items};
-  if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
-  else cudaMemsetAsync(status, 0, 16, st);
+  if (n_items > 0x7FFFFFF0L) return GAAC_E_ARG;
+  const FinishParams fin{(const uint16_t*)k_tok, (const uint16_t*)v_tok, row_stride, L, n_kv, h0, (uint16_t*)K->tail, (uint16_t*)V->tail, seq_len, tail_len, K->ovf_used, V->ovf_used, status};
+  if (ntiles == 0) {
+    if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
+    else prefill_finish_kernel<<<1, 128, 0, st>>>(fin);
+    return launch_status();
+  }
+  // Three launches for both kinds: encode, offsets, copy (whose last block does the tails and counters); the encode clears the words that the
+  // copy reports into.  scratch: escape slots of K, of V, then the tile sizes of K, of V
   const gaac_store* side[2] = {K, V};
   const void* tok[2] = {k_tok, v_tok};
-  for (int kind = 0; kind < 2 && ntiles > 0; kind++) {
+  EncodeParams ep{}; ScanParams sp{}; CompactParams cp{};
+  for (int kind = 0; kind < 2; kind++) {
     const gaac_store* s = side[kind];
+    uint8_t* slots = scratch + kind * n_items * TILE_MAX_ESC;
+    int32_t* tbytes = reinterpret_cast<int32_t*>(scratch + 2 * n_items * TILE_MAX_ESC) + kind * n_items;
     int32_t* toff = s->tile_off + h0 * tiles_cap;
-    if (!copy_only) {
-      const uint8_t* b3 = s->base3 + (h0 % n_base_rows) * D; const uint8_t* b4 = s->base4 + (h0 % n_base_rows) * D;      // consecutive heads, consecutive rows
-      dim3 grid((ntiles + ENC_WARPS * ENC_TILES_PER_WARP - 1) / (ENC_WARPS * ENC_TILES_PER_WARP), (unsigned)n_kv);
-      if (kind == 0)
-        encode_tiles_kernel<0><<<grid, ENC_WARPS * 32, 0, st>>>((const uint16_t*)tok[kind], S, D, row_stride, S_cap, b3, b4, nullptr, n_kv, s->sm + h0 * S_cap * D,
-                                                               s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots[kind], tbytes[kind], ntiles);
-      else
-        encode_tiles_kernel<1><<<grid, ENC_WARPS * 32, 0, st>>>((const uint16_t*)tok[kind], S, D, row_stride, S_cap, b3, b4, nullptr, n_kv, s->sm + h0 * S_cap * D,
-                                                               s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots[kind], tbytes[kind], ntiles);
-      tile_scan_kernel<<<(unsigned)n_kv, SCAN_THREADS, 0, st>>>(tbytes[kind], ntiles, toff, tiles_cap, s->ovf_used + h0);
-    }
-    compact_copy_kernel<<<(unsigned)((n_items + 3) / 4), 128, 0, st>>>(slots[kind], tbytes[kind], ntiles, toff, tiles_cap, nullptr, ovf_cap, s->ovf + h0 * ovf_cap, n_items,
-                                                                    nullptr, 0, 0, nullptr, 0, 0, ovf_cap - CACHE_READ_PAD, status + 2 * kind);
+    ep.side[kind] = EncodeSide{(const uint16_t*)tok[kind], s->base3 + (h0 % n_base_rows) * D, s->base4 + (h0 % n_base_rows) * D,          // consecutive heads, consecutive rows
+                               s->sm + h0 * S_cap * D, s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots, tbytes, status + 2 * kind};
+    sp.side[kind] = ScanSide{tbytes, toff, s->ovf_used + h0};
+    cp.side[kind] = CompactSide{slots, tbytes, toff, nullptr, s->ovf + h0 * ovf_cap, nullptr, nullptr, status + 2 * kind};
   }
-  if (!copy_only)
-    prefill_finish_kernel<<<1, 256, 0, st>>>((const uint16_t*)k_tok, (const uint16_t*)v_tok, row_stride, L, n_kv, h0, (uint16_t*)K->tail, (uint16_t*)V->tail,
-                                             seq_len, tail_len, K->ovf_used, V->ovf_used, status);
+  ep.S = S; ep.x_head_stride = D; ep.x_row_stride = row_stride; ep.S_pad = S_cap; ep.n_kv = n_kv; ep.ntiles = ntiles;
+  sp.ntiles = ntiles; sp.tile_off_stride = tiles_cap;
+  cp.ntiles = ntiles; cp.n_items = (unsigned)n_items; cp.tile_off_stride = tiles_cap; cp.head_stride = ovf_cap; cp.head_cap = ovf_cap - CACHE_READ_PAD;
+  cp.finish = !copy_only; cp.fin = fin;
+  if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
+  else {
+    encode_tiles_kernel<2><<<encode_grid(ntiles, n_kv, 2), ENC_WARPS * 32, 0, st>>>(ep);
+    tile_scan_kernel<<<dim3((unsigned)n_kv, 2), SCAN_THREADS, 0, st>>>(sp);
+  }
+  compact_copy_kernel<<<compact_grid(cp, 2), 128, 0, st>>>(cp);
   return launch_status();
 }

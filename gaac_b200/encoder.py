@@ -4,7 +4,7 @@ Mirror of gaac/encoder.py.  `encode_tiles` writes sign/mantissa, code and tag by
 tile's escape bytes in a bounded scratch slot (1280 B worst case); `compact` turns the per-tile byte counts into tile offsets and
 packs the slots into each head's escape stream.  `encode_into` chains the two on the device with no host round trip in
 between (the escape stream is caller-sized and the copy into it is bounded); `encode` builds a whole Page with it and reads the
-exact size once at the end.
+size in the middle, allocates the stream exactly and fills it.
 """
 from __future__ import annotations
 import torch
@@ -18,9 +18,12 @@ class TileEncoder:
     def __init__(self, kind: str, device="cuda"):
         self.kind = kind
         self.device = device
-        # index tables kept for callers that read them (the kernels do not need them)
-        self.perm = perm(kind).to(torch.int32)
         self._slots = None
+
+    # index tables kept for callers that read them (the kernels do not need them, and a dozen small torch operations per encoder are not free)
+    @property
+    def perm(self):
+        return perm(self.kind).to(torch.int32)
 
     @property
     def inv_sm(self):
@@ -77,8 +80,6 @@ class TileEncoder:
         return tile_off
 
     # ------------------------------------------------------------------ whole encode without a host round trip
-    GUESS_BYTES_PER_TILE = 128          # first guess for the escape stream of a Page (measured mean on model-like data: 30-60 B)
-
     def _status(self, dev) -> torch.Tensor:
         st = getattr(self, "_status_word", None)
         if st is None or st.device != dev:
@@ -128,9 +129,8 @@ class TileEncoder:
 
     def encode(self, codec: Codec, x: torch.Tensor) -> Page:
         """x: [H, S, D] bf16 -> Page, bit-identical to the reference Codec.encode(x, kind).  (gaac/encoder.py:111-123)
-        Everything is launched into an escape buffer of GUESS_BYTES_PER_TILE bytes per tile; ONE host read at the end (the total and
-        the status word) cuts the stream to its exact size, as the reference's is.  When the guess was too small the copy alone is
-        repeated into a buffer of the exact size."""
+        The kernels hand the size of the escape stream to the host through page-locked memory; the stream is then allocated at its exact
+        size, as the reference's is, and one more kernel fills it."""
         if not x.is_cuda:
             raise RuntimeError("TileEncoder needs CUDA tensors: gaac_b200 has no CPU path")
         H, S, _ = x.shape; dev = x.device
@@ -139,19 +139,22 @@ class TileEncoder:
         sm = torch.empty(H, S_pad * D, dtype=torch.uint8, device=dev)
         cd = torch.empty(H, S_pad * CB, dtype=torch.uint8, device=dev)
         flags = torch.empty(H, S_pad, dtype=torch.int32, device=dev)          # every row of every tile is written, padded rows as 0
-        meta = torch.zeros(H * ntiles + H + 2, dtype=torch.int32, device=dev)                     # tile offsets | head_start [H+1] | the call's status word
-        tile_off, head_start, status = meta[:H * ntiles].view(H, ntiles), meta[H * ntiles:H * ntiles + H + 1], meta[-1:]
         ovf_off = torch.empty(H, S, dtype=torch.int32, device=dev)
         if H == 0 or ntiles == 0:
-            return Page(sm, cd, flags, ovf_off, torch.zeros(8, dtype=torch.uint8, device=dev), head_start, tile_off, codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
-        cap = H * ntiles * self.GUESS_BYTES_PER_TILE + 8
-        ovf = torch.empty(cap, dtype=torch.uint8, device=dev)
-        _, retry = self.encode_into(x, codec.base3, codec.base4, codec.n_kv, sm, cd, flags, tile_off, ovf, S=S, S_pad=S_pad, head_start=head_start, ovf_off=ovf_off,
-                                    status=status)
-        total, st = meta[-2:].tolist()                                                            # the one host synchronisation: all bytes, status word
-        if st:                                                                                    # the guess was too small: now the size is known
-            ovf = torch.empty(total + 8, dtype=torch.uint8, device=dev)
-            retry(ovf)
-        elif cap != total + 8:
-            ovf = ovf[:total + 8].clone()
+            return Page(sm, cd, flags, ovf_off, torch.zeros(8, dtype=torch.uint8, device=dev), torch.zeros(H + 1, dtype=torch.int32, device=dev),
+                        torch.zeros(H, ntiles, dtype=torch.int32, device=dev), codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
+        meta = torch.empty(H * ntiles + H + 1, dtype=torch.int32, device=dev)                     # tile offsets | head_start [H+1]
+        tile_off, head_start = meta[:H * ntiles].view(H, ntiles), meta[H * ntiles:]
+        x = x.contiguous()
+        slots = self._scratch(H * ntiles * SLOT, dev)
+        work = torch.empty(H * ntiles + H, dtype=torch.int32, device=dev)                         # tile sizes | head sizes
+        total = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        L = _lib.lib(); st = _lib.stream_ptr(dev)
+        p_flags, p_slots, p_work, p_meta = flags.data_ptr(), slots.data_ptr(), work.data_ptr(), meta.data_ptr()
+        p_hs = p_meta + 4 * H * ntiles
+        _lib.check(L.gaac_encode_sized(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
+                                       sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_meta, p_work + 4 * H * ntiles, p_hs, total.data_ptr(), st), "gaac_encode_sized")
+        ovf = torch.empty(total.item() + 8, dtype=torch.uint8, device=dev)
+        _lib.check(L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_meta, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, 0, 0, None, st),
+                   "gaac_compact_copy")
         return Page(sm, cd, flags, ovf_off, ovf, head_start, tile_off, codec.base3, codec.base4, H, S, codec.n_kv, self.kind)

@@ -61,6 +61,13 @@ int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, in
                       uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, void* stream);
 
+/* gaac_encode_begin, then a wait for the stream: on return *total_pinned (page-locked host memory) holds head_start[H], which the
+ * kernels wrote there themselves.  For a caller that wants the escape stream at its exact size (TileEncoder.encode). */
+int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
+                      const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
+                      uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
+                      int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream);
+
 /* The copy half of gaac_compact with tile offsets that are already known: scratch slots -> ovf + head_start[h] + tile_off[h, t],
  * optionally the per-row offsets ovf_off [H, S], and zero_pad (0..32) zero bytes written behind the last head (the reference
  * allocates its stream with 8 bytes of over-read padding, gaac/encoder.py:121).  The copy is bounded, which lets a caller
