@@ -1,4 +1,5 @@
 // Block encoder, escape-stream compaction, page decoder and calibration kernels (sm_100a).
+#include <algorithm>
 #include "gaac_api.cuh"
 #include "gaac_warp.cuh"
 
@@ -239,60 +240,81 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) decode_page_kernel(
   }
 }
 
-// Exponent histogram: x [N, n_ch] bf16, hist [n_ch, 256] int64.  grid = (ceil(n_ch/128), row chunks); a thread owns one
-// channel and keeps a private 256-bin histogram of 16-bit counters in shared memory, flushed with atomics.
-constexpr int HIST_ROWS = 64;         // rows per CTA: short chunks put hundreds of CTAs on a 2048-token calibration sample (16-bit counters cannot overflow)
-__global__ void __launch_bounds__(128) exponent_hist_kernel(const uint16_t* __restrict__ x, long N, long n_ch, unsigned long long* __restrict__ hist) {
-  extern __shared__ unsigned short bins[];           // [256][128]: bin-major so a warp's increments spread over banks
+// Exponent histogram: x [N rows, n_ch] bf16, row r at x + r * row_stride; hist [n_ch, 256] counts.  grid = (ceil(n_ch/128), row chunks, kinds); a
+// thread owns one channel and a private 256-bin histogram of 8-bit counters in shared memory, flushed with atomics.  Counter (bin, channel) is
+// byte bin & 3 of word [bin >> 2][channel]: a warp's increments go to 32 banks whatever the exponents are, the table is cleared with 16-byte stores,
+// and the flush reads four bins at a time, nearly all of them empty.  16-bit counters by bin (64 KB, three CTAs per SM, 512 single stores and loads per
+// thread to clear and flush them for 64 rows) took most of the kernel's time.
+constexpr int HIST_ROWS = 128;        // rows per CTA (8-bit counters); twice the rows of one flush, and still 500 CTAs on a 4000-token prompt of 8 kv heads
+template <class Cnt> struct HistParams { const uint16_t* x[2]; Cnt* hist[2]; long N, n_ch, row_stride; };
+template <class Cnt>
+__global__ void __launch_bounds__(128) exponent_hist_kernel(const __grid_constant__ HistParams<Cnt> p) {
+  __shared__ __align__(16) u32 bins[64][128];
   const int tid = threadIdx.x;
   const long c = (long)blockIdx.x * 128 + tid;
-  for (int b = 0; b < 256; b++) bins[b * 128 + tid] = 0;
-  const long r0 = (long)blockIdx.y * HIST_ROWS, r1 = min(N, r0 + HIST_ROWS);
-  if (c < n_ch) {
-    long r = r0;
-    for (; r + 4 <= r1; r += 4) {                       // four independent loads in flight per thread
-      const unsigned a0 = x[r * n_ch + c], a1 = x[(r + 1) * n_ch + c], a2 = x[(r + 2) * n_ch + c], a3 = x[(r + 3) * n_ch + c];
-      bins[((a0 >> 7) & 0xFF) * 128 + tid]++; bins[((a1 >> 7) & 0xFF) * 128 + tid]++;
-      bins[((a2 >> 7) & 0xFF) * 128 + tid]++; bins[((a3 >> 7) & 0xFF) * 128 + tid]++;
-    }
-    for (; r < r1; r++) bins[((x[r * n_ch + c] >> 7) & 0xFF) * 128 + tid]++;
+#pragma unroll
+  for (int i = 0; i < 16; i++) reinterpret_cast<uint4*>(bins)[i * 128 + tid] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  if (c >= p.n_ch) return;
+  const uint16_t* x = p.x[blockIdx.z] + c;
+  uint8_t* mine = reinterpret_cast<uint8_t*>(&bins[0][tid]);
+  const auto count = [&](unsigned v) { mine[((v >> 9) & 0x3Fu) * 512u + ((v >> 7) & 3u)]++; };          // exponent = bits 7..14
+  const long r0 = (long)blockIdx.y * HIST_ROWS, r1 = min(p.N, r0 + HIST_ROWS);
+  long r = r0;
+  for (; r + 8 <= r1; r += 8) {                         // eight independent loads in flight per thread
+    unsigned v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = x[(r + i) * p.row_stride];
+#pragma unroll
+    for (int i = 0; i < 8; i++) count(v[i]);
   }
-  if (c < n_ch)
-    for (int b = 0; b < 256; b++) {
-      unsigned v = bins[b * 128 + tid];
-      if (v) atomicAdd(&hist[c * 256 + b], (unsigned long long)v);
+  for (; r < r1; r++) count(x[r * p.row_stride]);
+  Cnt* hist = p.hist[blockIdx.z] + c * 256;
+  for (int w = 0; w < 64; w++) {
+    const u32 four = bins[w][tid];
+    if (four) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) { const u32 n = (four >> (8 * i)) & 0xFFu; if (n) atomicAdd(&hist[4 * w + i], (Cnt)n); }
     }
+  }
 }
 
-// One warp per histogram row: densest 8- and 16-wide window, first maximum wins.
-__global__ void __launch_bounds__(128) bases_from_hist_kernel(const long long* __restrict__ hist, long n_rows, uint8_t* __restrict__ base3, uint8_t* __restrict__ base4) {
-  __shared__ long long cs[4][257];
+// One warp per histogram row: densest 8- and 16-wide window, first maximum wins.  grid y = kind.
+template <class Cnt> struct BasesParams { const Cnt* hist[2]; uint8_t *base3[2], *base4[2]; long n_rows; };
+template <class Cnt>
+__global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_constant__ BasesParams<Cnt> p) {
+  __shared__ Cnt cs[4][257];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long row = (long)blockIdx.x * 4 + warp;
-  if (row >= n_rows) return;
-  long long carry = 0;
+  if (row >= p.n_rows) return;
+  const Cnt* hist = p.hist[blockIdx.y] + row * 256;
+  Cnt carry = 0;
   if (lane == 0) cs[warp][0] = 0;
-  for (int b = 0; b < 256; b += 32) {
-    long long v = hist[row * 256 + b + lane], inc = v;
+  Cnt v[8];
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { long long u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
-    cs[warp][b + lane + 1] = carry + inc;
+  for (int b = 0; b < 8; b++) v[b] = hist[32 * b + lane];
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    Cnt inc = v[b];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { Cnt u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
+    cs[warp][32 * b + lane + 1] = carry + inc;
     carry += __shfl_sync(FULL, inc, 31);
   }
   __syncwarp();
   for (int k = 0; k < 2; k++) {
     const int w = k ? 16 : 8;
-    long long best = -1; int besti = 0;
+    Cnt best = -1; int besti = 0;
     for (int s = lane; s <= 256 - w; s += 32) {
-      long long v = cs[warp][s + w] - cs[warp][s];
+      Cnt v = cs[warp][s + w] - cs[warp][s];
       if (v > best) { best = v; besti = s; }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-      long long ob = __shfl_xor_sync(FULL, best, d); int oi = __shfl_xor_sync(FULL, besti, d);
+      Cnt ob = __shfl_xor_sync(FULL, best, d); int oi = __shfl_xor_sync(FULL, besti, d);
       if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
     }
-    if (lane == 0) (k ? base4 : base3)[row] = (uint8_t)besti;
+    if (lane == 0) (k ? p.base4[blockIdx.y] : p.base3[blockIdx.y])[row] = (uint8_t)besti;
   }
 }
 
@@ -422,22 +444,49 @@ extern "C" int gaac_decode_page(const uint8_t* sm, const uint8_t* codes, const i
   return launch_status();
 }
 
+static dim3 hist_grid(int64_t n_ch, int64_t N, int kinds) { return dim3((unsigned)((n_ch + 127) / 128), (unsigned)((N + HIST_ROWS - 1) / HIST_ROWS), (unsigned)kinds); }
+
 extern "C" int gaac_exponent_hist(const void* x_bf16, int64_t N, int64_t n_ch, long long* hist, void* stream) {
   if (!x_bf16 || !hist || N <= 0 || n_ch <= 0) return GAAC_E_ARG;
-  cudaFuncSetAttribute(exponent_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * 128 * 2);   // per device; cheap
-  dim3 grid((unsigned)((n_ch + 127) / 128), (unsigned)((N + HIST_ROWS - 1) / HIST_ROWS));
-  exponent_hist_kernel<<<grid, 128, 256 * 128 * 2, (cudaStream_t)stream>>>((const uint16_t*)x_bf16, N, n_ch, (unsigned long long*)hist);
+  // the grid's second dimension holds 65535 chunks: longer inputs take several launches
+  constexpr int64_t MOST = 65535LL * HIST_ROWS;
+  for (int64_t r = 0; r < N; r += MOST) {
+    const int64_t rows = std::min(MOST, N - r);
+    const HistParams<unsigned long long> p{{(const uint16_t*)x_bf16 + r * n_ch, nullptr}, {(unsigned long long*)hist, nullptr}, rows, n_ch, n_ch};
+    exponent_hist_kernel<<<hist_grid(n_ch, rows, 1), 128, 0, (cudaStream_t)stream>>>(p);
+  }
   return launch_status();
 }
 
 extern "C" int gaac_bases_from_hist(const long long* hist, int64_t n_rows, uint8_t* base3, uint8_t* base4, void* stream) {
   if (!hist || !base3 || !base4 || n_rows <= 0) return GAAC_E_ARG;
-  bases_from_hist_kernel<<<(unsigned)((n_rows + 3) / 4), 128, 0, (cudaStream_t)stream>>>(hist, n_rows, base3, base4);
+  const BasesParams<long long> p{{hist, nullptr}, {base3, nullptr}, {base4, nullptr}, n_rows};
+  bases_from_hist_kernel<<<(unsigned)((n_rows + 3) / 4), 128, 0, (cudaStream_t)stream>>>(p);
   return launch_status();
 }
 
 // ---------------------------------------------------------------------------------------------- slot cache: whole-prompt prefill
 constexpr int CACHE_READ_PAD = 8;      // bytes kept free behind a head's escape bytes (the readers may touch them)
+
+extern "C" size_t gaac_cache_calibrate_scratch_bytes(int n_kv) { return 2 * (size_t)(n_kv > 0 ? n_kv : 0) * D * 256 * sizeof(int32_t); }
+
+extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
+                                    int n_base_rows, uint8_t* scratch, size_t scratch_bytes, void* stream) {
+  if (!K || !V || !K->base3 || !K->base4 || !V->base3 || !V->base4 || !k_tok || !v_tok || !scratch) return GAAC_E_ARG;
+  if (L <= 0 || L > 65535LL * HIST_ROWS || row_stride < (int64_t)n_kv * D || slot < 0 || n_kv <= 0 || n_kv > 256 || n_base_rows < (slot + 1) * n_kv) return GAAC_E_ARG;
+  if (scratch_bytes < gaac_cache_calibrate_scratch_bytes(n_kv)) return GAAC_E_ARG;
+  if (reinterpret_cast<uintptr_t>(scratch) & 3) return GAAC_E_ALIGN;
+  cudaStream_t st = (cudaStream_t)stream;
+  const long n_ch = (long)n_kv * D, at = (long)slot * n_ch;
+  int* hist = reinterpret_cast<int*>(scratch);
+  cudaMemsetAsync(hist, 0, gaac_cache_calibrate_scratch_bytes(n_kv), st);
+  const HistParams<int> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + n_ch * 256}, L, n_ch, row_stride};
+  exponent_hist_kernel<<<hist_grid(n_ch, L, 2), 128, 0, st>>>(hp);
+  const BasesParams<int> bp{{hist, hist + n_ch * 256}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
+                            {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch};
+  bases_from_hist_kernel<<<dim3((unsigned)((n_ch + 3) / 4), 2), 128, 0, st>>>(bp);
+  return launch_status();
+}
 
 extern "C" size_t gaac_cache_prefill_scratch_bytes(int64_t L, int n_kv) {
   const size_t items = (size_t)(L > 0 ? L / T : 0) * (size_t)(n_kv > 0 ? n_kv : 0);

@@ -15,7 +15,7 @@ read them; the device work goes through libgaac_b200.so.
 from __future__ import annotations
 import torch
 from . import _lib
-from .codec import Codec, Page, D, T, CB, bases_from_hist, exponent_hist
+from .codec import Codec, Page, D, T, CB
 from .encoder import TileEncoder
 from .kernel import _ext, choose_nsplit, choose_nsplit_sm100
 
@@ -124,10 +124,13 @@ class CompressedKVCache:
         assert 0 <= slot < self.n_slots
         hs = self._heads(slot)
         k, v = self._token_rows(k), self._token_rows(v)
+        if _lib.row_stride(k) != _lib.row_stride(v):                                               # the library reads both with one stride
+            k, v = k.contiguous(), v.contiguous()
         if self.per_sequence_bases and L:
-            for st, x in ((self.k, k), (self.v, v)):
-                rows = x if x.is_contiguous() else x.contiguous()                                 # the histogram reads [L, n_kv * 128] rows
-                st.base3[hs], st.base4[hs] = bases_from_hist(exponent_hist(rows, self.n_kv), self.n_kv)
+            lib = _lib.lib()
+            hist = torch.empty(lib.gaac_cache_calibrate_scratch_bytes(self.n_kv), dtype=torch.uint8, device=k.device)
+            _lib.check(lib.gaac_cache_calibrate(self.k.c_store(), self.v.c_store(), k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.k.base3.shape[0],
+                                                hist.data_ptr(), hist.numel(), _lib.stream_ptr(k.device)), "gaac_cache_calibrate")
         need = _lib.lib().gaac_cache_prefill_scratch_bytes(L, self.n_kv)
         if check:
             self.settle_prefills()

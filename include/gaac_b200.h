@@ -254,6 +254,13 @@ typedef struct {
 int gaac_append_kv(const gaac_store* K, const gaac_store* V, const void* k_new, const void* v_new, const int32_t* slot, int B, int n_kv,
                    int32_t* tail_len, int32_t* seq_len, int64_t S_cap, int64_t ovf_cap, int n_base_rows, int32_t* err, void* stream);
 
+/* Exponent bases of one slot from its own prompt: histogram and densest windows of K and V [L, n_kv, 128] (rows row_stride elements
+ * apart) go to rows slot*n_kv .. of the base tables of K and V, which hold n_base_rows rows (one per cache head).  scratch:
+ * gaac_cache_calibrate_scratch_bytes(n_kv) bytes, 4-byte aligned.  Replaces the calibration of CompressedKVCache.prefill (gaac/kv_cache.py:149-169, gaac/codec.py:70-84). */
+size_t gaac_cache_calibrate_scratch_bytes(int n_kv);
+int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
+                         int n_base_rows, uint8_t* scratch, size_t scratch_bytes, void* stream);
+
 /* A whole prompt into one slot: k_tok / v_tok = the prompt's K and V as the model produces them, token-major: head h of token t
  * at x + t*row_stride + h*128 (bf16 elements; row_stride >= n_kv*128, rows 16-byte aligned), L tokens (L <= S_cap).  The
  * floor(L/16) whole tiles of every head of the slot are compressed straight into the store (tile 0 upward, the head's escape
