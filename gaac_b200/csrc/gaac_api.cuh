@@ -7,4 +7,22 @@
 namespace gaac {
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? GAAC_OK : GAAC_E_LAUNCH; }
+
+// ---- programmatic dependent launch.  A kernel launched with launch_overlapped may become resident while the kernel before it in the stream is still
+// running, once every block of that one has executed griddep_launch() or exited; it begins with griddep_wait(), which returns when that
+// kernel has completed and its writes are visible, and touches no memory before.  Behind an ordinary kernel, and with the switch off, all of
+// this does nothing.  It takes a launch's latency (1-2 us) off chains of short kernels.
+inline int g_launch_overlap = 1;      // see gaac_set_launch_overlap
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::); }
+template <class... Params, class... Args>
+int launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
+  return launch_status();
+}
 }  // namespace gaac

@@ -808,9 +808,6 @@ static int carve_workspace(void* ws, size_t ws_bytes, int B, int n_q, int nsplit
   return GAAC_OK;
 }
 
-// Programmatic dependent launch of the attention and merge kernels (see gaac_set_launch_overlap); on unless switched off.
-static int g_launch_overlap = 1;
-
 static void launch_row_order(const int* seq_lens, const int* slot, int n_kv, int B, int2* order, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(1); cfg.blockDim = dim3(ORDER_MAX_ROWS); cfg.stream = st;

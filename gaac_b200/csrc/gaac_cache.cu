@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(64) append_kv_kernel(const __grid_constant__ A
   __shared__ __align__(16) WarpScratch scratch[2];
   __shared__ int s_fit[2];
   const int i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  griddep_launch();                                   // the step's attention may set up its tables meanwhile
   const int sl = p.slot[i / p.n_kv];
   if (sl < 0) return;
   const long h = (long)sl * p.n_kv + i % p.n_kv;
@@ -142,11 +143,14 @@ __device__ __forceinline__ void store_one(WarpScratch& ws, const PagedParams& p,
 __global__ void __launch_bounds__(32) paged_store_kernel(const __grid_constant__ PagedParams p) {
   __shared__ __align__(16) WarpScratch ws;
   const int e = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
+  griddep_launch();
   if (t & 1) store_one<1>(ws, p, e, t, lane); else store_one<0>(ws, p, e, t, lane);
 }
 
 __global__ void __launch_bounds__(256) free_tiles_kernel(const int* __restrict__ freeq, int n_items, int* __restrict__ stack, int* __restrict__ top) {
   const int i = blockIdx.x * 256 + threadIdx.x;
+  griddep_wait();
+  griddep_launch();
   if (i >= n_items) return;
   const int r = freeq[i];
   if (r >= 0) { const int idx = atomicAdd(top, 1); stack[idx] = r; }
@@ -237,8 +241,8 @@ extern "C" int gaac_paged_store(const gaac_paged* st, const void* key, const voi
   cudaStream_t s = (cudaStream_t)stream;
   paged_store_kernel<<<dim3((unsigned)E, (unsigned)(2 * st->n_kv)), 32, 0, s>>>(p);
   const int n = E * 2 * st->n_kv;
-  free_tiles_kernel<<<(n + 255) / 256, 256, 0, s>>>(freeq, n, st->stack, st->top);
-  return launch_status();
+  if (int err = launch_status()) return err;
+  return launch_overlapped(free_tiles_kernel, dim3((n + 255) / 256), 256, s, freeq, n, st->stack, st->top);
 }
 
 extern "C" int gaac_paged_release(const gaac_paged* st, const int32_t* blocks, int F, void* stream) {

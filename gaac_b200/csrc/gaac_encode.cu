@@ -65,6 +65,7 @@ template <int KIND>
 __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(const __grid_constant__ EncodeParams p) {
   __shared__ __align__(16) WarpScratch scratch[2][ENC_WARPS];       // two per warp: the next tile's rows arrive while this one is encoded
   __shared__ __align__(16) uint8_t esc_stage[ENC_WARPS][TILE_MAX_ESC];
+  griddep_launch();
   const bool v = KIND == 2 ? blockIdx.z != 0 : KIND == 1;
   if (KIND != 0 && v) encode_tiles_cta<1>(p, p.side[KIND == 2 ? 1 : 0], scratch, esc_stage[threadIdx.x >> 5]);
   if (KIND != 1 && !v) encode_tiles_cta<0>(p, p.side[0], scratch, esc_stage[threadIdx.x >> 5]);
@@ -72,10 +73,25 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(const __gr
 static dim3 encode_grid(int ntiles, int64_t H, int kinds) { return dim3((ntiles + ENC_WARPS * ENC_TILES_PER_WARP - 1) / (ENC_WARPS * ENC_TILES_PER_WARP), (unsigned)H, (unsigned)kinds); }
 
 // head_start[0..H] = exclusive prefix of head_bytes, by one CTA of SCAN_THREADS threads (H is the number of cache heads).
-__device__ __forceinline__ void head_prefix(const int* head_bytes, int H, int* head_start) {
+// total: optional, the sum once more (page-locked host memory, which the end of the kernel makes visible).
+__device__ __forceinline__ void head_prefix(const int* head_bytes, int H, int* head_start, int* total) {
   __shared__ int hsum[32];
   __shared__ int hcarry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (H <= 64) {                                     // the usual case: one warp, no barriers
+    if (warp) return;
+    int carry = 0;
+    for (int base = 0; base < H; base += 32) {
+      int inc = base + lane < H ? __ldcg(head_bytes + base + lane) : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) { int u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
+      if (base + lane < H) head_start[base + lane + 1] = carry + inc;
+      carry += __shfl_sync(FULL, inc, 31);
+    }
+    if (lane == 0) head_start[0] = 0;
+    if (total && lane == 0) *(volatile int*)total = carry;
+    return;
+  }
   if (tid == 0) { hcarry = 0; head_start[0] = 0; }
   __syncthreads();
   for (int base = 0; base < H; base += blockDim.x) {
@@ -92,6 +108,7 @@ __device__ __forceinline__ void head_prefix(const int* head_bytes, int H, int* h
     if (tid == (int)blockDim.x - 1) hcarry = before + inc;
     __syncthreads();
   }
+  if (total && tid == 0) *(volatile int*)total = hcarry;
 }
 
 // Exclusive prefix of tile_bytes per head.  One CTA of 1024 threads per (head, kind), four tiles per thread and pass: a 64K-token
@@ -112,6 +129,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) tile_scan_kernel(const __grid_co
   const long h = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) carry_s = 0;
+  griddep_wait();
+  griddep_launch();
   __syncthreads();
   for (int base = 0; base < ntiles; base += 4 * SCAN_THREADS) {
     const int i0 = base + 4 * tid;
@@ -151,14 +170,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) tile_scan_kernel(const __grid_co
   __syncthreads();
   if (!last) return;
   __threadfence();
-  head_prefix(head_bytes, H, p.head_start);
-  if (tid == 0 && p.total) {
-    *(volatile int*)p.total = p.head_start[H];
-    __threadfence_system();
-  }
+  head_prefix(head_bytes, H, p.head_start, p.total);
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) head_prefix_kernel(const int* __restrict__ head_bytes, int H, int* __restrict__ head_start) { head_prefix(head_bytes, H, head_start); }
+__global__ void __launch_bounds__(SCAN_THREADS) head_prefix_kernel(const int* __restrict__ head_bytes, int H, int* __restrict__ head_start) { head_prefix(head_bytes, H, head_start, nullptr); }
 
 // What one kind's compaction reads and writes.
 struct CompactSide { const uint8_t* slots; const int *tile_bytes, *tile_off, *head_start; uint8_t* ovf; const int* flags; int* ovf_off; int* status; };
@@ -169,17 +184,16 @@ struct CompactParams {
   CompactSide side[2]; int ntiles; unsigned n_items; long tile_off_stride, head_stride, S, S_pad; int zero_pad; long ovf_cap, head_cap;
   int finish; FinishParams fin;
 };
-__device__ void prefill_finish(const FinishParams& p);
+__device__ void prefill_finish(const FinishParams& p, int h, int kind);
 
 // Escape bytes of every tile: slot -> ovf[head_start[h] + tile_off[h, tile]]; optionally the per-row escape offsets
 // ovf_off[h, row] = tile_off[h, tile] + (escape bytes of the tile's earlier rows), recomputed from the tag words.
 // Eight lanes per tile: a tile has some 55 escape bytes and 16 tag words, and what the kernel waits for are its loads (sizes and offsets, then the
 // bytes), so a warp keeps four tiles in flight.  grid y = kind.
 __global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant__ CompactParams p) {
-  if (p.finish && blockIdx.x == gridDim.x - 1) {     // one more block: the rest of a prompt's prefill
-    if (blockIdx.y == 0) prefill_finish(p.fin);
-    return;
-  }
+  griddep_wait();
+  const unsigned copies = (p.n_items + 15) / 16;
+  if (blockIdx.x >= copies) { prefill_finish(p.fin, blockIdx.x - copies, blockIdx.y); return; }       // the rest of a prompt's prefill
   const CompactSide& s = p.side[blockIdx.y];
   const int lane = threadIdx.x & 31, q = lane & 7;
   const unsigned first = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 4, item = first + (lane >> 3);
@@ -213,7 +227,7 @@ __global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant
     if (live && row + 1 < p.S) o[1] = toff + inc - s1;
   }
 }
-static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_items + 15) / 16 + (p.finish ? 1 : 0), (unsigned)kinds); }
+static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_items + 15) / 16 + (p.finish ? p.fin.n_kv : 0), (unsigned)kinds); }
 
 // One warp per (head, tile): compressed tile -> bf16 rows.
 template <int KIND_V>
@@ -240,38 +254,42 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) decode_page_kernel(
   }
 }
 
-// Exponent histogram: x [N rows, n_ch] bf16, row r at x + r * row_stride; hist [n_ch, 256] counts.  grid = (ceil(n_ch/128), row chunks, kinds); a
-// thread owns one channel and a private 256-bin histogram of 8-bit counters in shared memory, flushed with atomics.  Counter (bin, channel) is
-// byte bin & 3 of word [bin >> 2][channel]: a warp's increments go to 32 banks whatever the exponents are, the table is cleared with 16-byte stores,
-// and the flush reads four bins at a time, nearly all of them empty.  16-bit counters by bin (64 KB, three CTAs per SM, 512 single stores and loads per
-// thread to clear and flush them for 64 rows) took most of the kernel's time.
-constexpr int HIST_ROWS = 128;        // rows per CTA (8-bit counters); twice the rows of one flush, and still 500 CTAs on a 4000-token prompt of 8 kv heads
+// Exponent histogram: x [N rows, n_ch] bf16, row r at x + r * row_stride; hist [n_ch, 256] counts.  grid = (ceil(n_ch/128), row chunks, kinds).  A CTA
+// counts 128 channels in shared memory with 8-bit counters, four threads per channel, and flushes what is not zero with atomics.  Counter (bin,
+// channel) is byte bin & 3 of word [bin >> 2][channel]: a warp's increments go to 32 banks whatever the exponents are, and clearing and flushing handle
+// four bins at a time, nearly all of them empty.  Bound by latency, not by bytes: with one thread per channel and a load, add and store per
+// value it took 21 us for 2048 rows of 8 kv heads (15 us with 16-bit counters and chunks of 64 rows), now 7 us: the shared-memory atomic returns
+// nothing, so a thread never waits for a counter.
+constexpr int HIST_ROWS = 128, HIST_LANES = 4;         // rows per CTA (an 8-bit counter holds 255); threads per channel
 template <class Cnt> struct HistParams { const uint16_t* x[2]; Cnt* hist[2]; long N, n_ch, row_stride; };
 template <class Cnt>
-__global__ void __launch_bounds__(128) exponent_hist_kernel(const __grid_constant__ HistParams<Cnt> p) {
+__global__ void __launch_bounds__(128 * HIST_LANES) exponent_hist_kernel(const __grid_constant__ HistParams<Cnt> p) {
   __shared__ __align__(16) u32 bins[64][128];
-  const int tid = threadIdx.x;
-  const long c = (long)blockIdx.x * 128 + tid;
+  const int ch = threadIdx.x & 127, sub = threadIdx.x >> 7;
+  const long c = (long)blockIdx.x * 128 + ch;
+  for (int i = threadIdx.x; i < 64 * 128 / 4; i += 128 * HIST_LANES) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
+  griddep_launch();
+  __syncthreads();
+  if (c < p.n_ch) {
+    const uint16_t* x = p.x[blockIdx.z] + c;
+    const auto count = [&](u32 v) { atomicAdd(&bins[(v >> 9) & 0x3Fu][ch], 1u << (8u * ((v >> 7) & 3u))); };          // exponent = bits 7..14
+    const long r1 = min(p.N, ((long)blockIdx.y + 1) * HIST_ROWS);
+    long r = (long)blockIdx.y * HIST_ROWS + sub;
+    for (; r + 15 * HIST_LANES < r1; r += 16 * HIST_LANES) {          // sixteen independent loads in flight per thread
+      u32 v[16];
 #pragma unroll
-  for (int i = 0; i < 16; i++) reinterpret_cast<uint4*>(bins)[i * 128 + tid] = make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < 16; i++) v[i] = x[(r + i * HIST_LANES) * p.row_stride];
+#pragma unroll
+      for (int i = 0; i < 16; i++) count(v[i]);
+    }
+    for (; r < r1; r += HIST_LANES) count(x[r * p.row_stride]);
+  }
   __syncthreads();
   if (c >= p.n_ch) return;
-  const uint16_t* x = p.x[blockIdx.z] + c;
-  uint8_t* mine = reinterpret_cast<uint8_t*>(&bins[0][tid]);
-  const auto count = [&](unsigned v) { mine[((v >> 9) & 0x3Fu) * 512u + ((v >> 7) & 3u)]++; };          // exponent = bits 7..14
-  const long r0 = (long)blockIdx.y * HIST_ROWS, r1 = min(p.N, r0 + HIST_ROWS);
-  long r = r0;
-  for (; r + 8 <= r1; r += 8) {                         // eight independent loads in flight per thread
-    unsigned v[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = x[(r + i) * p.row_stride];
-#pragma unroll
-    for (int i = 0; i < 8; i++) count(v[i]);
-  }
-  for (; r < r1; r++) count(x[r * p.row_stride]);
   Cnt* hist = p.hist[blockIdx.z] + c * 256;
-  for (int w = 0; w < 64; w++) {
-    const u32 four = bins[w][tid];
+#pragma unroll 8
+  for (int w = sub; w < 64; w += HIST_LANES) {
+    const u32 four = bins[w][ch];
     if (four) {
 #pragma unroll
       for (int i = 0; i < 4; i++) { const u32 n = (four >> (8 * i)) & 0xFFu; if (n) atomicAdd(&hist[4 * w + i], (Cnt)n); }
@@ -288,6 +306,7 @@ __global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_const
   const long row = (long)blockIdx.x * 4 + warp;
   if (row >= p.n_rows) return;
   const Cnt* hist = p.hist[blockIdx.y] + row * 256;
+  griddep_wait();
   Cnt carry = 0;
   if (lane == 0) cs[warp][0] = 0;
   Cnt v[8];
@@ -318,32 +337,34 @@ __global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_const
   }
 }
 
-// Last step of a slot's prefill (one CTA): the prompt's remainder (L mod 16 rows) goes into the raw tails of the slot's heads,
-// the heads' token counters are set, and the largest escape stream of the slot per kind is reported for the host's capacity
-// check.  k_tok / v_tok: token-major rows, head h of token t at t * row_stride + h * 128 (bf16 elements).
-__device__ void prefill_finish(const FinishParams& p) {
-  const long n_full = p.L / T * T;
+// Last step of a slot's prefill, one CTA of 128 threads per (head, kind): the prompt's remainder (L mod 16 rows) goes into the head's raw tail
+// (two 16-byte pieces per thread: one CTA for all of them took 16 us for 15 rows of 8 heads), the head's token counters are set, and the largest
+// escape stream of the slot per kind is reported for the host's capacity check.  k_tok / v_tok: token-major rows, head h of token t at
+// t * row_stride + h * 128 (bf16 elements).
+__device__ void prefill_finish(const FinishParams& p, int h, int kind) {
+  const long n_full = p.L / T * T, head = p.h0 + h;
   const int rem = (int)(p.L - n_full), tid = threadIdx.x;
-  const int per_kind = rem * p.n_kv * 16;                            // 16-byte pieces
-  for (int i = tid; i < 2 * per_kind; i += blockDim.x) {
-    const int kind = i >= per_kind, j = i - kind * per_kind;
-    const int r = j / (p.n_kv * 16), h = (j >> 4) % p.n_kv, c = j & 15;
-    const uint16_t* src = (kind ? p.v_tok : p.k_tok) + (n_full + r) * p.row_stride + h * D + c * 8;
-    uint16_t* dst = (kind ? p.vtail : p.ktail) + ((p.h0 + h) * T + r) * D + c * 8;
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-  }
-  for (int h = tid; h < p.n_kv; h += blockDim.x) {
-    p.seq_len[p.h0 + h] = (int)n_full; p.tail_len[p.h0 + h] = rem;
-    if (n_full == 0) { p.used_k[p.h0 + h] = 0; p.used_v[p.h0 + h] = 0; }
-  }
+  const uint16_t* src = (kind ? p.v_tok : p.k_tok) + n_full * p.row_stride + h * D;
+  uint16_t* dst = (kind ? p.vtail : p.ktail) + head * T * D;
+#pragma unroll
+  for (int i = tid; i < T * 16; i += 128)
+    if ((i >> 4) < rem) *reinterpret_cast<uint4*>(dst + i * 8) = *reinterpret_cast<const uint4*>(src + (i >> 4) * p.row_stride + (i & 15) * 8);
+  int* used = kind ? p.used_v : p.used_k;
   if (tid == 0) {
-    int mk = 0, mv = 0;
-    if (n_full) for (int h = 0; h < p.n_kv; h++) { mk = max(mk, p.used_k[p.h0 + h]); mv = max(mv, p.used_v[p.h0 + h]); }
-    p.status[1] = mk; p.status[3] = mv;
-    if (n_full == 0) { p.status[0] = 0; p.status[2] = 0; }           // no copy in front of this step
+    if (kind == 0) { p.seq_len[head] = (int)n_full; p.tail_len[head] = rem; }
+    if (n_full == 0) used[head] = 0;
+  }
+  if (h == 0 && tid < 32) {
+    int m = 0;
+    if (n_full) for (int i = tid; i < p.n_kv; i += 32) m = max(m, used[p.h0 + i]);
+    m = __reduce_max_sync(FULL, m);
+    if (tid == 0) {
+      p.status[2 * kind + 1] = m;
+      if (n_full == 0) p.status[2 * kind] = 0;       // no copy in front of this step
+    }
   }
 }
-__global__ void __launch_bounds__(128) prefill_finish_kernel(const __grid_constant__ FinishParams p) { prefill_finish(p); }
+__global__ void __launch_bounds__(128) prefill_finish_kernel(const __grid_constant__ FinishParams p) { prefill_finish(p, blockIdx.x, blockIdx.y); }
 
 }  // namespace gaac
 
@@ -375,8 +396,7 @@ extern "C" int gaac_compact(const uint8_t* slots, const int32_t* tile_bytes, int
   if (!tile_bytes || !tile_off || H <= 0 || ntiles <= 0 || tile_off_stride < ntiles) return GAAC_E_ARG;
   if (head_start && (!ovf || !slots)) return GAAC_E_ARG;
   if (ovf_off && (!head_start || !flags || S <= 0 || S_pad < S)) return GAAC_E_ARG;
-  const ScanParams sp{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, tile_off_stride, nullptr, nullptr};
-  tile_scan_kernel<<<(unsigned)H, SCAN_THREADS, 0, (cudaStream_t)stream>>>(sp);
+  if (int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, tile_off_stride, nullptr, nullptr})) return e;
   if (head_start) return gaac_compact_copy(slots, tile_bytes, H, ntiles, head_start, ovf, tile_off, tile_off_stride, flags, S, S_pad, ovf_off, 0, 0, 0, nullptr, stream);
   return launch_status();
 }
@@ -387,9 +407,7 @@ static int encode_begin(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, 
   if (!tile_off || !head_bytes || !head_start) return GAAC_E_ARG;
   if (int e = encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, head_start + H, stream)) return e;
   const int64_t ntiles = (S + T - 1) / T;
-  const ScanParams sp{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, total};
-  tile_scan_kernel<<<(unsigned)H, SCAN_THREADS, 0, (cudaStream_t)stream>>>(sp);
-  return launch_status();
+  return launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, total});
 }
 
 extern "C" int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
@@ -418,8 +436,7 @@ extern "C" int gaac_compact_copy(const uint8_t* slots, const int32_t* tile_bytes
   p.side[0] = CompactSide{slots, tile_bytes, tile_off, head_start, ovf, flags, ovf_off, status};
   p.ntiles = (int)ntiles; p.n_items = (unsigned)(H * ntiles); p.tile_off_stride = tile_off_stride; p.S = S; p.S_pad = S_pad;
   p.zero_pad = zero_pad; p.ovf_cap = ovf_cap; p.head_cap = head_cap;
-  compact_copy_kernel<<<compact_grid(p, 1), 128, 0, (cudaStream_t)stream>>>(p);
-  return launch_status();
+  return launch_overlapped(compact_copy_kernel, compact_grid(p, 1), 128, (cudaStream_t)stream, p);
 }
 
 extern "C" int gaac_head_prefix(const int32_t* head_bytes, int64_t H, int32_t* head_start, void* stream) {
@@ -453,7 +470,7 @@ extern "C" int gaac_exponent_hist(const void* x_bf16, int64_t N, int64_t n_ch, l
   for (int64_t r = 0; r < N; r += MOST) {
     const int64_t rows = std::min(MOST, N - r);
     const HistParams<unsigned long long> p{{(const uint16_t*)x_bf16 + r * n_ch, nullptr}, {(unsigned long long*)hist, nullptr}, rows, n_ch, n_ch};
-    exponent_hist_kernel<<<hist_grid(n_ch, rows, 1), 128, 0, (cudaStream_t)stream>>>(p);
+    exponent_hist_kernel<<<hist_grid(n_ch, rows, 1), 128 * HIST_LANES, 0, (cudaStream_t)stream>>>(p);
   }
   return launch_status();
 }
@@ -461,8 +478,7 @@ extern "C" int gaac_exponent_hist(const void* x_bf16, int64_t N, int64_t n_ch, l
 extern "C" int gaac_bases_from_hist(const long long* hist, int64_t n_rows, uint8_t* base3, uint8_t* base4, void* stream) {
   if (!hist || !base3 || !base4 || n_rows <= 0) return GAAC_E_ARG;
   const BasesParams<long long> p{{hist, nullptr}, {base3, nullptr}, {base4, nullptr}, n_rows};
-  bases_from_hist_kernel<<<(unsigned)((n_rows + 3) / 4), 128, 0, (cudaStream_t)stream>>>(p);
-  return launch_status();
+  return launch_overlapped(bases_from_hist_kernel<long long>, dim3((unsigned)((n_rows + 3) / 4)), 128, (cudaStream_t)stream, p);
 }
 
 // ---------------------------------------------------------------------------------------------- slot cache: whole-prompt prefill
@@ -481,11 +497,10 @@ extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, co
   int* hist = reinterpret_cast<int*>(scratch);
   cudaMemsetAsync(hist, 0, gaac_cache_calibrate_scratch_bytes(n_kv), st);
   const HistParams<int> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + n_ch * 256}, L, n_ch, row_stride};
-  exponent_hist_kernel<<<hist_grid(n_ch, L, 2), 128, 0, st>>>(hp);
+  exponent_hist_kernel<<<hist_grid(n_ch, L, 2), 128 * HIST_LANES, 0, st>>>(hp);
   const BasesParams<int> bp{{hist, hist + n_ch * 256}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
                             {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch};
-  bases_from_hist_kernel<<<dim3((unsigned)((n_ch + 3) / 4), 2), 128, 0, st>>>(bp);
-  return launch_status();
+  return launch_overlapped(bases_from_hist_kernel<int>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
 }
 
 extern "C" size_t gaac_cache_prefill_scratch_bytes(int64_t L, int n_kv) {
@@ -514,7 +529,7 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   const FinishParams fin{(const uint16_t*)k_tok, (const uint16_t*)v_tok, row_stride, L, n_kv, h0, (uint16_t*)K->tail, (uint16_t*)V->tail, seq_len, tail_len, K->ovf_used, V->ovf_used, status};
   if (ntiles == 0) {
     if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
-    else prefill_finish_kernel<<<1, 128, 0, st>>>(fin);
+    else prefill_finish_kernel<<<dim3((unsigned)n_kv, 2), 128, 0, st>>>(fin);
     return launch_status();
   }
   // Three launches for both kinds: encode, offsets, copy (whose last block does the tails and counters); the encode clears the words that the
@@ -539,8 +554,7 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
   else {
     encode_tiles_kernel<2><<<encode_grid(ntiles, n_kv, 2), ENC_WARPS * 32, 0, st>>>(ep);
-    tile_scan_kernel<<<dim3((unsigned)n_kv, 2), SCAN_THREADS, 0, st>>>(sp);
+    if (int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)n_kv, 2), SCAN_THREADS, st, sp)) return e;
   }
-  compact_copy_kernel<<<compact_grid(cp, 2), 128, 0, st>>>(cp);
-  return launch_status();
+  return launch_overlapped(compact_copy_kernel, compact_grid(cp, 2), 128, st, cp);
 }

@@ -91,7 +91,7 @@ __device__ __forceinline__ void join_codes(u32 c0, u32 c1, u32 c2, u32 c3, u32* 
 // every lane holds its share in `lt` and the tile's escape byte count is returned (same in all lanes).
 // Bound by instruction issue: 16-bit loads one by one, a byte-exact subtraction per window, a table of tags in shared memory and a branch per
 // escape byte made 1205 warp instructions per tile; now the fragments come in by ldmatrix, a window is one subtraction per word and the
-// positions of the escape bytes come from one warp scan.
+// positions of the escape bytes come from one warp scan.  [8, 65536, 128]: 60 (K) / 66 us (V) -> 39 / 41, that is 5.9 / 5.6 TB/s of input and output.
 template <int KIND_V>
 __device__ __forceinline__ int encode_tile_warp(WarpScratch& ws, int nvalid, const u32* b3w, const u32* b4w, int lane, LaneTile& lt) {
   const int j = lane & 3, r = lane >> 2;
