@@ -61,6 +61,9 @@ struct AttnParams {
   const uint16_t* q; int B, n_q, n_kv, G; float scale_log2; int nsplit;
   int* counters; int* err; float* pm; float* pl; float* pa;     // err: set to 1 when a bounded wait inside the kernel ran out
   uint16_t* out; float* out_f32; float* part;
+  // balanced launches (units > 0; grid = (n_kv, units)): the rows share `units` ranges per kv head by their lengths, see row_share; nsplit is then the most
+  // that one row can get and only the stride of the partials
+  int units;
   // cross-GPU exchange (x_recv == NULL: unused): the partial of every query head is stored into every rank's receive
   // buffer, then this rank's arrival flag of the (row, kv head) group on every rank is set to the exchange number; with
   // x_fused the same CTA then waits (bounded) for the other ranks' flags, merges all ranks' rows and writes the output
@@ -128,17 +131,20 @@ __device__ __forceinline__ bool last_split(int* counter, int NS, int* s_last) {
 // another (no per-split dependent chain): scale factors first, then the weighted sum with one warp per split and 16-byte loads, then a
 // cross-warp sum in shared memory.
 template <int HMAX, class F>
-__device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area, long row0, int heads, const F& deliver) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, NS = p.nsplit;
+__device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area, long row0, int heads, int NS, const F& deliver) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, LD = p.nsplit;      // NS splits of LD places per head
   float* c_f = reinterpret_cast<float*>(area);        // [heads][NS]  m, then exp2(m - M)
   float* c_l = c_f + 8 * NS;                          // [heads][NS]  l
   float* c_ML = c_l + 8 * NS;                         // [8][2]       M, L per head
   float* c_red = c_ML + 16;                           // [W][8][128]  (NS <= 1024 keeps this inside the ring area)
-  for (int i = tid; i < heads * NS; i += ATT_THREADS) { c_f[i] = __ldcg(p.pm + row0 * NS + i); c_l[i] = __ldcg(p.pl + row0 * NS + i); }
+  for (int i = tid; i < heads * NS; i += ATT_THREADS) {
+    const long at = row0 * LD + (LD == NS ? i : i / NS * LD + i % NS);
+    c_f[i] = __ldcg(p.pm + at); c_l[i] = __ldcg(p.pl + at);
+  }
   float4 acc[HMAX];                                   // split `warp` of every head, in flight while M and L are computed
 #pragma unroll
   for (int g = 0; g < HMAX; g++)
-    acc[g] = (g < heads && warp < NS) ? __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * NS + warp) * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    acc[g] = (g < heads && warp < NS) ? __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * LD + warp) * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
   if (warp < heads) {
     float M = -CUDART_INF_F;
@@ -165,7 +171,7 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area,
 #pragma unroll
     for (int g = 0; g < HMAX; g++) {
       if (g < heads) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * NS + s2) * D) + lane);
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * LD + s2) * D) + lane);
         const float f = c_f[g * NS + s2];
         acc[g].x += v.x * f; acc[g].y += v.y * f; acc[g].z += v.z * f; acc[g].w += v.w * f;
       }
@@ -184,10 +190,32 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area,
   }
 }
 
-template <bool PAGED, bool DUMP, int NSET>
+// Balanced launches: lane = batch row, tiles = the row's tiles.  Every row gets ceil(tiles / C) ranges (at least one, so that an empty row is written
+// too), with the smallest C of at least SHARE_MIN_TILES for which all of them fit into `units`; a few steps of bisection between the bounds
+// total / units and total / (units - rows), which always fits.  Unit u then is range `split` of NS of row `row`; row >= 32: nothing to do.
+// A ragged batch split alike for every row waits for its longest row.
+constexpr int SHARE_MAX_ROWS = 32, SHARE_MIN_TILES = 4;
+__device__ __forceinline__ void row_share(int tiles, int B, int units, int u, int lane, int& row, int& split, int& NS) {
+  const unsigned n = lane < B ? (unsigned)tiles : 0u, total = __reduce_add_sync(FULLM, n), most = __reduce_max_sync(FULLM, n);
+  unsigned lo = max((unsigned)SHARE_MIN_TILES, (total + units - 1) / units);
+  unsigned hi = max(lo, units > B ? (total + (units - B) - 1) / (units - B) : most);
+  for (int it = 0; it < 6 && lo < hi; it++) {
+    const unsigned mid = (lo + hi) >> 1, want = lane < B ? max(1u, (n + mid - 1) / mid) : 0u;
+    if (__reduce_add_sync(FULLM, want) <= (unsigned)units) hi = mid; else lo = mid + 1;
+  }
+  const int ns = lane < B ? (int)max(1u, (n + hi - 1) / hi) : 0;
+  u32 inc = (u32)ns;
+  scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8); scan_step(inc, 16);
+  row = popc(__ballot_sync(FULLM, (int)inc <= u));
+  NS = __shfl_sync(FULLM, ns, row & 31);
+  split = u - ((int)__shfl_sync(FULLM, inc, row & 31) - NS);
+}
+
+// SHARE: a balanced launch (its own instantiation: the shares cost the other one registers that the main loop has none of, 1.5 % at 64K tokens)
+template <bool PAGED, bool DUMP, int NSET, bool SHARE>
 __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int s_next, s_last;
+  __shared__ int s_next, s_last, s_split, s_ns;        // (the last two are not needed inside the main loop, whose registers are all taken)
   const int tid = threadIdx.x, lane = tid & 31, j = lane & 3, r = lane >> 2;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
@@ -211,8 +239,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // Which (row, kv head, split) this CTA works on.  Normally the grid says so.  With a row order (ragged paged batches) the CTAs
   // are numbered in the order the hardware hands them out (x fastest) and that number walks the rows from the longest to the
   // shortest, all CTAs of a row together: the big CTAs start first and the small ones fill the SMs at the end.
-  int bh = blockIdx.x, split = blockIdx.y, S_paged = 0;
-  if (PAGED) {
+  int bh = blockIdx.x, split0 = blockIdx.y, S_paged = 0, ns0 = p.nsplit;
+  if (SHARE) {
+    int len = 0, row;
+    if (lane < p.B) {
+      if (PAGED) len = p.seq_len[lane];
+      else { const int sl = p.slot[lane]; len = sl < 0 ? 0 : p.seq_len[(long)sl * p.n_kv]; }        // a slot's first head stands for all of its heads
+    }
+    row_share((len + 15) >> 4, p.B, p.units, blockIdx.y, lane, row, split0, ns0);
+    if (row >= p.B) return;
+    bh = row * p.n_kv + blockIdx.x;
+    S_paged = __shfl_sync(FULLM, len, row);
+  } else if (PAGED) {
     // the row's token count for the grid's own numbering; the loads of the row order travel at the same time, so a batch whose
     // order is not used pays no extra latency for having one
     S_paged = p.seq_len[bh / p.n_kv];
@@ -220,9 +258,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       const int linear = blockIdx.y * gridDim.x + blockIdx.x, per_row = p.n_kv * p.nsplit;
       const int rr = linear / per_row, rem = linear - rr * per_row;
       const int2 e = p.row_order[rr], use = p.row_order[p.B];
-      if (use.x) { bh = e.x * p.n_kv + rem / p.nsplit; split = rem % p.nsplit; S_paged = e.y; }
+      if (use.x) { bh = e.x * p.n_kv + rem / p.nsplit; split0 = rem % p.nsplit; S_paged = e.y; }
       // the numbers came out of memory: tell the compiler that they are the same in every lane (see below)
-      bh = __shfl_sync(FULLM, bh, 0); split = __shfl_sync(FULLM, split, 0);
+      bh = __shfl_sync(FULLM, bh, 0); split0 = __shfl_sync(FULLM, split0, 0);
     }
   }
   const int b = bh / p.n_kv, kvh = bh % p.n_kv;
@@ -244,8 +282,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // These values are the same in every thread, but they were loaded from memory: passing them through a shuffle tells the
   // compiler so, and the address arithmetic built on them stays in uniform registers.
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
-  const int ntiles = (S + 15) >> 4, chunk = (ntiles + p.nsplit - 1) / p.nsplit;
-  const int tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo), nstages = (n + TPS - 1) / TPS;
+  const int ntiles = (S + 15) >> 4, chunk = (ntiles + ns0 - 1) / ns0;
+  const int tlo = min(split0 * chunk, ntiles), n = min(chunk, ntiles - tlo), nstages = (n + TPS - 1) / TPS;
   const long smh = (long)ch * p.S_pad * D, cdh = (long)ch * p.S_pad * CB, rowb = (long)ch * p.S_pad, tileb = (long)ch * (p.S_pad >> 4);
   ohk = __shfl_sync(FULLM, ohk, 0); ohv = __shfl_sync(FULLM, ohv, 0);
 
@@ -334,6 +372,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     const int brow = PAGED ? kvh : ch % p.n_base_rows;
     if (warp == ATT_WARPS - 2) fill_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
     if (warp == ATT_WARPS - 1) fill_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
+    if (SHARE && tid == 0) { s_split = split0; s_ns = ns0; }
     if (tid == 0) s_next = ATT_WARPS;                        // tiles 0 .. W-1 of the range go to warps 0 .. W-1, the rest is handed out on demand
     int* mk_s = reinterpret_cast<int*>(smem + TB_META);
     int* mv_s = mk_s + META_TILES;
@@ -418,8 +457,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
     it = nx;
   }
+  const int split = SHARE ? s_split : split0, NS = SHARE ? s_ns : p.nsplit;
   // ---- slot layout: the raw BF16 tail belongs to the last split's last warp
-  if (!PAGED && TL > 0 && split == p.nsplit - 1 && warp == ATT_WARPS - 1) {
+  if (!PAGED && TL > 0 && split == NS - 1 && warp == ATT_WARPS - 1) {
     const uint16_t* kraw = reinterpret_cast<const uint16_t*>(p.K.tail) + (long)ch * p.tail_cap * D;
     const uint16_t* vraw = reinterpret_cast<const uint16_t*>(p.V.tail) + (long)ch * p.tail_cap * D;
     for (int t0 = 0; t0 < TL; t0 += T) {
@@ -452,7 +492,6 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
   }
   __syncthreads();
-  const int NS = p.nsplit;
   const long qh0 = (long)b * p.n_q + kvh * G;
   const int d = tid & 127;
   // where a query head's merged (M, L, acc) goes when this is the last word of this GPU on it
@@ -489,14 +528,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
     if (NS == 1) deliver(g, M, Lc, Ac);              // nothing to merge with
     else {
-      const long pidx = (qh0 + g) * NS + split;
+      const long pidx = (qh0 + g) * p.nsplit + split;
       if (d == 0) { p.pm[pidx] = M; p.pl[pidx] = Lc; }
       p.pa[pidx * D + d] = Ac;
     }
   }
   if (NS > 1) {
     if (!last_split(p.counters + bh, NS, &s_last)) return;
-    merge_splits<4 * NSET>(p, smem + TB_RING, qh0, G, deliver);
+    merge_splits<4 * NSET>(p, smem + TB_RING, qh0, G, NS, deliver);
   }
   if (p.x_recv) {
     // Every entry carries the exchange number, so nothing else announces the rows (see x_store / x_load).
@@ -695,7 +734,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   if (NS == 1 || !last_split(p.counters + bh, NS, &s_last)) return;
   for (int first = 0; first < 2 * G; first += 8) {
     __syncthreads();                                   // the area is used again
-    merge_splits<8>(p, smem + T256_RING, row0 + first, min(8, 2 * G - first), [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
+    merge_splits<8>(p, smem + T256_RING, row0 + first, min(8, 2 * G - first), p.nsplit, [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
   }
 }
 
@@ -817,16 +856,16 @@ static void launch_row_order(const int* seq_lens, const int* slot, int n_kv, int
   if (cudaLaunchKernelEx(&cfg, row_order_kernel, seq_lens, slot, n_kv, B, order) != cudaSuccess) cudaGetLastError();     // the attention launch that follows reports
 }
 
-template <bool PAGED, bool DUMP, int NSET>
+template <bool PAGED, bool DUMP, int NSET, bool SHARE>
 static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
-  cudaFuncSetAttribute(decode_attn_kernel<PAGED, DUMP, NSET>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM);
+  cudaFuncSetAttribute(decode_attn_kernel<PAGED, DUMP, NSET, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit); cfg.blockDim = dim3(ATT_THREADS);
+  cfg.gridDim = SHARE ? dim3((unsigned)p.n_kv, (unsigned)p.units) : dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit); cfg.blockDim = dim3(ATT_THREADS);
   cfg.dynamicSmemBytes = ATT_SMEM; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, decode_attn_kernel<PAGED, DUMP, NSET>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
+  if (cudaLaunchKernelEx(&cfg, decode_attn_kernel<PAGED, DUMP, NSET, SHARE>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
   return launch_status();
 }
 template <int NSET>
@@ -843,7 +882,8 @@ static int launch_attn256(const AttnParams& p, cudaStream_t st) {
 }
 template <bool PAGED, bool DUMP>
 static int launch_attn(const AttnParams& p, cudaStream_t st) {
-  return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1>(p, st) : launch_attn_as<PAGED, DUMP, 2>(p, st);
+  if (!DUMP && p.units) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, true>(p, st) : launch_attn_as<PAGED, false, 2, true>(p, st);
+  return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1, false>(p, st) : launch_attn_as<PAGED, DUMP, 2, false>(p, st);
 }
 
 static int sm_count_of_current_device() {
@@ -862,6 +902,7 @@ static bool exchange_ok(const gaac_exchange* x) {
 struct SlotOut {
   void* out = nullptr; float* out_f32 = nullptr; float* part = nullptr;
   const gaac_exchange* x = nullptr; bool fused = false;
+  int units = 0;
   void* dump_k = nullptr; void* dump_v = nullptr; int64_t dump_S = 0;
 };
 
@@ -889,7 +930,7 @@ static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, cons
   AttnParams p{};
   p.K = *K; p.V = *V; p.slot = slot; p.seq_len = seq_len; p.S_uniform = (int)S_uniform; p.tail_len = tail_len; p.tail_cap = tail_cap; p.S_pad = S_pad; p.n_base_rows = n_base_rows;
   p.q = (const uint16_t*)q; p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.G = n_q / n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)o.out; p.out_f32 = o.out_f32; p.part = o.part;
+  p.out = (uint16_t*)o.out; p.out_f32 = o.out_f32; p.part = o.part; p.units = o.units;
   if (x) {
     p.x_recv = x->recv; p.x_epoch = x->epoch; p.x_ticket = x->ticket; p.x_err = x->err;
     p.x_rank = x->rank; p.x_world = x->world; p.x_rows_cap = x->rows_cap; p.x_fused = o.fused ? 1 : 0;
@@ -903,7 +944,7 @@ static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, cons
 }
 
 static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16, int B, int n_q, float scale,
-                      int nsplit, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* dump_k, void* dump_v, int64_t dump_S, void* stream) {
+                      int nsplit, int units, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* dump_k, void* dump_v, int64_t dump_S, void* stream) {
   if (!st || !bt || !seq_lens || !q_bf16 || !out_bf16 || !st->buf || !st->raw || !st->mt || !st->b3k || !st->b4k || !st->b3v || !st->b4v) return GAAC_E_ARG;
   if (B <= 0 || n_q <= 0 || st->n_kv <= 0 || nsplit <= 0 || nsplit > 1024 || bt_stride <= 0) return GAAC_E_ARG;
   if (n_q % st->n_kv || n_q / st->n_kv < 1 || n_q / st->n_kv > 8 || st->TS % 16 || st->TS != SLOT_OVF_OFF + st->ovf_slot) return GAAC_E_UNSUPPORTED;
@@ -913,7 +954,7 @@ static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride
   p.buf = st->buf; p.raw = (const uint16_t*)st->raw; p.mt = st->mt; p.bt = bt; p.bt_stride = bt_stride; p.TS = st->TS; p.ovf_slot = st->ovf_slot;
   p.b3k = st->b3k; p.b4k = st->b4k; p.b3v = st->b3v; p.b4v = st->b4v; p.seq_len = seq_lens;
   p.q = (const uint16_t*)q_bf16; p.B = B; p.n_q = n_q; p.n_kv = st->n_kv; p.G = n_q / st->n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr;
+  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr; p.units = units;
   if (int e = carve_workspace(workspace, workspace_bytes, B, n_q, nsplit, p)) return e;
   if (dump_k) {
     p.dump_k = (uint16_t*)dump_k; p.dump_v = (uint16_t*)dump_v; p.dump_S = dump_S;
@@ -921,7 +962,7 @@ static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride
   }
   // ragged batches: CTAs are handed out longest row first (one small launch sorts the rows; its output is read by the attention
   // kernel after its dependency wait)
-  if (B > 1 && B <= ORDER_MAX_ROWS && (int64_t)B * st->n_kv * nsplit > sm_count_of_current_device()) {
+  if (!units && B > 1 && B <= ORDER_MAX_ROWS && (int64_t)B * st->n_kv * nsplit > sm_count_of_current_device()) {
     launch_row_order(seq_lens, nullptr, 0, B, p.order_buf, (cudaStream_t)stream);
     p.row_order = p.order_buf;
   }
@@ -950,6 +991,14 @@ extern "C" int gaac_decode_attn(const gaac_side* K, const gaac_side* V, const vo
   if (!out_bf16 || !slot || !seq_len) return GAAC_E_ARG;
   SlotOut o; o.out = out_bf16; o.out_f32 = out_f32;
   return slot_attn(K, V, q_bf16, slot, B, n_q, n_kv, seq_len, 0, S_pad, scale, nsplit, tail_len, tail_cap, n_base_rows, workspace, workspace_bytes, o, stream);
+}
+
+extern "C" int gaac_decode_attn_balanced(const gaac_side* K, const gaac_side* V, const void* q_bf16, const int32_t* slot, int B, int n_q, int n_kv,
+                                         const int32_t* seq_len, int64_t S_pad, float scale, int units, const int32_t* tail_len, int tail_cap,
+                                         int n_base_rows, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* stream) {
+  if (!out_bf16 || !slot || !seq_len || B <= 0 || B > SHARE_MAX_ROWS || units < B || units - B + 1 > 1024) return GAAC_E_ARG;
+  SlotOut o; o.out = out_bf16; o.out_f32 = out_f32; o.units = units;
+  return slot_attn(K, V, q_bf16, slot, B, n_q, n_kv, seq_len, 0, S_pad, scale, units - B + 1, tail_len, tail_cap, n_base_rows, workspace, workspace_bytes, o, stream);
 }
 
 extern "C" int gaac_decode_attn_pages(const gaac_side* K, const gaac_side* V, const void* q_bf16, int B, int n_q, int n_kv, int64_t S, int64_t S_pad,
@@ -1013,7 +1062,14 @@ extern "C" int gaac_combine_parts(const float* parts, int64_t n_heads, int n_par
 extern "C" int gaac_paged_decode_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                                       int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
                                       void* out_bf16, float* out_f32, void* stream) {
-  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
+}
+
+extern "C" int gaac_paged_decode_attn_balanced(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                               int B, int n_q, float scale, int units, void* workspace, size_t workspace_bytes,
+                                               void* out_bf16, float* out_f32, void* stream) {
+  if (B <= 0 || B > SHARE_MAX_ROWS || units < B || units - B + 1 > 1024) return GAAC_E_ARG;
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, units - B + 1, units, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
 }
 
 extern "C" int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
@@ -1048,5 +1104,5 @@ extern "C" int gaac_debug_paged_decode_attn_rebuild(const gaac_paged* st, const 
                                                     int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes, void* out_bf16,
                                                     float* out_f32, void* k_rebuilt, void* v_rebuilt, int64_t rebuilt_S, void* stream) {
   if (!k_rebuilt || !v_rebuilt) return GAAC_E_ARG;
-  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, workspace, workspace_bytes, out_bf16, out_f32, k_rebuilt, v_rebuilt, rebuilt_S, stream);
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, workspace, workspace_bytes, out_bf16, out_f32, k_rebuilt, v_rebuilt, rebuilt_S, stream);
 }

@@ -69,6 +69,14 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
             w = rows * ns / sm_count
             return 0.0 if w >= 4 else 1.0 - w / -(-w // 1)
         return min(range(first, last + 1), key=lambda ns: (waste(ns) > 0.1, abs(ns - star)))
+    # Short contexts: when two tiles per warp would leave more than a quarter of the SMs idle, ranges go below that.  A CTA takes about 6.5 us +
+    # 0.215 us per tile (8.3 us at least, with the merge of the splits) and 4.5 us + 0.21 us per tile without splits, so up to 16 tiles one CTA is
+    # faster; beyond, splits pay down to four tiles each until there are 16 (one per warp of the merge), more only with 16 tiles each.  Batch 1, 8
+    # kv heads: 500 tokens 10.8 -> 8.4 us, 1000: 18.1 -> 8.3, 2000: 15.6 -> 8.8; 4 rows of 1000: 18.6 -> 9.9; 1 kv head, 8000 tokens: 16.3 in 15
+    # splits, 13.3 in 32, 17.4 in 125.  A second wave costs more than it shortens (4 rows of 1000 in 6 splits: 15.3).
+    wave = sm_count // rows
+    if wave > 1 and 4 * most <= 3 * wave:
+        return 1 if ntiles <= ATT_WARPS else min(wave, max(min(16, ntiles // 4), -(-ntiles // 16)))
     tile_us, tile_far_us, fixed_us, staged = 4.5, 5.2, 10.0, 512
     best, best_t = 1, None
     for ns in range(1, min(most, 2 * sm_count) + 1):
@@ -81,6 +89,19 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     return best
 
 
+def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> int:
+    """Ranges per kv head that the rows of a ragged batch share by their lengths (S: tokens of the longest), or 0 where every row is split alike
+    (choose_nsplit_sm100).  One wave over the SMs, for at most 32 rows (one per lane of the warp that shares them out) and ranges of at least four tiles.
+    Rounding to whole ranges costs a share of rows / units, so there must be room for two per row, and for four where rows are long and the several
+    waves of the other form cost little beside that.  us per call, other form -> this one (B, kv heads, tokens):  slots 8, 8, 200..3000: 27.3 -> 19.5;
+    17, 4, 500..6000: 55.0 -> 36.9;  paged 5, 8, 40..1500: 17.4 -> 11.5;  9, 8, 200..4000: 30.2 -> 27.7;  3, 8, 1000..30000: 53.6 -> 48.0;
+    8, 2, 500..30000: 44.3 -> 28.6;  but 8, 8, 4000..40000 (2.25 units per row): 160 -> 180."""
+    units = sm_count // n_kv
+    if not 2 <= B <= 32 or units < (2 if S <= 16384 else 4) * B:
+        return 0
+    return min(units, B * -(-max(S, 1) // 64))
+
+
 def _side(sm, codes, flags, tile_off, ovf, head_start, base3, base4, tail) -> _lib.Side:
     return _lib.Side(sm.data_ptr(), codes.data_ptr(), flags.data_ptr(), tile_off.data_ptr(), ovf.data_ptr(), head_start.data_ptr(),
                      ovf.numel(), base3.data_ptr(), base4.data_ptr(), _lib.ptr(tail))
@@ -91,13 +112,14 @@ class _Ext:
 
     @staticmethod
     def gaac_attn_launch(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, smv, cv, fv, tov, ovv, ohsv, b3v, b4v,
-                         q, slot, n_q, n_kv, SL, S_pad, scale, nsplit, kt, vt, TL, TCAP, out_f32=None, partial=None, exchange=None, fused=False):
+                         q, slot, n_q, n_kv, SL, S_pad, scale, nsplit, kt, vt, TL, TCAP, out_f32=None, partial=None, exchange=None, fused=False, units=0):
         """Same positional arguments as the reference launcher (gaac/kernel.py:296-300): 16 K/V buffers, q [B*n_q, 128] bf16,
         slot int32 [B], n_q, n_kv, SL int32 [heads], S_pad, scale, nsplit, K/V tails [heads, TCAP, 128] bf16 (empty = none),
         TL int32 [heads], TCAP.  Returns out [B*n_q, 128] bf16.  Extras: out_f32 (fp32 tensor to receive the un-rounded
         result), partial ([B*n_q, 130] fp32 tensor: write (m, l, acc) there instead of the output), exchange (a
         gaac_b200._lib.Exchange: push the partial rows into every rank's receive buffer instead and return None; with fused=True
-        the same launch also waits for the other ranks' rows, merges them and returns the output)."""
+        the same launch also waits for the other ranks' rows, merges them and returns the output), units (> 0: the rows share that many
+        ranges per kv head by their lengths, nsplit is not used)."""
         D = 128
         if q.size(-1) != D:
             raise RuntimeError("head_dim must be 128")
@@ -111,8 +133,16 @@ class _Ext:
         has_tail = kt.numel() > 0
         K = _side(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None)
         V = _side(smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None)
+        if units:
+            nsplit = units - B + 1
         ws = workspace(dev, B, n_q, nsplit)
         L = _lib.lib()
+        if units:
+            out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
+            _lib.check(L.gaac_decode_attn_balanced(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), units,
+                                                   TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel(),
+                                                   out.data_ptr(), _lib.ptr(out_f32), _lib.stream_ptr(dev)), "gaac_decode_attn_balanced")
+            return out
         common = (K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), int(nsplit),
                   TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel())
         if exchange is not None and fused:

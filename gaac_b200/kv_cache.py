@@ -17,7 +17,7 @@ import torch
 from . import _lib
 from .codec import Codec, Page, D, T, CB
 from .encoder import TileEncoder
-from .kernel import _ext, choose_nsplit, choose_nsplit_sm100
+from .kernel import _ext, choose_nsplit, choose_nsplit_sm100, choose_units
 
 TAIL = T                       # rows of the raw tail buffer of a head
 TILE_MAX_ESC = 1280            # a tile whose 256 groups are all raw has 256 * 5 escape bytes
@@ -216,13 +216,14 @@ class CompressedKVCache:
         (gaac/kv_cache.py:183-192)"""
         B, n_q, _ = q.shape
         self.settle_prefills()
+        units = choose_units(B, self.n_kv, max_len or self.cap) if nsplit is None else 0
         if nsplit is None:
             nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap)
         K, V = self.k, self.v
         out = _ext().gaac_attn_launch(K.sm, K.codes, K.flags, K.tile_off, K.ovf, K.head_start, K.base3, K.base4,
                                       V.sm, V.codes, V.flags, V.tile_off, V.ovf, V.head_start, V.base3, V.base4,
                                       q.reshape(B * n_q, D).contiguous(), slots, n_q, self.n_kv, self.S, self.cap, scale, nsplit,
-                                      K.tail, V.tail, self.tail_len, TAIL, out_f32=out_f32)
+                                      K.tail, V.tail, self.tail_len, TAIL, out_f32=out_f32, units=units)
         return out.view(B, n_q, D)
 
     # ------------------------------------------------------------------ housekeeping

@@ -226,6 +226,13 @@ int gaac_decode_attn_exchange(const gaac_side* K, const gaac_side* V, const void
                               int n_base_rows, void* workspace, size_t workspace_bytes, const gaac_exchange* x, void* out_bf16, float* out_f32,
                               void* stream);
 
+/* gaac_decode_attn for a ragged batch of at most 32 rows: instead of nsplit equal parts of every row, the rows share `units` ranges per kv head
+ * (units >= B) in proportion to their lengths, which the kernel reads itself: n_kv * units CTAs, at most as many as the GPU has SMs for one
+ * even wave (a slot's first head stands for all of its heads).  workspace: gaac_attn_workspace_bytes(B, n_q, units - B + 1). */
+int gaac_decode_attn_balanced(const gaac_side* K, const gaac_side* V, const void* q_bf16, const int32_t* slot, int B, int n_q, int n_kv,
+                              const int32_t* seq_len, int64_t S_pad, float scale, int units, const int32_t* tail_len, int tail_cap,
+                              int n_base_rows, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* stream);
+
 /* Decode attention over two Pages (all B*n_kv heads hold S tokens, row b reads heads b*n_kv .., no tail): the
  * `attention(q, kp, vp)` entry of the reference (gaac/kernel.py:345-359), which builds an identity slot map and a constant
  * length table for its launcher; here both are implied, so the kernel's prologue has no dependent table loads.  Exactly one
@@ -316,6 +323,11 @@ int gaac_paged_decode_blocks(const gaac_paged* st, const int32_t* pairs, int P, 
 int gaac_paged_decode_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                            int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
                            void* out_bf16, float* out_f32, void* stream);
+
+/* gaac_paged_decode_attn with the rows' ranges shared out by length, as in gaac_decode_attn_balanced. */
+int gaac_paged_decode_attn_balanced(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                    int B, int n_q, float scale, int units, void* workspace, size_t workspace_bytes,
+                                    void* out_bf16, float* out_f32, void* stream);
 
 /* The same for head_dim 256: a 256-dim head is stored as two 128-dim half-heads in neighbouring tile slots, each with its own
  * bases, so the store, the block decoder and the bases all see 2 * (256-dim kv heads) half-heads: st->n_kv is that number of
