@@ -90,13 +90,14 @@ __device__ __forceinline__ int pop_raw_tile(const gaac_paged& st, int lane) {
   return __shfl_sync(FULL, r, 0);
 }
 
-// One warp per (entry, tile slot t = 2*kvh + kind).  grid = (E, 2*n_kv).
+// One warp: entry e, tile slot t = 2*kvh + kind.  Returns (lane 0) the raw tile that the store set free, or -1: it may go back on the stack once no
+// warp of the step pops any more.
 template <int KIND_V>
-__device__ __forceinline__ void store_one(WarpScratch& ws, const PagedParams& p, int e, int t, int lane) {
+__device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, int e, int t, int lane) {
   const gaac_paged& st = p.st;
   const int kvh = t >> 1, NT = 2 * st.n_kv;
   const int blk = p.ent[4 * e], tok0 = p.ent[4 * e + 1], off0 = p.ent[4 * e + 2], n = p.ent[4 * e + 3];
-  if (blk < 0) { if (lane == 0) p.freeq[e * NT + t] = -1; return; }
+  if (blk < 0) return -1;
   const long pt = (long)blk * NT + t;
   const int old = st.mt[pt];
   const bool have = old < 0, full = (off0 + n == T);
@@ -134,17 +135,31 @@ __device__ __forceinline__ void store_one(WarpScratch& ws, const PagedParams& p,
       *reinterpret_cast<uint4*>(rawp + ((long)r * T + row) * D + col) = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
     }
   }
-  if (lane == 0) {
-    st.mt[pt] = fits ? (int)pt : ~r;
-    p.freeq[e * NT + t] = (fits && have) ? r_old : -1;
-  }
+  if (lane == 0) st.mt[pt] = fits ? (int)pt : ~r;
+  return fits && have ? r_old : -1;
 }
 
 __global__ void __launch_bounds__(32) paged_store_kernel(const __grid_constant__ PagedParams p) {
   __shared__ __align__(16) WarpScratch ws;
   const int e = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
   griddep_launch();
-  if (t & 1) store_one<1>(ws, p, e, t, lane); else store_one<0>(ws, p, e, t, lane);
+  const int freed = t & 1 ? store_one<1>(ws, p, e, t, lane) : store_one<0>(ws, p, e, t, lane);
+  if (lane == 0) p.freeq[e * 2 * p.st.n_kv + t] = freed;
+}
+
+// The same for a step of few tiles, as ONE cluster: the cluster's barrier stands between the pops and the pushes, so no second launch is needed to
+// return the raw tiles.  A warp per tile: 8 blocks x 10 warps, which covers 5 sequences of 8 kv heads (larger steps would put several tiles on a
+// warp one after the other, and their second launch is hidden behind the work).
+constexpr int STEP_WARPS = 10, STEP_CLUSTER = 8;
+__global__ void __launch_bounds__(STEP_WARPS * 32) paged_store_step_kernel(const __grid_constant__ PagedParams p, int n_items) {
+  __shared__ __align__(16) WarpScratch ws[STEP_WARPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * STEP_WARPS + warp, NT = 2 * p.st.n_kv;
+  griddep_launch();
+  int freed = -1;
+  if (i < n_items) freed = i & 1 ? store_one<1>(ws[warp], p, i / NT, i % NT, lane) : store_one<0>(ws[warp], p, i / NT, i % NT, lane);
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (lane == 0 && freed >= 0) p.st.stack[atomicAdd(p.st.top, 1)] = freed;
 }
 
 __global__ void __launch_bounds__(256) free_tiles_kernel(const int* __restrict__ freeq, int n_items, int* __restrict__ stack, int* __restrict__ top) {
@@ -239,6 +254,18 @@ extern "C" int gaac_paged_store(const gaac_paged* st, const void* key, const voi
   if (E == 0) return GAAC_OK;
   PagedParams p{*st, (const uint16_t*)key, (const uint16_t*)value, k_stride, v_stride, ent, freeq};
   cudaStream_t s = (cudaStream_t)stream;
+  const int64_t items = (int64_t)E * 2 * st->n_kv;
+  if (items <= STEP_WARPS * STEP_CLUSTER) {
+    unsigned blocks = 1;
+    while (blocks * STEP_WARPS < items) blocks *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(STEP_WARPS * 32); cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, paged_store_step_kernel, p, (int)items) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
+    return launch_status();
+  }
   paged_store_kernel<<<dim3((unsigned)E, (unsigned)(2 * st->n_kv)), 32, 0, s>>>(p);
   const int n = E * 2 * st->n_kv;
   if (int err = launch_status()) return err;

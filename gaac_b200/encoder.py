@@ -88,7 +88,7 @@ class TileEncoder:
 
     def encode_into(self, x: torch.Tensor, base3, base4, n_kv: int, sm, cd, flags, tile_off, ovf, *, S: int | None = None, S_pad: int | None = None,
                     head_start=None, head_base=None, head_cap: int = 0, head_bytes=None, ovf_off=None, bidx=None, zero_pad: int = 8, status=None):
-        """Encode x [H, S_in, D] (its first S tokens) into caller-owned buffers: four kernel launches, no host synchronisation, so
+        """Encode x [H, S_in, D] (its first S tokens) into caller-owned buffers: three kernel launches, no host synchronisation, so
         it can sit inside a CUDA graph (the serving path).  sm / cd / flags: [H, S_pad*..] rows as in a Page; tile_off int32
         [H, ntiles] contiguous, written.  Escape bytes go to `ovf`:
           packed   - head after head; head_start int32 [H+1] is written (head_start[H] = all bytes); bounded by ovf.numel()

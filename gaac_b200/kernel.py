@@ -44,12 +44,12 @@ def choose_nsplit(B: int, n_kv: int, S: int, target_ctas: int = 96, min_tok: int
 def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200, min_tiles_per_warp: int = 2, ragged: bool = False,
                         total_tokens: int | None = None) -> int:
     """Splits per (row, kv head) for a B200.  The kernel runs one 16-warp CTA per SM; a CTA keeps the metadata of the first
-    META_TILES (512) tiles of its range in shared memory and fetches the rest from global memory inside the loop.
+    META_TILES (1024) tiles of its range in shared memory and fetches the rest from global memory inside the loop.
 
     Equal lengths (S is every row's length): the split count minimises a cost model fitted to measurements,
         waves x ((tiles per warp + 0.5) x tile time + per-CTA fixed cost),   waves = ceil(rows x splits / SMs),
-    over the counts that leave every warp at least min_tiles_per_warp 16-token tiles.  Tile time: 4.5 us for a tile whose
-    metadata is staged, 5.2 us beyond; fixed cost (prologue, warp merge, split merge): 10 us.  Few rows end up with one wave that
+    over the counts that leave every warp at least min_tiles_per_warp 16-token tiles (fewer on short contexts, see the code).  Tile time: 4.5 us, 5.2 us
+    beyond 512 tiles of a range; fixed cost (prologue, warp merge, split merge): 10 us.  Few rows end up with one wave that
     fills the SMs, many rows with ranges of at most 512 tiles in several waves.
     Ragged lengths (ragged=True, S is the longest row; total_tokens is accepted and unused): every row gets the same split count;
     see the comment in the code."""

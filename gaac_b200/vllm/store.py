@@ -9,8 +9,8 @@ Two cases per tile slot.  A block that is still filling keeps its rows as plain 
 pool tile is taken from a free stack the first time the block is written, and the mode table remembers it as mt[p] = ~r.  A block
 that the step completes is compressed: if the tile's escape bytes fit the slot's escape area the tile goes into its slot,
 mt[p] = p again, and the pool tile goes back on the stack; if they do not fit the tile simply stays in the pool for good.
-Pool tiles are popped only by the store kernel and pushed back only by the kernel launched right behind it, so the two never
-race on the stack.  A pop from an empty stack is counted in `err` instead of trapping.
+Pool tiles are pushed back only when every pop of the step is through (behind a cluster barrier for small steps, by a kernel launched right behind
+the store for larger ones), so the two never race on the stack.  A pop from an empty stack is counted in `err` instead of trapping.
 """
 from __future__ import annotations
 import torch

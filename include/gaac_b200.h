@@ -272,7 +272,7 @@ int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, const void* k
  * at x + t*row_stride + h*128 (bf16 elements; row_stride >= n_kv*128, rows 16-byte aligned), L tokens (L <= S_cap).  The
  * floor(L/16) whole tiles of every head of the slot are compressed straight into the store (tile 0 upward, the head's escape
  * bytes from offset 0 of its share), the L mod 16 remaining rows go into the raw tails, seq_len / tail_len / ovf_used of the
- * slot's heads are set: seven launches, no host synchronisation, no transposed copy of the input.
+ * slot's heads are set: three launches, no host synchronisation, no transposed copy of the input.
  * Replaces CompressedKVCache.prefill's device work (gaac/kv_cache.py:149-169: Triton encode per kind, torch prefix sums, the
  * scatter of the escape bytes, tail copy, counter updates).
  *   scratch: gaac_cache_prefill_scratch_bytes(L, n_kv) bytes of device memory, kept by the caller until a copy_only repeat is
@@ -303,7 +303,7 @@ typedef struct {
 /* Store this step's new rows.  key/value: [num_tokens, n_kv, 128] bf16 with row strides k_stride/v_stride (elements);
  * ent [E,4] = (block, first row in key/value, offset in block, rows); block < 0: inactive entry.  freeq [E*2*n_kv] scratch.
  * Filling blocks go to a raw tile (popped from the free stack on first touch); a block completed by this step is
- * compressed into its slot when its escapes fit ovf_slot (its raw tile is queued in freeq and pushed back), else kept
+ * compressed into its slot when its escapes fit ovf_slot (its raw tile is pushed back once all pops of the call are through), else kept
  * raw.  A failed pop increments *err.  Replaces _store_tiles + _free_tiles (gaac/vllm/store.py:22-114, 204-213). */
 int gaac_paged_store(const gaac_paged* st, const void* key, const void* value, int64_t k_stride, int64_t v_stride,
                      const int32_t* ent, int E, int32_t* freeq, void* stream);

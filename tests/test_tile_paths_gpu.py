@@ -101,3 +101,26 @@ def test_paged_slots_of_any_alignment(ovf_slot):
     rows = np.r_[0:9, 16:16 * blocks]
     assert np.array_equal(bits(sk)[rows], k16[rows]) and np.array_equal(bits(sv)[rows], v16[rows]) and not sk[9:16].any()
     assert int((st.mt >= 0).sum()) > 0                 # some tiles are compressed
+
+
+# a step's tile slots around what one block and one cluster of the store take (10 and 80): raw tiles are popped, then all returned when the blocks fill
+@pytest.mark.parametrize("E", [1, 5, 6, 10, 11, 20, 21, 40, 41])
+def test_paged_store_steps_pop_and_return_raw_tiles(E):
+    import torch
+    from gaac_b200.vllm.store import LayerState, OVF_OFF
+    k16, v16 = (O.synth_kv(kind, 1, 16 * E, E, raw_frac=0.0, four_frac=0.05).transpose(1, 0, 2) for kind in "kv")
+    bases = {}
+    for kind, x16 in (("k", k16), ("v", v16)):
+        bases[kind + "3"], bases[kind + "4"] = (torch.from_numpy(b) for b in O.calibrate(np.ascontiguousarray(x16.transpose(1, 0, 2)), 1))
+    st = LayerState(E + 1, 1, raw_tiles=2 * E + 3, bases=bases, ovf_slot=512, device="cuda")
+    buf = torch.zeros((E + 1) * 2 * (OVF_OFF + 512), dtype=torch.uint8, device="cuda")
+    k, v = to_bf16_cuda(k16), to_bf16_cuda(v16)
+    freeq = torch.empty((E + 1) * 2, dtype=torch.int32, device="cuda")
+    for off, n in ((0, 15), (15, 1)):
+        ent = torch.tensor([[b + 1 if b < E else -1, 16 * b + off, off, n] for b in range(E + (E % 5 == 1))], dtype=torch.int32, device="cuda")      # sometimes with an inactive entry
+        st.store(k, v, buf, ent, freeq)
+        assert int(st.top) == (3 if off == 0 else 2 * E + 3) and int(st.err) == 0
+    assert sorted(st.stack.tolist()) == list(range(2 * E + 3)) and (st.mt >= 0).all()
+    sk = torch.zeros(16 * E, 1, 128, dtype=torch.bfloat16, device="cuda"); sv = torch.zeros_like(sk)
+    st.decode_blocks(buf, torch.tensor([[b + 1, 16 * b, 16] for b in range(E)], dtype=torch.int32, device="cuda"), sk, sv)
+    assert np.array_equal(bits(sk), k16) and np.array_equal(bits(sv), v16)
