@@ -19,6 +19,7 @@
 //
 // Fragment conventions follow the reference kernel (gaac/kernel.py:62-66,160-194), whose storage order they mirror.
 #include <algorithm>
+#include <atomic>
 #include "gaac_api.cuh"
 #include "gaac_attn_tile.cuh"
 
@@ -856,29 +857,40 @@ static void launch_row_order(const int* seq_lens, const int* slot, int n_kv, int
   if (cudaLaunchKernelEx(&cfg, row_order_kernel, seq_lens, slot, n_kv, B, order) != cudaSuccess) cudaGetLastError();     // the attention launch that follows reports
 }
 
-template <bool PAGED, bool DUMP, int NSET, bool SHARE>
-static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
-  cudaFuncSetAttribute(decode_attn_kernel<PAGED, DUMP, NSET, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM);
+// Launch of an attention kernel, one CTA of ATT_THREADS per SM.  The permission for its shared memory is asked for once per kernel and device, not on every
+// launch; where a launch fails with the permission believed to be there (it goes with a device reset), it is asked for again.
+template <auto Kernel>
+static int launch_big(const AttnParams& p, dim3 grid, int smem_bytes, cudaStream_t st) {
+  static std::atomic<unsigned long long> allowed{0};                  // one bit per device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = SHARE ? dim3((unsigned)p.n_kv, (unsigned)p.units) : dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit); cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = ATT_SMEM; cfg.stream = st;
+  cfg.gridDim = grid; cfg.blockDim = dim3(ATT_THREADS); cfg.dynamicSmemBytes = smem_bytes; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, decode_attn_kernel<PAGED, DUMP, NSET, SHARE>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
-  return launch_status();
+  bool asked = false;
+  while (true) {
+    if (asked || !(allowed.load(std::memory_order_relaxed) & bit)) {
+      cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+      allowed.fetch_or(bit, std::memory_order_relaxed);
+      asked = true;
+    }
+    if (cudaLaunchKernelEx(&cfg, Kernel, p) == cudaSuccess) return launch_status();
+    cudaGetLastError();
+    if (asked) return GAAC_E_LAUNCH;
+    asked = true;
+  }
+}
+template <bool PAGED, bool DUMP, int NSET, bool SHARE>
+static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
+  const dim3 grid = SHARE ? dim3((unsigned)p.n_kv, (unsigned)p.units) : dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit);
+  return launch_big<decode_attn_kernel<PAGED, DUMP, NSET, SHARE>>(p, grid, ATT_SMEM, st);
 }
 template <int NSET>
 static int launch_attn256(const AttnParams& p, cudaStream_t st) {
-  cudaFuncSetAttribute(paged256_attn_kernel<NSET>, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT256_SMEM);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit); cfg.blockDim = dim3(ATT_THREADS);
-  cfg.dynamicSmemBytes = ATT256_SMEM; cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, paged256_attn_kernel<NSET>, p) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
-  return launch_status();
+  return launch_big<paged256_attn_kernel<NSET>>(p, dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit), ATT256_SMEM, st);
 }
 template <bool PAGED, bool DUMP>
 static int launch_attn(const AttnParams& p, cudaStream_t st) {

@@ -89,6 +89,7 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     return best
 
 
+@functools.lru_cache(maxsize=4096)
 def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> int:
     """Ranges per kv head that the rows of a ragged batch share by their lengths (S: tokens of the longest), or 0 where every row is split alike
     (choose_nsplit_sm100).  One wave over the SMs, for at most 32 rows (one per lane of the warp that shares them out) and ranges of at least four tiles.

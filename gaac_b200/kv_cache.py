@@ -217,7 +217,7 @@ class CompressedKVCache:
         B, n_q, _ = q.shape
         self.settle_prefills()
         units = choose_units(B, self.n_kv, max_len or self.cap) if nsplit is None else 0
-        if nsplit is None:
+        if nsplit is None and not units:
             nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap)
         K, V = self.k, self.v
         out = _ext().gaac_attn_launch(K.sm, K.codes, K.flags, K.tile_off, K.ovf, K.head_start, K.base3, K.base4,
