@@ -212,12 +212,160 @@ __device__ __forceinline__ void row_share(int tiles, int B, int units, int u, in
   split = u - ((int)__shfl_sync(FULLM, inc, row & 31) - NS);
 }
 
+// Weights of a warp summed over its lanes; true when some sum of values is not finite although its weights are (see sum_exact).
+template <int NSET> __device__ __forceinline__ bool sum_warp(WarpAcc<NSET>& A) {
+  bool bad = false;
+#pragma unroll
+  for (int s = 0; s < NSET; s++) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) A.l[s] += __shfl_xor_sync(FULLM, A.l[s], o);
+    u32 most = 0u;
+#pragma unroll
+    for (int i = 0; i < 16; i++) most = max(most, __float_as_uint(A.acc[s][i >> 2][i & 3]) & 0x7FFFFFFFu);
+    bad |= most >= 0x7F800000u && A.l[s] < CUDART_INF_F;
+  }
+  return bad;
+}
+// A warp's sums on their way into the CTA's: m [W][8], l [W][8], acc [W][8][ACC_LD]
+template <int NSET> __device__ __forceinline__ void stage_warp(const WarpAcc<NSET>& A, uint8_t* area, int G, int warp, int lane) {
+  const int j = lane & 3, r = lane >> 2;
+  float* sh_m = reinterpret_cast<float*>(area);
+#pragma unroll
+  for (int s = 0; s < NSET; s++) {
+    const int h = 4 * s + j;
+    if (r == 0) { sh_m[warp * 8 + h] = A.m[s]; sh_m[ATT_WARPS * 8 + warp * 8 + h] = A.l[s]; }
+    if (h < G) {
+      float* a0 = sh_m + ATT_WARPS * 16 + (warp * 8 + h) * ACC_LD + r;
+#pragma unroll
+      for (int i = 0; i < 16; i++) a0[8 * i] = A.acc[s][i >> 2][i & 3];
+    }
+  }
+}
+static_assert(ATT_THREADS == 512, "a thread of the merge has every fourth head");
+// Head g of the warps w0, w0 + step, .. (N of them), as they left it in shared memory (m [W][8], l [W][8], acc [W][8][ACC_LD]) -> M, L and element d of the
+// sum
+template <int N> __device__ __forceinline__ void merge_warps(const uint8_t* area, int step, int w0, int g, int d, float& M, float& L, float& acc) {
+  const float *sh_m = reinterpret_cast<const float*>(area), *sh_l = sh_m + ATT_WARPS * 8, *sh_acc = sh_l + ATT_WARPS * 8;
+  M = -CUDART_INF_F; L = 0.f; acc = 0.f;
+#pragma unroll
+  for (int w = 0; w < N; w++) M = fmaxf(M, sh_m[(step * w + w0) * 8 + g]);
+#pragma unroll
+  for (int w = 0; w < N; w++) {
+    const int at = (step * w + w0) * 8 + g;
+    const float mw = sh_m[at], f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
+    L += sh_l[at] * f; acc += sh_acc[at * ACC_LD + d] * f;
+  }
+}
+// ---- V elements that are not finite.  In the value product a word meets a weight of zero for the other parity's channel, and the lower half of a
+// weight may be zero too: an infinite or NaN element makes its word's OTHER channel NaN as well (0 x Inf), and its own NaN where Inf is
+// right.  A CTA whose sum is not finite therefore takes its range once more in plain fp32, where an element meets its own weight only and tokens
+// behind the end meet none: range `split` of NS of (row, kv head) bh, straight from global memory, token by token, four channels per lane.  The
+// result lies where the warps of the main loop leave theirs.  Finite data never comes here, and what counts is what the presence of this code costs
+// the main loop: it looks everything up again and has little code and few registers.  32768 tokens, 8 kv heads: finite 33.8 -> 33.5 us, one infinite
+// element 608; GQA group 8: 66.5 -> 66.9 at 65536 tokens; head_dim 256: 36.1 -> 36.6, group 8 114.5 -> 118.  With the main loop's decoder in
+// its place a second pass took a fifth of that, but finite data 1 to 7 % more, inlined or called.
+template <bool PAGED, bool WIDE>
+__device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, int bh, int split, int NS) {
+  int tid = threadIdx.x;
+  asm volatile("" : "+r"(tid), "+r"(bh), "+r"(split), "+r"(NS));
+  const int lane = tid & 31, warp = tid >> 5, b = bh / p.n_kv, kvh = bh % p.n_kv, hf = WIDE ? warp & 1 : 0, HALVES = WIDE ? 2 : 1;
+  int S, ch = 0, TL = 0;
+  if (PAGED) S = p.seq_len[b];
+  else {
+    const int sl = p.slot ? p.slot[b] : b;
+    ch = max(sl, 0) * p.n_kv + kvh;
+    S = sl < 0 ? 0 : p.seq_len ? p.seq_len[ch] : p.S_uniform;
+    TL = sl >= 0 && p.tail_len && split == NS - 1 ? p.tail_len[ch] : 0;
+  }
+  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS, tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo);
+  float m[8], l[8], acc[8][4];
+#pragma unroll
+  for (int h = 0; h < 8; h++) { m[h] = -CUDART_INF_F; l[h] = acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.f; }
+#pragma unroll 1
+  for (int i = WIDE ? warp >> 1 : warp; i < n + ((TL + T - 1) >> 4); i += ATT_WARPS / HALVES) {
+    const int tile = tlo + i, valid = i < n ? min(T, S - tile * T) : min(T, TL - (i - n) * T);
+    PlainSide side[3];                               // K (of both halves where there are two), V
+    u32 tags[3]; int at[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (!WIDE && c == 1) continue;
+      const bool vs = c == 2;
+      PlainSide& s = side[c];
+      const uint8_t* fl;
+      if (PAGED) {
+        const int t = 2 * (HALVES * kvh + (vs ? hf : c)) + (vs ? 1 : 0), row = (t >> 1) * D, meta = p.mt[p.bt[(long)b * p.bt_stride + tile] * (2 * HALVES * p.n_kv) + t];
+        const uint8_t* t0 = p.buf + (long)meta * p.TS;
+        s = PlainSide{t0, t0 + SLOT_CD_OFF, t0 + SLOT_OVF_OFF, (vs ? p.b3v : p.b3k) + row, (vs ? p.b4v : p.b4k) + row, meta < 0 ? p.raw + (long)(~meta) * (T * D) : nullptr};
+        fl = t0 + SLOT_FL_OFF;
+      } else {
+        const gaac_side& g = vs ? p.V : p.K;
+        const long row = (long)ch * p.S_pad + (long)tile * T;
+        const int brow = ch % p.n_base_rows * D;
+        s = PlainSide{g.sm + row * D, g.codes + row * CB, nullptr, g.base3 + brow, g.base4 + brow, nullptr};
+        if (i < n) s.esc = g.ovf + ((long)g.head_start[ch] + g.tile_off[(long)ch * (p.S_pad >> 4) + tile]);
+        else s.raw = reinterpret_cast<const uint16_t*>(g.tail) + ((long)ch * p.tail_cap + (i - n) * T) * D;
+        fl = reinterpret_cast<const uint8_t*>(g.flags + row);
+      }
+      tags[c] = s.raw ? 0u : reinterpret_cast<const u32*>(fl)[lane & 15];
+      const u32 own = (u32)row_esc_bytes(tags[c]);
+      u32 inc = own;
+      scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8);
+      at[c] = (int)(inc - own);
+    }
+#pragma unroll 1
+    for (int tok = 0; tok < valid; tok++) {
+      float sc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < (WIDE ? 2 : 1); c++) {
+        const u32 tg = __shfl_sync(FULLM, tags[c], tok);
+        const int ea = __shfl_sync(FULLM, at[c], tok);
+#pragma unroll 1
+        for (int d = lane; d < D; d += 32) {
+          const float x = plain_element<false>(side[c], tok, d, tg, ea);
+#pragma unroll
+          for (int h = 0; h < 8; h++)
+            if (h < p.G) sc[h] += x * __uint_as_float((u32)p.q[(((long)b * p.n_q + kvh * p.G + h) * HALVES + c) * D + d] << 16);
+        }
+      }
+      const u32 tg = __shfl_sync(FULLM, tags[2], tok);
+      const int ea = __shfl_sync(FULLM, at[2], tok);
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) v[q] = plain_element<true>(side[2], tok, lane + 32 * q, tg, ea);
+#pragma unroll
+      for (int h = 0; h < 8; h++) {
+        float s = sc[h];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULLM, s, o);
+        s *= p.scale_log2;
+        if (s > m[h]) {
+          const float f = fast_exp2(m[h] - s);
+          l[h] *= f; m[h] = s;
+#pragma unroll
+          for (int q = 0; q < 4; q++) acc[h][q] *= f;
+        }
+        const float w = fast_exp2(s - fmaxf(m[h], -1e30f));
+        l[h] += w;
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[h][q] += w * v[q];
+      }
+    }
+  }
+  float* sh_m = reinterpret_cast<float*>(area);
+#pragma unroll
+  for (int h = 0; h < 8; h++) {
+    if (lane == 0) { sh_m[warp * 8 + h] = m[h]; sh_m[ATT_WARPS * 8 + warp * 8 + h] = l[h]; }
+#pragma unroll
+    for (int q = 0; q < 4; q++) sh_m[ATT_WARPS * 16 + (warp * 8 + h) * ACC_LD + lane + 32 * q] = acc[h][q];
+  }
+}
+
 // SHARE: a balanced launch (its own instantiation: the shares cost the other one registers that the main loop has none of, 1.5 % at 64K tokens)
 template <bool PAGED, bool DUMP, int NSET, bool SHARE>
 __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last, s_split, s_ns;        // (the last two are not needed inside the main loop, whose registers are all taken)
-  const int tid = threadIdx.x, lane = tid & 31, j = lane & 3, r = lane >> 2;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
   const u32 smem_s = (u32)__cvta_generic_to_shared(smem);
@@ -475,23 +623,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   }
 
   // ---- merge the warps of the CTA (the ring is free now)
-  __syncthreads();
-  float* sh_m = reinterpret_cast<float*>(smem + TB_RING);        // [W][8]
-  float* sh_l = sh_m + ATT_WARPS * 8;                            // [W][8]
-  float* sh_acc = sh_l + ATT_WARPS * 8;                          // [W][8][ACC_LD]
-#pragma unroll
-  for (int s = 0; s < NSET; s++) {
-    const int h = 4 * s + j;
-    float l = A.l[s];
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(FULLM, l, o);
-    if (r == 0) { sh_m[warp * 8 + h] = A.m[s]; sh_l[warp * 8 + h] = l; }
-    if (h < G) {
-      float* a0 = sh_acc + (warp * 8 + h) * ACC_LD + r;
-#pragma unroll
-      for (int i = 0; i < 16; i++) a0[8 * i] = A.acc[s][i >> 2][i & 3];
-    }
-  }
+  if (__syncthreads_or(sum_warp(A))) sum_exact<PAGED, false>(p, smem + TB_RING, bh, split, NS);
+  else stage_warp(A, smem + TB_RING, G, warp, lane);
   __syncthreads();
   const long qh0 = (long)b * p.n_q + kvh * G;
   const int d = tid & 127;
@@ -516,22 +649,21 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if (p.out_f32) p.out_f32[qh * D + d] = v;
     }
   };
-  for (int g = tid >> 7; g < G; g += ATT_THREADS / 128) {
-    float M = -CUDART_INF_F;
+  float M[NSET], Lc[NSET], Ac[NSET];                  // of heads tid / 128 and 4 above
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS; w++) M = fmaxf(M, sh_m[w * 8 + g]);
-    float Lc = 0.f, Ac = 0.f;
+  for (int i = 0; i < NSET; i++) {
+    const int g = (tid >> 7) + 4 * i;
+    if (g < G) merge_warps<ATT_WARPS>(smem + TB_RING, 1, 0, g, d, M[i], Lc[i], Ac[i]);
+  }
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS; w++) {
-      const float mw = sh_m[w * 8 + g];
-      const float f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
-      Lc += sh_l[w * 8 + g] * f; Ac += sh_acc[(w * 8 + g) * ACC_LD + d] * f;
-    }
-    if (NS == 1) deliver(g, M, Lc, Ac);              // nothing to merge with
+  for (int i = 0; i < NSET; i++) {
+    const int g = (tid >> 7) + 4 * i;
+    if (g >= G) continue;
+    if (NS == 1) deliver(g, M[i], Lc[i], Ac[i]);     // nothing to merge with
     else {
       const long pidx = (qh0 + g) * p.nsplit + split;
-      if (d == 0) { p.pm[pidx] = M; p.pl[pidx] = Lc; }
-      p.pa[pidx * D + d] = Ac;
+      if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
+      p.pa[pidx * D + d] = Ac[i];
     }
   }
   if (NS > 1) {
@@ -588,7 +720,7 @@ template <int NSET>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last;
-  const int bh = blockIdx.x, split = blockIdx.y, tid = threadIdx.x, lane = tid & 31, j = lane & 3, r = lane >> 2;
+  const int bh = blockIdx.x, split = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);
   const int hf = warp & 1, pair = warp >> 1;
   const int b = bh / p.n_kv, kvh = bh % p.n_kv, G = p.G, NT = 4 * p.n_kv;    // p.n_kv = 256-dim kv heads; NT tile slots per block
@@ -687,23 +819,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     __syncwarp();                                      // every lane has read this stage before its next copies are issued
   }
   // ---- merge the warps of the CTA, half by half: one partial per virtual head (2 * query head + half)
-  __syncthreads();
-  float* sh_m = reinterpret_cast<float*>(smem + T256_RING);
-  float* sh_l = sh_m + ATT_WARPS * 8;
-  float* sh_acc = sh_l + ATT_WARPS * 8;
-#pragma unroll
-  for (int s = 0; s < NSET; s++) {
-    const int h = 4 * s + j;
-    float l = A.l[s];
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(FULLM, l, o);
-    if (r == 0) { sh_m[warp * 8 + h] = A.m[s]; sh_l[warp * 8 + h] = l; }
-    if (h < G) {
-      float* a0 = sh_acc + (warp * 8 + h) * ACC_LD + r;
-#pragma unroll
-      for (int i = 0; i < 16; i++) a0[8 * i] = A.acc[s][i >> 2][i & 3];
-    }
-  }
+  if (__syncthreads_or(sum_warp(A))) sum_exact<true, true>(p, smem + T256_RING, bh, split, p.nsplit);
+  else stage_warp(A, smem + T256_RING, G, warp, lane);
   __syncthreads();
   const int d = tid & 127, NS = p.nsplit;
   const long row0 = 2 * ((long)b * p.n_q + kvh * G);
@@ -712,24 +829,21 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     p.out[row * D + d] = __bfloat16_as_ushort(__float2bfloat16(v));
     if (p.out_f32) p.out_f32[row * D + d] = v;
   };
-  for (int vg = tid >> 7; vg < 2 * G; vg += ATT_THREADS / 128) {
-    const int g = vg >> 1, h2 = vg & 1;
-    float M = -CUDART_INF_F;
+  float M[2 * NSET], Lc[2 * NSET], Ac[2 * NSET];      // of virtual heads tid / 128, 4 above, ..
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS / 2; w++) M = fmaxf(M, sh_m[(2 * w + h2) * 8 + g]);
-    float Lc = 0.f, Ac = 0.f;
+  for (int i = 0; i < 2 * NSET; i++) {
+    const int vg = (tid >> 7) + 4 * i;
+    if (vg < 2 * G) merge_warps<ATT_WARPS / 2>(smem + T256_RING, 2, vg & 1, vg >> 1, d, M[i], Lc[i], Ac[i]);
+  }
 #pragma unroll
-    for (int w = 0; w < ATT_WARPS / 2; w++) {
-      const int ww = 2 * w + h2;
-      const float mw = sh_m[ww * 8 + g];
-      const float f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
-      Lc += sh_l[ww * 8 + g] * f; Ac += sh_acc[(ww * 8 + g) * ACC_LD + d] * f;
-    }
-    if (NS == 1) deliver(row0 + vg, Lc, Ac);
+  for (int i = 0; i < 2 * NSET; i++) {
+    const int vg = (tid >> 7) + 4 * i;
+    if (vg >= 2 * G) continue;
+    if (NS == 1) deliver(row0 + vg, Lc[i], Ac[i]);
     else {
       const long pidx = (row0 + vg) * NS + split;
-      if (d == 0) { p.pm[pidx] = M; p.pl[pidx] = Lc; }
-      p.pa[pidx * D + d] = Ac;
+      if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
+      p.pa[pidx * D + d] = Ac[i];
     }
   }
   if (NS == 1 || !last_split(p.counters + bh, NS, &s_last)) return;

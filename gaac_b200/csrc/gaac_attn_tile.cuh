@@ -361,4 +361,25 @@ __device__ __forceinline__ void raw_accum(WarpAcc<NSET>& A, const uint16_t* vraw
   }
 }
 
+// ---- one element of a tile, read from global memory bit by bit (sum_exact): where the storage order puts it, its code, its group's tag and escape
+// bytes.  tags, esc_at: tag word of the token's row and position of the row's first escape byte inside the tile.
+struct PlainSide { const uint8_t *sm, *cd, *esc, *b3, *b4; const uint16_t* raw; };         // raw: the tile as BF16 rows, then nothing else is read
+template <bool VSIDE> __device__ __forceinline__ float plain_element(const PlainSide& s, int tok, int ch, u32 tags, int esc_at) {
+  if (s.raw) return __uint_as_float((u32)s.raw[tok * D + ch] << 16);
+  int group, k, sm_at, cd_at;                        // group of the row, element inside it, byte of the sign/mantissa, bit of the code
+  if (VSIDE) {
+    const int r = ch & 7, n = ch >> 3, lane = 4 * r + ((tok & 7) >> 1), t = (tok & 1) + 2 * (tok >> 3);
+    group = 2 * r + (n >> 3); k = n & 7; sm_at = 64 * lane + 16 * t + n; cd_at = 8 * (24 * lane + 6 * t) + 3 * n;
+  } else {
+    const int j = (ch & 7) >> 1, at = 4 * (ch >> 4) + (ch & 1) + 2 * ((ch >> 3) & 1), lane = 4 * (tok & 7) + j, o = tok >> 3;
+    group = 4 * j + (at >> 3); k = at & 7; sm_at = 1024 * o + 32 * lane + at; cd_at = 8 * (384 * o + 12 * lane) + 3 * at;
+  }
+  const u32 sm = s.sm[sm_at], two = (u32)s.cd[cd_at >> 3] | ((cd_at & 7) > 5 ? (u32)s.cd[(cd_at >> 3) + 1] << 8 : 0u), code = (two >> (cd_at & 7)) & 7u, tag = (tags >> (2 * group)) & 3u;
+  const uint8_t* esc = s.esc + esc_at + esc_prefix(tags, 2 * group);
+  u32 e = s.b3[ch] + code;
+  if (tag == 1u) e = s.b4[ch] + code + (((u32)esc[0] >> k) & 1u) * 8u;
+  if (tag == 3u) { const int bit = 5 * k; e = code | (((((u32)esc[bit >> 3] | ((bit & 7) > 3 ? (u32)esc[(bit >> 3) + 1] << 8 : 0u)) >> (bit & 7)) & 31u) << 3); }
+  return __uint_as_float(((sm & 0x80u) << 24) | ((e & 0xFFu) << 23) | ((sm & 0x7Fu) << 16));
+}
+
 }  // namespace gaac

@@ -138,7 +138,9 @@ size_t gaac_attn_workspace_header_bytes(int B, int n_q);
  * (slot[b] < 0: padded row, output exactly 0); seq_len[cache head] compressed tokens; tail_len[cache head] raw tail tokens
  * (NULL when there is no tail).  nsplit >= 1 context splits per (row, kv head).  out [B, n_q, 128] bf16; when out_f32 is
  * non-NULL the un-rounded fp32 result is written there as well.  workspace: gaac_attn_workspace_bytes bytes with a zeroed
- * header (see above).  n_base_rows: rows of the base tables (cache head h uses row h % n_base_rows).  Replaces gaac_attn_launch = gaac_attn<G> + gaac_tail<G> + gaac_combine<128>
+ * header (see above).  n_base_rows: rows of the base tables (cache head h uses row h % n_base_rows).  Here and in every other
+ * attention call an infinite or NaN element of V makes its own output channel infinite or NaN and no other; the ranges that hold one
+ * take about 18 times as long.  Replaces gaac_attn_launch = gaac_attn<G> + gaac_tail<G> + gaac_combine<128>
  * (gaac/kernel.py:48-326). */
 int gaac_decode_attn(const gaac_side* K, const gaac_side* V, const void* q_bf16, const int32_t* slot, int B, int n_q, int n_kv,
                      const int32_t* seq_len, int64_t S_pad, float scale, int nsplit, const int32_t* tail_len, int tail_cap,
