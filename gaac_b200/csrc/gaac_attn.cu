@@ -295,7 +295,7 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
       if (PAGED) {
         const int t = 2 * (HALVES * kvh + (vs ? hf : c)) + (vs ? 1 : 0), row = (t >> 1) * D, meta = p.mt[p.bt[(long)b * p.bt_stride + tile] * (2 * HALVES * p.n_kv) + t];
         const uint8_t* t0 = p.buf + (long)meta * p.TS;
-        s = PlainSide{t0, t0 + SLOT_CD_OFF, t0 + SLOT_OVF_OFF, (vs ? p.b3v : p.b3k) + row, (vs ? p.b4v : p.b4k) + row, meta < 0 ? p.raw + (long)(~meta) * (T * D) : nullptr};
+        s = PlainSide{t0, t0 + SLOT_CD_OFF, t0 + SLOT_OVF_OFF, (vs ? p.b3v : p.b3k) + row, (vs ? p.b4v : p.b4k) + row, meta < 0 ? p.raw + (long)raw_tile(meta) * (T * D) : nullptr};
         fl = t0 + SLOT_FL_OFF;
       } else {
         const gaac_side& g = vs ? p.V : p.K;
@@ -574,13 +574,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     const TilePlan plan = plan_tile(ks, vs, rawk, rawv, W, lane);
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
     if (!rawk) k_tile<DUMP>(sc, ks, plan, W, lane, Q, dump_k + (long)tile * T * D, nvalid);
-    else raw_scores<DUMP>(sc, p.raw + (long)(~cur.mk) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
+    else raw_scores<DUMP>(sc, p.raw + (long)raw_tile(cur.mk) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
     nx = __shfl_sync(FULLM, nx, 0);
     PFrag<NSET> P;
     if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
     else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
     if (!rawv) v_tile<DUMP, NSET>(A, vs, plan, W, lane, P, dump_v + (long)tile * T * D, nvalid);
-    else raw_accum<DUMP, NSET>(A, p.raw + (long)(~cur.mv) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
+    else raw_accum<DUMP, NSET>(A, p.raw + (long)raw_tile(cur.mv) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
     // the stage's bytes may have been written through ordinary stores (patch numbers): order those before the copy engine's next
     // writes to the same bytes, then count this warp out of the stage
     if (st + NSTG < nstages) {
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (ok) {
       plan = plan_tile(ks, vs, cur.mk < 0, cur.mv < 0, W, lane);
       if (cur.mk >= 0) k_tile<false>(sc, ks, plan, W, lane, Q, nullptr, nvalid);
-      else raw_scores<false>(sc, p.raw + (long)(~cur.mk) * (T * D), nvalid, lane, Q, nullptr);
+      else raw_scores<false>(sc, p.raw + (long)raw_tile(cur.mk) * (T * D), nvalid, lane, Q, nullptr);
     }
     // ---- the two halves' partial scores meet; the next tile's number and a failed wait travel with them
     uint8_t* slot = xch + par * XCH_PAR_BYTES;
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
     else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
     if (cur.mv >= 0) v_tile<false, NSET>(A, vs, plan, W, lane, P, nullptr, nvalid);
-    else raw_accum<false, NSET>(A, p.raw + (long)(~cur.mv) * (T * D), nvalid, lane, P, nullptr);
+    else raw_accum<false, NSET>(A, p.raw + (long)raw_tile(cur.mv) * (T * D), nvalid, lane, P, nullptr);
     cur = nxt; stg ^= 1; it = t1;
     __syncwarp();                                      // every lane has read this stage before its next copies are issued
   }

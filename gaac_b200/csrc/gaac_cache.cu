@@ -81,13 +81,20 @@ struct PagedParams {
   const int* ent; int* freeq;
 };
 
+// -1: the pool is empty, which is counted; top then stays below zero by the failed pops of the step.
 __device__ __forceinline__ int pop_raw_tile(const gaac_paged& st, int lane) {
-  int r = 0;
+  int r = -1;
   if (lane == 0) {
     const int idx = atomicAdd(st.top, -1) - 1;
-    if (idx >= 0) r = st.stack[idx]; else atomicAdd(st.err, 1);      // failed pop: tile 0 is written and the error counted
+    if (idx >= 0) r = st.stack[idx]; else atomicAdd(st.err, 1);
   }
   return __shfl_sync(FULL, r, 0);
+}
+// No pop is under way (they are in another launch or behind a barrier).  Failed pops took nothing, so a top below zero counts as zero; every
+// push sees to that before its own addition, and after the first one top never is below zero again.
+__device__ __forceinline__ void push_raw_tile(int* stack, int* top, int r) {
+  atomicMax(top, 0);
+  stack[atomicAdd(top, 1)] = r;
 }
 
 // One warp: entry e, tile slot t = 2*kvh + kind.  Returns (lane 0) the raw tile that the store set free, or -1: it may go back on the stack once no
@@ -100,8 +107,8 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   if (blk < 0) return -1;
   const long pt = (long)blk * NT + t;
   const int old = st.mt[pt];
-  const bool have = old < 0, full = (off0 + n == T);
-  const int r_old = have ? ~old : 0;
+  const bool have = old < 0 && old != ~RAW_NONE, full = (off0 + n == T);       // a block that found the pool empty before asks again
+  const int r_old = old < 0 ? raw_tile(old) : 0;
   const uint16_t* src = (KIND_V ? p.value : p.key) + (long)kvh * D;
   const long sstride = KIND_V ? p.v_stride : p.k_stride;
   uint16_t* rawp = reinterpret_cast<uint16_t*>(st.raw);
@@ -130,12 +137,12 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   if (!fits) {
     if (!have) r = pop_raw_tile(st, lane);
     // new rows, natural channel order, into raw tile r
-    for (int c = lane; c < n * 16; c += 32) {
+    for (int c = lane; c < (r < 0 ? 0 : n * 16); c += 32) {
       const int row = off0 + (c >> 4), col = (c & 15) * 8;
       *reinterpret_cast<uint4*>(rawp + ((long)r * T + row) * D + col) = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
     }
   }
-  if (lane == 0) st.mt[pt] = fits ? (int)pt : ~r;
+  if (lane == 0) st.mt[pt] = fits ? (int)pt : ~(r < 0 ? RAW_NONE : r);
   return fits && have ? r_old : -1;
 }
 
@@ -159,7 +166,7 @@ __global__ void __launch_bounds__(STEP_WARPS * 32) paged_store_step_kernel(const
   if (i < n_items) freed = i & 1 ? store_one<1>(ws[warp], p, i / NT, i % NT, lane) : store_one<0>(ws[warp], p, i / NT, i % NT, lane);
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (lane == 0 && freed >= 0) p.st.stack[atomicAdd(p.st.top, 1)] = freed;
+  if (lane == 0 && freed >= 0) push_raw_tile(p.st.stack, p.st.top, freed);
 }
 
 __global__ void __launch_bounds__(256) free_tiles_kernel(const int* __restrict__ freeq, int n_items, int* __restrict__ stack, int* __restrict__ top) {
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(256) free_tiles_kernel(const int* __restrict__
   griddep_launch();
   if (i >= n_items) return;
   const int r = freeq[i];
-  if (r >= 0) { const int idx = atomicAdd(top, 1); stack[idx] = r; }
+  if (r >= 0) push_raw_tile(stack, top, r);
 }
 
 __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restrict__ blocks, int NT, int* __restrict__ mt, int* __restrict__ stack, int* __restrict__ top) {
@@ -176,7 +183,7 @@ __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restric
   for (int t = threadIdx.x; t < NT; t += 32) {
     const long pt = blk * NT + t;
     const int m = mt[pt];
-    if (m < 0) { const int idx = atomicAdd(top, 1); stack[idx] = ~m; mt[pt] = (int)pt; }
+    if (m < 0) { if (m != ~RAW_NONE) push_raw_tile(stack, top, raw_tile(m)); mt[pt] = (int)pt; }
   }
 }
 
@@ -191,7 +198,7 @@ __device__ __forceinline__ void decode_block_one(DecodeScratch& ws, const PagedD
   const int m = st.mt[pt];
   uint16_t* dst = (KIND_V ? p.sv : p.sk) + (long)row0 * p.row_stride + (long)kvh * D;
   if (m < 0) {
-    const uint16_t* rawp = reinterpret_cast<const uint16_t*>(st.raw) + (long)(~m) * T * D;
+    const uint16_t* rawp = reinterpret_cast<const uint16_t*>(st.raw) + (long)raw_tile(m) * T * D;
     for (int c = lane; c < nvalid * 16; c += 32) {
       const int row = c >> 4, col = (c & 15) * 8;
       *reinterpret_cast<uint4*>(dst + (long)row * p.row_stride + col) = *reinterpret_cast<const uint4*>(rawp + row * D + col);

@@ -26,6 +26,9 @@ constexpr int TILE_SM = T * D;  // 2048
 constexpr int TILE_CD = T * CB; // 768
 constexpr int TILE_MAX_ESC = 1280;
 constexpr int SLOT_CD_OFF = 2048, SLOT_FL_OFF = 2816, SLOT_OVF_OFF = 2880;   // paged tile slot layout (gaac/vllm/store.py:18)
+// Mode-table entry m < 0 of the paged layout: the rows are in raw tile raw_tile(m) of the pool, ~m when the block owns that tile.  A block that found the
+// pool empty owns none: its entry is ~RAW_NONE, its rows are lost, readers get those of tile 0.
+constexpr int RAW_NONE = 1 << 30;
 
 // ---- portable intrinsics ---------------------------------------------------------------------------------------
 GAAC_HD u32 prmt(u32 a, u32 b, u32 sel) {
@@ -45,6 +48,7 @@ GAAC_HD u32 funnel_r(u32 lo, u32 hi, int sh) {          // (hi:lo) >> sh, 0 <= s
   return sh ? (u32)((((u64)hi << 32) | lo) >> sh) : lo;
 #endif
 }
+GAAC_HD int raw_tile(int m) { return ~m & (RAW_NONE - 1); }
 // the bits of a where the mask has ones, those of b elsewhere (one instruction; the compiler needs two for the and/and/or form)
 GAAC_HD u32 bits_of(u32 a, u32 b, u32 mask) {
 #if defined(__CUDA_ARCH__)

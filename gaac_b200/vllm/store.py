@@ -10,7 +10,8 @@ pool tile is taken from a free stack the first time the block is written, and th
 that the step completes is compressed: if the tile's escape bytes fit the slot's escape area the tile goes into its slot,
 mt[p] = p again, and the pool tile goes back on the stack; if they do not fit the tile simply stays in the pool for good.
 Pool tiles are pushed back only when every pop of the step is through (behind a cluster barrier for small steps, by a kernel launched right behind
-the store for larger ones), so the two never race on the stack.  A pop from an empty stack is counted in `err` instead of trapping.
+the store for larger ones), so the two never race on the stack.  A pop from an empty stack is counted in `err` instead of trapping: the
+block gets no tile (mt[p] = ~(1 << 30)) and its rows are dropped; the reference writes them over tile 0, whoever has that (gaac/vllm/store.py:68-70).
 """
 from __future__ import annotations
 import torch

@@ -295,7 +295,8 @@ int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, const void* k_t
 
 /* Paged store state of one layer (gaac/vllm/store.py:177-203).  Tile slot p = block*(2*n_kv) + 2*kvh + kind lives at
  * buf + p*TS: [0,2048) sign/mantissa, [2048,2816) codes, [2816,2880) 16 tag words, [2880,TS) escapes.
- * mt[p] == p: compressed in its slot; mt[p] == ~r: raw bf16 tile r of `raw` [raw_tiles,16,128]. */
+ * mt[p] == p: compressed in its slot; mt[p] == ~r: raw bf16 tile r of `raw` [raw_tiles,16,128]; mt[p] == ~(1 << 30): the pool was empty when
+ * the block wanted a raw tile, its rows are lost (and read as those of raw tile 0). */
 typedef struct {
   uint8_t* buf; void* raw; int32_t* mt; int32_t* stack; int32_t* top; int32_t* err;
   const uint8_t* b3k; const uint8_t* b4k; const uint8_t* b3v; const uint8_t* b4v;
@@ -306,7 +307,8 @@ typedef struct {
  * ent [E,4] = (block, first row in key/value, offset in block, rows); block < 0: inactive entry.  freeq [E*2*n_kv] scratch.
  * Filling blocks go to a raw tile (popped from the free stack on first touch); a block completed by this step is
  * compressed into its slot when its escapes fit ovf_slot (its raw tile is pushed back once all pops of the call are through), else kept
- * raw.  A failed pop increments *err.  Replaces _store_tiles + _free_tiles (gaac/vllm/store.py:22-114, 204-213). */
+ * raw.  A failed pop increments *err and leaves *top below zero until the next push; that block's rows are dropped, no other block's rows and
+ * nothing of the stack are touched, and its next store asks again.  Replaces _store_tiles + _free_tiles (gaac/vllm/store.py:22-114, 204-213). */
 int gaac_paged_store(const gaac_paged* st, const void* key, const void* value, int64_t k_stride, int64_t v_stride,
                      const int32_t* ent, int E, int32_t* freeq, void* stream);
 
