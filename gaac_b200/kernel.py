@@ -10,29 +10,31 @@ import functools
 import torch
 from . import _lib
 
-_WS = {}        # (device index, stream) -> workspace tensor, zeroed once: every call leaves its split counters at zero and the
-                # header in front of the partials has a fixed size, so calls of any shape can share it (B*n_q up to 16320)
+_WS = {}        # (device index, stream, 0) -> workspaces, the last one in use.  Zeroed once: every call leaves its split counters at zero and the header
+                # in front of the partials has a fixed size for B*n_q up to 16320, so calls of any such shape share one.  Above that the header
+                # depends on B*n_q, which then stands in the key.
 SM_COUNT_B200 = 148
 ATT_WARPS = 16  # warps per CTA of the CUDA kernel (one CTA per SM)
 
 
 def workspace(dev, B: int, n_q: int, nsplit: int) -> torch.Tensor:
+    """The workspace of the current stream.  One that became too small is kept beside its successor: a captured CUDA graph may hold its address, and the
+    successor has at least twice its size, so all of them together stay below twice the largest."""
     need = _lib.lib().gaac_attn_workspace_bytes(B, n_q, nsplit)
-    key = (torch.device(dev).index, torch.cuda.current_stream(dev).cuda_stream)
-    ws = _WS.get(key)
-    if ws is None or ws.numel() < need or B * n_q > 16320 or getattr(ws, "_gaac_big", False):
-        # a fresh zeroed buffer when none fits, and for the rare shapes whose counters outgrow the fixed-size header
-        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-        ws._gaac_big = B * n_q > 16320
-        _WS[key] = ws
-    return ws
+    key = (torch.device(dev).index, torch.cuda.current_stream(dev).cuda_stream, B * n_q if B * n_q > 16320 else 0)
+    held = _WS.get(key)
+    if held is None:
+        held = _WS.setdefault(key, [])
+    if not held or held[-1].numel() < need:
+        held.append(torch.zeros(max(need, 2 * held[-1].numel() if held else 1 << 20), dtype=torch.uint8, device=dev))
+    return held[-1]
 
 
 def workspace_error(dev, B: int = 0, n_q: int = 0) -> bool:
-    """True when a kernel that used the cached workspace of the current stream gave up on a bounded wait for its own asynchronous
+    """True when a kernel that used a cached workspace of the current stream gave up on a bounded wait for its own asynchronous
     copies (the int32 at the start of the workspace).  Reads device memory, so it synchronises; meant for tests and debugging."""
-    ws = _WS.get((torch.device(dev).index, torch.cuda.current_stream(dev).cuda_stream))
-    return bool(ws is not None and ws[0:4].view(torch.int32).item() != 0)
+    here = (torch.device(dev).index, torch.cuda.current_stream(dev).cuda_stream)
+    return any(ws[0:4].view(torch.int32).item() != 0 for key, held in _WS.items() if key[:2] == here for ws in held)
 
 
 def choose_nsplit(B: int, n_kv: int, S: int, target_ctas: int = 96, min_tok: int = 512, cap: int = 48) -> int:
