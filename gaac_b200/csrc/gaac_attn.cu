@@ -62,8 +62,8 @@ struct AttnParams {
   const uint16_t* q; int B, n_q, n_kv, G; float scale_log2; int nsplit;
   int* counters; int* err; float* pm; float* pl; float* pa;     // err: set to 1 when a bounded wait inside the kernel ran out
   uint16_t* out; float* out_f32; float* part;
-  // balanced launches (units > 0; grid = (n_kv, units)): the rows share `units` ranges per kv head by their lengths, see row_share; nsplit is then the most
-  // that one row can get and only the stride of the partials
+  // balanced launches (units > 0; grid = (n_kv, units)): the rows share `units` ranges per kv head by their lengths, see row_share; nsplit is not used, a
+  // unit of a kv head has one partial per query head, at (kvh * units + unit) * G
   int units;
   // cross-GPU exchange (x_recv == NULL: unused): the partial of every query head is stored into every rank's receive
   // buffer, then this rank's arrival flag of the (row, kv head) group on every rank is set to the exchange number; with
@@ -128,24 +128,24 @@ __device__ __forceinline__ bool last_split(int* counter, int NS, int* s_last) {
   __syncthreads();
   return *s_last != 0;
 }
-// Partials of rows row0 .. row0 + heads - 1 (heads <= HMAX <= 8) -> deliver(head, M, L, acc[threadIdx.x & 127]).  All loads are independent of one
+// Partials of `heads` heads (heads <= HMAX <= 8), that of head g and split s at first + g * per_head + s * per_split -> deliver(head, M, L, acc[threadIdx.x & 127]).  All loads are independent of one
 // another (no per-split dependent chain): scale factors first, then the weighted sum with one warp per split and 16-byte loads, then a
 // cross-warp sum in shared memory.
 template <int HMAX, class F>
-__device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area, long row0, int heads, int NS, const F& deliver) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, LD = p.nsplit;      // NS splits of LD places per head
+__device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area, long first, int per_head, int per_split, int heads, int NS, const F& deliver) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* c_f = reinterpret_cast<float*>(area);        // [heads][NS]  m, then exp2(m - M)
   float* c_l = c_f + 8 * NS;                          // [heads][NS]  l
   float* c_ML = c_l + 8 * NS;                         // [8][2]       M, L per head
   float* c_red = c_ML + 16;                           // [W][8][128]  (NS <= 1024 keeps this inside the ring area)
   for (int i = tid; i < heads * NS; i += ATT_THREADS) {
-    const long at = row0 * LD + (LD == NS ? i : i / NS * LD + i % NS);
+    const long at = first + (per_split == 1 ? i : i / NS * per_head + i % NS * per_split);          // (per_split 1: NS places per head)
     c_f[i] = __ldcg(p.pm + at); c_l[i] = __ldcg(p.pl + at);
   }
   float4 acc[HMAX];                                   // split `warp` of every head, in flight while M and L are computed
 #pragma unroll
   for (int g = 0; g < HMAX; g++)
-    acc[g] = (g < heads && warp < NS) ? __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * LD + warp) * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    acc[g] = (g < heads && warp < NS) ? __ldcg(reinterpret_cast<const float4*>(p.pa + (first + g * per_head + warp * per_split) * D) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
   if (warp < heads) {
     float M = -CUDART_INF_F;
@@ -172,7 +172,7 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area,
 #pragma unroll
     for (int g = 0; g < HMAX; g++) {
       if (g < heads) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.pa + ((row0 + g) * LD + s2) * D) + lane);
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.pa + (first + g * per_head + s2 * per_split) * D) + lane);
         const float f = c_f[g * NS + s2];
         acc[g].x += v.x * f; acc[g].y += v.y * f; acc[g].z += v.z * f; acc[g].w += v.w * f;
       }
@@ -661,14 +661,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (g >= G) continue;
     if (NS == 1) deliver(g, M[i], Lc[i], Ac[i]);     // nothing to merge with
     else {
-      const long pidx = (qh0 + g) * p.nsplit + split;
+      const long pidx = SHARE ? ((long)blockIdx.x * p.units + blockIdx.y) * G + g : (qh0 + g) * p.nsplit + split;
       if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
       p.pa[pidx * D + d] = Ac[i];
     }
   }
   if (NS > 1) {
     if (!last_split(p.counters + bh, NS, &s_last)) return;
-    merge_splits<4 * NSET>(p, smem + TB_RING, qh0, G, NS, deliver);
+    if (SHARE) merge_splits<4 * NSET>(p, smem + TB_RING, ((long)blockIdx.x * p.units + blockIdx.y - split) * G, 1, G, G, NS, deliver);
+    else merge_splits<4 * NSET>(p, smem + TB_RING, qh0 * NS, NS, 1, G, NS, deliver);
   }
   if (p.x_recv) {
     // Every entry carries the exchange number, so nothing else announces the rows (see x_store / x_load).
@@ -849,7 +850,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   if (NS == 1 || !last_split(p.counters + bh, NS, &s_last)) return;
   for (int first = 0; first < 2 * G; first += 8) {
     __syncthreads();                                   // the area is used again
-    merge_splits<8>(p, smem + T256_RING, row0 + first, min(8, 2 * G - first), p.nsplit, [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
+    merge_splits<8>(p, smem + T256_RING, (row0 + first) * NS, NS, 1, min(8, 2 * G - first), NS, [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
   }
 }
 
@@ -949,6 +950,8 @@ static size_t ws_bytes_needed(int B, int n_q, int nsplit) {
   const size_t n = (size_t)B * n_q * nsplit;
   return ws_header_bytes(B, n_q) + align256(4 * n) * 2 + align256(4 * n * D) + align256(sizeof(int2) * ((size_t)B + 1));     // header | pm | pl | pa | row order
 }
+// Splits per row whose room the partials of a balanced launch fit into: n_kv * units * G = n_q * units rows.
+static int share_splits(int B, int units) { return (units + B - 1) / B; }
 static int carve_workspace(void* ws, size_t ws_bytes, int B, int n_q, int nsplit, AttnParams& p) {
   const size_t n = (size_t)B * n_q * nsplit;
   if (!ws || ws_bytes < ws_bytes_needed(B, n_q, nsplit)) return GAAC_E_WORKSPACE;
@@ -1061,7 +1064,7 @@ static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, cons
     p.x_recv = x->recv; p.x_epoch = x->epoch; p.x_ticket = x->ticket; p.x_err = x->err;
     p.x_rank = x->rank; p.x_world = x->world; p.x_rows_cap = x->rows_cap; p.x_fused = o.fused ? 1 : 0;
   }
-  if (int e = carve_workspace(ws, ws_bytes, B, n_q, nsplit, p)) return e;
+  if (int e = carve_workspace(ws, ws_bytes, B, n_q, o.units ? share_splits(B, o.units) : nsplit, p)) return e;
   if (o.dump_k) {
     p.dump_k = (uint16_t*)o.dump_k; p.dump_v = (uint16_t*)o.dump_v; p.dump_S = o.dump_S;
     return launch_attn<false, true>(p, (cudaStream_t)stream);
@@ -1081,7 +1084,7 @@ static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride
   p.b3k = st->b3k; p.b4k = st->b4k; p.b3v = st->b3v; p.b4v = st->b4v; p.seq_len = seq_lens;
   p.q = (const uint16_t*)q_bf16; p.B = B; p.n_q = n_q; p.n_kv = st->n_kv; p.G = n_q / st->n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
   p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr; p.units = units;
-  if (int e = carve_workspace(workspace, workspace_bytes, B, n_q, nsplit, p)) return e;
+  if (int e = carve_workspace(workspace, workspace_bytes, B, n_q, units ? share_splits(B, units) : nsplit, p)) return e;
   if (dump_k) {
     p.dump_k = (uint16_t*)dump_k; p.dump_v = (uint16_t*)dump_v; p.dump_S = dump_S;
     return launch_attn<true, true>(p, (cudaStream_t)stream);

@@ -136,9 +136,7 @@ class _Ext:
         has_tail = kt.numel() > 0
         K = _side(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None)
         V = _side(smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None)
-        if units:
-            nsplit = units - B + 1
-        ws = workspace(dev, B, n_q, nsplit)
+        ws = workspace(dev, B, n_q, -(-units // B) if units else nsplit)
         L = _lib.lib()
         if units:
             out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)

@@ -28,7 +28,7 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     if TS % 16: raise RuntimeError("tile stride must be a multiple of 16")
     if not q.is_cuda: raise RuntimeError("gaac_b200 attention needs CUDA tensors: there is no CPU path")
     units = choose_units(B, n_kv, bt.shape[1] * 16) if nsplit is None else 0
-    if units: nsplit = units - B + 1
+    if units: nsplit = -(-units // B)            # what the workspace must have room for
     elif nsplit is None: nsplit = choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), n_kv, TS, TS - 2880)
