@@ -64,7 +64,7 @@ struct AttnParams {
   uint16_t* out; float* out_f32; float* part;
   // balanced launches (units > 0; grid = (n_kv, units)): the rows share `units` ranges per kv head by their lengths, see row_share; nsplit is not used, a
   // unit of a kv head has one partial per query head, at (kvh * units + unit) * G
-  int units;
+  int units, wave;                                  // wave: units of a kv head that run at a time
   // cross-GPU exchange (x_recv == NULL: unused): the partial of every query head is stored into every rank's receive
   // buffer, then this rank's arrival flag of the (row, kv head) group on every rank is set to the exchange number; with
   // x_fused the same CTA then waits (bounded) for the other ranks' flags, merges all ranks' rows and writes the output
@@ -192,17 +192,28 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area,
 }
 
 // Balanced launches: lane = batch row, tiles = the row's tiles.  Every row gets ceil(tiles / C) ranges (at least one, so that an empty row is written
-// too), with the smallest C of at least SHARE_MIN_TILES for which all of them fit into `units`; a few steps of bisection between the bounds
+// too), with the smallest C of at least SHARE_MIN_TILES for which all of them fit into the units there are; a few steps of bisection between the bounds
 // total / units and total / (units - rows), which always fits.  Unit u then is range `split` of NS of row `row`; row >= 32: nothing to do.
-// A ragged batch split alike for every row waits for its longest row.
-constexpr int SHARE_MAX_ROWS = 32, SHARE_MIN_TILES = 4;
-__device__ __forceinline__ void row_share(int tiles, int B, int units, int u, int lane, int& row, int& split, int& NS) {
+// A ragged batch split alike for every row waits for its longest row.  `wave` units run at a time; of a launch with more, those behind the first
+// wave are used only where that is faster: few units per row may leave much of the first wave idle (7 equal rows get 2 of 18 units each, in two waves 5
+// of 37).  A second wave costs a prologue, about as long as 40 tiles; CTAs that find nothing to do cost 12.
+constexpr int SHARE_MAX_ROWS = 32, SHARE_MIN_TILES = 4, SHARE_WAVE_TILES = 40 - 12;
+__device__ __forceinline__ void row_share(int tiles, int B, int units, int wave, int u, int lane, int& row, int& split, int& NS) {
   const unsigned n = lane < B ? (unsigned)tiles : 0u, total = __reduce_add_sync(FULLM, n), most = __reduce_max_sync(FULLM, n);
-  unsigned lo = max((unsigned)SHARE_MIN_TILES, (total + units - 1) / units);
-  unsigned hi = max(lo, units > B ? (total + (units - B) - 1) / (units - B) : most);
-  for (int it = 0; it < 6 && lo < hi; it++) {
-    const unsigned mid = (lo + hi) >> 1, want = lane < B ? max(1u, (n + mid - 1) / mid) : 0u;
-    if (__reduce_add_sync(FULLM, want) <= (unsigned)units) hi = mid; else lo = mid + 1;
+  auto smallest = [&](int units) {
+    unsigned lo = max((unsigned)SHARE_MIN_TILES, (total + units - 1) / units);
+    unsigned hi = max(lo, units > B ? (total + (units - B) - 1) / (units - B) : most);
+#pragma unroll 1
+    for (int it = 0; it < 6 && lo < hi; it++) {
+      const unsigned mid = (lo + hi) >> 1, want = lane < B ? max(1u, (n + mid - 1) / mid) : 0u;
+      if (__reduce_add_sync(FULLM, want) <= (unsigned)units) hi = mid; else lo = mid + 1;
+    }
+    return hi;
+  };
+  unsigned hi = smallest(min(units, wave));
+  if (units > wave) {
+    const unsigned two = smallest(units);
+    if (hi > SHARE_WAVE_TILES + 2 * two) hi = two;
   }
   const int ns = lane < B ? (int)max(1u, (n + hi - 1) / hi) : 0;
   u32 inc = (u32)ns;
@@ -395,7 +406,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if (PAGED) len = p.seq_len[lane];
       else { const int sl = p.slot[lane]; len = sl < 0 ? 0 : p.seq_len[(long)sl * p.n_kv]; }        // a slot's first head stands for all of its heads
     }
-    row_share((len + 15) >> 4, p.B, p.units, blockIdx.y, lane, row, split0, ns0);
+    row_share((len + 15) >> 4, p.B, p.units, p.wave, blockIdx.y, lane, row, split0, ns0);
     if (row >= p.B) return;
     bh = row * p.n_kv + blockIdx.x;
     S_paged = __shfl_sync(FULLM, len, row);
@@ -1023,6 +1034,8 @@ static int sm_count_of_current_device() {
   return cached[dev];
 }
 
+static int share_wave(int B, int n_kv) { return std::max(B, sm_count_of_current_device() / n_kv); }
+
 static bool exchange_ok(const gaac_exchange* x) {
   return x && x->recv && x->epoch && x->ticket && x->err && x->world >= 1 && x->world <= 64 && x->rank >= 0 && x->rank < x->world && x->rows_cap > 0;
 }
@@ -1059,7 +1072,7 @@ static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, cons
   AttnParams p{};
   p.K = *K; p.V = *V; p.slot = slot; p.seq_len = seq_len; p.S_uniform = (int)S_uniform; p.tail_len = tail_len; p.tail_cap = tail_cap; p.S_pad = S_pad; p.n_base_rows = n_base_rows;
   p.q = (const uint16_t*)q; p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.G = n_q / n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)o.out; p.out_f32 = o.out_f32; p.part = o.part; p.units = o.units;
+  p.out = (uint16_t*)o.out; p.out_f32 = o.out_f32; p.part = o.part; p.units = o.units; p.wave = o.units ? share_wave(B, n_kv) : 0;
   if (x) {
     p.x_recv = x->recv; p.x_epoch = x->epoch; p.x_ticket = x->ticket; p.x_err = x->err;
     p.x_rank = x->rank; p.x_world = x->world; p.x_rows_cap = x->rows_cap; p.x_fused = o.fused ? 1 : 0;
@@ -1083,7 +1096,7 @@ static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride
   p.buf = st->buf; p.raw = (const uint16_t*)st->raw; p.mt = st->mt; p.bt = bt; p.bt_stride = bt_stride; p.TS = st->TS; p.ovf_slot = st->ovf_slot;
   p.b3k = st->b3k; p.b4k = st->b4k; p.b3v = st->b3v; p.b4v = st->b4v; p.seq_len = seq_lens;
   p.q = (const uint16_t*)q_bf16; p.B = B; p.n_q = n_q; p.n_kv = st->n_kv; p.G = n_q / st->n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr; p.units = units;
+  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr; p.units = units; p.wave = units ? share_wave(B, st->n_kv) : 0;
   if (int e = carve_workspace(workspace, workspace_bytes, B, n_q, units ? share_splits(B, units) : nsplit, p)) return e;
   if (dump_k) {
     p.dump_k = (uint16_t*)dump_k; p.dump_v = (uint16_t*)dump_v; p.dump_S = dump_S;

@@ -98,10 +98,17 @@ def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> in
     Rounding to whole ranges costs a share of rows / units, so there must be room for two per row, and for four where rows are long and the several
     waves of the other form cost little beside that.  us per call, other form -> this one (B, kv heads, tokens):  slots 8, 8, 200..3000: 27.3 -> 19.5;
     17, 4, 500..6000: 55.0 -> 36.9;  paged 5, 8, 40..1500: 17.4 -> 11.5;  9, 8, 200..4000: 30.2 -> 27.7;  3, 8, 1000..30000: 53.6 -> 48.0;
-    8, 2, 500..30000: 44.3 -> 28.6;  but 8, 8, 4000..40000 (2.25 units per row): 160 -> 180."""
-    units = sm_count // n_kv
+    8, 2, 500..30000: 44.3 -> 28.6;  but 8, 8, 4000..40000 (2.25 units per row): 160 -> 180.
+    Rows of equal length can leave up to a third of a wave idle where there are two or three units per row (7 rows of 18 units: 2 each).  Where two
+    waves of shorter ranges would then be faster by 8 %, the units are those of two waves, and the kernel, which sees the lengths, decides; a CTA
+    takes about 8.7 us + 0.22 us per tile here.  One wave -> this:  slots 7, 8, 16000 each: 119.1 -> 108.6;  13, 4, 12000 each: 92.4 -> 86.1;  7, 8,
+    8000..16000: 92.4 -> 92.4;  but up to 3 us for CTAs that find nothing to do where few rows are long (13, 4, 2400 and one of 16000: 27.0 -> 30.3)."""
+    units, two = sm_count // n_kv, 2 * sm_count // n_kv
     if not 2 <= B <= 32 or units < (2 if S <= 16384 else 4) * B:
         return 0
+    tiles = -(-S // 16)
+    if units < 4 * B and 1.08 * 2 * (8.7 + 0.22 * -(-tiles // (two // B))) < 8.7 + 0.22 * -(-tiles // (units // B)):
+        units = two
     return min(units, B * -(-max(S, 1) // 64))
 
 

@@ -229,8 +229,8 @@ int gaac_decode_attn_exchange(const gaac_side* K, const gaac_side* V, const void
                               void* stream);
 
 /* gaac_decode_attn for a ragged batch of at most 32 rows: instead of nsplit equal parts of every row, the rows share `units` ranges per kv head
- * (units >= B) in proportion to their lengths, which the kernel reads itself: n_kv * units CTAs, at most as many as the GPU has SMs for one
- * even wave (a slot's first head stands for all of its heads).  workspace: gaac_attn_workspace_bytes(B, n_q, ceil(units / B)). */
+ * (units >= B) in proportion to their lengths, which the kernel reads itself: n_kv * units CTAs, as many as the GPU has SMs for one
+ * even wave; with more units than that the kernel uses two waves where the lengths make that faster (a slot's first head stands for all of its heads).  workspace: gaac_attn_workspace_bytes(B, n_q, ceil(units / B)). */
 int gaac_decode_attn_balanced(const gaac_side* K, const gaac_side* V, const void* q_bf16, const int32_t* slot, int B, int n_q, int n_kv,
                               const int32_t* seq_len, int64_t S_pad, float scale, int units, const int32_t* tail_len, int tail_cap,
                               int n_base_rows, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* stream);

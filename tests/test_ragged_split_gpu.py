@@ -64,3 +64,43 @@ def test_paged_rows_share_by_length(monkeypatch, n_kv, G, lens):
         pk.paged_attention(to_bf16_cuda(q16), out, buf, st.raw, st.mt, bt, sl, st.bases, st.TS, n_q, n_kv, out_f32=o32)
         for b in range(B):
             assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b], vs[b], SCALE, (b, units))
+
+
+def test_two_waves_only_where_one_is_mostly_idle():
+    from gaac_b200.kernel import choose_units
+    two = {(B, n, S) for n in (1, 2, 4, 8) for B in range(2, 33) for S in (1000, 4000, 8000, 12000, 16000, 30000) if choose_units(B, n, S) * n > 148}
+    assert two == {(B, n, S) for n, rows in ((8, (7,)), (4, (13, 14)), (2, range(25, 30))) for B in rows for S in (12000, 16000)}
+    assert all(choose_units(B, n, S) * n <= 296 for B, n, S in two)
+
+
+# units of two waves: rows of equal length that fit a second wave better, and ragged ones whose CTAs behind the first wave find nothing to do
+@pytest.mark.gpu
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("lens", [[4100] * 7, [3000, 60, 4100, 0, 700, 16, 1999]])
+def test_units_of_two_waves(monkeypatch, paged, lens):
+    import torch
+    import gaac_b200.kv_cache as kvc
+    import gaac_b200.vllm.paged_kernel as pk
+    n_kv, G, B = 8, 4, 7
+    q16 = O.f32_to_bf16((np.random.default_rng(3).standard_normal((B, n_kv * G, 128)) * 0.1).astype(np.float32))
+    o32 = torch.empty(B, n_kv * G, 128, dtype=torch.float32, device="cuda")
+    if paged:
+        st, buf, bt, ks, vs = _build_paged([max(x, 1) for x in lens], n_kv, sum(-(-max(x, 1) // 16) for x in lens) + 4, seed=3)
+        call = lambda: pk.paged_attention(to_bf16_cuda(q16), torch.empty(B, n_kv * G * 128, dtype=torch.bfloat16, device="cuda"), buf, st.raw, st.mt, bt,
+                                          torch.tensor(lens, dtype=torch.int32, device="cuda"), st.bases, st.TS, n_kv * G, n_kv, out_f32=o32)
+    else:
+        cache = kvc.CompressedKVCache(n_slots=B, n_kv=n_kv, capacity=4112, bases=None)
+        ks, vs = ([np.ascontiguousarray(O.kv_like(n_kv, max(x, 1), 7 * s + i).transpose(1, 0, 2))[:x] for s, x in enumerate(lens)] for i in (1, 2))
+        for s in range(B):
+            cache.prefill(s, to_bf16_cuda(ks[s]), to_bf16_cuda(vs[s]), check=False)
+        call = lambda: cache.attention(to_bf16_cuda(q16), torch.arange(B, dtype=torch.int32, device="cuda"), SCALE, max_len=4100, out_f32=o32)
+    for units in (19, 37, 37, 40):
+        monkeypatch.setattr(kvc, "choose_units", lambda *a, u=units: u)
+        monkeypatch.setattr(pk, "choose_units", lambda *a, u=units: u)
+        o32.fill_(float("nan"))
+        call()
+        for b in range(B):
+            if lens[b]:
+                assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b][:lens[b]], vs[b][:lens[b]], SCALE, (b, units))
+            else:
+                assert not o32[b].any()
