@@ -267,14 +267,14 @@ template <int N> __device__ __forceinline__ void merge_warps(const uint8_t* area
     L += sh_l[at] * f; acc += sh_acc[at * ACC_LD + d] * f;
   }
 }
-// ---- V elements that are not finite.  In the value product a word meets a weight of zero for the other parity's channel, and the lower half of a
-// weight may be zero too: an infinite or NaN element makes its word's OTHER channel NaN as well (0 x Inf), and its own NaN where Inf is
+// ---- V elements that are not finite.  In the value product of groups up to 4 a word meets a weight of zero for the other parity's channel, and the lower
+// half of a weight may be zero or negative in any group: an infinite or NaN element makes its word's OTHER channel NaN as well (0 x Inf), and its own NaN where Inf is
 // right.  A CTA whose sum is not finite therefore takes its range once more in plain fp32, where an element meets its own weight only and tokens
 // behind the end meet none: range `split` of NS of (row, kv head) bh, straight from global memory, token by token, four channels per lane.  The
 // result lies where the warps of the main loop leave theirs.  Finite data never comes here, and what counts is what the presence of this code costs
 // the main loop: it looks everything up again and has little code and few registers.  32768 tokens, 8 kv heads: finite 33.8 -> 33.5 us, one infinite
-// element 608; GQA group 8: 66.5 -> 66.9 at 65536 tokens; head_dim 256: 36.1 -> 36.6, group 8 114.5 -> 118.  With the main loop's decoder in
-// its place a second pass took a fifth of that, but finite data 1 to 7 % more, inlined or called.
+// element 608; head_dim 256: finite 36.1 -> 36.5.  With the main loop's decoder in its place a second pass took a fifth of that, but finite data
+// 1 to 7 % more, inlined or called.
 template <bool PAGED, bool WIDE>
 __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, int bh, int split, int NS) {
   int tid = threadIdx.x;

@@ -9,9 +9,12 @@
 // Head columns.  The tensor-core tile has 8 columns.  Query heads are handled in sets of four (NSET = 1 for a GQA group of up to
 // 4, 2 for 5..8); lane j of a quad works for head 4 * set + j throughout:
 //   scores  S^T[16 tok x 8] = K[16 x 128] . Q^T : column 2j = head j of set 0, column 2j + 1 = head j of set 1 (zero without it)
-//   values  O^T += V^T . P^T : a rebuilt word holds TWO channels of one token, so the contraction runs over (token, channel parity)
-//           and column 2j + parity takes (P, 0) or (0, P): the words go into the product as they were decoded, with no transpose
-//           (32 byte permutes per tile before), and each lane gets both channels of its own head.
+//   values, one set: a rebuilt word holds TWO channels of one token, so O^T += V^T . P^T contracts over (token, channel parity) and column
+//           2j + parity takes (P, 0) or (0, P): the words go into the product as they were decoded, with no transpose, and each lane
+//           gets both channels of its own head.  16 products per tile, as many as a transposed form has for 8 heads
+//   values, two sets: the columns are the heads, as for the scores, and the words of two tokens are transposed by 32 byte permutes per tile.  The form
+//           above takes 32 products and 16 registers of weights where this takes 16 and 4, and was slower: group of 8, 8 kv heads, 65536
+//           tokens 67.1 us, now 64.4; paged 32768 40.1 -> 38.7; head_dim 256, 8 x 8000: 119 -> 111
 #pragma once
 #include <cuda_bf16.h>
 #include <math_constants.h>
@@ -21,10 +24,11 @@ namespace gaac {
 
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
-__device__ __forceinline__ void mma16816(float* c, u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
+__device__ __forceinline__ void mma16816(float& c0, float& c1, float& c2, float& c3, u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+               : "+f"(c0), "+f"(c1), "+f"(c2), "+f"(c3) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma16816(float* c, u32 a0, u32 a1, u32 a2, u32 a3, u32 b0, u32 b1) { mma16816(c[0], c[1], c[2], c[3], a0, a1, a2, a3, b0, b1); }
 // ---- bulk asynchronous copies (TMA engine, no tensor map): global -> shared, completion counted in bytes on an mbarrier.
 // Both addresses are 16-byte aligned and the size is a multiple of 16 at every call site.
 __device__ __forceinline__ void mbar_init(u32 mbar, u32 count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(count)); }
@@ -91,9 +95,36 @@ __device__ __forceinline__ void load_q(QFrag& Q, const uint16_t* q0, long head_s
   }
 }
 
-// Weights of one tile as B-fragments of the value product: [0]: tokens 2j (b0) and 2j + 1 (b1), [1]: tokens 2j + 8 and 2j + 9.  A weight enters as the
-// sum of two BF16 numbers, its rounded value (hi) and the rounded remainder (lo), which brings its relative error to 2^-16.
-template <int NSET> struct PFrag { u32 hi[NSET][2][2], lo[NSET][2][2]; };
+// Weights of one tile as B-fragments of the value product.  A weight enters as the sum of two BF16 numbers, its rounded value (hi) and the rounded
+// remainder (lo), which brings its relative error to 2^-16.  One set: [0]: tokens 2j (b0) and 2j + 1 (b1), [1]: tokens 2j + 8 and 2j + 9.  Two: [0]:
+// tokens 2j, 2j + 1, [1]: tokens 2j + 8, 2j + 9.
+template <int NSET> struct PFrag;
+template <> struct PFrag<1> { u32 hi[2][2], lo[2][2]; };
+template <> struct PFrag<2> { u32 hi[2], lo[2]; };
+__device__ __forceinline__ u32 pack_bf16(float lo, float hi) { __nv_bfloat162 x = __floats2bfloat162_rn(lo, hi); return *reinterpret_cast<u32*>(&x); }
+// what the rounding of a pair dropped, which fp32 holds exactly, rounded in turn
+__device__ __forceinline__ u32 pack_rest(float lo, float hi, u32 rounded) { return pack_bf16(lo - __uint_as_float(rounded << 16), hi - __uint_as_float(rounded & 0xFFFF0000u)); }
+
+// p0, p8: this lane's weights of tokens r and r + 8 for head j of each set.
+// One set: as column r of the value product the lane needs those of head r >> 1 for tokens 2j, 2j + 1, 2j + 8, 2j + 9, in the low (parity 0) or high
+// (parity 1) half of a word whose other half is zero.
+__device__ __forceinline__ void put_weights(PFrag<1>& P, const float (&p0)[1], const float (&p8)[1], int lane) {
+  const int j = lane & 3, r = lane >> 2, src = 8 * j + (r >> 1);
+  const u32 sel0 = (r & 1) ? 0x1044u : 0x4410u, sel8 = (r & 1) ? 0x3244u : 0x4432u;
+  const u32 H = pack_bf16(p0[0], p8[0]), L = pack_rest(p0[0], p8[0], H);
+  const u32 ha = __shfl_sync(FULLM, H, src), hb = __shfl_sync(FULLM, H, src + 4), la = __shfl_sync(FULLM, L, src), lb = __shfl_sync(FULLM, L, src + 4);
+  P.hi[0][0] = prmt(ha, 0u, sel0); P.hi[0][1] = prmt(hb, 0u, sel0); P.hi[1][0] = prmt(ha, 0u, sel8); P.hi[1][1] = prmt(hb, 0u, sel8);
+  P.lo[0][0] = prmt(la, 0u, sel0); P.lo[0][1] = prmt(lb, 0u, sel0); P.lo[1][0] = prmt(la, 0u, sel8); P.lo[1][1] = prmt(lb, 0u, sel8);
+}
+// Two: column r is head r >> 1 of set r & 1, its words hold two tokens.
+__device__ __forceinline__ void put_weights(PFrag<2>& P, const float (&p0)[2], const float (&p8)[2], int lane) {
+  const int j = lane & 3, r = lane >> 2, src = 8 * j + (r >> 1);
+  const u32 sel = (r & 1) ? 0x7632u : 0x5410u;
+  const u32 h0 = pack_bf16(p0[0], p0[1]), h8 = pack_bf16(p8[0], p8[1]), l0 = pack_rest(p0[0], p0[1], h0), l8 = pack_rest(p8[0], p8[1], h8);
+  const u32 a0 = __shfl_sync(FULLM, h0, src), b0 = __shfl_sync(FULLM, h0, src + 4), a8 = __shfl_sync(FULLM, h8, src), b8 = __shfl_sync(FULLM, h8, src + 4);
+  const u32 c0 = __shfl_sync(FULLM, l0, src), d0 = __shfl_sync(FULLM, l0, src + 4), c8 = __shfl_sync(FULLM, l8, src), d8 = __shfl_sync(FULLM, l8, src + 4);
+  P.hi[0] = prmt(a0, b0, sel); P.hi[1] = prmt(a8, b8, sel); P.lo[0] = prmt(c0, d0, sel); P.lo[1] = prmt(c8, d8, sel);
+}
 
 // Online softmax on the score fragment.  The running maximum is only raised (and the accumulators rescaled) when some score of the
 // tile exceeds it by more than RESCALE_TAU in the exp2 domain; otherwise the tile is weighted against the stale maximum, so P stays
@@ -102,7 +133,7 @@ template <int NSET> struct PFrag { u32 hi[NSET][2][2], lo[NSET][2][2]; };
 constexpr float RESCALE_TAU = 16.f;
 template <int NSET, bool FULL_TILE>
 __device__ __forceinline__ void softmax_step(WarpAcc<NSET>& A, const float* sc, float scale_log2, int nvalid, int lane, PFrag<NSET>& P) {
-  const int j = lane & 3, r = lane >> 2;
+  const int r = lane >> 2;
   float s0[NSET], s8[NSET];
   bool over = false;
 #pragma unroll
@@ -123,34 +154,31 @@ __device__ __forceinline__ void softmax_step(WarpAcc<NSET>& A, const float* sc, 
       for (int i = 0; i < 4; i++) { A.acc[s][i][0] *= al; A.acc[s][i][1] *= al; A.acc[s][i][2] *= al; A.acc[s][i][3] *= al; }
     }
   }
-  // this lane has the weights of tokens r and r + 8 for head j; as column r of the value product it needs those of head r >> 1 for tokens
-  // 2j, 2j + 1, 2j + 8, 2j + 9, in the low (parity 0) or high (parity 1) half of a word whose other half is zero
-  const int src = 8 * j + (r >> 1);
-  const u32 sel0 = (r & 1) ? 0x1044u : 0x4410u, sel8 = (r & 1) ? 0x3244u : 0x4432u;
+  float p0[NSET], p8[NSET];
 #pragma unroll
   for (int s = 0; s < NSET; s++) {
     const float mu = fmaxf(A.m[s], -1e30f);                                          // a maximum of -inf (nothing seen yet) must not produce inf - inf
-    const float p0 = fast_exp2(s0[s] - mu), p8 = fast_exp2(s8[s] - mu);
-    A.l[s] += p0 + p8;
-    __nv_bfloat162 h = __floats2bfloat162_rn(p0, p8);
-    const u32 H = *reinterpret_cast<u32*>(&h);
-    __nv_bfloat162 l = __floats2bfloat162_rn(p0 - __uint_as_float(H << 16), p8 - __uint_as_float(H & 0xFFFF0000u));      // the remainders are exact in fp32
-    const u32 L = *reinterpret_cast<u32*>(&l);
-    const u32 ha = __shfl_sync(FULLM, H, src), hb = __shfl_sync(FULLM, H, src + 4), la = __shfl_sync(FULLM, L, src), lb = __shfl_sync(FULLM, L, src + 4);
-    P.hi[s][0][0] = prmt(ha, 0u, sel0); P.hi[s][0][1] = prmt(hb, 0u, sel0); P.hi[s][1][0] = prmt(ha, 0u, sel8); P.hi[s][1][1] = prmt(hb, 0u, sel8);
-    P.lo[s][0][0] = prmt(la, 0u, sel0); P.lo[s][0][1] = prmt(lb, 0u, sel0); P.lo[s][1][0] = prmt(la, 0u, sel8); P.lo[s][1][1] = prmt(lb, 0u, sel8);
+    p0[s] = fast_exp2(s0[s] - mu); p8[s] = fast_exp2(s8[s] - mu);
+    A.l[s] += p0[s] + p8[s];
   }
+  put_weights(P, p0, p8, lane);
 }
 
 // Value product of words i, i + 1 (i = 2 * mt) of the lane's four tokens (2j, 2j + 1, 2j + 8, 2j + 9).
-template <int NSET>
-__device__ __forceinline__ void pv_words(WarpAcc<NSET>& A, int mt, const u32 (&w0)[4], const u32 (&w1)[4], const PFrag<NSET>& P) {
+__device__ __forceinline__ void pv_words(WarpAcc<1>& A, int mt, const u32 (&w0)[4], const u32 (&w1)[4], const PFrag<1>& P) {
+  mma16816(A.acc[0][mt], w0[0], w1[0], w0[1], w1[1], P.hi[0][0], P.hi[0][1]);
+  mma16816(A.acc[0][mt], w0[0], w1[0], w0[1], w1[1], P.lo[0][0], P.lo[0][1]);
+  mma16816(A.acc[0][mt], w0[2], w1[2], w0[3], w1[3], P.hi[1][0], P.hi[1][1]);
+  mma16816(A.acc[0][mt], w0[2], w1[2], w0[3], w1[3], P.lo[1][0], P.lo[1][1]);
+}
+__device__ __forceinline__ void pv_words(WarpAcc<2>& A, int mt, const u32 (&w0)[4], const u32 (&w1)[4], const PFrag<2>& P) {
 #pragma unroll
-  for (int s = 0; s < NSET; s++) {
-    mma16816(A.acc[s][mt], w0[0], w1[0], w0[1], w1[1], P.hi[s][0][0], P.hi[s][0][1]);
-    mma16816(A.acc[s][mt], w0[0], w1[0], w0[1], w1[1], P.lo[s][0][0], P.lo[s][0][1]);
-    mma16816(A.acc[s][mt], w0[2], w1[2], w0[3], w1[3], P.hi[s][1][0], P.hi[s][1][1]);
-    mma16816(A.acc[s][mt], w0[2], w1[2], w0[3], w1[3], P.lo[s][1][0], P.lo[s][1][1]);
+  for (int h = 0; h < 2; h++) {                      // the two channels of word i + h are rows r and r + 8
+    const u32 (&w)[4] = h ? w1 : w0;
+    const u32 a0 = prmt(w[0], w[1], 0x5410), a1 = prmt(w[0], w[1], 0x7632), a2 = prmt(w[2], w[3], 0x5410), a3 = prmt(w[2], w[3], 0x7632);
+    float &c0 = A.acc[0][mt][2 * h], &c1 = A.acc[1][mt][2 * h], &c2 = A.acc[0][mt][2 * h + 1], &c3 = A.acc[1][mt][2 * h + 1];
+    mma16816(c0, c1, c2, c3, a0, a1, a2, a3, P.hi[0], P.hi[1]);
+    mma16816(c0, c1, c2, c3, a0, a1, a2, a3, P.lo[0], P.lo[1]);
   }
 }
 
@@ -314,7 +342,7 @@ __device__ __forceinline__ void v_decode(WarpAcc<NSET>& A, const SideView& s, co
     for (int h = 0; h < 2; h++) {
       const u32 w0[4] = {f[0][2 * h], f[1][2 * h], f[2][2 * h], f[3][2 * h]};
       const u32 w1[4] = {f[0][2 * h + 1], f[1][2 * h + 1], f[2][2 * h + 1], f[3][2 * h + 1]};
-      pv_words<NSET>(A, 2 * g + h, w0, w1, P);
+      pv_words(A, 2 * g + h, w0, w1, P);
     }
   }
 }
@@ -360,7 +388,7 @@ __device__ __forceinline__ void raw_accum(WarpAcc<NSET>& A, const uint16_t* vraw
         o[0] = (uint16_t)e0; o[8] = (uint16_t)e1; o[16] = (uint16_t)e2; o[24] = (uint16_t)e3;
       }
     }
-    pv_words<NSET>(A, mt, w0, w1, P);
+    pv_words(A, mt, w0, w1, P);
   }
 }
 
