@@ -713,20 +713,20 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 // (gaac/vllm/paged_kernel256.py:1-4): block = 2*n_kv half-heads x {K, V}, half-head hh = 2*kvh + half.  Two warps form a pair that
 // streams the same tiles: each warp owns one half - it stages and rebuilds its half's K tile, which yields a partial score, and
 // its half's V tile, which yields its 128 output dimensions.  The two partial scores meet in shared memory once per tile (one
-// 64-thread named barrier; the exchange slots alternate with the tile's parity so one barrier per tile is enough), after which
-// both warps run the same softmax step on the same numbers.  Tiles are handed to PAIRS from the CTA's counter; the even warp
-// takes the number and passes it through the exchange slot.  A warp whose bounded wait on its copies runs out says so in
-// the same slot, so that both warps of the pair leave the loop together and nobody is left at the barrier.
+// 64-thread named barrier is enough: a warp leaves its scores in its stage, over the K tile that it is done with, which is filled
+// again only behind the next tile's barrier), after which both warps run the same softmax step on the same numbers.  Tiles are
+// handed to PAIRS from the CTA's counter; the even warp takes the number and passes it on through shared memory.  A warp whose
+// bounded wait on its copies runs out says so in the same place, so that both warps of the pair leave the loop together and
+// nobody is left at the barrier.
 // Output: partials of "virtual heads" vq = 2 * query head + half, which the last CTA of a (row, kv head) merges into out [B, n_q, 256].
 
 constexpr int META256_TILES = 128;
-constexpr int PSLOT256 = SLOT_OVF_OFF + 144;                       // staged bytes of a tile slot, at most (what shared memory has room for)
-constexpr int XCH_PAR_BYTES = 2 * 32 * 16 + 16;                    // one parity: two halves x 32 lanes x float4, then {next tile, fail flag of half 0, of half 1, -}
-constexpr int T256_BASES = LUTX_BYTES, T256_ZERO = T256_BASES + 2 * BASES_BYTES, T256_META = T256_ZERO + 16, T256_XCH = T256_META + META256_TILES * 16;
-constexpr int T256_SCRATCH = T256_XCH + (ATT_WARPS / 2) * 2 * XCH_PAR_BYTES, T256_RING = T256_SCRATCH + ATT_WARPS * WARP_SCRATCH;
-constexpr int STAGE256_BYTES = 16 + 2 * PSLOT256, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
+constexpr int CTL_BYTES = 16;                                      // of a pair and tile parity: {next tile, fail flag of half 0, of half 1, -}
+constexpr int T256_BASES = LUTX_BYTES, T256_ZERO = T256_BASES + 2 * BASES_BYTES, T256_META = T256_ZERO + 16, T256_CTL = T256_META + META256_TILES * 16;
+constexpr int T256_SCRATCH = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SCRATCH + ATT_WARPS * WARP_SCRATCH;
+constexpr int STAGE256_BYTES = 16 + 2 * PSLOT, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
 constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES;
-static_assert(T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_XCH % 16 == 0 && ATT256_SMEM + 64 <= 232448, "one CTA per SM");
+static_assert(T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 64 <= 232448, "one CTA per SM");
 
 template <int NSET>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   const u32 smem_s = (u32)__cvta_generic_to_shared(smem), ring_s = smem_s + ring;
   if (tid < 256) fill_lutx(reinterpret_cast<u32x2*>(smem), tid);
   if (tid >= 256 && tid < 260) reinterpret_cast<u32*>(smem + T256_ZERO)[tid - 256] = 0u;
-  for (int i = tid; i < (ATT_WARPS / 2) * 2 * XCH_PAR_BYTES / 4; i += ATT_THREADS) reinterpret_cast<u32*>(smem + T256_XCH)[i] = 0u;      // exchange slots start out zero
+  if (tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
   if (lane == 0) {
     mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   const int S = __shfl_sync(FULLM, p.seq_len[b], 0);
   const int ntiles = (S + 15) >> 4, chunk = (ntiles + p.nsplit - 1) / p.nsplit;
   const int tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo);
-  uint8_t* xch = smem + T256_XCH + pair * (2 * XCH_PAR_BYTES);
+  int* const ctl_pair = reinterpret_cast<int*>(smem + T256_CTL + pair * (2 * CTL_BYTES));
   const int4* meta_s = reinterpret_cast<const int4*>(smem + T256_META);        // per tile: mode-table entries of {K, V} of half 0, of half 1
   auto slot_of = [&](int i) { return p.bt[(long)b * p.bt_stride + tlo + i] * NT + 4 * kvh; };
   auto meta_of = [&](int i) -> TileMeta {
@@ -758,13 +758,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     const int pc = slot_of(i) + 2 * hf;
     return TileMeta{p.mt[pc], p.mt[pc + 1]};
   };
-  const u32 slot_bytes = (u32)min(p.TS, PSLOT256);
+  const u32 slot_bytes = (u32)min(p.TS, PSLOT);
   auto issue = [&](u32 st, const TileMeta& m) {                                // executed by lane 0
     // the stage may have been written through ordinary stores (patch numbers): order those before the copy engine's writes
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(st, (m.mk >= 0 ? slot_bytes : 0u) + (m.mv >= 0 ? slot_bytes : 0u));
     if (m.mk >= 0) bulk_g2s(st + 16, p.buf + (long)m.mk * p.TS, slot_bytes, st);
-    if (m.mv >= 0) bulk_g2s(st + 16 + PSLOT256, p.buf + (long)m.mv * p.TS, slot_bytes, st);
+    if (m.mv >= 0) bulk_g2s(st + 16 + PSLOT, p.buf + (long)m.mv * p.TS, slot_bytes, st);
   };
   int it = pair;
   TileMeta cur{0, 0};
@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
     const u32 esc = smem_s + so + SLOT_OVF_OFF;
     const SideView ks{stage, stage + SLOT_CD_OFF, stage + SLOT_FL_OFF, esc, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF, avail};
-    const SideView vs{stage + PSLOT256, stage + PSLOT256 + SLOT_CD_OFF, stage + PSLOT256 + SLOT_FL_OFF, esc + PSLOT256, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, avail};
+    const SideView vs{stage + PSLOT, stage + PSLOT + SLOT_CD_OFF, stage + PSLOT + SLOT_FL_OFF, esc + PSLOT, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, avail};
     TilePlan plan{};
     if (ok) {
       plan = plan_tile(ks, vs, cur.mk < 0, cur.mv < 0, W, lane);
@@ -809,12 +809,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
       else raw_scores<false>(sc, p.raw + (long)raw_tile(cur.mk) * (T * D), nvalid, lane, Q, nullptr);
     }
     // ---- the two halves' partial scores meet; the next tile's number and a failed wait travel with them
-    uint8_t* slot = xch + par * XCH_PAR_BYTES;
-    reinterpret_cast<float4*>(slot + hf * 512)[lane] = make_float4(sc[0], sc[1], sc[2], sc[3]);
-    int* ctl = reinterpret_cast<int*>(slot + 1024);
+    __syncwarp();                                      // every lane is done with the K tile
+    reinterpret_cast<float4*>(smem + so)[lane] = make_float4(sc[0], sc[1], sc[2], sc[3]);
+    int* ctl = ctl_pair + par * (CTL_BYTES / 4);
     if (lane == 0) { if (hf == 0) ctl[0] = t1; if (!ok) ctl[1 + hf] = 1; }
     asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
-    const float4 other = reinterpret_cast<const float4*>(slot + (hf ^ 1) * 512)[lane];
+    const float4 other = reinterpret_cast<const float4*>(smem + so + (hf ? -WARP256_BYTES : WARP256_BYTES))[lane];      // the same stage of the other warp
     sc[0] += other.x; sc[1] += other.y; sc[2] += other.z; sc[3] += other.w;
     t1 = ctl[0];
     const bool failed = (ctl[1] | ctl[2]) != 0;
