@@ -155,9 +155,11 @@ __global__ void __launch_bounds__(32) paged_store_kernel(const __grid_constant__
 }
 
 // The same for a step of few tiles, as ONE cluster: the cluster's barrier stands between the pops and the pushes, so no second launch is needed to
-// return the raw tiles.  A warp per tile: 8 blocks x 10 warps, which covers 5 sequences of 8 kv heads (larger steps would put several tiles on a
-// warp one after the other, and their second launch is hidden behind the work).
-constexpr int STEP_WARPS = 10, STEP_CLUSTER = 8;
+// return the raw tiles.  A warp per tile, 8 blocks (the portable cluster size) of as many warps as 48 KB of static shared memory have room for.  us per
+// call, two launches -> this: 16 to 80 tiles 3.0 -> 2.5 where no block completes, 4.2 -> 3.9 where all do.  With 16 warps (128 tiles) steps of 96
+// to 128 tiles take 2.8 -> 2.5 and 4.0 -> 4.3, and completing blocks in smaller steps 0.3 more: the warps of an SM share its units while they encode.
+constexpr int STEP_WARPS = 11, STEP_CLUSTER = 8;
+static_assert(STEP_WARPS * sizeof(WarpScratch) <= 48 * 1024 && (STEP_WARPS + 1) * sizeof(WarpScratch) > 48 * 1024, "");
 __global__ void __launch_bounds__(STEP_WARPS * 32) paged_store_step_kernel(const __grid_constant__ PagedParams p, int n_items) {
   __shared__ __align__(16) WarpScratch ws[STEP_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * STEP_WARPS + warp, NT = 2 * p.st.n_kv;

@@ -8,7 +8,7 @@ from oracle import gaac_oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("E", [1, 4, 40, 41, 60])    # 2 * E tile slots; up to 80 are one launch
+@pytest.mark.parametrize("E", [1, 4, 11, 12, 44, 45, 60])    # 2 * E tile slots; up to 88 are one launch, of 11 per block
 @pytest.mark.parametrize("short", [1, 2])
 @pytest.mark.parametrize("end", ["fill", "release"])
 def test_pool_runs_empty(E, short, end):
