@@ -495,12 +495,18 @@ extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, co
   cudaStream_t st = (cudaStream_t)stream;
   const long n_ch = (long)n_kv * D, at = (long)slot * n_ch;
   int* hist = reinterpret_cast<int*>(scratch);
-  cudaMemsetAsync(hist, 0, gaac_cache_calibrate_scratch_bytes(n_kv), st);
+  if (cudaMemsetAsync(hist, 0, gaac_cache_calibrate_scratch_bytes(n_kv), st) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
   const HistParams<int> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + n_ch * 256}, L, n_ch, row_stride};
   exponent_hist_kernel<<<hist_grid(n_ch, L, 2), 128 * HIST_LANES, 0, st>>>(hp);
   const BasesParams<int> bp{{hist, hist + n_ch * 256}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
                             {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch};
   return launch_overlapped(bases_from_hist_kernel<int>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
+}
+
+static int clear_status(int32_t* status, cudaStream_t st) {           // the words that say whether an escape stream had room
+  if (cudaMemsetAsync(status, 0, 4, st) == cudaSuccess && cudaMemsetAsync(status + 2, 0, 4, st) == cudaSuccess) return GAAC_OK;
+  cudaGetLastError();
+  return GAAC_E_LAUNCH;
 }
 
 extern "C" size_t gaac_cache_prefill_scratch_bytes(int64_t L, int n_kv) {
@@ -528,7 +534,7 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   if (n_items > 0x7FFFFFF0L) return GAAC_E_ARG;
   const FinishParams fin{(const uint16_t*)k_tok, (const uint16_t*)v_tok, row_stride, L, n_kv, h0, (uint16_t*)K->tail, (uint16_t*)V->tail, seq_len, tail_len, K->ovf_used, V->ovf_used, status};
   if (ntiles == 0) {
-    if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
+    if (copy_only) { if (int e = clear_status(status, st)) return e; }
     else prefill_finish_kernel<<<dim3((unsigned)n_kv, 2), 128, 0, st>>>(fin);
     return launch_status();
   }
@@ -551,7 +557,7 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   sp.ntiles = ntiles; sp.tile_off_stride = tiles_cap;
   cp.ntiles = ntiles; cp.n_items = (unsigned)n_items; cp.tile_off_stride = tiles_cap; cp.head_stride = ovf_cap; cp.head_cap = ovf_cap - CACHE_READ_PAD;
   cp.finish = !copy_only; cp.fin = fin;
-  if (copy_only) { cudaMemsetAsync(status, 0, 4, st); cudaMemsetAsync(status + 2, 0, 4, st); }
+  if (copy_only) { if (int e = clear_status(status, st)) return e; }
   else {
     encode_tiles_kernel<2><<<encode_grid(ntiles, n_kv, 2), ENC_WARPS * 32, 0, st>>>(ep);
     if (int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)n_kv, 2), SCAN_THREADS, st, sp)) return e;
