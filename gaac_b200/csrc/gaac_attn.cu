@@ -199,7 +199,7 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area,
 // of 37).  A second wave costs a prologue, about as long as 40 tiles; CTAs that find nothing to do cost 12.
 constexpr int SHARE_MAX_ROWS = 32, SHARE_MIN_TILES = 4, SHARE_WAVE_TILES = 40 - 12;
 __device__ __forceinline__ void row_share(int tiles, int B, int units, int wave, int u, int lane, int& row, int& split, int& NS) {
-  const unsigned n = lane < B ? (unsigned)tiles : 0u, total = __reduce_add_sync(FULLM, n), most = __reduce_max_sync(FULLM, n);
+  const unsigned n = lane < B ? (unsigned)max(tiles, 0) : 0u, total = __reduce_add_sync(FULLM, n), most = __reduce_max_sync(FULLM, n);
   auto smallest = [&](int units) {
     unsigned lo = max((unsigned)SHARE_MIN_TILES, (total + units - 1) / units);
     unsigned hi = max(lo, units > B ? (total + (units - B) - 1) / (units - B) : most);

@@ -104,3 +104,23 @@ def test_units_of_two_waves(monkeypatch, paged, lens):
                 assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b][:lens[b]], vs[b][:lens[b]], SCALE, (b, units))
             else:
                 assert not o32[b].any()
+
+
+# a row whose length is negative is an empty one, as it is where every row is split alike: its output is zero and its neighbours get their ranges
+@pytest.mark.gpu
+@pytest.mark.parametrize("units", [4, 9, 40])
+def test_negative_length_is_empty(monkeypatch, units):
+    import torch
+    import gaac_b200.vllm.paged_kernel as pk
+    n_kv, G, lens = 2, 4, [700, 64, 33, 1500]
+    st, buf, bt, ks, vs = _build_paged(lens, n_kv, 200, seed=9)
+    q16 = O.f32_to_bf16((np.random.default_rng(1).standard_normal((4, n_kv * G, 128)) * 0.3).astype(np.float32))
+    monkeypatch.setattr(pk, "choose_units", lambda *a: units)
+    for gone in (-1, -16, -40, -(1 << 20)):
+        sl = torch.tensor([700, gone, 33, 1500], dtype=torch.int32, device="cuda")
+        out = torch.full((4, n_kv * G * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+        o32 = torch.full((4, n_kv * G, 128), float("nan"), dtype=torch.float32, device="cuda")
+        pk.paged_attention(to_bf16_cuda(q16), out, buf, st.raw, st.mt, bt, sl, st.bases, st.TS, n_kv * G, n_kv, out_f32=o32)
+        assert not o32[1].any()
+        for b in (0, 2, 3):
+            assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b], vs[b], SCALE, (b, units, gone))
