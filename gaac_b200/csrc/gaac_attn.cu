@@ -928,16 +928,14 @@ __global__ void __launch_bounds__(128) combine_parts_kernel(const float* __restr
 // (rows of about equal length keep the grid's own numbering, which costs nothing).  One CTA; every thread finds the place of its
 // own row by counting the rows that come before it.
 constexpr int ORDER_MAX_ROWS = 1024;
-__global__ void __launch_bounds__(ORDER_MAX_ROWS) row_order_kernel(const int* __restrict__ seq_lens, const int* __restrict__ slot, int n_kv, int B,
-                                                                   int2* __restrict__ order) {
+__global__ void __launch_bounds__(ORDER_MAX_ROWS) row_order_kernel(const int* __restrict__ seq_lens, int B, int2* __restrict__ order) {
   __shared__ int len_s[ORDER_MAX_ROWS];
   __shared__ int mx_s, mn_s;
   const int t = threadIdx.x;
   asm volatile("griddepcontrol.wait;" ::: "memory");                   // resident early behind the previous kernel, as the attention kernels are
   asm volatile("griddepcontrol.launch_dependents;" ::);
   if (t == 0) { mx_s = 0; mn_s = 0x7fffffff; }
-  // paged layout: seq_lens[row]; slot layout: the tokens of the row's first head, seq_lens[slot[row] * n_kv] (0 for a padding row)
-  if (t < B) len_s[t] = slot ? (slot[t] < 0 ? 0 : seq_lens[(long)slot[t] * n_kv]) : seq_lens[t];
+  if (t < B) len_s[t] = seq_lens[t];
   __syncthreads();
   if (t < B) {
     const int mine = len_s[t];
@@ -976,13 +974,13 @@ static int carve_workspace(void* ws, size_t ws_bytes, int B, int n_q, int nsplit
   return GAAC_OK;
 }
 
-static void launch_row_order(const int* seq_lens, const int* slot, int n_kv, int B, int2* order, cudaStream_t st) {
+static void launch_row_order(const int* seq_lens, int B, int2* order, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(1); cfg.blockDim = dim3(ORDER_MAX_ROWS); cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, row_order_kernel, seq_lens, slot, n_kv, B, order) != cudaSuccess) cudaGetLastError();     // the attention launch that follows reports
+  if (cudaLaunchKernelEx(&cfg, row_order_kernel, seq_lens, B, order) != cudaSuccess) cudaGetLastError();     // the attention launch that follows reports
 }
 
 // Launch of an attention kernel, one CTA of ATT_THREADS per SM.  The permission for its shared memory is asked for once per kernel and device, not on every
@@ -1105,7 +1103,7 @@ static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride
   // ragged batches: CTAs are handed out longest row first (one small launch sorts the rows; its output is read by the attention
   // kernel after its dependency wait)
   if (!units && B > 1 && B <= ORDER_MAX_ROWS && (int64_t)B * st->n_kv * nsplit > sm_count_of_current_device()) {
-    launch_row_order(seq_lens, nullptr, 0, B, p.order_buf, (cudaStream_t)stream);
+    launch_row_order(seq_lens, B, p.order_buf, (cudaStream_t)stream);
     p.row_order = p.order_buf;
   }
   return launch_attn<true, false>(p, (cudaStream_t)stream);

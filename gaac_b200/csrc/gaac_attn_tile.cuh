@@ -36,7 +36,6 @@ __device__ __forceinline__ void mbar_expect_tx(u32 mbar, u32 bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void mbar_add_tx(u32 mbar, u32 bytes) { asm volatile("mbarrier.expect_tx.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory"); }
-__device__ __forceinline__ void mbar_arrive(u32 mbar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory"); }
 __device__ __forceinline__ void bulk_g2s(u32 dst, const void* src, u32 bytes, u32 mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
 }
@@ -224,10 +223,9 @@ __device__ __forceinline__ bool build_raw_patches(u32 raw_bits, const TilePlan& 
       const u32 below = (t.tags >> first) & ((1u << (bit - 1u - first)) - 1u);
       const u32 pl = (isv ? esc_v : esc_k) + lds_u16(mine + ((bit >> 2) << 1)) + seg_esc(below);
       const u32 k = base + (u32)popc(some & ((1u << lane) - 1u));
-      const u32 sh = 8u * (pl & 3u), w0 = lds_u32(pl & ~3u), w1 = lds_u32((pl & ~3u) + 4u);
-      const u32 lo = funnel_r(w0, w1, (int)sh), hi = w1 >> sh;         // bytes 0-3 and byte 4 of the payload
       const u32x4 bw = lds_u128(w.bases + (isv ? BASES_V + 32u * r + 8u * (bit & 2u) : 64u * j + 8u * (bit & 6u)));
-      sts_u64(w.scratch + 8u * k, spread_hi5_dev(lo & 0xFFFFFu) - (bw.x + bw.z), spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - (bw.y + bw.w));
+      const u32x2 x = raw_addends(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * (pl & 3u), bw.x + bw.z, bw.y + bw.w);
+      sts_u64(w.scratch + 8u * k, x.x, x.y);
       sts_u8(pl, k);
     }
     base = n;

@@ -1,5 +1,5 @@
-// Device pieces that the encoder, the decoder and the attention kernels share: multiply-add forms, where a lane's escape bytes lie, and the
-// rebuild of a group.
+// Device pieces that the encoder, the decoder and the attention kernels share: where a lane's escape bytes lie, and where the rebuild of a group gets
+// its addends from.  The arithmetic itself is in gaac_tile.h.
 #pragma once
 #include <cuda_runtime.h>
 #include "gaac_tile.h"
@@ -8,20 +8,10 @@ namespace gaac {
 
 constexpr unsigned FULLM = 0xffffffffu;
 
-// ---- byte-SWAR pieces written for the pipes of the SM: logic ops (LOP3 / PRMT / SHF) run on the ALU pipe, whose rate is half
-// the issue rate, so shifts that can be merged with an add are written as multiply-adds (FMA pipe)
-template <u32 K> __device__ __forceinline__ u32 mad_k(u32 a, u32 c) {
-  u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "n"(K), "r"(c)); return d;
-}
-__device__ __forceinline__ u32 mad(u32 a, u32 b, u32 c) { u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d; }
 // one step of an inclusive scan over a warp: v += v of the lane `d` below, where there is one
 __device__ __forceinline__ void scan_step(u32& v, int d) {
   asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
 }
-// Escape bytes of up to four groups whose tags are t (upper bits clear): one for a promoted group (tag 01), five for a raw one (11), which
-// is one bit per tag bit and three more copies of every upper bit.
-__device__ __forceinline__ u32 seg_esc(u32 t) { return (u32)popc((t & 0xAAu) * 0x01010100u + t); }
-
 // ---- escape positions of a lane's segments inside the tile side, for K, for V or (the attention kernels) for both in step.
 // K: the lanes of an octet are in the order of the tile's escape bytes, so ONE warp scan over both octets' segment sizes (packed in a word) gives
 //    every lane its two positions (kpos, low and high half).  k0, k1: tags of the lane's four groups in each octet (8 bits).
@@ -70,25 +60,6 @@ __device__ __forceinline__ u32x4 lds_u128(u32 a) { u32x4 v; asm volatile("ld.sha
 __device__ __forceinline__ void sts_u8(u32 a, u32 v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts_u64(u32 a, u32 x, u32 y) { asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
 __device__ __forceinline__ void sts_u128(u32 a, u32 x, u32 y, u32 z, u32 w) { asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory"); }
-__device__ __forceinline__ void bf16x4_dev(u32 sm4, u32 e4, u32& p01, u32& p23) {
-  const u32 eh = __umulhi(e4, 0x80000000u);                          // e4 >> 1
-  const u32 el = mad_k<128u>(e4, 0u);                                // e4 << 7
-  const u32 h4 = bits_of(sm4, eh, 0x80808080u), l4 = bits_of(el, sm4, 0x80808080u);
-  p01 = prmt(l4, h4, 0x5140); p23 = prmt(l4, h4, 0x7362);
-}
-// four 5-bit fields at bits 0..19 of u -> field << 3 per byte (raw-tier exponent high bits); same result as spread_hi5
-__device__ __forceinline__ u32 spread_hi5_dev(u32 u) {
-  const u32 y = mad_k<64u>(u & 0xFFC00u, u & 0x3FFu);               // fields 0,1 at bits 0-9, fields 2,3 at bits 16-25
-  return mad_k<64u>(y & 0x03E003E0u, (y & 0x001F001Fu) << 3);       // odd fields up 3 more bits, everything << 3
-}
-// The 24 code bits of a group, picked out of two neighbouring words by one byte permute that already puts codes 4..7 at the top:
-// bits 0..11 = codes 0..3, bits 20..31 = codes 4..7 (B = byte offset of the group in the lane's code string).
-template <int B> __device__ __forceinline__ u32 group_codes(const u32* cd) {
-  constexpr int i = B & 3;
-  constexpr u32 sel = (u32)i | (u32)(i + 1) << 4 | (u32)(i + 1) << 8 | (u32)(i + 2) << 12;
-  return prmt(cd[B >> 2], i >= 2 ? cd[(B >> 2) + 1] : 0u, sel);
-}
-
 // Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, pos =
 // position of the group's escape bytes, advanced past them.
 // WIN: the escape bytes are staged; pos counts from the zero byte (a group without an escape byte reads that), and raw groups were turned
@@ -100,44 +71,30 @@ template <int B> __device__ __forceinline__ u32 group_codes(const u32* cd) {
 template <bool WIN>
 __device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& pos, const uint8_t* glob, const WarpView& w, const u32x4& bw, u32 out[4]) {
   const u32 m1 = tg & 1u;                             // promoted (tags are 0, 1 or 3)
-  const u32 blo = mad(m1, bw.z, bw.x), bhi = mad(m1, bw.w, bw.y);
-  u32 x0, x1;
+  u32x2 x;
   if (WIN) {
     const u32 r2 = tg & 2u;                           // 2 for a raw group: its table is the patch table
     const u32 xe = lds_u8(mad(m1, pos, w.zero));
-    const u32x2 x = lds_u64(mad_k<8u>(xe, mad(r2, (w.scratch - w.lutx) >> 1, w.lutx)));
-    x0 = x.x; x1 = x.y;
+    x = lds_u64(mad_k<8u>(xe, mad(r2, (w.scratch - w.lutx) >> 1, w.lutx)));
     pos = mad_k<2u>(r2, pos);                         // a raw payload is five bytes: four here, one below with every promoted group
   } else {
-    const u32x2 x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
-    x0 = x.x; x1 = x.y;
-    if (tg & 2u) {                                    // raw exponents: e = code | hi5 << 3 (the base must not contribute)
+    x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
+    if (tg & 2u) {
       const uint8_t* p = glob + pos;
-      const int sh = 8 * (int)(reinterpret_cast<uintptr_t>(p) & 3);
       const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-      const u32 w0 = a[0], w1 = a[1];
-      const u32 lo = funnel_r(w0, w1, sh), hi = w1 >> sh;              // bytes 0-3 and byte 4 of the payload
-      x0 = spread_hi5_dev(lo & 0xFFFFFu) - blo;
-      x1 = spread_hi5_dev(funnel_r(lo, hi, 20) & 0xFFFFFu) - bhi;
+      x = raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
       pos += 4;
     }
   }
   pos += m1;
-  // four 3-bit codes -> four bytes in two steps; each step moves the upper fields with a multiply-add: (t & M) * (2^k - 1) + t
-  const u32 th = z >> 20;
-  const u32 xl = mad_k<1023u>(z & 0xFC0u, z & 0xFFFu), xh = mad_k<1023u>(th & 0xFC0u, th);
-  bf16x4_dev(sm_lo, mad_k<31u>(xl & 0x00380038u, xl) + blo + x0, out[0], out[1]);
-  bf16x4_dev(sm_hi, mad_k<31u>(xh & 0x00380038u, xh) + bhi + x1, out[2], out[3]);
+  rebuild_group(sm_lo, sm_hi, z, m1, bw, x, out);
 }
 
 // ---- base words of a side, {b3lo, b3hi, b4lo - b3lo, b4hi - b3hi} per group (16 bytes; K: lane class jj, group gg at 64 * jj + 16 * gg; V: lane class rr,
 // group gg at 32 * rr + 16 * gg).  Thread t < 32 makes word t of the 32 half groups: eight byte loads that do not wait for one another.
 template <bool VSIDE>
 __device__ __forceinline__ void fill_bases(uint8_t* bases, const uint8_t* b3, const uint8_t* b4, int t) {
-  int d0, d1, d2, d3;                                // channels of the half group (see k_base_words, v_base_words)
-  if (VSIDE) { d0 = 32 * (t & 3) + (t >> 2); d1 = d0 + 8; d2 = d0 + 16; d3 = d0 + 24; }
-  else { d0 = 16 * (t & 7) + 2 * (t >> 3); d1 = d0 + 1; d2 = d0 + 8; d3 = d0 + 9; }
-  const u32 w3 = (u32)b3[d0] | (u32)b3[d1] << 8 | (u32)b3[d2] << 16 | (u32)b3[d3] << 24, w4 = (u32)b4[d0] | (u32)b4[d1] << 8 | (u32)b4[d2] << 16 | (u32)b4[d3] << 24;
+  const u32 w3 = half_group_word<VSIDE>(b3, t), w4 = half_group_word<VSIDE>(b4, t);
   u32* o = reinterpret_cast<u32*>(bases + (VSIDE ? BASES_V : 0) + 16 * (t >> 1)) + (t & 1);
   o[0] = w3; o[2] = w4 - w3;
 }

@@ -1,5 +1,5 @@
 // Byte-SWAR building blocks of the GAAC tile format, shared by every kernel (encoder, decoder, fused attention).
-// All functions are __host__ __device__ so the bit logic can be exercised on the CPU by the test-suite.
+// All functions are __host__ __device__: the test-suite runs them on the CPU.
 //
 // Format facts used here (reference: gaac/codec.py:1-18,139-172; gaac/kernel.py:29-46):
 //   bf16 bits x  ->  e = (x >> 7) & 0xFF,  sm = ((x >> 8) & 0x80) | (x & 0x7F)
@@ -65,6 +65,23 @@ GAAC_HD int popc(u32 x) {
 #endif
 }
 
+// ---- multiply-adds.  Logic ops (LOP3 / PRMT / SHF) run on the ALU pipe, whose rate is half the issue rate, so shifts that can be merged with an add are
+// written as multiply-adds (FMA pipe)
+template <u32 K> GAAC_HD u32 mad_k(u32 a, u32 c) {
+#if defined(__CUDA_ARCH__)
+  u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "n"(K), "r"(c)); return d;
+#else
+  return a * K + c;
+#endif
+}
+GAAC_HD u32 mad(u32 a, u32 b, u32 c) {
+#if defined(__CUDA_ARCH__)
+  u32 d; asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c)); return d;
+#else
+  return a * b + c;
+#endif
+}
+
 // ---- tags -> escape byte counts --------------------------------------------------------------------------------
 // escape bytes of a row with tag word fl (tier 1 -> 1 byte, tier 2 -> 5 bytes)                  gaac/kernel.py:46
 GAAC_HD int row_esc_bytes(u32 fl) { return popc(fl & 0x55555555u) + 4 * popc(fl & 0xAAAAAAAAu); }
@@ -74,34 +91,28 @@ GAAC_HD int esc_prefix(u32 fl, int bits) {
   return popc(low & 0x55555555u) + 4 * popc(low & 0xAAAAAAAAu);
 }
 
+// Escape bytes of up to four groups whose tags are t (upper bits clear): one for a promoted group (tag 01), five for a raw one (11), which
+// is one bit per tag bit and three more copies of every upper bit.
+GAAC_HD u32 seg_esc(u32 t) { return (u32)popc((t & 0xAAu) * 0x01010100u + t); }
+
 // ---- decode side -----------------------------------------------------------------------------------------------
-// four 3-bit codes at bits 0..11 of u (higher bits ignored) -> one code per byte
-GAAC_HD u32 spread_codes4(u32 u) {
-  u32 v = u & 0xFFFu;
-  u32 y = (v | (v << 10)) & 0x003F003Fu;
-  return (y | (y << 5)) & 0x07070707u;
-}
 // four 1-bit flags at bits 0..3 of n (n < 16) -> 8 * flag per byte (the 4th bit of a 4-bit window code)
 GAAC_HD u32 spread_bit4(u32 n) { return (n * 0x01020408u) & 0x08080808u; }
-// four 5-bit fields at bits 0..19 of u (higher bits ignored) -> field << 3 per byte (raw-tier exponent high bits)
+// four 5-bit fields at bits 0..19 of u (the others clear) -> field << 3 per byte (raw-tier exponent high bits)
 GAAC_HD u32 spread_hi5(u32 u) {
-  u32 v = u & 0xFFFFFu;
-  u32 y = (v & 0x3FFu) | ((v << 6) & 0x03FF0000u);            // fields (0,1) in the low half, (2,3) in the high half
-  u32 z = (y & 0x001F001Fu) | ((y << 3) & 0x1F001F00u);       // one field per byte
-  return z << 3;
+  const u32 y = mad_k<64u>(u & 0xFFC00u, u & 0x3FFu);               // fields 0,1 at bits 0-9, fields 2,3 at bits 16-25
+  return mad_k<64u>(y & 0x03E003E0u, (y & 0x001F001Fu) << 3);       // odd fields up 3 more bits, everything << 3
 }
 // sign/mantissa bytes (4) + exponent bytes (4) -> bf16 pairs (elements 0,1) and (2,3)             gaac/kernel.py:34-36
 GAAC_HD void bf16x4(u32 sm4, u32 e4, u32& p01, u32& p23) {
-  u32 h4 = (sm4 & 0x80808080u) | ((e4 >> 1) & 0x7F7F7F7Fu);
-  u32 l4 = ((e4 << 7) & 0x80808080u) | (sm4 & 0x7F7F7F7Fu);
-  p01 = prmt(l4, h4, 0x5140);
-  p23 = prmt(l4, h4, 0x7362);
-}
-// 12-bit code field number s (0..7) of a 96-bit little-endian string held in c[0..2]
-GAAC_HD u32 code_field12(const u32* c, int s) {
-  int p = 12 * s;
-  u32 lo = c[p >> 5], hi = (p >> 5) < 2 ? c[(p >> 5) + 1] : 0u;
-  return funnel_r(lo, hi, p & 31);
+#if defined(__CUDA_ARCH__)
+  const u32 eh = __umulhi(e4, 0x80000000u);                          // e4 >> 1
+#else
+  const u32 eh = e4 >> 1;
+#endif
+  const u32 el = mad_k<128u>(e4, 0u);                                // e4 << 7
+  const u32 h4 = bits_of(sm4, eh, 0x80808080u), l4 = bits_of(el, sm4, 0x80808080u);
+  p01 = prmt(l4, h4, 0x5140); p23 = prmt(l4, h4, 0x7362);
 }
 
 // ---- encode side -----------------------------------------------------------------------------------------------
@@ -112,6 +123,13 @@ GAAC_HD void split_bytes4(u32 l4, u32 h4, u32& sm4, u32& e4) {
 }
 // two bf16 pairs (elements 0,1) (2,3) -> sign/mantissa bytes and exponent bytes
 GAAC_HD void split_bf16x4(u32 p01, u32 p23, u32& sm4, u32& e4) { split_bytes4(prmt(p01, p23, 0x6420), prmt(p01, p23, 0x7531), sm4, e4); }
+// four channels of two tokens, one word per channel (low half: the first token), -> the same for each token: a byte transpose sorts them by token and by
+// low / high byte
+GAAC_HD void split_token_pairs(u32 x0, u32 x1, u32 x2, u32 x3, u32& sm_a, u32& e_a, u32& sm_b, u32& e_b) {
+  const u32 p = prmt(x0, x1, 0x5140), q = prmt(x2, x3, 0x5140), p2 = prmt(x0, x1, 0x7362), q2 = prmt(x2, x3, 0x7362);
+  split_bytes4(prmt(p, q, 0x5410), prmt(p, q, 0x7632), sm_a, e_a);
+  split_bytes4(prmt(p2, q2, 0x5410), prmt(p2, q2, 0x7632), sm_b, e_b);
+}
 // bit 3 of each byte of lo (bits 0-3 of the result) and of hi (bits 4-7): the fields are 8 bits apart, so one multiply brings them side by side
 GAAC_HD u32 pack_bit4x2(u32 lo, u32 hi) { return (((hi & 0x08080808u) * 16u + (lo & 0x08080808u)) * 0x00204081u) >> 24; }
 // (byte >> 3) of each byte -> 20 bits
@@ -142,22 +160,4 @@ GAAC_HD u32 encode_group_codes(u32 e_lo, u32 e_hi, u32 b3_lo, u32 b3_hi, u32 b4_
 }
 // Escape payload of a raw group: the upper five bits of its eight exponents, 40 bits.
 GAAC_HD u64 raw_payload(u32 e_lo, u32 e_hi) { return (u64)pack_hi5(e_lo) | ((u64)pack_hi5(e_hi) << 20); }
-// The same with the payload of whatever tier came out (0 / one byte / 40 bits).
-GAAC_HD u32 encode_group(u32 e_lo, u32 e_hi, u32 b3_lo, u32 b3_hi, u32 b4_lo, u32 b4_hi, u32& codes24, u64& esc) {
-  u32 esc1;
-  const u32 tag = encode_group_codes(e_lo, e_hi, b3_lo, b3_hi, b4_lo, b4_hi, codes24, esc1);
-  esc = tag == 0u ? 0u : (tag == 1u ? (u64)esc1 : raw_payload(e_lo, e_hi));
-  return tag;
-}
-
-// Rebuild the exponent bytes of one half group (4 stored positions).
-//   code12: the four 3-bit codes; tag: 0/1/3; half: 0 = elements 0-3, 1 = elements 4-7 of the group;
-//   esc: escape payload of the group (tier 1: one byte, tier 2: 40 bits), ignored for tier 0.
-GAAC_HD u32 decode_half_group(u32 code12, u32 tag, int half, u64 esc, u32 b3w, u32 b4w) {
-  u32 c4 = spread_codes4(code12);
-  if (tag == 0u) return b3w + c4;
-  if (tag == 1u) return b4w + c4 + spread_bit4((u32)(esc >> (4 * half)) & 0xFu);
-  return c4 | spread_hi5((u32)(esc >> (20 * half)));
-}
-
 }  // namespace gaac

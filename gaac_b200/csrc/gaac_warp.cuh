@@ -82,11 +82,6 @@ template <bool TRANS> __device__ __forceinline__ void load_matrices(u32 (&w)[4],
 __device__ __forceinline__ u32 matrix_row_address(const WarpScratch& ws, int lane) {
   return (u32)__cvta_generic_to_shared(&ws.xs[(8 * (lane >> 4) + (lane & 7)) * XS_STRIDE + 8 * ((lane >> 3) & 1)]);
 }
-// Four groups of 24 code bits (bits 24..31 ignored) -> 96 bits
-__device__ __forceinline__ void join_codes(u32 c0, u32 c1, u32 c2, u32 c3, u32* cd) {
-  cd[0] = prmt(c0, c1, 0x4210); cd[1] = prmt(c1, c2, 0x5421); cd[2] = prmt(c2, c3, 0x6542);
-}
-
 // Encode the staged tile.  Rows >= nvalid become empty rows (sm = 0, codes = 0, tag word 0); they must have been staged as zeros.  On return
 // every lane holds its share in `lt` and the tile's escape byte count is returned (same in all lanes).
 // Bound by instruction issue: 16-bit loads one by one, a byte-exact subtraction per window, a table of tags in shared memory and a branch per
@@ -121,12 +116,7 @@ __device__ __forceinline__ int encode_tile_warp(WarpScratch& ws, int nvalid, con
         u32 a[4], b[4];
         load_matrices<true>(a, at, 2 * i); load_matrices<true>(b, at, 2 * i + 1);
 #pragma unroll
-        for (int th = 0; th < 2; th++) {             // tokens 2j, 2j + 1 (+ 8): a byte transpose sorts the pairs by token and by low / high byte
-          const u32 x0 = a[2 * th], x1 = a[2 * th + 1], x2 = b[2 * th], x3 = b[2 * th + 1];
-          const u32 p = prmt(x0, x1, 0x5140), q = prmt(x2, x3, 0x5140), p2 = prmt(x0, x1, 0x7362), q2 = prmt(x2, x3, 0x7362);
-          split_bytes4(prmt(p, q, 0x5410), prmt(p, q, 0x7632), lt.sm[8 * th + i], e[2 * th][h]);
-          split_bytes4(prmt(p2, q2, 0x5410), prmt(p2, q2, 0x7632), lt.sm[8 * th + 4 + i], e[2 * th + 1][h]);
-        }
+        for (int th = 0; th < 2; th++) split_token_pairs(a[2 * th], a[2 * th + 1], b[2 * th], b[2 * th + 1], lt.sm[8 * th + i], e[2 * th][h], lt.sm[8 * th + 4 + i], e[2 * th + 1][h]);      // tokens 2j, 2j + 1 (+ 8)
       }
 #pragma unroll
       for (int t = 0; t < 4; t++)

@@ -1,141 +1,130 @@
-// Host emulation of one warp encoding / rebuilding a GAAC tile with the SAME lane-level functions the CUDA kernels use
-// (gaac_b200/csrc/gaac_tile.h).  The warp-level glue (tag table, row prefix sums) is replaced by plain loops.
+// Host emulation of one warp encoding / rebuilding a GAAC tile with the SAME lane-level functions the CUDA kernels run
+// (gaac_b200/csrc/gaac_tile.h, gaac_swar.h).  What is warp-level there - matrix loads and stores, the scans that place the escape bytes, the
+// tables in shared memory - is plain loops here.
 // Built by the test-suite with g++ and driven through ctypes; checks the bit logic without a GPU.
 #include <cstring>
 #include "../../gaac_b200/csrc/gaac_tile.h"
 using namespace gaac;
 
-struct PtrEscH {
-  const uint8_t* p;
-  u32 byte(int pos) const { return p[pos]; }
-  u64 bytes5(int pos) const { u64 w = 0; for (int i = 0; i < 5; i++) w |= (u64)p[pos + i] << (8 * i); return w; }
-};
 static int v_tok(int j, int t) { return 2 * j + (t & 1) + 8 * (t >> 1); }
+static u32 pair(u32 lo, u32 hi) { return lo | hi << 16; }
+// position of a lane's escape bytes: those of the rows before and of the groups below `first` in the row
+static int esc_at(const uint32_t* fl, int row, int first) {
+  int at = 0;
+  for (int i = 0; i < row; i++) at += row_esc_bytes(fl[i]);
+  for (int g = 0; g < first; g++) at += (int)seg_esc((fl[row] >> (2 * g)) & 3u);
+  return at;
+}
 
 extern "C" int emu_encode_tile(int kind_v, const uint16_t* x, int nvalid, const uint8_t* b3row, const uint8_t* b4row,
                                uint8_t* sm_out, uint8_t* cd_out, uint32_t* fl_out, uint8_t* esc_out) {
-  uint8_t tag[16][16]; u64 escv[16][16];
-  memset(tag, 0, sizeof tag); memset(escv, 0, sizeof escv);
-  memset(sm_out, 0, 2048); memset(cd_out, 0, 768);
+  static const uint16_t zeros[128] = {};
+  auto at = [&](int tok) { return tok < nvalid ? x + 128 * tok : zeros; };
+  struct Group { u32 tag, esc1; u64 raw; } groups[16][16];
   for (int lane = 0; lane < 32; lane++) {
-    int j = lane & 3, r = lane >> 2;
+    const int j = lane & 3, r = lane >> 2;
+    u32 b3w[8], b4w[8], sm[16], cd[6], c24[8];
     if (!kind_v) {
-      u32 b3w[8], b4w[8]; k_base_words(b3row, j, b3w); k_base_words(b4row, j, b4w);
+      k_base_words(b3row, j, b3w); k_base_words(b4row, j, b4w);
       for (int o = 0; o < 2; o++) {
-        int row = 8 * o + r; if (row >= nvalid) continue;
-        u32 sm[8], cd[3], t8; u64 esc[4];
-        encode_k_lane(x + row * 128, j, b3w, b4w, sm, cd, t8, esc);
-        memcpy(sm_out + o * 1024 + 32 * lane, sm, 32); memcpy(cd_out + o * 384 + 12 * lane, cd, 12);
-        for (int g = 0; g < 4; g++) { tag[row][4 * j + g] = (t8 >> (2 * g)) & 3; escv[row][4 * j + g] = esc[g]; }
+        u32 e[8];
+        const uint16_t* row = at(8 * o + r);
+        for (int s = 0; s < 8; s++) { const uint16_t* p = row + 16 * s + 2 * j; split_bf16x4(pair(p[0], p[1]), pair(p[8], p[9]), sm[8 * o + s], e[s]); }
+        for (int g = 0; g < 4; g++) {
+          Group& G = groups[8 * o + r][4 * j + g];
+          G.tag = encode_group_codes(e[2 * g], e[2 * g + 1], b3w[2 * g], b3w[2 * g + 1], b4w[2 * g], b4w[2 * g + 1], c24[4 * o + g], G.esc1);
+          G.raw = raw_payload(e[2 * g], e[2 * g + 1]);
+          if (8 * o + r >= nvalid) G.tag = c24[4 * o + g] = 0;
+        }
       }
     } else {
-      u32 b3w[4], b4w[4]; v_base_words(b3row, r, b3w); v_base_words(b4row, r, b4w);
-      for (int t = 0; t < 4; t++) {
-        int row = v_tok(j, t); if (row >= nvalid) continue;
-        u32 sm[4], t4; u64 cd48, esc[2];
-        encode_v_lane(x + row * 128, r, b3w, b4w, sm, cd48, t4, esc);
-        memcpy(sm_out + 64 * lane + 16 * t, sm, 16); memcpy(cd_out + 24 * lane + 6 * t, &cd48, 6);
-        for (int g = 0; g < 2; g++) { tag[row][2 * r + g] = (t4 >> (2 * g)) & 3; escv[row][2 * r + g] = esc[g]; }
+      v_base_words(b3row, r, b3w); v_base_words(b4row, r, b4w);
+      u32 e[4][4];                                   // [token slot][word]
+      for (int i = 0; i < 4; i++)
+        for (int th = 0; th < 2; th++) {
+          const uint16_t *a = at(2 * j + 8 * th), *b = at(2 * j + 1 + 8 * th);
+          u32 w[4];
+          for (int q = 0; q < 4; q++) w[q] = pair(a[32 * i + 8 * q + r], b[32 * i + 8 * q + r]);
+          split_token_pairs(w[0], w[1], w[2], w[3], sm[8 * th + i], e[2 * th][i], sm[8 * th + 4 + i], e[2 * th + 1][i]);
+        }
+      for (int t = 0; t < 4; t++)
+        for (int g = 0; g < 2; g++) {
+          Group& G = groups[v_tok(j, t)][2 * r + g];
+          G.tag = encode_group_codes(e[t][2 * g], e[t][2 * g + 1], b3w[2 * g], b3w[2 * g + 1], b4w[2 * g], b4w[2 * g + 1], c24[2 * t + g], G.esc1);
+          G.raw = raw_payload(e[t][2 * g], e[t][2 * g + 1]);
+          if (v_tok(j, t) >= nvalid) G.tag = c24[2 * t + g] = 0;
+        }
+    }
+    join_codes(c24[0], c24[1], c24[2], c24[3], cd);
+    join_codes(c24[4], c24[5], c24[6], c24[7], cd + 3);
+    if (!kind_v)
+      for (int o = 0; o < 2; o++) { memcpy(sm_out + o * 1024 + 32 * lane, sm + 8 * o, 32); memcpy(cd_out + o * 384 + 12 * lane, cd + 3 * o, 12); }
+    else { memcpy(sm_out + 64 * lane, sm, 64); memcpy(cd_out + 24 * lane, cd, 24); }
+  }
+  int total = 0;
+  for (int row = 0; row < 16; row++) {
+    fl_out[row] = 0;
+    for (int g = 0; g < 16; g++) fl_out[row] |= groups[row][g].tag << (2 * g);
+    for (int g = 0; g < 16; g++) {
+      const Group& G = groups[row][g];
+      uint8_t* d = esc_out + esc_at(fl_out, row, g);
+      if (G.tag == 1u) d[0] = (uint8_t)G.esc1;
+      if (G.tag == 3u) for (int i = 0; i < 5; i++) d[i] = (uint8_t)(G.raw >> (8 * i));
+    }
+    total += row_esc_bytes(fl_out[row]);
+  }
+  return total;
+}
+
+// Rebuild.  PATCH false: the form that reads escape bytes where they are (decode_group_dev<false>); true: the form of staged tiles, where raw groups were
+// turned into table entries and the first payload byte of each into the entry's number (build_raw_patches, decode_group_dev<true>).  esc_in must be
+// readable to the end of the word behind its last byte.
+template <bool PATCH>
+static void decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in, const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
+  static u32x2 lutx[256]; static bool init = false;
+  if (!init) { for (int i = 0; i < 256; i++) fill_lutx(lutx, i); init = true; }
+  auto raw = [&](const uint8_t* p, u32 blo, u32 bhi) {
+    const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+    return raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3), blo, bhi);
+  };
+  const int SEGS = kind_v ? 4 : 2, PER = 8 / SEGS;
+  u32 base[32][2];                                   // {3-bit window, what the 4-bit one is above it} per half group
+  for (int t = 0; t < 32; t++) {
+    base[t][0] = kind_v ? half_group_word<true>(b3row, t) : half_group_word<false>(b3row, t);
+    base[t][1] = (kind_v ? half_group_word<true>(b4row, t) : half_group_word<false>(b4row, t)) - base[t][0];
+  }
+  for (int lane = 0; lane < 32; lane++) {
+    const int j = lane & 3, r = lane >> 2;
+    u32 sm[16], cd[6];
+    if (!kind_v) for (int o = 0; o < 2; o++) { memcpy(sm + 8 * o, sm_in + o * 1024 + 32 * lane, 32); memcpy(cd + 3 * o, cd_in + o * 384 + 12 * lane, 12); }
+    else { memcpy(sm, sm_in + 64 * lane, 64); memcpy(cd, cd_in + 24 * lane, 24); }
+    const u32 z[8] = {group_codes<0>(cd), group_codes<3>(cd), group_codes<6>(cd), group_codes<9>(cd), group_codes<12>(cd), group_codes<15>(cd), group_codes<18>(cd), group_codes<21>(cd)};
+    for (int s = 0; s < SEGS; s++) {
+      const int row = kind_v ? v_tok(j, s) : 8 * s + r, first = kind_v ? 2 * r : 4 * j;
+      for (int g = 0; g < PER; g++) {
+        const int idx = PER * s + g, hg = kind_v ? 4 * r + 2 * g : 8 * j + 2 * g;
+        const u32 tag = (fl_in[row] >> (2 * (first + g))) & 3u, m1 = tag & 1u;
+        const u32x4 bw{base[hg][0], base[hg + 1][0], base[hg][1], base[hg + 1][1]};
+        const uint8_t* p = esc_in + esc_at(fl_in, row, first + g);
+        u32x2 x = lutx[tag == 1u ? *p : 0];
+        if (tag & 2u) x = PATCH ? raw(p, bw.x + bw.z, bw.y + bw.w) : raw(p, mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
+        u32 f[4];
+        rebuild_group(sm[2 * idx], sm[2 * idx + 1], z[idx], m1, bw, x, f);
+        for (int q = 0; q < 4; q++) {
+          // K: words 2h, 2h + 1 = channels 16s + 2j (+ 1) and + 8 (+ 1) of s = 2g + h; V: word q = channels 8(8g + 2q) + r and 8(8g + 2q + 1) + r
+          const int c = kind_v ? 8 * (8 * g + 2 * q) + r : 16 * (2 * g + (q >> 1)) + 2 * j + 8 * (q & 1);
+          out[128 * row + c] = (uint16_t)f[q]; out[128 * row + c + (kind_v ? 8 : 1)] = (uint16_t)(f[q] >> 16);
+        }
       }
     }
   }
-  int pos = 0;
-  for (int row = 0; row < 16; row++) {
-    u32 fl = 0;
-    for (int g = 0; g < 16; g++) {
-      fl |= (u32)tag[row][g] << (2 * g);
-      int n = tag_esc_bytes(tag[row][g]);
-      for (int i = 0; i < n; i++) esc_out[pos++] = (uint8_t)(escv[row][g] >> (8 * i));
-    }
-    fl_out[row] = fl;
-  }
-  return pos;
 }
 
 extern "C" void emu_decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in,
                                 const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
-  int rowoff[16], acc = 0;
-  for (int row = 0; row < 16; row++) { rowoff[row] = acc; acc += row_esc_bytes(fl_in[row]); }
-  PtrEscH esc{esc_in};
-  for (int lane = 0; lane < 32; lane++) {
-    int j = lane & 3, r = lane >> 2;
-    if (!kind_v) {
-      u32 b3w[8], b4w[8]; k_base_words(b3row, j, b3w); k_base_words(b4row, j, b4w);
-      for (int o = 0; o < 2; o++) {
-        int row = 8 * o + r; u32 sm[8], cd[3];
-        memcpy(sm, sm_in + o * 1024 + 32 * lane, 32); memcpy(cd, cd_in + o * 384 + 12 * lane, 12);
-        u32 fl = fl_in[row]; int pos = rowoff[row] + esc_prefix(fl, 8 * j);
-        for (int g = 0; g < 4; g++) {
-          u32 o4[4];
-          decode_group(sm[2 * g], sm[2 * g + 1], k_group_codes(cd, g), (fl >> (8 * j + 2 * g)) & 3u, pos, esc, b3w[2 * g], b3w[2 * g + 1], b4w[2 * g] - b3w[2 * g], b4w[2 * g + 1] - b3w[2 * g + 1], o4);
-          for (int h = 0; h < 2; h++) {
-            int s = 2 * g + h; uint16_t* p = out + row * 128 + 16 * s + 2 * j;
-            p[0] = (uint16_t)o4[2 * h]; p[1] = (uint16_t)(o4[2 * h] >> 16); p[8] = (uint16_t)o4[2 * h + 1]; p[9] = (uint16_t)(o4[2 * h + 1] >> 16);
-          }
-        }
-      }
-    } else {
-      u32 b3w[4], b4w[4]; v_base_words(b3row, r, b3w); v_base_words(b4row, r, b4w);
-      u32 cd[6]; memcpy(cd, cd_in + 24 * lane, 24);
-      for (int t = 0; t < 4; t++) {
-        int row = v_tok(j, t); u32 sm[4]; memcpy(sm, sm_in + 64 * lane + 16 * t, 16);
-        u32 fl = fl_in[row]; int pos = rowoff[row] + esc_prefix(fl, 4 * r);
-        for (int g = 0; g < 2; g++) {
-          u32 o4[4];
-          decode_group(sm[2 * g], sm[2 * g + 1], v_group_codes(cd, t, g), (fl >> (4 * r + 2 * g)) & 3u, pos, esc, b3w[2 * g], b3w[2 * g + 1], b4w[2 * g] - b3w[2 * g], b4w[2 * g + 1] - b3w[2 * g + 1], o4);
-          for (int h = 0; h < 2; h++) {
-            int w = 2 * g + h; uint16_t* p = out + row * 128 + r;
-            p[8 * (4 * w)] = (uint16_t)o4[2 * h]; p[8 * (4 * w + 1)] = (uint16_t)(o4[2 * h] >> 16);
-            p[8 * (4 * w + 2)] = (uint16_t)o4[2 * h + 1]; p[8 * (4 * w + 3)] = (uint16_t)(o4[2 * h + 1] >> 16);
-          }
-        }
-      }
-    }
-  }
+  decode_tile<false>(kind_v, sm_in, cd_in, fl_in, esc_in, b3row, b4row, out);
 }
-
-// Same as emu_decode_tile through the table-driven group decoder of the fused attention kernel.
-// esc_in must be 4-byte aligned and readable 8 bytes past its last escape byte.
 extern "C" void emu_decode_tile_lut(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in,
                                     const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
-  static u32x2 lutx[256]; static bool init = false;
-  if (!init) { for (int i = 0; i < 256; i++) fill_lutx(lutx, i); init = true; }
-  static const uint32_t zero_word = 0; const uint8_t* zero = reinterpret_cast<const uint8_t*>(&zero_word);
-  int rowoff[16], acc = 0;
-  for (int row = 0; row < 16; row++) { rowoff[row] = acc; acc += row_esc_bytes(fl_in[row]); }
-  for (int lane = 0; lane < 32; lane++) {
-    int j = lane & 3, r = lane >> 2;
-    if (!kind_v) {
-      u32 b3w[8], b4w[8]; k_base_words(b3row, j, b3w); k_base_words(b4row, j, b4w);
-      for (int o = 0; o < 2; o++) {
-        int row = 8 * o + r; u32 sm[8], cd[3];
-        memcpy(sm, sm_in + o * 1024 + 32 * lane, 32); memcpy(cd, cd_in + o * 384 + 12 * lane, 12);
-        u32 fl = fl_in[row]; int pos = rowoff[row] + esc_prefix(fl, 8 * j);
-        for (int g = 0; g < 4; g++) {
-          u32 o4[4]; u32x4 bw{b3w[2 * g], b3w[2 * g + 1], b4w[2 * g] - b3w[2 * g], b4w[2 * g + 1] - b3w[2 * g + 1]};
-          decode_group_lut(sm[2 * g], sm[2 * g + 1], k_group_codes(cd, g), (fl >> (8 * j + 2 * g)) & 3u, pos, esc_in, zero, lutx, bw, o4);
-          for (int h = 0; h < 2; h++) {
-            int s = 2 * g + h; uint16_t* p = out + row * 128 + 16 * s + 2 * j;
-            p[0] = (uint16_t)o4[2 * h]; p[1] = (uint16_t)(o4[2 * h] >> 16); p[8] = (uint16_t)o4[2 * h + 1]; p[9] = (uint16_t)(o4[2 * h + 1] >> 16);
-          }
-        }
-      }
-    } else {
-      u32 b3w[4], b4w[4]; v_base_words(b3row, r, b3w); v_base_words(b4row, r, b4w);
-      u32 cd[6]; memcpy(cd, cd_in + 24 * lane, 24);
-      for (int t = 0; t < 4; t++) {
-        int row = v_tok(j, t); u32 sm[4]; memcpy(sm, sm_in + 64 * lane + 16 * t, 16);
-        u32 fl = fl_in[row]; int pos = rowoff[row] + esc_prefix(fl, 4 * r);
-        for (int g = 0; g < 2; g++) {
-          u32 o4[4]; u32x4 bw{b3w[2 * g], b3w[2 * g + 1], b4w[2 * g] - b3w[2 * g], b4w[2 * g + 1] - b3w[2 * g + 1]};
-          decode_group_lut(sm[2 * g], sm[2 * g + 1], v_group_codes(cd, t, g), (fl >> (4 * r + 2 * g)) & 3u, pos, esc_in, zero, lutx, bw, o4);
-          for (int h = 0; h < 2; h++) {
-            int w = 2 * g + h; uint16_t* p = out + row * 128 + r;
-            p[8 * (4 * w)] = (uint16_t)o4[2 * h]; p[8 * (4 * w + 1)] = (uint16_t)(o4[2 * h] >> 16);
-            p[8 * (4 * w + 2)] = (uint16_t)o4[2 * h + 1]; p[8 * (4 * w + 3)] = (uint16_t)(o4[2 * h + 1] >> 16);
-          }
-        }
-      }
-    }
-  }
+  decode_tile<true>(kind_v, sm_in, cd_in, fl_in, esc_in, b3row, b4row, out);
 }
