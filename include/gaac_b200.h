@@ -62,7 +62,7 @@ int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, in
                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, void* stream);
 
 /* gaac_encode_begin, then a wait for the stream: on return *total_pinned (page-locked host memory) holds head_start[H], which the
- * kernels wrote there themselves.  For a caller that wants the escape stream at its exact size (TileEncoder.encode). */
+ * kernels wrote there themselves.  The one call that synchronises: not for a stream that is being captured.  For a caller that wants the escape stream at its exact size (TileEncoder.encode). */
 int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                       const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                       uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
