@@ -51,7 +51,8 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     Equal lengths (S is every row's length): the split count minimises a cost model fitted to measurements,
         waves x ((tiles per warp + 0.5) x tile time + per-CTA fixed cost),   waves = ceil(rows x splits / SMs),
     over the counts that leave every warp at least min_tiles_per_warp 16-token tiles (fewer on short contexts, see the code).  Tile time: 4.5 us, 5.2 us
-    beyond 512 tiles of a range; fixed cost (prologue, warp merge, split merge): 10 us.  Few rows end up with one wave that
+    beyond 512 tiles of a range; fixed cost (prologue, warp merge, split merge): 10 us.  These were fitted to an earlier kernel (the present one takes about
+    6.5 us + 0.22 us per tile and CTA, and nothing changes at 512); the counts they choose were not refitted.  Few rows end up with one wave that
     fills the SMs, many rows with ranges of at most 512 tiles in several waves.
     Ragged lengths (ragged=True, S is the longest row; total_tokens is accepted and unused): every row gets the same split count;
     see the comment in the code."""
