@@ -11,11 +11,14 @@
 // finish merges the splits and writes the output, so one launch does the whole layer.
 //
 // What the measurements on B200 say (they shaped the code below):
-//  * the kernel is bound by instruction issue and by the ALU pipe, not by HBM.  With a private two-stage ring per warp every warp issued
-//    eight copies per tile pair, about 200 of 1354 instructions; one copy of four tiles, issued by the warp that is last to leave a
-//    stage, takes that to about 25 per tile pair.
+//  * the kernel is bound by instruction issue, not by HBM.  With a private two-stage ring per warp every warp issued eight copies per tile pair, about
+//    200 of 1354 instructions; one copy of four tiles, issued by the warp that is last to leave a stage, takes that to about 25 per tile pair.
+//  * a bulk copy takes the warp that issues it about 100 cycles, and a loop over the lanes before it where its operands are not known to be uniform: the
+//    eight copies of a stage took their warp 2300 cycles, issued by an elected lane of the converged warp 1150 (57.5 -> 56.7 us at 65536 tokens).
+//  * warps of their own for parts of the work lose: one that issues all copies is too slow by itself (56.3 us, but 620 instead of 500 on paged tiles), and with
+//    four, six or eight of the sixteen warps expanding escape bytes (plan_tile, one tile or a whole stage at a time) the others wait for them: 65 to 88 us.
 //  * bulk copies want few large copies (one 128-byte copy per row, which would allow a conflict-free skewed layout, was 15 % slower), so
-//    shared memory holds the storage order and the 16-byte fragment reads accept a 2-way (K) / 4-way (V) bank conflict.
+//    shared memory holds the storage order and the 16-byte fragment reads accept a 2-way bank conflict.
 //
 // Fragment conventions follow the reference kernel (gaac/kernel.py:62-66,160-194), whose storage order they mirror.
 #include <algorithm>
@@ -25,7 +28,7 @@
 
 namespace gaac {
 
-// Warps per CTA (20 warps at 96 registers measured 3 % slower: the kernel is short of issue slots, not of warps, and what they work on takes ring space).
+// Warps per CTA (18 or 20 warps at 96 registers: 64.5 us instead of 57.5 at 65536 tokens).
 constexpr int ATT_WARPS = 16, ATT_THREADS = ATT_WARPS * 32;
 // ---- ring of stages.  A stage holds TPS consecutive tiles.
 //   slot layout:  per side  sign/mantissa of the tiles (TPS x 2048) | codes (TPS x 768) | tag words (TPS x 64) | the tiles' escape bytes, which are
@@ -37,17 +40,16 @@ constexpr int SIDE_ESC = TPS * (ESC_WIN + 16);
 constexpr int SB_CD = TPS * TILE_SM, SB_FL = SB_CD + TPS * TILE_CD, SB_ESC = SB_FL + TPS * 4 * T, SIDE_BYTES = SB_ESC + SIDE_ESC;
 constexpr int STAGE_BYTES = 2 * SIDE_BYTES;
 static_assert(SIDE_BYTES == TPS * PSLOT, "both layouts use stages of the same size");
-constexpr int META_TILES = 1024;                   // tiles of a CTA's range whose metadata is staged (longer ranges read the rest from global)
-// CTA tables: escape-byte table, K / V base words, zero bytes, the stages' mbarriers, use counts
-// and escape windows {K start, K bytes, V start, V bytes}, the per-tile metadata of the range, the warps' scratch
-constexpr int TB_LUTX = 0, TB_BASES = LUTX_BYTES, TB_ZERO = TB_BASES + BASES_BYTES, TB_FULL = TB_ZERO + 16, TB_DONE = TB_FULL + 8 * NSTG, TB_WIN = TB_DONE + 4 * NSTG, TB_META = TB_WIN + 16 * NSTG,
-              TB_RING = TB_META + 2 * META_TILES * 4, TB_SCRATCH = TB_RING + NSTG * STAGE_BYTES;
-constexpr int ATT_SMEM = TB_SCRATCH + ATT_WARPS * WARP_SCRATCH;
-static_assert(TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_WIN % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
+// CTA tables: addend and segment table, K / V base words; per stage the mbarrier that counts arriving bytes and how many tiles of it the warps have left so far; per
+// tile of a stage {address of its escape bytes of K, how many are staged, the same of V}, its metadata, and the word (stage + 1) << 4 | bits 2, 3: the K / V tile is
+// raw, by which a warp knows the use of the slot: a parity can be two phases off for one that runs ahead of a slow one.  Then the warps' segment areas.
+constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + BASES_BYTES, TB_LEFT = TB_FULL + 8 * NSTG, TB_ESC = TB_LEFT + 4 * NSTG, TB_META = TB_ESC + 16 * TPS * NSTG,
+              TB_USE = TB_META + 8 * TPS * NSTG, TB_AREA = TB_USE + 4 * TPS * NSTG, TB_RING = TB_AREA + ATT_WARPS * AREA_BYTES;
+constexpr int ATT_SMEM = TB_RING + NSTG * STAGE_BYTES + 16;          // (an escape segment is read as whole words)
+static_assert(TB_BASES % 16 == 0 && TB_ESC % 16 == 0 && TB_AREA % 16 == 0 && TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
               "bulk copies need 16-byte aligned shared-memory destinations and sizes");
 static_assert(ATT_SMEM + 64 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
 static_assert(ATT_THREADS / 128 * 2 >= 8, "the fused exchange keeps at most two merged heads per thread");
-static_assert((TPS & (TPS - 1)) == 0 && (NSTG & (NSTG - 1)) == 0, "");
 constexpr int ACC_LD = D + 8;                        // row stride of the staged accumulators: 8j + r banks, conflict-free stores
 
 struct AttnParams {
@@ -248,7 +250,7 @@ template <int NSET> __device__ __forceinline__ void stage_warp(const WarpAcc<NSE
     if (h < G) {
       float* a0 = sh_m + ATT_WARPS * 16 + (warp * 8 + h) * ACC_LD + r;
 #pragma unroll
-      for (int i = 0; i < 16; i++) a0[8 * i] = A.acc[s][i >> 2][i & 3];
+      for (int i = 0; i < 16; i++) a0[8 * acc_channel(i >> 2, i & 3)] = A.acc[s][i >> 2][i & 3];
     }
   }
 }
@@ -380,17 +382,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
   const u32 smem_s = (u32)__cvta_generic_to_shared(smem);
-  int* const done = reinterpret_cast<int*>(smem + TB_DONE);
   // ---- programmatic dependent launch: the grid is launched with stream serialisation relaxed, so its CTAs can be made
   // resident while the previous kernel of the stream is still finishing (its split merge runs on a few SMs only).  What does not
   // depend on memory is set up before the wait; nothing is read before that kernel has completed; the next kernel of the stream may be
   // staged behind this one right away (it cannot become resident before this grid's CTAs leave their SMs).  Both instructions are no-ops
   // in a plain launch.
-  if (tid < 256) fill_lutx(reinterpret_cast<u32x2*>(smem + TB_LUTX), tid);
-  if (tid >= 256 && tid < 260) reinterpret_cast<u32*>(smem + TB_ZERO)[tid - 256] = 0u;
-  if (lane == 0 && warp < NSTG) {
+  if (tid < 256) fill_attn_tables(smem, tid);
+  if (tid >= 256 && tid < 256 + TPS * NSTG) reinterpret_cast<u32*>(smem + TB_USE)[tid - 256] = 0u;
+  if (lane == 0 && warp < NSTG) {                    // warp w fills stage w first
     mbar_init(smem_s + TB_FULL + 8 * warp, 1);
-    done[warp] = 0;
+    reinterpret_cast<int*>(smem + TB_LEFT)[warp] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -447,63 +448,76 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   const long smh = (long)ch * p.S_pad * D, cdh = (long)ch * p.S_pad * CB, rowb = (long)ch * p.S_pad, tileb = (long)ch * (p.S_pad >> 4);
   ohk = __shfl_sync(FULLM, ohk, 0); ohv = __shfl_sync(FULLM, ohv, 0);
 
-  const int* metak = reinterpret_cast<const int*>(smem + TB_META);
-  const int* metav = metak + META_TILES;
-  auto global_meta = [&](int i) -> TileMeta {         // i counts from the first tile of the CTA's range
+  auto meta_of = [&](int i) -> TileMeta {             // i counts from the first tile of the CTA's range
     const int tile = tlo + i;
     if (PAGED) { const int pc = p.bt[(long)b * p.bt_stride + tile] * (2 * p.n_kv) + 2 * kvh; return TileMeta{p.mt[pc], p.mt[pc + 1]}; }
     return TileMeta{p.K.tile_off[tileb + tile], p.V.tile_off[tileb + tile]};
   };
-  auto meta_of = [&](int i) -> TileMeta {             // valid after the CTA has staged its metadata
-    if (i < META_TILES) return TileMeta{metak[i], metav[i]};
-    return global_meta(i);
-  };
-  // ---- filling a stage, in two parts: what needs no metadata (slot layout only), and what does.  Executed by one lane.
-  auto issue_payload = [&](int st) {
-    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES;
-    const int first = st * TPS;
-    const u32 cnt = (u32)min(TPS, n - first);
-    const long tile = tlo + first;
-    mbar_add_tx(mb, 2 * cnt * (TILE_SM + TILE_CD + 4 * T));
-    bulk_g2s(dst, p.K.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb); bulk_g2s(dst + SIDE_BYTES, p.V.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb);
-    bulk_g2s(dst + SB_CD, p.K.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb); bulk_g2s(dst + SIDE_BYTES + SB_CD, p.V.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb);
-    bulk_g2s(dst + SB_FL, reinterpret_cast<const uint8_t*>(p.K.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
-    bulk_g2s(dst + SIDE_BYTES + SB_FL, reinterpret_cast<const uint8_t*>(p.V.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
+  // ---- filling a stage.  What a copy is given comes from uniform values or through a shuffle, so that the compiler knows it to be the same in every lane: the copy
+  // instruction takes uniform registers, and anything else costs it a loop over the lanes.
+  constexpr int FAR = 1 << 28;                        // "until the end of the allocation", as an escape offset
+  auto stage_meta = [&](int st) -> TileMeta {         // lane t < TPS: of tile t;  slot layout, lane TPS: of the tile behind, where the stage's escape bytes end
+    const int i = st * TPS + lane;
+    if (PAGED) return lane < TPS && i < n ? meta_of(i) : TileMeta{-1, -1};
+    return lane <= TPS && (i < n || tlo + i < ntiles) ? meta_of(i) : TileMeta{FAR, FAR};
   };
   // Escape window of a side for tiles whose escape bytes are [m0, m1) of the head's: from the 16-byte boundary at or below the first byte, a
-  // multiple of 16 bytes, at most SIDE_ESC, inside the allocation (no bytes when the boundary lies before it).
-  auto esc_window = [&](const gaac_side& sd, int oh, int m0, int m1, int& start, u32& bytes) {
-    const int w16 = (int)((reinterpret_cast<uintptr_t>(sd.ovf) + (unsigned)oh + (unsigned)m0) & 15);
-    const long to_end = (long)sd.ovf_bytes - oh - m0 + w16;
+  // multiple of 16 bytes, at most SIDE_ESC, inside the allocation (no bytes when the boundary lies before it).  phase: of the head's first byte;  to_end: bytes from there
+  // to the end of the allocation.
+  const int phk = PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.K.ovf) + (unsigned)ohk) & 15), phv = PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.V.ovf) + (unsigned)ohv) & 15);
+  const int k_end = PAGED ? 0 : (int)max(-1L, min((long)p.K.ovf_bytes - ohk, 0x7FFFFF00L)), v_end = PAGED ? 0 : (int)max(-1L, min((long)p.V.ovf_bytes - ohv, 0x7FFFFF00L));
+  auto esc_window = [&](int to_end, int phase, int oh, int m0, int m1, int& start, u32& bytes) {
+    const int w16 = (phase + m0) & 15, left = (int)((u32)to_end - (u32)m0 + (u32)w16);
     start = m0 - w16;
-    bytes = (long)oh + m0 < w16 || to_end <= 0 ? 0u : (u32)max(0L, min((long)min(SIDE_ESC, (m1 - m0 + w16 + 15) & ~15), to_end & ~15L));
+    bytes = oh < w16 - m0 || to_end < m0 - w16 ? 0u : (u32)max(0, min(min(SIDE_ESC, (m1 - m0 + w16 + 15) & ~15), left & ~15));
   };
-  auto issue_rest = [&](int st, const TileMeta& m0, const TileMeta& m1) {        // m0: metadata of the stage's first tile, m1: of the first one behind it (slot layout)
-    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES;
-    int4 w; u32 nk, nv;
-    esc_window(p.K, ohk, m0.mk, m1.mk, w.x, nk); esc_window(p.V, ohv, m0.mv, m1.mv, w.z, nv);
-    w.y = (int)nk; w.w = (int)nv;
-    *reinterpret_cast<int4*>(smem + TB_WIN + 16 * (st % NSTG)) = w;
-    mbar_expect_tx(mb, nk + nv);
-    if (nk > 0) bulk_g2s(dst + SB_ESC, p.K.ovf + ((long)ohk + w.x), nk, mb);
-    if (nv > 0) bulk_g2s(dst + SIDE_BYTES + SB_ESC, p.V.ovf + ((long)ohv + w.z), nv, mb);
-  };
-  auto behind = [&](int st, const TileMeta& none) { const int i = (st + 1) * TPS; return i < n || tlo + i < ntiles ? global_meta(i) : none; };
   const u32 slot_bytes = PAGED ? (u32)min(p.TS, PSLOT) : 0u;                   // a paged slot is one contiguous piece, escapes included
-  auto issue_paged = [&](int st, const TileMeta (&m)[TPS]) {
-    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES;
-    const int cnt = min(TPS, n - st * TPS);
-    u32 pieces = 0;
+  // Both are executed by a whole warp.  The part that needs no metadata (slot layout) ..
+  auto fill_payload = [&](int st) {
+    const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES, cnt = (u32)min(TPS, n - st * TPS);
+    const long tile = tlo + st * TPS;
+    warp_add_tx(mb, 2 * cnt * (TILE_SM + TILE_CD + 4 * T));
+    warp_g2s(dst + SB_FL, reinterpret_cast<const uint8_t*>(p.K.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
+    warp_g2s(dst + SIDE_BYTES + SB_FL, reinterpret_cast<const uint8_t*>(p.V.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
+    warp_g2s(dst, p.K.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb); warp_g2s(dst + SB_CD, p.K.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb);
+    warp_g2s(dst + SIDE_BYTES, p.V.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb); warp_g2s(dst + SIDE_BYTES + SB_CD, p.V.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb);
+  };
+  // .. and the rest, or all of a paged stage.  own: stage_meta
+  auto fill_rest = [&](int st, const TileMeta& own) {
+    const int slot = st % NSTG;
+    const u32 mb = smem_s + TB_FULL + 8 * slot, dst = smem_s + TB_RING + slot * STAGE_BYTES;
+    int4 info;
+    u32 pieces = 0u;
+    int k0 = 0, v0 = 0; u32 nk = 0u, nv = 0u;
+    if (PAGED) {
+      const u32 e = dst + 2 * lane * PSLOT + SLOT_OVF_OFF;
+      const int avail = min(p.ovf_slot, (int)slot_bytes - SLOT_OVF_OFF);
+      info = make_int4((int)e, avail, (int)(e + PSLOT), avail);
+      pieces = (u32)popc(__ballot_sync(FULLM, own.mk >= 0)) + (u32)popc(__ballot_sync(FULLM, own.mv >= 0));
+    } else {
+      const int m0k = __shfl_sync(FULLM, own.mk, 0), m0v = __shfl_sync(FULLM, own.mv, 0), m1k = __shfl_sync(FULLM, own.mk, TPS), m1v = __shfl_sync(FULLM, own.mv, TPS);
+      esc_window(k_end, phk, ohk, m0k, m1k, k0, nk); esc_window(v_end, phv, ohv, m0v, m1v, v0, nv);
+      info = make_int4((int)dst + SB_ESC + own.mk - k0, (int)nk - (own.mk - k0), (int)dst + SIDE_BYTES + SB_ESC + own.mv - v0, (int)nv - (own.mv - v0));
+    }
+    if (lane < min(TPS, n - st * TPS)) {
+      reinterpret_cast<int4*>(smem + TB_ESC)[slot * TPS + lane] = info;
+      reinterpret_cast<int2*>(smem + TB_META)[slot * TPS + lane] = make_int2(own.mk, own.mv);
+      asm volatile("st.relaxed.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_s + TB_USE + 4 * (slot * TPS + lane)), "r"((u32)(st + 1) << 4 | (PAGED && own.mk < 0 ? 4u : 0u) | (PAGED && own.mv < 0 ? 8u : 0u)) : "memory");
+    }
+    __syncwarp();
+    warp_expect_tx(mb, PAGED ? pieces * slot_bytes : nk + nv);
+    if (PAGED) {
 #pragma unroll
-    for (int t = 0; t < TPS; t++) pieces += t < cnt ? (m[t].mk >= 0 ? 1u : 0u) + (m[t].mv >= 0 ? 1u : 0u) : 0u;
-    mbar_expect_tx(mb, pieces * slot_bytes);
-#pragma unroll
-    for (int t = 0; t < TPS; t++) {
-      if (t < cnt && m[t].mk >= 0) bulk_g2s(dst + 2 * t * PSLOT, p.buf + (long)m[t].mk * p.TS, slot_bytes, mb);
-      if (t < cnt && m[t].mv >= 0) bulk_g2s(dst + (2 * t + 1) * PSLOT, p.buf + (long)m[t].mv * p.TS, slot_bytes, mb);
+      for (int t = 0; t < TPS; t++) {
+        const int k = __shfl_sync(FULLM, own.mk, t), v = __shfl_sync(FULLM, own.mv, t);
+        if (k >= 0) warp_g2s(dst + 2 * t * PSLOT, p.buf + (long)k * p.TS, slot_bytes, mb);
+        if (v >= 0) warp_g2s(dst + (2 * t + 1) * PSLOT, p.buf + (long)v * p.TS, slot_bytes, mb);
+      }
+    } else {
+      if (nk > 0) warp_g2s(dst + SB_ESC, p.K.ovf + ((long)ohk + k0), nk, mb);
+      if (nv > 0) warp_g2s(dst + SIDE_BYTES + SB_ESC, p.V.ovf + ((long)ohv + v0), nv, mb);
     }
   };
-  constexpr int FAR = 1 << 28;                        // "until the end of the allocation", as an escape offset
 
   // ---- prologue.  Everything that reads global memory is put in flight first and consumed afterwards: the first stages' payload (needs
   // no metadata in the slot layout), their metadata, the metadata of the CTA's range, the query rows; then the tables are built while
@@ -511,108 +525,75 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // HBM is idle when the grid starts and every CTA asks at once: the stages that the first tiles are in go first, the others follow once
   // the small loads are back (filling all eight at once held those loads, and with them the first tile, back for 5 us).
   constexpr int FIRST = (ATT_WARPS + TPS - 1) / TPS;
-  const bool filler = lane == 0 && warp < min(NSTG, nstages);                  // warp w fills stage w
-  TileMeta f0{0, 0}, f1{0, 0};
-  auto fill_paged = [&](int st) {
-    TileMeta m[TPS];
-#pragma unroll
-    for (int t = 0; t < TPS; t++) m[t] = st * TPS + t < n ? global_meta(st * TPS + t) : TileMeta{-1, -1};
-    issue_paged(st, m);
-  };
+  const bool filler = warp < min(NSTG, nstages);                               // warp w fills stage w
+  TileMeta ahead{};
   if (filler) {
-    if (!PAGED) { f0 = global_meta(warp * TPS); f1 = behind(warp, TileMeta{FAR, FAR}); }
-    if (warp < FIRST) { if (PAGED) fill_paged(warp); else issue_payload(warp); }
+    if (!PAGED && warp < FIRST) fill_payload(warp);
+    ahead = stage_meta(warp);
   }
-  const int nstaged = min(n, META_TILES);
-  TileMeta m_first{0, 0};
-  if (tid < nstaged) m_first = global_meta(tid);
   QFrag Q;
   load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * D, D, G, lane);
   {
     const int brow = PAGED ? kvh : ch % p.n_base_rows;
-    if (warp == ATT_WARPS - 2) fill_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
-    if (warp == ATT_WARPS - 1) fill_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
+    if (warp == ATT_WARPS - 2 && lane < 16) fill_pair_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
+    if (warp == ATT_WARPS - 1 && lane < 16) fill_pair_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
     if (SHARE && tid == 0) { s_split = split0; s_ns = ns0; }
     if (tid == 0) s_next = ATT_WARPS;                        // tiles 0 .. W-1 of the range go to warps 0 .. W-1, the rest is handed out on demand
-    int* mk_s = reinterpret_cast<int*>(smem + TB_META);
-    int* mv_s = mk_s + META_TILES;
-    if (tid < nstaged) { mk_s[tid] = m_first.mk; mv_s[tid] = m_first.mv; }
-    for (int i = tid + ATT_THREADS; i < nstaged; i += ATT_THREADS) { const TileMeta m = global_meta(i); mk_s[i] = m.mk; mv_s[i] = m.mv; }
   }
-  if (!PAGED && filler && warp < FIRST) issue_rest(warp, f0, f1);
+  if (filler && warp < FIRST) fill_rest(warp, ahead);
   WarpAcc<NSET> A;
   A.clear();
   __syncthreads();
-  if (filler && warp >= FIRST) { if (PAGED) fill_paged(warp); else { issue_payload(warp); issue_rest(warp, f0, f1); } }
+  if (filler && warp >= FIRST) { if (!PAGED) fill_payload(warp); fill_rest(warp, ahead); }
 
   uint16_t* const dump_k = DUMP ? p.dump_k + (long)bh * p.dump_S * D : nullptr;
   uint16_t* const dump_v = DUMP ? p.dump_v + (long)bh * p.dump_S * D : nullptr;
-  const WarpView W{smem_s + TB_LUTX, smem_s + TB_BASES, smem_s + TB_ZERO, smem_s + TB_SCRATCH + warp * WARP_SCRATCH};
-  const int paged_avail = PAGED ? min(p.ovf_slot, (int)slot_bytes - SLOT_OVF_OFF) : 0;
+  const AttnView W = attn_view(smem_s, smem_s + TB_BASES);
   // ---- main loop.  The warp's first tile is tile `warp` of the range; every further one is taken from the CTA's counter at the top of the
   // iteration, one tile ahead of its use, so fast and slow warps finish within about one tile of each other.  The warp that is the
   // last to leave a stage fills it again with the tiles NSTG stages on.
+  const u32 area = smem_s + TB_AREA + warp * AREA_BYTES;
   int it = warp;
   while (it < n) {
     int nx = 0;
     if (lane == 0) nx = atomicAdd(&s_next, 1);
-    const int st = it / TPS, ti = it % TPS, slot = st % NSTG;
-    const TileMeta cur = meta_of(it);
-    // A parity says one thing about two phases: the stage's wait is only right once its slot's previous use is over, that is, once all its tiles
-    // were counted out (a warp can be handed a tile whose slot still waits for its previous copies).
-    if (!__all_sync(FULLM, wait_count(smem_s + TB_DONE + 4 * slot, TPS * (st / NSTG)) && mbar_wait(smem_s + TB_FULL + 8 * slot, (u32)(st / NSTG) & 1u))) {     // the whole warp gives up together
+    const int st = it / TPS, ti = it % TPS, slot = st % NSTG, tile = tlo + it, nth = it % (TPS * NSTG);
+    u32 flags;
+    if (!__all_sync(FULLM, mbar_wait_use(smem_s + TB_FULL + 8 * slot, (u32)(st / NSTG) & 1u, smem_s + TB_USE + 4 * nth, (u32)st + 1u, flags))) {     // the whole warp gives up together
       if (lane == 0) atomicExch(p.err, 1);
       break;
     }
-    const int sb = TB_RING + slot * STAGE_BYTES, tile = tlo + it;
     const int nvalid = min(T, S - tile * T);
-    const bool rawk = PAGED && cur.mk < 0, rawv = PAGED && cur.mv < 0;
-    SideView ks, vs;
-    if (PAGED) {
-      const uint8_t* t0 = smem + sb + 2 * ti * PSLOT;
-      const u32 esc = smem_s + sb + 2 * ti * PSLOT + SLOT_OVF_OFF;
-      ks = SideView{t0, t0 + SLOT_CD_OFF, t0 + SLOT_FL_OFF, esc, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF, paged_avail};
-      vs = SideView{t0 + PSLOT, t0 + PSLOT + SLOT_CD_OFF, t0 + PSLOT + SLOT_FL_OFF, esc + PSLOT, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, paged_avail};
-    } else {
-      const int4 w = *reinterpret_cast<const int4*>(smem + TB_WIN + 16 * slot);
-      const uint8_t* t0 = smem + sb + ti * TILE_SM;
-      const uint8_t* c0 = smem + sb + SB_CD + ti * TILE_CD;
-      const uint8_t* f0 = smem + sb + SB_FL + ti * 4 * T;
-      const int ok = cur.mk - w.x, ov = cur.mv - w.z;
-      ks = SideView{t0, c0, f0, smem_s + sb + SB_ESC + ok, p.K.ovf + ((long)ohk + cur.mk), w.y - ok};
-      vs = SideView{t0 + SIDE_BYTES, c0 + SIDE_BYTES, f0 + SIDE_BYTES, smem_s + sb + SIDE_BYTES + SB_ESC + ov, p.V.ovf + ((long)ohv + cur.mv), w.w - ov};
-    }
-    const TilePlan plan = plan_tile(ks, vs, rawk, rawv, W, lane);
+    const bool rawk = PAGED && (flags & 4u), rawv = PAGED && (flags & 8u);
+    const int2 own = reinterpret_cast<const int2*>(smem + TB_ESC)[2 * nth + (lane >> 4)];           // the lane's side: where its escape bytes are
+    const u32 stage = smem_s + TB_RING + slot * STAGE_BYTES;
+    const u32 fl = PAGED ? stage + (2 * ti + (lane >> 4)) * PSLOT + SLOT_FL_OFF : stage + (lane >> 4) * SIDE_BYTES + SB_FL + 4 * T * ti;
+    const int win = plan_tile(!(lane >> 4 ? rawv : rawk), fl, (u32)own.x, own.y, W, area, PATCH_MAX, lane);
+    const int2 m = reinterpret_cast<const int2*>(smem + TB_META)[nth];
+    const uint8_t* const s0 = smem + TB_RING + slot * STAGE_BYTES;
+    const SideView ks = PAGED ? SideView{s0 + 2 * ti * PSLOT, s0 + 2 * ti * PSLOT + SLOT_CD_OFF, p.buf + (long)m.x * p.TS + SLOT_OVF_OFF}
+                              : SideView{s0 + ti * TILE_SM, s0 + SB_CD + ti * TILE_CD, p.K.ovf + ((long)ohk + m.x)};
+    const SideView vs = PAGED ? SideView{s0 + (2 * ti + 1) * PSLOT, s0 + (2 * ti + 1) * PSLOT + SLOT_CD_OFF, p.buf + (long)m.y * p.TS + SLOT_OVF_OFF}
+                              : SideView{s0 + SIDE_BYTES + ti * TILE_SM, s0 + SIDE_BYTES + SB_CD + ti * TILE_CD, p.V.ovf + ((long)ohv + m.y)};
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (!rawk) k_tile<DUMP>(sc, ks, plan, W, lane, Q, dump_k + (long)tile * T * D, nvalid);
-    else raw_scores<DUMP>(sc, p.raw + (long)raw_tile(cur.mk) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
+    if (!rawk) k_tile<DUMP>(sc, ks, win, area, W, lane, Q, dump_k + (long)tile * T * D, nvalid);
+    else raw_scores<DUMP>(sc, p.raw + (long)raw_tile(m.x) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
     nx = __shfl_sync(FULLM, nx, 0);
+    if (st + NSTG < nstages) ahead = stage_meta(st + NSTG);                  // in case that this warp fills the stage again
     PFrag<NSET> P;
     if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
     else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
-    if (!rawv) v_tile<DUMP, NSET>(A, vs, plan, W, lane, P, dump_v + (long)tile * T * D, nvalid);
-    else raw_accum<DUMP, NSET>(A, p.raw + (long)raw_tile(cur.mv) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
-    // the stage's bytes may have been written through ordinary stores (patch numbers): order those before the copy engine's next
-    // writes to the same bytes, then count this warp out of the stage
+    if (!rawv) v_tile<DUMP, NSET>(A, vs, win, area, W, lane, P, dump_v + (long)tile * T * D, nvalid);
+    else raw_accum<DUMP, NSET>(A, p.raw + (long)raw_tile(m.y) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
+    __syncwarp();                                    // every lane is done with the tile and with the area
     if (st + NSTG < nstages) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        int left;
-        asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(left) : "r"(smem_s + TB_DONE + 4 * slot) : "memory");
-        if ((left & (TPS - 1)) == TPS - 1) {
-          const int ns = st + NSTG, i0 = ns * TPS;
-          if (PAGED) {
-            TileMeta m[TPS];
-#pragma unroll
-            for (int t = 0; t < TPS; t++) m[t] = i0 + t < n ? meta_of(i0 + t) : TileMeta{-1, -1};
-            issue_paged(ns, m);
-          } else {
-            const TileMeta m0 = meta_of(i0), m1 = i0 + TPS < n ? meta_of(i0 + TPS) : TileMeta{FAR, FAR};
-            issue_payload(ns);
-            issue_rest(ns, m0, m1);
-          }
-        }
+      int left = 0;
+      if (lane == 0) asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(left) : "r"(smem_s + TB_LEFT + 4 * slot) : "memory");
+      left = __shfl_sync(FULLM, left, 0);
+      if ((left & (TPS - 1)) == TPS - 1) {
+        __syncwarp();
+        if (!PAGED) fill_payload(st + NSTG);
+        fill_rest(st + NSTG, ahead);
       }
     }
     it = nx;
@@ -720,13 +701,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 // nobody is left at the barrier.
 // Output: partials of "virtual heads" vq = 2 * query head + half, which the last CTA of a (row, kv head) merges into out [B, n_q, 256].
 
-constexpr int META256_TILES = 128;
+constexpr int META256_TILES = 64, PATCH256 = 48, SEG256_BYTES = SEG_PATCH + 8 * PATCH256;
 constexpr int CTL_BYTES = 16;                                      // of a pair and tile parity: {next tile, fail flag of half 0, of half 1, -}
-constexpr int T256_BASES = LUTX_BYTES, T256_ZERO = T256_BASES + 2 * BASES_BYTES, T256_META = T256_ZERO + 16, T256_CTL = T256_META + META256_TILES * 16;
-constexpr int T256_SCRATCH = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SCRATCH + ATT_WARPS * WARP_SCRATCH;
+constexpr int T256_BASES = ADDEND_BYTES + SEGTAB_BYTES, T256_META = T256_BASES + 2 * BASES_BYTES, T256_CTL = T256_META + META256_TILES * 16;
+constexpr int T256_SEG = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SEG + ATT_WARPS * SEG256_BYTES;
 constexpr int STAGE256_BYTES = 16 + 2 * PSLOT, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
-constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES;
-static_assert(T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 64 <= 232448, "one CTA per SM");
+constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;          // (an escape segment is read as whole words)
+static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 64 <= 232448, "one CTA per SM");
 
 template <int NSET>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
@@ -738,8 +719,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   const int b = bh / p.n_kv, kvh = bh % p.n_kv, G = p.G, NT = 4 * p.n_kv;    // p.n_kv = 256-dim kv heads; NT tile slots per block
   const int ring = T256_RING + warp * WARP256_BYTES;
   const u32 smem_s = (u32)__cvta_generic_to_shared(smem), ring_s = smem_s + ring;
-  if (tid < 256) fill_lutx(reinterpret_cast<u32x2*>(smem), tid);
-  if (tid >= 256 && tid < 260) reinterpret_cast<u32*>(smem + T256_ZERO)[tid - 256] = 0u;
+  if (tid < 256) fill_attn_tables(smem, tid);
   if (tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
   if (lane == 0) {
     mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
@@ -778,7 +758,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   if (warp >= 8 && warp < 12) {
     const int h2 = warp & 1, row = (2 * kvh + h2) * D;
     uint8_t* o = smem + T256_BASES + h2 * BASES_BYTES;
-    if (warp < 10) fill_bases<false>(o, p.b3k + row, p.b4k + row, lane); else fill_bases<true>(o, p.b3v + row, p.b4v + row, lane);
+    if (lane < 16) { if (warp < 10) fill_pair_bases<false>(o, p.b3k + row, p.b4k + row, lane); else fill_pair_bases<true>(o, p.b3v + row, p.b4v + row, lane); }
   }
   if (tid < min(n, META256_TILES)) { const int pc = slot_of(tid); reinterpret_cast<int4*>(smem + T256_META)[tid] = make_int4(p.mt[pc], p.mt[pc + 1], p.mt[pc + 2], p.mt[pc + 3]); }
   if (tid == 0) s_next = ATT_WARPS / 2;               // tiles 0 .. pairs - 1 of the range go to the pairs in order, the rest is handed out on demand
@@ -786,7 +766,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   A.clear();
   __syncthreads();
 
-  const WarpView W{smem_s, smem_s + T256_BASES + hf * BASES_BYTES, smem_s + T256_ZERO, smem_s + T256_SCRATCH + warp * WARP_SCRATCH};
+  const AttnView W = attn_view(smem_s, smem_s + T256_BASES + hf * BASES_BYTES);
+  const u32 area = smem_s + T256_SEG + warp * SEG256_BYTES;
   int stg = 0, par = 0;
   u32 phase = 0;
   const int avail = min(p.ovf_slot, (int)slot_bytes - SLOT_OVF_OFF);
@@ -799,13 +780,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     const uint8_t* stage = smem + so;
     const int nvalid = min(T, S - (tlo + it) * T);
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
-    const u32 esc = smem_s + so + SLOT_OVF_OFF;
-    const SideView ks{stage, stage + SLOT_CD_OFF, stage + SLOT_FL_OFF, esc, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF, avail};
-    const SideView vs{stage + PSLOT, stage + PSLOT + SLOT_CD_OFF, stage + PSLOT + SLOT_FL_OFF, esc + PSLOT, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF, avail};
-    TilePlan plan{};
+    const SideView ks{stage, stage + SLOT_CD_OFF, p.buf + (long)cur.mk * p.TS + SLOT_OVF_OFF};
+    const SideView vs{stage + PSLOT, stage + PSLOT + SLOT_CD_OFF, p.buf + (long)cur.mv * p.TS + SLOT_OVF_OFF};
+    int win = 0;
     if (ok) {
-      plan = plan_tile(ks, vs, cur.mk < 0, cur.mv < 0, W, lane);
-      if (cur.mk >= 0) k_tile<false>(sc, ks, plan, W, lane, Q, nullptr, nvalid);
+      const u32 t0 = smem_s + so + (lane >> 4) * PSLOT;
+      win = plan_tile((lane >> 4 ? cur.mv : cur.mk) >= 0, t0 + SLOT_FL_OFF, t0 + SLOT_OVF_OFF, avail, W, area, PATCH256, lane);
+      if (cur.mk >= 0) k_tile<false>(sc, ks, win, area, W, lane, Q, nullptr, nvalid);
       else raw_scores<false>(sc, p.raw + (long)raw_tile(cur.mk) * (T * D), nvalid, lane, Q, nullptr);
     }
     // ---- the two halves' partial scores meet; the next tile's number and a failed wait travel with them
@@ -825,7 +806,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     PFrag<NSET> P;
     if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
     else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
-    if (cur.mv >= 0) v_tile<false, NSET>(A, vs, plan, W, lane, P, nullptr, nvalid);
+    if (cur.mv >= 0) v_tile<false, NSET>(A, vs, win, area, W, lane, P, nullptr, nvalid);
     else raw_accum<false, NSET>(A, p.raw + (long)raw_tile(cur.mv) * (T * D), nvalid, lane, P, nullptr);
     cur = nxt; stg ^= 1; it = t1;
     __syncwarp();                                      // every lane has read this stage before its next copies are issued

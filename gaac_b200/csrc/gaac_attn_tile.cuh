@@ -1,10 +1,10 @@
 // Warp-level pieces of the fused decode attention: asynchronous copies, the rebuild of a compressed 16-token tile into tensor-core
 // fragments, the score and value products and the online softmax step.  Used by the kernels of gaac_attn.cu.
 //
-// What bounds them: instruction issue and the integer (ALU) pipe, whose rate is half the issue rate, not HBM.  Measured on a B200
-// at batch 1, 32 query / 8 kv heads, 65536 tokens: 1354 warp instructions per (K tile + V tile) at 67 % issue slots used before the
-// forms below, of which the group decoder itself is about 530; the rest was copy issue per warp, escape offsets through two
-// lookups per row, a transpose of the V fragments and softmax work for padding heads.
+// What bounds them: instruction issue, not HBM.  Measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens: 1090 warp instructions per (K
+// tile + V tile), the ALU pipe and the shared-memory pipe at 70 % each and 0.68 instructions per cycle and scheduler inside the main loop, with four warps
+// to a scheduler.  Timing-only builds of a near form: without the raw groups 50 us of 57, without any of plan_tile 41.  What did not help: moving shifts from the
+// ALU to the FMA pipe, fewer or longer chains at the same count of instructions, warps of their own for plan_tile or for the copies (see gaac_attn.cu).
 //
 // Head columns.  The tensor-core tile has 8 columns.  Query heads are handled in sets of four (NSET = 1 for a GQA group of up to
 // 4, 2 for 5..8); lane j of a quad works for head 4 * set + j throughout:
@@ -39,6 +39,17 @@ __device__ __forceinline__ void mbar_add_tx(u32 mbar, u32 bytes) { asm volatile(
 __device__ __forceinline__ void bulk_g2s(u32 dst, const void* src, u32 bytes, u32 mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
 }
+// The same issued by one lane of a converged warp.  Executed by the whole warp with operands that are uniform, so that they go straight into the copy instruction's
+// uniform registers: behind a branch on the lane number the compiler picks them up lane by lane in a loop.
+__device__ __forceinline__ void warp_expect_tx(u32 mbar, u32 bytes) {
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n @p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void warp_add_tx(u32 mbar, u32 bytes) {
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n @p mbarrier.expect_tx.shared::cta.b64 [%0], %1;\n}\n" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void warp_g2s(u32 dst, const void* src, u32 bytes, u32 mbar) {
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n @p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
+}
 // Bounded wait for a phase of the barrier: false when it gave up (the copies of a stage normally land within microseconds;
 // the bound is there so that a lost copy can never hang the GPU).
 constexpr int MBAR_WAIT_LIMIT = 1 << 22;
@@ -50,12 +61,14 @@ __device__ __forceinline__ bool mbar_wait(u32 mbar, u32 parity) {
   }
   return false;
 }
-// The same for a count in shared memory that other warps raise: waits until it is at least `least`.
-__device__ __forceinline__ bool wait_count(u32 addr, int least) {
+// The same for the phase that belongs to use number `use` of the barrier, as a word in shared memory says: it is `use` << 4 | flags when the phase has begun.
+__device__ __forceinline__ bool mbar_wait_use(u32 mbar, u32 parity, u32 word, u32 use, u32& flags) {
   for (int it = 0; it < MBAR_WAIT_LIMIT; it++) {
-    int v;
-    asm volatile("ld.relaxed.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-    if (v >= least) return true;
+    u32 v, ok;
+    asm volatile("ld.relaxed.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(word) : "memory");
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(mbar), "r"(parity) : "memory");
+    flags = v & 15u;
+    if (ok && v >> 4 == use) return true;
   }
   return false;
 }
@@ -65,8 +78,9 @@ __device__ __forceinline__ float fast_exp2(float x) { float y; asm("ex2.approx.f
 // escape bytes.  Paged layout: the mode-table entries (>= 0: compressed slot, < 0: bit-complement of a raw tile of the pool).
 struct TileMeta { int mk, mv; };
 
-// ---- running state of one warp.  acc[set][mt][c] = O[head 4 * set + j][channel 8 * (4 * mt + c) + r]; m, l in the exp2 domain, l summed over
-// this lane's tokens only
+// ---- running state of one warp.  acc[set][mt][c] = O[head 4 * set + j][channel 8 * acc_channel(mt, c) + r]; m, l in the exp2 domain, l summed over
+// this lane's tokens only.  Words mt and c >> 1 hold elements that are four apart.
+__host__ __device__ constexpr int acc_channel(int mt, int c) { return 8 * (mt >> 1) + 2 * (mt & 1) + (c >> 1) + 4 * (c & 1); }
 template <int NSET> struct WarpAcc {
   float acc[NSET][4][4];
   float m[NSET], l[NSET];
@@ -80,8 +94,8 @@ template <int NSET> struct WarpAcc {
   }
 };
 
-// Q^T B-fragments of the score product.  Lane (j, r) provides column r = head 4 * (r & 1) + (r >> 1): for k-step s the words
-// q[16s + 2j, +1] and q[16s + 2j + 8, +9] of that head (zero where the group has no such head).
+// Q^T B-fragments of the score product.  Lane (j, r) provides column r = head 4 * (r & 1) + (r >> 1), zero where the group has no such head; the words pair the
+// channels that a rebuilt word pairs: product 2g has c and c + 16, then c + 1 and c + 17 (c = 32g + 2j), product 2g + 1 the same 8 channels on.
 struct QFrag { u32 qa[8][2]; };
 __device__ __forceinline__ int q_head(int r) { return 4 * (r & 1) + (r >> 1); }
 __device__ __forceinline__ void load_q(QFrag& Q, const uint16_t* q0, long head_stride, int G, int lane) {
@@ -89,14 +103,15 @@ __device__ __forceinline__ void load_q(QFrag& Q, const uint16_t* q0, long head_s
   const uint16_t* qp = q0 + (h < G ? h : 0) * head_stride;
 #pragma unroll
   for (int s = 0; s < 8; s++) {
-    Q.qa[s][0] = h < G ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j) : 0u;
-    Q.qa[s][1] = h < G ? *reinterpret_cast<const u32*>(qp + 16 * s + 2 * j + 8) : 0u;
+    const uint16_t* c = qp + 32 * (s >> 1) + 2 * j + 8 * (s & 1);
+    const u32 a = h < G ? *reinterpret_cast<const u32*>(c) : 0u, b = h < G ? *reinterpret_cast<const u32*>(c + 16) : 0u;
+    Q.qa[s][0] = prmt(a, b, 0x5410); Q.qa[s][1] = prmt(a, b, 0x7632);
   }
 }
 
 // Weights of one tile as B-fragments of the value product.  A weight enters as the sum of two BF16 numbers, its rounded value (hi) and the rounded
-// remainder (lo), which brings its relative error to 2^-16.  One set: [0]: tokens 2j (b0) and 2j + 1 (b1), [1]: tokens 2j + 8 and 2j + 9.  Two: [0]:
-// tokens 2j, 2j + 1, [1]: tokens 2j + 8, 2j + 9.
+// remainder (lo), which brings its relative error to 2^-16.  One set: [0]: places 0 (b0) and 1 (b1) of slot_token, [1]: places 2 and 3.  Two: [0]:
+// places 0, 1, [1]: places 2, 3.
 template <int NSET> struct PFrag;
 template <> struct PFrag<1> { u32 hi[2][2], lo[2][2]; };
 template <> struct PFrag<2> { u32 hi[2], lo[2]; };
@@ -104,12 +119,17 @@ __device__ __forceinline__ u32 pack_bf16(float lo, float hi) { __nv_bfloat162 x 
 // what the rounding of a pair dropped, which fp32 holds exactly, rounded in turn
 __device__ __forceinline__ u32 pack_rest(float lo, float hi, u32 rounded) { return pack_bf16(lo - __uint_as_float(rounded << 16), hi - __uint_as_float(rounded & 0xFFFF0000u)); }
 
+// Token of the lane's place i in the value product: places 0, 1 are tokens 2j, 2j + 1 and places 2, 3 the same 8 on, for lanes j = 2, 3 the other way round.  A lane's four
+// tokens lie 64 bytes from the next lane's in a staged V tile; read in one order by all lanes they meet in a quarter of the banks, so that half of them start at
+// the other end.  (0.6 % of the kernel.)
+__device__ __forceinline__ int slot_token(int j, int i) { return 2 * j + (i & 1) + 8 * ((i >> 1) ^ (j >> 1)); }
 // p0, p8: this lane's weights of tokens r and r + 8 for head j of each set.
-// One set: as column r of the value product the lane needs those of head r >> 1 for tokens 2j, 2j + 1, 2j + 8, 2j + 9, in the low (parity 0) or high
+// One set: as column r of the value product the lane needs those of head r >> 1 for the tokens of its places, in the low (parity 0) or high
 // (parity 1) half of a word whose other half is zero.
 __device__ __forceinline__ void put_weights(PFrag<1>& P, const float (&p0)[1], const float (&p8)[1], int lane) {
   const int j = lane & 3, r = lane >> 2, src = 8 * j + (r >> 1);
-  const u32 sel0 = (r & 1) ? 0x1044u : 0x4410u, sel8 = (r & 1) ? 0x3244u : 0x4432u;
+  const bool sw = j >= 2;
+  const u32 selA = (r & 1) ? 0x1044u : 0x4410u, selB = (r & 1) ? 0x3244u : 0x4432u, sel0 = sw ? selB : selA, sel8 = sw ? selA : selB;
   const u32 H = pack_bf16(p0[0], p8[0]), L = pack_rest(p0[0], p8[0], H);
   const u32 ha = __shfl_sync(FULLM, H, src), hb = __shfl_sync(FULLM, H, src + 4), la = __shfl_sync(FULLM, L, src), lb = __shfl_sync(FULLM, L, src + 4);
   P.hi[0][0] = prmt(ha, 0u, sel0); P.hi[0][1] = prmt(hb, 0u, sel0); P.hi[1][0] = prmt(ha, 0u, sel8); P.hi[1][1] = prmt(hb, 0u, sel8);
@@ -119,7 +139,9 @@ __device__ __forceinline__ void put_weights(PFrag<1>& P, const float (&p0)[1], c
 __device__ __forceinline__ void put_weights(PFrag<2>& P, const float (&p0)[2], const float (&p8)[2], int lane) {
   const int j = lane & 3, r = lane >> 2, src = 8 * j + (r >> 1);
   const u32 sel = (r & 1) ? 0x7632u : 0x5410u;
-  const u32 h0 = pack_bf16(p0[0], p0[1]), h8 = pack_bf16(p8[0], p8[1]), l0 = pack_rest(p0[0], p0[1], h0), l8 = pack_rest(p8[0], p8[1], h8);
+  const bool sw = lane >= 16;                          // the lanes that read from this one have their places the other way round
+  const float x0 = sw ? p8[0] : p0[0], x1 = sw ? p8[1] : p0[1], y0 = sw ? p0[0] : p8[0], y1 = sw ? p0[1] : p8[1];
+  const u32 h0 = pack_bf16(x0, x1), h8 = pack_bf16(y0, y1), l0 = pack_rest(x0, x1, h0), l8 = pack_rest(y0, y1, h8);
   const u32 a0 = __shfl_sync(FULLM, h0, src), b0 = __shfl_sync(FULLM, h0, src + 4), a8 = __shfl_sync(FULLM, h8, src), b8 = __shfl_sync(FULLM, h8, src + 4);
   const u32 c0 = __shfl_sync(FULLM, l0, src), d0 = __shfl_sync(FULLM, l0, src + 4), c8 = __shfl_sync(FULLM, l8, src), d8 = __shfl_sync(FULLM, l8, src + 4);
   P.hi[0] = prmt(a0, b0, sel); P.hi[1] = prmt(a8, b8, sel); P.lo[0] = prmt(c0, d0, sel); P.lo[1] = prmt(c8, d8, sel);
@@ -163,7 +185,7 @@ __device__ __forceinline__ void softmax_step(WarpAcc<NSET>& A, const float* sc, 
   put_weights(P, p0, p8, lane);
 }
 
-// Value product of words i, i + 1 (i = 2 * mt) of the lane's four tokens (2j, 2j + 1, 2j + 8, 2j + 9).
+// Value product of two words (2 * mt and the next) of the lane's four tokens (2j, 2j + 1, 2j + 8, 2j + 9).
 __device__ __forceinline__ void pv_words(WarpAcc<1>& A, int mt, const u32 (&w0)[4], const u32 (&w1)[4], const PFrag<1>& P) {
   mma16816(A.acc[0][mt], w0[0], w1[0], w0[1], w1[1], P.hi[0][0], P.hi[0][1]);
   mma16816(A.acc[0][mt], w0[0], w1[0], w0[1], w1[1], P.lo[0][0], P.lo[0][1]);
@@ -187,80 +209,134 @@ __device__ __forceinline__ void pv_words(WarpAcc<2>& A, int mt, const u32 (&w0)[
 // promoted 48.5 us, now 36.1 (33.6 with tables that fit); paged, half of the channels off: 42.1, now 38.3.
 constexpr int ESC_WIN = 256;
 constexpr int PSLOT = SLOT_OVF_OFF + ESC_WIN + 16;          // staged bytes of a paged tile slot, at most
-constexpr int PATCH_MAX = 64;                               // raw groups of a tile (K and V together) that the patch table holds
-constexpr int PATCH_BYTES = PATCH_MAX * 8, WALK_BYTES = 32 * 16;
-constexpr int WARP_SCRATCH = PATCH_BYTES + WALK_BYTES;      // shared memory of a warp besides its stages: patch table, segment positions per lane
+// What a planned tile pair has in shared memory (its segment area): segment words of K and of V, [row][quarter of a row], 8 bytes per segment, then the entries of
+// its raw groups.  PATCH_MAX: raw groups of a tile pair (of 512) that have room; a pair with more takes the plain decoder.
+constexpr int PATCH_MAX = 64, SEG_K = 0, SEG_V = 64 * 8, SEG_PATCH = 2 * SEG_V;
+constexpr int AREA_BYTES = SEG_PATCH + 8 * PATCH_MAX;
+// Addend table: entry NO_ESC (zero) and entries 256 + byte, 8 bytes each; segment table: 256 entries of 8 bytes
+constexpr int ADDEND_BYTES = 8 + 257 * 8, SEGTAB_BYTES = 256 * 8;
 
-// One side (K or V) of a staged tile.  esc = shared-memory address of its first escape byte, glob = the same bytes in global memory, avail = staged escape
-// bytes.
-struct SideView { const uint8_t *sm, *cd, *fl; u32 esc; const uint8_t* glob; int avail; };
-// ---- where a lane's escape bytes are.  A lane owns 8 groups of a K tile (tokens r and r + 8, groups 4j .. 4j + 3 of each) and 8 of a V tile
-// (groups 2r, 2r + 1 of tokens 2j, 2j + 1, 2j + 8, 2j + 9).
-//   tags  2 bits per group: K segments (8 bits) at bits 0 and 8, V segments (4 bits) at bits 16, 20, 24, 28
-//   k, v  position of each segment's first escape byte inside the tile side, two per word
-//   win   bit 0 / 1: the K / V side takes the decoder with staged escape bytes
-struct TilePlan { u32 tags, k, v[2]; int win; };
-
-// Turn the raw-tier groups of a staged tile (K and V in one pass) into patch-table entries, so that the group decoder needs no branch.  A lane
-// walks its own raw groups: read the five payload bytes, spread the 5-bit fields to byte positions, take off the 4-bit-window base words (the
-// decoder adds them to every promoted group), store the two words as entry k, and write k over the first payload byte, which is where the
-// decoder looks.  Returns false when there are more than PATCH_MAX (the caller then takes the decoder that reads global memory, so the bytes
-// written over do not matter).  At a raw share of 0.75 % a tile pair has 3.8 raw groups, hardly ever two in one lane: one trip.
-__device__ __forceinline__ bool build_raw_patches(u32 raw_bits, const TilePlan& t, u32 esc_k, u32 esc_v, const WarpView& w, int lane) {
-  u32 some = __ballot_sync(FULLM, raw_bits != 0u);
-  if (!some) return true;
-  const u32 mine = w.scratch + PATCH_BYTES + 16 * lane, j = lane & 3, r = lane >> 2;
-  sts_u128(mine, prmt(t.k, 0u, 0x1010), prmt(t.k, 0u, 0x3232), t.v[0], t.v[1]);        // position by quarter of the tag word: the walk picks one at run time
-  u32 base = 0;
-  do {
-    const u32 n = base + (u32)popc(some);
-    if (n > PATCH_MAX) return false;
-    if (raw_bits) {
-      const u32 bit = (u32)__ffs((int)raw_bits) - 1u;                // upper tag bit of the group
-      raw_bits &= raw_bits - 1u;
-      const bool isv = bit >= 16u;
-      const u32 first = bit & (isv ? ~3u : ~7u);                     // first tag bit of its segment
-      const u32 below = (t.tags >> first) & ((1u << (bit - 1u - first)) - 1u);
-      const u32 pl = (isv ? esc_v : esc_k) + lds_u16(mine + ((bit >> 2) << 1)) + seg_esc(below);
-      const u32 k = base + (u32)popc(some & ((1u << lane) - 1u));
-      const u32x4 bw = lds_u128(w.bases + (isv ? BASES_V + 32u * r + 8u * (bit & 2u) : 64u * j + 8u * (bit & 6u)));
-      const u32x2 x = raw_addends(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * (pl & 3u), bw.x + bw.z, bw.y + bw.w);
-      sts_u64(w.scratch + 8u * k, x.x, x.y);
-      sts_u8(pl, k);
-    }
-    base = n;
-    some = __ballot_sync(FULLM, raw_bits != 0u);
-  } while (some);
-  __syncwarp();
-  return true;
+// Shared-memory addresses that do not change from tile to tile: entry 0 of the addend table (which begins with entry NO_ESC), the segment table, the base words
+// (K, then V).  Segment areas lie behind the tables.
+struct AttnView { u32 addends, segs, bases; };
+// Fill the tables with threads t = 0 .. 255.  at: ADDEND_BYTES + SEGTAB_BYTES on a 16-byte boundary; returned: the addresses of the view.
+__device__ __forceinline__ void fill_attn_tables(uint8_t* at, int t) {
+  const u32x2 x = pair_addends((u32)t), s = segment_entry((u32)t);
+  reinterpret_cast<uint2*>(at + 16)[t] = make_uint2(x.x, x.y);
+  reinterpret_cast<uint2*>(at + ADDEND_BYTES)[t] = make_uint2(s.x, s.y);
+  if (t == 0) reinterpret_cast<uint2*>(at + 8)[0] = make_uint2(0u, 0u);
+}
+__device__ __forceinline__ AttnView attn_view(u32 tables, u32 bases) { return AttnView{tables + 16 - 256 * 8, tables + ADDEND_BYTES, bases}; }
+// Base words of a side: group t of 16 by thread t (16 bytes each; K: lane class j, group g at 64 * j + 16 * g; V: class r, group g at 32 * r + 16 * g, 256 bytes on)
+template <bool VSIDE>
+__device__ __forceinline__ void fill_pair_bases(uint8_t* bases, const uint8_t* b3, const uint8_t* b4, int t) {
+  const u32x4 w = pair_base_words<VSIDE>(b3, b4, t);
+  *reinterpret_cast<uint4*>(bases + (VSIDE ? BASES_V : 0) + 16 * t) = make_uint4(w.x, w.y, w.z, w.w);
 }
 
-__device__ __forceinline__ TilePlan plan_tile(const SideView& ks, const SideView& vs, bool rawk, bool rawv, const WarpView& w, int lane) {
-  const int j = lane & 3, r = lane >> 2;
-  TilePlan t;
-  u32 k0 = 0, k1 = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-  if (!rawk) { k0 = ks.fl[lane]; k1 = ks.fl[32 + lane]; }                                     // byte j of row r's tag word is byte `lane` of the octet's 32
-  if (!rawv) {
-    const uint2 a = *reinterpret_cast<const uint2*>(vs.fl + 8 * j), b = *reinterpret_cast<const uint2*>(vs.fl + 32 + 8 * j);      // tag words of the four tokens
-    v0 = (a.x >> (4 * r)) & 15u; v1 = (a.y >> (4 * r)) & 15u; v2 = (b.x >> (4 * r)) & 15u; v3 = (b.y >> (4 * r)) & 15u;
+// One side (K or V) of a staged tile; glob = its escape bytes in global memory.
+struct SideView { const uint8_t *sm, *cd, *glob; };
+// ---- escape bytes of a tile pair.  A segment is four neighbouring groups of a row, one byte of its tag word.  It is expanded into a word per two groups with a
+// 16-bit index into the addend table for each (gaac_tile.h), which go to the tile pair's segment area, where the lanes that rebuild the groups find them.  A side whose escape bytes are not all staged has {tag byte | position << 16} there instead, and
+// its escape bytes are read from global memory.
+// Once per segment, because a group's share of it (tag bits, position, byte, table address) cost 10 of the 37 instructions of its rebuild.
+
+// One step of an inclusive scan over each half of a warp (scan_step over all of it).
+__device__ __forceinline__ void scan_step16(u32& v, int d) {
+  asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0x1000, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
+}
+// Make the segment area of a tile pair.  Lane l has row l & 15 of K (l < 16) or of V.  live: the lane's side is compressed; fl, esc: shared-memory addresses of its
+// tag words and of its escape bytes, of which `avail` are staged.  Returned: bit 0 / 1: those of K / V are all staged (and there are no more than `room` items of
+// raw_items, which have their entries, 8 bytes each, behind the segment words).  Bound by its chain of latencies, hence a scan over 16 rows and not over 64 segments,
+// sizes from the tag words while the segment table answers, and items taken as they are found: a tile pair has 4.8 at a raw share of 0.75 %, hardly two in a row.
+// About 190 of the 1090 instructions per tile pair.  65536 tokens, 8 kv heads: 59.0 us with a look-up per group and raw groups as table entries found by the decoder
+// (1192 instructions), 56.2 with this and rebuild_pairs; slot cache 64 x 32768, group of 8: 247 -> 233; paged 16 x 4096..65536, 8 kv heads: 516 -> 493.
+__device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avail, const AttnView& w, u32 area, u32 room, int lane) {
+  const u32 fl = live ? lds_u32(fl_at + 4u * (lane & 15)) : 0u;
+  const u32 size = (u32)row_esc_bytes(fl);
+  u32x2 e[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) e[q] = lds_u64(w.segs + (q < 3 ? 8u * ((fl >> (8 * q)) & 0xFFu) : 8u * (fl >> 24)));
+  u32 end = size;
+  scan_step16(end, 1); scan_step16(end, 2); scan_step16(end, 4); scan_step16(end, 8);
+  const u32 over = __ballot_sync(FULLM, live && (int)end > avail);
+  int staged = ((over & 0xFFFFu) ? 0 : 1) | ((over >> 16) ? 0 : 2);
+  const u32 mine = area + SEG_V * (lane >> 4) + 32u * (lane & 15);
+  bool fast = (staged >> (lane >> 4)) & 1;
+  u32 items = 0u;
+  if (fast) {
+    u32 at = live ? esc + end - size : area, a = at, four[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const u32 lo = lds_u32(a & ~3u), hi = lds_u32((a & ~3u) + 4u);
+      four[q] = __funnelshift_r(lo, hi, 8u * a);                             // (the shift counts modulo 32)
+      a += e[q].y;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q += 2)
+      sts_u128(mine + 8u * q, prmt(four[q], SEG_CONST, e[q].x), prmt(four[q], SEG_CONST, e[q].x >> 16), prmt(four[q + 1], SEG_CONST, e[q + 1].x), prmt(four[q + 1], SEG_CONST, e[q + 1].x >> 16));
+    items = raw_items(fl);
   }
-  u32 ktot, vtot;
-  tile_positions<true, true>(k0, k1, v0, v1, v2, v3, j, t.k, ktot, t.v, vtot);
-  t.tags = mad_k<256u>(k1, k0) + mad_k<65536u>(v0, mad_k<1048576u>(v1, mad_k<16777216u>(v2, mad_k<268435456u>(v3, 0u))));
-  const int total_k = (int)((ktot & 0xFFFFu) + (ktot >> 16)), total_v = (int)((vtot & 0xFFFFu) + (vtot >> 16));
-  t.win = (total_k <= ks.avail ? 1 : 0) | (total_v <= vs.avail ? 2 : 0);
-  const u32 sides = ((t.win & 1) ? 0xAAAAu : 0u) | ((t.win & 2) ? 0xAAAA0000u : 0u);
-  if (!build_raw_patches(t.tags & sides, t, ks.esc, vs.esc, w, lane)) t.win = 0;
-  return t;
+  u32 some, entry = area + SEG_PATCH;
+  while ((some = __ballot_sync(FULLM, items != 0u)) != 0u) {                 // an item of every row that has one
+    const u32 n = (u32)popc(some);
+    if (entry + 8u * n > area + SEG_PATCH + 8u * room) { staged = 0; fast = false; break; }
+    if (items) {
+      const u32 bit = (u32)__ffs((int)items) - 1u, pl = esc + end - size + (u32)esc_prefix(fl, (int)bit);       // bit: lower tag bit of the group, 2 * group
+      u32 index;
+      items &= items - 1u;
+      if ((fl >> bit) & 2u) {                          // the upper bits of the exponents, less what the decoder will add to them
+        const u32 own = entry + 8u * (u32)popc(some & ((1u << lane) - 1u));
+        index = (own - w.addends) >> 3;
+        const u32 m = index >> 8;
+        const u32x4 bw = lds_u128(w.bases + BASES_V * (lane >> 4) + 8u * bit);
+        const u32x2 x = pair_raw_addends(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * (pl & 3u));
+        sts_u64(own, x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w);
+      } else index = 256u + lds_u8(pl);
+      sts_u16(mine + bit, index);
+    }
+    entry += 8u * n;
+  }
+  if (!fast) {                                       // {tag byte | position << 16}
+    u32 pos = end - size;
+#pragma unroll
+    for (int q = 0; q < 4; q++) { sts_u64(mine + 8u * q, ((fl >> (8 * q)) & 0xFFu) | pos << 16, 0u); pos += e[q].y; }
+  }
+  __syncwarp();
+  return staged;
+}
+
+// One group whose escape bytes are staged: half = its 16 bits of the segment words are the upper ones.
+__device__ __forceinline__ void decode_staged(u32 sm_lo, u32 sm_hi, u32 u, u32 word, bool half, const AttnView& w, const u32x4& bw, u32 out[4]) {
+  const u32 index = half ? word >> 16 : word & 0xFFFFu, m = half ? word >> 24 : index >> 8;
+  rebuild_pairs(sm_lo, sm_hi, u, m, bw, lds_u64(mad_k<8u>(index, w.addends)), out);
+}
+// One group whose escape bytes are read from global memory at glob[pos]; tg = its tag in the low bits.  pos advances past them.
+__device__ __forceinline__ void decode_plain(u32 sm_lo, u32 sm_hi, u32 u, u32 tg, u32& pos, const uint8_t* glob, const AttnView& w, const u32x4& bw, u32 out[4]) {
+  const u32 m = tg & 1u;
+  u32x2 x = lds_u64(w.addends + 8u * (m ? 256u + glob[pos] : NO_ESC));
+  if (tg & 2u) {
+    const uint8_t* p = glob + pos;
+    const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+    x = pair_raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3));
+    x.x -= bw.x + bw.z; x.y -= bw.y + bw.w;
+    pos += 4;
+  }
+  pos += m;
+  rebuild_pairs(sm_lo, sm_hi, u, m, bw, x, out);
 }
 
 // ---- score product of one compressed K tile: sc += K . Q^T.  dump (debug instantiation only): where token 0 of this tile goes in the
 // [token][128] dump of the head; rows >= nvalid are left alone.
 template <bool WIN, bool DUMP>
-__device__ __forceinline__ void k_decode(float* sc, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const QFrag& Q, uint16_t* dump, int nvalid) {
+__device__ __forceinline__ void k_decode(float* sc, const SideView& s, u32 area, const AttnView& w, int lane, const QFrag& Q, uint16_t* dump, int nvalid) {
   const int j = lane & 3, r = lane >> 2;
-  const u32 from = WIN ? s.esc - w.zero : 0u;
-  u32 pos[2] = {(t.k & 0xFFFFu) + from, (t.k >> 16) + from};
+  u32 seg[2][2], pos[2] = {0u, 0u};                    // staged: the words of the lane's two segments;  not staged: tag bytes and positions
+#pragma unroll
+  for (int o = 0; o < 2; o++) {
+    const u32x2 v = lds_u64(area + SEG_K + 256u * o + 8u * lane);
+    seg[o][0] = WIN ? v.x : v.x & 0xFFu; seg[o][1] = v.y; pos[o] = v.x >> 16;
+  }
   uint4 s0[2], s1[2]; u32 cd[2][3];
   float s2[4] = {0.f, 0.f, 0.f, 0.f};                  // second accumulator: two dependent MMA chains of four instead of one of eight
 #pragma unroll
@@ -278,16 +354,17 @@ __device__ __forceinline__ void k_decode(float* sc, const SideView& s, const Til
     for (int o = 0; o < 2; o++) {
       const u32 smlo = g == 0 ? s0[o].x : g == 1 ? s0[o].z : g == 2 ? s1[o].x : s1[o].z;
       const u32 smhi = g == 0 ? s0[o].y : g == 1 ? s0[o].w : g == 2 ? s1[o].y : s1[o].w;
-      const u32 z = g == 0 ? group_codes<0>(cd[o]) : g == 1 ? group_codes<3>(cd[o]) : g == 2 ? group_codes<6>(cd[o]) : group_codes<9>(cd[o]);
-      decode_group_dev<WIN>(smlo, smhi, z, t.tags >> (8 * o + 2 * g), pos[o], s.glob, w, bw, f[o]);
+      const u32 u = g == 0 ? code_bytes<0>(cd[o]) : g == 1 ? code_bytes<3>(cd[o]) : g == 2 ? code_bytes<6>(cd[o]) : code_bytes<9>(cd[o]);
+      if (WIN) decode_staged(smlo, smhi, u, seg[o][g >> 1], g & 1, w, bw, f[o]);
+      else decode_plain(smlo, smhi, u, seg[o][0] >> (2 * g), pos[o], s.glob, w, bw, f[o]);
     }
     if (DUMP) {
 #pragma unroll
       for (int o = 0; o < 2; o++)
         if (8 * o + r < nvalid) {
-          u32* row = reinterpret_cast<u32*>(dump + (8 * o + r) * D);
-          row[(32 * g + 2 * j) >> 1] = f[o][0]; row[(32 * g + 2 * j + 8) >> 1] = f[o][1];
-          row[(32 * g + 16 + 2 * j) >> 1] = f[o][2]; row[(32 * g + 16 + 2 * j + 8) >> 1] = f[o][3];
+          uint16_t* row = dump + (8 * o + r) * D + 32 * g + 2 * j;
+#pragma unroll
+          for (int i = 0; i < 4; i++) { uint16_t* e = row + (i & 1) + 8 * (i >> 1); e[0] = (uint16_t)(f[o][i] & 0xFFFFu); e[16] = (uint16_t)(f[o][i] >> 16); }
         }
     }
     mma16816(sc, f[0][0], f[1][0], f[0][1], f[1][1], Q.qa[2 * g][0], Q.qa[2 * g][1]);
@@ -296,42 +373,52 @@ __device__ __forceinline__ void k_decode(float* sc, const SideView& s, const Til
   sc[0] += s2[0]; sc[1] += s2[1]; sc[2] += s2[2]; sc[3] += s2[3];
 }
 template <bool DUMP>
-__device__ __forceinline__ void k_tile(float* sc, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const QFrag& Q, uint16_t* dump, int nvalid) {
-  if (t.win & 1) k_decode<true, DUMP>(sc, s, t, w, lane, Q, dump, nvalid);
-  else k_decode<false, DUMP>(sc, s, t, w, lane, Q, dump, nvalid);
+__device__ __forceinline__ void k_tile(float* sc, const SideView& s, int win, u32 area, const AttnView& w, int lane, const QFrag& Q, uint16_t* dump, int nvalid) {
+  if (win & 1) k_decode<true, DUMP>(sc, s, area, w, lane, Q, dump, nvalid);
+  else k_decode<false, DUMP>(sc, s, area, w, lane, Q, dump, nvalid);
 }
 
 // ---- value product of one compressed V tile
 template <bool WIN, bool DUMP, int NSET>
-__device__ __forceinline__ void v_decode(WarpAcc<NSET>& A, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const PFrag<NSET>& P, uint16_t* dump, int nvalid) {
+__device__ __forceinline__ void v_decode(WarpAcc<NSET>& A, const SideView& s, u32 area, const AttnView& w, int lane, const PFrag<NSET>& P, uint16_t* dump, int nvalid) {
   const int j = lane & 3, r = lane >> 2;
-  const u32 from = WIN ? s.esc - w.zero : 0u;
-  u32 pos[4] = {(t.v[0] & 0xFFFFu) + from, (t.v[0] >> 16) + from, (t.v[1] & 0xFFFFu) + from, (t.v[1] >> 16) + from};
+  u32 seg[4], pos[4] = {0u, 0u, 0u, 0u};               // staged: the words of the lane's two groups of each token;  not staged: their tags and the position
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const u32 row = area + SEG_V + 32u * slot_token(j, i);
+    if (WIN) seg[i] = lds_u32(row + 4u * r);
+    else {
+      const u32 v = lds_u32(row + 8u * (r >> 1)), tg = v & 0xFFu;
+      seg[i] = r & 1 ? tg >> 4 : tg; pos[i] = (v >> 16) + (r & 1 ? seg_esc(tg & 15u) : 0u);
+    }
+  }
+  const int swap = j >> 1;
   uint4 sm[4]; u32 cd[6];
 #pragma unroll
-  for (int i = 0; i < 4; i++) sm[i] = *reinterpret_cast<const uint4*>(s.sm + 64 * lane + 16 * i);
-  {
-    const uint2* c2 = reinterpret_cast<const uint2*>(s.cd + 24 * lane);
-    const uint2 ca = c2[0], cb = c2[1], cc = c2[2];
-    cd[0] = ca.x; cd[1] = ca.y; cd[2] = cb.x; cd[3] = cb.y; cd[4] = cc.x; cd[5] = cc.y;
-  }
+  for (int i = 0; i < 4; i++) sm[i] = *reinterpret_cast<const uint4*>(s.sm + 64 * lane + 16 * (i & 1) + 32 * ((i >> 1) ^ swap));
+#pragma unroll
+  for (int i = 0; i < 6; i++) cd[i] = *reinterpret_cast<const u32*>(s.cd + 24 * lane + 4 * (i % 3) + 12 * ((i / 3) ^ swap));
 #pragma unroll
   for (int g = 0; g < 2; g++) {
     const u32x4 bw = lds_u128(w.bases + BASES_V + 32 * r + 16 * g);
     u32 f[4][4];
-    decode_group_dev<WIN>(g ? sm[0].z : sm[0].x, g ? sm[0].w : sm[0].y, g ? group_codes<3>(cd) : group_codes<0>(cd), t.tags >> (16 + 2 * g), pos[0], s.glob, w, bw, f[0]);
-    decode_group_dev<WIN>(g ? sm[1].z : sm[1].x, g ? sm[1].w : sm[1].y, g ? group_codes<9>(cd) : group_codes<6>(cd), t.tags >> (20 + 2 * g), pos[1], s.glob, w, bw, f[1]);
-    decode_group_dev<WIN>(g ? sm[2].z : sm[2].x, g ? sm[2].w : sm[2].y, g ? group_codes<15>(cd) : group_codes<12>(cd), t.tags >> (24 + 2 * g), pos[2], s.glob, w, bw, f[2]);
-    decode_group_dev<WIN>(g ? sm[3].z : sm[3].x, g ? sm[3].w : sm[3].y, g ? group_codes<21>(cd) : group_codes<18>(cd), t.tags >> (28 + 2 * g), pos[3], s.glob, w, bw, f[3]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const u32 lo = g ? sm[i].z : sm[i].x, hi = g ? sm[i].w : sm[i].y;
+      const u32 u = i == 0 ? (g ? code_bytes<3>(cd) : code_bytes<0>(cd)) : i == 1 ? (g ? code_bytes<9>(cd) : code_bytes<6>(cd)) :
+                    i == 2 ? (g ? code_bytes<15>(cd) : code_bytes<12>(cd)) : (g ? code_bytes<21>(cd) : code_bytes<18>(cd));
+      if (WIN) decode_staged(lo, hi, u, seg[i], g, w, bw, f[i]);
+      else decode_plain(lo, hi, u, seg[i] >> (2 * g), pos[i], s.glob, w, bw, f[i]);
+    }
     if (DUMP) {
 #pragma unroll
       for (int i = 0; i < 4; i++) {
-        const int tok = 2 * j + (i & 1) + 8 * (i >> 1);
+        const int tok = slot_token(j, i);
         if (tok < nvalid) {
 #pragma unroll
-          for (int q = 0; q < 4; q++) {                // word q = stored positions 16r + 8g + 2q, +1  <->  channels 8(8g + 2q) + r, 8(8g + 2q + 1) + r
-            dump[tok * D + 8 * (8 * g + 2 * q) + r] = (uint16_t)(f[i][q] & 0xFFFFu);
-            dump[tok * D + 8 * (8 * g + 2 * q + 1) + r] = (uint16_t)(f[i][q] >> 16);
+          for (int q = 0; q < 4; q++) {                // word q = stored positions 16r + 8g + q, + 4  <->  channels 8(8g + q) + r, 8(8g + q + 4) + r
+            dump[tok * D + 8 * (8 * g + q) + r] = (uint16_t)(f[i][q] & 0xFFFFu);
+            dump[tok * D + 8 * (8 * g + q + 4) + r] = (uint16_t)(f[i][q] >> 16);
           }
         }
       }
@@ -345,9 +432,9 @@ __device__ __forceinline__ void v_decode(WarpAcc<NSET>& A, const SideView& s, co
   }
 }
 template <bool DUMP, int NSET>
-__device__ __forceinline__ void v_tile(WarpAcc<NSET>& A, const SideView& s, const TilePlan& t, const WarpView& w, int lane, const PFrag<NSET>& P, uint16_t* dump, int nvalid) {
-  if (t.win & 2) v_decode<true, DUMP, NSET>(A, s, t, w, lane, P, dump, nvalid);
-  else v_decode<false, DUMP, NSET>(A, s, t, w, lane, P, dump, nvalid);
+__device__ __forceinline__ void v_tile(WarpAcc<NSET>& A, const SideView& s, int win, u32 area, const AttnView& w, int lane, const PFrag<NSET>& P, uint16_t* dump, int nvalid) {
+  if (win & 2) v_decode<true, DUMP, NSET>(A, s, area, w, lane, P, dump, nvalid);
+  else v_decode<false, DUMP, NSET>(A, s, area, w, lane, P, dump, nvalid);
 }
 
 // ---- raw BF16 tiles [16][128] in global memory (rows >= nvalid are not read): the slot layout's tail, the paged layout's filling block
@@ -357,15 +444,17 @@ __device__ __forceinline__ void raw_scores(float* sc, const uint16_t* kraw, int 
   const int j = lane & 3, r = lane >> 2;
 #pragma unroll
   for (int s = 0; s < 8; s++) {
-    const uint16_t* k0 = kraw + r * D + 16 * s + 2 * j;
-    const uint16_t* k8 = k0 + 8 * D;
-    const u32 a0 = r < nvalid ? *reinterpret_cast<const u32*>(k0) : 0u, a2 = r < nvalid ? *reinterpret_cast<const u32*>(k0 + 8) : 0u;
-    const u32 a1 = r + 8 < nvalid ? *reinterpret_cast<const u32*>(k8) : 0u, a3 = r + 8 < nvalid ? *reinterpret_cast<const u32*>(k8 + 8) : 0u;
-    if (DUMP) {
-      if (r < nvalid) { u32* row = reinterpret_cast<u32*>(dump + r * D); row[(16 * s + 2 * j) >> 1] = a0; row[(16 * s + 2 * j + 8) >> 1] = a2; }
-      if (r + 8 < nvalid) { u32* row = reinterpret_cast<u32*>(dump + (r + 8) * D); row[(16 * s + 2 * j) >> 1] = a1; row[(16 * s + 2 * j + 8) >> 1] = a3; }
+    u32 x[2][2];                                       // [row half][16 channels on]
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      const int at = (8 * o + r) * D + 32 * (s >> 1) + 2 * j + 8 * (s & 1);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        x[o][i] = 8 * o + r < nvalid ? *reinterpret_cast<const u32*>(kraw + at + 16 * i) : 0u;
+        if (DUMP && 8 * o + r < nvalid) *reinterpret_cast<u32*>(dump + at + 16 * i) = x[o][i];
+      }
     }
-    mma16816(sc, a0, a1, a2, a3, Q.qa[s][0], Q.qa[s][1]);
+    mma16816(sc, prmt(x[0][0], x[0][1], 0x5410), prmt(x[1][0], x[1][1], 0x5410), prmt(x[0][0], x[0][1], 0x7632), prmt(x[1][0], x[1][1], 0x7632), Q.qa[s][0], Q.qa[s][1]);
   }
 }
 template <bool DUMP, int NSET>
@@ -376,15 +465,16 @@ __device__ __forceinline__ void raw_accum(WarpAcc<NSET>& A, const uint16_t* vraw
     u32 w0[4], w1[4];
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-      const int tok = 2 * j + (t & 1) + 8 * (t >> 1);
-      const uint16_t* vr = vraw + tok * D + 8 * (4 * mt) + r;
+      const int tok = slot_token(j, t);
       const bool ok = tok < nvalid;
-      const u32 e0 = ok ? vr[0] : 0u, e1 = ok ? vr[8] : 0u, e2 = ok ? vr[16] : 0u, e3 = ok ? vr[24] : 0u;
-      w0[t] = e0 | (e1 << 16); w1[t] = e2 | (e3 << 16);
-      if (DUMP && ok) {
-        uint16_t* o = dump + tok * D + 8 * (4 * mt) + r;
-        o[0] = (uint16_t)e0; o[8] = (uint16_t)e1; o[16] = (uint16_t)e2; o[24] = (uint16_t)e3;
+      u32 e[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const int at = tok * D + 8 * acc_channel(mt, c) + r;
+        e[c] = ok ? vraw[at] : 0u;
+        if (DUMP && ok) dump[at] = (uint16_t)e[c];
       }
+      w0[t] = e[0] | (e[1] << 16); w1[t] = e[2] | (e[3] << 16);
     }
     pv_words(A, mt, w0, w1, P);
   }

@@ -1,5 +1,5 @@
-// Device pieces that the encoder, the decoder and the attention kernels share: where a lane's escape bytes lie, and where the rebuild of a group gets
-// its addends from.  The arithmetic itself is in gaac_tile.h.
+// Device pieces that the encoder and the decoder share: where a lane's escape bytes lie, and where the rebuild of a group gets its addends from; loads and
+// stores of shared memory.  The arithmetic itself is in gaac_tile.h.
 #pragma once
 #include <cuda_runtime.h>
 #include "gaac_tile.h"
@@ -12,7 +12,7 @@ constexpr unsigned FULLM = 0xffffffffu;
 __device__ __forceinline__ void scan_step(u32& v, int d) {
   asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
 }
-// ---- escape positions of a lane's segments inside the tile side, for K, for V or (the attention kernels) for both in step.
+// ---- escape positions of a lane's segments inside the tile side.
 // K: the lanes of an octet are in the order of the tile's escape bytes, so ONE warp scan over both octets' segment sizes (packed in a word) gives
 //    every lane its two positions (kpos, low and high half).  k0, k1: tags of the lane's four groups in each octet (8 bits).
 // V: a scan over the lanes of equal j (one byte per token: a row has at most 80 escape bytes) places a lane inside its four rows, then a scan
@@ -48,43 +48,27 @@ __device__ __forceinline__ void tile_positions(u32 k0, u32 k1, u32 v0, u32 v1, u
 // ---- group decoder
 constexpr int LUTX_BYTES = 2048, BASES_V = 256, BASES_BYTES = 512;      // escape-byte table; base words of K, of V behind them
 
-// What does not change from tile to tile, as shared-memory addresses: the escape-byte table, the base words (K, then V), a zero byte, the warp's
-// scratch.
-struct WarpView { u32 lutx, bases, zero, scratch; };
+// Shared-memory addresses of the escape-byte table and of the base words (K, then V).
+struct WarpView { u32 lutx, bases; };
 
 __device__ __forceinline__ u32 lds_u8(u32 a) { u32 v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
-__device__ __forceinline__ u32 lds_u16(u32 a) { u32 v; asm volatile("{\n .reg .u16 t;\n ld.shared.u16 t, [%1];\n cvt.u32.u16 %0, t;\n}" : "=r"(v) : "r"(a)); return v; }
 __device__ __forceinline__ u32 lds_u32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
 __device__ __forceinline__ u32x2 lds_u64(u32 a) { u32x2 v; asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a)); return v; }
 __device__ __forceinline__ u32x4 lds_u128(u32 a) { u32x4 v; asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a)); return v; }
 __device__ __forceinline__ void sts_u8(u32 a, u32 v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts_u16(u32 a, u32 v) { asm volatile("{\n .reg .u16 t;\n cvt.u16.u32 t, %1;\n st.shared.u16 [%0], t;\n}" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts_u64(u32 a, u32 x, u32 y) { asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
 __device__ __forceinline__ void sts_u128(u32 a, u32 x, u32 y, u32 z, u32 w) { asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory"); }
-// Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, pos =
-// position of the group's escape bytes, advanced past them.
-// WIN: the escape bytes are staged; pos counts from the zero byte (a group without an escape byte reads that), and raw groups were turned
-//   into patch-table entries by build_raw_patches, which also left each entry's number in the first payload byte of its group: the addends
-//   of EVERY group come from one load, out of the escape-byte table (byte = the 4-bit-window escape byte, or the zero byte) or out of the
-//   patch table (byte = entry number), chosen by address arithmetic, and the decoder has no branch (a branch per group cost 13 % of the
-//   kernel although 0.75 % of the groups took it).
-// !WIN (tiles whose escape bytes are not all staged, or with more raw groups than the patch table holds): plain loads at glob[pos].
-template <bool WIN>
+// Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, pos = position of
+// the group's escape bytes, advanced past them.
 __device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& pos, const uint8_t* glob, const WarpView& w, const u32x4& bw, u32 out[4]) {
   const u32 m1 = tg & 1u;                             // promoted (tags are 0, 1 or 3)
-  u32x2 x;
-  if (WIN) {
-    const u32 r2 = tg & 2u;                           // 2 for a raw group: its table is the patch table
-    const u32 xe = lds_u8(mad(m1, pos, w.zero));
-    x = lds_u64(mad_k<8u>(xe, mad(r2, (w.scratch - w.lutx) >> 1, w.lutx)));
-    pos = mad_k<2u>(r2, pos);                         // a raw payload is five bytes: four here, one below with every promoted group
-  } else {
-    x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
-    if (tg & 2u) {
-      const uint8_t* p = glob + pos;
-      const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-      x = raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
-      pos += 4;
-    }
+  u32x2 x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
+  if (tg & 2u) {
+    const uint8_t* p = glob + pos;
+    const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+    x = raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
+    pos += 4;
   }
   pos += m1;
   rebuild_group(sm_lo, sm_hi, z, m1, bw, x, out);

@@ -81,6 +81,14 @@ GAAC_HD u32 mad(u32 a, u32 b, u32 c) {
   return a * b + c;
 #endif
 }
+// (a >> S) + c
+template <int S> GAAC_HD u32 mad_shr(u32 a, u32 c) {
+#if defined(__CUDA_ARCH__)
+  u32 d; asm("mad.hi.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "n"(1u << (32 - S)), "r"(c)); return d;
+#else
+  return (a >> S) + c;
+#endif
+}
 
 // ---- tags -> escape byte counts --------------------------------------------------------------------------------
 // escape bytes of a row with tag word fl (tier 1 -> 1 byte, tier 2 -> 5 bytes)                  gaac/kernel.py:46

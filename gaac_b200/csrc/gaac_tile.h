@@ -71,4 +71,68 @@ GAAC_HD void rebuild_group(u32 sm_lo, u32 sm_hi, u32 z, u32 m1, const u32x4& bw,
   bf16x4(sm_hi, mad_k<31u>(xh & 0x00380038u, xh) + bhi + x.y, out[2], out[3]);
 }
 
+// ---- decode, the form of the attention kernels.  A rebuilt word there may hold any two elements of a group, as long as the other operand of the matrix product
+// has the same two, so the codes go into bytes in two steps for the whole group ({0, 1}, {2, 3}, {4, 5}, {6, 7}: code_bytes), the exponents are made in two
+// words, of the even and of the odd elements, and a word pairs elements that lie four apart: bytes 0 and 2 of a word of exponents land on the exponent fields
+// of a bf16 pair when it is shifted up by 7, bytes 1 and 3 when it is shifted down by 1, whatever else the shift brings along is covered by the sign and
+// mantissa bits, and those come from one byte permute.  
+// The codes of a group, two to a byte (B = byte offset of the group in the lane's code string)
+template <int B> GAAC_HD u32 code_bytes(const u32* cd) {
+  constexpr int i = B & 3;
+  u32 t;                                                                 // codes 0..3 at bits 0..11, 4..7 at bits 16..27
+  if (i == 1) { const u32 z = cd[B >> 2] >> 8; t = mad_k<15u>(z & 0xFFF000u, z); }
+  else {
+    const u32 z = i ? prmt(cd[B >> 2], cd[(B >> 2) + (i ? 1 : 0)], i == 2 ? 0x5432 : 0x6543) : cd[B >> 2];      // the upper byte is the next group's
+    t = mad_k<16u>(z & 0xFFF000u, z & 0xFFFu);
+  }
+  return mad_k<3u>(t & 0x0FC00FC0u, t);
+}
+// Words of the bases {3-bit window: even elements, odd elements; what the 4-bit window is above them: even, odd} of group t of a side's 16 (K: 4 * (lane & 3)
+// + group, V: 2 * (lane >> 2) + group)
+template <bool VSIDE> GAAC_HD u32x4 pair_base_words(const uint8_t* row3, const uint8_t* row4, int t) {
+  const u32 a3 = half_group_word<VSIDE>(row3, 2 * t), b3 = half_group_word<VSIDE>(row3, 2 * t + 1), a4 = half_group_word<VSIDE>(row4, 2 * t), b4 = half_group_word<VSIDE>(row4, 2 * t + 1);
+  const u32 e3 = prmt(a3, b3, 0x6420), o3 = prmt(a3, b3, 0x7531);
+  return u32x4{e3, o3, prmt(a4, b4, 0x6420) - e3, prmt(a4, b4, 0x7531) - o3};
+}
+// What an escape byte adds to the exponents of its group: 8 in byte k for bit 2k (even elements) and for bit 2k + 1 (odd ones)
+GAAC_HD u32x2 pair_addends(u32 b) {
+  const u32 lo = spread_bit4(b & 15u), hi = spread_bit4(b >> 4);
+  return u32x2{prmt(lo, hi, 0x6420), prmt(lo, hi, 0x7531)};
+}
+// The same for a raw group, whose payload (8 x 5 bits) lies in (w1:w0) from bit sh (0, 8, 16, 24): the upper five bits of the exponents.  No base must contribute:
+// the caller takes off what rebuild_pairs adds.
+GAAC_HD u32x2 pair_raw_addends(u32 w0, u32 w1, u32 sh) {
+  const u32 lo = funnel_r(w0, w1, (int)sh), hi = sh == 24u ? w1 : funnel_r(w0, w1, (int)sh + 8);           // payload bits 0..31 and 8..39
+  const u32 ev = bits_of(bits_of(lo << 3, lo << 1, 0xFFu), bits_of(hi << 5, lo >> 1, 0xFF000000u), 0xFFFFu);
+  const u32 od = bits_of(bits_of(lo >> 2, lo >> 4, 0xFFu), bits_of(hi, lo >> 6, 0xFF000000u), 0xFFFFu);
+  return u32x2{ev & 0xF8F8F8F8u, od & 0xF8F8F8F8u};
+}
+// out[i] = elements i and i + 4.  u: code_bytes; m: what the bases' second half counts (1 for a promoted group); x: the addends.
+GAAC_HD void rebuild_pairs(u32 sm_lo, u32 sm_hi, u32 u, u32 m, const u32x4& bw, const u32x2& x, u32 out[4]) {
+  const u32 ev = (u & 0x07070707u) + mad(m, bw.z, bw.x) + x.x, od = mad_shr<3>(u & 0x38383838u, mad(m, bw.w, bw.y)) + x.y;
+  out[0] = bits_of(prmt(sm_lo, sm_hi, 0x4400), mad_k<128u>(ev, 0u), 0x807F807Fu);
+  out[1] = bits_of(prmt(sm_lo, sm_hi, 0x5511), mad_k<128u>(od, 0u), 0x807F807Fu);
+  out[2] = bits_of(prmt(sm_lo, sm_hi, 0x6622), ev >> 1, 0x807F807Fu);
+  out[3] = bits_of(prmt(sm_lo, sm_hi, 0x7733), od >> 1, 0x807F807Fu);
+}
+// ---- escape bytes of four neighbouring groups of a row (a segment), by its tag byte t.  Segment words hold a 16-bit index per group: NO_ESC for a group without
+// escape byte, 256 + byte for a promoted one; entry `index` of the addend table is what to add, index >> 8 the m of rebuild_pairs.  {x: two selectors of 16
+// bits that pick the indexes of groups 0, 1 and of groups 2, 3 out of the segment's first four escape bytes and SEG_CONST; y: escape bytes of the segment}.
+// The selectors are right for the groups up to the segment's first raw one; raw_items are the others.
+constexpr u32 NO_ESC = 255u, SEG_CONST = 0x000100FFu;
+GAAC_HD u32x2 segment_entry(u32 t) {
+  u32 sel = 0u, at = 0u;
+  for (int g = 0; g < 4; g++) {
+    const u32 tag = (t >> (2 * g)) & 3u;
+    sel |= (tag & 1u ? 0x60u | at : 0x54u) << (8 * g);
+    at += tag & 1u;
+  }
+  return u32x2{sel, seg_esc(t)};
+}
+// Groups of a row with tag word fl that the selectors leave out: the raw ones and the promoted ones behind a raw one of their segment, at their lower tag bits.
+GAAC_HD u32 raw_items(u32 fl) {
+  const u32 r = (fl >> 1) & 0x55555555u;
+  return (r | (mad_k<4u>(r & 0x15151515u, 0u) | mad_k<16u>(r & 0x05050505u, 0u) | mad_k<64u>(r & 0x01010101u, 0u))) & fl;
+}
+
 }  // namespace gaac

@@ -232,7 +232,7 @@ template <int KIND_V>
 __device__ __forceinline__ WarpView fill_decode_tables(DecodeTables& t, const uint8_t* b3row, const uint8_t* b4row) {
   for (int i = threadIdx.x; i < 256; i += blockDim.x) fill_lutx(t.lutx, i);
   if (threadIdx.x < 32) fill_bases<KIND_V != 0>(t.bases, b3row, b4row, threadIdx.x);
-  return WarpView{(u32)__cvta_generic_to_shared(t.lutx), (u32)__cvta_generic_to_shared(t.bases), 0u, 0u};
+  return WarpView{(u32)__cvta_generic_to_shared(t.lutx), (u32)__cvta_generic_to_shared(t.bases)};
 }
 template <bool TRANS> __device__ __forceinline__ void store_matrices(u32 at, int s, u32 w0, u32 w1, u32 w2, u32 w3) {       // the opposite of load_matrices
   if (!TRANS) asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(at + 32 * s), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
@@ -245,8 +245,8 @@ __device__ __forceinline__ void load_32(u32* w, const void* p) {
 
 // Rebuild a compressed tile into ws.xs (natural channel order, bf16 bits).  sm / cd / fl: tile-relative sources in global memory; esc: the tile's first
 // escape byte in global memory.  Everything but the escape bytes is asked for at once; those are fetched with one coalesced load as soon as the tags
-// say how many there are (a load per group waited for the one before it at every raw group's branch).  The group decoder is the attention
-// kernels'; the fragments go to shared memory by stmatrix.
+// say how many there are (a load per group waited for the one before it at every raw group's branch).  The fragments go to shared
+// memory by stmatrix.
 template <int KIND_V>
 __device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, const uint8_t* sm_src, const uint8_t* cd_src, const uint8_t* fl_src, const uint8_t* esc_src,
                                                  const WarpView& w, int lane) {
@@ -306,7 +306,7 @@ __device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, const uint8_
       const int b = 3 * (PER * i + g);               // byte of the group's codes in the lane's 24
       const u32 z = b == 0 ? group_codes<0>(cd) : b == 3 ? group_codes<3>(cd) : b == 6 ? group_codes<6>(cd) : b == 9 ? group_codes<9>(cd) :
                     b == 12 ? group_codes<12>(cd) : b == 15 ? group_codes<15>(cd) : b == 18 ? group_codes<18>(cd) : group_codes<21>(cd);
-      decode_group_dev<false>(sm[2 * (PER * i + g)], sm[2 * (PER * i + g) + 1], z, tags >> (2 * (PER * i + g)), pos[i], esc, w, bw, f[i]);
+      decode_group_dev(sm[2 * (PER * i + g)], sm[2 * (PER * i + g) + 1], z, tags >> (2 * (PER * i + g)), pos[i], esc, w, bw, f[i]);
     }
     if (!KIND_V) {
 #pragma unroll

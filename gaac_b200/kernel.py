@@ -45,8 +45,7 @@ def choose_nsplit(B: int, n_kv: int, S: int, target_ctas: int = 96, min_tok: int
 @functools.lru_cache(maxsize=4096)
 def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200, min_tiles_per_warp: int = 2, ragged: bool = False,
                         total_tokens: int | None = None) -> int:
-    """Splits per (row, kv head) for a B200.  The kernel runs one 16-warp CTA per SM; a CTA keeps the metadata of the first
-    META_TILES (1024) tiles of its range in shared memory and fetches the rest from global memory inside the loop.
+    """Splits per (row, kv head) for a B200.  The kernel runs one 16-warp CTA per SM.
 
     Equal lengths (S is every row's length): the split count minimises a cost model fitted to measurements,
         waves x ((tiles per warp + 0.5) x tile time + per-CTA fixed cost),   waves = ceil(rows x splits / SMs),

@@ -128,3 +128,60 @@ extern "C" void emu_decode_tile_lut(int kind_v, const uint8_t* sm_in, const uint
                                     const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
   decode_tile<true>(kind_v, sm_in, cd_in, fl_in, esc_in, b3row, b4row, out);
 }
+
+// Rebuild as the attention kernels do it: the tile's segments (four groups of a row) are expanded into indexes of the addend table, a raw group's index is that
+// of an entry of its own behind the table, and a word pairs elements that lie four apart.  first_patch: index of the first such entry.
+extern "C" int emu_decode_tile_pairs(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in,
+                                     const uint8_t* b3row, const uint8_t* b4row, int first_patch, uint16_t* out) {
+  static u32x2 addends[65536];
+  addends[NO_ESC] = u32x2{0u, 0u};
+  for (u32 b = 0; b < 256; b++) addends[256 + b] = pair_addends(b);
+  u32x4 base[16];
+  for (int t = 0; t < 16; t++) base[t] = kind_v ? pair_base_words<true>(b3row, b4row, t) : pair_base_words<false>(b3row, b4row, t);
+  u32 words[16][4][2];                               // segment words of row, quarter
+  int raws = 0;
+  for (int row = 0; row < 16; row++)
+    for (int q = 0; q < 4; q++) {
+      const u32 t = (fl_in[row] >> (8 * q)) & 0xFFu;
+      const u32x2 e = segment_entry(t);
+      const uint8_t* p = esc_in + esc_at(fl_in, row, 4 * q);
+      if (e.y != seg_esc(t)) return -1;
+      const u32 four = (u32)p[0] | (u32)p[1] << 8 | (u32)p[2] << 16 | (u32)p[3] << 24;
+      u32 (&w)[2] = words[row][q];
+      w[0] = prmt(four, SEG_CONST, e.x & 0xFFFFu); w[1] = prmt(four, SEG_CONST, e.x >> 16);
+      const u32 items = (raw_items(fl_in[row]) >> (8 * q)) & 0xFFu;
+      for (int g = 0; g < 4; g++)
+        if ((items >> (2 * g)) & 1u) {
+          const uint8_t* pl = p + seg_esc(t & ((1u << (2 * g)) - 1u));
+          u32 index = 256u + *pl;
+          if ((t >> (2 * g)) & 2u) {
+            const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(pl) & ~(uintptr_t)3);
+            u32x2 x = pair_raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(pl) & 3));
+            index = (u32)(first_patch + raws++);
+            const u32 m = index >> 8;
+            const u32x4& bw = base[4 * q + g];
+            addends[index] = u32x2{x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w};
+          }
+          w[g >> 1] = prmt(w[g >> 1], index, g & 1 ? 0x5410u : 0x3254u);
+        }
+    }
+  const int SEGS = kind_v ? 4 : 2, PER = 8 / SEGS;
+  for (int lane = 0; lane < 32; lane++) {
+    const int j = lane & 3, r = lane >> 2;
+    u32 sm[16], cd[6];
+    if (!kind_v) for (int o = 0; o < 2; o++) { memcpy(sm + 8 * o, sm_in + o * 1024 + 32 * lane, 32); memcpy(cd + 3 * o, cd_in + o * 384 + 12 * lane, 12); }
+    else { memcpy(sm, sm_in + 64 * lane, 64); memcpy(cd, cd_in + 24 * lane, 24); }
+    const u32 u[8] = {code_bytes<0>(cd), code_bytes<3>(cd), code_bytes<6>(cd), code_bytes<9>(cd), code_bytes<12>(cd), code_bytes<15>(cd), code_bytes<18>(cd), code_bytes<21>(cd)};
+    for (int idx = 0; idx < 8; idx++) {
+      const int s = idx / PER, g = idx % PER, row = kind_v ? v_tok(j, s) : 8 * s + r, group = (kind_v ? 2 * r : 4 * j) + g;
+      const u32 word = words[row][group >> 2][(group >> 1) & 1], index = group & 1 ? word >> 16 : word & 0xFFFFu;
+      u32 f[4];
+      rebuild_pairs(sm[2 * idx], sm[2 * idx + 1], u[idx], index >> 8, base[group], addends[index], f);
+      for (int q = 0; q < 4; q++) {                  // elements q and q + 4 of the group
+        const int c = kind_v ? 8 * (8 * g + q) + r : 32 * g + 2 * j + (q & 1) + 8 * (q >> 1);
+        out[128 * row + c] = (uint16_t)f[q]; out[128 * row + c + (kind_v ? 32 : 16)] = (uint16_t)(f[q] >> 16);
+      }
+    }
+  }
+  return raws;
+}

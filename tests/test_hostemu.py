@@ -47,3 +47,26 @@ def test_tile_encode_decode_matches_oracle(emu, trial):
         out2 = np.zeros((16, 128), np.uint16)
         emu.emu_decode_tile_lut(trial % 2, P(sm), P(cd), P(fl), ctypes.c_void_p(buf.ctypes.data + base), P(b3), P(b4), P(out2))
         assert np.array_equal(out2[:nvalid], x[0, :nvalid]), shift
+
+
+@pytest.mark.parametrize("trial", range(16))
+def test_tile_decode_in_pairs_matches_oracle(emu, trial):
+    """The attention kernels' rebuild: no escapes to all groups raw, raw entries at small and large indexes of the addend table."""
+    kind = "kv"[trial % 2]
+    rng = np.random.default_rng(100 + trial)
+    gen = [dict(raw_frac=0.0, four_frac=0.0), dict(raw_frac=0.01, four_frac=0.2), dict(raw_frac=0.3, four_frac=0.3), dict(raw_frac=0.0, four_frac=1.0)][trial // 2 % 4]
+    x = O.synth_kv(kind, 1, 16, trial, **gen) if trial < 12 else rng.integers(0, 65536, (1, 16, 128)).astype(np.uint16)
+    b3, b4 = O.calibrate(O.synth_kv(kind, 1, 512, trial), 1)
+    if trial % 4 == 3:
+        b3 = rng.integers(0, 249, (1, 128)).astype(np.uint8); b4 = rng.integers(0, 241, (1, 128)).astype(np.uint8)
+    pg = O.encode(x, b3, b4, kind, 1)
+    fl = np.ascontiguousarray(pg["flags"][0]).view(np.uint32)
+    for shift, first in ((0, 512), (1, 600), (2, 8000), (3, 65000)):
+        buf = np.zeros(1288 + 32, np.uint8)
+        base = (-buf.ctypes.data) % 4 + shift
+        buf[base:base + pg["ovf"].size] = pg["ovf"]
+        out = np.zeros((16, 128), np.uint16)
+        raws = emu.emu_decode_tile_pairs(trial % 2, P(np.ascontiguousarray(pg["sm"][0])), P(np.ascontiguousarray(pg["codes"][0])), P(fl), ctypes.c_void_p(buf.ctypes.data + base),
+                                         P(b3), P(b4), first, P(out))
+        assert raws == sum(bin(int(f) & 0xAAAAAAAA).count("1") for f in fl)
+        assert np.array_equal(out, x[0]), (shift, first)
