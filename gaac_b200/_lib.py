@@ -120,5 +120,17 @@ def ptr(t):
 
 
 def stream_ptr(device=None):
+    """The current stream of a device.  torch.cuda.current_stream makes a Stream object, 2.3 us of the ten or so that a call of this package costs; the function
+    underneath it takes 0.1 us."""
+    index = getattr(device, "index", None)
+    if index is not None and device.type == "cuda":
+        return _raw_stream(index)
     import torch
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def _raw_stream(index):
+    global _raw_stream
+    import torch
+    _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+    return _raw_stream(index)

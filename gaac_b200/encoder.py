@@ -143,18 +143,18 @@ class TileEncoder:
         if H == 0 or ntiles == 0:
             return Page(sm, cd, flags, ovf_off, torch.zeros(8, dtype=torch.uint8, device=dev), torch.zeros(H + 1, dtype=torch.int32, device=dev),
                         torch.zeros(H, ntiles, dtype=torch.int32, device=dev), codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
-        meta = torch.empty(H * ntiles + H + 1, dtype=torch.int32, device=dev)                     # tile offsets | head_start [H+1]
-        tile_off, head_start = meta[:H * ntiles].view(H, ntiles), meta[H * ntiles:]
+        tile_off = torch.empty(H, ntiles, dtype=torch.int32, device=dev)
+        head_start = torch.empty(H + 1, dtype=torch.int32, device=dev)
         x = x.contiguous()
-        slots = self._scratch(H * ntiles * SLOT, dev)
-        work = torch.empty(H * ntiles + H, dtype=torch.int32, device=dev)                         # tile sizes | head sizes
+        items = H * ntiles
+        slots = self._scratch(items * SLOT + 4 * (items + H), dev)                                # escape slots | tile sizes | head sizes
         total = torch.empty(1, dtype=torch.int32, pin_memory=True)
         L = _lib.lib(); st = _lib.stream_ptr(dev)
-        p_flags, p_slots, p_work, p_meta = flags.data_ptr(), slots.data_ptr(), work.data_ptr(), meta.data_ptr()
-        p_hs = p_meta + 4 * H * ntiles
+        p_flags, p_slots, p_off, p_hs = flags.data_ptr(), slots.data_ptr(), tile_off.data_ptr(), head_start.data_ptr()
+        p_work = p_slots + items * SLOT
         _lib.check(L.gaac_encode_sized(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
-                                       sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_meta, p_work + 4 * H * ntiles, p_hs, total.data_ptr(), st), "gaac_encode_sized")
+                                       sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, total.data_ptr(), st), "gaac_encode_sized")
         ovf = torch.empty(total.item() + 8, dtype=torch.uint8, device=dev)
-        _lib.check(L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_meta, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, 0, 0, None, st),
+        _lib.check(L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, 0, 0, None, st),
                    "gaac_compact_copy")
         return Page(sm, cd, flags, ovf_off, ovf, head_start, tile_off, codec.base3, codec.base4, H, S, codec.n_kv, self.kind)

@@ -17,11 +17,17 @@ SM_COUNT_B200 = 148
 ATT_WARPS = 16  # warps per CTA of the CUDA kernel (one CTA per SM)
 
 
-def workspace(dev, B: int, n_q: int, nsplit: int) -> torch.Tensor:
+@functools.lru_cache(maxsize=4096)
+def _workspace_bytes(B: int, n_q: int, nsplit: int) -> int:
+    return _lib.lib().gaac_attn_workspace_bytes(B, n_q, nsplit)
+
+
+def workspace(dev, B: int, n_q: int, nsplit: int, stream: int | None = None) -> torch.Tensor:
     """The workspace of the current stream.  One that became too small is kept beside its successor: a captured CUDA graph may hold its address, and the
-    successor has at least twice its size, so all of them together stay below twice the largest."""
-    need = _lib.lib().gaac_attn_workspace_bytes(B, n_q, nsplit)
-    key = (torch.device(dev).index, torch.cuda.current_stream(dev).cuda_stream, B * n_q if B * n_q > 16320 else 0)
+    successor has at least twice its size, so all of them together stay below twice the largest.  stream: the current stream, where the caller knows it."""
+    need = _workspace_bytes(B, n_q, nsplit)
+    if not isinstance(dev, torch.device): dev = torch.device(dev)
+    key = (dev.index, _lib.stream_ptr(dev) if stream is None else stream, B * n_q if B * n_q > 16320 else 0)
     held = _WS.get(key)
     if held is None:
         held = _WS.setdefault(key, [])
@@ -143,28 +149,29 @@ class _Ext:
         has_tail = kt.numel() > 0
         K = _side(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None)
         V = _side(smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None)
-        ws = workspace(dev, B, n_q, -(-units // B) if units else nsplit)
+        stream = _lib.stream_ptr(dev)
+        ws = workspace(dev, B, n_q, -(-units // B) if units else nsplit, stream)
         L = _lib.lib()
         if units:
             out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
             _lib.check(L.gaac_decode_attn_balanced(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), units,
                                                    TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel(),
-                                                   out.data_ptr(), _lib.ptr(out_f32), _lib.stream_ptr(dev)), "gaac_decode_attn_balanced")
+                                                   out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_decode_attn_balanced")
             return out
         common = (K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), int(nsplit),
                   TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel())
         if exchange is not None and fused:
             out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
-            _lib.check(L.gaac_decode_attn_exchange(*common, exchange, out.data_ptr(), _lib.ptr(out_f32), _lib.stream_ptr(dev)), "gaac_decode_attn_exchange")
+            _lib.check(L.gaac_decode_attn_exchange(*common, exchange, out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_decode_attn_exchange")
             return out
         if exchange is not None:
-            _lib.check(L.gaac_decode_attn_push(*common, exchange, _lib.stream_ptr(dev)), "gaac_decode_attn_push")
+            _lib.check(L.gaac_decode_attn_push(*common, exchange, stream), "gaac_decode_attn_push")
             return None
         if partial is not None:
-            _lib.check(L.gaac_decode_attn_partial(*common, partial.data_ptr(), _lib.stream_ptr(dev)), "gaac_decode_attn_partial")
+            _lib.check(L.gaac_decode_attn_partial(*common, partial.data_ptr(), stream), "gaac_decode_attn_partial")
             return partial
         out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
-        _lib.check(L.gaac_decode_attn(*common, out.data_ptr(), _lib.ptr(out_f32), _lib.stream_ptr(dev)), "gaac_decode_attn")
+        _lib.check(L.gaac_decode_attn(*common, out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_decode_attn")
         return out
 
 
@@ -195,14 +202,15 @@ def attention(q, kp, vp, scale=None, nsplit=None, out_f32=None, out=None):
     G = n_q // max(1, n_kv)
     if not (1 <= G <= 8 and G * n_kv == n_q):
         raise RuntimeError("GQA group size must be 1..8")
-    dev = q.device
     if nsplit is None: nsplit = choose_nsplit_sm100(B, n_kv, kp.S)
     if out is None:
-        out = torch.empty(B * n_q, Dq, dtype=q.dtype, device=dev)
-    elif not (out.is_contiguous() and out.dtype == q.dtype and out.numel() == B * n_q * Dq):
+        out = torch.empty(B, n_q, Dq, dtype=q.dtype, device=q.device)
+    elif out.is_contiguous() and out.dtype == q.dtype and out.numel() == B * n_q * Dq:
+        out = out.view(B, n_q, Dq)
+    else:
         raise RuntimeError("out must be a contiguous bf16 tensor with B*n_q*128 elements")
     _pages_call(q, kp, vp, B, n_q, n_kv, scale, nsplit, out=out, out_f32=out_f32)
-    return out.view(B, n_q, Dq)
+    return out
 
 
 def _page_side(pg) -> _lib.Side:
@@ -225,13 +233,13 @@ def _pages_call(q, kp, vp, B, n_q, n_kv, scale, nsplit, out=None, out_f32=None, 
     which is all the identity slot map and the constant length table of the reference's entry point said
     (gaac/kernel.py:349-352); the kernel needs neither table."""
     dev = q.device
-    q2 = q.reshape(B * n_q, 128)
-    if not q2.is_contiguous(): q2 = q2.contiguous()
-    ws = workspace(dev, B, n_q, nsplit)
-    _lib.check(_lib.lib().gaac_decode_attn_pages(_page_side(kp), _page_side(vp), q2.data_ptr(), B, n_q, n_kv, kp.S, max(16, kp.sm.shape[1] // 128),
+    if not q.is_contiguous(): q = q.contiguous()
+    stream = _lib.stream_ptr(dev)
+    ws = workspace(dev, B, n_q, nsplit, stream)
+    _lib.check(_lib.lib().gaac_decode_attn_pages(_page_side(kp), _page_side(vp), q.data_ptr(), B, n_q, n_kv, kp.S, max(16, kp.sm.shape[1] // 128),
                                                  float(scale if scale is not None else 128 ** -0.5), int(nsplit), kp.base3.size(0),
                                                  ws.data_ptr(), ws.numel(), _lib.ptr(out), _lib.ptr(out_f32), _lib.ptr(part), exchange,
-                                                 1 if fused else 0, _lib.stream_ptr(dev)), "gaac_decode_attn_pages")
+                                                 1 if fused else 0, stream), "gaac_decode_attn_pages")
 
 
 def combine(pm: torch.Tensor, pl: torch.Tensor, pa: torch.Tensor, out_f32: torch.Tensor | None = None) -> torch.Tensor:

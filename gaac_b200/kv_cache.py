@@ -57,8 +57,8 @@ class _Store:
         self._set_escape_stream(wider.view(-1), ovf_cap)
 
     def c_store(self) -> _lib.Store:
-        p = lambda t: t.data_ptr()
-        return _lib.Store(p(self.sm), p(self.codes), p(self.flags), p(self.tile_off), p(self.ovf), p(self.ovf_used), p(self.tail), p(self.base3), p(self.base4))
+        return _lib.Store(self.sm.data_ptr(), self.codes.data_ptr(), self.flags.data_ptr(), self.tile_off.data_ptr(), self.ovf.data_ptr(), self.ovf_used.data_ptr(),
+                          self.tail.data_ptr(), self.base3.data_ptr(), self.base4.data_ptr())
 
 
 class CompressedKVCache:
@@ -122,18 +122,20 @@ class CompressedKVCache:
         L = k.shape[0]
         assert L <= self.cap, f"sequence of {L} tokens exceeds the cache capacity {self.cap}"
         assert 0 <= slot < self.n_slots
-        hs = self._heads(slot)
         k, v = self._token_rows(k), self._token_rows(v)
         if _lib.row_stride(k) != _lib.row_stride(v):                                               # the library reads both with one stride
             k, v = k.contiguous(), v.contiguous()
+        stores = self.k.c_store(), self.v.c_store()
         if self.per_sequence_bases and L:
             lib = _lib.lib()
             hist = torch.empty(lib.gaac_cache_calibrate_scratch_bytes(self.n_kv), dtype=torch.uint8, device=k.device)
-            _lib.check(lib.gaac_cache_calibrate(self.k.c_store(), self.v.c_store(), k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.k.base3.shape[0],
+            _lib.check(lib.gaac_cache_calibrate(*stores, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.k.base3.shape[0],
                                                 hist.data_ptr(), hist.numel(), _lib.stream_ptr(k.device)), "gaac_cache_calibrate")
         need = _lib.lib().gaac_cache_prefill_scratch_bytes(L, self.n_kv)
         if check:
-            self.settle_prefills()
+            if self._pending:
+                self.settle_prefills()
+                stores = None                                                                      # the escape streams may have moved
             if self._scratch is None or self._scratch.numel() < need:
                 self._scratch = torch.empty(need, dtype=torch.uint8, device=k.device)
             scratch, status = self._scratch, self._slot_status[slot]
@@ -143,8 +145,9 @@ class CompressedKVCache:
                 self._pending_bytes -= old[1].numel()
             if self._pending_bytes + need > self.pending_scratch_limit:
                 self.settle_prefills()
+                stores = None                                                                      # the escape streams may have moved
             scratch, status = torch.empty(need, dtype=torch.uint8, device=k.device), self._slot_status[slot]
-        self._prefill_launch(slot, L, k, v, scratch, status, copy_only=0)
+        self._prefill_launch(slot, L, k, v, scratch, status, copy_only=0, stores=stores)
         if not check:
             self._pending[slot] = (L, scratch)
             self._pending_bytes += need
@@ -157,9 +160,10 @@ class CompressedKVCache:
         if short_k or short_v:
             self._prefill_launch(slot, L, None, None, scratch, status, copy_only=1)
 
-    def _prefill_launch(self, slot, L, k, v, scratch, status, copy_only: int):
+    def _prefill_launch(self, slot, L, k, v, scratch, status, copy_only: int, stores=None):
         dev = self.S.device
-        _lib.check(_lib.lib().gaac_cache_prefill(self.k.c_store(), self.v.c_store(), _lib.ptr(k), _lib.ptr(v), L, _lib.row_stride(k) if k is not None else self.n_kv * D,
+        K, V = stores or (self.k.c_store(), self.v.c_store())
+        _lib.check(_lib.lib().gaac_cache_prefill(K, V, _lib.ptr(k), _lib.ptr(v), L, _lib.row_stride(k) if k is not None else self.n_kv * D,
                                                  slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(), self.cap, self.k.ovf_cap, self.k.base3.shape[0],
                                                  scratch.data_ptr(), scratch.numel(), status.data_ptr(), copy_only, _lib.stream_ptr(dev)), "gaac_cache_prefill")
 
@@ -171,7 +175,11 @@ class CompressedKVCache:
             return
         pending, self._pending, self._pending_bytes = self._pending, {}, 0
         slots = list(pending)
-        words = self._slot_status[torch.tensor(slots, dtype=torch.long, device=self.S.device)].tolist()
+        if self.n_slots <= 4096:                     # one copy of all words (18 us) costs less than uploading the slots' numbers and picking theirs out (38 us)
+            rows = self._slot_status.tolist()
+            words = [rows[slot] for slot in slots]
+        else:
+            words = self._slot_status[torch.tensor(slots, dtype=torch.long, device=self.S.device)].tolist()
         wanted = max(max(w[1], w[3]) for w in words) + TILE_MAX_ESC + _OVER_READ
         if wanted > self.k.ovf_cap:
             try:

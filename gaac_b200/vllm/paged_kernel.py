@@ -32,8 +32,9 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     elif nsplit is None: nsplit = choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), n_kv, TS, TS - 2880)
-    ws = workspace(q.device, B, n_q, nsplit)
+    stream = _lib.stream_ptr(q.device)
+    ws = workspace(q.device, B, n_q, nsplit, stream)
     launch = _lib.lib().gaac_paged_decode_attn_balanced if units else _lib.lib().gaac_paged_decode_attn
     _lib.check(launch(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), units or int(nsplit),
-                      ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), _lib.stream_ptr(q.device)), "gaac_paged_decode_attn")
+                      ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_paged_decode_attn")
     return out
