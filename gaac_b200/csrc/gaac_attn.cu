@@ -48,7 +48,7 @@ constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + BASES
 constexpr int ATT_SMEM = TB_RING + NSTG * STAGE_BYTES + 16;          // (an escape segment is read as whole words)
 static_assert(TB_BASES % 16 == 0 && TB_ESC % 16 == 0 && TB_AREA % 16 == 0 && TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
               "bulk copies need 16-byte aligned shared-memory destinations and sizes");
-static_assert(ATT_SMEM + 64 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
+static_assert(ATT_SMEM + 112 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
 static_assert(ATT_THREADS / 128 * 2 >= 8, "the fused exchange keeps at most two merged heads per thread");
 constexpr int ACC_LD = D + 8;                        // row stride of the staged accumulators: 8j + r banks, conflict-free stores
 
@@ -67,6 +67,7 @@ struct AttnParams {
   // balanced launches (units > 0; grid = (n_kv, units)): the rows share `units` ranges per kv head by their lengths, see row_share; nsplit is not used, a
   // unit of a kv head has one partial per query head, at (kvh * units + unit) * G
   int units, wave;                                  // wave: units of a kv head that run at a time
+  int flat;                                         // flat launches: CTAs (0: not one); nsplit is not used, see FlatWalk
   // cross-GPU exchange (x_recv == NULL: unused): the partial of every query head is stored into every rank's receive
   // buffer, then this rank's arrival flag of the (row, kv head) group on every rank is set to the exchange number; with
   // x_fused the same CTA then waits (bounded) for the other ranks' flags, merges all ranks' rows and writes the output
@@ -278,7 +279,7 @@ template <int N> __device__ __forceinline__ void merge_warps(const uint8_t* area
 // element 608; head_dim 256: finite 36.1 -> 36.5.  With the main loop's decoder in its place a second pass took a fifth of that, but finite data
 // 1 to 7 % more, inlined or called.
 template <bool PAGED, bool WIDE>
-__device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, int bh, int split, int NS) {
+__device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, int bh, int split, int NS, const int* range = nullptr) {
   int tid = threadIdx.x;
   asm volatile("" : "+r"(tid), "+r"(bh), "+r"(split), "+r"(NS));
   const int lane = tid & 31, warp = tid >> 5, b = bh / p.n_kv, kvh = bh % p.n_kv, hf = WIDE ? warp & 1 : 0, HALVES = WIDE ? 2 : 1;
@@ -290,7 +291,7 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
     S = sl < 0 ? 0 : p.seq_len ? p.seq_len[ch] : p.S_uniform;
     TL = sl >= 0 && p.tail_len && split == NS - 1 ? p.tail_len[ch] : 0;
   }
-  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS, tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo);
+  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS, tlo = range ? range[0] : min(split * chunk, ntiles), n = range ? range[1] : min(chunk, ntiles - tlo);
   float m[8], l[8], acc[8][4];
 #pragma unroll
   for (int h = 0; h < 8; h++) { m[h] = -CUDART_INF_F; l[h] = acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.f; }
@@ -373,11 +374,68 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
   }
 }
 
-// SHARE: a balanced launch (its own instantiation: the shares cost the other one registers that the main loop has none of, 1.5 % at 64K tokens)
-template <bool PAGED, bool DUMP, int NSET, bool SHARE>
+// ---- flat launches: one wave of CTAs over all (row, kv head) pairs, one behind the other, each CTA an equal share of their tiles.  A pair counts FLAT_EXTRA tiles more
+// than it has, which lie in front of its own: what a CTA pays for every pair that it works on (tables of the bases, queries, first copies, merges).  CTA c has
+// [c * share, (c + 1) * share) of the line; a pair's pieces are those of the CTAs that have tiles of it, in order, and an empty pair (its output is zero) goes to the
+// CTA that has its last place.  Piece (CTA, pair) has its partials at (c + pair) * G, which no two pieces share.
+// A grid of several waves pays a prologue, the merges and the wait for its slowest CTA with every wave, about 8.5 us, and half a wave is as dear as a whole one.
+// us, grid -> flat: 16 rows x 8 kv heads of 4K-64K tokens 472 -> 422, 64 x 1 of 32K (groups of 8) 228 -> 218, 8 x 8 of 4K-16K 94 -> 80 (a balanced launch before).
+// FLAT_EXTRA 24 / 36 / 48: 16 x 8 421 / 422 / 424, 12 x 8 of 500-6000 - / 43.0 / 44.5, 64 x 1 - / 218 / 216, 64 x 8 of 100-400 40.1 / 41.4 / 42.5.
+constexpr int FLAT_EXTRA = 36;
+struct FlatWalk {
+  int share, lo, hi;                                  // of the CTA
+  int row, kvh, at, tiles;                            // the pair that is looked at next: its first place on the line, its tiles
+  int pair, range[2], split, ns;                      // the piece found: pair = row * n_kv + kvh (below zero: no more), its first tile and how many, which of the pair's pieces
+};
+// Executed by one warp; every lane knows the same.
+template <class F> __device__ __forceinline__ void flat_start(FlatWalk& f, int B, int n_kv, int cta, int ctas, int lane, const F& tiles_of) {
+  u32 total = 0u;
+  for (int r0 = 0; r0 < B; r0 += 32) total += __reduce_add_sync(FULLM, r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + tiles_of(r0 + lane))) : 0u);
+  f.share = (int)((total + ctas - 1) / ctas);
+  f.lo = (int)min((long)cta * f.share, (long)total); f.hi = (int)min((long)f.lo + f.share, (long)total);
+  f.row = B; f.kvh = 0; f.at = 0; f.tiles = 0; f.pair = 0;
+  u32 before = 0u;
+  for (int r0 = 0; r0 < B && f.lo < f.hi; r0 += 32) {
+    const int t = r0 + lane < B ? tiles_of(r0 + lane) : 0;
+    const u32 own = r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + t)) : 0u;
+    u32 inc = own;
+    scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8); scan_step(inc, 16);
+    const u32 past = __ballot_sync(FULLM, before + inc > (u32)f.lo);
+    if (past) {                                       // the row that the CTA's first place lies in
+      const int l = __ffs((int)past) - 1;
+      f.row = r0 + l; f.tiles = __shfl_sync(FULLM, t, l);
+      const int row_at = (int)(before + __shfl_sync(FULLM, inc - own, l));
+      f.kvh = (f.lo - row_at) / (FLAT_EXTRA + f.tiles);
+      f.at = row_at + f.kvh * (FLAT_EXTRA + f.tiles);
+      break;
+    }
+    before += __shfl_sync(FULLM, inc, 31);
+  }
+}
+template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int cta, const F& tiles_of) {
+  f.pair = -1;
+  while (f.row < B && f.pair < 0) {
+    const int first = f.at + FLAT_EXTRA - (f.tiles > 0 ? 0 : 1), last = first + max(f.tiles, 1) - 1;
+    if (first >= f.hi) return;
+    if (last >= f.lo) {
+      const int c0 = first / f.share;
+      f.pair = f.row * n_kv + f.kvh; f.split = cta - c0; f.ns = last / f.share - c0 + 1;
+      f.range[0] = f.tiles > 0 ? max(f.lo, first) - first : 0; f.range[1] = f.tiles > 0 ? min(f.hi - 1, last) - first + 1 - f.range[0] : 0;
+    }
+    f.at += FLAT_EXTRA + f.tiles;
+    if (++f.kvh == n_kv) { f.kvh = 0; if (++f.row < B) f.tiles = tiles_of(f.row); }
+  }
+}
+
+// How the rows are shared out.  GRID: (row, kv head) x splits;  SHARED: a balanced launch;  FLAT_LINE: above.  Instantiations of their own: the shares cost the others
+// registers that the main loop has none of, 1.5 % at 64K tokens.
+enum { GRID, SHARED, FLAT_LINE };
+template <bool PAGED, bool DUMP, int NSET, int MODE>
 __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __grid_constant__ AttnParams p) {
+  constexpr bool SHARE = MODE == SHARED, FLAT = MODE == FLAT_LINE;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int s_next, s_last, s_split, s_ns;        // (the last two are not needed inside the main loop, whose registers are all taken)
+  __shared__ int s_next, s_last, s_split, s_ns, s_tail, s_esc[6];        // (from s_split on: not needed inside the main loop, whose registers are all taken)
+  __shared__ FlatWalk s_flat;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
@@ -424,7 +482,40 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       bh = __shfl_sync(FULLM, bh, 0); split0 = __shfl_sync(FULLM, split0, 0);
     }
   }
-  const int b = bh / p.n_kv, kvh = bh % p.n_kv;
+  auto tiles_of = [&](int row) -> int {               // (a slot's first head stands for all of its heads)
+    if (PAGED) return max((p.seq_len[row] + 15) >> 4, 0);
+    const int sl = p.slot[row];
+    return sl < 0 ? 0 : max((p.seq_len[(long)sl * p.n_kv] + 15) >> 4, 0);
+  };
+  if (FLAT && warp == 0) {
+    FlatWalk f;
+    flat_start(f, p.B, p.n_kv, blockIdx.x, gridDim.x, lane, tiles_of);
+    if (lane == 0) s_flat = f;
+    __syncwarp();
+  }
+  do {
+  if (FLAT) {                                        // the next piece
+    if (warp == 0) {
+      FlatWalk f = s_flat;
+      __syncwarp();
+      flat_next(f, p.B, p.n_kv, blockIdx.x, tiles_of);
+      if (lane == 0) { s_flat = f; s_split = f.split; s_ns = f.ns; }
+    }
+    // the ring begins again (every copy of the piece before has landed, and its last waits are behind the barrier at the end of the loop)
+    if (warp == ATT_WARPS - 1) reinterpret_cast<u32*>(smem + TB_USE)[lane] = 0u;
+    if (lane == 0 && warp < NSTG) {
+      asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_s + TB_FULL + 8 * warp) : "memory");
+      mbar_init(smem_s + TB_FULL + 8 * warp, 1);
+      reinterpret_cast<int*>(smem + TB_LEFT)[warp] = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // the ring was written by the merges of the piece before
+    __syncthreads();
+    bh = __shfl_sync(FULLM, s_flat.pair, 0);
+    if (bh < 0) return;
+    if (PAGED) S_paged = p.seq_len[bh / p.n_kv];
+  }
+  int b = bh / p.n_kv, kvh = bh % p.n_kv;
 
   // ---- which cache head, how many tokens, this CTA's tile range [tlo, tlo + n)
   // (without a slot map row b reads slot b; without a length table every head holds S_uniform tokens: the two dependent
@@ -444,14 +535,17 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // compiler so, and the address arithmetic built on them stays in uniform registers.
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
   const int ntiles = (S + 15) >> 4, chunk = (ntiles + ns0 - 1) / ns0;
-  const int tlo = min(split0 * chunk, ntiles), n = min(chunk, ntiles - tlo), nstages = (n + TPS - 1) / TPS;
-  const long smh = (long)ch * p.S_pad * D, cdh = (long)ch * p.S_pad * CB, rowb = (long)ch * p.S_pad, tileb = (long)ch * (p.S_pad >> 4);
+  const int tlo = FLAT ? min(__shfl_sync(FULLM, s_flat.range[0], 0), ntiles) : min(split0 * chunk, ntiles);
+  // (the last piece of a pair has what there is to the end, should a head be longer than the first one)
+  const int n = FLAT ? (__shfl_sync(FULLM, s_split + 1 - s_ns, 0) == 0 ? ntiles - tlo : min(__shfl_sync(FULLM, s_flat.range[1], 0), ntiles - tlo)) : min(chunk, ntiles - tlo);
+  const int nstages = (n + TPS - 1) / TPS;
   ohk = __shfl_sync(FULLM, ohk, 0); ohv = __shfl_sync(FULLM, ohv, 0);
 
   auto meta_of = [&](int i) -> TileMeta {             // i counts from the first tile of the CTA's range
     const int tile = tlo + i;
     if (PAGED) { const int pc = p.bt[(long)b * p.bt_stride + tile] * (2 * p.n_kv) + 2 * kvh; return TileMeta{p.mt[pc], p.mt[pc + 1]}; }
-    return TileMeta{p.K.tile_off[tileb + tile], p.V.tile_off[tileb + tile]};
+    const long at = (long)ch * (p.S_pad >> 4) + tile;
+    return TileMeta{p.K.tile_off[at], p.V.tile_off[at]};
   };
   // ---- filling a stage.  What a copy is given comes from uniform values or through a shuffle, so that the compiler knows it to be the same in every lane: the copy
   // instruction takes uniform registers, and anything else costs it a loop over the lanes.
@@ -464,8 +558,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // Escape window of a side for tiles whose escape bytes are [m0, m1) of the head's: from the 16-byte boundary at or below the first byte, a
   // multiple of 16 bytes, at most SIDE_ESC, inside the allocation (no bytes when the boundary lies before it).  phase: of the head's first byte;  to_end: bytes from there
   // to the end of the allocation.
-  const int phk = PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.K.ovf) + (unsigned)ohk) & 15), phv = PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.V.ovf) + (unsigned)ohv) & 15);
-  const int k_end = PAGED ? 0 : (int)max(-1L, min((long)p.K.ovf_bytes - ohk, 0x7FFFFF00L)), v_end = PAGED ? 0 : (int)max(-1L, min((long)p.V.ovf_bytes - ohv, 0x7FFFFF00L));
+  struct HeadEsc { int ohk, ohv, phk, phv, k_end, v_end; };
+  const HeadEsc head_esc{ohk, ohv, PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.K.ovf) + (unsigned)ohk) & 15), PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.V.ovf) + (unsigned)ohv) & 15),
+                         PAGED ? 0 : (int)max(-1L, min((long)p.K.ovf_bytes - ohk, 0x7FFFFF00L)), PAGED ? 0 : (int)max(-1L, min((long)p.V.ovf_bytes - ohv, 0x7FFFFF00L))};
   auto esc_window = [&](int to_end, int phase, int oh, int m0, int m1, int& start, u32& bytes) {
     const int w16 = (phase + m0) & 15, left = (int)((u32)to_end - (u32)m0 + (u32)w16);
     start = m0 - w16;
@@ -475,15 +570,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // Both are executed by a whole warp.  The part that needs no metadata (slot layout) ..
   auto fill_payload = [&](int st) {
     const u32 mb = smem_s + TB_FULL + 8 * (st % NSTG), dst = smem_s + TB_RING + (st % NSTG) * STAGE_BYTES, cnt = (u32)min(TPS, n - st * TPS);
-    const long tile = tlo + st * TPS;
+    const long row = (long)ch * p.S_pad + (long)(tlo + st * TPS) * T;
     warp_add_tx(mb, 2 * cnt * (TILE_SM + TILE_CD + 4 * T));
-    warp_g2s(dst + SB_FL, reinterpret_cast<const uint8_t*>(p.K.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
-    warp_g2s(dst + SIDE_BYTES + SB_FL, reinterpret_cast<const uint8_t*>(p.V.flags) + (rowb + tile * T) * 4, cnt * 4 * T, mb);
-    warp_g2s(dst, p.K.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb); warp_g2s(dst + SB_CD, p.K.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb);
-    warp_g2s(dst + SIDE_BYTES, p.V.sm + smh + tile * TILE_SM, cnt * TILE_SM, mb); warp_g2s(dst + SIDE_BYTES + SB_CD, p.V.codes + cdh + tile * TILE_CD, cnt * TILE_CD, mb);
+    warp_g2s(dst + SB_FL, reinterpret_cast<const uint8_t*>(p.K.flags) + row * 4, cnt * 4 * T, mb);
+    warp_g2s(dst + SIDE_BYTES + SB_FL, reinterpret_cast<const uint8_t*>(p.V.flags) + row * 4, cnt * 4 * T, mb);
+    warp_g2s(dst, p.K.sm + row * D, cnt * TILE_SM, mb); warp_g2s(dst + SB_CD, p.K.codes + row * CB, cnt * TILE_CD, mb);
+    warp_g2s(dst + SIDE_BYTES, p.V.sm + row * D, cnt * TILE_SM, mb); warp_g2s(dst + SIDE_BYTES + SB_CD, p.V.codes + row * CB, cnt * TILE_CD, mb);
   };
   // .. and the rest, or all of a paged stage.  own: stage_meta
-  auto fill_rest = [&](int st, const TileMeta& own) {
+  auto fill_rest = [&](int st, const TileMeta& own, const HeadEsc& h) {
     const int slot = st % NSTG;
     const u32 mb = smem_s + TB_FULL + 8 * slot, dst = smem_s + TB_RING + slot * STAGE_BYTES;
     int4 info;
@@ -496,7 +591,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       pieces = (u32)popc(__ballot_sync(FULLM, own.mk >= 0)) + (u32)popc(__ballot_sync(FULLM, own.mv >= 0));
     } else {
       const int m0k = __shfl_sync(FULLM, own.mk, 0), m0v = __shfl_sync(FULLM, own.mv, 0), m1k = __shfl_sync(FULLM, own.mk, TPS), m1v = __shfl_sync(FULLM, own.mv, TPS);
-      esc_window(k_end, phk, ohk, m0k, m1k, k0, nk); esc_window(v_end, phv, ohv, m0v, m1v, v0, nv);
+      esc_window(h.k_end, h.phk, h.ohk, m0k, m1k, k0, nk); esc_window(h.v_end, h.phv, h.ohv, m0v, m1v, v0, nv);
       info = make_int4((int)dst + SB_ESC + own.mk - k0, (int)nk - (own.mk - k0), (int)dst + SIDE_BYTES + SB_ESC + own.mv - v0, (int)nv - (own.mv - v0));
     }
     if (lane < min(TPS, n - st * TPS)) {
@@ -514,8 +609,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
         if (v >= 0) warp_g2s(dst + (2 * t + 1) * PSLOT, p.buf + (long)v * p.TS, slot_bytes, mb);
       }
     } else {
-      if (nk > 0) warp_g2s(dst + SB_ESC, p.K.ovf + ((long)ohk + k0), nk, mb);
-      if (nv > 0) warp_g2s(dst + SIDE_BYTES + SB_ESC, p.V.ovf + ((long)ohv + v0), nv, mb);
+      if (nk > 0) warp_g2s(dst + SB_ESC, p.K.ovf + ((long)h.ohk + k0), nk, mb);
+      if (nv > 0) warp_g2s(dst + SIDE_BYTES + SB_ESC, p.V.ovf + ((long)h.ohv + v0), nv, mb);
     }
   };
 
@@ -538,13 +633,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (warp == ATT_WARPS - 2 && lane < 16) fill_pair_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
     if (warp == ATT_WARPS - 1 && lane < 16) fill_pair_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
     if (SHARE && tid == 0) { s_split = split0; s_ns = ns0; }
+    if (FLAT && tid == 0) s_tail = TL;
     if (tid == 0) s_next = ATT_WARPS;                        // tiles 0 .. W-1 of the range go to warps 0 .. W-1, the rest is handed out on demand
   }
-  if (filler && warp < FIRST) fill_rest(warp, ahead);
+  if (filler && warp < FIRST) fill_rest(warp, ahead, head_esc);
+  if (!PAGED && tid == 0) *reinterpret_cast<HeadEsc*>(s_esc) = head_esc;
   WarpAcc<NSET> A;
   A.clear();
   __syncthreads();
-  if (filler && warp >= FIRST) { if (!PAGED) fill_payload(warp); fill_rest(warp, ahead); }
+  if (filler && warp >= FIRST) { if (!PAGED) fill_payload(warp); fill_rest(warp, ahead, head_esc); }
 
   uint16_t* const dump_k = DUMP ? p.dump_k + (long)bh * p.dump_S * D : nullptr;
   uint16_t* const dump_v = DUMP ? p.dump_v + (long)bh * p.dump_S * D : nullptr;
@@ -572,9 +669,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     const int2 m = reinterpret_cast<const int2*>(smem + TB_META)[nth];
     const uint8_t* const s0 = smem + TB_RING + slot * STAGE_BYTES;
     const SideView ks = PAGED ? SideView{s0 + 2 * ti * PSLOT, s0 + 2 * ti * PSLOT + SLOT_CD_OFF, p.buf + (long)m.x * p.TS + SLOT_OVF_OFF}
-                              : SideView{s0 + ti * TILE_SM, s0 + SB_CD + ti * TILE_CD, p.K.ovf + ((long)ohk + m.x)};
+                              : SideView{s0 + ti * TILE_SM, s0 + SB_CD + ti * TILE_CD, p.K.ovf + ((long)s_esc[0] + m.x)};
     const SideView vs = PAGED ? SideView{s0 + (2 * ti + 1) * PSLOT, s0 + (2 * ti + 1) * PSLOT + SLOT_CD_OFF, p.buf + (long)m.y * p.TS + SLOT_OVF_OFF}
-                              : SideView{s0 + SIDE_BYTES + ti * TILE_SM, s0 + SIDE_BYTES + SB_CD + ti * TILE_CD, p.V.ovf + ((long)ohv + m.y)};
+                              : SideView{s0 + SIDE_BYTES + ti * TILE_SM, s0 + SIDE_BYTES + SB_CD + ti * TILE_CD, p.V.ovf + ((long)s_esc[1] + m.y)};
     float sc[4] = {0.f, 0.f, 0.f, 0.f};
     if (!rawk) k_tile<DUMP>(sc, ks, win, area, W, lane, Q, dump_k + (long)tile * T * D, nvalid);
     else raw_scores<DUMP>(sc, p.raw + (long)raw_tile(m.x) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
@@ -593,12 +690,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if ((left & (TPS - 1)) == TPS - 1) {
         __syncwarp();
         if (!PAGED) fill_payload(st + NSTG);
-        fill_rest(st + NSTG, ahead);
+        fill_rest(st + NSTG, ahead, PAGED ? head_esc : HeadEsc{__shfl_sync(FULLM, s_esc[0], 0), __shfl_sync(FULLM, s_esc[1], 0), __shfl_sync(FULLM, s_esc[2], 0), __shfl_sync(FULLM, s_esc[3], 0), __shfl_sync(FULLM, s_esc[4], 0), __shfl_sync(FULLM, s_esc[5], 0)});
       }
     }
     it = nx;
   }
-  const int split = SHARE ? s_split : split0, NS = SHARE ? s_ns : p.nsplit;
+  const int split = SHARE || FLAT ? s_split : split0, NS = SHARE || FLAT ? s_ns : p.nsplit;
+  if (FLAT) { bh = __shfl_sync(FULLM, s_flat.pair, 0); b = bh / p.n_kv; kvh = bh % p.n_kv; TL = __shfl_sync(FULLM, s_tail, 0); }
   // ---- slot layout: the raw BF16 tail belongs to the last split's last warp
   if (!PAGED && TL > 0 && split == NS - 1 && warp == ATT_WARPS - 1) {
     const uint16_t* kraw = reinterpret_cast<const uint16_t*>(p.K.tail) + (long)ch * p.tail_cap * D;
@@ -615,7 +713,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   }
 
   // ---- merge the warps of the CTA (the ring is free now)
-  if (__syncthreads_or(sum_warp(A))) sum_exact<PAGED, false>(p, smem + TB_RING, bh, split, NS);
+  if (__syncthreads_or(sum_warp(A))) sum_exact<PAGED, false>(p, smem + TB_RING, bh, split, NS, FLAT ? s_flat.range : nullptr);
   else stage_warp(A, smem + TB_RING, G, warp, lane);
   __syncthreads();
   const long qh0 = (long)b * p.n_q + kvh * G;
@@ -653,14 +751,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (g >= G) continue;
     if (NS == 1) deliver(g, M[i], Lc[i], Ac[i]);     // nothing to merge with
     else {
-      const long pidx = SHARE ? ((long)blockIdx.x * p.units + blockIdx.y) * G + g : (qh0 + g) * p.nsplit + split;
+      const long pidx = FLAT ? (long)(blockIdx.x + bh) * G + g : SHARE ? ((long)blockIdx.x * p.units + blockIdx.y) * G + g : (qh0 + g) * p.nsplit + split;
       if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
       p.pa[pidx * D + d] = Ac[i];
     }
   }
   if (NS > 1) {
-    if (!last_split(p.counters + bh, NS, &s_last)) return;
-    if (SHARE) merge_splits<4 * NSET>(p, smem + TB_RING, ((long)blockIdx.x * p.units + blockIdx.y - split) * G, 1, G, G, NS, deliver);
+    const bool last = last_split(p.counters + bh, NS, &s_last);
+    if (!FLAT && !last) return;
+    if (FLAT) { if (last) merge_splits<4 * NSET>(p, smem + TB_RING, (long)(blockIdx.x - split + bh) * G, 1, G, G, NS, deliver); }
+    else if (SHARE) merge_splits<4 * NSET>(p, smem + TB_RING, ((long)blockIdx.x * p.units + blockIdx.y - split) * G, 1, G, G, NS, deliver);
     else merge_splits<4 * NSET>(p, smem + TB_RING, qh0 * NS, NS, 1, G, NS, deliver);
   }
   if (p.x_recv) {
@@ -687,6 +787,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if (atomicAdd(p.x_ticket, 1) == (int)gridDim.x - 1) { *p.x_ticket = 0; __threadfence(); atomicAdd(p.x_epoch, 1); }
     }
   }
+  if (FLAT) __syncthreads();                         // the shared memory is used again
+  } while (FLAT);
 }
 
 // ------------------------------------------------------------------------------------------------ head_dim 256, paged layout
@@ -990,10 +1092,10 @@ static int launch_big(const AttnParams& p, dim3 grid, int smem_bytes, cudaStream
     asked = true;
   }
 }
-template <bool PAGED, bool DUMP, int NSET, bool SHARE>
+template <bool PAGED, bool DUMP, int NSET, int MODE>
 static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
-  const dim3 grid = SHARE ? dim3((unsigned)p.n_kv, (unsigned)p.units) : dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit);
-  return launch_big<decode_attn_kernel<PAGED, DUMP, NSET, SHARE>>(p, grid, ATT_SMEM, st);
+  const dim3 grid = MODE == FLAT_LINE ? dim3((unsigned)p.flat) : MODE == SHARED ? dim3((unsigned)p.n_kv, (unsigned)p.units) : dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit);
+  return launch_big<decode_attn_kernel<PAGED, DUMP, NSET, MODE>>(p, grid, ATT_SMEM, st);
 }
 template <int NSET>
 static int launch_attn256(const AttnParams& p, cudaStream_t st) {
@@ -1001,8 +1103,9 @@ static int launch_attn256(const AttnParams& p, cudaStream_t st) {
 }
 template <bool PAGED, bool DUMP>
 static int launch_attn(const AttnParams& p, cudaStream_t st) {
-  if (!DUMP && p.units) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, true>(p, st) : launch_attn_as<PAGED, false, 2, true>(p, st);
-  return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1, false>(p, st) : launch_attn_as<PAGED, DUMP, 2, false>(p, st);
+  if (!DUMP && p.flat) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, FLAT_LINE>(p, st) : launch_attn_as<PAGED, false, 2, FLAT_LINE>(p, st);
+  if (!DUMP && p.units) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, SHARED>(p, st) : launch_attn_as<PAGED, false, 2, SHARED>(p, st);
+  return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1, GRID>(p, st) : launch_attn_as<PAGED, DUMP, 2, GRID>(p, st);
 }
 
 static int sm_count_of_current_device() {
@@ -1023,9 +1126,14 @@ static bool exchange_ok(const gaac_exchange* x) {
 struct SlotOut {
   void* out = nullptr; float* out_f32 = nullptr; float* part = nullptr;
   const gaac_exchange* x = nullptr; bool fused = false;
-  int units = 0;
+  int units = 0, flat = 0;
   void* dump_k = nullptr; void* dump_v = nullptr; int64_t dump_S = 0;
 };
+// Splits per row whose room the partials of a flat launch fit into, and whether the line's places can be counted in an int.
+static int flat_splits(int B, int n_kv, int ctas) { return 1 + (int)(((int64_t)ctas + (int64_t)B * n_kv - 1) / ((int64_t)B * n_kv)); }
+static bool flat_ok(int B, int n_kv, int ctas, int64_t longest) {
+  return B > 0 && n_kv > 0 && ctas > 0 && ctas <= 1024 && longest >= 0 && longest < (1LL << 36) && (int64_t)B * n_kv < (1 << 24) && (int64_t)B * n_kv * (longest / T + 1 + FLAT_EXTRA) + ctas < 0x7FFFFFFFLL;
+}
 
 static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, const int32_t* slot, int B, int n_q, int n_kv, const int32_t* seq_len,
                      int64_t S_uniform, int64_t S_pad, float scale, int nsplit, const int32_t* tail_len, int tail_cap, int n_base_rows, void* ws, size_t ws_bytes,
@@ -1051,12 +1159,12 @@ static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, cons
   AttnParams p{};
   p.K = *K; p.V = *V; p.slot = slot; p.seq_len = seq_len; p.S_uniform = (int)S_uniform; p.tail_len = tail_len; p.tail_cap = tail_cap; p.S_pad = S_pad; p.n_base_rows = n_base_rows;
   p.q = (const uint16_t*)q; p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.G = n_q / n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)o.out; p.out_f32 = o.out_f32; p.part = o.part; p.units = o.units; p.wave = o.units ? share_wave(B, n_kv) : 0;
+  p.out = (uint16_t*)o.out; p.out_f32 = o.out_f32; p.part = o.part; p.units = o.units; p.wave = o.units ? share_wave(B, n_kv) : 0; p.flat = o.flat;
   if (x) {
     p.x_recv = x->recv; p.x_epoch = x->epoch; p.x_ticket = x->ticket; p.x_err = x->err;
     p.x_rank = x->rank; p.x_world = x->world; p.x_rows_cap = x->rows_cap; p.x_fused = o.fused ? 1 : 0;
   }
-  if (int e = carve_workspace(ws, ws_bytes, B, n_q, o.units ? share_splits(B, o.units) : nsplit, p)) return e;
+  if (int e = carve_workspace(ws, ws_bytes, B, n_q, o.flat ? flat_splits(B, n_kv, o.flat) : o.units ? share_splits(B, o.units) : nsplit, p)) return e;
   if (o.dump_k) {
     p.dump_k = (uint16_t*)o.dump_k; p.dump_v = (uint16_t*)o.dump_v; p.dump_S = o.dump_S;
     return launch_attn<false, true>(p, (cudaStream_t)stream);
@@ -1065,7 +1173,7 @@ static int slot_attn(const gaac_side* K, const gaac_side* V, const void* q, cons
 }
 
 static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16, int B, int n_q, float scale,
-                      int nsplit, int units, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* dump_k, void* dump_v, int64_t dump_S, void* stream) {
+                      int nsplit, int units, int flat, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* dump_k, void* dump_v, int64_t dump_S, void* stream) {
   if (!st || !bt || !seq_lens || !q_bf16 || !out_bf16 || !st->buf || !st->raw || !st->mt || !st->b3k || !st->b4k || !st->b3v || !st->b4v) return GAAC_E_ARG;
   if (B <= 0 || n_q <= 0 || st->n_kv <= 0 || nsplit <= 0 || nsplit > 1024 || bt_stride <= 0) return GAAC_E_ARG;
   if (n_q % st->n_kv || n_q / st->n_kv < 1 || n_q / st->n_kv > 8 || st->TS % 16 || st->TS != SLOT_OVF_OFF + st->ovf_slot) return GAAC_E_UNSUPPORTED;
@@ -1075,15 +1183,15 @@ static int paged_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride
   p.buf = st->buf; p.raw = (const uint16_t*)st->raw; p.mt = st->mt; p.bt = bt; p.bt_stride = bt_stride; p.TS = st->TS; p.ovf_slot = st->ovf_slot;
   p.b3k = st->b3k; p.b4k = st->b4k; p.b3v = st->b3v; p.b4v = st->b4v; p.seq_len = seq_lens;
   p.q = (const uint16_t*)q_bf16; p.B = B; p.n_q = n_q; p.n_kv = st->n_kv; p.G = n_q / st->n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr; p.units = units; p.wave = units ? share_wave(B, st->n_kv) : 0;
-  if (int e = carve_workspace(workspace, workspace_bytes, B, n_q, units ? share_splits(B, units) : nsplit, p)) return e;
+  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.part = nullptr; p.units = units; p.wave = units ? share_wave(B, st->n_kv) : 0; p.flat = flat;
+  if (int e = carve_workspace(workspace, workspace_bytes, B, n_q, flat ? flat_splits(B, st->n_kv, flat) : units ? share_splits(B, units) : nsplit, p)) return e;
   if (dump_k) {
     p.dump_k = (uint16_t*)dump_k; p.dump_v = (uint16_t*)dump_v; p.dump_S = dump_S;
     return launch_attn<true, true>(p, (cudaStream_t)stream);
   }
   // ragged batches: CTAs are handed out longest row first (one small launch sorts the rows; its output is read by the attention
   // kernel after its dependency wait)
-  if (!units && B > 1 && B <= ORDER_MAX_ROWS && (int64_t)B * st->n_kv * nsplit > sm_count_of_current_device()) {
+  if (!units && !flat && B > 1 && B <= ORDER_MAX_ROWS && (int64_t)B * st->n_kv * nsplit > sm_count_of_current_device()) {
     launch_row_order(seq_lens, B, p.order_buf, (cudaStream_t)stream);
     p.row_order = p.order_buf;
   }
@@ -1120,6 +1228,14 @@ extern "C" int gaac_decode_attn_balanced(const gaac_side* K, const gaac_side* V,
   if (!out_bf16 || !slot || !seq_len || B <= 0 || B > SHARE_MAX_ROWS || units < B || units - B + 1 > 1024) return GAAC_E_ARG;
   SlotOut o; o.out = out_bf16; o.out_f32 = out_f32; o.units = units;
   return slot_attn(K, V, q_bf16, slot, B, n_q, n_kv, seq_len, 0, S_pad, scale, units - B + 1, tail_len, tail_cap, n_base_rows, workspace, workspace_bytes, o, stream);
+}
+
+extern "C" int gaac_decode_attn_flat(const gaac_side* K, const gaac_side* V, const void* q_bf16, const int32_t* slot, int B, int n_q, int n_kv,
+                                     const int32_t* seq_len, int64_t S_pad, float scale, int ctas, const int32_t* tail_len, int tail_cap,
+                                     int n_base_rows, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* stream) {
+  if (!out_bf16 || !slot || !seq_len || !flat_ok(B, n_kv, ctas, S_pad)) return GAAC_E_ARG;
+  SlotOut o; o.out = out_bf16; o.out_f32 = out_f32; o.flat = ctas;
+  return slot_attn(K, V, q_bf16, slot, B, n_q, n_kv, seq_len, 0, S_pad, scale, 1, tail_len, tail_cap, n_base_rows, workspace, workspace_bytes, o, stream);
 }
 
 extern "C" int gaac_decode_attn_pages(const gaac_side* K, const gaac_side* V, const void* q_bf16, int B, int n_q, int n_kv, int64_t S, int64_t S_pad,
@@ -1183,14 +1299,21 @@ extern "C" int gaac_combine_parts(const float* parts, int64_t n_heads, int n_par
 extern "C" int gaac_paged_decode_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                                       int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
                                       void* out_bf16, float* out_f32, void* stream) {
-  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, 0, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
 }
 
 extern "C" int gaac_paged_decode_attn_balanced(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                                                int B, int n_q, float scale, int units, void* workspace, size_t workspace_bytes,
                                                void* out_bf16, float* out_f32, void* stream) {
   if (B <= 0 || B > SHARE_MAX_ROWS || units < B || units - B + 1 > 1024) return GAAC_E_ARG;
-  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, units - B + 1, units, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, units - B + 1, units, 0, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
+}
+
+extern "C" int gaac_paged_decode_attn_flat(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                           int B, int n_q, float scale, int ctas, void* workspace, size_t workspace_bytes,
+                                           void* out_bf16, float* out_f32, void* stream) {
+  if (!st || bt_stride <= 0 || bt_stride > (1LL << 32) || !flat_ok(B, st->n_kv, ctas, bt_stride * T)) return GAAC_E_ARG;
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, 1, 0, ctas, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
 }
 
 extern "C" int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
@@ -1225,5 +1348,5 @@ extern "C" int gaac_debug_paged_decode_attn_rebuild(const gaac_paged* st, const 
                                                     int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes, void* out_bf16,
                                                     float* out_f32, void* k_rebuilt, void* v_rebuilt, int64_t rebuilt_S, void* stream) {
   if (!k_rebuilt || !v_rebuilt) return GAAC_E_ARG;
-  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, workspace, workspace_bytes, out_bf16, out_f32, k_rebuilt, v_rebuilt, rebuilt_S, stream);
+  return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, 0, workspace, workspace_bytes, out_bf16, out_f32, k_rebuilt, v_rebuilt, rebuilt_S, stream);
 }

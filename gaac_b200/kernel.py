@@ -118,6 +118,30 @@ def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> in
     return min(units, B * -(-max(S, 1) // 64))
 
 
+@functools.lru_cache(maxsize=4096)
+def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int = 4, sm_count: int = SM_COUNT_B200) -> int:
+    """CTAs of a flat launch (one wave that shares the tiles of all rows and kv heads evenly), or 0 where the form that it would replace is no slower: nsplit splits per
+    (row, kv head), or `units` ranges per kv head (S: tokens of the longest row, group: query heads per kv head).
+    A flat launch saves what comes with the waves of a grid, and the idle end of the last one; it pays some 8 us for every piece of a row that a CTA has beyond its
+    first.  us, other form -> flat:
+      grids of several waves: 64 rows x 1 kv head, 32K tokens 228 -> 218;  16 x 8, 4K-64K 472 -> 422;  40 x 4, 2K-6K 95 -> 80;  20 x 8, 2K-3K 71 -> 56;  64 x 8, up to 4200
+        124 -> 120.  Short rows lose: 32 x 8, 20-2000 tokens 49 -> 56;  64 x 8, 100-400 33 -> 41;  24 x 8, 64-600 17 -> 24
+      one wave that leaves SMs idle: 64 x 2, 4K-8K 116 -> 101;  64 x 1, 8K-16K 118 -> 91.  An eighth or less idle loses if all rows are as long: 18 x 8, 8K 111 -> 119
+      shares of units, which come in whole ones: a fifth of them or more for the rows' first units 8 x 8, 4K-16K 94 -> 80;  4 x 8, 20K-32K 104 -> 95;  5 x 8, up to 9K 31.7 ->
+        30.6;  fewer, 16 x 1 36 -> 39, 8 x 1 36.4 -> 36.9;  more than four query heads per kv head, 6 x 8 61 -> 64."""
+    rows, tiles = B * n_kv, -(-S // 16)
+    if B <= 1 or tiles < 160 or rows * tiles < 120 * sm_count or rows * (tiles + 64) >= 1 << 30:
+        return 0
+    if units:
+        return sm_count if group <= 4 and 5 * B >= units else 0
+    ctas = rows * nsplit
+    return 0 if 7 * sm_count < 8 * ctas <= 8 * sm_count else sm_count
+
+
+def _flat_splits(B: int, n_kv: int, ctas: int) -> int:
+    return 1 + -(-ctas // (B * n_kv))            # what the workspace must have room for
+
+
 def _side(sm, codes, flags, tile_off, ovf, head_start, base3, base4, tail) -> _lib.Side:
     return _lib.Side(sm.data_ptr(), codes.data_ptr(), flags.data_ptr(), tile_off.data_ptr(), ovf.data_ptr(), head_start.data_ptr(),
                      ovf.numel(), base3.data_ptr(), base4.data_ptr(), _lib.ptr(tail))
@@ -128,14 +152,14 @@ class _Ext:
 
     @staticmethod
     def gaac_attn_launch(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, smv, cv, fv, tov, ovv, ohsv, b3v, b4v,
-                         q, slot, n_q, n_kv, SL, S_pad, scale, nsplit, kt, vt, TL, TCAP, out_f32=None, partial=None, exchange=None, fused=False, units=0):
+                         q, slot, n_q, n_kv, SL, S_pad, scale, nsplit, kt, vt, TL, TCAP, out_f32=None, partial=None, exchange=None, fused=False, units=0, flat=0):
         """Same positional arguments as the reference launcher (gaac/kernel.py:296-300): 16 K/V buffers, q [B*n_q, 128] bf16,
         slot int32 [B], n_q, n_kv, SL int32 [heads], S_pad, scale, nsplit, K/V tails [heads, TCAP, 128] bf16 (empty = none),
         TL int32 [heads], TCAP.  Returns out [B*n_q, 128] bf16.  Extras: out_f32 (fp32 tensor to receive the un-rounded
         result), partial ([B*n_q, 130] fp32 tensor: write (m, l, acc) there instead of the output), exchange (a
         gaac_b200._lib.Exchange: push the partial rows into every rank's receive buffer instead and return None; with fused=True
         the same launch also waits for the other ranks' rows, merges them and returns the output), units (> 0: the rows share that many
-        ranges per kv head by their lengths, nsplit is not used)."""
+        ranges per kv head by their lengths, nsplit is not used), flat (> 0: one wave of that many CTAs, see choose_flat)."""
         D = 128
         if q.size(-1) != D:
             raise RuntimeError("head_dim must be 128")
@@ -150,11 +174,12 @@ class _Ext:
         K = _side(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None)
         V = _side(smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None)
         stream = _lib.stream_ptr(dev)
-        ws = workspace(dev, B, n_q, -(-units // B) if units else nsplit, stream)
+        ws = workspace(dev, B, n_q, _flat_splits(B, n_kv, flat) if flat else -(-units // B) if units else nsplit, stream)
         L = _lib.lib()
-        if units:
+        if flat or units:
             out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
-            _lib.check(L.gaac_decode_attn_balanced(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), units,
+            launch = L.gaac_decode_attn_flat if flat else L.gaac_decode_attn_balanced
+            _lib.check(launch(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), flat or units,
                                                    TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel(),
                                                    out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_decode_attn_balanced")
             return out

@@ -17,7 +17,7 @@ import torch
 from . import _lib
 from .codec import Codec, Page, D, T, CB
 from .encoder import TileEncoder
-from .kernel import _ext, choose_nsplit, choose_nsplit_sm100, choose_units
+from .kernel import _ext, choose_flat, choose_nsplit, choose_nsplit_sm100, choose_units
 
 TAIL = T                       # rows of the raw tail buffer of a head
 TILE_MAX_ESC = 1280            # a tile whose 256 groups are all raw has 256 * 5 escape bytes
@@ -225,13 +225,15 @@ class CompressedKVCache:
         B, n_q, _ = q.shape
         self.settle_prefills()
         units = choose_units(B, self.n_kv, max_len or self.cap) if nsplit is None else 0
-        if nsplit is None and not units:
-            nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap)
+        flat = 0
+        if nsplit is None:
+            if not units: nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap)
+            flat = choose_flat(B, self.n_kv, max_len or self.cap, nsplit or 0, units, q.shape[1] // self.n_kv)
         K, V = self.k, self.v
         out = _ext().gaac_attn_launch(K.sm, K.codes, K.flags, K.tile_off, K.ovf, K.head_start, K.base3, K.base4,
                                       V.sm, V.codes, V.flags, V.tile_off, V.ovf, V.head_start, V.base3, V.base4,
                                       q.reshape(B * n_q, D).contiguous(), slots, n_q, self.n_kv, self.S, self.cap, scale, nsplit,
-                                      K.tail, V.tail, self.tail_len, TAIL, out_f32=out_f32, units=units)
+                                      K.tail, V.tail, self.tail_len, TAIL, out_f32=out_f32, units=units, flat=flat)
         return out.view(B, n_q, D)
 
     # ------------------------------------------------------------------ housekeeping

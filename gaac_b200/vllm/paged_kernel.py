@@ -9,7 +9,7 @@ all read by the one fused kernel: there is no decompression pass.
 from __future__ import annotations
 import torch
 from .. import _lib
-from ..kernel import workspace, choose_nsplit_sm100, choose_units
+from ..kernel import workspace, choose_flat, choose_nsplit_sm100, choose_units, _flat_splits
 
 
 def choose_nsplit(B, n_kv, S, target_ctas=96, min_tok=512, cap=48):
@@ -27,14 +27,19 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     if not (1 <= G <= 8): raise RuntimeError("G must be 1..8")
     if TS % 16: raise RuntimeError("tile stride must be a multiple of 16")
     if not q.is_cuda: raise RuntimeError("gaac_b200 attention needs CUDA tensors: there is no CPU path")
-    units = choose_units(B, n_kv, bt.shape[1] * 16) if nsplit is None else 0
-    if units: nsplit = -(-units // B)            # what the workspace must have room for
-    elif nsplit is None: nsplit = choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)
+    units = flat = 0
+    if nsplit is None:
+        units = choose_units(B, n_kv, bt.shape[1] * 16)
+        nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)        # with units: what the workspace must have room for
+        # (the library bounds a row's length by the table's row stride)
+        flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv) if B * n_kv * (bt.stride(0) + 64) < 1 << 30 else 0
+        if flat: nsplit = _flat_splits(B, n_kv, flat)
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, n_q, nsplit, stream)
-    launch = _lib.lib().gaac_paged_decode_attn_balanced if units else _lib.lib().gaac_paged_decode_attn
-    _lib.check(launch(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), units or int(nsplit),
+    lib = _lib.lib()
+    launch = lib.gaac_paged_decode_attn_flat if flat else lib.gaac_paged_decode_attn_balanced if units else lib.gaac_paged_decode_attn
+    _lib.check(launch(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit),
                       ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_paged_decode_attn")
     return out

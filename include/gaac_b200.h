@@ -235,6 +235,13 @@ int gaac_decode_attn_balanced(const gaac_side* K, const gaac_side* V, const void
                               const int32_t* seq_len, int64_t S_pad, float scale, int units, const int32_t* tail_len, int tail_cap,
                               int n_base_rows, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* stream);
 
+/* gaac_decode_attn as ONE wave of `ctas` CTAs (1..1024, as many as run at a time) that share the tiles of all (row, kv head) pairs evenly: for batches
+ * whose grid would be several waves.  Workspace as for gaac_decode_attn with 1 + ceil(ctas / (B * n_kv)) splits.  The length of a slot's first head stands
+ * for its other heads' where the work is shared out. */
+int gaac_decode_attn_flat(const gaac_side* K, const gaac_side* V, const void* q_bf16, const int32_t* slot, int B, int n_q, int n_kv,
+                          const int32_t* seq_len, int64_t S_pad, float scale, int ctas, const int32_t* tail_len, int tail_cap,
+                          int n_base_rows, void* workspace, size_t workspace_bytes, void* out_bf16, float* out_f32, void* stream);
+
 /* Decode attention over two Pages (all B*n_kv heads hold S tokens, row b reads heads b*n_kv .., no tail): the
  * `attention(q, kp, vp)` entry of the reference (gaac/kernel.py:345-359), which builds an identity slot map and a constant
  * length table for its launcher; here both are implied, so the kernel's prologue has no dependent table loads.  Exactly one
@@ -332,6 +339,11 @@ int gaac_paged_decode_attn(const gaac_paged* st, const int32_t* bt, int64_t bt_s
 int gaac_paged_decode_attn_balanced(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                                     int B, int n_q, float scale, int units, void* workspace, size_t workspace_bytes,
                                     void* out_bf16, float* out_f32, void* stream);
+
+/* gaac_paged_decode_attn as one wave of CTAs, as in gaac_decode_attn_flat. */
+int gaac_paged_decode_attn_flat(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                int B, int n_q, float scale, int ctas, void* workspace, size_t workspace_bytes,
+                                void* out_bf16, float* out_f32, void* stream);
 
 /* The same for head_dim 256: a 256-dim head is stored as two 128-dim half-heads in neighbouring tile slots, each with its own
  * bases, so the store, the block decoder and the bases all see 2 * (256-dim kv heads) half-heads: st->n_kv is that number of

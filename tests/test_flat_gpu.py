@@ -1,0 +1,94 @@
+"""One wave of CTAs over the tiles of all rows and kv heads (gaac_decode_attn_flat, gaac_paged_decode_attn_flat): every row against the fp64 oracle, with one CTA
+for everything, a few, as many as there are SMs and more than there are tiles; empty rows, rows that are all tail, padding rows, 1 to 70 rows; V
+elements that are not finite (their CTA repeats its piece)."""
+import numpy as np
+import pytest
+from common import to_bf16_cuda, assert_attention_close
+from oracle import gaac_oracle as O
+from test_paged_gpu import _build_paged
+
+SCALE = 128 ** -0.5
+
+
+def test_choose_flat_bounds():
+    from gaac_b200.kernel import choose_flat, choose_nsplit_sm100, choose_units
+    for n_kv in (1, 2, 8, 148, 149):
+        for B in (1, 2, 7, 33, 64, 300, 1025):
+            for S in (1, 300, 5000, 10 ** 6):
+                units = choose_units(B, n_kv, S)
+                flat = choose_flat(B, n_kv, S, choose_nsplit_sm100(B, n_kv, S), units)
+                assert flat in (0, 148) and not (flat and (B == 1 or S <= 2544))
+    assert choose_flat(64, 1, 32769, 9, 0) == 148 and choose_flat(148, 1, 1000, 1, 0) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [0, 5, 16, 1000, 17]), (1, 8, [700]), (3, 5, [3, 33, 64, 65, 900, 1, 0, 300, 15, 16, 31, 47, 48, 49] * 5)])
+def test_slots_flat(monkeypatch, n_kv, G, lens):
+    import torch
+    import gaac_b200.kv_cache as kvc
+    B, hist = len(lens), {}
+    cache = kvc.CompressedKVCache(n_slots=B, n_kv=n_kv, capacity=1024, bases=None)
+    for s, L in enumerate(lens):
+        k, v = (np.ascontiguousarray(O.kv_like(n_kv, max(L, 1), 7 * s + i).transpose(1, 0, 2))[:L] for i in (1, 2))
+        cache.prefill(s, to_bf16_cuda(k), to_bf16_cuda(v), check=False)
+        hist[s] = (k, v)
+    rng = np.random.default_rng(B)
+    order = rng.permutation(B)
+    order[B // 2] = -1 if B > 1 else order[B // 2]
+    slots = torch.tensor(order, dtype=torch.int32, device="cuda")
+    q16 = O.f32_to_bf16((rng.standard_normal((B, n_kv * G, 128)) * 0.1).astype(np.float32))
+    for ctas in (1, 3, 37, 148, 148, 1000):                                     # the same call twice: the split counters are left at zero
+        monkeypatch.setattr(kvc, "choose_flat", lambda *a, n=ctas: n)
+        o32 = torch.empty(B, n_kv * G, 128, dtype=torch.float32, device="cuda")
+        out = cache.attention(to_bf16_cuda(q16), slots, SCALE, max_len=1000, out_f32=o32)
+        for b, s in enumerate(order):
+            if s < 0 or lens[s] == 0:
+                assert not out[b].any(), (b, s, ctas)
+            else:
+                assert_attention_close(o32[b].cpu().numpy(), q16[b], *hist[s], SCALE, (b, s, ctas))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [16, 37, 333, 1000, 5]), (1, 8, [1500, 1]), (4, 1, [1, 500] * 20)])
+def test_paged_flat(monkeypatch, n_kv, G, lens):
+    import torch
+    import gaac_b200.vllm.paged_kernel as pk
+    blocks = sum(-(-x // 16) for x in lens)
+    st, buf, bt, ks, vs = _build_paged(lens, n_kv, blocks + 4, seed=n_kv, adversarial_every=5, raw_tiles=2 * n_kv * blocks)
+    assert int(st.err) == 0
+    B, n_q = len(lens), n_kv * G
+    q16 = O.f32_to_bf16((np.random.default_rng(1).standard_normal((B, n_q, 128)) * 0.3).astype(np.float32))
+    lens_now = list(lens)
+    lens_now[B // 2] = 0                                                        # a row without tokens between others
+    sl = torch.tensor(lens_now, dtype=torch.int32, device="cuda")
+    for ctas in (1, 3, 37, 148, 1000):
+        monkeypatch.setattr(pk, "choose_flat", lambda *a, n=ctas: n)
+        o32 = torch.empty(B, n_q, 128, dtype=torch.float32, device="cuda")
+        out = torch.full((B, n_q * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+        pk.paged_attention(to_bf16_cuda(q16), out, buf, st.raw, st.mt, bt, sl, st.bases, st.TS, n_q, n_kv, out_f32=o32)
+        for b in range(B):
+            if lens_now[b] == 0:
+                assert not out[b].any(), (b, ctas)
+            else:
+                assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b], vs[b], SCALE, (b, ctas))
+
+
+@pytest.mark.gpu
+def test_flat_pieces_with_infinite_elements(monkeypatch):
+    import torch
+    import gaac_b200.kv_cache as kvc
+    n_kv, G, lens = 1, 4, [400, 90, 1000]
+    cache = kvc.CompressedKVCache(n_slots=3, n_kv=n_kv, capacity=1024, bases=None)
+    q16 = O.f32_to_bf16((np.random.default_rng(3).standard_normal((3, n_kv * G, 128)) * 0.1).astype(np.float32))
+    for s, L in enumerate(lens):
+        k, v = (np.ascontiguousarray(O.kv_like(n_kv, L, 9 * s + i, outliers=0.0).transpose(1, 0, 2)) for i in (1, 2))        # (no weight underflows: 0 x Inf is NaN)
+        v[L // 2, 0, 5] = 0x7F80                                                # one infinite element of channel 5
+        cache.prefill(s, to_bf16_cuda(k), to_bf16_cuda(v))
+    slots = torch.arange(3, dtype=torch.int32, device="cuda")
+    want = cache.attention(to_bf16_cuda(q16), slots, SCALE, nsplit=2).float()
+    for ctas in (1, 4, 148):
+        monkeypatch.setattr(kvc, "choose_flat", lambda *a, n=ctas: n)
+        got = cache.attention(to_bf16_cuda(q16), slots, SCALE, max_len=1000).float()
+        assert torch.isinf(got[:, :, 5]).all() and torch.isfinite(got[:, :, :5]).all() and torch.isfinite(got[:, :, 6:]).all()
+        keep = [c for c in range(128) if c != 5]
+        assert torch.allclose(got[:, :, keep], want[:, :, keep], rtol=2 ** -7, atol=1e-3)        # BF16 results of the same sums in another order
