@@ -75,6 +75,7 @@ _SIGNATURES = {
     "gaac_paged_decode_attn_balanced": (i32, [C.POINTER(Paged), vp, i64, vp, vp, i32, i32, f32, i32, vp, sz, vp, vp, vp]),
     "gaac_decode_attn_flat": (i32, [C.POINTER(Side), C.POINTER(Side), vp, vp, i32, i32, i32, vp, i64, f32, i32, vp, i32, i32, vp, sz, vp, vp, vp]),
     "gaac_paged_decode_attn_flat": (i32, [C.POINTER(Paged), vp, i64, vp, vp, i32, i32, f32, i32, vp, sz, vp, vp, vp]),
+    "gaac_paged_decode_attn256_flat": (i32, [C.POINTER(Paged), vp, i64, vp, vp, i32, i32, f32, i32, vp, sz, vp, vp, vp]),
     "gaac_decode_attn_static": (i32, [C.POINTER(Side), C.POINTER(Side), vp, vp, i32, i32, i32, vp, i64, f32, i32, vp, i32, i32, vp, vp, vp]),
     "gaac_static_workspace_bytes": (sz, []),
     "gaac_static_workspace_error": (i32, [vp, i32, vp]),

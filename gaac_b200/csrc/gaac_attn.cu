@@ -48,7 +48,7 @@ constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + BASES
 constexpr int ATT_SMEM = TB_RING + NSTG * STAGE_BYTES + 16;          // (an escape segment is read as whole words)
 static_assert(TB_BASES % 16 == 0 && TB_ESC % 16 == 0 && TB_AREA % 16 == 0 && TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
               "bulk copies need 16-byte aligned shared-memory destinations and sizes");
-static_assert(ATT_SMEM + 112 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
+static_assert(ATT_SMEM + 240 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
 static_assert(ATT_THREADS / 128 * 2 >= 8, "the fused exchange keeps at most two merged heads per thread");
 constexpr int ACC_LD = D + 8;                        // row stride of the staged accumulators: 8j + r banks, conflict-free stores
 
@@ -378,25 +378,35 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
 // than it has, which lie in front of its own: what a CTA pays for every pair that it works on (tables of the bases, queries, first copies, merges).  CTA c has
 // [c * share, (c + 1) * share) of the line; a pair's pieces are those of the CTAs that have tiles of it, in order, and an empty pair (its output is zero) goes to the
 // CTA that has its last place.  Piece (CTA, pair) has its partials at (c + pair) * G, which no two pieces share.
+// Where the longest pair in k = CTAs / pairs equal pieces gives no CTA more than that share, every pair is in k pieces and a CTA has one: rows of about one length.
 // A grid of several waves pays a prologue, the merges and the wait for its slowest CTA with every wave, about 8.5 us, and half a wave is as dear as a whole one.
 // us, grid -> flat: 16 rows x 8 kv heads of 4K-64K tokens 472 -> 422, 64 x 1 of 32K (groups of 8) 228 -> 218, 8 x 8 of 4K-16K 94 -> 80 (a balanced launch before).
 // FLAT_EXTRA 24 / 36 / 48: 16 x 8 421 / 422 / 424, 12 x 8 of 500-6000 - / 43.0 / 44.5, 64 x 1 - / 218 / 216, 64 x 8 of 100-400 40.1 / 41.4 / 42.5.
 constexpr int FLAT_EXTRA = 36;
 struct FlatWalk {
-  int share, lo, hi;                                  // of the CTA
+  int share, lo, hi;                                  // of the CTA; share < 0: the pairs are in -share equal pieces each
   int row, kvh, at, tiles;                            // the pair that is looked at next: its first place on the line, its tiles
   int pair, range[2], split, ns;                      // the piece found: pair = row * n_kv + kvh (below zero: no more), its first tile and how many, which of the pair's pieces
 };
 // Executed by one warp; every lane knows the same.
-template <class F> __device__ __forceinline__ void flat_start(FlatWalk& f, int B, int n_kv, int cta, int ctas, int lane, const F& tiles_of) {
-  u32 total = 0u;
-  for (int r0 = 0; r0 < B; r0 += 32) total += __reduce_add_sync(FULLM, r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + tiles_of(r0 + lane))) : 0u);
+// first32: where the first 32 rows' tiles are left for flat_next, which would wait for their loads again.
+template <class F> __device__ __forceinline__ void flat_start(FlatWalk& f, int B, int n_kv, int cta, int ctas, int lane, int* first32, const F& tiles_of) {
+  u32 total = 0u, longest = 0u;
+  for (int r0 = 0; r0 < B; r0 += 32) {
+    const int t = r0 + lane < B ? tiles_of(r0 + lane) : 0;
+    if (r0 == 0) first32[lane] = t;
+    total += __reduce_add_sync(FULLM, r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + t)) : 0u);
+    longest = max(longest, __reduce_max_sync(FULLM, (u32)t));
+  }
   f.share = (int)((total + ctas - 1) / ctas);
+  f.row = 0; f.pair = 0;
+  const u32 k = (u32)ctas / (u32)(B * n_kv);
+  if (k && (longest + k - 1) / k <= (u32)f.share) { f.share = -(int)k; return; }
   f.lo = (int)min((long)cta * f.share, (long)total); f.hi = (int)min((long)f.lo + f.share, (long)total);
   f.row = B; f.kvh = 0; f.at = 0; f.tiles = 0; f.pair = 0;
   u32 before = 0u;
   for (int r0 = 0; r0 < B && f.lo < f.hi; r0 += 32) {
-    const int t = r0 + lane < B ? tiles_of(r0 + lane) : 0;
+    const int t = r0 == 0 ? first32[lane] : r0 + lane < B ? tiles_of(r0 + lane) : 0;
     const u32 own = r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + t)) : 0u;
     u32 inc = own;
     scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8); scan_step(inc, 16);
@@ -412,8 +422,18 @@ template <class F> __device__ __forceinline__ void flat_start(FlatWalk& f, int B
     before += __shfl_sync(FULLM, inc, 31);
   }
 }
-template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int cta, const F& tiles_of) {
+template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int cta, const int* first32, const F& tiles_of_far) {
+  const auto tiles_of = [&](int row) { return row < 32 ? first32[row] : tiles_of_far(row); };
   f.pair = -1;
+  if (f.share < 0) {
+    const int k = -f.share, pair = cta / k;
+    if (f.row < B && pair < B * n_kv) {
+      const int t = tiles_of(pair / n_kv), chunk = (t + k - 1) / k;
+      f.pair = pair; f.split = cta - pair * k; f.ns = k; f.range[0] = min(f.split * chunk, t); f.range[1] = min(chunk, t - f.range[0]);
+    }
+    f.row = B;
+    return;
+  }
   while (f.row < B && f.pair < 0) {
     const int first = f.at + FLAT_EXTRA - (f.tiles > 0 ? 0 : 1), last = first + max(f.tiles, 1) - 1;
     if (first >= f.hi) return;
@@ -436,6 +456,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last, s_split, s_ns, s_tail, s_esc[6];        // (from s_split on: not needed inside the main loop, whose registers are all taken)
   __shared__ FlatWalk s_flat;
+  __shared__ int s_tiles[FLAT ? 32 : 1];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
@@ -489,7 +510,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   };
   if (FLAT && warp == 0) {
     FlatWalk f;
-    flat_start(f, p.B, p.n_kv, blockIdx.x, gridDim.x, lane, tiles_of);
+    flat_start(f, p.B, p.n_kv, blockIdx.x, gridDim.x, lane, s_tiles, tiles_of);
     if (lane == 0) s_flat = f;
     __syncwarp();
   }
@@ -498,7 +519,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (warp == 0) {
       FlatWalk f = s_flat;
       __syncwarp();
-      flat_next(f, p.B, p.n_kv, blockIdx.x, tiles_of);
+      flat_next(f, p.B, p.n_kv, blockIdx.x, s_tiles, tiles_of);
       if (lane == 0) { s_flat = f; s_split = f.split; s_ns = f.ns; }
     }
     // the ring begins again (every copy of the piece before has landed, and its last waits are behind the barrier at the end of the loop)
@@ -809,29 +830,60 @@ constexpr int T256_BASES = ADDEND_BYTES + SEGTAB_BYTES, T256_META = T256_BASES +
 constexpr int T256_SEG = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SEG + ATT_WARPS * SEG256_BYTES;
 constexpr int STAGE256_BYTES = 16 + 2 * PSLOT, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
 constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;          // (an escape segment is read as whole words)
-static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 64 <= 232448, "one CTA per SM");
+static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 208 <= 232448, "one CTA per SM");
 
-template <int NSET>
+// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.7 -> 26.8 us, 20 x 8 of up to 3K 97 -> 74 (a grid before, rows as they come).
+template <int NSET, bool FLAT>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last;
-  const int bh = blockIdx.x, split = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  __shared__ FlatWalk s_flat;
+  __shared__ int s_tiles[FLAT ? 32 : 1];
+  const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);
   const int hf = warp & 1, pair = warp >> 1;
-  const int b = bh / p.n_kv, kvh = bh % p.n_kv, G = p.G, NT = 4 * p.n_kv;    // p.n_kv = 256-dim kv heads; NT tile slots per block
+  const int G = p.G, NT = 4 * p.n_kv;                // p.n_kv = 256-dim kv heads; NT tile slots per block
   const int ring = T256_RING + warp * WARP256_BYTES;
   const u32 smem_s = (u32)__cvta_generic_to_shared(smem), ring_s = smem_s + ring;
   if (tid < 256) fill_attn_tables(smem, tid);
-  if (tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
+  if (!FLAT && tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
   if (lane == 0) {
     mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
+  auto tiles_of = [&](int row) -> int { return max((p.seq_len[row] + 15) >> 4, 0); };
+  if (FLAT && warp == 0) {
+    FlatWalk f;
+    flat_start(f, p.B, p.n_kv, blockIdx.x, gridDim.x, lane, s_tiles, tiles_of);
+    if (lane == 0) s_flat = f;
+    __syncwarp();
+  }
+  int bh = blockIdx.x, split = blockIdx.y, NS = p.nsplit;
+  do {
+  if (FLAT) {                                        // the next piece, with the ring and the pairs' words as they were at first
+    if (warp == 0) {
+      FlatWalk f = s_flat;
+      __syncwarp();
+      flat_next(f, p.B, p.n_kv, blockIdx.x, s_tiles, tiles_of);
+      if (lane == 0) s_flat = f;
+    }
+    if (tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
+    if (lane == 0) {
+      asm volatile("mbarrier.inval.shared::cta.b64 [%0];\nmbarrier.inval.shared::cta.b64 [%1];\n" ::"r"(ring_s), "r"(ring_s + STAGE256_BYTES) : "memory");
+      mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // the ring was written by the merges of the piece before
+    __syncthreads();
+    bh = __shfl_sync(FULLM, s_flat.pair, 0); split = __shfl_sync(FULLM, s_flat.split, 0); NS = __shfl_sync(FULLM, s_flat.ns, 0);
+    if (bh < 0) return;
+  }
+  int b = bh / p.n_kv, kvh = bh % p.n_kv;
   const int S = __shfl_sync(FULLM, p.seq_len[b], 0);
-  const int ntiles = (S + 15) >> 4, chunk = (ntiles + p.nsplit - 1) / p.nsplit;
-  const int tlo = min(split * chunk, ntiles), n = min(chunk, ntiles - tlo);
+  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS;
+  const int tlo = FLAT ? __shfl_sync(FULLM, s_flat.range[0], 0) : min(split * chunk, ntiles), n = FLAT ? __shfl_sync(FULLM, s_flat.range[1], 0) : min(chunk, ntiles - tlo);
   int* const ctl_pair = reinterpret_cast<int*>(smem + T256_CTL + pair * (2 * CTL_BYTES));
   const int4* meta_s = reinterpret_cast<const int4*>(smem + T256_META);        // per tile: mode-table entries of {K, V} of half 0, of half 1
   auto slot_of = [&](int i) { return p.bt[(long)b * p.bt_stride + tlo + i] * NT + 4 * kvh; };
@@ -913,11 +965,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     cur = nxt; stg ^= 1; it = t1;
     __syncwarp();                                      // every lane has read this stage before its next copies are issued
   }
+  if (FLAT) {                                        // (not kept in registers across the main loop)
+    bh = __shfl_sync(FULLM, s_flat.pair, 0); split = __shfl_sync(FULLM, s_flat.split, 0); NS = __shfl_sync(FULLM, s_flat.ns, 0);
+    b = bh / p.n_kv; kvh = bh % p.n_kv;
+  }
   // ---- merge the warps of the CTA, half by half: one partial per virtual head (2 * query head + half)
-  if (__syncthreads_or(sum_warp(A))) sum_exact<true, true>(p, smem + T256_RING, bh, split, p.nsplit);
+  if (__syncthreads_or(sum_warp(A))) sum_exact<true, true>(p, smem + T256_RING, bh, split, NS, FLAT ? s_flat.range : nullptr);
   else stage_warp(A, smem + T256_RING, G, warp, lane);
   __syncthreads();
-  const int d = tid & 127, NS = p.nsplit;
+  const int d = tid & 127;
   const long row0 = 2 * ((long)b * p.n_q + kvh * G);
   auto deliver = [&](long row, float L, float Ac) {
     const float v = L > 0.f ? Ac / L : 0.f;
@@ -936,16 +992,20 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (vg >= 2 * G) continue;
     if (NS == 1) deliver(row0 + vg, Lc[i], Ac[i]);
     else {
-      const long pidx = (row0 + vg) * NS + split;
+      const long pidx = FLAT ? (long)(blockIdx.x + bh) * 2 * G + vg : (row0 + vg) * NS + split;
       if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
       p.pa[pidx * D + d] = Ac[i];
     }
   }
-  if (NS == 1 || !last_split(p.counters + bh, NS, &s_last)) return;
-  for (int first = 0; first < 2 * G; first += 8) {
+  const bool last = NS > 1 && last_split(p.counters + bh, NS, &s_last);
+  if (!FLAT && !last) return;
+  for (int first = 0; last && first < 2 * G; first += 8) {
     __syncthreads();                                   // the area is used again
-    merge_splits<8>(p, smem + T256_RING, (row0 + first) * NS, NS, 1, min(8, 2 * G - first), NS, [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
+    merge_splits<8>(p, smem + T256_RING, FLAT ? (long)(blockIdx.x - split + bh) * 2 * G + first : (row0 + first) * NS, FLAT ? 1 : NS, FLAT ? 2 * G : 1, min(8, 2 * G - first), NS,
+                    [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
   }
+  if (FLAT) __syncthreads();                         // the shared memory is used again
+  } while (FLAT);
 }
 
 // Second half of the cross-GPU exchange as a launch of its own (the attention kernel was launched push-only): wait until
@@ -1099,7 +1159,8 @@ static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
 }
 template <int NSET>
 static int launch_attn256(const AttnParams& p, cudaStream_t st) {
-  return launch_big<paged256_attn_kernel<NSET>>(p, dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit), ATT256_SMEM, st);
+  if (p.flat) return launch_big<paged256_attn_kernel<NSET, true>>(p, dim3((unsigned)p.flat), ATT256_SMEM, st);
+  return launch_big<paged256_attn_kernel<NSET, false>>(p, dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit), ATT256_SMEM, st);
 }
 template <bool PAGED, bool DUMP>
 static int launch_attn(const AttnParams& p, cudaStream_t st) {
@@ -1316,9 +1377,9 @@ extern "C" int gaac_paged_decode_attn_flat(const gaac_paged* st, const int32_t* 
   return paged_attn(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, 1, 0, ctas, workspace, workspace_bytes, out_bf16, out_f32, nullptr, nullptr, 0, stream);
 }
 
-extern "C" int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
-                                         int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
-                                         void* out_bf16, float* out_f32, void* stream) {
+static int paged_attn256(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                         int B, int n_q, float scale, int nsplit, int flat, void* workspace, size_t workspace_bytes,
+                         void* out_bf16, float* out_f32, void* stream) {
   if (!st || !bt || !seq_lens || !q_bf16 || !out_bf16 || !st->buf || !st->raw || !st->mt || !st->b3k || !st->b4k || !st->b3v || !st->b4v) return GAAC_E_ARG;
   if (B <= 0 || n_q <= 0 || st->n_kv <= 0 || nsplit <= 0 || nsplit > 1024 || bt_stride <= 0) return GAAC_E_ARG;
   if (st->n_kv % 2) return GAAC_E_UNSUPPORTED;                                // half-heads come in pairs
@@ -1329,9 +1390,22 @@ extern "C" int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt
   p.buf = st->buf; p.raw = (const uint16_t*)st->raw; p.mt = st->mt; p.bt = bt; p.bt_stride = bt_stride; p.TS = st->TS; p.ovf_slot = st->ovf_slot;
   p.b3k = st->b3k; p.b4k = st->b4k; p.b3v = st->b3v; p.b4v = st->b4v; p.seq_len = seq_lens;
   p.q = (const uint16_t*)q_bf16; p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.G = n_q / n_kv; p.scale_log2 = scale * LOG2E; p.nsplit = nsplit;
-  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32;
-  if (int e = carve_workspace(workspace, workspace_bytes, B, 2 * n_q, nsplit, p)) return e;     // one partial per (query head, half)
+  p.out = (uint16_t*)out_bf16; p.out_f32 = out_f32; p.flat = flat;
+  if (int e = carve_workspace(workspace, workspace_bytes, B, 2 * n_q, flat ? flat_splits(B, n_kv, flat) : nsplit, p)) return e;     // one partial per (query head, half)
   return p.G <= 4 ? launch_attn256<1>(p, (cudaStream_t)stream) : launch_attn256<2>(p, (cudaStream_t)stream);
+}
+
+extern "C" int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                         int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
+                                         void* out_bf16, float* out_f32, void* stream) {
+  return paged_attn256(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, nsplit, 0, workspace, workspace_bytes, out_bf16, out_f32, stream);
+}
+
+extern "C" int gaac_paged_decode_attn256_flat(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                              int B, int n_q, float scale, int ctas, void* workspace, size_t workspace_bytes,
+                                              void* out_bf16, float* out_f32, void* stream) {
+  if (!st || st->n_kv <= 0 || st->n_kv % 2 || bt_stride <= 0 || bt_stride > (1LL << 32) || !flat_ok(B, st->n_kv / 2, ctas, bt_stride * T)) return GAAC_E_ARG;
+  return paged_attn256(st, bt, bt_stride, seq_lens, q_bf16, B, n_q, scale, 1, ctas, workspace, workspace_bytes, out_bf16, out_f32, stream);
 }
 
 // ---- test hooks: the same kernels, instantiated so that every rebuilt BF16 fragment is also written to memory

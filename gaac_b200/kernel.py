@@ -126,7 +126,8 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
     first.  us, other form -> flat:
       grids of several waves: 64 rows x 1 kv head, 32K tokens 228 -> 218;  16 x 8, 4K-64K 472 -> 422;  40 x 4, 2K-6K 95 -> 80;  20 x 8, 2K-3K 71 -> 56;  64 x 8, up to 4200
         124 -> 120.  Short rows lose: 32 x 8, 20-2000 tokens 49 -> 56;  64 x 8, 100-400 33 -> 41;  24 x 8, 64-600 17 -> 24
-      one wave that leaves SMs idle: 64 x 2, 4K-8K 116 -> 101;  64 x 1, 8K-16K 118 -> 91.  An eighth or less idle loses if all rows are as long: 18 x 8, 8K 111 -> 119
+      one wave: 64 x 2, 4K-8K 116 -> 101;  64 x 1, 8K-16K 118 -> 91;  37 x 4, up to 8K 108 -> 71;  35 x 1, up to 12K 47 -> 33.  A full wave of equal rows pays for the walk: 37 x 4,
+        8K 110.9 -> 114.1
       shares of units, which come in whole ones: a fifth of them or more for the rows' first units 8 x 8, 4K-16K 94 -> 80;  4 x 8, 20K-32K 104 -> 95;  5 x 8, up to 9K 31.7 ->
         30.6;  fewer, 16 x 1 36 -> 39, 8 x 1 36.4 -> 36.9;  more than four query heads per kv head, 6 x 8 61 -> 64."""
     rows, tiles = B * n_kv, -(-S // 16)
@@ -134,8 +135,18 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
         return 0
     if units:
         return sm_count if group <= 4 and 5 * B >= units else 0
-    ctas = rows * nsplit
-    return 0 if 7 * sm_count < 8 * ctas <= 8 * sm_count else sm_count
+    return sm_count
+
+
+@functools.lru_cache(maxsize=4096)
+def choose_flat256(B: int, n_kv: int, S: int, nsplit: int, sm_count: int = SM_COUNT_B200) -> int:
+    """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.7 -> 26.8;  20 x 8, up to 3K 97 -> 74;  32 x 2, up
+    to 4K 57 -> 42;  6 x 2, up to 60K 129 -> 94;  2 x 8 of 1000 31 -> 13;  9 x 4, up to 1500 24.5 -> 19.3;  30 x 4, up to 2K 56 -> 48.  Many short rows lose: 32 x 4, up to 1000
+    31 -> 34.5;  32 x 8 52.8 -> 54.8.  A full wave of equal rows pays for the walk: 12 x 4 of 4000 46.3 -> 48.5;  one sequence has nothing to gain: 1 x 4 of 8K 18.4 -> 18.6."""
+    rows, tiles = B * n_kv, -(-S // 16)
+    if B <= 1 or rows * (tiles + 64) >= 1 << 30:
+        return 0
+    return sm_count if tiles >= (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 160) else 0
 
 
 def _flat_splits(B: int, n_kv: int, ctas: int) -> int:

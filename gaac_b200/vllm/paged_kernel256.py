@@ -9,7 +9,7 @@ dimensions of its half of V.
 from __future__ import annotations
 import torch
 from .. import _lib
-from ..kernel import workspace, choose_nsplit_sm100
+from ..kernel import workspace, choose_flat256, choose_nsplit_sm100, _flat_splits
 
 
 def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, nsplit=None, scale=None, out_f32=None):
@@ -22,12 +22,17 @@ def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv,
     if not (1 <= G <= 8 and G * n_kv == n_q): raise RuntimeError("GQA group size must be 1..8")
     if TS % 16: raise RuntimeError("tile stride must be a multiple of 16")
     if not q.is_cuda: raise RuntimeError("gaac_b200 attention needs CUDA tensors: there is no CPU path")
-    if nsplit is None: nsplit = choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)
+    flat = 0
+    if nsplit is None:
+        nsplit = choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)
+        flat = choose_flat256(B, n_kv, bt.shape[1] * 16, nsplit) if B * n_kv * (bt.stride(0) + 64) < 1 << 30 else 0
+        if flat: nsplit = _flat_splits(B, n_kv, flat)                                          # what the workspace must have room for
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), 2 * n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, 2 * n_q, nsplit, stream)
-    _lib.check(_lib.lib().gaac_paged_decode_attn256(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q,
-                                                    float(scale) if scale is not None else 256 ** -0.5, int(nsplit), ws.data_ptr(), ws.numel(),
+    lib = _lib.lib()
+    _lib.check((lib.gaac_paged_decode_attn256_flat if flat else lib.gaac_paged_decode_attn256)(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q,
+                                                    float(scale) if scale is not None else 256 ** -0.5, flat or int(nsplit), ws.data_ptr(), ws.numel(),
                                                     out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_paged_decode_attn256")
     return out

@@ -355,6 +355,11 @@ int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt, int64_t b
                               int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
                               void* out_bf16, float* out_f32, void* stream);
 
+/* gaac_paged_decode_attn256 as one wave of CTAs, as in gaac_decode_attn_flat (n_kv: 256-dim kv heads; workspace for 2 * n_q query heads). */
+int gaac_paged_decode_attn256_flat(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
+                                   int B, int n_q, float scale, int ctas, void* workspace, size_t workspace_bytes,
+                                   void* out_bf16, float* out_f32, void* stream);
+
 /* ---------------------------------------------------------------------------------------------- test hooks */
 
 /* gaac_decode_attn / gaac_paged_decode_attn compiled so that every BF16 fragment word the kernel rebuilds on its way to the

@@ -22,7 +22,7 @@ def test_choose_flat_bounds():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [0, 5, 16, 1000, 17]), (1, 8, [700]), (3, 5, [3, 33, 64, 65, 900, 1, 0, 300, 15, 16, 31, 47, 48, 49] * 5)])
+@pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [0, 5, 16, 1000, 17]), (1, 8, [700]), (2, 1, [333] * 6), (3, 5, [3, 33, 64, 65, 900, 1, 0, 300, 15, 16, 31, 47, 48, 49] * 5)])
 def test_slots_flat(monkeypatch, n_kv, G, lens):
     import torch
     import gaac_b200.kv_cache as kvc
@@ -92,3 +92,29 @@ def test_flat_pieces_with_infinite_elements(monkeypatch):
         assert torch.isinf(got[:, :, 5]).all() and torch.isfinite(got[:, :, :5]).all() and torch.isfinite(got[:, :, 6:]).all()
         keep = [c for c in range(128) if c != 5]
         assert torch.allclose(got[:, :, keep], want[:, :, keep], rtol=2 ** -7, atol=1e-3)        # BF16 results of the same sums in another order
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [16, 37, 333, 1000, 5]), (1, 8, [1500, 1]), (3, 1, [1, 260] * 17), (1, 6, [900])])
+def test_paged256_flat(monkeypatch, n_kv, G, lens):
+    import torch
+    import gaac_b200.vllm.paged_kernel256 as pk
+    blocks = sum(-(-x // 16) for x in lens)
+    st, buf, bt, ks, vs = _build_paged(lens, 2 * n_kv, blocks + 4, seed=n_kv, adversarial_every=5, raw_tiles=4 * n_kv * blocks)
+    assert int(st.err) == 0
+    B, n_q = len(lens), n_kv * G
+    q16 = O.f32_to_bf16((np.random.default_rng(1).standard_normal((B, n_q, 256)) * 0.3).astype(np.float32))
+    lens_now = list(lens)
+    if B > 1: lens_now[B // 2] = 0                                              # a row without tokens between others
+    sl = torch.tensor(lens_now, dtype=torch.int32, device="cuda")
+    for ctas in (1, 3, 37, 148, 148, 1000):
+        monkeypatch.setattr(pk, "choose_flat256", lambda *a, n=ctas: n)
+        o32 = torch.empty(B, n_q, 256, dtype=torch.float32, device="cuda")
+        out = torch.full((B, n_q * 256), float("nan"), dtype=torch.bfloat16, device="cuda")
+        pk.paged_attention256(to_bf16_cuda(q16), out, buf, st.raw, st.mt, bt, sl, st.bases, st.TS, n_q, n_kv, out_f32=o32)
+        for b in range(B):
+            L = lens_now[b]
+            if L == 0:
+                assert not out[b].any(), (b, ctas)
+            else:
+                assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b].reshape(-1, n_kv, 256)[:L], vs[b].reshape(-1, n_kv, 256)[:L], 256 ** -0.5, (b, ctas))
