@@ -243,18 +243,25 @@ __device__ __forceinline__ void load_32(u32* w, const void* p) {
   asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
 }
 
-// Rebuild a compressed tile into ws.xs (natural channel order, bf16 bits).  sm / cd / fl: tile-relative sources in global memory; esc: the tile's first
-// escape byte in global memory.  Everything but the escape bytes is asked for at once; those are fetched with one coalesced load as soon as the tags
-// say how many there are (a load per group waited for the one before it at every raw group's branch).  The fragments go to shared
-// memory by stmatrix.
+// A compressed tile on its way: one lane's words as they lie in memory.
+template <int KIND_V> struct TileWords {
+  static constexpr int SEGS = KIND_V ? 4 : 2;
+  u32 sm[16], cd[6], fl[SEGS];
+  u32 esc; int n_esc; const uint8_t* esc_src;         // word `lane` of the escape bytes, from the 4-byte boundary at or below the first; how many bytes were asked for
+};
+// Ask for a tile.  sm / cd / fl: tile-relative sources in global memory; esc_src: the tile's first escape byte.  n_esc: bytes from there on that may be read and are
+// likely to be the tile's (0: not known), so that they travel with the rest instead of behind the tags.
 template <int KIND_V>
-__device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, const uint8_t* sm_src, const uint8_t* cd_src, const uint8_t* fl_src, const uint8_t* esc_src,
-                                                 const WarpView& w, int lane) {
-  const int j = lane & 3, r = lane >> 2;
-  constexpr int STEP = KIND_V ? 32 : 1024, SEGS = KIND_V ? 4 : 2;
-  u32 sm[16], cd[6], tags, total, none, pos[SEGS];
+__device__ __forceinline__ void load_tile_words(TileWords<KIND_V>& tw, const uint8_t* sm_src, const uint8_t* cd_src, const uint8_t* fl_src, const uint8_t* esc_src, int n_esc, int lane) {
+  const int j = lane & 3;
+  constexpr int STEP = KIND_V ? 32 : 1024, SEGS = TileWords<KIND_V>::SEGS;
+  u32 (&sm)[16] = tw.sm; u32 (&cd)[6] = tw.cd; u32 (&fl)[SEGS] = tw.fl;
   const uint8_t* s0 = sm_src + (KIND_V ? 64 : 32) * lane;
-  u32 fl[SEGS];
+  {
+    const int ofs = (int)(reinterpret_cast<uintptr_t>(esc_src) & 3);
+    tw.esc_src = esc_src; tw.n_esc = max(min(n_esc, 128 - ofs), 0); tw.esc = 0u;
+    if (tw.n_esc > 0 && 4 * lane < tw.n_esc + ofs) tw.esc = reinterpret_cast<const u32*>(esc_src - ofs)[lane];
+  }
   if (!KIND_V) { fl[0] = fl_src[lane]; fl[1] = fl_src[32 + lane]; }                            // byte j of row r's tag word is byte `lane` of the octet's 32
   else {
     const u32* f = reinterpret_cast<const u32*>(fl_src);
@@ -272,12 +279,26 @@ __device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, const uint8_
   if (!KIND_V) {
 #pragma unroll
     for (int i = 0; i < 6; i++) cd[i] = reinterpret_cast<const u32*>(cd_src + (i / 3) * 384 + 12 * lane)[i % 3];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 3; i++) { const uint2 c = reinterpret_cast<const uint2*>(cd_src + 24 * lane)[i]; cd[2 * i] = c.x; cd[2 * i + 1] = c.y; }
+  }
+}
+// Rebuild the tile into ws.xs (natural channel order, bf16 bits).  The escape bytes that did not come with the rest are fetched with one coalesced load as soon as the
+// tags say how many there are (a load per group waited for the one before it at every raw group's branch).  The fragments go to shared memory by
+// stmatrix.
+template <int KIND_V>
+__device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, TileWords<KIND_V>& tw, const WarpView& w, int lane) {
+  const int j = lane & 3, r = lane >> 2;
+  constexpr int SEGS = TileWords<KIND_V>::SEGS;
+  u32 tags, total, none, pos[SEGS];
+  u32 (&sm)[16] = tw.sm; u32 (&cd)[6] = tw.cd; u32 (&fl)[SEGS] = tw.fl;
+  const uint8_t* esc_src = tw.esc_src;
+  if (!KIND_V) {
     u32 kp, nv[2];
     tile_positions<true, false>(fl[0], fl[1], 0u, 0u, 0u, 0u, j, kp, total, nv, none);
     tags = fl[0] | (fl[1] << 8); pos[0] = kp & 0xFFFFu; pos[1] = kp >> 16;
   } else {
-#pragma unroll
-    for (int i = 0; i < 3; i++) { const uint2 c = reinterpret_cast<const uint2*>(cd_src + 24 * lane)[i]; cd[2 * i] = c.x; cd[2 * i + 1] = c.y; }
 #pragma unroll
     for (int t = 0; t < SEGS; t++) fl[t] = (fl[t] >> (4 * r)) & 15u;
     u32 vp[2];
@@ -291,7 +312,9 @@ __device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, const uint8_
   __syncwarp();                                      // the scratch is no longer in use
   if (n <= ESC_STAGE) {
     const u32* g = reinterpret_cast<const u32*>(esc_src - ofs);
-    for (int i = lane; 4 * i < (n > 0 ? n + ofs : 0); i += 32) ws.esc[i] = g[i];
+    const int have = tw.n_esc > 0 ? (tw.n_esc + ofs + 3) >> 2 : 0;                           // words that came with the rest
+    if (lane < have) ws.esc[lane] = tw.esc;
+    for (int i = have + lane; 4 * i < (n > 0 ? n + ofs : 0); i += 32) ws.esc[i] = g[i];
     esc = reinterpret_cast<const uint8_t*>(ws.esc) + ofs;
   }
   __syncwarp();
