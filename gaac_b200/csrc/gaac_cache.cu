@@ -191,8 +191,9 @@ __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restric
 
 // One warp per (entry, tile slot); the CTA's four entries have the slot index t = 2*kvh + kind in common, and with it the tables.
 // grid = (ceil(P / 4), 2*n_kv).
-// Bound by its chain of loads (entry, mode table, tile, escape bytes behind the tags, then the stores): the first three are asked for before the tables are made, the escape bytes
-// with the tile, 128 bytes of its slot.  384 blocks of 16 tiles decoded and 1500 tokens stored: 19.0 -> 18.1 us.
+// Bound by its chain of loads (entry, mode table, tile, escape bytes behind the tags, then the stores): the first three are asked for before the tables are made.  384
+// blocks of 16 tiles decoded and 1500 tokens stored: 24.7 -> 24.6 us.  128 bytes of the slot's escape bytes asked for with the tile: 19.0 -> 18.1 with everything in L2,
+// but 24.4 and nothing gained from memory, where most of them are not the tile's.
 constexpr int PDEC_WARPS = 4;
 struct PagedDecodeParams { gaac_paged st; const int* pairs; int P; uint16_t *sk, *sv; long row_stride; };
 
@@ -209,7 +210,7 @@ __device__ __forceinline__ void decode_blocks_cta(DecodeScratch* scratch, Decode
     const long pt = (long)p.pairs[3 * e] * NT + t;
     const uint8_t* base = st.buf + pt * st.TS;
     m = st.mt[pt];
-    if (m >= 0) load_tile_words<KIND_V>(tw, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, base + SLOT_OVF_OFF, st.ovf_slot & ~3, lane);
+    if (m >= 0) load_tile_words<KIND_V>(tw, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, base + SLOT_OVF_OFF, 0, lane);
   }
   const WarpView w = fill_decode_tables<KIND_V>(tables, (KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D);
   __syncthreads();
