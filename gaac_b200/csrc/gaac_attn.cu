@@ -291,7 +291,8 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
     S = sl < 0 ? 0 : p.seq_len ? p.seq_len[ch] : p.S_uniform;
     TL = sl >= 0 && p.tail_len && split == NS - 1 ? p.tail_len[ch] : 0;
   }
-  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS, tlo = range ? range[0] : min(split * chunk, ntiles), n = range ? range[1] : min(chunk, ntiles - tlo);
+  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS, tlo = range ? min(range[0], ntiles) : min(split * chunk, ntiles);
+  const int n = range ? (split == NS - 1 ? ntiles - tlo : min(range[1], ntiles - tlo)) : min(chunk, ntiles - tlo);                  // (as the main loop takes it)
   float m[8], l[8], acc[8][4];
 #pragma unroll
   for (int h = 0; h < 8; h++) { m[h] = -CUDART_INF_F; l[h] = acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.f; }

@@ -95,6 +95,80 @@ def test_flat_pieces_with_infinite_elements(monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n_kv,G", [(3, 4), (2, 6)])
+@pytest.mark.parametrize("where", [None, 5, -3])
+def test_heads_of_different_lengths(monkeypatch, n_kv, G, where):
+    """A slot's first head is 64 and 320 tokens shorter, or 208 longer, than the others (a refused append leaves one head's counters alone); where: a row of the LAST head
+    that holds an infinite element, which its CTA's repeat of the piece has to find as well."""
+    import torch
+    import gaac_b200.kv_cache as kvc
+    cache = kvc.CompressedKVCache(n_slots=3, n_kv=n_kv, capacity=1024, bases=None)
+    full, first, rest, hist = [640, 960, 800], [576, 640, 800], [640, 960, 592], []
+    for s, L in enumerate(full):
+        k, v = (np.ascontiguousarray(O.kv_like(n_kv, L, 9 * s + i, outliers=0.0).transpose(1, 0, 2)) for i in (1, 2))
+        if where is not None: v[where % rest[s], n_kv - 1, 5] = 0x7F80
+        cache.prefill(s, to_bf16_cuda(k), to_bf16_cuda(v))
+        cache.S[s * n_kv:(s + 1) * n_kv] = torch.tensor([first[s]] + [rest[s]] * (n_kv - 1))
+        hist.append((k, v))
+    q16 = O.f32_to_bf16((np.random.default_rng(n_kv).standard_normal((3, n_kv * G, 128)) * 0.1).astype(np.float32))
+    slots = torch.arange(3, dtype=torch.int32, device="cuda")
+    for ctas in (0, 1, 4, 37, 148):                                             # 0: the grid
+        monkeypatch.setattr(kvc, "choose_flat", lambda *a, n=ctas: n)
+        o32 = torch.empty(3, n_kv * G, 128, dtype=torch.float32, device="cuda")
+        cache.attention(to_bf16_cuda(q16), slots, SCALE, max_len=1000, nsplit=None if ctas else 2, out_f32=o32)
+        for b, (k, v) in enumerate(hist):
+            for h in range(n_kv):
+                L = rest[b] if h else first[b]
+                got, vh = o32[b, h * G:(h + 1) * G].cpu().numpy(), v[:L, h:h + 1].copy()
+                if where is not None and h == n_kv - 1:
+                    assert np.isposinf(got[:, 5]).all(), (b, h, ctas)
+                    vh[where % rest[b], 0, 5] = 0; got[:, 5] = 0
+                    ref = O.attention_ref(q16[b, h * G:(h + 1) * G], k[:L, h:h + 1], vh, SCALE)
+                    got[:, 5] = ref[:, 5]
+                assert_attention_close(got, q16[b, h * G:(h + 1) * G], k[:L, h:h + 1], vh, SCALE, (b, h, ctas))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("G", [4, 7])
+def test_paged_pieces_with_infinite_elements(monkeypatch, wide, G):
+    """The repeat of a piece in the paged forms: every channel without an infinite element against the fp64 oracle."""
+    import torch
+    import gaac_b200.vllm.paged_kernel as pk, gaac_b200.vllm.paged_kernel256 as pk256
+    from gaac_b200.vllm.store import LayerState, OVF_OFF
+    dim, heads, lens = (256, 2, [700, 33, 1200]) if wide else (128, 1, [700, 33, 1200])
+    need = [-(-L // 16) for L in lens]
+    ks, vs = ([np.ascontiguousarray(O.kv_like(heads, L, 5 * i + s, outliers=0.0).transpose(1, 0, 2)) for i, L in enumerate(lens)] for s in (1, 2))
+    bases = {}
+    for kind, xs in (("k", ks), ("v", vs)):
+        bases[kind + "3"], bases[kind + "4"] = (torch.from_numpy(b) for b in O.calibrate(np.ascontiguousarray(xs[2].transpose(1, 0, 2)), heads))
+    for i, L in enumerate(lens):
+        vs[i][L - 1, 0, 5] = vs[i][L // 2, heads - 1, 9] = 0x7F80
+    st = LayerState(sum(need), heads, raw_tiles=2 * sum(need) * heads, bases=bases, ovf_slot=128, device="cuda")
+    buf = torch.zeros(sum(need) * 2 * heads * (OVF_OFF + 128), dtype=torch.uint8, device="cuda")
+    bt, at = np.zeros((3, max(need)), np.int32), 0
+    for i, L in enumerate(lens):
+        bt[i, :need[i]] = np.arange(at, at + need[i]); at += need[i]
+        ent = torch.tensor([[bt[i, t], 16 * t, 0, min(16, L - 16 * t)] for t in range(need[i])], dtype=torch.int32, device="cuda")
+        st.store(to_bf16_cuda(ks[i]), to_bf16_cuda(vs[i]), buf, ent, torch.empty(need[i] * 2 * heads, dtype=torch.int32, device="cuda"))
+    assert int(st.err) == 0
+    q16 = O.f32_to_bf16((np.random.default_rng(3).standard_normal((3, G, dim)) * 0.1).astype(np.float32))
+    call = pk256.paged_attention256 if wide else pk.paged_attention
+    for ctas in (1, 4, 148):
+        monkeypatch.setattr(*((pk256, "choose_flat256") if wide else (pk, "choose_flat")), lambda *a, n=ctas: n)
+        o32 = torch.empty(3, G, dim, dtype=torch.float32, device="cuda")
+        out = torch.empty(3, G * dim, dtype=torch.bfloat16, device="cuda")
+        call(to_bf16_cuda(q16), out, buf, st.raw, st.mt, torch.from_numpy(bt).cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), st.bases, st.TS, G, 1, out_f32=o32)
+        for b, L in enumerate(lens):
+            k, v, got = ks[b].reshape(L, 1, dim), vs[b].reshape(L, 1, dim), o32[b].cpu().numpy()
+            hit = ((v & 0x7FFF) == 0x7F80).any((0, 1))
+            assert np.isposinf(got[:, hit]).all() and hit.sum() == 2, (b, ctas)
+            v = np.where((v & 0x7FFF) == 0x7F80, np.uint16(0), v)
+            got[:, hit] = O.attention_ref(q16[b], k, v, dim ** -0.5)[:, hit]
+            assert_attention_close(got, q16[b], k, v, dim ** -0.5, (b, ctas))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [16, 37, 333, 1000, 5]), (1, 8, [1500, 1]), (3, 1, [1, 260] * 17), (1, 6, [900])])
 def test_paged256_flat(monkeypatch, n_kv, G, lens):
     import torch
