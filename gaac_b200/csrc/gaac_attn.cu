@@ -468,12 +468,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // staged behind this one right away (it cannot become resident before this grid's CTAs leave their SMs).  Both instructions are no-ops
   // in a plain launch.
   if (tid < 256) fill_attn_tables(smem, tid);
-  if (tid >= 256 && tid < 256 + TPS * NSTG) reinterpret_cast<u32*>(smem + TB_USE)[tid - 256] = 0u;
-  if (lane == 0 && warp < NSTG) {                    // warp w fills stage w first
+  // Warp w fills stage w first, and clears the words of its tiles: a lane that publishes one has cleared it itself, so no other warp has to be waited for.
+  if (warp < NSTG && lane < TPS) reinterpret_cast<u32*>(smem + TB_USE)[warp * TPS + lane] = 0u;
+  if (lane == 0 && warp < NSTG) {
     mbar_init(smem_s + TB_FULL + 8 * warp, 1);
     reinterpret_cast<int*>(smem + TB_LEFT)[warp] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  __syncwarp();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
 
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if (lane == 0) { s_flat = f; s_split = f.split; s_ns = f.ns; }
     }
     // the ring begins again (every copy of the piece before has landed, and its last waits are behind the barrier at the end of the loop)
-    if (warp == ATT_WARPS - 1) reinterpret_cast<u32*>(smem + TB_USE)[lane] = 0u;
+    if (warp < NSTG && lane < TPS) reinterpret_cast<u32*>(smem + TB_USE)[warp * TPS + lane] = 0u;
     if (lane == 0 && warp < NSTG) {
       asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_s + TB_FULL + 8 * warp) : "memory");
       mbar_init(smem_s + TB_FULL + 8 * warp, 1);

@@ -63,3 +63,30 @@ def test_graphs_of_descending_batch_sizes():
             for b in (0, B - 1):
                 assert_attention_close(o32[b].cpu().numpy(), q16[b], k16, v16, 128 ** -0.5, (B, b))
         assert all(bool((t == 0x5A).all()) for t in junk)          # and no replay wrote into anybody else's memory
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,n_kv,L", [(1, 8, 40), (3, 8, 200), (40, 4, 70)])
+def test_no_wait_runs_out_in_short_launches(B, n_kv, L):
+    """Launches whose first stages are published a few cycles after the ring was cleared (grid, ranges by length, one wave): a word that was cleared late would leave its
+    tiles out and set the error word."""
+    import torch
+    from gaac_b200 import CompressedKVCache
+    from gaac_b200.kernel import workspace_error
+    k16, v16 = (np.ascontiguousarray(O.kv_like(n_kv, L, i).transpose(1, 0, 2)) for i in (1, 2))
+    cache = CompressedKVCache(n_slots=B, n_kv=n_kv, capacity=4096, bases=None)
+    for s in range(B):
+        cache.prefill(s, to_bf16_cuda(k16), to_bf16_cuda(v16), check=False)
+    q16 = O.f32_to_bf16((np.random.default_rng(0).standard_normal((B, 4 * n_kv, 128)) * 0.1).astype(np.float32))
+    q, slots = to_bf16_cuda(q16), torch.arange(B, dtype=torch.int32, device="cuda")
+    refs = {}
+    for b in {0, B - 1}:                                                        # every call is held against the oracle, on the device
+        ref, mag = O.attention_ref(q16[b], k16, v16, 128 ** -0.5, with_abs=True)
+        refs[b] = torch.from_numpy(ref).cuda(), torch.from_numpy(O.attention_bound(mag)).cuda()
+    worst = torch.zeros((), dtype=torch.float64, device="cuda")
+    for i in range(300):
+        o32 = torch.empty(B, 4 * n_kv, 128, dtype=torch.float32, device="cuda")
+        cache.attention(q, slots, 128 ** -0.5, max_len=(L, 4096, None)[i % 3], nsplit=None if i % 4 else 1, out_f32=o32)
+        for b, (ref, bound) in refs.items():
+            worst = torch.maximum(worst, ((o32[b].double() - ref).abs() / bound).max())
+    assert not workspace_error("cuda:0") and float(worst) <= 1.0
