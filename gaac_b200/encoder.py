@@ -147,7 +147,9 @@ class TileEncoder:
         head_start = torch.empty(H + 1, dtype=torch.int32, device=dev)
         x = x.contiguous()
         items = H * ntiles
-        slots = self._scratch(items * SLOT + 4 * (items + H), dev)                                # escape slots | tile sizes | head sizes
+        # escape slots | tile sizes | head sizes: of this call alone, since another one on the same encoder (a second stream, a second thread while this one waits) may
+        # run before the copy has read them
+        slots = torch.empty(items * SLOT + 4 * (items + H), dtype=torch.uint8, device=dev)
         total = torch.empty(1, dtype=torch.int32, pin_memory=True)
         L = _lib.lib(); st = _lib.stream_ptr(dev)
         p_flags, p_slots, p_off, p_hs = flags.data_ptr(), slots.data_ptr(), tile_off.data_ptr(), head_start.data_ptr()
@@ -155,6 +157,6 @@ class TileEncoder:
         _lib.check(L.gaac_encode_sized(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
                                        sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, total.data_ptr(), st), "gaac_encode_sized")
         ovf = torch.empty(total.item() + 8, dtype=torch.uint8, device=dev)
-        _lib.check(L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, 0, 0, None, st),
+        _lib.check(L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, ovf.numel(), 0, None, st),
                    "gaac_compact_copy")
         return Page(sm, cd, flags, ovf_off, ovf, head_start, tile_off, codec.base3, codec.base4, H, S, codec.n_kv, self.kind)

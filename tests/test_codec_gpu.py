@@ -160,3 +160,76 @@ def test_full_size_roundtrip_property():
         d = page_to_dict(pg)
         assert np.array_equal(d["flags"][:, :4096], ref["flags"]) and np.array_equal(d["tile_off"][:, :256], ref["tile_off"])
         assert np.array_equal(d["sm"][:, :4096 * 128], ref["sm"]) and np.array_equal(d["codes"][:, :4096 * 48], ref["codes"])
+
+
+@pytest.mark.parametrize("other", [(1, 48), (3, 700), (4, 3000)])
+def test_encodes_that_overlap_on_one_encoder(monkeypatch, other):
+    """A second encode of another size on the same encoder runs between the first one's kernels and its copy (as one of another thread does while the first waits for the
+    GPU): both Pages are right.  Then two threads, each with its own stream."""
+    import threading
+    import torch
+    from gaac_b200 import TileEncoder, Codec, _lib
+    lib, enc, n_kv = _lib.lib(), TileEncoder("k"), 1
+    codec = Codec(n_kv).calibrate(to_bf16_cuda(O.kv_like(n_kv, 512, seed=1)))
+    b3, b4 = codec.base3.cpu().numpy(), codec.base4.cpu().numpy()
+    xs = [O.kv_like(3, 700, seed=5), np.random.default_rng(1).integers(0, 65536, (*other, 128)).astype(np.uint16)]           # (random bits: the most escape bytes)
+    refs, dev = [O.encode(x, b3, b4, "k", n_kv) for x in xs], [to_bf16_cuda(x) for x in xs]
+    inner = []
+
+    class Nested:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+            if name != "gaac_compact_copy":
+                return fn
+
+            def copy(*a):
+                m.undo()                                                        # the inner call goes straight through
+                inner.append(enc.encode(codec, dev[1]))
+                return fn(*a)
+            return copy
+    nested = Nested()
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "lib", lambda: nested)
+        first = enc.encode(codec, dev[0])
+    assert_pages_equal(page_to_dict(first), refs[0])
+    assert_pages_equal(page_to_dict(inner[0]), refs[1])
+    pages = [[], []]
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                pages[i].append(enc.encode(codec, dev[i]))
+            torch.cuda.current_stream().synchronize()
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in (0, 1)]
+    for t in threads: t.start()
+    for t in threads: t.join()
+    for i in (0, 1):
+        assert len(pages[i]) == 20
+        for p in pages[i]:
+            assert_pages_equal(page_to_dict(p), refs[i])
+
+
+def test_copy_keeps_inside_its_bound():
+    """gaac_compact_copy with room for a part of the stream only: the tiles that fit are there, the bytes behind the bound are as they were, the status says so."""
+    import torch
+    from gaac_b200 import TileEncoder, Codec, _lib
+    x16 = O.kv_like(2, 640, seed=3)
+    codec = Codec(1).calibrate(to_bf16_cuda(O.kv_like(1, 512, seed=1)))
+    ref = O.encode(x16, codec.base3.cpu().numpy(), codec.base4.cpu().numpy(), "v", 1)
+    x, enc = to_bf16_cuda(x16), TileEncoder("v")
+    u8, i32 = dict(dtype=torch.uint8, device="cuda"), dict(dtype=torch.int32, device="cuda")
+    sm, cd, flags = torch.empty(2, 640 * 128, **u8), torch.empty(2, 640 * 48, **u8), torch.empty(2, 640, **i32)
+    sizes = enc.encode_tiles(x, codec.base3, codec.base4, sm, cd, flags, 640, 640, 1)
+    off, heads = enc.tile_offsets(sizes)
+    start = torch.cat([torch.zeros(1, **i32), heads.cumsum(0).int()])
+    n = int(start[-1])
+    cap = n // 2
+    ovf, status = torch.full((n + 8,), 0xA5, **u8), torch.zeros(1, **i32)
+    _lib.check(_lib.lib().gaac_compact_copy(enc._slots.data_ptr(), sizes.data_ptr(), 2, 40, start.data_ptr(), ovf.data_ptr(), off.data_ptr(), 40, None, 640, 640, None, 8, cap, 0,
+                                            status.data_ptr(), torch.cuda.current_stream().cuda_stream), "gaac_compact_copy")
+    got = ovf.cpu().numpy()
+    assert int(status) & 1 and (got[cap:] == 0xA5).all()
+    starts, ends = (ref["ovf_head_start"][:-1, None] + ref["tile_off"]).ravel(), np.r_[(ref["ovf_head_start"][:-1, None] + ref["tile_off"]).ravel()[1:], n]
+    for a, b in zip(starts, ends):
+        assert np.array_equal(got[a:b], ref["ovf"][a:b]) if b + 8 <= cap else (got[a:b] == 0xA5).all(), (a, b, cap)
