@@ -118,8 +118,14 @@ def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> in
     return min(units, B * -(-max(S, 1) // 64))
 
 
+def _flat_line(rows: int, most: int) -> bool:
+    """The places of a flat launch's line are counted in 32 bits, and the library refuses one that could be longer.  It goes by what a row MAY hold (`most` tokens: the capacity
+    of a slot, the row stride of a block table), not by what the caller says the longest row has."""
+    return rows * (-(-most // 16) + 64) < 1 << 30
+
+
 @functools.lru_cache(maxsize=4096)
-def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int = 4, sm_count: int = SM_COUNT_B200) -> int:
+def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int = 4, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
     """CTAs of a flat launch (one wave that shares the tiles of all rows and kv heads evenly), or 0 where the form that it would replace is no slower: nsplit splits per
     (row, kv head), or `units` ranges per kv head (S: tokens of the longest row, group: query heads per kv head).
     A flat launch saves what comes with the waves of a grid, and the idle end of the last one; it pays some 8 us for every piece of a row that a CTA has beyond its
@@ -131,7 +137,7 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
       shares of units, which come in whole ones: a fifth of them or more for the rows' first units 8 x 8, 4K-16K 94 -> 80;  4 x 8, 20K-32K 104 -> 95;  5 x 8, up to 9K 31.7 ->
         30.6;  fewer, 16 x 1 36 -> 39, 8 x 1 36.4 -> 36.9;  more than four query heads per kv head, 6 x 8 61 -> 64."""
     rows, tiles = B * n_kv, -(-S // 16)
-    if B <= 1 or tiles < 160 or rows * tiles < 120 * sm_count or rows * (tiles + 64) >= 1 << 30:
+    if B <= 1 or tiles < 160 or rows * tiles < 120 * sm_count or not _flat_line(rows, max(S, most)):
         return 0
     if units:
         return sm_count if group <= 4 and 5 * B >= units else 0
@@ -139,12 +145,12 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
 
 
 @functools.lru_cache(maxsize=4096)
-def choose_flat256(B: int, n_kv: int, S: int, nsplit: int, sm_count: int = SM_COUNT_B200) -> int:
+def choose_flat256(B: int, n_kv: int, S: int, nsplit: int, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
     """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.7 -> 26.8;  20 x 8, up to 3K 97 -> 74;  32 x 2, up
     to 4K 57 -> 42;  6 x 2, up to 60K 129 -> 94;  2 x 8 of 1000 31 -> 13;  9 x 4, up to 1500 24.5 -> 19.3;  30 x 4, up to 2K 56 -> 48.  Many short rows lose: 32 x 4, up to 1000
     31 -> 34.5;  32 x 8 52.8 -> 54.8.  A full wave of equal rows pays for the walk: 12 x 4 of 4000 46.3 -> 48.5;  one sequence has nothing to gain: 1 x 4 of 8K 18.4 -> 18.6."""
     rows, tiles = B * n_kv, -(-S // 16)
-    if B <= 1 or rows * (tiles + 64) >= 1 << 30:
+    if B <= 1 or not _flat_line(rows, max(S, most)):
         return 0
     return sm_count if tiles >= (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 160) else 0
 

@@ -228,7 +228,7 @@ class CompressedKVCache:
         flat = 0
         if nsplit is None:
             if not units: nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap)
-            flat = choose_flat(B, self.n_kv, max_len or self.cap, nsplit or 0, units, q.shape[1] // self.n_kv)
+            flat = choose_flat(B, self.n_kv, max_len or self.cap, nsplit or 0, units, q.shape[1] // self.n_kv, self.cap)
         K, V = self.k, self.v
         out = _ext().gaac_attn_launch(K.sm, K.codes, K.flags, K.tile_off, K.ovf, K.head_start, K.base3, K.base4,
                                       V.sm, V.codes, V.flags, V.tile_off, V.ovf, V.head_start, V.base3, V.base4,

@@ -31,8 +31,7 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     if nsplit is None:
         units = choose_units(B, n_kv, bt.shape[1] * 16)
         nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)        # with units: what the workspace must have room for
-        # (the library bounds a row's length by the table's row stride)
-        flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv) if B * n_kv * (bt.stride(0) + 64) < 1 << 30 else 0
+        flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv, _lib.row_stride(bt) * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), n_kv, TS, TS - 2880)

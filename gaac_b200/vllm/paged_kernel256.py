@@ -25,7 +25,7 @@ def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv,
     flat = 0
     if nsplit is None:
         nsplit = choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)
-        flat = choose_flat256(B, n_kv, bt.shape[1] * 16, nsplit) if B * n_kv * (bt.stride(0) + 64) < 1 << 30 else 0
+        flat = choose_flat256(B, n_kv, bt.shape[1] * 16, nsplit, _lib.row_stride(bt) * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)                                          # what the workspace must have room for
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), 2 * n_kv, TS, TS - 2880)

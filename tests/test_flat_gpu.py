@@ -21,6 +21,26 @@ def test_choose_flat_bounds():
     assert choose_flat(64, 1, 32769, 9, 0) == 148 and choose_flat(148, 1, 1000, 1, 0) == 0
 
 
+@pytest.mark.parametrize("B,cap", [(64, 32768), (1024, 1 << 20), (1024, 1 << 25), (4096, 1 << 22), (4096, 1 << 23)])
+def test_flat_launches_are_chosen_where_the_library_takes_them(monkeypatch, B, cap):
+    """max_len only steers the choice: a cache whose capacity is so large that the line of a flat launch could not be counted gets another form, not a refusal."""
+    import ctypes, types
+    import torch
+    import gaac_b200.kv_cache as kvc
+    from gaac_b200 import _lib
+    cache = object.__new__(kvc.CompressedKVCache)
+    store = types.SimpleNamespace(**{n: None for n in ("sm", "codes", "flags", "tile_off", "ovf", "head_start", "base3", "base4", "tail")})
+    cache.n_kv, cache.cap, cache.k, cache.v, cache._pending, cache.S, cache.tail_len = 1, cap, store, store, {}, None, None
+    seen = []
+    monkeypatch.setattr(kvc, "_ext", lambda: types.SimpleNamespace(gaac_attn_launch=lambda *a, flat, **k: (seen.append(flat), a[16])[1]))
+    fake, side = ctypes.c_void_p(0x1000), _lib.Side(0x1000, 0x1000, 0x1000, 0x1000, 0x1000, 0x1000, 64, 0x1000, 0x1000, None)
+    for max_len in (3000, 8192, None):
+        cache.attention(torch.zeros(B, 4, 128, dtype=torch.bfloat16), torch.zeros(B, dtype=torch.int32), SCALE, max_len=max_len)
+        if seen[-1]:                                                            # 5: only the workspace is too small
+            assert _lib.lib().gaac_decode_attn_flat(side, side, fake, fake, B, 4, 1, fake, cap, 0.1, seen[-1], None, 0, 1, fake, 64, fake, None, None) == 5
+    assert any(seen) == (B * (cap // 16 + 64) < 1 << 30)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_kv,G,lens", [(2, 4, [0, 5, 16, 1000, 17]), (1, 8, [700]), (2, 1, [333] * 6), (3, 5, [3, 33, 64, 65, 900, 1, 0, 300, 15, 16, 31, 47, 48, 49] * 5)])
 def test_slots_flat(monkeypatch, n_kv, G, lens):
