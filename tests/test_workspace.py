@@ -30,6 +30,18 @@ def test_outgrown_workspaces_stay_and_are_bounded(monkeypatch):
     assert K.workspace("cpu", 64, 8, 2) is seen[5]() and K.workspace("cpu", 2, 9000, 2) is seen[8]() is not seen[7]()       # shapes above the fixed header share nothing
 
 
+def test_stream_pointer_takes_every_form_of_a_device(monkeypatch):
+    import types
+    import torch
+    from gaac_b200 import _lib
+    asked = []
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: (asked.append(dev), types.SimpleNamespace(cuda_stream=7))[1])
+    monkeypatch.setattr(_lib, "_raw_stream", lambda index: 100 + index)
+    assert _lib.stream_ptr(torch.device("cuda", 1)) == 101 and not asked
+    forms = [None, "cuda", "cuda:0", 0, torch.device("cuda"), torch.device("cpu")]
+    assert [_lib.stream_ptr(d) for d in forms] == [7] * len(forms) and asked == forms
+
+
 @pytest.mark.gpu
 def test_graphs_of_descending_batch_sizes():
     """Graphs captured for 64 rows, then 32, then 4 on one stream; then what the allocator would have got back is overwritten, and all are replayed."""
