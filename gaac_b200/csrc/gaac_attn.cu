@@ -827,7 +827,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 // nobody is left at the barrier.
 // Output: partials of "virtual heads" vq = 2 * query head + half, which the last CTA of a (row, kv head) merges into out [B, n_q, 256].
 
-constexpr int META256_TILES = 64, PATCH256 = 48, SEG256_BYTES = SEG_PATCH + 8 * PATCH256;
+// (what shared memory has room for)
+constexpr int META256_TILES = 64, PATCH256 = 56, SEG256_BYTES = SEG_PATCH + 8 * PATCH256;
 constexpr int CTL_BYTES = 16;                                      // of a pair and tile parity: {next tile, fail flag of half 0, of half 1, -}
 constexpr int T256_BASES = ADDEND_BYTES + SEGTAB_BYTES, T256_META = T256_BASES + 2 * BASES_BYTES, T256_CTL = T256_META + META256_TILES * 16;
 constexpr int T256_SEG = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SEG + ATT_WARPS * SEG256_BYTES;

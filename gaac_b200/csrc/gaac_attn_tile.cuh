@@ -246,26 +246,33 @@ __device__ __forceinline__ void scan_step16(u32& v, int d) {
   asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0x1000, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
 }
 // Make the segment area of a tile pair.  Lane l has row l & 15 of K (l < 16) or of V.  live: the lane's side is compressed; fl, esc: shared-memory addresses of its
-// tag words and of its escape bytes, of which `avail` are staged.  Returned: bit 0 / 1: those of K / V are all staged (and there are no more than `room` items of
-// raw_items, which have their entries, 8 bytes each, behind the segment words).  Bound by its chain of latencies, hence a scan over 16 rows and not over 64 segments,
-// sizes from the tag words while the segment table answers, and items taken as they are found: a tile pair has 4.8 at a raw share of 0.75 %, hardly two in a row.
-// About 190 of the 1090 instructions per tile pair.  65536 tokens, 8 kv heads: 59.0 us with a look-up per group and raw groups as table entries found by the decoder
-// (1192 instructions), 56.2 with this and rebuild_pairs; slot cache 64 x 32768, group of 8: 247 -> 233; paged 16 x 4096..65536, 8 kv heads: 516 -> 493.
+// tag words and of its escape bytes, of which `avail` are staged.  Returned: bit 0 / 1: those of K / V are all staged (and the staged sides have no more than `room` raw
+// groups, which have their entries, 8 bytes each, behind the segment words; the other groups of raw_items need none).
+// Bound by its chain of latencies, hence a scan over 16 rows and not over 64 segments, and sizes from the tag words while the segment table answers.  The scan counts the
+// raw groups along with the escape bytes, so that a row knows its entries' places and takes its items without asking the others: with a vote per item and a place
+// for every item, promoted groups behind raw ones included, 65536 tokens took 56.9 us, now 54.9 (64 x 32768 220 -> 211, paged 16 x 4096..65536 443 -> 428), and at 32768
+// tokens tile pairs of 44 raw and 250 promoted groups ran out of places: 61.1 us, now 43.4.
+// Before that, against a look-up per group and raw groups as table entries found by the decoder: 59.0 -> 56.2, 247 -> 233, 516 -> 493.
 __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avail, const AttnView& w, u32 area, u32 room, int lane) {
   const u32 fl = live ? lds_u32(fl_at + 4u * (lane & 15)) : 0u;
-  const u32 size = (u32)row_esc_bytes(fl);
+  const u32 size = (u32)row_esc_bytes(fl), own_raws = (u32)popc(fl & 0xAAAAAAAAu);
   u32x2 e[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) e[q] = lds_u64(w.segs + (q < 3 ? 8u * ((fl >> (8 * q)) & 0xFFu) : 8u * (fl >> 24)));
-  u32 end = size;
-  scan_step16(end, 1); scan_step16(end, 2); scan_step16(end, 4); scan_step16(end, 8);
+  u32 sum = mad_k<65536u>(own_raws, size);                                   // escape bytes | raw groups << 16
+  scan_step16(sum, 1); scan_step16(sum, 2); scan_step16(sum, 4); scan_step16(sum, 8);
+  const u32 end = sum & 0xFFFFu, k_raws = __shfl_sync(FULLM, sum, 15) >> 16;
   const u32 over = __ballot_sync(FULLM, live && (int)end > avail);
   int staged = ((over & 0xFFFFu) ? 0 : 1) | ((over >> 16) ? 0 : 2);
   const u32 mine = area + SEG_V * (lane >> 4) + 32u * (lane & 15);
+  // places behind the row's entries: those of K first, if its side needs any
+  const u32 past = (sum >> 16) + (lane >= 16 && (staged & 1) ? k_raws : 0u);
   bool fast = (staged >> (lane >> 4)) & 1;
-  u32 items = 0u;
+  if (__any_sync(FULLM, fast && past > room)) { staged = 0; fast = false; }
+  u32 pos = end - size;
   if (fast) {
-    u32 at = live ? esc + end - size : area, a = at, four[4];
+    const u32 at = live ? esc + pos : area;
+    u32 a = at, four[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const u32 lo = lds_u32(a & ~3u), hi = lds_u32((a & ~3u) + 4u);
@@ -275,30 +282,21 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
 #pragma unroll
     for (int q = 0; q < 4; q += 2)
       sts_u128(mine + 8u * q, prmt(four[q], SEG_CONST, e[q].x), prmt(four[q], SEG_CONST, e[q].x >> 16), prmt(four[q + 1], SEG_CONST, e[q + 1].x), prmt(four[q + 1], SEG_CONST, e[q + 1].x >> 16));
-    items = raw_items(fl);
-  }
-  u32 some, entry = area + SEG_PATCH;
-  while ((some = __ballot_sync(FULLM, items != 0u)) != 0u) {                 // an item of every row that has one
-    const u32 n = (u32)popc(some);
-    if (entry + 8u * n > area + SEG_PATCH + 8u * room) { staged = 0; fast = false; break; }
-    if (items) {
-      const u32 bit = (u32)__ffs((int)items) - 1u, pl = esc + end - size + (u32)esc_prefix(fl, (int)bit);       // bit: lower tag bit of the group, 2 * group
+    u32 entry = area + SEG_PATCH + 8u * (past - own_raws);
+    for (u32 items = raw_items(fl); items; items &= items - 1u) {
+      const u32 bit = (u32)__ffs((int)items) - 1u, pl = at + (u32)esc_prefix(fl, (int)bit);       // bit: lower tag bit of the group, 2 * group
       u32 index;
-      items &= items - 1u;
       if ((fl >> bit) & 2u) {                          // the upper bits of the exponents, less what the decoder will add to them
-        const u32 own = entry + 8u * (u32)popc(some & ((1u << lane) - 1u));
-        index = (own - w.addends) >> 3;
+        index = (entry - w.addends) >> 3;
         const u32 m = index >> 8;
         const u32x4 bw = lds_u128(w.bases + BASES_V * (lane >> 4) + 8u * bit);
         const u32x2 x = pair_raw_addends(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * (pl & 3u));
-        sts_u64(own, x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w);
+        sts_u64(entry, x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w);
+        entry += 8u;
       } else index = 256u + lds_u8(pl);
       sts_u16(mine + bit, index);
     }
-    entry += 8u * n;
-  }
-  if (!fast) {                                       // {tag byte | position << 16}
-    u32 pos = end - size;
+  } else {                                           // {tag byte | position << 16}
 #pragma unroll
     for (int q = 0; q < 4; q++) { sts_u64(mine + 8u * q, ((fl >> (8 * q)) & 0xFFu) | pos << 16, 0u); pos += e[q].y; }
   }
