@@ -48,7 +48,7 @@ constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + BASES
 constexpr int ATT_SMEM = TB_RING + NSTG * STAGE_BYTES + 16;          // (an escape segment is read as whole words)
 static_assert(TB_BASES % 16 == 0 && TB_ESC % 16 == 0 && TB_AREA % 16 == 0 && TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
               "bulk copies need 16-byte aligned shared-memory destinations and sizes");
-static_assert(ATT_SMEM + 240 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
+static_assert(ATT_SMEM + 368 <= 232448, "one CTA per SM: at most 227 KB of shared memory, static part included");
 static_assert(ATT_THREADS / 128 * 2 >= 8, "the fused exchange keeps at most two merged heads per thread");
 constexpr int ACC_LD = D + 8;                        // row stride of the staged accumulators: 8j + r banks, conflict-free stores
 
@@ -375,39 +375,139 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
   }
 }
 
-// ---- flat launches: one wave of CTAs over all (row, kv head) pairs, one behind the other, each CTA an equal share of their tiles.  A pair counts FLAT_EXTRA tiles more
-// than it has, which lie in front of its own: what a CTA pays for every pair that it works on (tables of the bases, queries, first copies, merges).  CTA c has
-// [c * share, (c + 1) * share) of the line; a pair's pieces are those of the CTAs that have tiles of it, in order, and an empty pair (its output is zero) goes to the
-// CTA that has its last place.  Piece (CTA, pair) has its partials at (c + pair) * G, which no two pieces share.
-// Where the longest pair in k = CTAs / pairs equal pieces gives no CTA more than that share, every pair is in k pieces and a CTA has one: rows of about one length.
+// ---- flat launches: one wave of CTAs shares the (row, kv head) pairs; every CTA sees the lengths and makes the same plan, one of three.  A piece of a pair costs its CTA
+// about as much as FLAT_EXTRA tiles beside its own (tables of the bases, queries, first copies, merges).
+//  line    all pairs one behind the other, FLAT_EXTRA places in front of each, every CTA an equal share of the places: CTA c has [c * share, (c + 1) * share).  An
+//          empty pair (its output is zero) goes to the CTA that has its last place.  A CTA begins in the middle of a pair and pays for that piece: share + FLAT_EXTRA.
+//  single  no more pairs than CTAs: every pair in ceil(tiles / C) equal pieces (or in as many as every other, where they are about equally long), one piece per CTA, where
+//          the smallest C for which the CTAs suffice is no more than share.
+//  whole   more pairs than CTAs: the pairs in order of length, longest first, dealt out forth and back.  Where the CTA that gets most has no more than the line's, it saves the
+//          pieces in the middle and the merges.  That is what short rows want, and a caller who has a table (or a capacity) much wider than its rows are long.
+// A piece has its partials at (CTA + pair) * G, which no two pieces share: pieces of a pair are those of consecutive CTAs, in order.
 // A grid of several waves pays a prologue, the merges and the wait for its slowest CTA with every wave, about 8.5 us, and half a wave is as dear as a whole one.
-// us, grid -> flat: 16 rows x 8 kv heads of 4K-64K tokens 472 -> 422, 64 x 1 of 32K (groups of 8) 228 -> 218, 8 x 8 of 4K-16K 94 -> 80 (a balanced launch before).
-// FLAT_EXTRA 24 / 36 / 48: 16 x 8 421 / 422 / 424, 12 x 8 of 500-6000 - / 43.0 / 44.5, 64 x 1 - / 218 / 216, 64 x 8 of 100-400 40.1 / 41.4 / 42.5.
+// us, grid -> flat: 16 rows x 8 kv heads of 4K-64K tokens 455 -> 402, 64 x 1 of 32K (groups of 8) 222 -> 202, 8 x 8 of 4K-16K 94 -> 80 (a balanced launch before).
+// The line alone, and now: 64 x 8 of 100-400 in a table of 8192 39.9 -> 32.0, 32 x 8 of 20-2000 49.1 -> 42.2, 24 x 8 of 64-600 23.9 -> 16.7, 512 x 1 of 50-600 48.4 -> 38.7, 8 x 8 of 200-3000
+// 18.4 -> 15.7, 37 x 4 of 8K 113.8 -> 108.0, 300 x 1 of 100-2000 67.3 -> 66.6;  head_dim 256: 32 x 8 of up to 1000 53.8 -> 40.1, 8 x 4 of 100-700 15.1 -> 13.2.
+// FLAT_EXTRA 24 / 36 / 48 (of the line): 16 x 8 421 / 422 / 424, 12 x 8 of 500-6000 - / 43.0 / 44.5, 64 x 1 - / 218 / 216.
 constexpr int FLAT_EXTRA = 36;
+constexpr int FLAT_ROWS = 2048, FLAT_SORT = ATT_THREADS, FLAT_WHOLE = 32;               // rows whose tiles are held while the plan is made; rows that are sorted; pairs of a CTA that are dealt out
+constexpr int FLAT_SCRATCH = 4 * (FLAT_ROWS + 2 * FLAT_SORT + 4 * ATT_WARPS);
 struct FlatWalk {
-  int share, lo, hi;                                  // of the CTA; share < 0: the pairs are in -share equal pieces each
-  int row, kvh, at, tiles;                            // the pair that is looked at next: its first place on the line, its tiles
-  int pair, range[2], split, ns;                      // the piece found: pair = row * n_kv + kvh (below zero: no more), its first tile and how many, which of the pair's pieces
+  int share, lo, hi;                                  // of the CTA, on the line; share 0: single, below zero: whole
+  int row, kvh, at, tiles;                            // the pair that is looked at next: its first place on the line, its tiles; single, whole: `at` pieces are left
+  int pair, range[2], split, ns, tokens;              // the piece found: pair = row * n_kv + kvh (below zero: no more), its first tile and how many, which of the pair's pieces; the row's tokens
 };
-// Executed by one warp; every lane knows the same.
-// first32: where the first 32 rows' tiles are left for flat_next, which would wait for their loads again.
-template <class F> __device__ __forceinline__ void flat_start(FlatWalk& f, int B, int n_kv, int cta, int ctas, int lane, int* first32, const F& tiles_of) {
-  u32 total = 0u, longest = 0u;
-  for (int r0 = 0; r0 < B; r0 += 32) {
-    const int t = r0 + lane < B ? tiles_of(r0 + lane) : 0;
-    if (r0 == 0) first32[lane] = t;
-    total += __reduce_add_sync(FULLM, r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + t)) : 0u);
-    longest = max(longest, __reduce_max_sync(FULLM, (u32)t));
+__device__ __forceinline__ int tiles_in(int tokens) { return max((tokens + 15) >> 4, 0); }
+// Executed by the whole CTA; warp 0 gets the walk.  window: 64 words for flat_next;  scratch: FLAT_SCRATCH bytes that are free until the first piece begins;  least: tiles
+// of a piece of `single`, at least.
+template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B, int n_kv, int least, int* window, int* scratch, const F& tokens_of) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, ctas = gridDim.x, pairs = B * n_kv;
+  int* const held = scratch;                          // the rows' tokens
+  int* const order = held + FLAT_ROWS;
+  int* const keys = order + FLAT_SORT;
+  u32* const red = reinterpret_cast<u32*>(keys + FLAT_SORT);
+  u32 sum = 0u, longest = 0u, shortest = 0xFFFFFFFFu;
+  for (int r = tid; r < B; r += ATT_THREADS) {
+    const int tokens = tokens_of(r);
+    const u32 t = (u32)tiles_in(tokens);
+    if (r < FLAT_ROWS) held[r] = tokens;
+    sum += t; longest = max(longest, t); shortest = min(shortest, t);
   }
-  f.share = (int)((total + ctas - 1) / ctas);
-  f.row = 0; f.pair = 0;
-  const u32 k = (u32)ctas / (u32)(B * n_kv);
-  if (k && (longest + k - 1) / k <= (u32)f.share) { f.share = -(int)k; return; }
+  sum = __reduce_add_sync(FULLM, sum); longest = __reduce_max_sync(FULLM, longest); shortest = __reduce_min_sync(FULLM, shortest);
+  if (lane == 0) { red[warp] = sum; red[ATT_WARPS + warp] = longest; red[2 * ATT_WARPS + warp] = shortest; }
+  __syncthreads();
+  const int w = lane & (ATT_WARPS - 1);
+  sum = __reduce_add_sync(FULLM, lane < ATT_WARPS ? red[w] : 0u); longest = __reduce_max_sync(FULLM, red[ATT_WARPS + w]); shortest = __reduce_min_sync(FULLM, red[2 * ATT_WARPS + w]);
+  const u32 total = (u32)n_kv * (sum + (u32)(FLAT_EXTRA * B)), share = (total + ctas - 1) / ctas, most = share + FLAT_EXTRA;
+  f.row = f.kvh = f.at = f.tiles = f.tokens = 0; f.pair = -1;
+  if (pairs <= ctas) {
+    const u32 lo = max((u32)least, ((u32)n_kv * sum + ctas - 1) / ctas), hi = max(lo, share), same = (u32)(ctas / pairs), even = (longest + same - 1) / same;
+    f.share = 0;
+    if (even <= min(hi, lo + 2 + lo / 16)) {           // rows of about one length, or so few tiles that nothing is left to gain: as many pieces of every pair
+      if (warp != 0) return;
+      const int pair = cta / (int)same, r = pair / n_kv;
+      if (pair < pairs) {
+        const int t = tiles_in(held[r]), chunk = (t + (int)same - 1) / (int)same;
+        f.at = 1; f.pair = pair; f.split = cta - pair * (int)same; f.ns = (int)same; f.tokens = held[r];
+        f.range[0] = min(f.split * chunk, t); f.range[1] = min(chunk, t - f.range[0]);
+      }
+      return;
+    }
+    // sixteen sizes between the smallest that might do and share, a warp each (one after the other by bisection they took 0.5 us)
+    auto pieces_of = [&](int r, u32 C) { return r < B ? max(1u, ((u32)tiles_in(held[r]) + C - 1) / C) : 0u; };
+    {
+      const u32 C = lo + ((hi - lo) * (u32)(warp + 1) + ATT_WARPS - 1) / ATT_WARPS;
+      u32 n = 0u;
+      for (int r = lane; r < B; r += 32) n += pieces_of(r, C);
+      n = (u32)n_kv * __reduce_add_sync(FULLM, n);
+      if (lane == 0) red[3 * ATT_WARPS + warp] = n <= (u32)ctas ? C : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    const u32 C = __reduce_min_sync(FULLM, red[3 * ATT_WARPS + w]);
+    if (C != 0xFFFFFFFFu) {
+      if (warp != 0) return;
+      f.at = 1;
+      u32 before = 0u;
+      for (int r0 = 0; r0 < B; r0 += 32) {
+        const u32 n = pieces_of(r0 + lane, C), own = (u32)n_kv * n;
+        u32 inc = own;
+        scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8); scan_step(inc, 16);
+        const u32 past = __ballot_sync(FULLM, before + inc > (u32)cta);
+        if (past) {                                   // the row that the CTA's piece is of
+          const int l = __ffs((int)past) - 1, rest = cta - (int)(before + __shfl_sync(FULLM, inc - own, l)), t = tiles_in(held[r0 + l]);
+          f.ns = (int)__shfl_sync(FULLM, n, l); f.tokens = held[r0 + l];
+          const int h = rest / f.ns, chunk = (t + f.ns - 1) / f.ns;
+          f.pair = (r0 + l) * n_kv + h; f.split = rest - h * f.ns;
+          f.range[0] = min(f.split * chunk, t); f.range[1] = min(chunk, t - f.range[0]);
+          break;
+        }
+        before += __shfl_sync(FULLM, inc, 31);
+      }
+      return;
+    }
+  } else {
+    const int k = (pairs + ctas - 1) / ctas;
+    if (B <= FLAT_SORT && k <= FLAT_WHOLE && longest <= share && (u32)k * (FLAT_EXTRA + shortest) <= most && longest < 1u << 22) {
+      static_assert(FLAT_SORT <= 512, "nine bits of a key");
+      const int mine = tid < B ? tiles_in(held[tid]) << 9 | (511 - tid) : -1;           // (no two alike)
+      keys[tid] = mine;
+      __syncthreads();
+      int rank = 0;
+      for (int j = 0; j < B; j += 4) {
+        const int4 other = *reinterpret_cast<const int4*>(keys + j);
+        rank += (other.x > mine) + (other.y > mine) + (other.z > mine) + (other.w > mine);
+      }
+      if (tid < B) order[rank] = tid;
+      __syncthreads();
+      auto place = [&](int i, int c) { return i & 1 ? (i + 1) * ctas - 1 - c : i * ctas + c; };
+      u32 load = 0u;
+      for (int c = tid; c < ctas; c += ATT_THREADS) {
+        u32 own = 0u;
+        for (int i = 0; i < k; i++)
+          if (place(i, c) < pairs) own += FLAT_EXTRA + tiles_in(held[order[place(i, c) / n_kv]]);
+        load = max(load, own);
+      }
+      load = __reduce_max_sync(FULLM, load);
+      if (lane == 0) red[3 * ATT_WARPS + warp] = load;
+      __syncthreads();
+      if (__reduce_max_sync(FULLM, red[3 * ATT_WARPS + w]) <= most) {
+        if (warp == 0) {
+          f.share = -1; f.at = place(k - 1, cta) < pairs ? k : k - 1;
+          if (lane < f.at) { const int at = place(lane, cta), r = order[at / n_kv]; window[lane] = r * n_kv + at % n_kv; window[32 + lane] = held[r]; }
+          __syncwarp();
+        }
+        return;
+      }
+    }
+  }
+  if (warp != 0) return;
+  auto tokens_at = [&](int r) { return r < FLAT_ROWS ? held[r] : tokens_of(r); };
+  f.share = (int)share;
   f.lo = (int)min((long)cta * f.share, (long)total); f.hi = (int)min((long)f.lo + f.share, (long)total);
-  f.row = B; f.kvh = 0; f.at = 0; f.tiles = 0; f.pair = 0;
+  f.row = B;
   u32 before = 0u;
   for (int r0 = 0; r0 < B && f.lo < f.hi; r0 += 32) {
-    const int t = r0 == 0 ? first32[lane] : r0 + lane < B ? tiles_of(r0 + lane) : 0;
+    const int tokens = r0 + lane < B ? tokens_at(r0 + lane) : 0, t = tiles_in(tokens);
     const u32 own = r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + t)) : 0u;
     u32 inc = own;
     scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8); scan_step(inc, 16);
@@ -418,35 +518,45 @@ template <class F> __device__ __forceinline__ void flat_start(FlatWalk& f, int B
       const int row_at = (int)(before + __shfl_sync(FULLM, inc - own, l));
       f.kvh = (f.lo - row_at) / (FLAT_EXTRA + f.tiles);
       f.at = row_at + f.kvh * (FLAT_EXTRA + f.tiles);
+      window[lane] = tokens;
+      __syncwarp();
       break;
     }
     before += __shfl_sync(FULLM, inc, 31);
   }
 }
-template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int cta, const int* first32, const F& tiles_of_far) {
-  const auto tiles_of = [&](int row) { return row < 32 ? first32[row] : tiles_of_far(row); };
-  f.pair = -1;
-  if (f.share < 0) {
-    const int k = -f.share, pair = cta / k;
-    if (f.row < B && pair < B * n_kv) {
-      const int t = tiles_of(pair / n_kv), chunk = (t + k - 1) / k;
-      f.pair = pair; f.split = cta - pair * k; f.ns = k; f.range[0] = min(f.split * chunk, t); f.range[1] = min(chunk, t - f.range[0]);
-    }
-    f.row = B;
+// The next piece, by the whole of warp 0.  On the line, window has the tokens of the 32 rows that the walk is among.
+template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int lane, int* window, const F& tokens_of) {
+  if (f.share <= 0) {
+    if (f.at == 0) f.pair = -1;
+    else if (--f.at, f.share < 0) { f.pair = window[f.at]; f.tokens = window[32 + f.at]; f.range[0] = 0; f.range[1] = tiles_in(f.tokens); f.split = 0; f.ns = 1; }
     return;
   }
+  f.pair = -1;
   while (f.row < B && f.pair < 0) {
     const int first = f.at + FLAT_EXTRA - (f.tiles > 0 ? 0 : 1), last = first + max(f.tiles, 1) - 1;
     if (first >= f.hi) return;
     if (last >= f.lo) {
       const int c0 = first / f.share;
-      f.pair = f.row * n_kv + f.kvh; f.split = cta - c0; f.ns = last / f.share - c0 + 1;
+      f.pair = f.row * n_kv + f.kvh; f.split = blockIdx.x - c0; f.ns = last / f.share - c0 + 1; f.tokens = window[f.row % 32];
       f.range[0] = f.tiles > 0 ? max(f.lo, first) - first : 0; f.range[1] = f.tiles > 0 ? min(f.hi - 1, last) - first + 1 - f.range[0] : 0;
     }
     f.at += FLAT_EXTRA + f.tiles;
-    if (++f.kvh == n_kv) { f.kvh = 0; if (++f.row < B) f.tiles = tiles_of(f.row); }
+    if (++f.kvh == n_kv) {
+      f.kvh = 0;
+      if (++f.row < B) {
+        if (f.row % 32 == 0) {
+          __syncwarp();
+          window[lane] = f.row + lane < B ? tokens_of(f.row + lane) : 0;
+          __syncwarp();
+        }
+        f.tiles = tiles_in(window[f.row % 32]);
+      }
+    }
   }
 }
+
+static_assert(FLAT_SCRATCH <= ATT_WARPS * AREA_BYTES, "planned in the segment areas");
 
 // How the rows are shared out.  GRID: (row, kv head) x splits;  SHARED: a balanced launch;  FLAT_LINE: above.  Instantiations of their own: the shares cost the others
 // registers that the main loop has none of, 1.5 % at 64K tokens.
@@ -457,7 +567,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last, s_split, s_ns, s_tail, s_esc[6];        // (from s_split on: not needed inside the main loop, whose registers are all taken)
   __shared__ FlatWalk s_flat;
-  __shared__ int s_tiles[FLAT ? 32 : 1];
+  __shared__ int s_rows[FLAT ? 64 : 1];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);   // the same value, but known to the compiler to be uniform across the warp
   const int G = p.G;
@@ -469,13 +579,17 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // in a plain launch.
   if (tid < 256) fill_attn_tables(smem, tid);
   // Warp w fills stage w first, and clears the words of its tiles: a lane that publishes one has cleared it itself, so no other warp has to be waited for.
-  if (warp < NSTG && lane < TPS) reinterpret_cast<u32*>(smem + TB_USE)[warp * TPS + lane] = 0u;
-  if (lane == 0 && warp < NSTG) {
-    mbar_init(smem_s + TB_FULL + 8 * warp, 1);
-    reinterpret_cast<int*>(smem + TB_LEFT)[warp] = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncwarp();
+  auto begin_ring = [&](bool again) {
+    if (warp < NSTG && lane < TPS) reinterpret_cast<u32*>(smem + TB_USE)[warp * TPS + lane] = 0u;
+    if (lane == 0 && warp < NSTG) {
+      if (again) asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_s + TB_FULL + 8 * warp) : "memory");
+      mbar_init(smem_s + TB_FULL + 8 * warp, 1);
+      reinterpret_cast<int*>(smem + TB_LEFT)[warp] = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncwarp();
+  };
+  begin_ring(false);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
 
@@ -506,15 +620,15 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       bh = __shfl_sync(FULLM, bh, 0); split0 = __shfl_sync(FULLM, split0, 0);
     }
   }
-  auto tiles_of = [&](int row) -> int {               // (a slot's first head stands for all of its heads)
-    if (PAGED) return max((p.seq_len[row] + 15) >> 4, 0);
+  auto tokens_of = [&](int row) -> int {              // (a slot's first head stands for all of its heads)
+    if (PAGED) return p.seq_len[row];
     const int sl = p.slot[row];
-    return sl < 0 ? 0 : max((p.seq_len[(long)sl * p.n_kv] + 15) >> 4, 0);
+    return sl < 0 ? 0 : p.seq_len[(long)sl * p.n_kv];
   };
-  if (FLAT && warp == 0) {
+  if (FLAT) {
     FlatWalk f;
-    flat_start(f, p.B, p.n_kv, blockIdx.x, gridDim.x, lane, s_tiles, tiles_of);
-    if (lane == 0) s_flat = f;
+    flat_plan(f, p.B, p.n_kv, 4, s_rows, reinterpret_cast<int*>(smem + TB_AREA), tokens_of);
+    if (tid == 0) s_flat = f;
     __syncwarp();
   }
   do {
@@ -522,22 +636,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (warp == 0) {
       FlatWalk f = s_flat;
       __syncwarp();
-      flat_next(f, p.B, p.n_kv, blockIdx.x, s_tiles, tiles_of);
+      flat_next(f, p.B, p.n_kv, lane, s_rows, tokens_of);
       if (lane == 0) { s_flat = f; s_split = f.split; s_ns = f.ns; }
     }
-    // the ring begins again (every copy of the piece before has landed, and its last waits are behind the barrier at the end of the loop)
-    if (warp < NSTG && lane < TPS) reinterpret_cast<u32*>(smem + TB_USE)[warp * TPS + lane] = 0u;
-    if (lane == 0 && warp < NSTG) {
-      asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_s + TB_FULL + 8 * warp) : "memory");
-      mbar_init(smem_s + TB_FULL + 8 * warp, 1);
-      reinterpret_cast<int*>(smem + TB_LEFT)[warp] = 0;
-      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // the ring was written by the merges of the piece before
     __syncthreads();
     bh = __shfl_sync(FULLM, s_flat.pair, 0);
     if (bh < 0) return;
-    if (PAGED) S_paged = p.seq_len[bh / p.n_kv];
+    if (PAGED) S_paged = s_flat.tokens;
   }
   int b = bh / p.n_kv, kvh = bh % p.n_kv;
 
@@ -811,7 +916,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if (atomicAdd(p.x_ticket, 1) == (int)gridDim.x - 1) { *p.x_ticket = 0; __threadfence(); atomicAdd(p.x_epoch, 1); }
     }
   }
-  if (FLAT) __syncthreads();                         // the shared memory is used again
+  if (FLAT) {                                        // every copy of the piece has landed, and its last waits are behind this barrier.  (At the top of the loop the same
+    __syncthreads();                                 // takes 0.5 us of a short launch and spills.)
+    begin_ring(true);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // the ring was written by the merges
+  }
   } while (FLAT);
 }
 
@@ -828,21 +937,23 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 // Output: partials of "virtual heads" vq = 2 * query head + half, which the last CTA of a (row, kv head) merges into out [B, n_q, 256].
 
 // (what shared memory has room for)
-constexpr int META256_TILES = 64, PATCH256 = 56, SEG256_BYTES = SEG_PATCH + 8 * PATCH256;
+constexpr int META256_TILES = 48, PATCH256 = 56, SEG256_BYTES = SEG_PATCH + 8 * PATCH256;
 constexpr int CTL_BYTES = 16;                                      // of a pair and tile parity: {next tile, fail flag of half 0, of half 1, -}
 constexpr int T256_BASES = ADDEND_BYTES + SEGTAB_BYTES, T256_META = T256_BASES + 2 * BASES_BYTES, T256_CTL = T256_META + META256_TILES * 16;
 constexpr int T256_SEG = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SEG + ATT_WARPS * SEG256_BYTES;
 constexpr int STAGE256_BYTES = 16 + 2 * PSLOT, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
 constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;          // (an escape segment is read as whole words)
-static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 208 <= 232448, "one CTA per SM");
+static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 336 <= 232448, "one CTA per SM");
 
-// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.7 -> 26.8 us, 20 x 8 of up to 3K 97 -> 74 (a grid before, rows as they come).
+static_assert(FLAT_SCRATCH <= ATT_WARPS * SEG256_BYTES, "planned in the segment areas");
+// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.4 -> 24.9 us, 20 x 8 of up to 3K 89 -> 72 (a grid, rows as they come).  Pieces of two tiles on short rows: of four
+// 0.5 us slower on 2 x 4 of 700.
 template <int NSET, bool FLAT>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last;
   __shared__ FlatWalk s_flat;
-  __shared__ int s_tiles[FLAT ? 32 : 1];
+  __shared__ int s_rows[FLAT ? 64 : 1];
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(FULLM, tid >> 5, 0);
   const int hf = warp & 1, pair = warp >> 1;
@@ -850,44 +961,42 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   const int ring = T256_RING + warp * WARP256_BYTES;
   const u32 smem_s = (u32)__cvta_generic_to_shared(smem), ring_s = smem_s + ring;
   if (tid < 256) fill_attn_tables(smem, tid);
-  if (!FLAT && tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
-  if (lane == 0) {
-    mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
+  auto begin_ring = [&] {
+    if (tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
+    if (lane == 0) {
+      mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+  };
+  if (!FLAT) begin_ring();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
-  auto tiles_of = [&](int row) -> int { return max((p.seq_len[row] + 15) >> 4, 0); };
-  if (FLAT && warp == 0) {
+  auto tokens_of = [&](int row) -> int { return p.seq_len[row]; };
+  if (FLAT) {
     FlatWalk f;
-    flat_start(f, p.B, p.n_kv, blockIdx.x, gridDim.x, lane, s_tiles, tiles_of);
-    if (lane == 0) s_flat = f;
+    flat_plan(f, p.B, p.n_kv, 2, s_rows, reinterpret_cast<int*>(smem + T256_SEG), tokens_of);
+    if (tid == 0) s_flat = f;
     __syncwarp();
   }
   int bh = blockIdx.x, split = blockIdx.y, NS = p.nsplit;
   do {
-  if (FLAT) {                                        // the next piece, with the ring and the pairs' words as they were at first
+  if (FLAT) {                                        // the next piece
     if (warp == 0) {
       FlatWalk f = s_flat;
       __syncwarp();
-      flat_next(f, p.B, p.n_kv, blockIdx.x, s_tiles, tiles_of);
+      flat_next(f, p.B, p.n_kv, lane, s_rows, tokens_of);
       if (lane == 0) s_flat = f;
     }
-    if (tid < (ATT_WARPS / 2) * 2 * CTL_BYTES / 4) reinterpret_cast<u32*>(smem + T256_CTL)[tid] = 0u;
-    if (lane == 0) {
-      asm volatile("mbarrier.inval.shared::cta.b64 [%0];\nmbarrier.inval.shared::cta.b64 [%1];\n" ::"r"(ring_s), "r"(ring_s + STAGE256_BYTES) : "memory");
-      mbar_init(ring_s, 1); mbar_init(ring_s + STAGE256_BYTES, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
+    begin_ring();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // the ring was written by the merges of the piece before
     __syncthreads();
     bh = __shfl_sync(FULLM, s_flat.pair, 0); split = __shfl_sync(FULLM, s_flat.split, 0); NS = __shfl_sync(FULLM, s_flat.ns, 0);
     if (bh < 0) return;
   }
   int b = bh / p.n_kv, kvh = bh % p.n_kv;
-  const int S = __shfl_sync(FULLM, p.seq_len[b], 0);
+  const int S = __shfl_sync(FULLM, FLAT ? s_flat.tokens : p.seq_len[b], 0);
   const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS;
-  const int tlo = FLAT ? __shfl_sync(FULLM, s_flat.range[0], 0) : min(split * chunk, ntiles), n = FLAT ? __shfl_sync(FULLM, s_flat.range[1], 0) : min(chunk, ntiles - tlo);
+  const int tlo = min(FLAT ? __shfl_sync(FULLM, s_flat.range[0], 0) : split * chunk, ntiles), n = min(FLAT ? __shfl_sync(FULLM, s_flat.range[1], 0) : chunk, ntiles - tlo);
   int* const ctl_pair = reinterpret_cast<int*>(smem + T256_CTL + pair * (2 * CTL_BYTES));
   const int4* meta_s = reinterpret_cast<const int4*>(smem + T256_META);        // per tile: mode-table entries of {K, V} of half 0, of half 1
   auto slot_of = [&](int i) { return p.bt[(long)b * p.bt_stride + tlo + i] * NT + 4 * kvh; };
@@ -970,6 +1079,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     __syncwarp();                                      // every lane has read this stage before its next copies are issued
   }
   if (FLAT) {                                        // (not kept in registers across the main loop)
+    // the merges write over the warp's barriers
+    if (lane == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];\nmbarrier.inval.shared::cta.b64 [%1];\n" ::"r"(ring_s), "r"(ring_s + STAGE256_BYTES) : "memory");
     bh = __shfl_sync(FULLM, s_flat.pair, 0); split = __shfl_sync(FULLM, s_flat.split, 0); NS = __shfl_sync(FULLM, s_flat.ns, 0);
     b = bh / p.n_kv; kvh = bh % p.n_kv;
   }

@@ -127,15 +127,18 @@ def _flat_line(rows: int, most: int) -> bool:
 @functools.lru_cache(maxsize=4096)
 def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int = 4, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
     """CTAs of a flat launch (one wave that shares the tiles of all rows and kv heads evenly), or 0 where the form that it would replace is no slower: nsplit splits per
-    (row, kv head), or `units` ranges per kv head (S: tokens of the longest row, group: query heads per kv head).
+    (row, kv head), or `units` ranges per kv head (S: tokens that the longest row may have, group: query heads per kv head, most: tokens that any row may hold; nsplit itself
+    does not enter).  S is often a bound far above the rows' lengths (a block table as wide as the longest sequence allowed, a cache's capacity): the launch reads the
+    lengths and plans accordingly, the grid's split count cannot.
     A flat launch saves what comes with the waves of a grid, and the idle end of the last one; it pays some 8 us for every piece of a row that a CTA has beyond its
     first.  us, other form -> flat:
-      grids of several waves: 64 rows x 1 kv head, 32K tokens 228 -> 218;  16 x 8, 4K-64K 472 -> 422;  40 x 4, 2K-6K 95 -> 80;  20 x 8, 2K-3K 71 -> 56;  64 x 8, up to 4200
-        124 -> 120.  Short rows lose: 32 x 8, 20-2000 tokens 49 -> 56;  64 x 8, 100-400 33 -> 41;  24 x 8, 64-600 17 -> 24
-      one wave: 64 x 2, 4K-8K 116 -> 101;  64 x 1, 8K-16K 118 -> 91;  37 x 4, up to 8K 108 -> 71;  35 x 1, up to 12K 47 -> 33.  A full wave of equal rows pays for the walk: 37 x 4,
-        8K 110.9 -> 114.1
+      grids of several waves: 64 rows x 1 kv head, 32K tokens 222 -> 202;  16 x 8, 4K-64K 455 -> 402;  40 x 4, 2K-6K 95 -> 76;  20 x 8, 2K-3K 71 -> 53;  64 x 8, 500-4200 164 -> 143.
+        Short rows in a table that fits them are even: 64 x 8, 100-400 31.7 -> 32.0;  32 x 8, 20-2000 41 -> 42;  24 x 8, 64-600 16.3 -> 16.7;  in one of 8192 tokens they take 58, 69 and 33 as
+        a grid
+      one wave: 64 x 2, 4K-8K 116 -> 101;  64 x 1, 8K-16K 118 -> 91;  37 x 4, 8K each 110 -> 108
       shares of units, which come in whole ones: a fifth of them or more for the rows' first units 8 x 8, 4K-16K 94 -> 80;  4 x 8, 20K-32K 104 -> 95;  5 x 8, up to 9K 31.7 ->
-        30.6;  fewer, 16 x 1 36 -> 39, 8 x 1 36.4 -> 36.9;  more than four query heads per kv head, 6 x 8 61 -> 64."""
+        30.6;  short rows there pay up to 0.8 us for the plan (8 x 8, 200-3000 14.9 -> 15.7);  fewer, 16 x 1 36 -> 39, 8 x 1 36.4 -> 36.9;  more than four query heads per kv head, 6 x 8
+        61 -> 64."""
     rows, tiles = B * n_kv, -(-S // 16)
     if B <= 1 or tiles < 160 or rows * tiles < 120 * sm_count or not _flat_line(rows, max(S, most)):
         return 0
@@ -146,9 +149,10 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
 
 @functools.lru_cache(maxsize=4096)
 def choose_flat256(B: int, n_kv: int, S: int, nsplit: int, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
-    """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.7 -> 26.8;  20 x 8, up to 3K 97 -> 74;  32 x 2, up
-    to 4K 57 -> 42;  6 x 2, up to 60K 129 -> 94;  2 x 8 of 1000 31 -> 13;  9 x 4, up to 1500 24.5 -> 19.3;  30 x 4, up to 2K 56 -> 48.  Many short rows lose: 32 x 4, up to 1000
-    31 -> 34.5;  32 x 8 52.8 -> 54.8.  A full wave of equal rows pays for the walk: 12 x 4 of 4000 46.3 -> 48.5;  one sequence has nothing to gain: 1 x 4 of 8K 18.4 -> 18.6."""
+    """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.4 -> 24.9;  20 x 8, up to 3K 89 -> 72;  32 x 2, up
+    to 4K 57 -> 42;  6 x 2, up to 60K 129 -> 94;  8 x 4, 100-700 22.3 -> 13.2;  2 x 8 of 1000 31 -> 13;  32 x 4, up to 1000 30.7 -> 31.3, in a table of 8192 44 -> 31.3;  32 x 8 the same 53 -> 40,
+    66 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.6 -> 47.4;  so are a few very short ones: 4 x 4 of 50-300 in a table of 8192 9.3 -> 11.0;  one sequence has nothing
+    to gain: 1 x 4 of 8K 18.4 -> 18.6."""
     rows, tiles = B * n_kv, -(-S // 16)
     if B <= 1 or not _flat_line(rows, max(S, most)):
         return 0

@@ -212,3 +212,72 @@ def test_paged256_flat(monkeypatch, n_kv, G, lens):
                 assert not out[b].any(), (b, ctas)
             else:
                 assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b].reshape(-1, n_kv, 256)[:L], vs[b].reshape(-1, n_kv, 256)[:L], 256 ** -0.5, (b, ctas))
+
+
+# Many rows over a few stored sequences.  Rows that are dealt out whole (1 to 32 pairs a CTA), too many rows for that (513), too many to be held while the plan is made
+# (2049), more pairs than are dealt out (7 CTAs); one piece per CTA (1000 CTAs), rows of one length and of very different ones
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,short", [(40, True), (160, True), (160, False), (512, True), (513, True), (2049, False)])
+@pytest.mark.parametrize("paged", [False, True])
+def test_plans_of_many_rows(monkeypatch, rows, short, paged):
+    import torch
+    import gaac_b200.kv_cache as kvc, gaac_b200.vllm.paged_kernel as pk
+    n_kv, G = 2, 4
+    rng = np.random.default_rng(rows)
+    lens = [int(x) for x in rng.integers(1, 260, 12)] + [16, 1, 0, 0] if short else [1500, 3, 40, 700, 16, 90, 0, 33]
+    pick = rng.integers(0, len(lens), rows)
+    pick[: len(lens)] = np.arange(len(lens))[: rows]
+    q16 = O.f32_to_bf16((rng.standard_normal((len(lens), n_kv * G, 128)) * 0.1).astype(np.float32))
+    q, idx = to_bf16_cuda(q16)[torch.from_numpy(pick)].contiguous(), torch.from_numpy(pick).cuda()
+    if paged:
+        full = [max(L, 1) for L in lens]
+        st, buf, bt, ks, vs = _build_paged(full, n_kv, sum(-(-L // 16) for L in full) + 4, seed=3, raw_tiles=4 * n_kv * len(lens))
+        sl = torch.tensor(lens, dtype=torch.int32, device="cuda")[idx]
+        out, bt = torch.empty(rows, n_kv * G * 128, dtype=torch.bfloat16, device="cuda"), bt[idx].contiguous()
+        call = lambda o32: pk.paged_attention(q, out, buf, st.raw, st.mt, bt, sl, st.bases, st.TS, n_kv * G, n_kv, out_f32=o32)
+    else:
+        ks, vs = ([np.ascontiguousarray(O.kv_like(n_kv, max(L, 1), 7 * i + s).transpose(1, 0, 2)) for i, L in enumerate(lens)] for s in (1, 2))
+        cache = kvc.CompressedKVCache(n_slots=len(lens), n_kv=n_kv, capacity=1536, bases=None)
+        for i, L in enumerate(lens):
+            if L: cache.prefill(i, to_bf16_cuda(ks[i]), to_bf16_cuda(vs[i]), check=False)
+        call = lambda o32: cache.attention(q, idx.int(), SCALE, max_len=1500, out_f32=o32)
+    refs = [O.attention_ref(q16[i], ks[i][:L], vs[i][:L], SCALE, with_abs=True) for i, L in enumerate(lens)]
+    ref = torch.from_numpy(np.stack([r for r, _ in refs])).cuda()
+    bound = torch.from_numpy(np.stack([O.attention_bound(m) for _, m in refs])).cuda()
+    for ctas in (7, 37, 148, 148, 1000):
+        monkeypatch.setattr(kvc, "choose_flat", lambda *a, n=ctas: n)
+        monkeypatch.setattr(pk, "choose_flat", lambda *a, n=ctas: n)
+        o32 = torch.full((rows, n_kv * G, 128), float("nan"), dtype=torch.float32, device="cuda")
+        call(o32)
+        worst = ((o32.double() - ref[idx]).abs() / bound[idx]).amax((1, 2))
+        assert bool((worst <= 1.0).all()), (ctas, [int(b) for b in (~(worst <= 1.0)).nonzero().ravel()[:8]])
+
+
+@pytest.mark.gpu
+def test_short_rows_in_a_wide_table_are_no_slower_than_in_a_narrow_one():
+    """The launch that the rule picks for a table of 8192 tokens, rows of 100 to 400 tokens: the grid of a table that fits takes 32 us, pieces of equal shares of a line 40."""
+    import torch
+    import gaac_b200.vllm.paged_kernel as pk
+    from gaac_b200.kernel import choose_flat
+    B, n_kv, G = 64, 8, 4
+    lens = [int(x) for x in np.random.default_rng(5).integers(100, 400, B)]
+    st, buf, bt, ks, vs = _build_paged(lens, n_kv, sum(-(-L // 16) for L in lens) + 4, seed=3, raw_tiles=2 * n_kv * B + 64)
+    wide = torch.nn.functional.pad(bt, (0, 512 - bt.shape[1])).contiguous()
+    assert choose_flat(B, n_kv, 8192, 1, 0, G) == 148                           # reached through the rule itself
+    q16 = O.f32_to_bf16((np.random.default_rng(1).standard_normal((B, n_kv * G, 128)) * 0.3).astype(np.float32))
+    q, sl = to_bf16_cuda(q16), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    out, best = torch.empty(B, n_kv * G * 128, dtype=torch.bfloat16, device="cuda"), {}
+    o32 = torch.empty(B, n_kv * G, 128, dtype=torch.float32, device="cuda")
+    call = lambda t, **k: pk.paged_attention(q, out, buf, st.raw, st.mt, t, sl, st.bases, st.TS, n_kv * G, n_kv, **k)
+    call(wide, out_f32=o32)
+    for b in (0, 17, B - 1):
+        assert_attention_close(o32[b].cpu().numpy(), q16[b], ks[b], vs[b], SCALE, b)
+    for name, table in (("narrow", bt), ("wide", wide)) * 10:
+        a, e = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        call(table)
+        a.record()
+        for _ in range(20): call(table)
+        e.record()
+        torch.cuda.synchronize()
+        best[name] = min(best.get(name, 1e9), a.elapsed_time(e) * 50)
+    assert best["wide"] < 1.12 * best["narrow"], best
