@@ -35,7 +35,6 @@ __device__ __forceinline__ void mbar_init(u32 mbar, u32 count) { asm volatile("m
 __device__ __forceinline__ void mbar_expect_tx(u32 mbar, u32 bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_add_tx(u32 mbar, u32 bytes) { asm volatile("mbarrier.expect_tx.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory"); }
 __device__ __forceinline__ void bulk_g2s(u32 dst, const void* src, u32 bytes, u32 mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(mbar) : "memory");
 }

@@ -148,7 +148,7 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
 
 
 @functools.lru_cache(maxsize=4096)
-def choose_flat256(B: int, n_kv: int, S: int, nsplit: int, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
+def choose_flat256(B: int, n_kv: int, S: int, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
     """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.4 -> 24.9;  20 x 8, up to 3K 89 -> 72;  32 x 2, up
     to 4K 57 -> 42;  6 x 2, up to 60K 129 -> 94;  8 x 4, 100-700 22.3 -> 13.2;  2 x 8 of 1000 31 -> 13;  32 x 4, up to 1000 30.7 -> 31.3, in a table of 8192 44 -> 31.3;  32 x 8 the same 53 -> 40,
     66 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.6 -> 47.4;  so are a few very short ones: 4 x 4 of 50-300 in a table of 8192 9.3 -> 11.0;  one sequence has nothing
@@ -199,10 +199,10 @@ class _Ext:
         L = _lib.lib()
         if flat or units:
             out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
-            launch = L.gaac_decode_attn_flat if flat else L.gaac_decode_attn_balanced
-            _lib.check(launch(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), flat or units,
-                                                   TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel(),
-                                                   out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_decode_attn_balanced")
+            name = "gaac_decode_attn_flat" if flat else "gaac_decode_attn_balanced"
+            _lib.check(getattr(L, name)(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), flat or units,
+                                        TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel(),
+                                        out.data_ptr(), _lib.ptr(out_f32), stream), name)
             return out
         common = (K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), int(nsplit),
                   TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel())

@@ -38,7 +38,7 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, n_q, nsplit, stream)
     lib = _lib.lib()
-    launch = lib.gaac_paged_decode_attn_flat if flat else lib.gaac_paged_decode_attn_balanced if units else lib.gaac_paged_decode_attn
-    _lib.check(launch(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit),
-                      ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_paged_decode_attn")
+    name = "gaac_paged_decode_attn_flat" if flat else "gaac_paged_decode_attn_balanced" if units else "gaac_paged_decode_attn"
+    _lib.check(getattr(lib, name)(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit),
+                                  ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), name)
     return out

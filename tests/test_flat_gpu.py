@@ -281,3 +281,16 @@ def test_short_rows_in_a_wide_table_are_no_slower_than_in_a_narrow_one():
         torch.cuda.synchronize()
         best[name] = min(best.get(name, 1e9), a.elapsed_time(e) * 50)
     assert best["wide"] < 1.12 * best["narrow"], best
+
+
+@pytest.mark.parametrize("flat,units,name", [(148, 0, "gaac_decode_attn_flat"), (0, 12, "gaac_decode_attn_balanced")])
+def test_a_refused_call_is_reported_by_its_own_name(monkeypatch, flat, units, name):
+    import types
+    import torch
+    from gaac_b200 import _lib, kernel
+    monkeypatch.setattr(kernel, "workspace", lambda *a: torch.zeros(64, dtype=torch.uint8))
+    monkeypatch.setattr(_lib, "stream_ptr", lambda dev=None: None)
+    t, i = torch.zeros(16, 128, dtype=torch.uint8), torch.zeros(16, dtype=torch.int32)
+    q = types.SimpleNamespace(size=lambda d: 128, is_cuda=True, device="cpu", dtype=torch.bfloat16, data_ptr=lambda: 16)
+    with pytest.raises(RuntimeError, match=name + ":"):
+        kernel._Ext.gaac_attn_launch(t, t, i, i, t, i, t, t, t, t, i, i, t, i, t, t, q, i[:4], 4, 1, i, 17, 0.1, None, t[:0], t[:0], i, 0, units=units, flat=flat)          # (a capacity of 17 tokens)
