@@ -16,7 +16,7 @@ def _cache(n_slots):
     return cache
 
 
-@pytest.mark.parametrize("n_slots", [1, 7, 4096, 4097, 8192, 8193])
+@pytest.mark.parametrize("n_slots", [1, 7, 64, 65, 4096, 4097, 8192, 8193])
 def test_words_of_the_pending_slots_are_read(n_slots):
     import torch
     from gaac_b200.kv_cache import TILE_MAX_ESC, _OVER_READ
