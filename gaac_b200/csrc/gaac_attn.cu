@@ -11,8 +11,9 @@
 // finish merges the splits and writes the output, so one launch does the whole layer.
 //
 // What the measurements on B200 say (they shaped the code below):
-//  * the kernel is bound by instruction issue, not by HBM.  With a private two-stage ring per warp every warp issued eight copies per tile pair, about
-//    200 of 1354 instructions; one copy of four tiles, issued by the warp that is last to leave a stage, takes that to about 25 per tile pair.
+//  * the kernel is bound by the rebuild's instructions and by the latency that four warps per scheduler leave open, not by HBM (figures in gaac_attn_tile.cuh).  With a
+//    private two-stage ring per warp every warp issued eight copies per tile pair, about 200 of 1354 instructions; one copy of four tiles, issued by the warp that is
+//    last to leave a stage, takes that to about 25 per tile pair.
 //  * a bulk copy takes the warp that issues it about 100 cycles, and a loop over the lanes before it where its operands are not known to be uniform: the
 //    eight copies of a stage took their warp 2300 cycles, issued by an elected lane of the converged warp 1150 (57.5 -> 56.7 us at 65536 tokens).
 //  * warps of their own for parts of the work lose: one that issues all copies is too slow by itself (56.3 us, but 620 instead of 500 on paged tiles), and with
@@ -385,7 +386,7 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
 //          pieces in the middle and the merges.  That is what short rows want, and a caller who has a table (or a capacity) much wider than its rows are long.
 // A piece has its partials at (CTA + pair) * G, which no two pieces share: pieces of a pair are those of consecutive CTAs, in order.
 // A grid of several waves pays a prologue, the merges and the wait for its slowest CTA with every wave, about 8.5 us, and half a wave is as dear as a whole one.
-// us, grid -> flat: 16 rows x 8 kv heads of 4K-64K tokens 455 -> 402, 64 x 1 of 32K (groups of 8) 222 -> 202, 8 x 8 of 4K-16K 94 -> 80 (a balanced launch before).
+// us, grid -> flat: 16 rows x 8 kv heads of 4K-64K tokens 452 -> 403, 64 x 1 of 32K (groups of 8) 219 -> 202, 8 x 8 of 4K-16K 89 -> 77 (a balanced launch before).
 // The line alone, and now: 64 x 8 of 100-400 in a table of 8192 39.9 -> 32.0, 32 x 8 of 20-2000 49.1 -> 42.2, 24 x 8 of 64-600 23.9 -> 16.7, 512 x 1 of 50-600 48.4 -> 38.7, 8 x 8 of 200-3000
 // 18.4 -> 15.7, 37 x 4 of 8K 113.8 -> 108.0, 300 x 1 of 100-2000 67.3 -> 66.6;  head_dim 256: 32 x 8 of up to 1000 53.8 -> 40.1, 8 x 4 of 100-700 15.1 -> 13.2.
 // FLAT_EXTRA 24 / 36 / 48 (of the line): 16 x 8 421 / 422 / 424, 12 x 8 of 500-6000 - / 43.0 / 44.5, 64 x 1 - / 218 / 216.
@@ -946,7 +947,7 @@ constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;         
 static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 336 <= 232448, "one CTA per SM");
 
 static_assert(FLAT_SCRATCH <= ATT_WARPS * SEG256_BYTES, "planned in the segment areas");
-// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.4 -> 24.9 us, 20 x 8 of up to 3K 89 -> 72 (a grid, rows as they come).  Pieces of two tiles on short rows: of four
+// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.1 -> 24.8 us, 20 x 8 of up to 3K 95 -> 73 (a grid, rows as they come).  Pieces of two tiles on short rows: of four
 // 0.5 us slower on 2 x 4 of 700.
 template <int NSET, bool FLAT>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {

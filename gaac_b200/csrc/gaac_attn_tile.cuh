@@ -1,10 +1,12 @@
 // Warp-level pieces of the fused decode attention: asynchronous copies, the rebuild of a compressed 16-token tile into tensor-core
 // fragments, the score and value products and the online softmax step.  Used by the kernels of gaac_attn.cu.
 //
-// What bounds them: instruction issue, not HBM.  Measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens: 1090 warp instructions per (K
-// tile + V tile), the ALU pipe and the shared-memory pipe at 70 % each and 0.68 instructions per cycle and scheduler inside the main loop, with four warps
-// to a scheduler.  Timing-only builds of a near form: without the raw groups 50 us of 57, without any of plan_tile 41.  What did not help: moving shifts from the
-// ALU to the FMA pipe, fewer or longer chains at the same count of instructions, warps of their own for plan_tile or for the copies (see gaac_attn.cu).
+// What bounds them, measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens: 1062 warp instructions per (K tile + V tile) at 0.64 per cycle and scheduler, with
+// four warps to a scheduler; ALU pipe 65 %, shared-memory pipe 62 % (of all cycles), DRAM 39 %.  A warp issues every 6.25 cycles and spends, of these, 1.2 waiting for a
+// result of fixed latency, 1.1 ready but not chosen, 0.9 on shared memory, 0.8 on a busy pipe (the ALU), 0.3 at barriers, 0.25 on global memory: instructions
+// first, then latency, since a third of the issue slots finds no warp ready.  More warps do not fit (gaac_attn.cu: 18 or 20 at 96 registers).  Timing-only builds of an earlier
+// form: without the raw groups 50 us of 57, without any of plan_tile 41.  What did not help: moving shifts from the ALU to the FMA pipe, fewer or longer chains at the same
+// count of instructions, warps of their own for plan_tile or for the copies.
 //
 // Head columns.  The tensor-core tile has 8 columns.  Query heads are handled in sets of four (NSET = 1 for a GQA group of up to
 // 4, 2 for 5..8); lane j of a quad works for head 4 * set + j throughout:

@@ -132,13 +132,12 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
     lengths and plans accordingly, the grid's split count cannot.
     A flat launch saves what comes with the waves of a grid, and the idle end of the last one; it pays some 8 us for every piece of a row that a CTA has beyond its
     first.  us, other form -> flat:
-      grids of several waves: 64 rows x 1 kv head, 32K tokens 222 -> 202;  16 x 8, 4K-64K 455 -> 402;  40 x 4, 2K-6K 95 -> 76;  20 x 8, 2K-3K 71 -> 53;  64 x 8, 500-4200 164 -> 143.
-        Short rows in a table that fits them are even: 64 x 8, 100-400 31.7 -> 32.0;  32 x 8, 20-2000 41 -> 42;  24 x 8, 64-600 16.3 -> 16.7;  in one of 8192 tokens they take 58, 69 and 33 as
+      grids of several waves: 64 rows x 1 kv head, 32K tokens 219 -> 202;  16 x 8, 4K-64K 452 -> 403;  40 x 4, 2K-6K 98 -> 76;  20 x 8, 2K-3K 68 -> 54;  64 x 8, 500-4200 162 -> 143.
+        Short rows in a table that fits them are even: 64 x 8, 100-400 31.6 -> 32.0;  32 x 8, 20-2000 41 -> 42;  24 x 8, 64-600 16.4 -> 16.8;  in one of 8192 tokens they take 57, 68 and 32 as
         a grid
-      one wave: 64 x 2, 4K-8K 116 -> 101;  64 x 1, 8K-16K 118 -> 91;  37 x 4, 8K each 110 -> 108
-      shares of units, which come in whole ones: a fifth of them or more for the rows' first units 8 x 8, 4K-16K 94 -> 80;  4 x 8, 20K-32K 104 -> 95;  5 x 8, up to 9K 31.7 ->
-        30.6;  short rows there pay up to 0.8 us for the plan (8 x 8, 200-3000 14.9 -> 15.7);  fewer, 16 x 1 36 -> 39, 8 x 1 36.4 -> 36.9;  more than four query heads per kv head, 6 x 8
-        61 -> 64."""
+      one wave: 64 x 2, 4K-8K 98 -> 86;  64 x 1, 8K-16K 113 -> 87;  37 x 4, 8K each, paged 118 -> 108, slots 105.5 -> 108.1
+      shares of units, which come in whole ones: a fifth of them or more for the rows' first units 8 x 8, 4K-16K 89 -> 77;  4 x 8, 20K-32K 99 -> 91;  5 x 8, 1K-9K 25.3 -> 25.9;  short rows
+        there pay for the plan (8 x 8, 200-3000 14.9 -> 15.6);  fewer, 16 x 1 24.6 -> 25.4, 8 x 1 24.8 -> 26.2;  more than four query heads per kv head, 6 x 8 37.6 -> 38.1."""
     rows, tiles = B * n_kv, -(-S // 16)
     if B <= 1 or tiles < 160 or rows * tiles < 120 * sm_count or not _flat_line(rows, max(S, most)):
         return 0
@@ -149,10 +148,10 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
 
 @functools.lru_cache(maxsize=4096)
 def choose_flat256(B: int, n_kv: int, S: int, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
-    """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.4 -> 24.9;  20 x 8, up to 3K 89 -> 72;  32 x 2, up
-    to 4K 57 -> 42;  6 x 2, up to 60K 129 -> 94;  8 x 4, 100-700 22.3 -> 13.2;  2 x 8 of 1000 31 -> 13;  32 x 4, up to 1000 30.7 -> 31.3, in a table of 8192 44 -> 31.3;  32 x 8 the same 53 -> 40,
-    66 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.6 -> 47.4;  so are a few very short ones: 4 x 4 of 50-300 in a table of 8192 9.3 -> 11.0;  one sequence has nothing
-    to gain: 1 x 4 of 8K 18.4 -> 18.6."""
+    """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.1 -> 24.8;  20 x 8, up to 3K 95 -> 73;  32 x 2, up
+    to 4K 56 -> 40;  6 x 2, up to 60K 124 -> 93;  8 x 4, 100-700 22.0 -> 13.2;  2 x 8 of 1000 30 -> 13;  9 x 4, up to 1500 23.8 -> 16.6;  30 x 4, up to 2K 55 -> 48;  32 x 4, up to 1000 30.7 -> 31.4,
+    in a table of 8192 43 -> 31;  32 x 8 the same 53 -> 40, 65 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.3 -> 47.6;  so are a few very short ones: 4 x 4 of 50-300 in a
+    table of 8192 9.4 -> 11.0;  one sequence has nothing to gain: 1 x 4 of 8K 17.9 -> 18.4."""
     rows, tiles = B * n_kv, -(-S // 16)
     if B <= 1 or not _flat_line(rows, max(S, most)):
         return 0

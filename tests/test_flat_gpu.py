@@ -1,5 +1,5 @@
 """One wave of CTAs over the tiles of all rows and kv heads (gaac_decode_attn_flat, gaac_paged_decode_attn_flat): every row against the fp64 oracle, with one CTA
-for everything, a few, as many as there are SMs and more than there are tiles; empty rows, rows that are all tail, padding rows, 1 to 70 rows; V
+for everything, a few, as many as there are SMs and more than there are tiles; empty rows, rows that are all tail, padding rows, 1 to 2049 rows; V
 elements that are not finite (their CTA repeats its piece)."""
 import numpy as np
 import pytest
