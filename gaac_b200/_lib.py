@@ -125,8 +125,9 @@ def ptr(t):
 def stream_ptr(device=None):
     """The current stream of a device.  torch.cuda.current_stream makes a Stream object, 2.3 us of the ten or so that a call of this package costs; the function
     underneath it takes 0.1 us."""
-    if getattr(device, "type", None) == "cuda" and device.index is not None:          # (a string has an `index` too; "cuda:0", a number or None take the way below)
-        return _raw_stream(device.index)
+    index = getattr(device, "index", None)
+    if type(index) is int and device.type == "cuda":           # (a string's `index` is a method; "cuda:0", a number or None take the way below)
+        return _raw_stream(index)
     import torch
     return torch.cuda.current_stream(device).cuda_stream
 

@@ -27,11 +27,12 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     if not (1 <= G <= 8): raise RuntimeError("G must be 1..8")
     if TS % 16: raise RuntimeError("tile stride must be a multiple of 16")
     if not q.is_cuda: raise RuntimeError("gaac_b200 attention needs CUDA tensors: there is no CPU path")
+    bt_stride = _lib.row_stride(bt)
     units = flat = 0
     if nsplit is None:
         units = choose_units(B, n_kv, bt.shape[1] * 16)
         nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)        # with units: what the workspace must have room for
-        flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv, _lib.row_stride(bt) * 16)
+        flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv, bt_stride * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)
     st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
                     bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), n_kv, TS, TS - 2880)
@@ -39,6 +40,6 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     ws = workspace(q.device, B, n_q, nsplit, stream)
     lib = _lib.lib()
     name = "gaac_paged_decode_attn_flat" if flat else "gaac_paged_decode_attn_balanced" if units else "gaac_paged_decode_attn"
-    _lib.check(getattr(lib, name)(st, bt.data_ptr(), _lib.row_stride(bt), seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit),
+    _lib.check(getattr(lib, name)(st, bt.data_ptr(), bt_stride, seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit),
                                   ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), name)
     return out
