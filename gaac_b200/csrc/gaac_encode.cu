@@ -6,7 +6,16 @@
 namespace gaac {
 
 constexpr int ENC_WARPS = 4;          // warps per CTA
-constexpr int ENC_TILES_PER_WARP = 4; // consecutive work items of one warp share the head's base words
+// Tiles of a warp, which share the head's base words (and, in the decoder, the CTA's tables).  A launch that fits the SMs a few times over is as long as a warp's tiles take one after
+// the other, so a warp has one while the CTAs are fewer than twice what the SMs hold, and more only as the waves of CTAs become many.
+//  encoder (5 CTAs per SM)  us with 1 / 2 / 4 tiles: [8, 1111, 128] 3.3 / 4.2 / 6.3;  a prompt of 4001 tokens, 8 heads, K and V 8.0 / 8.2 / 9.2;  [8, 65536, 128] 47.4 / 42.3 / 41.7 (12: 46.1)
+//  decoder (8 CTAs per SM)  [8, 4001, 128] 4.9 / 5.9 / 8.4;  [8, 65536, 128] K and V 86.7 / 83.1 / 83.8 (7, every SM filled exactly once: 93.7)
+constexpr int ENC_RESIDENT = 5 * 148, ENC_MOST = 4, DEC_RESIDENT = 8 * 148, DEC_MOST = 2;
+static_assert(2 * DEC_MOST <= 32, "a lane for either end of each tile's escape bytes");
+static int tiles_per_warp(int64_t ntiles, int64_t rows, int resident, int most) {
+  const int64_t ctas = (ntiles + ENC_WARPS - 1) / ENC_WARPS * rows;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(most, ctas / resident));
+}
 
 // What one kind's encode reads and writes.
 struct EncodeSide {
@@ -14,7 +23,7 @@ struct EncodeSide {
   uint8_t *sm, *codes; int* flags; uint8_t* slots; int* tile_bytes;
   int* clear;                     // optional: a word that the first block sets to zero (the ticket of the scan, a status word)
 };
-struct EncodeParams { EncodeSide side[2]; long S, x_head_stride, x_row_stride, S_pad; const int* bidx; int n_kv, ntiles; };
+struct EncodeParams { EncodeSide side[2]; long S, x_head_stride, x_row_stride, S_pad; const int* bidx; int n_kv, ntiles, per_warp; };
 
 // One warp per (head, tile).  Token t of head h is read at x + h * x_head_stride + t * x_row_stride (bf16 elements): head-major [H, S_in, 128] or
 // token-major [L, n_kv, 128] input.
@@ -26,7 +35,7 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
   const int brow = p.bidx ? p.bidx[h] : (int)(h % p.n_kv);
   u32 b3w[8], b4w[8];
   load_base_words<KIND_V>(s.base3 + (long)brow * D, s.base4 + (long)brow * D, lane, b3w, b4w);
-  const int tile0 = blockIdx.x * (ENC_WARPS * ENC_TILES_PER_WARP) + warp;
+  const int tile0 = blockIdx.x * (ENC_WARPS * p.per_warp) + warp;
   const uint16_t* xh = s.x + h * p.x_head_stride;
   auto fetch = [&](int i) {                           // rows of the warp's i-th tile into scratch[i & 1]
     const long row0 = (long)(tile0 + i * ENC_WARPS) * T;
@@ -34,10 +43,10 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
     async_commit();
   };
   if (tile0 < ntiles) fetch(0);
-  for (int i = 0; i < ENC_TILES_PER_WARP; i++) {
+  for (int i = 0; i < p.per_warp; i++) {
     const int tile = tile0 + i * ENC_WARPS;
     if (tile >= ntiles) break;                       // warp-uniform
-    const bool more = i + 1 < ENC_TILES_PER_WARP && tile + ENC_WARPS < ntiles;
+    const bool more = i + 1 < p.per_warp && tile + ENC_WARPS < ntiles;
     __syncwarp();                                    // the other scratch was read by the tile before this one
     if (more) { fetch(i + 1); async_wait<1>(); } else async_wait<0>();
     WarpScratch& ws = scratch[i & 1][warp];
@@ -59,7 +68,7 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
     if (lane == 0) s.tile_bytes[h * ntiles + tile] = total;
   }
 }
-// KIND 0 / 1: K or V alone, grid = (ceil(ntiles / 16), H).  2: both, grid z = kind (a prompt's K and V: one launch, and short prompts leave
+// KIND 0 / 1: K or V alone, grid = (ceil(ntiles / (4 * per_warp)), H).  2: both, grid z = kind (a prompt's K and V: one launch, and short prompts leave
 // half as much of the GPU idle).
 template <int KIND>
 __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(const __grid_constant__ EncodeParams p) {
@@ -70,7 +79,7 @@ __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(const __gr
   if (KIND != 0 && v) encode_tiles_cta<1>(p, p.side[KIND == 2 ? 1 : 0], scratch, esc_stage[threadIdx.x >> 5]);
   if (KIND != 1 && !v) encode_tiles_cta<0>(p, p.side[0], scratch, esc_stage[threadIdx.x >> 5]);
 }
-static dim3 encode_grid(int ntiles, int64_t H, int kinds) { return dim3((ntiles + ENC_WARPS * ENC_TILES_PER_WARP - 1) / (ENC_WARPS * ENC_TILES_PER_WARP), (unsigned)H, (unsigned)kinds); }
+static dim3 encode_grid(int ntiles, int64_t H, int kinds, int per_warp) { return dim3((ntiles + ENC_WARPS * per_warp - 1) / (ENC_WARPS * per_warp), (unsigned)H, (unsigned)kinds); }
 
 // head_start[0..H] = exclusive prefix of head_bytes, by one CTA of SCAN_THREADS threads (H is the number of cache heads).
 // total: optional, the sum once more (page-locked host memory, which the end of the kernel makes visible).
@@ -231,22 +240,25 @@ static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_i
 
 // One warp per (head, tile): compressed tile -> bf16 rows.  Bound by latency and the warps that hide it: the escape bytes are asked for with the tile, their number taken from
 // the offset of the next tile (not of a head's last one), and the registers leave room for 8 CTAs of K, 7 of V.  [8, 65536, 128] K and V: 98.5 -> 93.7 us; with 6
-// CTAs each 102, and with the next tile's words asked for while one is rebuilt (5 CTAs) 101.
+// CTAs each 102, and with the next tile's words asked for while one is rebuilt (5 CTAs) 101.  Launched overlapped, with two tiles per warp: 90.3 -> 83.1 a call of each.  No help: 32-byte
+// stores (85.6), evict-first stores (83.5) or loads (85.4), CTAs of two warps (92.6).
 template <int KIND_V>
 __global__ void __launch_bounds__(ENC_WARPS * 32, KIND_V ? 7 : 8) decode_page_kernel(
     const uint8_t* __restrict__ sm, const uint8_t* __restrict__ codes, const int* __restrict__ flags, const int* __restrict__ tile_off,
     long tile_off_stride, const uint8_t* __restrict__ ovf, const int* __restrict__ head_start, const uint8_t* __restrict__ base3,
-    const uint8_t* __restrict__ base4, const int* __restrict__ bidx, int n_kv, long S, long S_pad, uint16_t* __restrict__ out, int ntiles) {
+    const uint8_t* __restrict__ base4, const int* __restrict__ bidx, int n_kv, long S, long S_pad, uint16_t* __restrict__ out, int ntiles, int per_warp) {
   __shared__ __align__(16) DecodeScratch scratch[ENC_WARPS];
   __shared__ __align__(16) DecodeTables tables;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long h = blockIdx.y;
   DecodeScratch& ws = scratch[warp];
+  griddep_wait();
+  griddep_launch();
   const int brow = bidx ? bidx[h] : (int)(h % n_kv);
   const uint8_t* esc_head = ovf + (long)head_start[h];
-  const int tile0 = blockIdx.x * (ENC_WARPS * ENC_TILES_PER_WARP) + warp;
+  const int tile0 = blockIdx.x * (ENC_WARPS * per_warp) + warp;
   const int mine = tile0 + (lane >> 1) * ENC_WARPS + (lane & 1);                           // lanes 2i, 2i + 1: where the warp's i-th tile's escape bytes begin and end
-  const int off = lane < 2 * ENC_TILES_PER_WARP && mine < ntiles ? tile_off[h * tile_off_stride + mine] : 0;
+  const int off = lane < 2 * per_warp && mine < ntiles ? tile_off[h * tile_off_stride + mine] : 0;
   TileWords<KIND_V> tw;
   const auto ask = [&](int i) {                       // the words of the warp's i-th tile, escape bytes included where the next tile's offset says how many
     const int tile = tile0 + i * ENC_WARPS, from = __shfl_sync(FULL, off, 2 * i), to = __shfl_sync(FULL, off, 2 * i + 1);
@@ -257,7 +269,7 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, KIND_V ? 7 : 8) decode_page_ke
   const WarpView w = fill_decode_tables<KIND_V>(tables, base3 + (long)brow * D, base4 + (long)brow * D);
   __syncthreads();
 #pragma unroll 1
-  for (int i = 0; i < ENC_TILES_PER_WARP; i++) {
+  for (int i = 0; i < per_warp; i++) {
     const int tile = tile0 + i * ENC_WARPS;
     if (tile >= ntiles) break;
     const long row0 = (long)tile * T;
@@ -390,10 +402,10 @@ static int encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, 
   if (H <= 0 || S <= 0 || S_in < S || S_pad < (S + T - 1) / T * T || S_pad % T || n_kv <= 0 || H > 65535 || (kind != GAAC_KIND_K && kind != GAAC_KIND_V)) return GAAC_E_ARG;
   if (!aligned16(x_bf16) || !aligned16(sm) || !aligned16(codes)) return GAAC_E_ALIGN;
   const int ntiles = (int)((S + T - 1) / T);
-  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles};
+  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles, tiles_per_warp(ntiles, H, ENC_RESIDENT, ENC_MOST)};
   cudaStream_t st = (cudaStream_t)stream;
-  if (kind == GAAC_KIND_K) encode_tiles_kernel<0><<<encode_grid(ntiles, H, 1), ENC_WARPS * 32, 0, st>>>(p);
-  else encode_tiles_kernel<1><<<encode_grid(ntiles, H, 1), ENC_WARPS * 32, 0, st>>>(p);
+  if (kind == GAAC_KIND_K) encode_tiles_kernel<0><<<encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, 0, st>>>(p);
+  else encode_tiles_kernel<1><<<encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, 0, st>>>(p);
   return launch_status();
 }
 
@@ -465,13 +477,10 @@ extern "C" int gaac_decode_page(const uint8_t* sm, const uint8_t* codes, const i
   if (H <= 0 || S <= 0 || S_pad < (S + T - 1) / T * T || S_pad % T || n_kv <= 0 || H > 65535 || (kind != GAAC_KIND_K && kind != GAAC_KIND_V)) return GAAC_E_ARG;
   if (!aligned16(sm) || !aligned16(codes) || !aligned16(out_bf16)) return GAAC_E_ALIGN;
   const int ntiles = (int)((S + T - 1) / T);
-  dim3 grid((ntiles + ENC_WARPS * ENC_TILES_PER_WARP - 1) / (ENC_WARPS * ENC_TILES_PER_WARP), (unsigned)H);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (kind == GAAC_KIND_K)
-    decode_page_kernel<0><<<grid, ENC_WARPS * 32, 0, st>>>(sm, codes, flags, tile_off, tile_off_stride, ovf, head_start, base3, base4, bidx, n_kv, S, S_pad, (uint16_t*)out_bf16, ntiles);
-  else
-    decode_page_kernel<1><<<grid, ENC_WARPS * 32, 0, st>>>(sm, codes, flags, tile_off, tile_off_stride, ovf, head_start, base3, base4, bidx, n_kv, S, S_pad, (uint16_t*)out_bf16, ntiles);
-  return launch_status();
+  const int per_warp = tiles_per_warp(ntiles, H, DEC_RESIDENT, DEC_MOST);
+  const dim3 grid((ntiles + ENC_WARPS * per_warp - 1) / (ENC_WARPS * per_warp), (unsigned)H);
+  return launch_overlapped(kind == GAAC_KIND_K ? decode_page_kernel<0> : decode_page_kernel<1>, grid, ENC_WARPS * 32, (cudaStream_t)stream, sm, codes, flags, tile_off, tile_off_stride, ovf,
+                           head_start, base3, base4, bidx, n_kv, S, S_pad, (uint16_t*)out_bf16, ntiles, per_warp);
 }
 
 static dim3 hist_grid(int64_t n_ch, int64_t N, int kinds) { return dim3((unsigned)((n_ch + 127) / 128), (unsigned)((N + HIST_ROWS - 1) / HIST_ROWS), (unsigned)kinds); }
@@ -566,13 +575,13 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
     sp.side[kind] = ScanSide{tbytes, toff, s->ovf_used + h0};
     cp.side[kind] = CompactSide{slots, tbytes, toff, nullptr, s->ovf + h0 * ovf_cap, nullptr, nullptr, status + 2 * kind};
   }
-  ep.S = S; ep.x_head_stride = D; ep.x_row_stride = row_stride; ep.S_pad = S_cap; ep.n_kv = n_kv; ep.ntiles = ntiles;
+  ep.S = S; ep.x_head_stride = D; ep.x_row_stride = row_stride; ep.S_pad = S_cap; ep.n_kv = n_kv; ep.ntiles = ntiles; ep.per_warp = tiles_per_warp(ntiles, 2 * n_kv, ENC_RESIDENT, ENC_MOST);
   sp.ntiles = ntiles; sp.tile_off_stride = tiles_cap;
   cp.ntiles = ntiles; cp.n_items = (unsigned)n_items; cp.tile_off_stride = tiles_cap; cp.head_stride = ovf_cap; cp.head_cap = ovf_cap - CACHE_READ_PAD;
   cp.finish = !copy_only; cp.fin = fin;
   if (copy_only) { if (int e = clear_status(status, st)) return e; }
   else {
-    encode_tiles_kernel<2><<<encode_grid(ntiles, n_kv, 2), ENC_WARPS * 32, 0, st>>>(ep);
+    encode_tiles_kernel<2><<<encode_grid(ntiles, n_kv, 2, ep.per_warp), ENC_WARPS * 32, 0, st>>>(ep);
     if (int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)n_kv, 2), SCAN_THREADS, st, sp)) return e;
   }
   return launch_overlapped(compact_copy_kernel, compact_grid(cp, 2), 128, st, cp);
