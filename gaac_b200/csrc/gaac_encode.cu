@@ -279,83 +279,122 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, KIND_V ? 7 : 8) decode_page_ke
   }
 }
 
-// Exponent histogram: x [N rows, n_ch] bf16, row r at x + r * row_stride; hist [n_ch, 256] counts.  grid = (ceil(n_ch/128), row chunks, kinds).  A CTA
-// counts 128 channels in shared memory with 8-bit counters, four threads per channel, and flushes what is not zero with atomics.  Counter (bin,
-// channel) is byte bin & 3 of word [bin >> 2][channel]: a warp's increments go to 32 banks whatever the exponents are, and clearing and flushing handle
-// four bins at a time, nearly all of them empty.  Bound by latency, not by bytes: with one thread per channel and a load, add and store per
-// value it took 21 us for 2048 rows of 8 kv heads (15 us with 16-bit counters and chunks of 64 rows), now 7 us: the shared-memory atomic returns
-// nothing, so a thread never waits for a counter.
-constexpr int HIST_ROWS = 128, HIST_LANES = 4;         // rows per CTA (an 8-bit counter holds 255); threads per channel
+// Exponent histogram: x [N rows, n_ch] bf16, row r at x + r * row_stride; counts of channel c at hist + c * PER_CHANNEL.  grid = (ceil(n_ch/128), row chunks, kinds).  A CTA
+// counts 128 channels in shared memory with 8-bit counters and flushes what is not zero with atomics.  Counter (bin, place) is byte bin & 3 of word
+// [bin >> 2][place]: a warp's increments go to 32 banks whatever the exponents are, and clearing and flushing handle four bins at a time, nearly all of them empty.  PAIRS
+// (even strides, rows on 4-byte boundaries): a thread reads two neighbouring channels with one load, whose places are 64 apart.
+// Bound by latency and by the atomics of the flush, which go to a line each: so the prompt's histogram has 16-bit counts, four to a 64-bit atomic (Packed: prompts of up to 65535
+// tokens), which is a third of the atomics.  With one thread per channel and a load, add and store per value it took 21 us for 2048 rows of 8 kv heads (15 us with
+// 16-bit counters and chunks of 64 rows), 7 us as shared-memory atomics that return nothing.
+// Rows per CTA (an 8-bit counter holds 255) and threads.  us of a prompt's tables, 8 heads x 4001 tokens / 8 x 32768 / 1 x 4096: 128 rows, 256 threads 11.7 / 44 / 6.7;  512 threads 13.0 / 46 /
+// 6.2;  192 rows 11.8 / 41 / 7.2;  96 rows 12.7 / 49 / 6.5;  before, one channel per load and 32-bit counts 15.2 / 65 / 7.6.
+constexpr int HIST_ROWS = 128, HIST_THREADS = 256;
+typedef unsigned long long u64_t;
+struct Packed { u64_t four; };                        // counts of bins 4w .. 4w + 3, 16 bits each
+template <class Cnt> constexpr int PER_CHANNEL = 256;
+template <> constexpr int PER_CHANNEL<Packed> = 64;
 template <class Cnt> struct HistParams { const uint16_t* x[2]; Cnt* hist[2]; long N, n_ch, row_stride; };
-template <class Cnt>
-__global__ void __launch_bounds__(128 * HIST_LANES) exponent_hist_kernel(const __grid_constant__ HistParams<Cnt> p) {
+__device__ __forceinline__ void add_four(Packed* hist, int w, u32 four) { atomicAdd(&hist[w].four, (u64_t)prmt(four, 0u, 0x4140) | (u64_t)prmt(four, 0u, 0x4342) << 32); }
+template <class Cnt> __device__ __forceinline__ void add_four(Cnt* hist, int w, u32 four) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) { const u32 n = (four >> (8 * i)) & 0xFFu; if (n) atomicAdd(&hist[4 * w + i], (Cnt)n); }
+}
+// WAITS: the counters are cleared by the kernel in front, which this one does not wait for before it adds to them; x was there before that kernel.
+template <class Cnt, bool PAIRS, bool WAITS>
+__global__ void __launch_bounds__(HIST_THREADS) exponent_hist_kernel(const __grid_constant__ HistParams<Cnt> p) {
   __shared__ __align__(16) u32 bins[64][128];
-  const int ch = threadIdx.x & 127, sub = threadIdx.x >> 7;
-  const long c = (long)blockIdx.x * 128 + ch;
-  for (int i = threadIdx.x; i < 64 * 128 / 4; i += 128 * HIST_LANES) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
+  constexpr int WIDE = PAIRS ? 2 : 1, COLS = 128 / WIDE, LANES = HIST_THREADS / COLS;      // channels and threads side by side, threads per channel
+  const int col = threadIdx.x % COLS, sub = threadIdx.x / COLS;
+  const long c = (long)blockIdx.x * 128 + WIDE * col;
+  for (int i = threadIdx.x; i < 64 * 128 / 4; i += HIST_THREADS) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
   griddep_launch();
   __syncthreads();
   if (c < p.n_ch) {
     const uint16_t* x = p.x[blockIdx.z] + c;
-    const auto count = [&](u32 v) { atomicAdd(&bins[(v >> 9) & 0x3Fu][ch], 1u << (8u * ((v >> 7) & 3u))); };          // exponent = bits 7..14
+    const auto load = [&](long r) -> u32 { return PAIRS ? *reinterpret_cast<const u32*>(x + r * p.row_stride) : x[r * p.row_stride]; };
+    const auto count = [&](u32 v) {                   // exponent = bits 7..14
+      atomicAdd(&bins[(v >> 9) & 0x3Fu][col], 1u << (8u * ((v >> 7) & 3u)));
+      if (PAIRS) atomicAdd(&bins[(v >> 25) & 0x3Fu][64 + col], 1u << (8u * ((v >> 23) & 3u)));
+    };
     const long r1 = min(p.N, ((long)blockIdx.y + 1) * HIST_ROWS);
     long r = (long)blockIdx.y * HIST_ROWS + sub;
-    for (; r + 15 * HIST_LANES < r1; r += 16 * HIST_LANES) {          // sixteen independent loads in flight per thread
+    for (; r + 15 * LANES < r1; r += 16 * LANES) {    // sixteen independent loads in flight per thread
       u32 v[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) v[i] = x[(r + i * HIST_LANES) * p.row_stride];
+      for (int i = 0; i < 16; i++) v[i] = load(r + i * LANES);
 #pragma unroll
       for (int i = 0; i < 16; i++) count(v[i]);
     }
-    for (; r < r1; r += HIST_LANES) count(x[r * p.row_stride]);
+    for (; r < r1; r += LANES) count(load(r));
   }
   __syncthreads();
-  if (c >= p.n_ch) return;
-  Cnt* hist = p.hist[blockIdx.z] + c * 256;
+  const int place = threadIdx.x & 127;
+  const long ch = (long)blockIdx.x * 128 + (PAIRS ? 2 * (place & 63) + (place >> 6) : place);
+  if (WAITS) griddep_wait();
+  if (ch >= p.n_ch) return;
+  Cnt* hist = p.hist[blockIdx.z] + ch * PER_CHANNEL<Cnt>;
 #pragma unroll 8
-  for (int w = sub; w < 64; w += HIST_LANES) {
-    const u32 four = bins[w][ch];
-    if (four) {
-#pragma unroll
-      for (int i = 0; i < 4; i++) { const u32 n = (four >> (8 * i)) & 0xFFu; if (n) atomicAdd(&hist[4 * w + i], (Cnt)n); }
-    }
+  for (int w = threadIdx.x >> 7; w < 64; w += HIST_THREADS / 128) {
+    const u32 four = bins[w][place];
+    if (four) add_four(hist, w, four);
   }
 }
+// The counters of a prompt's histogram cleared (a kernel and not a memset, so that the counting need not wait for it).
+__global__ void __launch_bounds__(256) clear_kernel(u32* p, int n) {
+  griddep_launch();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) p[i] = 0u;
+}
 
-// One warp per histogram row: densest 8- and 16-wide window, first maximum wins.  grid y = kind.
+// One warp per histogram row: densest 8- and 16-wide window, first maximum wins.  grid y = kind.  A lane has eight neighbouring bins, so one scan over the lanes makes the prefix.
 template <class Cnt> struct BasesParams { const Cnt* hist[2]; uint8_t *base3[2], *base4[2]; long n_rows; };
+template <class Cnt> struct Counts {
+  typedef Cnt Sum;
+  static __device__ __forceinline__ void load(const Cnt* row, int lane, Cnt (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = row[8 * lane + i];
+  }
+};
+template <> struct Counts<Packed> {
+  typedef int Sum;
+  static __device__ __forceinline__ void load(const Packed* row, int lane, int (&v)[8]) {
+    const uint4 q = reinterpret_cast<const uint4*>(row)[lane];
+    const u32 w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = (int)((w[i >> 1] >> (16 * (i & 1))) & 0xFFFFu);
+  }
+};
 template <class Cnt>
 __global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_constant__ BasesParams<Cnt> p) {
-  __shared__ Cnt cs[4][257];
+  typedef typename Counts<Cnt>::Sum Sum;
+  __shared__ Sum cs[4][256 + 8 + 1];                  // [row of the CTA][bin + (bin >> 5)]: prefix of the counts, the lanes' eights in different banks
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long row = (long)blockIdx.x * 4 + warp;
-  if (row >= p.n_rows) return;
-  const Cnt* hist = p.hist[blockIdx.y] + row * 256;
   griddep_wait();
-  Cnt carry = 0;
-  if (lane == 0) cs[warp][0] = 0;
-  Cnt v[8];
+  griddep_launch();
+  if (row >= p.n_rows) return;
+  Sum v[8], own = 0;
+  Counts<Cnt>::load(p.hist[blockIdx.y] + row * PER_CHANNEL<Cnt>, lane, v);
 #pragma unroll
-  for (int b = 0; b < 8; b++) v[b] = hist[32 * b + lane];
+  for (int i = 0; i < 8; i++) own += v[i];
+  Sum inc = own;
 #pragma unroll
-  for (int b = 0; b < 8; b++) {
-    Cnt inc = v[b];
+  for (int d = 1; d < 32; d <<= 1) { const Sum u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
+  const auto at = [](int bin) { return bin + (bin >> 5); };
+  Sum before = inc - own;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { Cnt u = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += u; }
-    cs[warp][32 * b + lane + 1] = carry + inc;
-    carry += __shfl_sync(FULL, inc, 31);
-  }
+  for (int i = 0; i < 8; i++) { cs[warp][at(8 * lane + i)] = before; before += v[i]; }
+  if (lane == 31) cs[warp][at(256)] = before;
   __syncwarp();
   for (int k = 0; k < 2; k++) {
     const int w = k ? 16 : 8;
-    Cnt best = -1; int besti = 0;
+    Sum best = -1; int besti = 0;
     for (int s = lane; s <= 256 - w; s += 32) {
-      Cnt v = cs[warp][s + w] - cs[warp][s];
-      if (v > best) { best = v; besti = s; }
+      const Sum n = cs[warp][at(s + w)] - cs[warp][at(s)];
+      if (n > best) { best = n; besti = s; }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-      Cnt ob = __shfl_xor_sync(FULL, best, d); int oi = __shfl_xor_sync(FULL, besti, d);
+      const Sum ob = __shfl_xor_sync(FULL, best, d); const int oi = __shfl_xor_sync(FULL, besti, d);
       if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
     }
     if (lane == 0) (k ? p.base4[blockIdx.y] : p.base3[blockIdx.y])[row] = (uint8_t)besti;
@@ -483,6 +522,8 @@ extern "C" int gaac_decode_page(const uint8_t* sm, const uint8_t* codes, const i
                            head_start, base3, base4, bidx, n_kv, S, S_pad, (uint16_t*)out_bf16, ntiles, per_warp);
 }
 
+// a thread may read two channels at a time
+static bool hist_pairs(const void* x, int64_t n_ch, int64_t row_stride) { return (reinterpret_cast<uintptr_t>(x) & 3) == 0 && n_ch % 2 == 0 && row_stride % 2 == 0; }
 static dim3 hist_grid(int64_t n_ch, int64_t N, int kinds) { return dim3((unsigned)((n_ch + 127) / 128), (unsigned)((N + HIST_ROWS - 1) / HIST_ROWS), (unsigned)kinds); }
 
 extern "C" int gaac_exponent_hist(const void* x_bf16, int64_t N, int64_t n_ch, long long* hist, void* stream) {
@@ -492,7 +533,8 @@ extern "C" int gaac_exponent_hist(const void* x_bf16, int64_t N, int64_t n_ch, l
   for (int64_t r = 0; r < N; r += MOST) {
     const int64_t rows = std::min(MOST, N - r);
     const HistParams<unsigned long long> p{{(const uint16_t*)x_bf16 + r * n_ch, nullptr}, {(unsigned long long*)hist, nullptr}, rows, n_ch, n_ch};
-    exponent_hist_kernel<<<hist_grid(n_ch, rows, 1), 128 * HIST_LANES, 0, (cudaStream_t)stream>>>(p);
+    if (hist_pairs(p.x[0], n_ch, n_ch)) exponent_hist_kernel<unsigned long long, true, false><<<hist_grid(n_ch, rows, 1), HIST_THREADS, 0, (cudaStream_t)stream>>>(p);
+    else exponent_hist_kernel<unsigned long long, false, false><<<hist_grid(n_ch, rows, 1), HIST_THREADS, 0, (cudaStream_t)stream>>>(p);
   }
   return launch_status();
 }
@@ -508,6 +550,20 @@ constexpr int CACHE_READ_PAD = 8;      // bytes kept free behind a head's escape
 
 extern "C" size_t gaac_cache_calibrate_scratch_bytes(int n_kv) { return 2 * (size_t)(n_kv > 0 ? n_kv : 0) * D * 256 * sizeof(int32_t); }
 
+// Three launches: counters cleared, histograms of both kinds, windows into the slot's rows of the tables.
+template <class Cnt>
+static int calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, long n_ch, long at, uint8_t* scratch, bool pairs, cudaStream_t st) {
+  Cnt* hist = reinterpret_cast<Cnt*>(scratch);
+  const long one = n_ch * PER_CHANNEL<Cnt>;
+  const int n = (int)(2 * one * sizeof(Cnt) / 4);
+  clear_kernel<<<std::min(n / 256, 8 * 148), 256, 0, st>>>(reinterpret_cast<u32*>(scratch), n);
+  const HistParams<Cnt> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + one}, L, n_ch, row_stride};
+  if (int e = launch_overlapped(pairs ? exponent_hist_kernel<Cnt, true, true> : exponent_hist_kernel<Cnt, false, true>, hist_grid(n_ch, L, 2), HIST_THREADS, st, hp)) return e;
+  const BasesParams<Cnt> bp{{hist, hist + one}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
+                            {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch};
+  return launch_overlapped(bases_from_hist_kernel<Cnt>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
+}
+
 extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
                                     int n_base_rows, uint8_t* scratch, size_t scratch_bytes, void* stream) {
   if (!K || !V || !K->base3 || !K->base4 || !V->base3 || !V->base4 || !k_tok || !v_tok || !scratch) return GAAC_E_ARG;
@@ -516,13 +572,9 @@ extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, co
   if (reinterpret_cast<uintptr_t>(scratch) & 3) return GAAC_E_ALIGN;
   cudaStream_t st = (cudaStream_t)stream;
   const long n_ch = (long)n_kv * D, at = (long)slot * n_ch;
-  int* hist = reinterpret_cast<int*>(scratch);
-  if (cudaMemsetAsync(hist, 0, gaac_cache_calibrate_scratch_bytes(n_kv), st) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
-  const HistParams<int> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + n_ch * 256}, L, n_ch, row_stride};
-  exponent_hist_kernel<<<hist_grid(n_ch, L, 2), 128 * HIST_LANES, 0, st>>>(hp);
-  const BasesParams<int> bp{{hist, hist + n_ch * 256}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
-                            {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch};
-  return launch_overlapped(bases_from_hist_kernel<int>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
+  const bool pairs = hist_pairs(k_tok, n_ch, row_stride) && hist_pairs(v_tok, n_ch, row_stride);
+  return L <= 0xFFFF && !(reinterpret_cast<uintptr_t>(scratch) & 15) ? calibrate<Packed>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, pairs, st)
+                                                                      : calibrate<int>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, pairs, st);
 }
 
 static int clear_status(int32_t* status, cudaStream_t st) {           // the words that say whether an escape stream had room
