@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(64) append_kv_kernel(const __grid_constant__ A
   __shared__ __align__(16) WarpScratch scratch[2];
   __shared__ int s_fit[2];
   const int i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  griddep_wait();
   griddep_launch();                                   // the step's attention may set up its tables meanwhile
   const int sl = p.slot[i / p.n_kv];
   if (sl < 0) return;
@@ -149,6 +150,7 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
 __global__ void __launch_bounds__(32) paged_store_kernel(const __grid_constant__ PagedParams p) {
   __shared__ __align__(16) WarpScratch ws;
   const int e = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
+  griddep_wait();
   griddep_launch();
   const int freed = t & 1 ? store_one<1>(ws, p, e, t, lane) : store_one<0>(ws, p, e, t, lane);
   if (lane == 0) p.freeq[e * 2 * p.st.n_kv + t] = freed;
@@ -163,6 +165,7 @@ static_assert(STEP_WARPS * sizeof(WarpScratch) <= 48 * 1024 && (STEP_WARPS + 1) 
 __global__ void __launch_bounds__(STEP_WARPS * 32) paged_store_step_kernel(const __grid_constant__ PagedParams p, int n_items) {
   __shared__ __align__(16) WarpScratch ws[STEP_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x * STEP_WARPS + warp, NT = 2 * p.st.n_kv;
+  griddep_wait();
   griddep_launch();
   int freed = -1;
   if (i < n_items) freed = i & 1 ? store_one<1>(ws[warp], p, i / NT, i % NT, lane) : store_one<0>(ws[warp], p, i / NT, i % NT, lane);
@@ -202,6 +205,8 @@ __device__ __forceinline__ void decode_blocks_cta(DecodeScratch* scratch, Decode
   const gaac_paged& st = p.st;
   const int kvh = t >> 1, NT = 2 * st.n_kv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x * PDEC_WARPS + warp;
   DecodeScratch& ws = scratch[warp];
+  griddep_wait();
+  griddep_launch();
   // the tile travels while the tables are made
   int row0 = 0, nvalid = 0, m = 0;
   TileWords<KIND_V> tw;
@@ -256,8 +261,7 @@ extern "C" int gaac_append_kv(const gaac_store* K, const gaac_store* V, const vo
   }
   if ((reinterpret_cast<uintptr_t>(k_new) & 7) || (reinterpret_cast<uintptr_t>(v_new) & 7)) return GAAC_E_ALIGN;
   AppendParams p{*K, *V, (const uint16_t*)k_new, (const uint16_t*)v_new, slot, n_kv, tail_len, seq_len, S_cap, ovf_cap, n_base_rows, err};
-  append_kv_kernel<<<(unsigned)(B * n_kv), 64, 0, (cudaStream_t)stream>>>(p);
-  return launch_status();
+  return launch_overlapped(append_kv_kernel, dim3((unsigned)(B * n_kv)), 64, (cudaStream_t)stream, p);
 }
 
 extern "C" int gaac_paged_store(const gaac_paged* st, const void* key, const void* value, int64_t k_stride, int64_t v_stride,
@@ -274,15 +278,15 @@ extern "C" int gaac_paged_store(const gaac_paged* st, const void* key, const voi
     while (blocks * STEP_WARPS < items) blocks *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(STEP_WARPS * 32); cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = g_launch_overlap;
+    cfg.attrs = at; cfg.numAttrs = 2;
     if (cudaLaunchKernelEx(&cfg, paged_store_step_kernel, p, (int)items) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
     return launch_status();
   }
-  paged_store_kernel<<<dim3((unsigned)E, (unsigned)(2 * st->n_kv)), 32, 0, s>>>(p);
+  if (int err = launch_overlapped(paged_store_kernel, dim3((unsigned)E, (unsigned)(2 * st->n_kv)), 32, s, p)) return err;
   const int n = E * 2 * st->n_kv;
-  if (int err = launch_status()) return err;
   return launch_overlapped(free_tiles_kernel, dim3((n + 255) / 256), 256, s, freeq, n, st->stack, st->top);
 }
 
@@ -300,8 +304,7 @@ extern "C" int gaac_paged_decode_blocks(const gaac_paged* st, const int32_t* pai
   if (!aligned16(sk) || !aligned16(sv) || row_stride % 8) return GAAC_E_ALIGN;
   if (P == 0) return GAAC_OK;
   PagedDecodeParams p{*st, pairs, P, (uint16_t*)sk, (uint16_t*)sv, row_stride};
-  paged_decode_blocks_kernel<<<dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)), PDEC_WARPS * 32, 0, (cudaStream_t)stream>>>(p);
-  return launch_status();
+  return launch_overlapped(paged_decode_blocks_kernel, dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)), PDEC_WARPS * 32, (cudaStream_t)stream, p);
 }
 
 extern "C" const char* gaac_status_string(int status) {

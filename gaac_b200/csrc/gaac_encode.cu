@@ -74,6 +74,7 @@ template <int KIND>
 __global__ void __launch_bounds__(ENC_WARPS * 32) encode_tiles_kernel(const __grid_constant__ EncodeParams p) {
   __shared__ __align__(16) WarpScratch scratch[2][ENC_WARPS];       // two per warp: the next tile's rows arrive while this one is encoded
   __shared__ __align__(16) uint8_t esc_stage[ENC_WARPS][TILE_MAX_ESC];
+  griddep_wait();
   griddep_launch();
   const bool v = KIND == 2 ? blockIdx.z != 0 : KIND == 1;
   if (KIND != 0 && v) encode_tiles_cta<1>(p, p.side[KIND == 2 ? 1 : 0], scratch, esc_stage[threadIdx.x >> 5]);
@@ -442,10 +443,7 @@ static int encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, 
   if (!aligned16(x_bf16) || !aligned16(sm) || !aligned16(codes)) return GAAC_E_ALIGN;
   const int ntiles = (int)((S + T - 1) / T);
   const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles, tiles_per_warp(ntiles, H, ENC_RESIDENT, ENC_MOST)};
-  cudaStream_t st = (cudaStream_t)stream;
-  if (kind == GAAC_KIND_K) encode_tiles_kernel<0><<<encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, 0, st>>>(p);
-  else encode_tiles_kernel<1><<<encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, 0, st>>>(p);
-  return launch_status();
+  return launch_overlapped(kind == GAAC_KIND_K ? encode_tiles_kernel<0> : encode_tiles_kernel<1>, encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, (cudaStream_t)stream, p);
 }
 
 extern "C" int gaac_encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
@@ -633,7 +631,7 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   cp.finish = !copy_only; cp.fin = fin;
   if (copy_only) { if (int e = clear_status(status, st)) return e; }
   else {
-    encode_tiles_kernel<2><<<encode_grid(ntiles, n_kv, 2, ep.per_warp), ENC_WARPS * 32, 0, st>>>(ep);
+    if (int e = launch_overlapped(encode_tiles_kernel<2>, encode_grid(ntiles, n_kv, 2, ep.per_warp), ENC_WARPS * 32, st, ep)) return e;
     if (int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)n_kv, 2), SCAN_THREADS, st, sp)) return e;
   }
   return launch_overlapped(compact_copy_kernel, compact_grid(cp, 2), 128, st, cp);
