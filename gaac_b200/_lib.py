@@ -66,6 +66,8 @@ _SIGNATURES = {
     "gaac_cache_calibrate": (i32, [C.POINTER(Store), C.POINTER(Store), vp, vp, i64, i64, i32, i32, i32, vp, C.c_size_t, vp]),
     "gaac_cache_prefill_scratch_bytes": (C.c_size_t, [i64, i32]),
     "gaac_cache_prefill": (i32, [C.POINTER(Store), C.POINTER(Store), vp, vp, i64, i64, i32, i32, vp, vp, i64, i64, i32, vp, C.c_size_t, vp, i32, vp]),
+    "gaac_cache_tables_workspace_bytes": (C.c_size_t, [i32]),
+    "gaac_cache_prefill_own": (i32, [C.POINTER(Store), C.POINTER(Store), vp, vp, i64, i64, i32, i32, vp, vp, i64, i64, i32, vp, C.c_size_t, vp, vp, C.c_size_t, vp]),
     "gaac_paged_store": (i32, [C.POINTER(Paged), vp, vp, i64, i64, vp, i32, vp, vp]),
     "gaac_paged_release": (i32, [C.POINTER(Paged), vp, i32, vp]),
     "gaac_paged_decode_blocks": (i32, [C.POINTER(Paged), vp, i32, vp, vp, i64, vp]),

@@ -22,6 +22,7 @@ struct EncodeSide {
   const uint16_t* x; const uint8_t *base3, *base4;
   uint8_t *sm, *codes; int* flags; uint8_t* slots; int* tile_bytes;
   int* clear;                     // optional: a word that the first block sets to zero (the ticket of the scan, a status word)
+  int* cta_bytes;                 // optional: escape bytes of the tiles of every CTA, [H][gridDim.x]
 };
 struct EncodeParams { EncodeSide side[2]; long S, x_head_stride, x_row_stride, S_pad; const int* bidx; int n_kv, ntiles, per_warp; };
 
@@ -43,6 +44,7 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
     async_commit();
   };
   if (tile0 < ntiles) fetch(0);
+  int sum = 0;
   for (int i = 0; i < p.per_warp; i++) {
     const int tile = tile0 + i * ENC_WARPS;
     if (tile >= ntiles) break;                       // warp-uniform
@@ -66,6 +68,18 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
       for (int k = lane; 4 * k < total; k += 32) dst[k] = src[k];
     }
     if (lane == 0) s.tile_bytes[h * ntiles + tile] = total;
+    sum += total;
+  }
+  if (s.cta_bytes) {
+    __shared__ int warp_sum[ENC_WARPS];
+    if (lane == 0) warp_sum[warp] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int all = 0;
+#pragma unroll
+      for (int w = 0; w < ENC_WARPS; w++) all += warp_sum[w];
+      s.cta_bytes[h * gridDim.x + blockIdx.x] = all;
+    }
   }
 }
 // KIND 0 / 1: K or V alone, grid = (ceil(ntiles / (4 * per_warp)), H).  2: both, grid z = kind (a prompt's K and V: one launch, and short prompts leave
@@ -187,14 +201,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) head_prefix_kernel(const int* __
 
 // What one kind's compaction reads and writes.
 struct CompactSide { const uint8_t* slots; const int *tile_bytes, *tile_off, *head_start; uint8_t* ovf; const int* flags; int* ovf_off; int* status; };
-struct FinishParams {              // the end of a prompt's prefill, see prefill_finish
-  const uint16_t *k_tok, *v_tok; long row_stride, L; int n_kv; long h0; uint16_t *ktail, *vtail; int *seq_len, *tail_len, *used_k, *used_v, *status;
-};
-struct CompactParams {
-  CompactSide side[2]; int ntiles; unsigned n_items; long tile_off_stride, head_stride, S, S_pad; int zero_pad; long ovf_cap, head_cap;
-  int finish; FinishParams fin;
-};
-__device__ void prefill_finish(const FinishParams& p, int h, int kind);
+struct CompactParams { CompactSide side[2]; int ntiles; unsigned n_items; long tile_off_stride, head_stride, S, S_pad; int zero_pad; long ovf_cap, head_cap; };
 
 // Escape bytes of every tile: slot -> ovf[head_start[h] + tile_off[h, tile]]; optionally the per-row escape offsets
 // ovf_off[h, row] = tile_off[h, tile] + (escape bytes of the tile's earlier rows), recomputed from the tag words.
@@ -202,8 +209,6 @@ __device__ void prefill_finish(const FinishParams& p, int h, int kind);
 // bytes), so a warp keeps four tiles in flight.  grid y = kind.
 __global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant__ CompactParams p) {
   griddep_wait();
-  const unsigned copies = (p.n_items + 15) / 16;
-  if (blockIdx.x >= copies) { prefill_finish(p.fin, blockIdx.x - copies, blockIdx.y); return; }       // the rest of a prompt's prefill
   const CompactSide& s = p.side[blockIdx.y];
   const int lane = threadIdx.x & 31, q = lane & 7;
   const unsigned first = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 4, item = first + (lane >> 3);
@@ -237,7 +242,7 @@ __global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant
     if (live && row + 1 < p.S) o[1] = toff + inc - s1;
   }
 }
-static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_items + 15) / 16 + (p.finish ? p.fin.n_kv : 0), (unsigned)kinds); }
+static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_items + 15) / 16, (unsigned)kinds); }
 
 // One warp per (head, tile): compressed tile -> bf16 rows.  Bound by latency and the warps that hide it: the escape bytes are asked for with the tile, their number taken from
 // the offset of the next tile (not of a head's last one), and the registers leave room for 8 CTAs of K, 7 of V.  [8, 65536, 128] K and V: 98.5 -> 93.7 us; with 6
@@ -300,38 +305,41 @@ template <class Cnt> __device__ __forceinline__ void add_four(Cnt* hist, int w, 
 #pragma unroll
   for (int i = 0; i < 4; i++) { const u32 n = (four >> (8 * i)) & 0xFFu; if (n) atomicAdd(&hist[4 * w + i], (Cnt)n); }
 }
-// WAITS: the counters are cleared by the kernel in front, which this one does not wait for before it adds to them; x was there before that kernel.
-template <class Cnt, bool PAIRS, bool WAITS>
+// A thread's rows of the CTA's chunk: x is at its channels' first value, col, sub its place in the CTA.
+template <bool PAIRS> __device__ __forceinline__ void count_rows(u32 (&bins)[64][128], const uint16_t* x, long N, long row_stride, int col, int sub) {
+  constexpr int LANES = HIST_THREADS / (PAIRS ? 64 : 128);
+  const auto load = [&](long r) -> u32 { return PAIRS ? *reinterpret_cast<const u32*>(x + r * row_stride) : x[r * row_stride]; };
+  const auto count = [&](u32 v) {                     // exponent = bits 7..14
+    atomicAdd(&bins[(v >> 9) & 0x3Fu][col], 1u << (8u * ((v >> 7) & 3u)));
+    if (PAIRS) atomicAdd(&bins[(v >> 25) & 0x3Fu][64 + col], 1u << (8u * ((v >> 23) & 3u)));
+  };
+  const long r1 = min(N, ((long)blockIdx.y + 1) * HIST_ROWS);
+  long r = (long)blockIdx.y * HIST_ROWS + sub;
+  for (; r + 15 * LANES < r1; r += 16 * LANES) {      // sixteen independent loads in flight per thread
+    u32 v[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = load(r + i * LANES);
+#pragma unroll
+    for (int i = 0; i < 16; i++) count(v[i]);
+  }
+  for (; r < r1; r += LANES) count(load(r));
+}
+// Behind clear_kernel x was there before that kernel, so the counting need not wait for it, only the flush (EARLY).
+template <class Cnt, bool PAIRS, bool EARLY>
 __global__ void __launch_bounds__(HIST_THREADS) exponent_hist_kernel(const __grid_constant__ HistParams<Cnt> p) {
   __shared__ __align__(16) u32 bins[64][128];
-  constexpr int WIDE = PAIRS ? 2 : 1, COLS = 128 / WIDE, LANES = HIST_THREADS / COLS;      // channels and threads side by side, threads per channel
+  constexpr int WIDE = PAIRS ? 2 : 1, COLS = 128 / WIDE;                                   // channels of a thread, threads side by side
   const int col = threadIdx.x % COLS, sub = threadIdx.x / COLS;
   const long c = (long)blockIdx.x * 128 + WIDE * col;
   for (int i = threadIdx.x; i < 64 * 128 / 4; i += HIST_THREADS) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
+  if (!EARLY) griddep_wait();
   griddep_launch();
   __syncthreads();
-  if (c < p.n_ch) {
-    const uint16_t* x = p.x[blockIdx.z] + c;
-    const auto load = [&](long r) -> u32 { return PAIRS ? *reinterpret_cast<const u32*>(x + r * p.row_stride) : x[r * p.row_stride]; };
-    const auto count = [&](u32 v) {                   // exponent = bits 7..14
-      atomicAdd(&bins[(v >> 9) & 0x3Fu][col], 1u << (8u * ((v >> 7) & 3u)));
-      if (PAIRS) atomicAdd(&bins[(v >> 25) & 0x3Fu][64 + col], 1u << (8u * ((v >> 23) & 3u)));
-    };
-    const long r1 = min(p.N, ((long)blockIdx.y + 1) * HIST_ROWS);
-    long r = (long)blockIdx.y * HIST_ROWS + sub;
-    for (; r + 15 * LANES < r1; r += 16 * LANES) {    // sixteen independent loads in flight per thread
-      u32 v[16];
-#pragma unroll
-      for (int i = 0; i < 16; i++) v[i] = load(r + i * LANES);
-#pragma unroll
-      for (int i = 0; i < 16; i++) count(v[i]);
-    }
-    for (; r < r1; r += LANES) count(load(r));
-  }
+  if (c < p.n_ch) count_rows<PAIRS>(bins, p.x[blockIdx.z] + c, p.N, p.row_stride, col, sub);
   __syncthreads();
   const int place = threadIdx.x & 127;
   const long ch = (long)blockIdx.x * 128 + (PAIRS ? 2 * (place & 63) + (place >> 6) : place);
-  if (WAITS) griddep_wait();
+  if (EARLY) griddep_wait();
   if (ch >= p.n_ch) return;
   Cnt* hist = p.hist[blockIdx.z] + ch * PER_CHANNEL<Cnt>;
 #pragma unroll 8
@@ -347,13 +355,14 @@ __global__ void __launch_bounds__(256) clear_kernel(u32* p, int n) {
 }
 
 // One warp per histogram row: densest 8- and 16-wide window, first maximum wins.  grid y = kind.  A lane has eight neighbouring bins, so one scan over the lanes makes the prefix.
-template <class Cnt> struct BasesParams { const Cnt* hist[2]; uint8_t *base3[2], *base4[2]; long n_rows; };
+template <class Cnt> struct BasesParams { const Cnt* hist[2]; uint8_t *base3[2], *base4[2]; long n_rows; bool clear; };       // clear: the counters are left zero
 template <class Cnt> struct Counts {
   typedef Cnt Sum;
   static __device__ __forceinline__ void load(const Cnt* row, int lane, Cnt (&v)[8]) {
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = row[8 * lane + i];
   }
+  static __device__ __forceinline__ void clear(Cnt*, int) {}
 };
 template <> struct Counts<Packed> {
   typedef int Sum;
@@ -363,6 +372,7 @@ template <> struct Counts<Packed> {
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = (int)((w[i >> 1] >> (16 * (i & 1))) & 0xFFFFu);
   }
+  static __device__ __forceinline__ void clear(Packed* row, int lane) { reinterpret_cast<uint4*>(row)[lane] = make_uint4(0u, 0u, 0u, 0u); }
 };
 template <class Cnt>
 __global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_constant__ BasesParams<Cnt> p) {
@@ -375,6 +385,7 @@ __global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_const
   if (row >= p.n_rows) return;
   Sum v[8], own = 0;
   Counts<Cnt>::load(p.hist[blockIdx.y] + row * PER_CHANNEL<Cnt>, lane, v);
+  if (p.clear) Counts<Cnt>::clear(const_cast<Cnt*>(p.hist[blockIdx.y]) + row * PER_CHANNEL<Cnt>, lane);
 #pragma unroll
   for (int i = 0; i < 8; i++) own += v[i];
   Sum inc = own;
@@ -402,34 +413,109 @@ __global__ void __launch_bounds__(128) bases_from_hist_kernel(const __grid_const
   }
 }
 
-// Last step of a slot's prefill, one CTA of 128 threads per (head, kind): the prompt's remainder (L mod 16 rows) goes into the head's raw tail
-// (two 16-byte pieces per thread: one CTA for all of them took 16 us for 15 rows of 8 heads), the head's token counters are set, and the largest
-// escape stream of the slot per kind is reported for the host's capacity check.  k_tok / v_tok: token-major rows, head h of token t at
-// t * row_stride + h * 128 (bf16 elements).
-__device__ void prefill_finish(const FinishParams& p, int h, int kind) {
-  const long n_full = p.L / T * T, head = p.h0 + h;
-  const int rem = (int)(p.L - n_full), tid = threadIdx.x;
-  const uint16_t* src = (kind ? p.v_tok : p.k_tok) + n_full * p.row_stride + h * D;
-  uint16_t* dst = (kind ? p.vtail : p.ktail) + head * T * D;
+// ---- end of a slot's prefill: offsets, escape bytes, tails and counters in ONE launch behind the encode.
+struct FinishSide { const uint8_t* slots; const int *tile_bytes, *cta_bytes; int* tile_off; uint8_t* ovf; int *used, *status; const uint16_t* tok; uint16_t* tail; };       // (used, ovf, ..: of the slot's heads)
+struct FinishParams { FinishSide side[2]; long L, row_stride, tile_off_stride, ovf_cap, head_cap; int n_kv, ntiles, per_cta, ctas, chunk, chunks; int *seq_len, *tail_len; };
+constexpr int FINISH_THREADS = 128, FINISH_TILES = FINISH_THREADS / 8, FINISH_STAGE = 128 * FINISH_TILES;
+
+// The prompt's remainder (L mod 16 rows) goes into the head's raw tail, the head's counters are set; the block of head 0 also has the heads' escape bytes from the encoder's
+// sums and reports the largest for the host's capacity check.
+__device__ __forceinline__ void finish_head(const FinishParams& p, const FinishSide& s, int h, int kind) {
+  const long n_full = p.L / T * T;
+  const int rem = (int)(p.L - n_full), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint16_t* src = s.tok + n_full * p.row_stride + h * D;
+  uint16_t* dst = s.tail + (long)h * T * D;
 #pragma unroll
-  for (int i = tid; i < T * 16; i += 128)
+  for (int i = tid; i < T * 16; i += FINISH_THREADS)
     if ((i >> 4) < rem) *reinterpret_cast<uint4*>(dst + i * 8) = *reinterpret_cast<const uint4*>(src + (i >> 4) * p.row_stride + (i & 15) * 8);
-  int* used = kind ? p.used_v : p.used_k;
-  if (tid == 0) {
-    if (kind == 0) { p.seq_len[head] = (int)n_full; p.tail_len[head] = rem; }
-    if (n_full == 0) used[head] = 0;
+  if (tid == 0 && kind == 0) { p.seq_len[h] = (int)n_full; p.tail_len[h] = rem; }
+  if (h) return;
+  __shared__ int most[FINISH_THREADS / 32];
+  int m = 0;
+  for (int k = warp; k < p.n_kv; k += FINISH_THREADS / 32) {
+    int n = 0;
+    for (int i = lane; i < p.ctas; i += 32) n += s.cta_bytes[(long)k * p.ctas + i];
+    n = __reduce_add_sync(FULL, n);
+    if (lane == 0) s.used[k] = n;
+    m = max(m, n);
   }
-  if (h == 0 && tid < 32) {
-    int m = 0;
-    if (n_full) for (int i = tid; i < p.n_kv; i += 32) m = max(m, used[p.h0 + i]);
-    m = __reduce_max_sync(FULL, m);
-    if (tid == 0) {
-      p.status[2 * kind + 1] = m;
-      if (n_full == 0) p.status[2 * kind] = 0;       // no copy in front of this step
-    }
+  if (lane == 0) most[warp] = m;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < FINISH_THREADS / 32; w++) m = max(m, most[w]);
+    s.status[1] = m;
+    if (p.ntiles == 0) s.status[0] = 0;              // (no encode in front that cleared it)
   }
 }
-__global__ void __launch_bounds__(128) prefill_finish_kernel(const __grid_constant__ FinishParams p) { prefill_finish(p, blockIdx.x, blockIdx.y); }
+// A block has `chunk` tiles of a head (up to 16, whole CTAs of the encoder), eight lanes per tile.  Where they begin in the head's stream is the sum of what the encoder's CTAs before them have, where
+// a tile begins follows from a scan over the block, and the bytes go through shared memory so that they leave in 16-byte stores.  Bound by latency, so everything that is
+// read is asked for at once, the first 64 bytes of a tile's slot (55 is usual) before their number is known, and blocks are small: 4001 tokens of 8 heads
+// with 64 tiles each 3.7 us, now 3.4;  the whole prompt with every group raw 39, now 28.  A prompt of 8 heads with its tables in four launches (encode, this, histogram, windows) against six (a clear, and
+// offsets and copy apart): 500 tokens 19.8 -> 12.7 us, 4001 30.9 -> 22.4, 32768 113 -> 87;  every group raw 25 -> 14, 31 -> 28, 90 -> 90 (without tables).
+__global__ void __launch_bounds__(FINISH_THREADS) prefill_finish_kernel(const __grid_constant__ FinishParams p) {
+  __shared__ __align__(16) uint8_t stage[FINISH_STAGE + 16];
+  __shared__ int warp_tiles[FINISH_THREADS / 32], warp_before[FINISH_THREADS / 32];
+  const FinishSide& s = p.side[blockIdx.y];
+  griddep_wait();
+  griddep_launch();
+  const int copies = p.n_kv * p.chunks;
+  if ((int)blockIdx.x >= copies) { finish_head(p, s, blockIdx.x - copies, blockIdx.y); return; }
+  const int h = blockIdx.x / p.chunks, tile0 = (blockIdx.x % p.chunks) * p.chunk, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = tid >> 3, q = tid & 7;
+  const bool live = t < min(p.chunk, p.ntiles - tile0);
+  const long item = (long)h * p.ntiles + tile0 + t;
+  const uint8_t* slot = s.slots + item * TILE_MAX_ESC;
+  const int n = live ? s.tile_bytes[item] : 0;
+  u32 first[2] = {0u, 0u};
+  if (live) { first[0] = reinterpret_cast<const u32*>(slot)[2 * q]; first[1] = reinterpret_cast<const u32*>(slot)[2 * q + 1]; }
+  int part = 0;
+  for (int i = tid; i < tile0 / p.per_cta; i += FINISH_THREADS) part += s.cta_bytes[(long)h * p.ctas + i];
+  int inc = n;                                       // of the warp's tiles up to this one
+#pragma unroll
+  for (int d = 8; d < 32; d <<= 1) { const int v = __shfl_up_sync(FULL, inc, d); if (lane >= d) inc += v; }
+  part = __reduce_add_sync(FULL, part);
+  if (lane == 31) { warp_tiles[warp] = inc; warp_before[warp] = part; }
+  __syncthreads();
+  int begin = 0, local = inc - n, total = 0;         // of the block inside the head, of the tile inside the block
+#pragma unroll
+  for (int w = 0; w < FINISH_THREADS / 32; w++) { begin += warp_before[w]; if (w < warp) local += warp_tiles[w]; total += warp_tiles[w]; }
+  if (live && q == 0) s.tile_off[h * p.tile_off_stride + tile0 + t] = begin + local;
+  uint8_t* const dst = s.ovf + (long)h * p.ovf_cap + begin;
+  if (total > FINISH_STAGE || (long)begin + total > p.head_cap) {           // more than the stage holds, or some tiles do not fit the head's share: these are not written
+    const bool fits = (long)begin + local + n <= p.head_cap;
+    if (!fits && live && q == 0) atomicOr(s.status, 1);
+    for (int k = 0; k < 4; k++) {                    // the warp's tiles one by one: words of the destination out of two of the slot
+      const int size = __shfl_sync(FULL, fits ? n : 0, 8 * k);
+      uint8_t* const d = dst + __shfl_sync(FULL, local, 8 * k);
+      const uint8_t* const b = s.slots + (item - t + 4 * warp + k) * TILE_MAX_ESC;
+      const int odd = min(size, (int)(-reinterpret_cast<uintptr_t>(d) & 3)), words = (size - odd) >> 2, rest = odd + 4 * words;
+      const u32* const from = reinterpret_cast<const u32*>(b);
+      for (int i = lane; i < words; i += 32 * 5) {     // (five loads that do not wait for the stores)
+        u32 v[5];
+#pragma unroll
+        for (int j = 0; j < 5; j++)
+          if (i + 32 * j < words) v[j] = odd ? __funnelshift_r(from[i + 32 * j], from[i + 32 * j + 1], 8 * odd) : from[i + 32 * j];
+#pragma unroll
+        for (int j = 0; j < 5; j++)
+          if (i + 32 * j < words) reinterpret_cast<u32*>(d + odd)[i + 32 * j] = v[j];
+      }
+      if (lane < odd) d[lane] = b[lane];
+      if (rest + lane < size) d[rest + lane] = b[rest + lane];
+    }
+    return;
+  }
+  const int phase = (int)(reinterpret_cast<uintptr_t>(dst) & 15);
+  uint8_t* const to = stage + phase + local;
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+    if (8 * q + i < n) to[8 * q + i] = (uint8_t)(first[i >> 2] >> (8 * (i & 3)));
+  for (int i = 64 + q; i < n; i += 8) to[i] = slot[i];
+  __syncthreads();
+  for (int k = tid; 16 * k < phase + total; k += FINISH_THREADS) {
+    uint8_t* const line = dst - phase + 16 * k;
+    if (16 * k >= phase && 16 * k + 16 <= phase + total) *reinterpret_cast<uint4*>(line) = reinterpret_cast<const uint4*>(stage)[k];
+    else for (int i = max(0, phase - 16 * k); i < min(16, phase + total - 16 * k); i++) line[i] = stage[16 * k + i];
+  }
+}
 
 }  // namespace gaac
 
@@ -442,7 +528,7 @@ static int encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, 
   if (H <= 0 || S <= 0 || S_in < S || S_pad < (S + T - 1) / T * T || S_pad % T || n_kv <= 0 || H > 65535 || (kind != GAAC_KIND_K && kind != GAAC_KIND_V)) return GAAC_E_ARG;
   if (!aligned16(x_bf16) || !aligned16(sm) || !aligned16(codes)) return GAAC_E_ALIGN;
   const int ntiles = (int)((S + T - 1) / T);
-  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles, tiles_per_warp(ntiles, H, ENC_RESIDENT, ENC_MOST)};
+  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear, nullptr}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles, tiles_per_warp(ntiles, H, ENC_RESIDENT, ENC_MOST)};
   return launch_overlapped(kind == GAAC_KIND_K ? encode_tiles_kernel<0> : encode_tiles_kernel<1>, encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, (cudaStream_t)stream, p);
 }
 
@@ -539,7 +625,7 @@ extern "C" int gaac_exponent_hist(const void* x_bf16, int64_t N, int64_t n_ch, l
 
 extern "C" int gaac_bases_from_hist(const long long* hist, int64_t n_rows, uint8_t* base3, uint8_t* base4, void* stream) {
   if (!hist || !base3 || !base4 || n_rows <= 0) return GAAC_E_ARG;
-  const BasesParams<long long> p{{hist, nullptr}, {base3, nullptr}, {base4, nullptr}, n_rows};
+  const BasesParams<long long> p{{hist, nullptr}, {base3, nullptr}, {base4, nullptr}, n_rows, false};
   return launch_overlapped(bases_from_hist_kernel<long long>, dim3((unsigned)((n_rows + 3) / 4)), 128, (cudaStream_t)stream, p);
 }
 
@@ -548,17 +634,19 @@ constexpr int CACHE_READ_PAD = 8;      // bytes kept free behind a head's escape
 
 extern "C" size_t gaac_cache_calibrate_scratch_bytes(int n_kv) { return 2 * (size_t)(n_kv > 0 ? n_kv : 0) * D * 256 * sizeof(int32_t); }
 
-// Three launches: counters cleared, histograms of both kinds, windows into the slot's rows of the tables.
+// Histograms of both kinds, windows into the slot's rows of the tables.  zeroed: the counters are zero, and are left so; else they are cleared first, which takes a launch more.
 template <class Cnt>
-static int calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, long n_ch, long at, uint8_t* scratch, bool pairs, cudaStream_t st) {
-  Cnt* hist = reinterpret_cast<Cnt*>(scratch);
+static int calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, long n_ch, long at, uint8_t* counters, bool zeroed, cudaStream_t st) {
+  Cnt* hist = reinterpret_cast<Cnt*>(counters);
   const long one = n_ch * PER_CHANNEL<Cnt>;
   const int n = (int)(2 * one * sizeof(Cnt) / 4);
-  clear_kernel<<<std::min(n / 256, 8 * 148), 256, 0, st>>>(reinterpret_cast<u32*>(scratch), n);
+  if (!zeroed) clear_kernel<<<std::min(n / 256, 8 * 148), 256, 0, st>>>(reinterpret_cast<u32*>(counters), n);
   const HistParams<Cnt> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + one}, L, n_ch, row_stride};
-  if (int e = launch_overlapped(pairs ? exponent_hist_kernel<Cnt, true, true> : exponent_hist_kernel<Cnt, false, true>, hist_grid(n_ch, L, 2), HIST_THREADS, st, hp)) return e;
+  const bool pairs = hist_pairs(k_tok, n_ch, row_stride) && hist_pairs(v_tok, n_ch, row_stride);
+  const auto kernel = zeroed ? (pairs ? exponent_hist_kernel<Cnt, true, false> : exponent_hist_kernel<Cnt, false, false>) : (pairs ? exponent_hist_kernel<Cnt, true, true> : exponent_hist_kernel<Cnt, false, true>);
+  if (int e = launch_overlapped(kernel, hist_grid(n_ch, L, 2), HIST_THREADS, st, hp)) return e;
   const BasesParams<Cnt> bp{{hist, hist + one}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
-                            {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch};
+                            {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch, zeroed};
   return launch_overlapped(bases_from_hist_kernel<Cnt>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
 }
 
@@ -570,9 +658,27 @@ extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, co
   if (reinterpret_cast<uintptr_t>(scratch) & 3) return GAAC_E_ALIGN;
   cudaStream_t st = (cudaStream_t)stream;
   const long n_ch = (long)n_kv * D, at = (long)slot * n_ch;
-  const bool pairs = hist_pairs(k_tok, n_ch, row_stride) && hist_pairs(v_tok, n_ch, row_stride);
-  return L <= 0xFFFF && !(reinterpret_cast<uintptr_t>(scratch) & 15) ? calibrate<Packed>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, pairs, st)
-                                                                      : calibrate<int>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, pairs, st);
+  return L <= 0xFFFF && aligned16(scratch) ? calibrate<Packed>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, false, st)
+                                           : calibrate<int>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, false, st);
+}
+
+extern "C" size_t gaac_cache_tables_workspace_bytes(int n_kv) { return n_kv > 0 ? 2 * (size_t)n_kv * D * 64 * sizeof(Packed) : 0; }
+
+extern "C" int gaac_cache_prefill_own(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
+                                      int32_t* tail_len, int32_t* seq_len, int64_t S_cap, int64_t ovf_cap, int n_base_rows, uint8_t* scratch, size_t scratch_bytes,
+                                      int32_t* status, uint8_t* workspace, size_t workspace_bytes, void* stream) {
+  if (!K || !V || !K->base3 || !K->base4 || !V->base3 || !V->base4 || !k_tok || !v_tok || !scratch || !workspace) return GAAC_E_ARG;
+  if (L <= 0 || L > S_cap || row_stride < (int64_t)n_kv * D || slot < 0 || n_kv <= 0 || n_kv > 256 || n_base_rows < (slot + 1) * n_kv) return GAAC_E_ARG;
+  if (scratch_bytes < gaac_cache_prefill_scratch_bytes(L, n_kv)) return GAAC_E_ARG;
+  if (workspace_bytes < gaac_cache_tables_workspace_bytes(n_kv)) return GAAC_E_WORKSPACE;
+  if (!aligned16(workspace)) return GAAC_E_ALIGN;
+  if (L > 0xFFFF) {                                  // counts of 32 bits, in the scratch of the encode that follows (which has 2568 bytes for every 16 tokens of a head)
+    if (int e = gaac_cache_calibrate(K, V, k_tok, v_tok, L, row_stride, slot, n_kv, n_base_rows, scratch, scratch_bytes, stream)) return e;
+  } else {
+    const long n_ch = (long)n_kv * D;
+    if (int e = calibrate<Packed>(K, V, k_tok, v_tok, L, row_stride, n_ch, (long)slot * n_ch, workspace, true, (cudaStream_t)stream)) return e;
+  }
+  return gaac_cache_prefill(K, V, k_tok, v_tok, L, row_stride, slot, n_kv, tail_len, seq_len, S_cap, ovf_cap, n_base_rows, scratch, scratch_bytes, status, 0, stream);
 }
 
 static int clear_status(int32_t* status, cudaStream_t st) {           // the words that say whether an escape stream had room
@@ -583,7 +689,8 @@ static int clear_status(int32_t* status, cudaStream_t st) {           // the wor
 
 extern "C" size_t gaac_cache_prefill_scratch_bytes(int64_t L, int n_kv) {
   const size_t items = (size_t)(L > 0 ? L / T : 0) * (size_t)(n_kv > 0 ? n_kv : 0);
-  return 2 * items * (TILE_MAX_ESC + sizeof(int32_t)) + 256;
+  const size_t ctas = ((size_t)(L > 0 ? L / T : 0) + ENC_WARPS - 1) / ENC_WARPS * (size_t)(n_kv > 0 ? n_kv : 0);       // of the encoder, at most
+  return 2 * items * (TILE_MAX_ESC + sizeof(int32_t)) + 2 * ctas * sizeof(int32_t) + 256;
 }
 
 extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot,
@@ -604,35 +711,34 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
   const int ntiles = (int)(L / T);
   const long S = (long)ntiles * T, tiles_cap = S_cap / T, n_items = (long)n_kv * ntiles;
   if (n_items > 0x7FFFFFF0L) return GAAC_E_ARG;
-  const FinishParams fin{(const uint16_t*)k_tok, (const uint16_t*)v_tok, row_stride, L, n_kv, h0, (uint16_t*)K->tail, (uint16_t*)V->tail, seq_len, tail_len, K->ovf_used, V->ovf_used, status};
-  if (ntiles == 0) {
-    if (copy_only) { if (int e = clear_status(status, st)) return e; }
-    else prefill_finish_kernel<<<dim3((unsigned)n_kv, 2), 128, 0, st>>>(fin);
-    return launch_status();
-  }
-  // Three launches for both kinds: encode, offsets, copy (whose last block does the tails and counters); the encode clears the words that the
-  // copy reports into.  scratch: escape slots of K, of V, then the tile sizes of K, of V
+  // Two launches for both kinds: encode, then offsets, copy, tails and counters; the encode clears the words that the
+  // copy reports into.  scratch: escape slots of K, of V, then the tile sizes of K, of V, then those of the encoder's CTAs
   const gaac_store* side[2] = {K, V};
   const void* tok[2] = {k_tok, v_tok};
-  EncodeParams ep{}; ScanParams sp{}; CompactParams cp{};
+  EncodeParams ep{}; FinishParams fp{}; CompactParams cp{};
+  ep.per_warp = tiles_per_warp(ntiles, 2 * n_kv, ENC_RESIDENT, ENC_MOST);
+  const dim3 grid = encode_grid(ntiles, n_kv, 2, ep.per_warp);
+  int32_t* const sizes = reinterpret_cast<int32_t*>(scratch + 2 * n_items * TILE_MAX_ESC);
   for (int kind = 0; kind < 2; kind++) {
     const gaac_store* s = side[kind];
     uint8_t* slots = scratch + kind * n_items * TILE_MAX_ESC;
-    int32_t* tbytes = reinterpret_cast<int32_t*>(scratch + 2 * n_items * TILE_MAX_ESC) + kind * n_items;
-    int32_t* toff = s->tile_off + h0 * tiles_cap;
+    int32_t *tbytes = sizes + kind * n_items, *cbytes = sizes + 2 * n_items + (int64_t)kind * n_kv * grid.x, *toff = s->tile_off + h0 * tiles_cap;
     ep.side[kind] = EncodeSide{(const uint16_t*)tok[kind], s->base3 + (h0 % n_base_rows) * D, s->base4 + (h0 % n_base_rows) * D,          // consecutive heads, consecutive rows
-                               s->sm + h0 * S_cap * D, s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots, tbytes, status + 2 * kind};
-    sp.side[kind] = ScanSide{tbytes, toff, s->ovf_used + h0};
+                               s->sm + h0 * S_cap * D, s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots, tbytes, status + 2 * kind, cbytes};
+    fp.side[kind] = FinishSide{slots, tbytes, cbytes, toff, s->ovf + h0 * ovf_cap, s->ovf_used + h0, status + 2 * kind, (const uint16_t*)tok[kind], (uint16_t*)s->tail + h0 * T * D};
     cp.side[kind] = CompactSide{slots, tbytes, toff, nullptr, s->ovf + h0 * ovf_cap, nullptr, nullptr, status + 2 * kind};
   }
-  ep.S = S; ep.x_head_stride = D; ep.x_row_stride = row_stride; ep.S_pad = S_cap; ep.n_kv = n_kv; ep.ntiles = ntiles; ep.per_warp = tiles_per_warp(ntiles, 2 * n_kv, ENC_RESIDENT, ENC_MOST);
-  sp.ntiles = ntiles; sp.tile_off_stride = tiles_cap;
-  cp.ntiles = ntiles; cp.n_items = (unsigned)n_items; cp.tile_off_stride = tiles_cap; cp.head_stride = ovf_cap; cp.head_cap = ovf_cap - CACHE_READ_PAD;
-  cp.finish = !copy_only; cp.fin = fin;
-  if (copy_only) { if (int e = clear_status(status, st)) return e; }
-  else {
-    if (int e = launch_overlapped(encode_tiles_kernel<2>, encode_grid(ntiles, n_kv, 2, ep.per_warp), ENC_WARPS * 32, st, ep)) return e;
-    if (int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)n_kv, 2), SCAN_THREADS, st, sp)) return e;
+  if (copy_only) {
+    cp.ntiles = ntiles; cp.n_items = (unsigned)n_items; cp.tile_off_stride = tiles_cap; cp.head_stride = ovf_cap; cp.head_cap = ovf_cap - CACHE_READ_PAD;
+    if (int e = clear_status(status, st)) return e;
+    return ntiles ? launch_overlapped(compact_copy_kernel, compact_grid(cp, 2), 128, st, cp) : launch_status();
   }
-  return launch_overlapped(compact_copy_kernel, compact_grid(cp, 2), 128, st, cp);
+  fp.L = L; fp.row_stride = row_stride; fp.tile_off_stride = tiles_cap; fp.ovf_cap = ovf_cap; fp.head_cap = ovf_cap - CACHE_READ_PAD; fp.n_kv = n_kv; fp.ntiles = ntiles;
+  fp.per_cta = ENC_WARPS * ep.per_warp; fp.ctas = (int)grid.x; fp.chunk = FINISH_TILES / fp.per_cta * fp.per_cta; fp.chunks = (ntiles + fp.chunk - 1) / fp.chunk;
+  fp.seq_len = seq_len + h0; fp.tail_len = tail_len + h0;
+  if (ntiles) {
+    ep.S = S; ep.x_head_stride = D; ep.x_row_stride = row_stride; ep.S_pad = S_cap; ep.n_kv = n_kv; ep.ntiles = ntiles;
+    if (int e = launch_overlapped(encode_tiles_kernel<2>, grid, ENC_WARPS * 32, st, ep)) return e;
+  }
+  return launch_overlapped(prefill_finish_kernel, dim3((unsigned)(n_kv * fp.chunks + n_kv), 2), FINISH_THREADS, st, fp);
 }

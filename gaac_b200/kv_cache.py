@@ -61,6 +61,18 @@ class _Store:
                           self.tail.data_ptr(), self.base3.data_ptr(), self.base4.data_ptr())
 
 
+_TABLES = {}     # (device index, stream) -> counters of a prompt's tables, 128 KB per kv head: zeroed once, left zero by every call, shared by all caches
+
+
+def _tables_workspace(lib, dev, stream: int, n_kv: int) -> torch.Tensor:
+    """The counters of the current stream.  Nothing but calls on that stream uses them, so one that became too small can go."""
+    need, key = lib.gaac_cache_tables_workspace_bytes(n_kv), (dev.index, stream)
+    ws = _TABLES.get(key)
+    if ws is None or ws.numel() < need:
+        ws = _TABLES[key] = torch.zeros(need, dtype=torch.uint8, device=dev)
+    return ws
+
+
 class CompressedKVCache:
     def __init__(self, n_slots: int, n_kv: int, capacity: int, bases: dict | None = None,
                  ovf_bytes_per_tile: int = 128, device="cuda"):
@@ -125,47 +137,51 @@ class CompressedKVCache:
         k, v = self._token_rows(k), self._token_rows(v)
         if _lib.row_stride(k) != _lib.row_stride(v):                                               # the library reads both with one stride
             k, v = k.contiguous(), v.contiguous()
-        stores = self.k.c_store(), self.v.c_store()
-        if self.per_sequence_bases and L:
-            lib = _lib.lib()
-            hist = torch.empty(lib.gaac_cache_calibrate_scratch_bytes(self.n_kv), dtype=torch.uint8, device=k.device)
-            _lib.check(lib.gaac_cache_calibrate(*stores, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.k.base3.shape[0],
-                                                hist.data_ptr(), hist.numel(), _lib.stream_ptr(k.device)), "gaac_cache_calibrate")
         need = _lib.lib().gaac_cache_prefill_scratch_bytes(L, self.n_kv)
         if check:
             if self._pending:
-                self.settle_prefills()
-                stores = None                                                                      # the escape streams may have moved
+                self.settle_prefills()                                                             # (the escape streams may move)
             if self._scratch is None or self._scratch.numel() < need:
                 self._scratch = torch.empty(need, dtype=torch.uint8, device=k.device)
-            scratch, status = self._scratch, self._slot_status[slot]
+            scratch = self._scratch
         else:
             old = self._pending.pop(slot, None)
             if old is not None:
                 self._pending_bytes -= old[1].numel()
             if self._pending_bytes + need > self.pending_scratch_limit:
                 self.settle_prefills()
-                stores = None                                                                      # the escape streams may have moved
-            scratch, status = torch.empty(need, dtype=torch.uint8, device=k.device), self._slot_status[slot]
-        self._prefill_launch(slot, L, k, v, scratch, status, copy_only=0, stores=stores)
+            scratch = torch.empty(need, dtype=torch.uint8, device=k.device)
+        self._prefill_launch(slot, L, k, v, scratch, copy_only=0)
         if not check:
             self._pending[slot] = (L, scratch)
             self._pending_bytes += need
             return
-        short_k, used_k, short_v, used_v = status.tolist()                                         # the one host synchronisation
+        short_k, used_k, short_v, used_v = self._slot_status[slot].tolist()                             # the one host synchronisation
         # room for these tiles and for one more worst-case tile, which an append may add before the next check_capacity
         wanted = max(used_k, used_v) + TILE_MAX_ESC + _OVER_READ
         if wanted > self.k.ovf_cap:
             self._grow(wanted)
         if short_k or short_v:
-            self._prefill_launch(slot, L, None, None, scratch, status, copy_only=1)
+            self._prefill_launch(slot, L, None, None, scratch, copy_only=1)
 
-    def _prefill_launch(self, slot, L, k, v, scratch, status, copy_only: int, stores=None):
-        dev = self.S.device
-        K, V = stores or (self.k.c_store(), self.v.c_store())
-        _lib.check(_lib.lib().gaac_cache_prefill(K, V, _lib.ptr(k), _lib.ptr(v), L, _lib.row_stride(k) if k is not None else self.n_kv * D,
-                                                 slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(), self.cap, self.k.ovf_cap, self.k.base3.shape[0],
-                                                 scratch.data_ptr(), scratch.numel(), status.data_ptr(), copy_only, _lib.stream_ptr(dev)), "gaac_cache_prefill")
+    def _prefill_launch(self, slot, L, k, v, scratch, copy_only: int):
+        lib, dev = _lib.lib(), self.S.device
+        K, V, stream, status = self.k.c_store(), self.v.c_store(), _lib.stream_ptr(dev), self._slot_status.data_ptr() + 16 * slot
+        rows = self.k.base3.shape[0]
+        own = self.per_sequence_bases and L and not copy_only                                      # tables from the prompt itself
+        if own and not torch.cuda.is_current_stream_capturing():
+            ws = _tables_workspace(lib, dev, stream, self.n_kv)
+            _lib.check(lib.gaac_cache_prefill_own(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(),
+                                                  self.cap, self.k.ovf_cap, rows, scratch.data_ptr(), scratch.numel(), status, ws.data_ptr(), ws.numel(), stream),
+                       "gaac_cache_prefill_own")
+            return
+        if own:                                      # a workspace made or cleared while a graph is captured would be so only when the graph runs
+            hist = torch.empty(lib.gaac_cache_calibrate_scratch_bytes(self.n_kv), dtype=torch.uint8, device=dev)
+            _lib.check(lib.gaac_cache_calibrate(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, rows, hist.data_ptr(), hist.numel(), stream),
+                       "gaac_cache_calibrate")
+        _lib.check(lib.gaac_cache_prefill(K, V, _lib.ptr(k), _lib.ptr(v), L, _lib.row_stride(k) if k is not None else self.n_kv * D,
+                                          slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(), self.cap, self.k.ovf_cap, rows,
+                                          scratch.data_ptr(), scratch.numel(), status, copy_only, stream), "gaac_cache_prefill")
 
     def settle_prefills(self):
         """Host check of every prefill made with check=False: one read of their status words; the escape streams grow when one
@@ -194,7 +210,7 @@ class CompressedKVCache:
         for slot, w in zip(slots, words):
             if w[0] or w[2]:
                 L, scratch = pending[slot]
-                self._prefill_launch(slot, L, None, None, scratch, self._slot_status[slot], copy_only=1)
+                self._prefill_launch(slot, L, None, None, scratch, copy_only=1)
 
     @staticmethod
     def _token_rows(x: torch.Tensor) -> torch.Tensor:

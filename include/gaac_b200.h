@@ -281,7 +281,7 @@ int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, const void* k
  * at x + t*row_stride + h*128 (bf16 elements; row_stride >= n_kv*128, rows 16-byte aligned), L tokens (L <= S_cap).  The
  * floor(L/16) whole tiles of every head of the slot are compressed straight into the store (tile 0 upward, the head's escape
  * bytes from offset 0 of its share), the L mod 16 remaining rows go into the raw tails, seq_len / tail_len / ovf_used of the
- * slot's heads are set: three launches, no host synchronisation, no transposed copy of the input.
+ * slot's heads are set: two launches, no host synchronisation, no transposed copy of the input.
  * Replaces CompressedKVCache.prefill's device work (gaac/kv_cache.py:149-169: Triton encode per kind, torch prefix sums, the
  * scatter of the escape bytes, tail copy, counter updates).
  *   scratch: gaac_cache_prefill_scratch_bytes(L, n_kv) bytes of device memory, kept by the caller until a copy_only repeat is
@@ -297,6 +297,14 @@ size_t gaac_cache_prefill_scratch_bytes(int64_t L, int n_kv);
 int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot,
                        int n_kv, int32_t* tail_len, int32_t* seq_len, int64_t S_cap, int64_t ovf_cap, int n_base_rows, uint8_t* scratch,
                        size_t scratch_bytes, int32_t* status, int copy_only, void* stream);
+
+/* gaac_cache_calibrate and gaac_cache_prefill of a prompt (L > 0) in one call and, up to 65535 tokens, four launches in all: the same tables, bytes and
+ * status.  workspace: gaac_cache_tables_workspace_bytes(n_kv) bytes, 16-byte aligned, zero before its first use; every call leaves it zero, so one serves all calls on a
+ * stream, whatever their n_kv (it must be large enough for each).  Calls that may overlap on the GPU need one each. */
+size_t gaac_cache_tables_workspace_bytes(int n_kv);
+int gaac_cache_prefill_own(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
+                           int32_t* tail_len, int32_t* seq_len, int64_t S_cap, int64_t ovf_cap, int n_base_rows, uint8_t* scratch, size_t scratch_bytes,
+                           int32_t* status, uint8_t* workspace, size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------------------- paged layout (layout B) */
 

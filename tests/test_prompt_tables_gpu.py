@@ -60,3 +60,76 @@ def test_histogram_of_odd_channels(n_ch, offset):
     _lib.check(_lib.lib().gaac_exponent_hist(x.data_ptr(), 300, n_ch, hist.data_ptr(), torch.cuda.current_stream().cuda_stream), "gaac_exponent_hist")
     e = (x16.reshape(300, n_ch) >> 7) & 0xFF
     assert np.array_equal(hist.cpu().numpy(), np.stack([np.bincount(e[:, c], minlength=256) for c in range(n_ch)]))
+
+
+@pytest.mark.parametrize("L", [1, 15, 16, 128, 129, 700, 65535, 65536])
+def test_prefill_makes_the_same_tables(L):
+    """gaac_cache_prefill_own: the tables of the two-call form, its counters zero again behind every call, one set of counters for caches of different sizes."""
+    import torch
+    from gaac_b200 import CompressedKVCache, kv_cache
+    for n_kv in ((1,) if L > 1000 else (3, 1, 5)):
+        rows = [np.ascontiguousarray(O.kv_like(n_kv, L, seed=10 * n_kv + s).transpose(1, 0, 2)) for s in (1, 2)]
+        cache = CompressedKVCache(2, n_kv, L)
+        for _ in range(2):
+            cache.prefill(1, *(to_bf16_cuda(r) for r in rows))
+        _check([r.reshape(L, -1) for r in rows], [(s.base3[n_kv:].cpu().numpy(), s.base4[n_kv:].cpu().numpy()) for s in (cache.k, cache.v)], n_kv)
+        assert all(not bool(ws.any()) for ws in kv_cache._TABLES.values()) and len(kv_cache._TABLES) >= 1
+        k, v = cache.decompress(1)
+        for got, r in zip((k, v), rows):
+            assert np.array_equal(got.contiguous().view(torch.int16).cpu().numpy().view(np.uint16), r)
+
+
+def test_prefill_in_a_captured_graph():
+    import torch
+    from gaac_b200 import CompressedKVCache
+    n_kv, L = 2, 300
+    x = [to_bf16_cuda(np.ascontiguousarray(O.kv_like(n_kv, L, seed=s).transpose(1, 0, 2))) for s in (1, 2, 3, 4)]
+    cache, k, v = CompressedKVCache(1, n_kv, L), x[0].clone(), x[1].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        cache.prefill(0, k, v, check=False)
+    k.copy_(x[2]); v.copy_(x[3])
+    graph.replay()
+    assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(cache.decompress(0), (k, v)))
+    cache.prefill(0, x[0], x[1])
+    assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(cache.decompress(0), x))
+
+
+@pytest.mark.parametrize("tiles", [0, 1, 63, 65, 369, 370, 555, 740])         # from 370 on two, three, four tiles per warp of the encoder: blocks of 64, 64, 60 and 64 tiles behind it
+@pytest.mark.parametrize("room", [1280, 100])                                # 100: the streams are too small, the copy is repeated into larger ones
+def test_streams_behind_the_encode(tiles, room):
+    """A slot's offsets, escape bytes, counters and tails against a Page of the same tokens: blocks of ordinary tiles, of tiles with every group raw, and of both."""
+    import torch
+    from gaac_b200 import Codec, CompressedKVCache
+    n_kv, L = 8, 16 * tiles + 7
+    base = O.kv_like(n_kv, max(L, 16), seed=5)
+    if tiles > 64:
+        wild = np.random.default_rng(2).integers(0, 65536, base.shape).astype(np.uint16)
+        t = np.arange(base.shape[1]) // 16
+        base = np.where(((t % 9 == 4) | ((t >= 64) & (t < 72)) | (t == tiles - 1))[None, :, None], wild, base)
+    x = to_bf16_cuda(np.ascontiguousarray(base[:, :L].transpose(1, 0, 2)))
+    c = Codec(n_kv).calibrate(to_bf16_cuda(O.kv_like(n_kv, 512, seed=1)))
+    cache = CompressedKVCache(3, n_kv, L, bases={"k3": c.base3, "k4": c.base4, "v3": c.base3, "v4": c.base4}, ovf_bytes_per_tile=room)
+    small = cache.k.ovf_cap
+    for check in (True, False):
+        cache.prefill(1, x, x.flip(1).contiguous(), check=check)
+        cache.settle_prefills()
+    heads = slice(n_kv, 2 * n_kv)
+    for st, rows in ((cache.k, x), (cache.v, x.flip(1))):
+        assert torch.equal(st.tail[heads, :L % 16].view(torch.int16), rows[L // 16 * 16:].transpose(0, 1).contiguous().view(torch.int16))
+        if tiles == 0:
+            assert int(st.ovf_used[heads].max()) == 0
+            continue
+        page = c.encode(rows[:16 * tiles].transpose(0, 1).contiguous(), st.kind)
+        size = page.ovf_head_start[1:] - page.ovf_head_start[:-1]
+        assert torch.equal(st.ovf_used[heads], size) and torch.equal(st.tile_off[heads, :tiles], page.tile_off)
+        assert torch.equal(st.flags[heads, :16 * tiles], page.flags)
+        at = page.ovf_head_start.tolist()
+        for h in range(n_kv):
+            n = at[h + 1] - at[h]
+            o = (n_kv + h) * st.ovf_cap
+            assert torch.equal(st.ovf[o:o + n], page.ovf[at[h]:at[h] + n]), h
+            assert not bool(st.ovf[o + n:o + st.ovf_cap].any())                 # nothing behind a head's bytes
+        assert not bool(st.ovf_used[:n_kv].any()) and not bool(st.ovf_used[2 * n_kv:].any()) and not bool(st.ovf[:n_kv * st.ovf_cap].any())
+    assert room != 100 or cache.k.ovf_cap > small
+    assert cache.S[heads].tolist() == [16 * tiles] * n_kv and cache.tail_len[heads].tolist() == [L % 16] * n_kv
