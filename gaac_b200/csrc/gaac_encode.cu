@@ -1,5 +1,6 @@
 // Block encoder, escape-stream compaction, page decoder and calibration kernels (sm_100a).
 #include <algorithm>
+#include <atomic>
 #include "gaac_api.cuh"
 #include "gaac_warp.cuh"
 
@@ -563,6 +564,31 @@ extern "C" int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64
                                  uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
                                  int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, void* stream) {
   return encode_begin(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, tile_off, head_bytes, head_start, nullptr, stream);
+}
+
+extern "C" int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
+                                  const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
+                                  uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
+                                  int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream) {
+  if (!total_pinned) return GAAC_E_ARG;
+  *reinterpret_cast<volatile int32_t*>(total_pinned) = -1;
+  return encode_begin(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, tile_off, head_bytes, head_start, total_pinned, stream);
+}
+
+// The word is polled, since a wait for the stream would also wait for what was queued behind the kernel that writes it, and takes longer to return.  Now and then the stream is asked, which
+// ends the wait when the kernels have failed.
+extern "C" int gaac_wait_total(const int32_t* total_pinned, void* stream) {
+  if (!total_pinned) return GAAC_E_ARG;
+  const volatile int32_t* const word = total_pinned;
+  while (true) {
+    for (int i = 0; i < 4096; i++) {
+      if (*word >= 0) { std::atomic_thread_fence(std::memory_order_acquire); return GAAC_OK; }
+      __builtin_ia32_pause();
+    }
+    const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+    if (e == cudaErrorNotReady) { cudaGetLastError(); continue; }
+    return e == cudaSuccess && *word >= 0 ? GAAC_OK : GAAC_E_LAUNCH;
+  }
 }
 
 extern "C" int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,

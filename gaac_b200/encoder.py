@@ -12,6 +12,8 @@ from . import _lib
 from .codec import Codec, Page, D, T, CB, perm, storage_index, row_offsets
 
 SLOT = 1280
+ROOM = 80       # escape bytes per tile that encode makes room for before it knows their number, 3 % of a tile.  Tables calibrated on the data leave 50 to 60; the copy is repeated for more.
+                # us of K and V, a copy launched after a wait for the size -> one queued behind the kernels: [8, 1111, 128] 110 -> 91, [8, 65536, 128] 194 -> 175.
 
 
 class TileEncoder:
@@ -129,8 +131,8 @@ class TileEncoder:
 
     def encode(self, codec: Codec, x: torch.Tensor) -> Page:
         """x: [H, S, D] bf16 -> Page, bit-identical to the reference Codec.encode(x, kind).  (gaac/encoder.py:111-123)
-        The kernels hand the size of the escape stream to the host through page-locked memory; the stream is then allocated at its exact
-        size, as the reference's is, and one more kernel fills it."""
+        The kernels hand the size of the escape stream to the host through page-locked memory while the copy into a stream with room for ROOM bytes per tile is under
+        way; ovf is the part of it that the bytes take.  Where they take more, a stream of exactly that size is made and the copy repeated."""
         if not x.is_cuda:
             raise RuntimeError("TileEncoder needs CUDA tensors: gaac_b200 has no CPU path")
         H, S, _ = x.shape; dev = x.device
@@ -139,10 +141,9 @@ class TileEncoder:
         sm = torch.empty(H, S_pad * D, dtype=torch.uint8, device=dev)
         cd = torch.empty(H, S_pad * CB, dtype=torch.uint8, device=dev)
         flags = torch.empty(H, S_pad, dtype=torch.int32, device=dev)          # every row of every tile is written, padded rows as 0
-        ovf_off = torch.empty(H, S, dtype=torch.int32, device=dev)
         if H == 0 or ntiles == 0:
-            return Page(sm, cd, flags, ovf_off, torch.zeros(8, dtype=torch.uint8, device=dev), torch.zeros(H + 1, dtype=torch.int32, device=dev),
-                        torch.zeros(H, ntiles, dtype=torch.int32, device=dev), codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
+            return Page(sm, cd, flags, torch.empty(H, S, dtype=torch.int32, device=dev), torch.zeros(8, dtype=torch.uint8, device=dev),
+                        torch.zeros(H + 1, dtype=torch.int32, device=dev), torch.zeros(H, ntiles, dtype=torch.int32, device=dev), codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
         tile_off = torch.empty(H, ntiles, dtype=torch.int32, device=dev)
         head_start = torch.empty(H + 1, dtype=torch.int32, device=dev)
         x = x.contiguous()
@@ -152,11 +153,25 @@ class TileEncoder:
         slots = torch.empty(items * SLOT + 4 * (items + H), dtype=torch.uint8, device=dev)
         total = torch.empty(1, dtype=torch.int32, pin_memory=True)
         L = _lib.lib(); st = _lib.stream_ptr(dev)
-        p_flags, p_slots, p_off, p_hs = flags.data_ptr(), slots.data_ptr(), tile_off.data_ptr(), head_start.data_ptr()
+        p_flags, p_slots, p_off, p_hs, p_total = flags.data_ptr(), slots.data_ptr(), tile_off.data_ptr(), head_start.data_ptr(), total.data_ptr()
         p_work = p_slots + items * SLOT
-        _lib.check(L.gaac_encode_sized(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
-                                       sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, total.data_ptr(), st), "gaac_encode_sized")
-        ovf = torch.empty(total.item() + 8, dtype=torch.uint8, device=dev)
-        _lib.check(L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, ovf.numel(), 0, None, st),
-                   "gaac_compact_copy")
+        _lib.check(L.gaac_encode_queued(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
+                                        sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, p_total, st), "gaac_encode_queued")
+
+        def copy(ovf):
+            return L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, ovf.numel(), 0, None, st)
+        try:                                         # (the kernels write `total`: whatever happens here, it stays until they have)
+            ovf_off = torch.empty(H, S, dtype=torch.int32, device=dev)
+            ovf = torch.empty(items * ROOM + 8, dtype=torch.uint8, device=dev)
+            copied = copy(ovf)
+        finally:
+            waited = L.gaac_wait_total(p_total, st)
+        _lib.check(waited, "gaac_wait_total")
+        _lib.check(copied, "gaac_compact_copy")
+        n = total.item() + 8
+        if n <= ovf.numel():
+            ovf = ovf[:n]
+        else:
+            ovf = torch.empty(n, dtype=torch.uint8, device=dev)
+            _lib.check(copy(ovf), "gaac_compact_copy")
         return Page(sm, cd, flags, ovf_off, ovf, head_start, tile_off, codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
