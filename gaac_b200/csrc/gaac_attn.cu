@@ -132,11 +132,50 @@ __device__ __forceinline__ bool last_split(int* counter, int NS, int* s_last) {
   __syncthreads();
   return *s_last != 0;
 }
-// Partials of `heads` heads (heads <= HMAX <= 8), that of head g and split s at first + g * per_head + s * per_split -> deliver(head, M, L, acc[threadIdx.x & 127]).  All loads are independent of one
-// another (no per-split dependent chain): scale factors first, then the weighted sum with one warp per split and 16-byte loads, then a
-// cross-warp sum in shared memory.
+// Partials of a head, that of split s at first + s * step -> M, L and element d of the sum, by the whole warp.  A lane has the weights of one split, so nothing but
+// shuffles passes between the loads of up to 32 splits, which are all in flight at once, and the result.  (With a split per warp, weights and sums through shared memory and the
+// splits beyond 16 loaded behind the others, the CTA that is last took 2.1 us at 18 splits, 1.9 at 8; now 1.4.)
+template <int N> __device__ __forceinline__ void merge_splits(const AttnParams& p, long first, int step, int NS, int d, float& M, float& L, float& acc) {
+  const int lane = threadIdx.x & 31;
+  M = -CUDART_INF_F; L = 0.f; acc = 0.f;
+#pragma unroll 1
+  for (int s0 = 0; s0 < NS; s0 += N) {
+    const int n = min(N, NS - s0);
+    const long at = first + (long)s0 * step;
+    const float* v0 = p.pa + at * D + d;
+    float v[N];
+#pragma unroll
+    for (int k = 0; k < N; k += 8)
+      if (k < n) {
+#pragma unroll
+        for (int s = k; s < k + 8; s++) v[s] = __ldcg(v0 + (long)min(s, n - 1) * step * D);
+      }
+    const float m = lane < n ? __ldcg(p.pm + at + (long)lane * step) : -CUDART_INF_F, l = lane < n ? __ldcg(p.pl + at + (long)lane * step) : 0.f;
+    float most = m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(FULLM, most, o));
+    most = fmaxf(most, M);
+    const float keep = M == -CUDART_INF_F ? 0.f : fast_exp2(M - most), f = m == -CUDART_INF_F ? 0.f : fast_exp2(m - most);
+    float sum = l * f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULLM, sum, o);
+    M = most; L = L * keep + sum; acc *= keep;
+#pragma unroll
+    for (int k = 0; k < N; k += 8)
+      if (k < n) {
+#pragma unroll
+        for (int s = k; s < k + 8; s++) {
+          const float w = __shfl_sync(FULLM, f, s);
+          if (s < n) acc += w * v[s];                // (an infinite value and a weight of zero make NaN)
+        }
+      }
+  }
+}
+
+// The same of `heads` heads (heads <= HMAX <= 8), that of head g and split s at first + g * per_head + s * per_split -> deliver(head, M, L, acc[threadIdx.x & 127]), through shared memory: the
+// flat launches' loop over pieces leaves no registers for the form above (64 x 32768 tokens, groups of 8: 220 us with it and 100 bytes of spills, 210 with this), and their pairs have few pieces.
 template <int HMAX, class F>
-__device__ __forceinline__ void merge_splits(const AttnParams& p, uint8_t* area, long first, int per_head, int per_split, int heads, int NS, const F& deliver) {
+__device__ __forceinline__ void merge_pieces(const AttnParams& p, uint8_t* area, long first, int per_head, int per_split, int heads, int NS, const F& deliver) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* c_f = reinterpret_cast<float*>(area);        // [heads][NS]  m, then exp2(m - M)
   float* c_l = c_f + 8 * NS;                          // [heads][NS]  l
@@ -259,17 +298,20 @@ template <int NSET> __device__ __forceinline__ void stage_warp(const WarpAcc<NSE
 static_assert(ATT_THREADS == 512, "a thread of the merge has every fourth head");
 // Head g of the warps w0, w0 + step, .. (N of them), as they left it in shared memory (m [W][8], l [W][8], acc [W][8][ACC_LD]) -> M, L and element d of the
 // sum
+// (A lane has the weight of one warp: with all of them by every thread, 48 loads from shared memory instead of 18, the CTA took 0.2 us more.)
 template <int N> __device__ __forceinline__ void merge_warps(const uint8_t* area, int step, int w0, int g, int d, float& M, float& L, float& acc) {
   const float *sh_m = reinterpret_cast<const float*>(area), *sh_l = sh_m + ATT_WARPS * 8, *sh_acc = sh_l + ATT_WARPS * 8;
-  M = -CUDART_INF_F; L = 0.f; acc = 0.f;
+  const int own = (step * (threadIdx.x % N) + w0) * 8 + g;
+  const float m = sh_m[own], l = sh_l[own];
+  M = m;
 #pragma unroll
-  for (int w = 0; w < N; w++) M = fmaxf(M, sh_m[(step * w + w0) * 8 + g]);
+  for (int o = N / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(FULLM, M, o));
+  const float f = m == -CUDART_INF_F ? 0.f : fast_exp2(m - M);
+  L = l * f; acc = 0.f;
 #pragma unroll
-  for (int w = 0; w < N; w++) {
-    const int at = (step * w + w0) * 8 + g;
-    const float mw = sh_m[at], f = (mw == -CUDART_INF_F) ? 0.f : fast_exp2(mw - M);
-    L += sh_l[at] * f; acc += sh_acc[at * ACC_LD + d] * f;
-  }
+  for (int o = N / 2; o > 0; o >>= 1) L += __shfl_xor_sync(FULLM, L, o);
+#pragma unroll
+  for (int w = 0; w < N; w++) acc += sh_acc[((step * w + w0) * 8 + g) * ACC_LD + d] * __shfl_sync(FULLM, f, w);
 }
 // ---- V elements that are not finite.  In the value product of groups up to 4 a word meets a weight of zero for the other parity's channel, and the lower
 // half of a weight may be zero or negative in any group: an infinite or NaN element makes its word's OTHER channel NaN as well (0 x Inf), and its own NaN where Inf is
@@ -591,13 +633,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     __syncwarp();
   };
   begin_ring(false);
+  // What the grid's own numbering gives is worked out ahead of the wait: the divisions are a quarter of the time from there to the first copy.
+  int bh = blockIdx.x, b = bh / p.n_kv, kvh = bh - b * p.n_kv, chunk_all = MODE == GRID && !PAGED ? (((p.S_uniform + 15) >> 4) + p.nsplit - 1) / p.nsplit : 0;
+  if (MODE == GRID) asm volatile("" : "+r"(b), "+r"(kvh), "+r"(chunk_all));
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
 
   // Which (row, kv head, split) this CTA works on.  Normally the grid says so.  With a row order (ragged paged batches) the CTAs
   // are numbered in the order the hardware hands them out (x fastest) and that number walks the rows from the longest to the
   // shortest, all CTAs of a row together: the big CTAs start first and the small ones fill the SMs at the end.
-  int bh = blockIdx.x, split0 = blockIdx.y, S_paged = 0, ns0 = p.nsplit;
+  int split0 = blockIdx.y, S_paged = 0, ns0 = p.nsplit;
   if (SHARE) {
     int len = 0, row;
     if (lane < p.B) {
@@ -611,7 +656,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   } else if (PAGED) {
     // the row's token count for the grid's own numbering; the loads of the row order travel at the same time, so a batch whose
     // order is not used pays no extra latency for having one
-    S_paged = p.seq_len[bh / p.n_kv];
+    S_paged = p.seq_len[b];
     if (p.row_order) {
       const int linear = blockIdx.y * gridDim.x + blockIdx.x, per_row = p.n_kv * p.nsplit;
       const int rr = linear / per_row, rem = linear - rr * per_row;
@@ -619,6 +664,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if (use.x) { bh = e.x * p.n_kv + rem / p.nsplit; split0 = rem % p.nsplit; S_paged = e.y; }
       // the numbers came out of memory: tell the compiler that they are the same in every lane (see below)
       bh = __shfl_sync(FULLM, bh, 0); split0 = __shfl_sync(FULLM, split0, 0);
+      b = bh / p.n_kv; kvh = bh - b * p.n_kv;
     }
   }
   auto tokens_of = [&](int row) -> int {              // (a slot's first head stands for all of its heads)
@@ -645,7 +691,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (bh < 0) return;
     if (PAGED) S_paged = s_flat.tokens;
   }
-  int b = bh / p.n_kv, kvh = bh % p.n_kv;
+  if (MODE != GRID) { b = bh / p.n_kv; kvh = bh - b * p.n_kv; }
 
   // ---- which cache head, how many tokens, this CTA's tile range [tlo, tlo + n)
   // (without a slot map row b reads slot b; without a length table every head holds S_uniform tokens: the two dependent
@@ -664,12 +710,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // These values are the same in every thread, but they were loaded from memory: passing them through a shuffle tells the
   // compiler so, and the address arithmetic built on them stays in uniform registers.
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
-  const int ntiles = (S + 15) >> 4, chunk = (ntiles + ns0 - 1) / ns0;
+  const int ntiles = (S + 15) >> 4, chunk = MODE == GRID && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
   const int tlo = FLAT ? min(__shfl_sync(FULLM, s_flat.range[0], 0), ntiles) : min(split0 * chunk, ntiles);
   // (the last piece of a pair has what there is to the end, should a head be longer than the first one)
   const int n = FLAT ? (__shfl_sync(FULLM, s_split + 1 - s_ns, 0) == 0 ? ntiles - tlo : min(__shfl_sync(FULLM, s_flat.range[1], 0), ntiles - tlo)) : min(chunk, ntiles - tlo);
   const int nstages = (n + TPS - 1) / TPS;
-  ohk = __shfl_sync(FULLM, ohk, 0); ohv = __shfl_sync(FULLM, ohv, 0);
 
   auto meta_of = [&](int i) -> TileMeta {             // i counts from the first tile of the CTA's range
     const int tile = tlo + i;
@@ -689,8 +734,6 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // multiple of 16 bytes, at most SIDE_ESC, inside the allocation (no bytes when the boundary lies before it).  phase: of the head's first byte;  to_end: bytes from there
   // to the end of the allocation.
   struct HeadEsc { int ohk, ohv, phk, phv, k_end, v_end; };
-  const HeadEsc head_esc{ohk, ohv, PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.K.ovf) + (unsigned)ohk) & 15), PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.V.ovf) + (unsigned)ohv) & 15),
-                         PAGED ? 0 : (int)max(-1L, min((long)p.K.ovf_bytes - ohk, 0x7FFFFF00L)), PAGED ? 0 : (int)max(-1L, min((long)p.V.ovf_bytes - ohv, 0x7FFFFF00L))};
   auto esc_window = [&](int to_end, int phase, int oh, int m0, int m1, int& start, u32& bytes) {
     const int w16 = (phase + m0) & 15, left = (int)((u32)to_end - (u32)m0 + (u32)w16);
     start = m0 - w16;
@@ -744,22 +787,33 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
   };
 
-  // ---- prologue.  Everything that reads global memory is put in flight first and consumed afterwards: the first stages' payload (needs
-  // no metadata in the slot layout), their metadata, the metadata of the CTA's range, the query rows; then the tables are built while
-  // those loads travel.
-  // HBM is idle when the grid starts and every CTA asks at once: the stages that the first tiles are in go first, the others follow once
-  // the small loads are back (filling all eight at once held those loads, and with them the first tile, back for 5 us).
+  // ---- prologue.  HBM is idle when the grid starts and every CTA asks at once: what the first tiles need goes first, the small loads ahead of the first stages' payload (which needs
+  // no metadata in the slot layout), the other stages when the first tiles are there.  Each kind of load has warps of its own, since a warp comes to the barrier when its last
+  // load is back: bases, queries, metadata and payload.  us from the end of the grid's wait to the first tile, 8 heads x 500 tokens 2.5 -> 1.7, x 65536 3.7 -> 3.5 (there the first
+  // stages of all CTAs are 14 MB).
   constexpr int FIRST = (ATT_WARPS + TPS - 1) / TPS;
   const bool filler = warp < min(NSTG, nstages);                               // warp w fills stage w
   TileMeta ahead{};
-  if (filler) {
-    if (!PAGED && warp < FIRST) fill_payload(warp);
-    ahead = stage_meta(warp);
-  }
+  // The queries, by one warp for all, through the last stage's place, which is not filled before the second barrier.  Every warp on its own asked for them behind the first stages'
+  // payload and had them 1.1 us later.  (Not in a flat launch, whose pieces begin at different times: 425 -> 433 us for 16 x 4096..65536.)
+  static_assert(FIRST < NSTG && 2048 <= STAGE_BYTES, "the last stage is not one of the first");
+  uint4* const q_place = reinterpret_cast<uint4*>(smem + TB_RING + (NSTG - 1) * STAGE_BYTES) + lane;
   QFrag Q;
-  load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * D, D, G, lane);
+  if (!FLAT && warp == ATT_WARPS - 3) {
+    load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * D, D, G, lane);
+#pragma unroll
+    for (int i = 0; i < 4; i++) q_place[32 * i] = make_uint4(Q.qa[2 * i][0], Q.qa[2 * i][1], Q.qa[2 * i + 1][0], Q.qa[2 * i + 1][1]);
+  }
+  if (filler) {
+    ahead = stage_meta(warp);
+    if (!PAGED && warp < FIRST) fill_payload(warp);
+  }
+  if (FLAT) load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * D, D, G, lane);
+  ohk = __shfl_sync(FULLM, ohk, 0); ohv = __shfl_sync(FULLM, ohv, 0);          // (not before: whoever needs them waits for them)
+  const HeadEsc head_esc{ohk, ohv, PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.K.ovf) + (unsigned)ohk) & 15), PAGED ? 0 : (int)((reinterpret_cast<uintptr_t>(p.V.ovf) + (unsigned)ohv) & 15),
+                         PAGED ? 0 : (int)max(-1L, min((long)p.K.ovf_bytes - ohk, 0x7FFFFF00L)), PAGED ? 0 : (int)max(-1L, min((long)p.V.ovf_bytes - ohv, 0x7FFFFF00L))};
   {
-    const int brow = PAGED ? kvh : ch % p.n_base_rows;
+    const int brow = PAGED || p.n_base_rows == p.n_kv ? kvh : ch < p.n_base_rows ? ch : ch % p.n_base_rows;
     if (warp == ATT_WARPS - 2 && lane < 16) fill_pair_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
     if (warp == ATT_WARPS - 1 && lane < 16) fill_pair_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
     if (SHARE && tid == 0) { s_split = split0; s_ns = ns0; }
@@ -771,7 +825,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   WarpAcc<NSET> A;
   A.clear();
   __syncthreads();
-  if (filler && warp >= FIRST) { if (!PAGED) fill_payload(warp); fill_rest(warp, ahead, head_esc); }
+  if (!FLAT) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) { const uint4 w = q_place[32 * i]; Q.qa[2 * i][0] = w.x; Q.qa[2 * i][1] = w.y; Q.qa[2 * i + 1][0] = w.z; Q.qa[2 * i + 1][1] = w.w; }
+    __syncthreads();
+  }
+  if (filler && warp >= FIRST) {                     // (where all CTAs begin together, behind the warp's own first tile: any earlier, and these copies hold back the first stages')
+    u32 flags;
+    if (!FLAT) __all_sync(FULLM, mbar_wait_use(smem_s + TB_FULL + 8 * (warp / TPS), 0u, smem_s + TB_USE + 4 * warp, (u32)(warp / TPS) + 1u, flags));          // (one that runs out is met again in the main loop)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // the queries came through the last stage by ordinary stores
+    if (!PAGED) fill_payload(warp);
+    fill_rest(warp, ahead, head_esc);
+  }
 
   uint16_t* const dump_k = DUMP ? p.dump_k + (long)bh * p.dump_S * D : nullptr;
   uint16_t* const dump_v = DUMP ? p.dump_v + (long)bh * p.dump_S * D : nullptr;
@@ -873,25 +938,26 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 #pragma unroll
   for (int i = 0; i < NSET; i++) {
     const int g = (tid >> 7) + 4 * i;
-    if (g < G) merge_warps<ATT_WARPS>(smem + TB_RING, 1, 0, g, d, M[i], Lc[i], Ac[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < NSET; i++) {
-    const int g = (tid >> 7) + 4 * i;
     if (g >= G) continue;
-    if (NS == 1) deliver(g, M[i], Lc[i], Ac[i]);     // nothing to merge with
-    else {
+    merge_warps<ATT_WARPS>(smem + TB_RING, 1, 0, g, d, M[i], Lc[i], Ac[i]);
+    if (FLAT && NS == 1) deliver(g, M[i], Lc[i], Ac[i]);
+    if (NS > 1) {
       const long pidx = FLAT ? (long)(blockIdx.x + bh) * G + g : SHARE ? ((long)blockIdx.x * p.units + blockIdx.y) * G + g : (qh0 + g) * p.nsplit + split;
       if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
       p.pa[pidx * D + d] = Ac[i];
     }
   }
-  if (NS > 1) {
-    const bool last = last_split(p.counters + bh, NS, &s_last);
-    if (!FLAT && !last) return;
-    if (FLAT) { if (last) merge_splits<4 * NSET>(p, smem + TB_RING, (long)(blockIdx.x - split + bh) * G, 1, G, G, NS, deliver); }
-    else if (SHARE) merge_splits<4 * NSET>(p, smem + TB_RING, ((long)blockIdx.x * p.units + blockIdx.y - split) * G, 1, G, G, NS, deliver);
-    else merge_splits<4 * NSET>(p, smem + TB_RING, qh0 * NS, NS, 1, G, NS, deliver);
+  const bool last = NS == 1 || last_split(p.counters + bh, NS, &s_last);        // (of one split there is nothing to merge)
+  if (!FLAT && !last) return;
+  if (FLAT) { if (NS > 1 && last) merge_pieces<4 * NSET>(p, smem + TB_RING, (long)(blockIdx.x - split + bh) * G, 1, G, G, NS, deliver); }
+  else {
+#pragma unroll
+    for (int i = 0; i < NSET; i++) {
+      const int g = (tid >> 7) + 4 * i;
+      if (g >= G) continue;
+      if (NS > 1) merge_splits<32>(p, SHARE ? ((long)blockIdx.x * p.units + blockIdx.y - split) * G + g : (qh0 + g) * NS, SHARE ? G : 1, NS, d, M[i], Lc[i], Ac[i]);
+      deliver(g, M[i], Lc[i], Ac[i]);
+    }
   }
   if (p.x_recv) {
     // Every entry carries the exchange number, so nothing else announces the rows (see x_store / x_load).
@@ -1115,10 +1181,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   }
   const bool last = NS > 1 && last_split(p.counters + bh, NS, &s_last);
   if (!FLAT && !last) return;
-  for (int first = 0; last && first < 2 * G; first += 8) {
-    __syncthreads();                                   // the area is used again
-    merge_splits<8>(p, smem + T256_RING, FLAT ? (long)(blockIdx.x - split + bh) * 2 * G + first : (row0 + first) * NS, FLAT ? 1 : NS, FLAT ? 2 * G : 1, min(8, 2 * G - first), NS,
-                    [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
+  if (FLAT) {
+    for (int first = 0; last && first < 2 * G; first += 8) {
+      __syncthreads();                                 // the area is used again
+      merge_pieces<8>(p, smem + T256_RING, (long)(blockIdx.x - split + bh) * 2 * G + first, 1, 2 * G, min(8, 2 * G - first), NS, [&](int g, float, float L, float Ac) { deliver(row0 + first + g, L, Ac); });
+    }
+  } else {
+#pragma unroll 1
+    for (int vg = tid >> 7; vg < 2 * G; vg += ATT_THREADS / 128) {
+      float Mv, Lv, Av;
+      merge_splits<32>(p, (row0 + vg) * NS, 1, NS, d, Mv, Lv, Av);
+      deliver(row0 + vg, Lv, Av);
+    }
   }
   if (FLAT) __syncthreads();                         // the shared memory is used again
   } while (FLAT);
