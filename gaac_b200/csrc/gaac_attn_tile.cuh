@@ -257,9 +257,7 @@ __device__ __forceinline__ void scan_step16(u32& v, int d) {
 __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avail, const AttnView& w, u32 area, u32 room, int lane) {
   const u32 fl = live ? lds_u32(fl_at + 4u * (lane & 15)) : 0u;
   const u32 size = (u32)row_esc_bytes(fl), own_raws = (u32)popc(fl & 0xAAAAAAAAu);
-  u32x2 e[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) e[q] = lds_u64(w.segs + (q < 3 ? 8u * ((fl >> (8 * q)) & 0xFFu) : 8u * (fl >> 24)));
+  const u32x2 e[4] = {lds_u64(mad_byte<0, 8u>(fl, w.segs)), lds_u64(mad_byte<1, 8u>(fl, w.segs)), lds_u64(mad_byte<2, 8u>(fl, w.segs)), lds_u64(mad_byte<3, 8u>(fl, w.segs))};
   u32 sum = mad_k<65536u>(own_raws, size);                                   // escape bytes | raw groups << 16
   scan_step16(sum, 1); scan_step16(sum, 2); scan_step16(sum, 4); scan_step16(sum, 8);
   const u32 end = sum & 0xFFFFu, k_raws = __shfl_sync(FULLM, sum, 15) >> 16;
@@ -305,10 +303,11 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
   return staged;
 }
 
-// One group whose escape bytes are staged: half = its 16 bits of the segment words are the upper ones.
-__device__ __forceinline__ void decode_staged(u32 sm_lo, u32 sm_hi, u32 u, u32 word, bool half, const AttnView& w, const u32x4& bw, u32 out[4]) {
-  const u32 index = half ? word >> 16 : word & 0xFFFFu, m = half ? word >> 24 : index >> 8;
-  rebuild_pairs(sm_lo, sm_hi, u, m, bw, lds_u64(mad_k<8u>(index, w.addends)), out);
+// One group whose escape bytes are staged: H = half of the segment word with its index.  The addend's address and the group's m (byte 1 of the index) come out of the word by a dot product
+// each: by shifts and masks they took 16 instructions more per tile pair, all of them on the ALU, which is the busiest pipe.  65536 tokens 53.4 -> 52.6 us, 64 x 32768 211 -> 207, 16 x
+// 4096..65536 paged 424 -> 421.  (Not so the shifts and additions of rebuild_pairs as multiply-adds: 52.6 -> 52.6 and 53.7.)
+template <int H> __device__ __forceinline__ void decode_staged(u32 sm_lo, u32 sm_hi, u32 u, u32 word, const AttnView& w, const u32x4& bw, u32 out[4]) {
+  rebuild_pairs(sm_lo, sm_hi, u, mad_byte<2 * H + 1, 1u>(word, 0u), bw, lds_u64(mad_half<H, 8u>(word, w.addends)), out);
 }
 // One group whose escape bytes are read from global memory at glob[pos]; tg = its tag in the low bits.  pos advances past them.
 __device__ __forceinline__ void decode_plain(u32 sm_lo, u32 sm_hi, u32 u, u32 tg, u32& pos, const uint8_t* glob, const AttnView& w, const u32x4& bw, u32 out[4]) {
@@ -354,7 +353,7 @@ __device__ __forceinline__ void k_decode(float* sc, const SideView& s, u32 area,
       const u32 smlo = g == 0 ? s0[o].x : g == 1 ? s0[o].z : g == 2 ? s1[o].x : s1[o].z;
       const u32 smhi = g == 0 ? s0[o].y : g == 1 ? s0[o].w : g == 2 ? s1[o].y : s1[o].w;
       const u32 u = g == 0 ? code_bytes<0>(cd[o]) : g == 1 ? code_bytes<3>(cd[o]) : g == 2 ? code_bytes<6>(cd[o]) : code_bytes<9>(cd[o]);
-      if (WIN) decode_staged(smlo, smhi, u, seg[o][g >> 1], g & 1, w, bw, f[o]);
+      if (WIN) { if (g & 1) decode_staged<1>(smlo, smhi, u, seg[o][g >> 1], w, bw, f[o]); else decode_staged<0>(smlo, smhi, u, seg[o][g >> 1], w, bw, f[o]); }
       else decode_plain(smlo, smhi, u, seg[o][0] >> (2 * g), pos[o], s.glob, w, bw, f[o]);
     }
     if (DUMP) {
@@ -406,7 +405,7 @@ __device__ __forceinline__ void v_decode(WarpAcc<NSET>& A, const SideView& s, u3
       const u32 lo = g ? sm[i].z : sm[i].x, hi = g ? sm[i].w : sm[i].y;
       const u32 u = i == 0 ? (g ? code_bytes<3>(cd) : code_bytes<0>(cd)) : i == 1 ? (g ? code_bytes<9>(cd) : code_bytes<6>(cd)) :
                     i == 2 ? (g ? code_bytes<15>(cd) : code_bytes<12>(cd)) : (g ? code_bytes<21>(cd) : code_bytes<18>(cd));
-      if (WIN) decode_staged(lo, hi, u, seg[i], g, w, bw, f[i]);
+      if (WIN) { if (g) decode_staged<1>(lo, hi, u, seg[i], w, bw, f[i]); else decode_staged<0>(lo, hi, u, seg[i], w, bw, f[i]); }
       else decode_plain(lo, hi, u, seg[i] >> (2 * g), pos[i], s.glob, w, bw, f[i]);
     }
     if (DUMP) {

@@ -90,6 +90,23 @@ template <int S> GAAC_HD u32 mad_shr(u32 a, u32 c) {
 #endif
 }
 
+// byte B of a, times K (K < 256), plus c: one dot product of four bytes, where a byte's extraction is an instruction of the ALU and the multiply-add another
+template <int B, u32 K> GAAC_HD u32 mad_byte(u32 a, u32 c) {
+#if defined(__CUDA_ARCH__)
+  u32 d; asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(K << (8 * B)), "r"(c)); return d;
+#else
+  return ((a >> (8 * B)) & 0xFFu) * K + c;
+#endif
+}
+// the same for half H (0: the lower, 1: the upper) of a
+template <int H, u32 K> GAAC_HD u32 mad_half(u32 a, u32 c) {
+#if defined(__CUDA_ARCH__)
+  u32 d; asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(K << (8 * H)), "r"(c)); return d;
+#else
+  return ((a >> (16 * H)) & 0xFFFFu) * K + c;
+#endif
+}
+
 // ---- tags -> escape byte counts --------------------------------------------------------------------------------
 // escape bytes of a row with tag word fl (tier 1 -> 1 byte, tier 2 -> 5 bytes)                  gaac/kernel.py:46
 GAAC_HD int row_esc_bytes(u32 fl) { return popc(fl & 0x55555555u) + 4 * popc(fl & 0xAAAAAAAAu); }
