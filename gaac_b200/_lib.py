@@ -44,7 +44,7 @@ _SIGNATURES = {
     "gaac_head_prefix": (i32, [vp, i64, vp, vp]),
     "gaac_encode_begin": (i32, [vp, i64, i64, i64, i64, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     "gaac_encode_sized": (i32, [vp, i64, i64, i64, i64, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
-    "gaac_encode_queued": (i32, [vp, i64, i64, i64, i64, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+    "gaac_encode_queued": (i32, [vp, i64, i64, i64, i64, vp, vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     "gaac_wait_total": (i32, [vp, vp]),
     "gaac_compact_copy": (i32, [vp, vp, i64, i64, vp, vp, vp, i64, vp, i64, i64, vp, i32, i64, i64, vp, vp]),
     "gaac_decode_page": (i32, [vp, vp, vp, vp, i64, vp, vp, vp, vp, vp, i32, i32, i64, i64, i64, vp, vp]),

@@ -24,6 +24,8 @@ struct EncodeSide {
   uint8_t *sm, *codes; int* flags; uint8_t* slots; int* tile_bytes;
   int* clear;                     // optional: a word that the first block sets to zero (the ticket of the scan, a status word)
   int* cta_bytes;                 // optional: escape bytes of the tiles of every CTA, [H][gridDim.x]
+  unsigned long long* counter;    // optional: CTAs that are done << 32 | their escape bytes; zero on entry, left zero
+  int* total;                     // with counter: the last CTA writes all escape bytes here (page-locked host memory)
 };
 struct EncodeParams { EncodeSide side[2]; long S, x_head_stride, x_row_stride, S_pad; const int* bidx; int n_kv, ntiles, per_warp; };
 
@@ -71,7 +73,7 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
     if (lane == 0) s.tile_bytes[h * ntiles + tile] = total;
     sum += total;
   }
-  if (s.cta_bytes) {
+  if (s.cta_bytes || s.counter) {
     __shared__ int warp_sum[ENC_WARPS];
     if (lane == 0) warp_sum[warp] = sum;
     __syncthreads();
@@ -79,7 +81,11 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
       int all = 0;
 #pragma unroll
       for (int w = 0; w < ENC_WARPS; w++) all += warp_sum[w];
-      s.cta_bytes[h * gridDim.x + blockIdx.x] = all;
+      if (s.cta_bytes) s.cta_bytes[h * gridDim.x + blockIdx.x] = all;
+      if (s.counter) {
+        const unsigned long long before = atomicAdd(s.counter, 1ull << 32 | (u32)all);
+        if ((u32)(before >> 32) == gridDim.x * gridDim.y - 1u) { *s.counter = 0ull; *(volatile int*)s.total = (int)((u32)before + (u32)all); }
+      }
     }
   }
 }
@@ -524,12 +530,13 @@ using namespace gaac;
 
 // gaac_encode_tiles with a word that the kernel clears
 static int encode_tiles(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad, const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
-                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes, int32_t* clear, void* stream) {
+                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes, int32_t* clear, void* stream,
+                        unsigned long long* counter = nullptr, int32_t* total = nullptr) {
   if (!x_bf16 || !base3 || !base4 || !sm || !codes || !flags || !slots || !tile_bytes) return GAAC_E_ARG;
   if (H <= 0 || S <= 0 || S_in < S || S_pad < (S + T - 1) / T * T || S_pad % T || n_kv <= 0 || H > 65535 || (kind != GAAC_KIND_K && kind != GAAC_KIND_V)) return GAAC_E_ARG;
   if (!aligned16(x_bf16) || !aligned16(sm) || !aligned16(codes)) return GAAC_E_ALIGN;
   const int ntiles = (int)((S + T - 1) / T);
-  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear, nullptr}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles, tiles_per_warp(ntiles, H, ENC_RESIDENT, ENC_MOST)};
+  const EncodeParams p{{{(const uint16_t*)x_bf16, base3, base4, sm, codes, flags, slots, tile_bytes, clear, nullptr, counter, total}, {}}, S, S_in * D, D, S_pad, bidx, n_kv, ntiles, tiles_per_warp(ntiles, H, ENC_RESIDENT, ENC_MOST)};
   return launch_overlapped(kind == GAAC_KIND_K ? encode_tiles_kernel<0> : encode_tiles_kernel<1>, encode_grid(ntiles, H, 1, p.per_warp), ENC_WARPS * 32, (cudaStream_t)stream, p);
 }
 
@@ -569,10 +576,13 @@ extern "C" int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64
 extern "C" int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                                   const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                                   uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
-                                  int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream) {
-  if (!total_pinned) return GAAC_E_ARG;
+                                  int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, uint64_t* counter, void* stream) {
+  if (!total_pinned || !counter || !tile_off || !head_bytes || !head_start) return GAAC_E_ARG;
+  if (reinterpret_cast<uintptr_t>(counter) & 7) return GAAC_E_ALIGN;
   *reinterpret_cast<volatile int32_t*>(total_pinned) = -1;
-  return encode_begin(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, tile_off, head_bytes, head_start, total_pinned, stream);
+  if (int e = encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, head_start + H, stream, reinterpret_cast<unsigned long long*>(counter), total_pinned)) return e;
+  const int64_t ntiles = (S + T - 1) / T;
+  return launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, nullptr});
 }
 
 // The word is polled, since a wait for the stream would also wait for what was queued behind the kernel that writes it, and takes longer to return.  Now and then the stream is asked, which
@@ -750,7 +760,7 @@ extern "C" int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, cons
     uint8_t* slots = scratch + kind * n_items * TILE_MAX_ESC;
     int32_t *tbytes = sizes + kind * n_items, *cbytes = sizes + 2 * n_items + (int64_t)kind * n_kv * grid.x, *toff = s->tile_off + h0 * tiles_cap;
     ep.side[kind] = EncodeSide{(const uint16_t*)tok[kind], s->base3 + (h0 % n_base_rows) * D, s->base4 + (h0 % n_base_rows) * D,          // consecutive heads, consecutive rows
-                               s->sm + h0 * S_cap * D, s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots, tbytes, status + 2 * kind, cbytes};
+                               s->sm + h0 * S_cap * D, s->codes + h0 * S_cap * CB, s->flags + h0 * S_cap, slots, tbytes, status + 2 * kind, cbytes, nullptr, nullptr};
     fp.side[kind] = FinishSide{slots, tbytes, cbytes, toff, s->ovf + h0 * ovf_cap, s->ovf_used + h0, status + 2 * kind, (const uint16_t*)tok[kind], (uint16_t*)s->tail + h0 * T * D};
     cp.side[kind] = CompactSide{slots, tbytes, toff, nullptr, s->ovf + h0 * ovf_cap, nullptr, nullptr, status + 2 * kind};
   }

@@ -69,11 +69,12 @@ int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, in
                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream);
 
 /* The same in two halves: gaac_encode_queued returns as soon as the kernels are queued, gaac_wait_total when *total_pinned holds head_start[H] (until then it is
- * -1, and the memory must stay).  What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller learns the size. */
+ * -1, and the memory must stay), which is when the encode itself is done.  What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller
+ * learns the size.  counter: a device word of 8 bytes, zero before its first use; every call leaves it zero, so one serves all calls on a stream. */
 int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                        const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
-                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream);
+                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, uint64_t* counter, void* stream);
 int gaac_wait_total(const int32_t* total_pinned, void* stream);
 
 /* The copy half of gaac_compact with tile offsets that are already known: scratch slots -> ovf + head_start[h] + tile_off[h, t],

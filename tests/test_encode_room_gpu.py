@@ -26,6 +26,7 @@ def test_room(kind, monkeypatch):
             assert pg.ovf.numel() == n + 8 and bool((pg.ovf[n:] == 0).all())
             assert_pages_equal(page_to_dict(pg), ref)
             assert torch.equal(Codec.decode(pg).view(torch.int16), x.view(torch.int16))
+            assert len(encoder._COUNTERS) >= 1 and not any(int(w) for w in encoder._COUNTERS.values())
 
 
 def test_failed_allocation_waits_for_the_kernels(monkeypatch):
@@ -51,3 +52,22 @@ def test_failed_allocation_waits_for_the_kernels(monkeypatch):
             c.encode(x, "k")
     assert len(waits) == 1
     assert_pages_equal(page_to_dict(c.encode(x, "k")), O.encode(x16, c.base3.cpu().numpy(), c.base4.cpu().numpy(), "k", 2))
+
+
+def test_refused_in_a_capture():
+    """A counter made in a capture would be zero only when the graph runs: the encode is refused, and works on that stream afterwards."""
+    import torch
+    from gaac_b200 import Codec
+    x16 = O.kv_like(2, 100, seed=2)
+    x = to_bf16_cuda(x16)
+    c = Codec(2).calibrate(x)
+    side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(g, stream=side):
+            c.encode(x, "k")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        pg = c.encode(x, "k")
+    torch.cuda.synchronize()
+    assert_pages_equal(page_to_dict(pg), O.encode(x16, c.base3.cpu().numpy(), c.base4.cpu().numpy(), "k", 2))
