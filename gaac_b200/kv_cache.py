@@ -151,7 +151,7 @@ class CompressedKVCache:
             if self._pending_bytes + need > self.pending_scratch_limit:
                 self.settle_prefills()
             scratch = torch.empty(need, dtype=torch.uint8, device=k.device)
-        self._prefill_launch(slot, L, k, v, scratch, copy_only=0)
+        self._prefill_launch(slot, L, k, v, scratch, None, copy_only=0)
         if not check:
             self._pending[slot] = (L, scratch)
             self._pending_bytes += need
@@ -162,11 +162,13 @@ class CompressedKVCache:
         if wanted > self.k.ovf_cap:
             self._grow(wanted)
         if short_k or short_v:
-            self._prefill_launch(slot, L, None, None, scratch, copy_only=1)
+            self._prefill_launch(slot, L, None, None, scratch, self._slot_status[slot], copy_only=1)
 
-    def _prefill_launch(self, slot, L, k, v, scratch, copy_only: int):
+    def _prefill_launch(self, slot, L, k, v, scratch, status, copy_only: int):
+        """status: the slot's four words as a tensor, or None where their address is enough (indexing costs a microsecond)."""
         lib, dev = _lib.lib(), self.S.device
-        K, V, stream, status = self.k.c_store(), self.v.c_store(), _lib.stream_ptr(dev), self._slot_status.data_ptr() + 16 * slot
+        K, V, stream = self.k.c_store(), self.v.c_store(), _lib.stream_ptr(dev)
+        status = self._slot_status.data_ptr() + 16 * slot if status is None else status.data_ptr()
         rows = self.k.base3.shape[0]
         own = self.per_sequence_bases and L and not copy_only                                      # tables from the prompt itself
         if own and not torch.cuda.is_current_stream_capturing():
@@ -210,7 +212,7 @@ class CompressedKVCache:
         for slot, w in zip(slots, words):
             if w[0] or w[2]:
                 L, scratch = pending[slot]
-                self._prefill_launch(slot, L, None, None, scratch, copy_only=1)
+                self._prefill_launch(slot, L, None, None, scratch, self._slot_status[slot], copy_only=1)
 
     @staticmethod
     def _token_rows(x: torch.Tensor) -> torch.Tensor:
