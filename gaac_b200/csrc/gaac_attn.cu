@@ -44,7 +44,7 @@ static_assert(SIDE_BYTES == TPS * PSLOT, "both layouts use stages of the same si
 // CTA tables: addend and segment table, K / V base words; per stage the mbarrier that counts arriving bytes and how many tiles of it the warps have left so far; per
 // tile of a stage {address of its escape bytes of K, how many are staged, the same of V}, its metadata, and the word (stage + 1) << 4 | bits 2, 3: the K / V tile is
 // raw, by which a warp knows the use of the slot: a parity can be two phases off for one that runs ahead of a slow one.  Then the warps' segment areas.
-constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + BASES_BYTES, TB_LEFT = TB_FULL + 8 * NSTG, TB_ESC = TB_LEFT + 4 * NSTG, TB_META = TB_ESC + 16 * TPS * NSTG,
+constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + PAIR_BASES_BYTES, TB_LEFT = TB_FULL + 8 * NSTG, TB_ESC = TB_LEFT + 4 * NSTG, TB_META = TB_ESC + 16 * TPS * NSTG,
               TB_USE = TB_META + 8 * TPS * NSTG, TB_AREA = TB_USE + 4 * TPS * NSTG, TB_RING = TB_AREA + ATT_WARPS * AREA_BYTES;
 constexpr int ATT_SMEM = TB_RING + NSTG * STAGE_BYTES + 16;          // (an escape segment is read as whole words)
 static_assert(TB_BASES % 16 == 0 && TB_ESC % 16 == 0 && TB_AREA % 16 == 0 && TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
@@ -1006,7 +1006,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
 // (what shared memory has room for)
 constexpr int META256_TILES = 48, PATCH256 = 56, SEG256_BYTES = SEG_PATCH + 8 * PATCH256;
 constexpr int CTL_BYTES = 16;                                      // of a pair and tile parity: {next tile, fail flag of half 0, of half 1, -}
-constexpr int T256_BASES = ADDEND_BYTES + SEGTAB_BYTES, T256_META = T256_BASES + 2 * BASES_BYTES, T256_CTL = T256_META + META256_TILES * 16;
+constexpr int T256_BASES = ADDEND_BYTES + SEGTAB_BYTES, T256_META = T256_BASES + 2 * PAIR_BASES_BYTES, T256_CTL = T256_META + META256_TILES * 16;
 constexpr int T256_SEG = T256_CTL + (ATT_WARPS / 2) * 2 * CTL_BYTES, T256_RING = T256_SEG + ATT_WARPS * SEG256_BYTES;
 constexpr int STAGE256_BYTES = 16 + 2 * PSLOT, WARP256_BYTES = 2 * STAGE256_BYTES;      // stage: mbarrier, then the warp's K slot and V slot
 constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;          // (an escape segment is read as whole words)
@@ -1091,7 +1091,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * (2 * D) + hf * D, 2 * D, G, lane);
   if (warp >= 8 && warp < 12) {
     const int h2 = warp & 1, row = (2 * kvh + h2) * D;
-    uint8_t* o = smem + T256_BASES + h2 * BASES_BYTES;
+    uint8_t* o = smem + T256_BASES + h2 * PAIR_BASES_BYTES;
     if (lane < 16) { if (warp < 10) fill_pair_bases<false>(o, p.b3k + row, p.b4k + row, lane); else fill_pair_bases<true>(o, p.b3v + row, p.b4v + row, lane); }
   }
   if (tid < min(n, META256_TILES)) { const int pc = slot_of(tid); reinterpret_cast<int4*>(smem + T256_META)[tid] = make_int4(p.mt[pc], p.mt[pc + 1], p.mt[pc + 2], p.mt[pc + 3]); }
@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   A.clear();
   __syncthreads();
 
-  const AttnView W = attn_view(smem_s, smem_s + T256_BASES + hf * BASES_BYTES);
+  const AttnView W = attn_view(smem_s, smem_s + T256_BASES + hf * PAIR_BASES_BYTES);
   const u32 area = smem_s + T256_SEG + warp * SEG256_BYTES;
   int stg = 0, par = 0;
   u32 phase = 0;
