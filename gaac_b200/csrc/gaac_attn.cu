@@ -29,7 +29,7 @@
 
 namespace gaac {
 
-// Warps per CTA (18 or 20 warps at 96 registers: 64.5 us instead of 57.5 at 65536 tokens).
+// Warps per CTA (18 or 20 warps at 96 registers: 64.5 us instead of 57.5 at 65536 tokens; with the queries in shared memory, so that they spill 28 bytes only, 58.1 and 58.8 instead of 55.3).
 constexpr int ATT_WARPS = 16, ATT_THREADS = ATT_WARPS * 32;
 // ---- ring of stages.  A stage holds TPS consecutive tiles.
 //   slot layout:  per side  sign/mantissa of the tiles (TPS x 2048) | codes (TPS x 768) | tag words (TPS x 64) | the tiles' escape bytes, which are

@@ -1,10 +1,10 @@
 // Warp-level pieces of the fused decode attention: asynchronous copies, the rebuild of a compressed 16-token tile into tensor-core
 // fragments, the score and value products and the online softmax step.  Used by the kernels of gaac_attn.cu.
 //
-// What bounds them, measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens: 1062 warp instructions per (K tile + V tile) at 0.64 per cycle and scheduler, with
-// four warps to a scheduler; ALU pipe 65 %, shared-memory pipe 62 % (of all cycles), DRAM 39 %.  A warp issues every 6.25 cycles and spends, of these, 1.2 waiting for a
-// result of fixed latency, 1.1 ready but not chosen, 0.9 on shared memory, 0.8 on a busy pipe (the ALU), 0.3 at barriers, 0.25 on global memory: instructions
-// first, then latency, since a third of the issue slots finds no warp ready.  More warps do not fit (gaac_attn.cu: 18 or 20 at 96 registers).  Timing-only builds of an earlier
+// What bounds them, measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens: 1052 warp instructions per (K tile + V tile) at 0.66 per cycle and scheduler (0.74 in the main loop), with
+// four warps to a scheduler; ALU pipe 61 %, the shared-memory pipe 282 cycles of the main loop's 345 per tile pair, DRAM 42 %.  A warp issues every 6 cycles and spends, of these, 1.2 waiting for a
+// result of fixed latency, 1.1 ready but not chosen, 0.9 on shared memory, 0.7 on a busy pipe (the ALU), 0.3 at barriers, 0.25 on global memory: instructions and cycles of shared memory
+// first, then latency, since a third of the issue slots finds no warp ready.  More warps do not help (gaac_attn.cu: 18 or 20 at 96 registers).  Timing-only builds of an earlier
 // form: without the raw groups 50 us of 57, without any of plan_tile 41.  What did not help: moving shifts from the ALU to the FMA pipe, fewer or longer chains at the same
 // count of instructions, warps of their own for plan_tile or for the copies.
 //
