@@ -582,7 +582,9 @@ extern "C" int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int6
   *reinterpret_cast<volatile int32_t*>(total_pinned) = -1;
   if (int e = encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, head_start + H, stream, reinterpret_cast<unsigned long long*>(counter), total_pinned)) return e;
   const int64_t ntiles = (S + T - 1) / T;
-  return launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, nullptr});
+  const int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, nullptr});
+  if (e) { cudaStreamSynchronize((cudaStream_t)stream); cudaGetLastError(); }                  // the encode still writes *total_pinned, which goes with a failed call
+  return e;
 }
 
 // The word is polled, since a wait for the stream would also wait for what was queued behind the kernel that writes it, and takes longer to return.  Now and then the stream is asked, which
