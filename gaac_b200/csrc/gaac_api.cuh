@@ -10,7 +10,7 @@ inline int launch_status() { return cudaGetLastError() == cudaSuccess ? GAAC_OK 
 
 // ---- programmatic dependent launch.  A kernel launched with launch_overlapped may become resident while the kernel before it in the stream is still
 // running, once every block of that one has executed griddep_launch() or exited; it begins with griddep_wait(), which returns when that
-// kernel has completed and its writes are visible, and touches no memory before.  Behind an ordinary kernel, and with the switch off, all of
+// kernel has completed and its writes are visible, and touches no memory before (but see exponent_hist_kernel behind clear_kernel).  Behind an ordinary kernel, and with the switch off, all of
 // this does nothing.  It takes a launch's latency (1-2 us) off chains of short kernels.
 inline int g_launch_overlap = 1;      // see gaac_set_launch_overlap
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

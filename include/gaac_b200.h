@@ -123,9 +123,9 @@ typedef struct {
   const void* tail;           /* [heads, tail_cap, 128] bf16 raw tail, or NULL */
 } gaac_side;
 
-/* The attention and exchange-merge kernels, and the short kernels that follow another one inside a call (offset scan, escape copy, window
- * search, return of raw tiles), are launched with programmatic stream serialisation allowed and begin with griddepcontrol.wait: behind a kernel that signals early (these do) their CTAs become resident while that kernel is still
- * finishing, so consecutive attention layers overlap by a few microseconds; nothing is read or written before the wait returns.
+/* Nearly all kernels (not the public histogram, gaac_head_prefix, gaac_paged_release and the clearing of a prompt's counters) are launched with programmatic
+ * stream serialisation allowed and wait with griddepcontrol.wait: behind a kernel that signals early (these do) their CTAs become resident while that kernel is still
+ * finishing, so consecutive attention layers overlap by a few microseconds; nothing that an earlier kernel may write is read, and nothing written, before the wait returns.
  * enabled = 0 switches this off for later launches of the process (every launch then starts after its predecessor has finished
  * entirely, which is what a measurement of one launch's own duration wants); 1, the default, switches it back on.  Not
  * thread-safe against concurrent launches.  No counterpart in the reference. */
