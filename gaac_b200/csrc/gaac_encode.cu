@@ -1,6 +1,7 @@
 // Block encoder, escape-stream compaction, page decoder and calibration kernels (sm_100a).
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 #include "gaac_api.cuh"
 #include "gaac_warp.cuh"
 
@@ -700,6 +701,13 @@ extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, co
                                            : calibrate<int>(K, V, k_tok, v_tok, L, row_stride, n_ch, at, scratch, false, st);
 }
 
+// Between the launches of a call its counters hold a prompt's counts, so the launches of another call with the same workspace must not come in between: the workspace's lock is
+// held while they are queued (one of 64 by the address).
+static std::mutex& workspace_lock(const void* workspace) {
+  static std::mutex locks[64];
+  return locks[(reinterpret_cast<uintptr_t>(workspace) >> 9) % 64];
+}
+
 extern "C" size_t gaac_cache_tables_workspace_bytes(int n_kv) { return n_kv > 0 ? 2 * (size_t)n_kv * D * 64 * sizeof(Packed) : 0; }
 
 extern "C" int gaac_cache_prefill_own(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
@@ -714,6 +722,7 @@ extern "C" int gaac_cache_prefill_own(const gaac_store* K, const gaac_store* V, 
     if (int e = gaac_cache_calibrate(K, V, k_tok, v_tok, L, row_stride, slot, n_kv, n_base_rows, scratch, scratch_bytes, stream)) return e;
   } else {
     const long n_ch = (long)n_kv * D;
+    const std::lock_guard<std::mutex> held(workspace_lock(workspace));
     if (int e = calibrate<Packed>(K, V, k_tok, v_tok, L, row_stride, n_ch, (long)slot * n_ch, workspace, true, (cudaStream_t)stream)) return e;
   }
   return gaac_cache_prefill(K, V, k_tok, v_tok, L, row_stride, slot, n_kv, tail_len, seq_len, S_cap, ovf_cap, n_base_rows, scratch, scratch_bytes, status, 0, stream);

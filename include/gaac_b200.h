@@ -309,7 +309,8 @@ int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, const void* k_t
 
 /* gaac_cache_calibrate and gaac_cache_prefill of a prompt (L > 0) in one call and, up to 65535 tokens, four launches in all: the same tables, bytes and
  * status.  workspace: gaac_cache_tables_workspace_bytes(n_kv) bytes, 16-byte aligned, zero before its first use; every call leaves it zero, so one serves all calls on a
- * stream, whatever their n_kv (it must be large enough for each).  Calls that may overlap on the GPU need one each. */
+ * stream, whatever their n_kv (it must be large enough for each) and whichever host thread they come from (a lock keeps the launches of two calls apart).  Calls that may overlap on
+ * the GPU need one each. */
 size_t gaac_cache_tables_workspace_bytes(int n_kv);
 int gaac_cache_prefill_own(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,
                            int32_t* tail_len, int32_t* seq_len, int64_t S_cap, int64_t ovf_cap, int n_base_rows, uint8_t* scratch, size_t scratch_bytes,
