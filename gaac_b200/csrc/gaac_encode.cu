@@ -673,7 +673,8 @@ constexpr int CACHE_READ_PAD = 8;      // bytes kept free behind a head's escape
 
 extern "C" size_t gaac_cache_calibrate_scratch_bytes(int n_kv) { return 2 * (size_t)(n_kv > 0 ? n_kv : 0) * D * 256 * sizeof(int32_t); }
 
-// Histograms of both kinds, windows into the slot's rows of the tables.  zeroed: the counters are zero, and are left so; else they are cleared first, which takes a launch more.
+// Histograms of both kinds, windows into the slot's rows of the tables.  zeroed: the counters are zero, and are left so, by a call that fails too; else they are cleared first,
+// which takes a launch more.
 template <class Cnt>
 static int calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, long n_ch, long at, uint8_t* counters, bool zeroed, cudaStream_t st) {
   Cnt* hist = reinterpret_cast<Cnt*>(counters);
@@ -683,10 +684,12 @@ static int calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok
   const HistParams<Cnt> hp{{(const uint16_t*)k_tok, (const uint16_t*)v_tok}, {hist, hist + one}, L, n_ch, row_stride};
   const bool pairs = hist_pairs(k_tok, n_ch, row_stride) && hist_pairs(v_tok, n_ch, row_stride);
   const auto kernel = zeroed ? (pairs ? exponent_hist_kernel<Cnt, true, false> : exponent_hist_kernel<Cnt, false, false>) : (pairs ? exponent_hist_kernel<Cnt, true, true> : exponent_hist_kernel<Cnt, false, true>);
-  if (int e = launch_overlapped(kernel, hist_grid(n_ch, L, 2), HIST_THREADS, st, hp)) return e;
+  int e = launch_overlapped(kernel, hist_grid(n_ch, L, 2), HIST_THREADS, st, hp);
   const BasesParams<Cnt> bp{{hist, hist + one}, {const_cast<uint8_t*>(K->base3) + at, const_cast<uint8_t*>(V->base3) + at},
                             {const_cast<uint8_t*>(K->base4) + at, const_cast<uint8_t*>(V->base4) + at}, n_ch, zeroed};
-  return launch_overlapped(bases_from_hist_kernel<Cnt>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
+  if (!e) e = launch_overlapped(bases_from_hist_kernel<Cnt>, dim3((unsigned)((n_ch + 3) / 4), 2), 128, st, bp);
+  if (e && zeroed) { cudaMemsetAsync(counters, 0, 4 * (size_t)n, st); cudaGetLastError(); }      // (the histogram may be queued: an error that an earlier call left behind is reported here too)
+  return e;
 }
 
 extern "C" int gaac_cache_calibrate(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,

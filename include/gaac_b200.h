@@ -308,8 +308,8 @@ int gaac_cache_prefill(const gaac_store* K, const gaac_store* V, const void* k_t
                        size_t scratch_bytes, int32_t* status, int copy_only, void* stream);
 
 /* gaac_cache_calibrate and gaac_cache_prefill of a prompt (L > 0) in one call and, up to 65535 tokens, four launches in all: the same tables, bytes and
- * status.  workspace: gaac_cache_tables_workspace_bytes(n_kv) bytes, 16-byte aligned, zero before its first use; every call leaves it zero, so one serves all calls on a
- * stream, whatever their n_kv (it must be large enough for each) and whichever host thread they come from (a lock keeps the launches of two calls apart).  Calls that may overlap on
+ * status.  workspace: gaac_cache_tables_workspace_bytes(n_kv) bytes, 16-byte aligned, zero before its first use; every call, a failed one too, leaves it zero, so one
+ * serves all calls on a stream, whatever their n_kv (it must be large enough for each) and whichever host thread they come from (a lock keeps the launches of two calls apart).  Calls that may overlap on
  * the GPU need one each. */
 size_t gaac_cache_tables_workspace_bytes(int n_kv);
 int gaac_cache_prefill_own(const gaac_store* K, const gaac_store* V, const void* k_tok, const void* v_tok, int64_t L, int64_t row_stride, int slot, int n_kv,

@@ -1,0 +1,36 @@
+"""Calls that fail although their kernels were queued (an error that an earlier call of the program left behind is reported by the launch that finds it): what they share with later calls, and
+what the caller may free, is in order when they return."""
+import ctypes
+import numpy as np
+import pytest
+from common import to_bf16_cuda
+from oracle import gaac_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _leave_an_error_behind():
+    """A CUDA call that is refused on the host and whose error nobody has taken."""
+    assert ctypes.CDLL("libcudart.so.12").cudaSetDevice(9999) != 0
+
+
+def test_prompt_counters():
+    import torch
+    from gaac_b200 import CompressedKVCache, _lib
+    n_kv, L, lib = 2, 300, _lib.lib()
+    rows = [np.ascontiguousarray(O.kv_like(n_kv, L, seed=s).transpose(1, 0, 2)) for s in (1, 2)]
+    rows[0] = np.full_like(rows[0], 0x3F80)          # its counts would outweigh those of any other prompt
+    x, c = [to_bf16_cuda(r) for r in rows], CompressedKVCache(2, n_kv, L)
+    ws = torch.zeros(lib.gaac_cache_tables_workspace_bytes(n_kv), dtype=torch.uint8, device="cuda")
+    scratch = torch.empty(lib.gaac_cache_prefill_scratch_bytes(L, n_kv), dtype=torch.uint8, device="cuda")
+    stream = _lib.stream_ptr(torch.device("cuda", 0))
+    call = lambda slot: lib.gaac_cache_prefill_own(c.k.c_store(), c.v.c_store(), x[slot].data_ptr(), x[slot].data_ptr(), L, n_kv * 128, slot, n_kv, c.tail_len.data_ptr(), c.S.data_ptr(),
+                                                   c.cap, c.k.ovf_cap, 2 * n_kv, scratch.data_ptr(), scratch.numel(), c._slot_status.data_ptr() + 16 * slot, ws.data_ptr(), ws.numel(), stream)
+    torch.cuda.synchronize()
+    _leave_an_error_behind()
+    assert call(0) != 0
+    assert call(1) == 0
+    for st in (c.k, c.v):
+        b3, b4 = O.calibrate(np.ascontiguousarray(rows[1].transpose(1, 0, 2)), n_kv)
+        assert np.array_equal(st.base3[n_kv:].cpu().numpy(), b3) and np.array_equal(st.base4[n_kv:].cpu().numpy(), b4)
+    assert not bool(ws.any())
