@@ -581,10 +581,11 @@ extern "C" int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int6
   if (!total_pinned || !counter || !tile_off || !head_bytes || !head_start) return GAAC_E_ARG;
   if (reinterpret_cast<uintptr_t>(counter) & 7) return GAAC_E_ALIGN;
   *reinterpret_cast<volatile int32_t*>(total_pinned) = -1;
-  if (int e = encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, head_start + H, stream, reinterpret_cast<unsigned long long*>(counter), total_pinned)) return e;
+  int e = encode_tiles(x_bf16, H, S, S_in, S_pad, base3, base4, bidx, n_kv, kind, sm, codes, flags, slots, tile_bytes, head_start + H, stream, reinterpret_cast<unsigned long long*>(counter), total_pinned);
   const int64_t ntiles = (S + T - 1) / T;
-  const int e = launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, nullptr});
-  if (e) { cudaStreamSynchronize((cudaStream_t)stream); cudaGetLastError(); }                  // the encode still writes *total_pinned, which goes with a failed call
+  if (!e) e = launch_overlapped(tile_scan_kernel, dim3((unsigned)H), SCAN_THREADS, (cudaStream_t)stream, ScanParams{{{tile_bytes, tile_off, head_bytes}, {}}, (int)ntiles, ntiles, head_start, nullptr});
+  // The encode may be queued, since a launch also reports an error that an earlier call left behind, and then still writes *total_pinned, which goes with a failed call.
+  if (e == GAAC_E_LAUNCH) { cudaStreamSynchronize((cudaStream_t)stream); cudaGetLastError(); }
   return e;
 }
 

@@ -34,3 +34,28 @@ def test_prompt_counters():
         b3, b4 = O.calibrate(np.ascontiguousarray(rows[1].transpose(1, 0, 2)), n_kv)
         assert np.array_equal(st.base3[n_kv:].cpu().numpy(), b3) and np.array_equal(st.base4[n_kv:].cpu().numpy(), b4)
     assert not bool(ws.any())
+
+
+def test_encode_has_written_its_total():
+    """A caller frees the total with a call that failed: by then the kernel that writes it has ended, although it was queued behind others."""
+    import torch
+    from gaac_b200 import Codec, _lib
+    S, lib = 65536, _lib.lib()
+    x16 = O.kv_like(1, S, seed=2)
+    x = to_bf16_cuda(x16)
+    c = Codec(1).calibrate(x)
+    u8, i32 = dict(dtype=torch.uint8, device="cuda"), dict(dtype=torch.int32, device="cuda")
+    sm, codes, slots = torch.empty(S * 128, **u8), torch.empty(S * 48, **u8), torch.empty(S // 16 * 1280, **u8)
+    flags, sizes, off, ends = torch.empty(S, **i32), torch.empty(S // 16, **i32), torch.empty(S // 16, **i32), torch.empty(3, **i32)
+    counter, total, work = torch.zeros(1, dtype=torch.int64, device="cuda"), torch.full((1,), 7, dtype=torch.int32, pin_memory=True), torch.zeros(1 << 28, **u8)
+    call = lambda: lib.gaac_encode_queued(x.data_ptr(), 1, S, S, S, c.base3.data_ptr(), c.base4.data_ptr(), None, 1, 0, sm.data_ptr(), codes.data_ptr(), flags.data_ptr(), slots.data_ptr(),
+                                          sizes.data_ptr(), off.data_ptr(), ends.data_ptr() + 8, ends.data_ptr(), total.data_ptr(), counter.data_ptr(), stream)
+    stream = _lib.stream_ptr(torch.device("cuda", 0))
+    torch.cuda.synchronize()
+    for _ in range(10): work.add_(1)                 # about a millisecond
+    _leave_an_error_behind()
+    assert call() != 0
+    n = int(total)
+    page = c.encode(x, "k")
+    assert n == int(page.ovf_head_start[-1]) and int(counter) == 0
+    assert call() == 0 and lib.gaac_wait_total(total.data_ptr(), stream) == 0 and int(total) == n
