@@ -600,7 +600,8 @@ extern "C" int gaac_wait_total(const int32_t* total_pinned, void* stream) {
       __builtin_ia32_pause();
     }
     const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
-    if (e == cudaErrorNotReady) { cudaGetLastError(); continue; }
+    if (e != cudaSuccess) cudaGetLastError();        // (reported here, so not by a later launch as well)
+    if (e == cudaErrorNotReady) continue;
     return e == cudaSuccess && *word >= 0 ? GAAC_OK : GAAC_E_LAUNCH;
   }
 }

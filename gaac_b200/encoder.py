@@ -22,8 +22,6 @@ _COUNTERS = {}  # (device index, stream) -> the word that the encoder's CTAs cou
 def _counter(dev, stream: int) -> int:
     word = _COUNTERS.get((dev.index, stream))
     if word is None:
-        if torch.cuda.is_current_stream_capturing():                            # (it would be zero only when the graph runs)
-            raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
         word = _COUNTERS.setdefault((dev.index, stream), torch.zeros(1, dtype=torch.int64, device=dev))
     return word.data_ptr()
 
@@ -150,6 +148,8 @@ class TileEncoder:
         H, S, _ = x.shape; dev = x.device
         S_pad = (S + T - 1) // T * T
         ntiles = S_pad // T
+        if H and ntiles and torch.cuda.is_current_stream_capturing():           # before anything that would become part of the graph
+            raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
         sm = torch.empty(H, S_pad * D, dtype=torch.uint8, device=dev)
         cd = torch.empty(H, S_pad * CB, dtype=torch.uint8, device=dev)
         flags = torch.empty(H, S_pad, dtype=torch.int32, device=dev)          # every row of every tile is written, padded rows as 0

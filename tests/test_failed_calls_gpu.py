@@ -11,7 +11,11 @@ pytestmark = pytest.mark.gpu
 
 def _leave_an_error_behind():
     """A CUDA call that is refused on the host and whose error nobody has taken."""
-    assert ctypes.CDLL("libcudart.so.12").cudaSetDevice(9999) != 0
+    assert _cudart().cudaSetDevice(9999) != 0
+
+
+def _cudart():
+    return ctypes.CDLL("libcudart.so.12")
 
 
 def test_prompt_counters():
@@ -59,3 +63,38 @@ def test_encode_has_written_its_total():
     page = c.encode(x, "k")
     assert n == int(page.ovf_head_start[-1]) and int(counter) == 0
     assert call() == 0 and lib.gaac_wait_total(total.data_ptr(), stream) == 0 and int(total) == n
+
+
+def test_encode_is_refused_in_a_capture_of_a_stream_that_has_encoded():
+    """.. before anything of it is captured: the graph goes on without it."""
+    import torch
+    from gaac_b200 import Codec
+    x = to_bf16_cuda(O.kv_like(2, 100, seed=2))
+    c, side, graph, y = Codec(2).calibrate(x), torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros(4, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        c.encode(x, "k")
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        with pytest.raises(RuntimeError, match="cannot be captured"):
+            c.encode(x, "k")
+        assert c.encode(x[:0], "k").S == 100         # (no heads: no kernels)
+        y.add_(1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert y.tolist() == [1.0] * 4
+
+
+def test_wait_for_a_total_takes_its_error():
+    """A stream that is being captured cannot be asked: the wait says so, and no later launch does."""
+    import torch
+    from gaac_b200 import _lib
+    side, word, graph, rt = torch.cuda.Stream(), ctypes.c_int32(-1), ctypes.c_void_p(), _cudart()
+    stream = ctypes.c_void_p(side.cuda_stream)
+    assert rt.cudaStreamBeginCapture(stream, 2) == 0
+    try:
+        assert _lib.lib().gaac_wait_total(ctypes.byref(word), stream) == 4
+        assert rt.cudaPeekAtLastError() == 0
+    finally:
+        assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) != 0        # the question ended the capture
+        rt.cudaGetLastError()
