@@ -13,6 +13,7 @@ Buffer shapes, field names and the byte accounting follow gaac/kv_cache.py:99-14
 read them; the device work goes through libgaac_b200.so.
 """
 from __future__ import annotations
+import operator
 import torch
 from . import _lib
 from .codec import Codec, Page, D, T, CB
@@ -131,7 +132,7 @@ class CompressedKVCache:
         slots (160 B per token and kv head) until settle_prefills() - which append, attention, decompress, check_capacity
         and stats call first - reads the status words of all such prefills in one go and repairs the slots whose streams were
         too small.  A step that prefills several prompts then waits for the GPU once, not once per prompt."""
-        L = k.shape[0]
+        L, slot = k.shape[0], operator.index(slot)   # (a slot number out of an array or a tensor, which is no int where an address is computed)
         assert L <= self.cap, f"sequence of {L} tokens exceeds the cache capacity {self.cap}"
         assert 0 <= slot < self.n_slots
         k, v = self._token_rows(k), self._token_rows(v)
