@@ -226,9 +226,9 @@ __global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant
   const int toff = live ? s.tile_off[h * p.tile_off_stride + t] : 0;
   const uint8_t* src = s.slots + (long)item * TILE_MAX_ESC;
   // bounds: the whole stream must fit ovf_cap bytes (ovf_cap > 0), a head's part head_cap bytes (head_cap > 0), read padding
-  // included; a tile that does not fit is not written and bit 0 of *status is set
+  // included; a tile that does not fit is not written and bit 0 of *status is set.  Offsets below zero are those of a stream that 31 bits cannot count: they fit nowhere.
   const long at = (s.head_start ? (long)s.head_start[h] : (long)h * p.head_stride) + toff;        // no table: head h's stream starts at h * head_stride
-  const bool fits = (p.ovf_cap <= 0 || at + n + p.zero_pad <= p.ovf_cap) && (p.head_cap <= 0 || (long)toff + n + p.zero_pad <= p.head_cap);
+  const bool fits = at >= 0 && toff >= 0 && (p.ovf_cap <= 0 || at + n + p.zero_pad <= p.ovf_cap) && (p.head_cap <= 0 || (long)toff + n + p.zero_pad <= p.head_cap);
   if (fits) {
     uint8_t* dst = s.ovf + at;
 #pragma unroll 4
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(128) compact_copy_kernel(const __grid_constant
   } else if (live && q == 0 && s.status) atomicOr(s.status, 1);
   if (p.zero_pad && p.head_cap <= 0 && s.head_start && first == 0 && lane < p.zero_pad) {                              // over-read padding behind the last head (packed stream)
     const long end = (long)s.head_start[p.n_items / (unsigned)p.ntiles];
-    if (p.ovf_cap <= 0 || end + p.zero_pad <= p.ovf_cap) s.ovf[end + lane] = 0;
+    if (end >= 0 && (p.ovf_cap <= 0 || end + p.zero_pad <= p.ovf_cap)) s.ovf[end + lane] = 0;
     else if (lane == 0 && s.status) atomicOr(s.status, 1);
   }
   if (s.ovf_off) {
