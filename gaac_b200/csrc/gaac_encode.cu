@@ -19,14 +19,18 @@ static int tiles_per_warp(int64_t ntiles, int64_t rows, int resident, int most) 
   return (int)std::max<int64_t>(1, std::min<int64_t>(most, ctas / resident));
 }
 
+// 2^40 escape bytes are those of 3.5 TB of BF16, 2^24 CTAs (of 16 tiles in a launch of so many, and at most one more per head) those of 1.1 TB: neither part overflows.
+constexpr int DONE_SHIFT = 40;
+constexpr int TOTAL_TOO_LARGE = -2;
+
 // What one kind's encode reads and writes.
 struct EncodeSide {
   const uint16_t* x; const uint8_t *base3, *base4;
   uint8_t *sm, *codes; int* flags; uint8_t* slots; int* tile_bytes;
   int* clear;                     // optional: a word that the first block sets to zero (the ticket of the scan, a status word)
   int* cta_bytes;                 // optional: escape bytes of the tiles of every CTA, [H][gridDim.x]
-  unsigned long long* counter;    // optional: CTAs that are done << 32 | their escape bytes; zero on entry, left zero
-  int* total;                     // with counter: the last CTA writes all escape bytes here (page-locked host memory)
+  unsigned long long* counter;    // optional: CTAs that are done << DONE_SHIFT | their escape bytes; zero on entry, left zero
+  int* total;                     // with counter: the last CTA writes all escape bytes here (page-locked host memory), -2 for more than 31 bits hold
 };
 struct EncodeParams { EncodeSide side[2]; long S, x_head_stride, x_row_stride, S_pad; const int* bidx; int n_kv, ntiles, per_warp; };
 
@@ -84,8 +88,12 @@ __device__ __forceinline__ void encode_tiles_cta(const EncodeParams& p, const En
       for (int w = 0; w < ENC_WARPS; w++) all += warp_sum[w];
       if (s.cta_bytes) s.cta_bytes[h * gridDim.x + blockIdx.x] = all;
       if (s.counter) {
-        const unsigned long long before = atomicAdd(s.counter, 1ull << 32 | (u32)all);
-        if ((u32)(before >> 32) == gridDim.x * gridDim.y - 1u) { *s.counter = 0ull; *(volatile int*)s.total = (int)((u32)before + (u32)all); }
+        const unsigned long long before = atomicAdd(s.counter, 1ull << DONE_SHIFT | (u32)all);
+        if ((u32)(before >> DONE_SHIFT) == gridDim.x * gridDim.y - 1u) {
+          const unsigned long long bytes = (before & ((1ull << DONE_SHIFT) - 1)) + (u32)all;
+          *s.counter = 0ull;
+          *(volatile int*)s.total = bytes > 0x7FFFFFFFull ? TOTAL_TOO_LARGE : (int)bytes;
+        }
       }
     }
   }
@@ -596,7 +604,8 @@ extern "C" int gaac_wait_total(const int32_t* total_pinned, void* stream) {
   const volatile int32_t* const word = total_pinned;
   while (true) {
     for (int i = 0; i < 4096; i++) {
-      if (*word >= 0) { std::atomic_thread_fence(std::memory_order_acquire); return GAAC_OK; }
+      const int32_t total = *word;
+      if (total != -1) { std::atomic_thread_fence(std::memory_order_acquire); return total >= 0 ? GAAC_OK : GAAC_E_ARG; }
       __builtin_ia32_pause();
     }
     const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);

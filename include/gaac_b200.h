@@ -69,7 +69,7 @@ int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, in
                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream);
 
 /* The same in two halves: gaac_encode_queued returns as soon as the kernels are queued, gaac_wait_total when *total_pinned holds head_start[H] (until then it is
- * -1, and the memory must stay), which is when the encode itself is done.  What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller
+ * -1, and the memory must stay), which is when the encode itself is done; GAAC_E_ARG says that there are more bytes than 31 bits count, and the offsets are not valid.  What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller
  * learns the size.  counter: a device word of 8 bytes, zero before its first use; every call leaves it zero, so one serves all calls on a stream. */
 int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                        const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
