@@ -5,6 +5,8 @@ There is no fallback: if the library is missing or a call fails, a RuntimeError 
 from __future__ import annotations
 import ctypes as C
 import os
+import threading
+import weakref
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("GAAC_B200_LIB") or os.path.join(_HERE, "libgaac_b200.so")     # GAAC_B200_LIB: use a library built elsewhere
@@ -119,6 +121,47 @@ def row_stride(t) -> int:
     for s in t.shape[1:]:
         n *= s
     return max(n, 1)
+
+
+class _Buffers(dict):                                # (device index, stream) -> buffer, oldest first
+    __slots__ = ("__weakref__",)
+
+
+class Kept:
+    """Zeroed device buffers that every call leaves zero, so that one per stream serves all objects that make such calls.  They live as long as one of the objects that have
+    asked for them; beyond MOST streams the oldest goes.  A buffer that goes is the allocator's again on the stream that it was made and used on; the caller holds what it was given until
+    its launches are queued, since another thread's call may drop it here."""
+    MOST = 32
+
+    def __init__(self, dtype: str):
+        self._dtype, self._users, self._now, self._lock = dtype, weakref.WeakKeyDictionary(), lambda: None, threading.RLock()
+
+    def of(self, user, dev, stream: int, n: int):
+        """n or more elements for `user`'s calls on the current stream of dev, which must not be capturing (they would be zero only when the graph runs)."""
+        buffers = self._users.get(user)
+        if buffers is None:
+            with self._lock:
+                buffers = self._now()
+                if buffers is None:
+                    buffers = _Buffers()
+                    self._now = weakref.ref(buffers)
+                self._users[user] = buffers
+        t = buffers.get((dev.index, stream))
+        if t is None or t.numel() < n:
+            import torch
+            t = torch.zeros(n, dtype=getattr(torch, self._dtype), device=dev)
+            with self._lock:
+                buffers.pop((dev.index, stream), None)
+                buffers[dev.index, stream] = t
+                while len(buffers) > self.MOST:
+                    del buffers[next(iter(buffers))]
+        return t
+
+    def values(self) -> list:
+        return list((self._now() or {}).values())
+
+    def __len__(self):
+        return len(self._now() or ())
 
 
 def ptr(t):

@@ -16,14 +16,7 @@ ROOM = 80       # escape bytes per tile that encode makes room for before it kno
                 # us of K and V, a copy launched after a wait for the size -> one queued behind the kernels: [8, 1111, 128] 110 -> 91, [8, 65536, 128] 194 -> 175.
 
 
-_COUNTERS = {}  # (device index, stream) -> the word that the encoder's CTAs count themselves in: zeroed once, left zero by every call
-
-
-def _counter(dev, stream: int) -> int:
-    word = _COUNTERS.get((dev.index, stream))
-    if word is None:
-        word = _COUNTERS.setdefault((dev.index, stream), torch.zeros(1, dtype=torch.int64, device=dev))
-    return word.data_ptr()
+_COUNTERS = _lib.Kept("int64")       # the word that the encoder's CTAs count themselves in
 
 
 class TileEncoder:
@@ -167,8 +160,9 @@ class TileEncoder:
         L = _lib.lib(); st = _lib.stream_ptr(dev)
         p_flags, p_slots, p_off, p_hs, p_total = flags.data_ptr(), slots.data_ptr(), tile_off.data_ptr(), head_start.data_ptr(), total.data_ptr()
         p_work = p_slots + items * SLOT
+        word = _COUNTERS.of(codec if isinstance(codec, Codec) else self, dev, st, 1)
         _lib.check(L.gaac_encode_queued(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
-                                        sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, p_total, _counter(dev, st), st), "gaac_encode_queued")
+                                        sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, p_total, word.data_ptr(), st), "gaac_encode_queued")
 
         def copy(ovf):
             return L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, ovf.numel(), 0, None, st)

@@ -62,16 +62,7 @@ class _Store:
                           self.tail.data_ptr(), self.base3.data_ptr(), self.base4.data_ptr())
 
 
-_TABLES = {}     # (device index, stream) -> counters of a prompt's tables, 128 KB per kv head: zeroed once, left zero by every call, shared by all caches
-
-
-def _tables_workspace(lib, dev, stream: int, n_kv: int) -> torch.Tensor:
-    """The counters of the current stream.  Nothing but calls on that stream uses them, so one that became too small can go."""
-    need, key = lib.gaac_cache_tables_workspace_bytes(n_kv), (dev.index, stream)
-    ws = _TABLES.get(key)
-    if ws is None or ws.numel() < need:
-        ws = _TABLES[key] = torch.zeros(need, dtype=torch.uint8, device=dev)
-    return ws
+_TABLES = _lib.Kept("uint8")         # counters of a prompt's tables, 128 KB per kv head
 
 
 class CompressedKVCache:
@@ -173,7 +164,7 @@ class CompressedKVCache:
         rows = self.k.base3.shape[0]
         own = self.per_sequence_bases and L and not copy_only                                      # tables from the prompt itself
         if own and not torch.cuda.is_current_stream_capturing():
-            ws = _tables_workspace(lib, dev, stream, self.n_kv)
+            ws = _TABLES.of(self, dev, stream, lib.gaac_cache_tables_workspace_bytes(self.n_kv))
             _lib.check(lib.gaac_cache_prefill_own(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(),
                                                   self.cap, self.k.ovf_cap, rows, scratch.data_ptr(), scratch.numel(), status, ws.data_ptr(), ws.numel(), stream),
                        "gaac_cache_prefill_own")
