@@ -27,6 +27,7 @@ def _paged(E):
     import torch
     from gaac_b200 import Codec
     from gaac_b200.vllm.store import LayerState, OVF_OFF
+    from gaac_b200.vllm.paged_kernel import paged_attention
     x = to_bf16_cuda(O.kv_like(N_KV, 16 * E + 64, 2))
     rows = x.transpose(0, 1).contiguous()
     c = Codec(N_KV).calibrate(x)
@@ -34,16 +35,24 @@ def _paged(E):
     blocks = 2 * E + 2
     st = LayerState(blocks, N_KV, blocks * 2 * N_KV, bases, 128, "cuda")
     buf = torch.zeros(blocks * 2 * N_KV * (OVF_OFF + 128), dtype=torch.uint8, device="cuda")
-    freeq = torch.empty(E * 2 * N_KV, dtype=torch.int32, device="cuda")
-    sk, sv, out = torch.zeros(16 * E, N_KV, 128, dtype=torch.bfloat16, device="cuda"), torch.zeros(16 * E, N_KV, 128, dtype=torch.bfloat16, device="cuda"), []
-    for r in range(6):                               # fill blocks by halves, read them back, write what was read into the other half of the pool, and back
-        at = (r % 2) * E
-        for half in (0, 1):
-            ent = torch.tensor([[at + e, 16 * e + 8 * half, 8 * half, 8] for e in range(E)], dtype=torch.int32, device="cuda")
-            st.store(rows if r == 0 else sk, rows[:16 * E].flip(0) if r == 0 else sv, buf, ent, freeq)
-        st.decode_blocks(buf, torch.tensor([[at + e, 16 * e, 16] for e in range(E)], dtype=torch.int32, device="cuda"), sk, sv)
-        out += [sk.clone(), sv.clone()]
-    return [buf, st.top, st.err] + out, []
+    i32 = lambda rows: torch.tensor(rows, dtype=torch.int32, device="cuda")
+    # everything that a call takes is there before the first one, so that nothing but the calls' own kernels is in the stream
+    freeq, rounds = torch.empty(E * 2 * N_KV, dtype=torch.int32, device="cuda"), 6
+    ent = [[i32([[at + e, 16 * e + 8 * half, 8 * half, 8] for e in range(E)]) for half in (0, 1)] for at in (0, E)]
+    pairs, table, lens = [i32([[at + e, 16 * e, 16] for e in range(E)]) for at in (0, E)], [i32([[at + e for e in range(E)]]) for at in (0, E)], i32([16 * E])
+    back = torch.zeros(rounds, 2, 2, 16 * E, N_KV, 128, dtype=torch.bfloat16, device="cuda")
+    q, out = rows[:1].repeat(1, G, 1).contiguous(), torch.zeros(rounds, 1, G * N_KV * 128, dtype=torch.bfloat16, device="cuda")
+    first, flipped = rows[:16 * E].contiguous(), rows[:16 * E].flip(0).contiguous()
+    # fill blocks by halves, read them back, attend over them, write over them at once with K and V exchanged, read them back; then the other end of the pool with what was read
+    for r in range(rounds):
+        w = r % 2
+        k, v = (first, flipped) if r == 0 else back[r - 1, 1]
+        for again, (a, b) in enumerate(((k, v), (v, k))):
+            for half in (0, 1):
+                st.store(a, b, buf, ent[w][half], freeq)
+            st.decode_blocks(buf, pairs[w], back[r, again, 0], back[r, again, 1])
+            if not again: paged_attention(q, out[r], buf, st.raw, st.mt, table[w], lens, st.bases, st.TS, G * N_KV, N_KV)
+    return [buf, st.top, st.err, back], [out]
 
 
 def _pages():

@@ -95,7 +95,8 @@ def test_prefill_in_a_captured_graph():
     assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(cache.decompress(0), x))
 
 
-@pytest.mark.parametrize("tiles", [0, 1, 63, 65, 369, 370, 555, 740])         # from 370 on two, three, four tiles per warp of the encoder: blocks of 64, 64, 60 and 64 tiles behind it
+# one tile per warp of the encoder, from 369 tiles on two, from 553 three, from 737 four: blocks of 16, 16, 12 and 16 tiles behind it
+@pytest.mark.parametrize("tiles", [0, 1, 15, 16, 17, 63, 65, 368, 369, 370, 552, 553, 555, 564, 565, 736, 737, 740])
 @pytest.mark.parametrize("room", [1280, 100])                                # 100: the streams are too small, the copy is repeated into larger ones
 def test_streams_behind_the_encode(tiles, room):
     """A slot's offsets, escape bytes, counters and tails against a Page of the same tokens: blocks of ordinary tiles, of tiles with every group raw, and of both."""
