@@ -62,15 +62,17 @@ int gaac_encode_begin(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, in
                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, void* stream);
 
 /* gaac_encode_begin, then a wait for the stream: on return *total_pinned (page-locked host memory) holds head_start[H], which the
- * kernels wrote there themselves.  Synchronises: not for a stream that is being captured.  For a caller that wants the escape stream at its exact size (TileEncoder.encode). */
+ * kernels wrote there themselves.  Synchronises: not for a stream that is being captured.  For a caller that allocates the escape stream at its exact size and has no use
+ * for the time until then; TileEncoder.encode takes the two halves below. */
 int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                       const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                       uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,
                       int32_t* tile_off, int32_t* head_bytes, int32_t* head_start, int32_t* total_pinned, void* stream);
 
 /* The same in two halves: gaac_encode_queued returns as soon as the kernels are queued, gaac_wait_total when *total_pinned holds head_start[H] (until then it is
- * -1, and the memory must stay), which is when the encode itself is done; GAAC_E_ARG says that there are more bytes than 31 bits count, and the offsets are not valid.  What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller
- * learns the size.  counter: a device word of 8 bytes, zero before its first use; every call leaves it zero, so one serves all calls on a stream. */
+ * -1, and the memory must stay), which is when the encode itself is done; GAAC_E_ARG says that there are more bytes than 31 bits count, and the offsets are not valid.
+ * What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller learns the size.  counter: a device word of 8 bytes, zero before its
+ * first use; every call leaves it zero, so one serves all calls on a stream.  A capture would hold the first half only: the total is learnt on the host. */
 int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                        const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,

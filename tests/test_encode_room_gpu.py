@@ -71,3 +71,23 @@ def test_refused_in_a_capture():
         pg = c.encode(x, "k")
     torch.cuda.synchronize()
     assert_pages_equal(page_to_dict(pg), O.encode(x16, c.base3.cpu().numpy(), c.base4.cpu().numpy(), "k", 2))
+
+
+@pytest.mark.parametrize("H,n_kv", [(3, 3), (96, 3)])                           # prefix over the heads by one warp; by a whole CTA
+def test_sized_entry_point(H, n_kv):
+    """gaac_encode_sized, for C callers: the total, the offsets and the tiles of Codec.encode."""
+    import torch
+    from gaac_b200 import Codec, _lib
+    x16 = np.ascontiguousarray(np.resize(O.kv_like(n_kv, 333, seed=2), (H, 333, 128)))
+    x, S, nt = to_bf16_cuda(x16), 333, 21
+    c = Codec(n_kv).calibrate(x)
+    page, lib = c.encode(x, "v"), _lib.lib()
+    u8, i32 = dict(dtype=torch.uint8, device="cuda"), dict(dtype=torch.int32, device="cuda")
+    sm, codes, slots = torch.empty(H, nt * 2048, **u8), torch.empty(H, nt * 768, **u8), torch.empty(H * nt * 1280, **u8)
+    flags, sizes, off, sums, ends = torch.empty(H, nt * 16, **i32), torch.empty(H * nt, **i32), torch.empty(H, nt, **i32), torch.empty(H, **i32), torch.empty(H + 1, **i32)
+    total = torch.full((1,), -1, dtype=torch.int32, pin_memory=True)
+    _lib.check(lib.gaac_encode_sized(x.data_ptr(), H, S, S, nt * 16, c.base3.data_ptr(), c.base4.data_ptr(), None, n_kv, 1, sm.data_ptr(), codes.data_ptr(), flags.data_ptr(), slots.data_ptr(),
+                                     sizes.data_ptr(), off.data_ptr(), sums.data_ptr(), ends.data_ptr(), total.data_ptr(), _lib.stream_ptr(x.device)), "gaac_encode_sized")
+    assert int(total) == int(page.ovf_head_start[-1])                           # (it has waited: the word is read before anything else)
+    for got, ref in ((sm, page.sm), (codes, page.codes), (flags, page.flags), (off, page.tile_off), (ends, page.ovf_head_start)):
+        assert torch.equal(got, ref)
