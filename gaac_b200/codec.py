@@ -86,6 +86,8 @@ class Page:
       sm, codes        uint8 [H, S_pad*128], [H, S_pad*48]   sign+mantissa byte and 3-bit code of every element
       flags            int32 [H, S_pad]                      one tag word per token row, 2 bits per group; padding rows are 0
       ovf              uint8 [n + 8]                         the escape bytes of all heads back to back, 8 spare bytes behind
+                                                             (of an encode: usually a slice of a tensor with room for 80 bytes per tile,
+                                                             all of which torch.save of the slice writes; a clone is of its own size)
       ovf_head_start   int32 [H + 1]                         where each head's escape bytes begin in ovf
       tile_off         int32 [H, S_pad/16]                   where each tile's escape bytes begin inside its head's share
       ovf_off          int32 [H, S]                          the same per token row (only the reference's torch decoder reads it)

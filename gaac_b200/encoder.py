@@ -3,8 +3,8 @@
 Mirror of gaac/encoder.py.  `encode_tiles` writes sign/mantissa, code and tag bytes in the kernel's fragment order and leaves each
 tile's escape bytes in a bounded scratch slot (1280 B worst case); `compact` turns the per-tile byte counts into tile offsets and
 packs the slots into each head's escape stream.  `encode_into` chains the two on the device with no host round trip in
-between (the escape stream is caller-sized and the copy into it is bounded); `encode` builds a whole Page with it and reads the
-size in the middle, allocates the stream exactly and fills it.
+between (the escape stream is caller-sized and the copy into it is bounded); `encode` builds a whole Page: the copy into a stream of
+a likely size is queued behind the encode, and the host learns the exact size while it runs.
 """
 from __future__ import annotations
 import torch
@@ -13,8 +13,10 @@ from .codec import Codec, Page, D, T, CB, perm, storage_index, row_offsets
 
 SLOT = 1280
 ROOM = 80       # escape bytes per tile that encode makes room for before it knows their number, 3 % of a tile.  Tables calibrated on the data leave 50 to 60; the copy is repeated for more.
-                # us of K and V, a copy launched after a wait for the size -> one queued behind the kernels: [8, 1111, 128] 110 -> 91, [8, 65536, 128] 194 -> 175.
-
+                # us of an encode of K and one of V, a copy launched after a wait for the size -> one queued behind the kernels:
+                #   50 bytes per tile   [8, 1111, 128]  97 -> 74..95, [8, 16384, 128] 115 -> 87,  [8, 65536, 128] 169 -> 143
+                #   100 to 240           96 -> 85, 115 -> 98, 171 -> 155: with the copy that was not enough and a second allocation, since the size is known when the encode ends
+                #   noise (1280)        101 -> 85, 128 -> 118, 293 -> 304: the one form that lost, by the copy that was not enough (308 with the row offsets written twice)
 
 _COUNTERS = _lib.Kept("int64")       # the word that the encoder's CTAs count themselves in
 
@@ -164,12 +166,12 @@ class TileEncoder:
         _lib.check(L.gaac_encode_queued(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
                                         sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, p_total, word.data_ptr(), st), "gaac_encode_queued")
 
-        def copy(ovf):
-            return L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, ovf_off.data_ptr(), 8, ovf.numel(), 0, None, st)
+        def copy(ovf, rows):
+            return L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, rows, 8, ovf.numel(), 0, None, st)
         try:                                         # (the kernels write `total`: whatever happens here, it stays until they have)
             ovf_off = torch.empty(H, S, dtype=torch.int32, device=dev)
             ovf = torch.empty(items * ROOM + 8, dtype=torch.uint8, device=dev)
-            copied = copy(ovf)
+            copied = copy(ovf, ovf_off.data_ptr())
         finally:
             waited = L.gaac_wait_total(p_total, st)
         _lib.check(waited, "gaac_wait_total")
@@ -179,5 +181,5 @@ class TileEncoder:
             ovf = ovf[:n]
         else:
             ovf = torch.empty(n, dtype=torch.uint8, device=dev)
-            _lib.check(copy(ovf), "gaac_compact_copy")
+            _lib.check(copy(ovf, None), "gaac_compact_copy")                    # (the row offsets are there from the first copy)
         return Page(sm, cd, flags, ovf_off, ovf, head_start, tile_off, codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
