@@ -126,26 +126,33 @@ def row_stride(t) -> int:
 class _Buffers(dict):                                # (device index, stream) -> buffer, oldest first
     __slots__ = ("__weakref__",)
 
+    def __reduce__(self):                            # copied and pickled with its user as None: the copy asks for itself
+        return type(None), ()
+
 
 class Kept:
     """Zeroed device buffers that every call leaves zero, so that one per stream serves all objects that make such calls.  They live as long as one of the objects that have
-    asked for them; beyond MOST streams the oldest goes.  A buffer that goes is the allocator's again on the stream that it was made and used on; the caller holds what it was given until
-    its launches are queued, since another thread's call may drop it here."""
+    asked for them (which hold them as `_kept`, or None until then); beyond MOST streams the oldest goes.  A buffer that goes is the allocator's again on the stream that it was made and used on; the
+    caller holds what it was given until its launches are queued, since another thread's call may drop it here."""
     MOST = 32
 
     def __init__(self, dtype: str):
-        self._dtype, self._users, self._now, self._lock = dtype, weakref.WeakKeyDictionary(), lambda: None, threading.RLock()
+        self._dtype, self._now, self._lock = dtype, lambda: None, threading.RLock()
+
+    def join(self) -> _Buffers:
+        """What a user holds as `_kept`."""
+        with self._lock:
+            buffers = self._now()
+            if buffers is None:
+                buffers = _Buffers()
+                self._now = weakref.ref(buffers)
+        return buffers
 
     def of(self, user, dev, stream: int, n: int):
         """n or more elements for `user`'s calls on the current stream of dev, which must not be capturing (they would be zero only when the graph runs)."""
-        buffers = self._users.get(user)
+        buffers = user._kept
         if buffers is None:
-            with self._lock:
-                buffers = self._now()
-                if buffers is None:
-                    buffers = _Buffers()
-                    self._now = weakref.ref(buffers)
-                self._users[user] = buffers
+            buffers = user._kept = self.join()
         t = buffers.get((dev.index, stream))
         if t is None or t.numel() < n:
             import torch
@@ -162,6 +169,18 @@ class Kept:
 
     def __len__(self):
         return len(self._now() or ())
+
+
+ENCODE_COUNTERS = Kept("int64")       # the word that the encoder's CTAs count themselves in
+TABLE_COUNTERS = Kept("uint8")        # counters of a prompt's tables, 128 KB per kv head
+
+
+def capturing() -> bool:
+    """torch.cuda.is_current_stream_capturing without the Python function around it."""
+    global capturing
+    import torch
+    capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
+    return capturing()
 
 
 def ptr(t):

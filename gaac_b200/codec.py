@@ -124,10 +124,12 @@ class Page:
 class Codec:
     """Holds the exponent bases of n_kv kv heads and turns [H, S, 128] bf16 into a Page and back (gaac/codec.py:115-218).
     Encoding and decoding produce the reference's bytes, computed by the CUDA kernels."""
+    _kept = None                  # the encoder's counters (_lib.Kept)
 
     def __init__(self, n_kv: int, device: str = "cuda"):
         self.n_kv, self.device = n_kv, device
         self.base3 = self.base4 = None
+        self._kept = _lib.ENCODE_COUNTERS.join()
 
     def _as_table(self, t: torch.Tensor) -> torch.Tensor:
         return t.to(self.device, torch.uint8).reshape(self.n_kv, D).contiguous()

@@ -18,10 +18,12 @@ ROOM = 80       # escape bytes per tile that encode makes room for before it kno
                 #   100 to 240           96 -> 85, 115 -> 98, 171 -> 155: with the copy that was not enough and a second allocation, since the size is known when the encode ends
                 #   noise (1280)        101 -> 85, 128 -> 118, 293 -> 304: the one form that lost, by the copy that was not enough (308 with the row offsets written twice)
 
-_COUNTERS = _lib.Kept("int64")       # the word that the encoder's CTAs count themselves in
+_COUNTERS = _lib.ENCODE_COUNTERS
 
 
 class TileEncoder:
+    _kept = None
+
     def __init__(self, kind: str, device="cuda"):
         self.kind = kind
         self.device = device
@@ -143,7 +145,9 @@ class TileEncoder:
         H, S, _ = x.shape; dev = x.device
         S_pad = (S + T - 1) // T * T
         ntiles = S_pad // T
-        if H and ntiles and torch.cuda.is_current_stream_capturing():           # before anything that would become part of the graph
+        if H and ntiles and _lib.capturing():           # before anything that would become part of the graph
+            raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
+        if H and ntiles and _lib.capturing():        # before anything that would become part of the graph
             raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
         sm = torch.empty(H, S_pad * D, dtype=torch.uint8, device=dev)
         cd = torch.empty(H, S_pad * CB, dtype=torch.uint8, device=dev)

@@ -62,10 +62,12 @@ class _Store:
                           self.tail.data_ptr(), self.base3.data_ptr(), self.base4.data_ptr())
 
 
-_TABLES = _lib.Kept("uint8")         # counters of a prompt's tables, 128 KB per kv head
+_TABLES = _lib.TABLE_COUNTERS
 
 
 class CompressedKVCache:
+    _kept = None                      # the prompt tables' counters (_lib.Kept)
+
     def __init__(self, n_slots: int, n_kv: int, capacity: int, bases: dict | None = None,
                  ovf_bytes_per_tile: int = 128, device="cuda"):
         """capacity: tokens a sequence may hold (rounded up to whole tiles).  bases: {'k3','k4','v3','v4'} -> uint8 [n_kv, 128],
@@ -77,6 +79,7 @@ class CompressedKVCache:
         self.cap = _round_up_tokens(capacity)
         self.H = n_slots * n_kv
         self.per_sequence_bases = bases is None
+        if self.per_sequence_bases: self._kept = _TABLES.join()
         ovf_cap = (self.cap // T) * ovf_bytes_per_tile + _OVER_READ
         tables = {}
         for key in ("k3", "k4", "v3", "v4"):
@@ -163,7 +166,7 @@ class CompressedKVCache:
         status = self._slot_status.data_ptr() + 16 * slot if status is None else status.data_ptr()
         rows = self.k.base3.shape[0]
         own = self.per_sequence_bases and L and not copy_only                                      # tables from the prompt itself
-        if own and not torch.cuda.is_current_stream_capturing():
+        if own and not _lib.capturing():
             ws = _TABLES.of(self, dev, stream, lib.gaac_cache_tables_workspace_bytes(self.n_kv))
             _lib.check(lib.gaac_cache_prefill_own(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(),
                                                   self.cap, self.k.ovf_cap, rows, scratch.data_ptr(), scratch.numel(), status, ws.data_ptr(), ws.numel(), stream),

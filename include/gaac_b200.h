@@ -72,7 +72,8 @@ int gaac_encode_sized(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, in
 /* The same in two halves: gaac_encode_queued returns as soon as the kernels are queued, gaac_wait_total when *total_pinned holds head_start[H] (until then it is
  * -1, and the memory must stay), which is when the encode itself is done; GAAC_E_ARG says that there are more bytes than 31 bits count, and the offsets are not valid.
  * What was queued in between, such as a gaac_compact_copy into a stream of a likely size, runs on while the caller learns the size.  counter: a device word of 8 bytes, zero before its
- * first use; every call leaves it zero, so one serves all calls on a stream.  A capture would hold the first half only: the total is learnt on the host. */
+ * first use; every call leaves it zero, so one serves all calls on a stream.  Not for a stream that is being captured: the total is
+ * learnt on the host. */
 int gaac_encode_queued(const void* x_bf16, int64_t H, int64_t S, int64_t S_in, int64_t S_pad,
                        const uint8_t* base3, const uint8_t* base4, const int32_t* bidx, int n_kv, int kind,
                        uint8_t* sm, uint8_t* codes, int32_t* flags, uint8_t* slots, int32_t* tile_bytes,

@@ -85,6 +85,32 @@ def test_encode_is_refused_in_a_capture_of_a_stream_that_has_encoded():
     assert y.tolist() == [1.0] * 4
 
 
+def test_encode_is_refused_in_a_capture_whatever_the_allocators_hold():
+    """A first encode on the stream, and one whose total finds no page-locked word free: the graph goes on without either."""
+    import torch
+    from gaac_b200 import Codec
+    x = to_bf16_cuda(O.kv_like(2, 100, seed=2))
+    for first in (True, False):
+        c, side, graph, y = Codec(2).calibrate(x), torch.cuda.Stream(priority=-1), torch.cuda.CUDAGraph(), torch.zeros(4, device="cuda")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            if not first: c.encode(x, "k")
+            ref = c.encode(x, "v") if not first else None
+        words = [torch.empty(1, dtype=torch.int32, pin_memory=True) for _ in range(200)]
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            with pytest.raises(RuntimeError, match="cannot be captured"):
+                c.encode(x, "k")
+            y.add_(1)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert y.tolist() == [1.0] * 4 and len(words) == 200
+        with torch.cuda.stream(side):
+            page = c.encode(x, "v")
+        torch.cuda.synchronize()
+        assert ref is None or torch.equal(page.ovf, ref.ovf)
+
+
 def test_wait_for_a_total_takes_its_error():
     """A stream that is being captured cannot be asked: the wait says so, and no later launch does."""
     import torch

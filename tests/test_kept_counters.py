@@ -6,7 +6,7 @@ from common import to_bf16_cuda
 
 
 class User:
-    pass
+    _kept = None
 
 
 def test_buffers_of_a_stream():
@@ -31,6 +31,18 @@ def test_buffers_of_a_stream():
     assert len(kept) == 0 and kept.values() == [] and all(r() is None for r in refs)
     c = User()
     assert kept.of(c, dev, 7, 1).numel() == 1 and len(kept) == 1
+
+
+def test_copies_and_pickles_of_a_user():
+    import copy
+    import pickle
+    import torch
+    from gaac_b200 import Codec, _lib
+    kept, codec, dev = _lib.ENCODE_COUNTERS, Codec(1, "cpu"), torch.device("cpu")
+    t = kept.of(codec, dev, 7, 1)
+    for other in (copy.copy(codec), copy.deepcopy(codec), pickle.loads(pickle.dumps(codec))):
+        assert kept.of(other, dev, 7, 1) is t
+    assert pickle.loads(pickle.dumps(codec)).__dict__["_kept"] is None          # nothing of the GPU's is written
 
 
 def test_many_threads():

@@ -25,7 +25,7 @@ def _cache(monkeypatch, n_slots, own):
             return call
     monkeypatch.setattr(kvc._lib, "lib", lambda: Recording())
     monkeypatch.setattr(kvc._lib, "stream_ptr", lambda dev: 0)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(kvc._lib, "capturing", lambda: False)
     cache = object.__new__(kvc.CompressedKVCache)
     cache.n_slots, cache.n_kv, cache.cap, cache.per_sequence_bases = n_slots, 2, 64, own
     cache.S = cache.tail_len = torch.zeros(2 * n_slots, dtype=torch.int32)
