@@ -306,8 +306,8 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
 }
 
 // One group whose escape bytes are staged: H = half of the segment word with its index.  The addend's address and the group's m (byte 1 of the index) come out of the word by a dot product
-// each: by shifts and masks they took 16 instructions more per tile pair, all of them on the ALU, which is the busiest pipe.  65536 tokens 53.4 -> 52.6 us, 64 x 32768 211 -> 207, 16 x
-// 4096..65536 paged 424 -> 421.  (Not so the shifts and additions of rebuild_pairs as multiply-adds: 52.6 -> 52.6 and 53.7.)
+// each: by shifts and masks they took 16 instructions more per tile pair, all of them on the ALU, which is the busiest pipe.  In graphs: 65536 tokens 53.4 -> 52.6 us, steps of 64 x 32768
+// 211 -> 207 and of 16 x 4096..65536 paged 424 -> 421 (their public calls 440 -> 437, which is within the spread of runs).  (Not so the shifts and additions of rebuild_pairs as multiply-adds: 52.6 -> 52.6 and 53.7.)
 template <int H> __device__ __forceinline__ void decode_staged(u32 sm_lo, u32 sm_hi, u32 u, u32 word, const AttnView& w, const u32x4& bw, u32 out[4]) {
   rebuild_pairs(sm_lo, sm_hi, u, mad_byte<2 * H + 1, 1u>(word, 0u), bw, lds_u64(mad_half<H, 8u>(word, w.addends)), out);
 }

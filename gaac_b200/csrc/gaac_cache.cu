@@ -197,7 +197,8 @@ __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restric
 // Bound by its chain of loads (entry, mode table, tile, escape bytes behind the tags, then the stores): the first three are asked for before the tables are made.  384
 // blocks of 16 tiles decoded and 1500 tokens stored: 24.7 -> 24.6 us.  128 bytes of the slot's escape bytes asked for with the tile: 19.0 -> 18.1 with everything in L2,
 // but 24.4 and nothing gained from memory, where most of them are not the tile's.  9 CTAs per SM (56 registers, no spills): with 7 (72 registers) the chunk takes 20.9 us, now 20.0, and one behind 32768
-// tokens 57.7, now 54.4;  8 20.4 and 55.1;  10 (spills) 22.8 and 67.
+// tokens 57.7, now 54.4;  8 20.4 and 55.1;  10 (spills) 22.8 and 67.  All of these with the same blocks again and again, out of L2: where no earlier pass has touched them, the whole chunk (with
+// the overlapped launches 24.6 -> 20.4) gains about 1 %.
 constexpr int PDEC_WARPS = 4;
 struct PagedDecodeParams { gaac_paged st; const int* pairs; int P; uint16_t *sk, *sv; long row_stride; };
 

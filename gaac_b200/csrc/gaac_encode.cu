@@ -11,7 +11,7 @@ constexpr int ENC_WARPS = 4;          // warps per CTA
 // Tiles of a warp, which share the head's base words (and, in the decoder, the CTA's tables).  A launch that fits the SMs a few times over is as long as a warp's tiles take one after
 // the other, so a warp has one while the CTAs are fewer than twice what the SMs hold, and more only as the waves of CTAs become many.
 //  encoder (5 CTAs per SM)  us with 1 / 2 / 4 tiles: [8, 1111, 128] 3.3 / 4.2 / 6.3;  a prompt of 4001 tokens, 8 heads, K and V 8.0 / 8.2 / 9.2;  [8, 65536, 128] 47.4 / 42.3 / 41.7 (12: 46.1)
-//  decoder (8 CTAs per SM)  [8, 4001, 128] 4.9 / 5.9 / 8.4;  [8, 65536, 128] K and V 86.7 / 83.1 / 83.8 (7, every SM filled exactly once: 93.7)
+//  decoder (8 CTAs per SM)  [8, 4001, 128] 4.9 / 5.9 / 8.4;  [8, 65536, 128] K and V, two passes queued at once, 86.7 / 83.1 / 83.8 (7, every SM filled exactly once: 93.7)
 constexpr int ENC_RESIDENT = 5 * 148, ENC_MOST = 4, DEC_RESIDENT = 8 * 148, DEC_MOST = 2;
 static_assert(2 * DEC_MOST <= 32, "a lane for either end of each tile's escape bytes");
 static int tiles_per_warp(int64_t ntiles, int64_t rows, int resident, int most) {
@@ -262,7 +262,8 @@ static dim3 compact_grid(const CompactParams& p, int kinds) { return dim3((p.n_i
 
 // One warp per (head, tile): compressed tile -> bf16 rows.  Bound by latency and the warps that hide it: the escape bytes are asked for with the tile, their number taken from
 // the offset of the next tile (not of a head's last one), and the registers leave room for 8 CTAs of K, 7 of V.  [8, 65536, 128] K and V: 98.5 -> 93.7 us; with 6
-// CTAs each 102, and with the next tile's words asked for while one is rebuilt (5 CTAs) 101.  Launched overlapped, with two tiles per warp: 90.3 -> 83.1 a call of each.  No help: 32-byte
+// CTAs each 102, and with the next tile's words asked for while one is rebuilt (5 CTAs) 101.  Launched overlapped, with two tiles per warp: 90.3 -> 83.1 for two
+// passes over K and V queued at once (the public calls, over three Pages in turn: 90.6 -> 88.7).  No help: 32-byte
 // stores (85.6), evict-first stores (83.5) or loads (85.4), CTAs of two warps (92.6).
 template <int KIND_V>
 __global__ void __launch_bounds__(ENC_WARPS * 32, KIND_V ? 7 : 8) decode_page_kernel(
