@@ -148,8 +148,7 @@ class Codec:
 
     def encode(self, x: torch.Tensor, kind: str) -> Page:
         """x: [H, S, D] bf16 -> Page."""
-        from .encoder import TileEncoder
-        return TileEncoder(kind, self.device).encode(self, x.to(self.device))
+        return encoder.TileEncoder(kind, self.device).encode(self, x.to(self.device))
 
     @staticmethod
     def decode(page: Page) -> torch.Tensor:
@@ -182,3 +181,6 @@ def row_offsets(flags: torch.Tensor, S: int) -> torch.Tensor:
         return (v * 0x01010101 >> 24) & 0xFF
     rb = popc(even) + 4 * popc(odd)
     return (torch.cumsum(rb, 1) - rb).to(torch.int32).contiguous()
+
+
+from . import encoder  # noqa: E402  (it needs the names above; an import inside Codec.encode is 0.6 us of every call)

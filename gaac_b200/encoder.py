@@ -145,8 +145,6 @@ class TileEncoder:
         H, S, _ = x.shape; dev = x.device
         S_pad = (S + T - 1) // T * T
         ntiles = S_pad // T
-        if H and ntiles and _lib.capturing():           # before anything that would become part of the graph
-            raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
         if H and ntiles and _lib.capturing():        # before anything that would become part of the graph
             raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
         sm = torch.empty(H, S_pad * D, dtype=torch.uint8, device=dev)
