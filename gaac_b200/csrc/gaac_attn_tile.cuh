@@ -224,7 +224,7 @@ struct AttnView { u32 addends, segs, bases; };
 __device__ __forceinline__ void fill_attn_tables(uint8_t* at, int t) {
   const u32x2 x = pair_addends((u32)t), s = segment_entry((u32)t);
   reinterpret_cast<uint2*>(at + 16)[t] = make_uint2(x.x, x.y);
-  reinterpret_cast<uint2*>(at + ADDEND_BYTES)[t] = make_uint2(s.x, s.y);
+  reinterpret_cast<uint2*>(at + ADDEND_BYTES)[t] = make_uint2((s.x & 0xFFFFu) | s.y << 16, s.x >> 16);           // (a permute takes the lower half of a selector)
   if (t == 0) reinterpret_cast<uint2*>(at + 8)[0] = make_uint2(0u, 0u);
 }
 __device__ __forceinline__ AttnView attn_view(u32 tables, u32 bases) { return AttnView{tables + 16 - 256 * 8, tables + ADDEND_BYTES, bases}; }
@@ -251,26 +251,32 @@ __device__ __forceinline__ void scan_step16(u32& v, int d) {
 // Make the segment area of a tile pair.  Lane l has row l & 15 of K (l < 16) or of V.  live: the lane's side is compressed; fl, esc: shared-memory addresses of its
 // tag words and of its escape bytes, of which `avail` are staged.  Returned: bit 0 / 1: those of K / V are all staged (and the staged sides have no more than `room` raw
 // groups, which have their entries, 8 bytes each, behind the segment words; the other groups of raw_items need none).
-// Bound by its chain of latencies, hence a scan over 16 rows and not over 64 segments, and sizes from the tag words while the segment table answers.  The scan counts the
-// raw groups along with the escape bytes, so that a row knows its entries' places and takes its items without asking the others: with a vote per item and a place
-// for every item, promoted groups behind raw ones included, 65536 tokens took 56.9 us, now 54.9 (64 x 32768 220 -> 211, paged 16 x 4096..65536 443 -> 428), and at 32768
-// tokens tile pairs of 44 raw and 250 promoted groups ran out of places: 61.1 us, now 43.4.
-// Before that, against a look-up per group and raw groups as table entries found by the decoder: 59.0 -> 56.2, 247 -> 233, 516 -> 493.
+// Bound by its instructions, 282 of 1052 per tile pair before, about 235 now, and by its chain of latencies; hence a scan over 16 rows and not over 64 segments, and sizes from the tag words
+// while the segment table answers.  The scan counts the raw groups along with the escape bytes, so that a row knows its entries' places and takes its items without asking the
+// others.  The raw groups, 4 of 512, took half of it (147 instructions: 1.8 trips of a loop in which both kinds of item lay on either side of a branch; a timing-only build without that loop 51.3 -> 46.6 us).
+// Now each kind has a loop of its own, from the last item to the first, where the mask of what lies below an item also takes it off, and one vote asks whether everything is staged and
+// has room, which it nearly always has.  65536 tokens 51.4 -> 49.8 us, 64 x 32768 205.3 -> 199.3, paged 16 x 4096..65536 422 -> 406 (steps in graphs).
 __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avail, const AttnView& w, u32 area, u32 room, int lane) {
   const u32 fl = live ? lds_u32(fl_at + 4u * (lane & 15)) : 0u;
-  const u32 size = (u32)row_esc_bytes(fl), own_raws = (u32)popc(fl & 0xAAAAAAAAu);
+  const u32 ones = (u32)popc(fl & 0x55555555u), own_raws = (u32)popc(fl & 0xAAAAAAAAu), own = mad_k<65540u>(own_raws, ones);            // escape bytes | raw groups << 16
   const u32x2 e[4] = {lds_u64(mad_byte<0, 8u>(fl, w.segs)), lds_u64(mad_byte<1, 8u>(fl, w.segs)), lds_u64(mad_byte<2, 8u>(fl, w.segs)), lds_u64(mad_byte<3, 8u>(fl, w.segs))};
-  u32 sum = mad_k<65536u>(own_raws, size);                                   // escape bytes | raw groups << 16
+  u32 sum = own;
   scan_step16(sum, 1); scan_step16(sum, 2); scan_step16(sum, 4); scan_step16(sum, 8);
-  const u32 end = sum & 0xFFFFu, k_raws = __shfl_sync(FULLM, sum, 15) >> 16;
-  const u32 over = __ballot_sync(FULLM, live && (int)end > avail);
-  int staged = ((over & 0xFFFFu) ? 0 : 1) | ((over >> 16) ? 0 : 2);
-  const u32 mine = area + SEG_V * (lane >> 4) + 32u * (lane & 15);
-  // places behind the row's entries: those of K first, if its side needs any
-  const u32 past = (sum >> 16) + (lane >= 16 && (staged & 1) ? k_raws : 0u);
-  bool fast = (staged >> (lane >> 4)) & 1;
-  if (__any_sync(FULLM, fast && past > room)) { staged = 0; fast = false; }
-  u32 pos = end - size;
+  const u32 end = sum & 0xFFFFu, k_raws = __shfl_sync(FULLM, sum, 15) >> 16, mine = area + 32u * lane;
+  u32 past = (sum >> 16) + (lane >= 16 ? k_raws : 0u), pos = (sum - own) & 0xFFFFu;           // places behind the row's entries, those of K first;  the row's first escape byte
+  int staged = 3;
+  bool fast = true;
+  if (__any_sync(FULLM, (live && (int)end > avail) || past > room)) {
+    const u32 over = __ballot_sync(FULLM, live && (int)end > avail);
+    staged = ((over & 0xFFFFu) ? 0 : 1) | ((over >> 16) ? 0 : 2);
+    if (lane >= 16 && !(staged & 1)) past -= k_raws;         // (K's side needs no entries)
+    fast = (staged >> (lane >> 4)) & 1;
+    if (__any_sync(FULLM, fast && past > room)) { staged = 0; fast = false; }
+    if (!fast) {                                     // {tag byte | position << 16}
+#pragma unroll
+      for (int q = 0; q < 4; q++) { sts_u64(mine + 8u * q, ((fl >> (8 * q)) & 0xFFu) | pos << 16, 0u); pos += e[q].x >> 16; }
+    }
+  }
   if (fast) {
     const u32 at = live ? esc + pos : area;
     u32 a = at, four[4];
@@ -278,28 +284,33 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
     for (int q = 0; q < 4; q++) {
       const u32 lo = lds_u32(a & ~3u), hi = lds_u32((a & ~3u) + 4u);
       four[q] = __funnelshift_r(lo, hi, 8u * a);                             // (the shift counts modulo 32)
-      a += e[q].y;
+      a += e[q].x >> 16;
     }
 #pragma unroll
     for (int q = 0; q < 4; q += 2)
-      sts_u128(mine + 8u * q, prmt(four[q], SEG_CONST, e[q].x), prmt(four[q], SEG_CONST, e[q].x >> 16), prmt(four[q + 1], SEG_CONST, e[q + 1].x), prmt(four[q + 1], SEG_CONST, e[q + 1].x >> 16));
-    u32 entry = area + SEG_PATCH + 8u * (past - own_raws);
-    for (u32 items = raw_items(fl); items; items &= items - 1u) {
-      const u32 bit = (u32)__ffs((int)items) - 1u, pl = at + (u32)esc_prefix(fl, (int)bit);       // bit: lower tag bit of the group, 2 * group
-      u32 index;
-      if ((fl >> bit) & 2u) {                          // the upper bits of the exponents, less what the decoder will add to them
-        index = (entry - w.addends) >> 3;
-        const u32 m = index >> 8;
-        const u32x4 bw = lds_u128(w.bases + (lane >= 16 ? PAIR_BASES_V : 16u * (bit >> 3)) + 8u * bit);
-        const u32x2 x = pair_raw_addends(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * (pl & 3u));
-        sts_u64(entry, x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w);
-        entry += 8u;
-      } else index = 256u + lds_u8(pl);
+      sts_u128(mine + 8u * q, prmt(four[q], SEG_CONST, e[q].x), prmt(four[q], SEG_CONST, e[q].y), prmt(four[q + 1], SEG_CONST, e[q + 1].x), prmt(four[q + 1], SEG_CONST, e[q + 1].y));
+    // the raw groups, and the promoted ones behind a raw one of their segment, from the last to the first:  bit: lower tag bit of the group, 2 * group
+    u32 raws = (fl >> 1) & fl & 0x55555555u;
+    u32 behind = raw_items(fl) & ~raws;
+    u32 index = ((area + SEG_PATCH - w.addends) >> 3) + past;
+    const u32 side = w.bases + (lane >= 16 ? PAIR_BASES_V : 0), skew = lane >= 16 ? 0u : 16u;
+    while (raws) {
+      u32 bit; asm("bfind.u32 %0, %1;" : "=r"(bit) : "r"(raws));
+      const u32 below = ~(0xFFFFFFFFu << bit);
+      raws &= below; index--;
+      const u32 pl = at + (u32)popc(fl & below & 0x55555555u) + 4u * (u32)popc(fl & below & 0xAAAAAAAAu);
+      const u32x4 bw = lds_u128(side + 8u * bit + skew * (bit >> 3));
+      const u32x2 x = pair_payload(__funnelshift_r(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * pl), lds_u8(pl + 4u));
+      const u32 m = index >> 8;
+      sts_u64(w.addends + 8u * index, x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w);          // the upper bits of the exponents, less what the decoder will add to them
       sts_u16(mine + bit, index);
     }
-  } else {                                           // {tag byte | position << 16}
-#pragma unroll
-    for (int q = 0; q < 4; q++) { sts_u64(mine + 8u * q, ((fl >> (8 * q)) & 0xFFu) | pos << 16, 0u); pos += e[q].y; }
+    while (behind) {
+      u32 bit; asm("bfind.u32 %0, %1;" : "=r"(bit) : "r"(behind));
+      const u32 below = ~(0xFFFFFFFFu << bit);
+      behind &= below;
+      sts_u16(mine + bit, 256u + lds_u8(at + (u32)popc(fl & below & 0x55555555u) + 4u * (u32)popc(fl & below & 0xAAAAAAAAu)));
+    }
   }
   __syncwarp();
   return staged;

@@ -99,13 +99,16 @@ GAAC_HD u32x2 pair_addends(u32 b) {
   const u32 lo = spread_bit4(b & 15u), hi = spread_bit4(b >> 4);
   return u32x2{prmt(lo, hi, 0x6420), prmt(lo, hi, 0x7531)};
 }
+// The upper five bits of the exponents of a raw group's even and odd elements, from its payload of 8 x 5 bits: bits 0..31, and from bit 32 on (more bits may follow).  Two fields
+// side by side at bits 0 and 16 of a word, for the first four and for the last, and one byte permute each for the even and the odd ones.
+GAAC_HD u32x2 pair_payload(u32 lo, u32 byte4) {
+  const u32 z = funnel_r(lo, byte4, 20), a = bits_of(lo, mad_k<64u>(lo, 0u), 0x3FFu), b = bits_of(z, mad_k<64u>(z, 0u), 0x3FFu);
+  return u32x2{mad_k<8u>(prmt(a, b, 0x6420), 0u) & 0xF8F8F8F8u, prmt(a >> 2, b >> 2, 0x6420) & 0xF8F8F8F8u};
+}
 // The same for a raw group, whose payload (8 x 5 bits) lies in (w1:w0) from bit sh (0, 8, 16, 24): the upper five bits of the exponents.  No base must contribute:
 // the caller takes off what rebuild_pairs adds.
 GAAC_HD u32x2 pair_raw_addends(u32 w0, u32 w1, u32 sh) {
-  const u32 lo = funnel_r(w0, w1, (int)sh), hi = sh == 24u ? w1 : funnel_r(w0, w1, (int)sh + 8);           // payload bits 0..31 and 8..39
-  const u32 ev = bits_of(bits_of(lo << 3, lo << 1, 0xFFu), bits_of(hi << 5, lo >> 1, 0xFF000000u), 0xFFFFu);
-  const u32 od = bits_of(bits_of(lo >> 2, lo >> 4, 0xFFu), bits_of(hi, lo >> 6, 0xFF000000u), 0xFFFFu);
-  return u32x2{ev & 0xF8F8F8F8u, od & 0xF8F8F8F8u};
+  return pair_payload(funnel_r(w0, w1, (int)sh), w1 >> sh);
 }
 // out[i] = elements i and i + 4.  u: code_bytes; m: what the bases' second half counts (1 for a promoted group); x: the addends.
 GAAC_HD void rebuild_pairs(u32 sm_lo, u32 sm_hi, u32 u, u32 m, const u32x4& bw, const u32x2& x, u32 out[4]) {
