@@ -76,16 +76,17 @@ GAAC_HD void rebuild_group(u32 sm_lo, u32 sm_hi, u32 z, u32 m1, const u32x4& bw,
 // words, of the even and of the odd elements, and a word pairs elements that lie four apart: bytes 0 and 2 of a word of exponents land on the exponent fields
 // of a bf16 pair when it is shifted up by 7, bytes 1 and 3 when it is shifted down by 1, whatever else the shift brings along is covered by the sign and
 // mantissa bits, and those come from one byte permute.  
-// The codes of a group, two to a byte (B = byte offset of the group in the lane's code string)
+// The codes of a group, two to a byte, at bits 0..5; the bits above are anything (B = byte offset of the group in the lane's code string).  A step is a shift and a select: with the fields
+// masked and moved by multiply-adds a group took one operation of the ALU more (12 of 1010 instructions per tile pair; 65536 tokens 49.8 -> 49.3 us, paged 16 x 4096..65536 406 -> 404).
 template <int B> GAAC_HD u32 code_bytes(const u32* cd) {
   constexpr int i = B & 3;
   u32 t;                                                                 // codes 0..3 at bits 0..11, 4..7 at bits 16..27
-  if (i == 1) { const u32 z = cd[B >> 2] >> 8; t = mad_k<15u>(z & 0xFFF000u, z); }
+  if (i == 1) t = bits_of(cd[B >> 2] >> 8, cd[B >> 2] >> 4, 0xFFFu);
   else {
     const u32 z = i ? prmt(cd[B >> 2], cd[(B >> 2) + (i ? 1 : 0)], i == 2 ? 0x5432 : 0x6543) : cd[B >> 2];      // the upper byte is the next group's
-    t = mad_k<16u>(z & 0xFFF000u, z & 0xFFFu);
+    t = bits_of(z, mad_k<16u>(z, 0u), 0xFFFu);
   }
-  return mad_k<3u>(t & 0x0FC00FC0u, t);
+  return bits_of(t, mad_k<4u>(t, 0u), 0x003F003Fu);
 }
 // Words of the bases {3-bit window: even elements, odd elements; what the 4-bit window is above them: even, odd} of group t of a side's 16 (K: 4 * (lane & 3)
 // + group, V: 2 * (lane >> 2) + group)
