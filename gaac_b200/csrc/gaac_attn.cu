@@ -43,9 +43,11 @@ constexpr int STAGE_BYTES = 2 * SIDE_BYTES;
 static_assert(SIDE_BYTES == TPS * PSLOT, "both layouts use stages of the same size");
 // CTA tables: addend and segment table, K / V base words; per stage the mbarrier that counts arriving bytes and how many tiles of it the warps have left so far; per
 // tile of a stage {address of its escape bytes of K, how many are staged, the same of V}, its metadata, and the word (stage + 1) << 4 | bits 2, 3: the K / V tile is
-// raw, by which a warp knows the use of the slot: a parity can be two phases off for one that runs ahead of a slow one.  Then the warps' segment areas.
+// raw, by which a warp knows the use of the slot: a parity can be two phases off for one that runs ahead of a slow one.  Then the metadata of the tiles that come next into the stage
+// (and of the one behind them), which the warp that has the stage's last tile asks for and leaves there for the one that is last to leave the stage: asked for by each of the four in case that it
+// is the one, they cost 10 instructions per tile pair more (64 x 32768 198.8 -> 196.0 us, paged 16 x 4096..65536 404 -> 398, 65536 tokens 49.4 -> 49.2).  Then the warps' segment areas.
 constexpr int TB_BASES = ADDEND_BYTES + SEGTAB_BYTES, TB_FULL = TB_BASES + PAIR_BASES_BYTES, TB_LEFT = TB_FULL + 8 * NSTG, TB_ESC = TB_LEFT + 4 * NSTG, TB_META = TB_ESC + 16 * TPS * NSTG,
-              TB_USE = TB_META + 8 * TPS * NSTG, TB_AREA = TB_USE + 4 * TPS * NSTG, TB_RING = TB_AREA + ATT_WARPS * AREA_BYTES;
+              TB_USE = TB_META + 8 * TPS * NSTG, TB_NEXT = TB_USE + 4 * TPS * NSTG, TB_AREA = TB_NEXT + 8 * (TPS + 1) * NSTG, TB_RING = TB_AREA + ATT_WARPS * AREA_BYTES;
 constexpr int ATT_SMEM = TB_RING + NSTG * STAGE_BYTES + 16;          // (an escape segment is read as whole words)
 static_assert(TB_BASES % 16 == 0 && TB_ESC % 16 == 0 && TB_AREA % 16 == 0 && TB_RING % 16 == 0 && STAGE_BYTES % 16 == 0 && SIDE_BYTES % 16 == 0 && SB_ESC % 16 == 0 && SB_FL % 16 == 0 && PSLOT % 16 == 0 && TB_FULL % 8 == 0 && SIDE_ESC % 16 == 0,
               "bulk copies need 16-byte aligned shared-memory destinations and sizes");
@@ -871,12 +873,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (!rawk) k_tile<DUMP>(sc, ks, win, area, W, lane, Q, dump_k + (long)tile * T * D, nvalid);
     else raw_scores<DUMP>(sc, p.raw + (long)raw_tile(m.x) * (T * D), nvalid, lane, Q, dump_k + (long)tile * T * D);
     nx = __shfl_sync(FULLM, nx, 0);
-    if (st + NSTG < nstages) ahead = stage_meta(st + NSTG);                  // in case that this warp fills the stage again
+    const bool asks = ti == TPS - 1 && st + NSTG < nstages;
+    if (asks) ahead = stage_meta(st + NSTG);                                 // for the warp that will fill the stage again
     PFrag<NSET> P;
     if (nvalid == T) softmax_step<NSET, true>(A, sc, p.scale_log2, nvalid, lane, P);
     else softmax_step<NSET, false>(A, sc, p.scale_log2, nvalid, lane, P);
     if (!rawv) v_tile<DUMP, NSET>(A, vs, win, area, W, lane, P, dump_v + (long)tile * T * D, nvalid);
     else raw_accum<DUMP, NSET>(A, p.raw + (long)raw_tile(m.y) * (T * D), nvalid, lane, P, dump_v + (long)tile * T * D);
+    if (asks && lane <= TPS) reinterpret_cast<int2*>(smem + TB_NEXT)[slot * (TPS + 1) + lane] = make_int2(ahead.mk, ahead.mv);
     __syncwarp();                                    // every lane is done with the tile and with the area
     if (st + NSTG < nstages) {
       int left = 0;
@@ -885,6 +889,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
       if ((left & (TPS - 1)) == TPS - 1) {
         __syncwarp();
         if (!PAGED) fill_payload(st + NSTG);
+        ahead = TileMeta{-1, -1};
+        if (lane <= TPS) { const int2 e = reinterpret_cast<const int2*>(smem + TB_NEXT)[slot * (TPS + 1) + lane]; ahead = TileMeta{e.x, e.y}; }
         fill_rest(st + NSTG, ahead, PAGED ? head_esc : HeadEsc{__shfl_sync(FULLM, s_esc[0], 0), __shfl_sync(FULLM, s_esc[1], 0), __shfl_sync(FULLM, s_esc[2], 0), __shfl_sync(FULLM, s_esc[3], 0), __shfl_sync(FULLM, s_esc[4], 0), __shfl_sync(FULLM, s_esc[5], 0)});
       }
     }

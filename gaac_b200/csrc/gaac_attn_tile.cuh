@@ -211,8 +211,8 @@ __device__ __forceinline__ void pv_words(WarpAcc<2>& A, int mt, const u32 (&w0)[
 constexpr int ESC_WIN = 256;
 constexpr int PSLOT = SLOT_OVF_OFF + ESC_WIN + 16;          // staged bytes of a paged tile slot, at most
 // What a planned tile pair has in shared memory (its segment area): segment words of K and of V, [row][quarter of a row], 8 bytes per segment, then the entries of
-// its raw groups.  PATCH_MAX: raw groups of a tile pair (of 512) that have room; a pair with more takes the plain decoder.
-constexpr int PATCH_MAX = 64, SEG_K = 0, SEG_V = 64 * 8, SEG_PATCH = 2 * SEG_V;
+// its raw groups.  PATCH_MAX: raw groups of a tile pair (of 512) that have room (what shared memory leaves); a pair with more takes the plain decoder.
+constexpr int PATCH_MAX = 62, SEG_K = 0, SEG_V = 64 * 8, SEG_PATCH = 2 * SEG_V;
 constexpr int AREA_BYTES = SEG_PATCH + 8 * PATCH_MAX;
 // Addend table: entry NO_ESC (zero) and entries 256 + byte, 8 bytes each; segment table: 256 entries of 8 bytes
 constexpr int ADDEND_BYTES = 8 + 257 * 8, SEGTAB_BYTES = 256 * 8;
