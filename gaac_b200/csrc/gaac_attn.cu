@@ -846,11 +846,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // ---- main loop.  The warp's first tile is tile `warp` of the range; every further one is taken from the CTA's counter at the top of the
   // iteration, one tile ahead of its use, so fast and slow warps finish within about one tile of each other.  The warp that is the
   // last to leave a stage fills it again with the tiles NSTG stages on.
-  const u32 area = smem_s + TB_AREA + warp * AREA_BYTES;
+  const u32 area = smem_s + TB_AREA + warp * AREA_BYTES, next_at = (u32)__cvta_generic_to_shared(&s_next);
   int it = warp;
   while (it < n) {
-    int nx = 0;
-    if (lane == 0) nx = atomicAdd(&s_next, 1);
+    int nx = lane_inc<false>(next_at, lane);
     const int st = it / TPS, ti = it % TPS, slot = st % NSTG, tile = tlo + it, nth = it % (TPS * NSTG);
     u32 flags;
     if (!__all_sync(FULLM, mbar_wait_use(smem_s + TB_FULL + 8 * slot, (u32)(st / NSTG) & 1u, smem_s + TB_USE + 4 * nth, (u32)st + 1u, flags))) {     // the whole warp gives up together
@@ -883,9 +882,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (asks && lane <= TPS) reinterpret_cast<int2*>(smem + TB_NEXT)[slot * (TPS + 1) + lane] = make_int2(ahead.mk, ahead.mv);
     __syncwarp();                                    // every lane is done with the tile and with the area
     if (st + NSTG < nstages) {
-      int left = 0;
-      if (lane == 0) asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(left) : "r"(smem_s + TB_LEFT + 4 * slot) : "memory");
-      left = __shfl_sync(FULLM, left, 0);
+      const int left = __shfl_sync(FULLM, lane_inc<true>(smem_s + TB_LEFT + 4 * slot, lane), 0);
       if ((left & (TPS - 1)) == TPS - 1) {
         __syncwarp();
         if (!PAGED) fill_payload(st + NSTG);
