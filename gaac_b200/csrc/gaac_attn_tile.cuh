@@ -253,6 +253,8 @@ struct SideView { const uint8_t *sm, *cd, *glob; };
 // its escape bytes are read from global memory.
 // Once per segment, because a group's share of it (tag bits, position, byte, table address) cost 10 of the 37 instructions of its rebuild.
 
+// prmt with a selector that is not known: the intrinsic masks it first.
+__device__ __forceinline__ u32 permute(u32 a, u32 b, u32 sel) { u32 d; asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel)); return d; }
 // One step of an inclusive scan over each half of a warp (scan_step over all of it).
 __device__ __forceinline__ void scan_step16(u32& v, int d) {
   asm volatile("{\n .reg .pred p;\n .reg .u32 t;\n shfl.sync.up.b32 t|p, %0, %1, 0x1000, 0xffffffff;\n @p add.u32 %0, %0, t;\n}\n" : "+r"(v) : "r"(d));
@@ -297,7 +299,7 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
     }
 #pragma unroll
     for (int q = 0; q < 4; q += 2)
-      sts_u128(mine + 8u * q, prmt(four[q], SEG_CONST, e[q].x), prmt(four[q], SEG_CONST, e[q].y), prmt(four[q + 1], SEG_CONST, e[q + 1].x), prmt(four[q + 1], SEG_CONST, e[q + 1].y));
+      sts_u128(mine + 8u * q, permute(four[q], SEG_CONST, e[q].x), permute(four[q], SEG_CONST, e[q].y), permute(four[q + 1], SEG_CONST, e[q + 1].x), permute(four[q + 1], SEG_CONST, e[q + 1].y));
     // the raw groups, and the promoted ones behind a raw one of their segment, from the last to the first:  bit: lower tag bit of the group, 2 * group
     u32 raws = (fl >> 1) & fl & 0x55555555u;
     u32 behind = raw_items(fl) & ~raws;

@@ -135,8 +135,8 @@ GAAC_HD u32x2 segment_entry(u32 t) {
 }
 // Groups of a row with tag word fl that the selectors leave out: the raw ones and the promoted ones behind a raw one of their segment, at their lower tag bits.
 GAAC_HD u32 raw_items(u32 fl) {
-  const u32 r = (fl >> 1) & 0x55555555u;
-  return (r | (mad_k<4u>(r & 0x15151515u, 0u) | mad_k<16u>(r & 0x05050505u, 0u) | mad_k<64u>(r & 0x01010101u, 0u))) & fl;
+  const u32 r = (fl >> 1) & fl & 0x55555555u;
+  return (r | (0x80808080u - r)) & fl & 0x55555555u;                     // bits 0..6 of a byte's 0x80 - r: those of -r, ones above the lowest one of r
 }
 
 }  // namespace gaac
