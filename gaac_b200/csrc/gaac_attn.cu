@@ -1104,13 +1104,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   __syncthreads();
 
   const AttnView W = attn_view(smem_s, smem_s + T256_BASES + hf * PAIR_BASES_BYTES);
-  const u32 area = smem_s + T256_SEG + warp * SEG256_BYTES;
+  const u32 area = smem_s + T256_SEG + warp * SEG256_BYTES, next_at = (u32)__cvta_generic_to_shared(&s_next);
   int stg = 0, par = 0;
   u32 phase = 0;
   const int avail = min(p.ovf_slot, (int)slot_bytes - SLOT_OVF_OFF);
   while (it < n) {
-    int t1 = 0;
-    if (hf == 0 && lane == 0) t1 = atomicAdd(&s_next, 1);
+    int t1 = hf == 0 ? lane_inc<false>(next_at, lane) : 0;
     const bool ok = __all_sync(FULLM, mbar_wait(ring_s + stg * STAGE256_BYTES, (phase >> stg) & 1u));
     phase ^= 1u << stg;
     const int so = ring + stg * STAGE256_BYTES + 16;
