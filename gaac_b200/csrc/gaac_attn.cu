@@ -603,6 +603,17 @@ template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B,
 
 static_assert(FLAT_SCRATCH <= ATT_WARPS * AREA_BYTES, "planned in the segment areas");
 
+// Ranges of a row of a grid, where its length is only known here: the caller goes by a bound on the rows' lengths, the width of a block table or a capacity, and its split count (ns, the most there
+// may be) may be far too large for the rows that there are.  A row that fits the warps of one CTA (`at_once` tiles) is not split;  beyond, ranges go down to four tiles until there are 16 of them (24 at
+// head_dim 256, whose CTAs work on eight tiles at a time), then down to a tile per warp.  CTAs that get none leave before they load anything.  So the callers' rules may fill one wave: in a table of 2048
+// tokens 4 x 4 rows of 53 took 9.8 us in nine ranges each, 7.0 by shares of units and take 6.5 now;  in one of 8192 at head_dim 256 a row of 2000 17.5 in 128 ranges, now 10.1.
+__device__ __forceinline__ void fewer_ranges(int tiles, int at_once, int& ns, int& chunk) {
+  if (tiles <= at_once) { ns = 1; chunk = tiles; return; }
+  const int least = max(4, min(at_once, at_once == 16 ? (tiles + 15) >> 4 : tiles / 24));
+  if (chunk >= least) return;
+  ns = (tiles + least - 1) / least;
+  chunk = (tiles + ns - 1) / ns;                     // (as sum_exact takes it)
+}
 // How the rows are shared out.  GRID: (row, kv head) x splits;  SHARED: a balanced launch;  FLAT_LINE: above.  Instantiations of their own: the shares cost the others
 // registers that the main loop has none of, 1.5 % at 64K tokens.
 enum { GRID, SHARED, FLAT_LINE };
@@ -712,7 +723,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // These values are the same in every thread, but they were loaded from memory: passing them through a shuffle tells the
   // compiler so, and the address arithmetic built on them stays in uniform registers.
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
-  const int ntiles = (S + 15) >> 4, chunk = MODE == GRID && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
+  const int ntiles = (S + 15) >> 4;
+  int chunk = MODE == GRID && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
+  if (MODE == GRID && p.nsplit > 1) {
+    if (PAGED || p.seq_len) { fewer_ranges(ntiles, ATT_WARPS, ns0, chunk); if (split0 >= ns0) return; }
+    if (tid == 0) s_ns = ns0;
+  }
   const int tlo = FLAT ? min(__shfl_sync(FULLM, s_flat.range[0], 0), ntiles) : min(split0 * chunk, ntiles);
   // (the last piece of a pair has what there is to the end, should a head be longer than the first one)
   const int n = FLAT ? (__shfl_sync(FULLM, s_split + 1 - s_ns, 0) == 0 ? ntiles - tlo : min(__shfl_sync(FULLM, s_flat.range[1], 0), ntiles - tlo)) : min(chunk, ntiles - tlo);
@@ -818,7 +834,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     const int brow = PAGED || p.n_base_rows == p.n_kv ? kvh : ch < p.n_base_rows ? ch : ch % p.n_base_rows;
     if (warp == ATT_WARPS - 2 && lane < 16) fill_pair_bases<false>(smem + TB_BASES, (PAGED ? p.b3k : p.K.base3) + brow * D, (PAGED ? p.b4k : p.K.base4) + brow * D, lane);
     if (warp == ATT_WARPS - 1 && lane < 16) fill_pair_bases<true>(smem + TB_BASES, (PAGED ? p.b3v : p.V.base3) + brow * D, (PAGED ? p.b4v : p.V.base4) + brow * D, lane);
-    if (SHARE && tid == 0) { s_split = split0; s_ns = ns0; }
+    if (SHARE && tid == 0) s_split = split0;
+    if (SHARE && tid == 0) s_ns = ns0;
     if (FLAT && tid == 0) s_tail = TL;
     if (tid == 0) s_next = ATT_WARPS;                        // tiles 0 .. W-1 of the range go to warps 0 .. W-1, the rest is handed out on demand
   }
@@ -893,7 +910,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
     it = nx;
   }
-  const int split = SHARE || FLAT ? s_split : split0, NS = SHARE || FLAT ? s_ns : p.nsplit;
+  const int split = SHARE || FLAT ? s_split : split0, NS = MODE == GRID && p.nsplit == 1 ? 1 : s_ns;
   if (FLAT) { bh = __shfl_sync(FULLM, s_flat.pair, 0); b = bh / p.n_kv; kvh = bh % p.n_kv; TL = __shfl_sync(FULLM, s_tail, 0); }
   // ---- slot layout: the raw BF16 tail belongs to the last split's last warp
   if (!PAGED && TL > 0 && split == NS - 1 && warp == ATT_WARPS - 1) {
@@ -958,7 +975,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     for (int i = 0; i < NSET; i++) {
       const int g = (tid >> 7) + 4 * i;
       if (g >= G) continue;
-      if (NS > 1) merge_splits<32>(p, SHARE ? ((long)blockIdx.x * p.units + blockIdx.y - split) * G + g : (qh0 + g) * NS, SHARE ? G : 1, NS, d, M[i], Lc[i], Ac[i]);
+      if (NS > 1) merge_splits<32>(p, SHARE ? ((long)blockIdx.x * p.units + blockIdx.y - split) * G + g : (qh0 + g) * p.nsplit, SHARE ? G : 1, NS, d, M[i], Lc[i], Ac[i]);
       deliver(g, M[i], Lc[i], Ac[i]);
     }
   }
@@ -1021,7 +1038,7 @@ static_assert(FLAT_SCRATCH <= ATT_WARPS * SEG256_BYTES, "planned in the segment 
 template <int NSET, bool FLAT>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int s_next, s_last;
+  __shared__ int s_next, s_last, s_ns;
   __shared__ FlatWalk s_flat;
   __shared__ int s_rows[FLAT ? 64 : 1];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -1065,7 +1082,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   }
   int b = bh / p.n_kv, kvh = bh % p.n_kv;
   const int S = __shfl_sync(FULLM, FLAT ? s_flat.tokens : p.seq_len[b], 0);
-  const int ntiles = (S + 15) >> 4, chunk = (ntiles + NS - 1) / NS;
+  const int ntiles = (S + 15) >> 4;
+  int chunk = (ntiles + NS - 1) / NS;
+  if (!FLAT) {
+    if (p.nsplit > 1) fewer_ranges(ntiles, ATT_WARPS / 2, NS, chunk);
+    if (split >= NS) return;
+    if (tid == 0) s_ns = NS;
+  }
   const int tlo = min(FLAT ? __shfl_sync(FULLM, s_flat.range[0], 0) : split * chunk, ntiles), n = min(FLAT ? __shfl_sync(FULLM, s_flat.range[1], 0) : chunk, ntiles - tlo);
   int* const ctl_pair = reinterpret_cast<int*>(smem + T256_CTL + pair * (2 * CTL_BYTES));
   const int4* meta_s = reinterpret_cast<const int4*>(smem + T256_META);        // per tile: mode-table entries of {K, V} of half 0, of half 1
@@ -1152,7 +1175,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (lane == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];\nmbarrier.inval.shared::cta.b64 [%1];\n" ::"r"(ring_s), "r"(ring_s + STAGE256_BYTES) : "memory");
     bh = __shfl_sync(FULLM, s_flat.pair, 0); split = __shfl_sync(FULLM, s_flat.split, 0); NS = __shfl_sync(FULLM, s_flat.ns, 0);
     b = bh / p.n_kv; kvh = bh % p.n_kv;
-  }
+  } else NS = s_ns;
   // ---- merge the warps of the CTA, half by half: one partial per virtual head (2 * query head + half)
   if (__syncthreads_or(sum_warp(A))) sum_exact<true, true>(p, smem + T256_RING, bh, split, NS, FLAT ? s_flat.range : nullptr);
   else stage_warp(A, smem + T256_RING, G, warp, lane);
@@ -1176,7 +1199,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (vg >= 2 * G) continue;
     if (NS == 1) deliver(row0 + vg, Lc[i], Ac[i]);
     else {
-      const long pidx = FLAT ? (long)(blockIdx.x + bh) * 2 * G + vg : (row0 + vg) * NS + split;
+      const long pidx = FLAT ? (long)(blockIdx.x + bh) * 2 * G + vg : (row0 + vg) * p.nsplit + split;
       if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
       p.pa[pidx * D + d] = Ac[i];
     }
@@ -1192,7 +1215,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
 #pragma unroll 1
     for (int vg = tid >> 7; vg < 2 * G; vg += ATT_THREADS / 128) {
       float Mv, Lv, Av;
-      merge_splits<32>(p, (row0 + vg) * NS, 1, NS, d, Mv, Lv, Av);
+      merge_splits<32>(p, (row0 + vg) * p.nsplit, 1, NS, d, Mv, Lv, Av);
       deliver(row0 + vg, Lv, Av);
     }
   }

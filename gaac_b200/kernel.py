@@ -64,7 +64,7 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     rows = max(1, B * n_kv)
     ntiles = max(1, (S + 15) // 16)
     most = max(1, ntiles // (ATT_WARPS * min_tiles_per_warp))
-    if ragged and B > 1:
+    if ragged and B > 1 and not _short_ranges(rows, ntiles, sm_count):
         # CTAs are handed out longest row first, so the end of the launch is filled by the small ones and what remains is a
         # trade between the per-CTA fixed cost (grows with the split count) and the last chunks of the longest row (shrink with
         # it): the measured optimum follows sqrt(1.8 x longest row's tiles / rows).  Near it, a count whose CTAs fill whole waves
@@ -97,6 +97,14 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     return best
 
 
+def _short_ranges(rows: int, ntiles: int, sm_count: int = SM_COUNT_B200) -> bool:
+    """One wave of CTAs, every row split alike, leaves none of them more than about a tile per warp: then it hardly matters which row is the longest, and a plain grid, which plans nothing,
+    is the faster launch.  us, shares of units -> this, rows of hi / 8 to hi tokens (B x kv heads):  paged 2 x 8 of 300 8.1 -> 7.0;  8 x 8 of 160 8.5 -> 6.1;  16 x 4 of 500 9.1 -> 8.7;  8 x 4 of
+    1100 9.4 -> 8.9;  slots 8 x 8 of 500 10.0 -> 9.0;  32 x 1 of 500 9.2 -> 7.9.  Longer ranges are as fast or faster by shares (3 x 8 of 2000, 21 tiles: 10.3 and 10.2; 16 x 1 of 4000, 28 tiles:
+    10.2 and 10.9)."""
+    return ntiles <= 17 * (sm_count // rows) + 1 and rows <= sm_count
+
+
 @functools.lru_cache(maxsize=4096)
 def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> int:
     """Ranges per kv head that the rows of a ragged batch share by their lengths (S: tokens of the longest), or 0 where every row is split alike
@@ -110,6 +118,8 @@ def choose_units(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> in
     takes about 8.7 us + 0.22 us per tile here.  One wave -> this:  slots 7, 8, 16000 each: 119.1 -> 108.6;  13, 4, 12000 each: 92.4 -> 86.1;  7, 8,
     8000..16000: 92.4 -> 92.4;  but up to 3 us for CTAs that find nothing to do where few rows are long (13, 4, 2400 and one of 16000: 27.0 -> 30.3)."""
     units, two = sm_count // n_kv, 2 * sm_count // n_kv
+    if B > 1 and _short_ranges(B * n_kv, -(-S // 16), sm_count):
+        return 0
     if not 2 <= B <= 32 or units < (2 if S <= 16384 else 4) * B:
         return 0
     tiles = -(-S // 16)
@@ -151,11 +161,27 @@ def choose_flat256(B: int, n_kv: int, S: int, most: int = 0, sm_count: int = SM_
     """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.1 -> 24.8;  20 x 8, up to 3K 95 -> 73;  32 x 2, up
     to 4K 56 -> 40;  6 x 2, up to 60K 124 -> 93;  8 x 4, 100-700 22.0 -> 13.2;  2 x 8 of 1000 30 -> 13;  9 x 4, up to 1500 23.8 -> 16.6;  30 x 4, up to 2K 55 -> 48;  32 x 4, up to 1000 30.7 -> 31.4,
     in a table of 8192 43 -> 31;  32 x 8 the same 53 -> 40, 65 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.3 -> 47.6;  so are a few very short ones: 4 x 4 of 50-300 in a
-    table of 8192 9.4 -> 11.0;  one sequence has nothing to gain: 1 x 4 of 8K 17.9 -> 18.4."""
+    table of 8192 9.4 -> 11.0;  one sequence has nothing to gain: 1 x 4 of 8K 17.9 -> 18.4.  More rows than SMs, 32 x 8: up to 500 22.1 -> 23.4, up to 740 35.5 -> 33.6, up to 1100 53.0 -> 44.4."""
     rows, tiles = B * n_kv, -(-S // 16)
-    if B <= 1 or not _flat_line(rows, max(S, most)):
+    if B <= 1 or not _flat_line(rows, max(S, most)) or _splits256(rows, tiles, sm_count):
         return 0
-    return sm_count if tiles >= (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 160) else 0
+    return sm_count if tiles >= (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 64) else 0
+
+
+def _splits256(rows: int, tiles: int, sm_count: int = SM_COUNT_B200) -> int:
+    """Splits of one wave in which every row is split alike, where that leaves a CTA at most three tiles per pair of its warps, or 0."""
+    wave = sm_count // rows if rows <= sm_count else 1
+    ns = min(wave, max(1, min(8, tiles // 3), tiles // 4))
+    return ns if wave > 1 and tiles <= 24 * ns else 0
+
+
+@functools.lru_cache(maxsize=4096)
+def choose_nsplit256(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> int:
+    """Splits per (row, kv head) at head_dim 256, whose CTAs work on eight tiles at a time.  S may be a bound far above the rows' lengths: the kernel takes fewer ranges for a row of few
+    tiles.  One wave of short ranges comes first; us, the counts made for 16 warps, or a flat launch, -> this, rows of hi / 8 to hi tokens (B x kv heads): 2 x 1 of 740 17.3 -> 8.9;  8 x 4 of 500 16.0 -> 10.8;
+    5 x 8 of 740 20.9 -> 13.5;  2 x 4 of 4000 15.8 (flat) -> 13.7;  8 x 8 of 1100 20.8 (flat) -> 19.2;  1 x 1 of 300 10.2 -> 8.2.  Where ranges are longer a flat launch is as fast or faster (2 x 8 of
+    4000, 28 tiles: 17.8 and 18;  8 x 4 of 2000, 31 tiles: 16.5 and 17)."""
+    return _splits256(B * n_kv, -(-S // 16), sm_count) or choose_nsplit_sm100(B, n_kv, S, ragged=True)
 
 
 def _flat_splits(B: int, n_kv: int, ctas: int) -> int:
