@@ -106,6 +106,24 @@ def lib():
     return _lib
 
 
+_load, _host = lib, None
+
+
+def host():
+    """The module whose functions are the library's hot ones and take tensors as they are (csrc/gaac_host.cpp).  Like the library it has no substitute."""
+    global _host
+    if _host is None:
+        import torch                                 # (its libraries are what the module is linked to)
+        handle = _load()._handle
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(f"gaac_b200/_host.so is missing or does not fit this torch ({torch.__version__}): build it with `python -m gaac_b200.build --force`") from e
+        module.bind(handle)
+        _host = module
+    return _host
+
+
 def check(status: int, what: str):
     if status != 0:
         raise RuntimeError(f"{what}: {lib().gaac_status_string(status).decode()} (status {status})")

@@ -155,7 +155,8 @@ class Codec:
         """Bit-exact reconstruction: Page -> [H, S, D] bf16."""
         sm = _cuda(page.sm, "page.sm")
         H, S = page.H, page.S
-        out = torch.empty(H, S, D, dtype=torch.bfloat16, device=sm.device)
+        host = _lib.host()
+        out = host.empty(sm, 2, H, S, D)
         if H == 0 or S == 0:
             return out
         S_pad = page.sm.shape[1] // D
@@ -163,10 +164,8 @@ class Codec:
         bidx = None
         if nb != page.n_kv:                          # one base row per head (per-sequence calibration)
             bidx = (torch.arange(H, device=sm.device, dtype=torch.int32) % nb).contiguous()
-        _lib.check(_lib.lib().gaac_decode_page(
-            page.sm.data_ptr(), page.codes.data_ptr(), page.flags.data_ptr(), page.tile_off.data_ptr(), _lib.row_stride(page.tile_off),
-            page.ovf.data_ptr(), page.ovf_head_start.data_ptr(), page.base3.data_ptr(), page.base4.data_ptr(), _lib.ptr(bidx),
-            page.n_kv, 0 if page.kind == "k" else 1, H, S, S_pad, out.data_ptr(), _lib.stream_ptr(sm.device)), "gaac_decode_page")
+        _lib.check(host.gaac_decode_page(page.sm, page.codes, page.flags, page.tile_off, _lib.row_stride(page.tile_off), page.ovf, page.ovf_head_start, page.base3, page.base4, bidx,
+                                         page.n_kv, 0 if page.kind == "k" else 1, H, S, S_pad, out, _lib.stream_ptr(sm.device)), "gaac_decode_page")
         return out
 
 

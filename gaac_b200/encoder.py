@@ -147,26 +147,25 @@ class TileEncoder:
         ntiles = S_pad // T
         if H and ntiles and _lib.capturing():        # before anything that would become part of the graph
             raise RuntimeError("Codec.encode learns a size on the host: it cannot be captured in a CUDA graph (TileEncoder.encode_into can)")
-        sm = torch.empty(H, S_pad * D, dtype=torch.uint8, device=dev)
-        cd = torch.empty(H, S_pad * CB, dtype=torch.uint8, device=dev)
-        flags = torch.empty(H, S_pad, dtype=torch.int32, device=dev)          # every row of every tile is written, padded rows as 0
+        host = _lib.host()
+        sm, cd = host.empty(x, 0, H, S_pad * D), host.empty(x, 0, H, S_pad * CB)
+        flags = host.empty(x, 1, H, S_pad)           # every row of every tile is written, padded rows as 0
         if H == 0 or ntiles == 0:
             return Page(sm, cd, flags, torch.empty(H, S, dtype=torch.int32, device=dev), torch.zeros(8, dtype=torch.uint8, device=dev),
                         torch.zeros(H + 1, dtype=torch.int32, device=dev), torch.zeros(H, ntiles, dtype=torch.int32, device=dev), codec.base3, codec.base4, H, S, codec.n_kv, self.kind)
-        tile_off = torch.empty(H, ntiles, dtype=torch.int32, device=dev)
-        head_start = torch.empty(H + 1, dtype=torch.int32, device=dev)
+        tile_off, head_start = host.empty(x, 1, H, ntiles), host.empty(x, 1, H + 1)
         x = x.contiguous()
         items = H * ntiles
         # escape slots | tile sizes | head sizes: of this call alone, since another one on the same encoder (a second stream, a second thread while this one waits) may
         # run before the copy has read them
-        slots = torch.empty(items * SLOT + 4 * (items + H), dtype=torch.uint8, device=dev)
+        slots = host.empty(x, 0, items * SLOT + 4 * (items + H))
         total = torch.empty(1, dtype=torch.int32, pin_memory=True)
         L = _lib.lib(); st = _lib.stream_ptr(dev)
         p_flags, p_slots, p_off, p_hs, p_total = flags.data_ptr(), slots.data_ptr(), tile_off.data_ptr(), head_start.data_ptr(), total.data_ptr()
         p_work = p_slots + items * SLOT
         word = _COUNTERS.of(codec if isinstance(codec, Codec) else self, dev, st, 1)
-        _lib.check(L.gaac_encode_queued(x.data_ptr(), H, S, S, S_pad, codec.base3.data_ptr(), codec.base4.data_ptr(), None, codec.n_kv, 0 if self.kind == "k" else 1,
-                                        sm.data_ptr(), cd.data_ptr(), p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, p_total, word.data_ptr(), st), "gaac_encode_queued")
+        _lib.check(host.gaac_encode_queued(x, H, S, S, S_pad, codec.base3, codec.base4, None, codec.n_kv, 0 if self.kind == "k" else 1,
+                                           sm, cd, p_flags, p_slots, p_work, p_off, p_work + 4 * items, p_hs, p_total, word, st), "gaac_encode_queued")
 
         def copy(ovf, rows):
             return L.gaac_compact_copy(p_slots, p_work, H, ntiles, p_hs, ovf.data_ptr(), p_off, ntiles, p_flags, S, S_pad, rows, 8, ovf.numel(), 0, None, st)

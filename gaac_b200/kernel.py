@@ -217,18 +217,19 @@ class _Ext:
         dev = q.device
         B = slot.size(0)
         has_tail = kt.numel() > 0
-        K = _side(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None)
-        V = _side(smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None)
         stream = _lib.stream_ptr(dev)
         ws = workspace(dev, B, n_q, _flat_splits(B, n_kv, flat) if flat else -(-units // B) if units else nsplit, stream)
-        L = _lib.lib()
-        if flat or units:
-            out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
-            name = "gaac_decode_attn_flat" if flat else "gaac_decode_attn_balanced"
-            _lib.check(getattr(L, name)(K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), flat or units,
-                                        TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel(),
-                                        out.data_ptr(), _lib.ptr(out_f32), stream), name)
+        if exchange is None and partial is None:
+            H = _lib.host()
+            out = H.empty(q, 3, B * n_q, D) if isinstance(q, torch.Tensor) else torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
+            name = "gaac_decode_attn_flat" if flat else "gaac_decode_attn_balanced" if units else "gaac_decode_attn"
+            _lib.check(getattr(H, name)((smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None), (smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None),
+                                        q.data_ptr(), slot, B, n_q, n_kv, SL, S_pad, float(scale), flat or units or int(nsplit), TL if has_tail else None, int(TCAP) if has_tail else 0,
+                                        b3k.size(0), ws, ws.numel(), out, out_f32, stream), name)
             return out
+        L = _lib.lib()
+        K = _side(smk, ck, fk, tok, ovk, ohsk, b3k, b4k, kt if has_tail else None)
+        V = _side(smv, cv, fv, tov, ovv, ohsv, b3v, b4v, vt if has_tail else None)
         common = (K, V, q.data_ptr(), slot.data_ptr(), B, n_q, n_kv, SL.data_ptr(), S_pad, float(scale), int(nsplit),
                   TL.data_ptr() if has_tail else None, int(TCAP) if has_tail else 0, b3k.size(0), ws.data_ptr(), ws.numel())
         if exchange is not None and fused:
@@ -238,12 +239,8 @@ class _Ext:
         if exchange is not None:
             _lib.check(L.gaac_decode_attn_push(*common, exchange, stream), "gaac_decode_attn_push")
             return None
-        if partial is not None:
-            _lib.check(L.gaac_decode_attn_partial(*common, partial.data_ptr(), stream), "gaac_decode_attn_partial")
-            return partial
-        out = torch.empty(B * n_q, D, dtype=q.dtype, device=dev)
-        _lib.check(L.gaac_decode_attn(*common, out.data_ptr(), _lib.ptr(out_f32), stream), "gaac_decode_attn")
-        return out
+        _lib.check(L.gaac_decode_attn_partial(*common, partial.data_ptr(), stream), "gaac_decode_attn_partial")
+        return partial
 
 
 _mod = None
@@ -262,8 +259,8 @@ def attention(q, kp, vp, scale=None, nsplit=None, out_f32=None, out=None):
     q: [B, n_q, D] bf16 (one query token per sequence) -> [B, n_q, D] bf16.  (gaac/kernel.py:345-359)
     out (contiguous bf16 tensor of B*n_q*D elements) receives the result instead of a new tensor; out_f32 (fp32, same shape)
     additionally receives the result before its rounding to BF16.
-    nsplit=None picks the B200 heuristic; an explicit nsplit is honoured as given.  The two gaac_side descriptors are built
-    once and kept on the Page objects, so a decode loop pays one library call per layer."""
+    nsplit=None picks the B200 heuristic; an explicit nsplit is honoured as given.  us a call over 500 tokens, through ctypes and descriptors kept on the
+    Pages -> the native module, which reads the Pages: 10.7 -> 7.3, the kernel's own time."""
     B, n_q, Dq = q.shape
     if Dq != 128:
         raise RuntimeError("head_dim must be 128")
@@ -275,7 +272,7 @@ def attention(q, kp, vp, scale=None, nsplit=None, out_f32=None, out=None):
         raise RuntimeError("GQA group size must be 1..8")
     if nsplit is None: nsplit = choose_nsplit_sm100(B, n_kv, kp.S)
     if out is None:
-        out = torch.empty(B, n_q, Dq, dtype=q.dtype, device=q.device)
+        out = _lib.host().empty(q, 3, B, n_q, Dq)
     elif out.is_contiguous() and out.dtype == q.dtype and out.numel() == B * n_q * Dq:
         out = out.view(B, n_q, Dq)
     else:
@@ -285,7 +282,7 @@ def attention(q, kp, vp, scale=None, nsplit=None, out_f32=None, out=None):
 
 
 def _page_side(pg) -> _lib.Side:
-    """The gaac_side descriptor of a Page, built once and kept on the Page object (rebuilt when its escape stream was replaced)."""
+    """The gaac_side descriptor of a Page for ctypes calls (an exchange, a Page without tokens), built once and kept on the Page object (rebuilt when its escape stream was replaced)."""
     sd = getattr(pg, "_attn_side", None)
     if pg.S == 0:                                  # a Page without tokens (a rank past the end of a short context): nothing is read through
         if sd is None:                             # these pointers, but the library wants them non-null, so they point at a small zero buffer
@@ -307,6 +304,10 @@ def _pages_call(q, kp, vp, B, n_q, n_kv, scale, nsplit, out=None, out_f32=None, 
     if not q.is_contiguous(): q = q.contiguous()
     stream = _lib.stream_ptr(dev)
     ws = workspace(dev, B, n_q, nsplit, stream)
+    if exchange is None and kp.S > 0:
+        _lib.check(_lib.host().gaac_decode_attn_pages(kp, vp, q, B, n_q, n_kv, kp.S, max(16, kp.sm.shape[1] // 128), float(scale if scale is not None else 128 ** -0.5), int(nsplit),
+                                                      kp.base3.size(0), ws, ws.numel(), out, out_f32, part, None, 1 if fused else 0, stream), "gaac_decode_attn_pages")
+        return
     _lib.check(_lib.lib().gaac_decode_attn_pages(_page_side(kp), _page_side(vp), q.data_ptr(), B, n_q, n_kv, kp.S, max(16, kp.sm.shape[1] // 128),
                                                  float(scale if scale is not None else 128 ** -0.5), int(nsplit), kp.base3.size(0),
                                                  ws.data_ptr(), ws.numel(), _lib.ptr(out), _lib.ptr(out_f32), _lib.ptr(part), exchange,

@@ -34,12 +34,9 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
         nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)        # with units: what the workspace must have room for
         flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv, bt_stride * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)
-    st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
-                    bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), n_kv, TS, TS - 2880)
+    st = (buf, raw, mt, None, None, None, *bases, n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, n_q, nsplit, stream)
-    lib = _lib.lib()
     name = "gaac_paged_decode_attn_flat" if flat else "gaac_paged_decode_attn_balanced" if units else "gaac_paged_decode_attn"
-    _lib.check(getattr(lib, name)(st, bt.data_ptr(), bt_stride, seq_lens.data_ptr(), q.data_ptr(), B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit),
-                                  ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), name)
+    _lib.check(getattr(_lib.host(), name)(st, bt, bt_stride, seq_lens, q, B, n_q, 1.0 / (D ** 0.5), flat or units or int(nsplit), ws, ws.numel(), out, out_f32, stream), name)
     return out

@@ -28,12 +28,9 @@ def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv,
         nsplit = choose_nsplit256(B, n_kv, bt.shape[1] * 16)
         flat = choose_flat256(B, n_kv, bt.shape[1] * 16, bt_stride * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)                                          # what the workspace must have room for
-    st = _lib.Paged(buf.data_ptr(), raw.data_ptr(), mt.data_ptr(), None, None, None,
-                    bases[0].data_ptr(), bases[1].data_ptr(), bases[2].data_ptr(), bases[3].data_ptr(), 2 * n_kv, TS, TS - 2880)
+    st = (buf, raw, mt, None, None, None, *bases, 2 * n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, 2 * n_q, nsplit, stream)
-    lib = _lib.lib()
     name = "gaac_paged_decode_attn256_flat" if flat else "gaac_paged_decode_attn256"
-    _lib.check(getattr(lib, name)(st, bt.data_ptr(), bt_stride, seq_lens.data_ptr(), q.data_ptr(), B, n_q, float(scale) if scale is not None else 256 ** -0.5,
-                                  flat or int(nsplit), ws.data_ptr(), ws.numel(), out.data_ptr(), _lib.ptr(out_f32), stream), name)
+    _lib.check(getattr(_lib.host(), name)(st, bt, bt_stride, seq_lens, q, B, n_q, float(scale) if scale is not None else 256 ** -0.5, flat or int(nsplit), ws, ws.numel(), out, out_f32, stream), name)
     return out

@@ -48,6 +48,9 @@ class LayerState:
         return _lib.Paged(buf.data_ptr(), self.raw.data_ptr(), self.mt.data_ptr(), self.stack.data_ptr(), self.top.data_ptr(), self.err.data_ptr(),
                           self.b3k.data_ptr(), self.b4k.data_ptr(), self.b3v.data_ptr(), self.b4v.data_ptr(), self.n_kv, self.TS, self.ovf_slot)
 
+    def _fields(self, buf: torch.Tensor) -> tuple:
+        return (buf, self.raw, self.mt, self.stack, self.top, self.err, self.b3k, self.b4k, self.b3v, self.b4v, self.n_kv, self.TS, self.ovf_slot)
+
     def store(self, key: torch.Tensor, value: torch.Tensor, buf: torch.Tensor, ent: torch.Tensor, freeq: torch.Tensor):
         """key/value: [num_tokens, n_kv, D] bf16 (or int16 views of them); buf: uint8 flat block buffer; ent: int32 [E,4] =
         (blk, tok0, off0, n); freeq: int32 [E*2*n_kv] scratch.  (gaac/vllm/store.py:204-213)"""
@@ -55,8 +58,7 @@ class LayerState:
         if E == 0: return
         assert key.stride(-1) == 1 and value.stride(-1) == 1
         assert (key.shape[1] == 1 or key.stride(1) == D) and (value.shape[1] == 1 or value.stride(1) == D)
-        _lib.check(_lib.lib().gaac_paged_store(self.c_state(buf), key.data_ptr(), value.data_ptr(), _lib.row_stride(key), _lib.row_stride(value),
-                                               ent.data_ptr(), E, freeq.data_ptr(), _lib.stream_ptr(buf.device)), "gaac_paged_store")
+        _lib.check(_lib.host().gaac_paged_store(self._fields(buf), key, value, _lib.row_stride(key), _lib.row_stride(value), ent, E, freeq, _lib.stream_ptr(buf.device)), "gaac_paged_store")
 
     def decode_blocks(self, buf: torch.Tensor, pairs: torch.Tensor, sk: torch.Tensor, sv: torch.Tensor):
         """pairs: int32 [P,3] (block, first scratch row, valid rows); sk/sv: flat scratch K/V [rows, n_kv, D] bf16 (written).
@@ -64,8 +66,7 @@ class LayerState:
         P = pairs.shape[0]
         if P == 0: return
         assert _lib.row_stride(sk) == self.n_kv * D and _lib.row_stride(sv) == self.n_kv * D
-        _lib.check(_lib.lib().gaac_paged_decode_blocks(self.c_state(buf), pairs.data_ptr(), P, sk.data_ptr(), sv.data_ptr(), _lib.row_stride(sk),
-                                                       _lib.stream_ptr(buf.device)), "gaac_paged_decode_blocks")
+        _lib.check(_lib.host().gaac_paged_decode_blocks(self._fields(buf), pairs, P, sk, sv, _lib.row_stride(sk), _lib.stream_ptr(buf.device)), "gaac_paged_decode_blocks")
 
     def release_blocks(self, blocks: torch.Tensor):
         """blocks: int32 [F] block ids whose content is dead (freed without prefix caching).  (gaac/vllm/store.py:223-227)"""
