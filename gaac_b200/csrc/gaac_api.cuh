@@ -1,6 +1,7 @@
 // Helpers shared by the C-ABI entry points.
 #pragma once
 #include <cuda_runtime.h>
+#include <utility>
 #include <stdint.h>
 #include "../../include/gaac_b200.h"
 
@@ -16,13 +17,17 @@ inline int g_launch_overlap = 1;      // see gaac_set_launch_overlap
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::); }
 template <class... Params, class... Args>
-int launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
+int launch_overlapped_with(int shared_bytes, void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = stream;
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = shared_bytes; cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
   cfg.attrs = at; cfg.numAttrs = 1;
   if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
   return launch_status();
+}
+template <class... Params, class... Args>
+int launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
+  return launch_overlapped_with(0, kernel, grid, threads, stream, std::forward<Args>(args)...);
 }
 }  // namespace gaac

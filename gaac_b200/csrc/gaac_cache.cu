@@ -1,4 +1,5 @@
 // Cache maintenance kernels (sm_100a): slot-layout append, paged-layout store / release / block decode.
+#include <algorithm>
 #include "gaac_api.cuh"
 #include "gaac_warp.cuh"
 
@@ -203,10 +204,10 @@ constexpr int PDEC_WARPS = 4;
 struct PagedDecodeParams { gaac_paged st; const int* pairs; int P; uint16_t *sk, *sv; long row_stride; };
 
 template <int KIND_V>
-__device__ __forceinline__ void decode_blocks_cta(DecodeScratch* scratch, DecodeTables& tables, const PagedDecodeParams& p, int t) {
+__device__ __forceinline__ void decode_blocks_cta(uint8_t* scratch, DecodeTables& tables, const PagedDecodeParams& p, int t) {
   const gaac_paged& st = p.st;
   const int kvh = t >> 1, NT = 2 * st.n_kv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = blockIdx.x * PDEC_WARPS + warp;
-  DecodeScratch& ws = scratch[warp];
+  WarpScratch& ws = *reinterpret_cast<WarpScratch*>(scratch + warp * decode_scratch_bytes(min(st.ovf_slot, TILE_MAX_ESC)));
   griddep_wait();
   griddep_launch();
   // the tile travels while the tables are made
@@ -219,7 +220,7 @@ __device__ __forceinline__ void decode_blocks_cta(DecodeScratch* scratch, Decode
     m = st.mt[pt];
     if (m >= 0) load_tile_words<KIND_V>(tw, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, base + SLOT_OVF_OFF, 0, lane);
   }
-  const WarpView w = fill_decode_tables<KIND_V>(tables, (KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D);
+  const u32 w = fill_decode_tables<KIND_V>(tables, (KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D);
   __syncthreads();
   if (e >= p.P) return;
   uint16_t* dst = (KIND_V ? p.sv : p.sk) + (long)row0 * p.row_stride + (long)kvh * D;
@@ -231,11 +232,11 @@ __device__ __forceinline__ void decode_blocks_cta(DecodeScratch* scratch, Decode
     }
     return;
   }
-  decode_tile_warp<KIND_V>(ws, tw, w, lane);
+  decode_tile_warp<KIND_V>(ws, tw, w, lane, min(st.ovf_slot, TILE_MAX_ESC));
   unstage_rows(ws, dst, p.row_stride, nvalid, lane);
 }
 __global__ void __launch_bounds__(PDEC_WARPS * 32, 9) paged_decode_blocks_kernel(const __grid_constant__ PagedDecodeParams p) {
-  __shared__ __align__(16) DecodeScratch scratch[PDEC_WARPS];
+  extern __shared__ __align__(16) uint8_t scratch[];
   __shared__ __align__(16) DecodeTables tables;
   const int t = blockIdx.y;
   if (t & 1) decode_blocks_cta<1>(scratch, tables, p, t); else decode_blocks_cta<0>(scratch, tables, p, t);
@@ -306,7 +307,8 @@ extern "C" int gaac_paged_decode_blocks(const gaac_paged* st, const int32_t* pai
   if (!aligned16(sk) || !aligned16(sv) || row_stride % 8) return GAAC_E_ALIGN;
   if (P == 0) return GAAC_OK;
   PagedDecodeParams p{*st, pairs, P, (uint16_t*)sk, (uint16_t*)sv, row_stride};
-  return launch_overlapped(paged_decode_blocks_kernel, dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)), PDEC_WARPS * 32, (cudaStream_t)stream, p);
+  return launch_overlapped_with(PDEC_WARPS * decode_scratch_bytes(std::min(st->ovf_slot, TILE_MAX_ESC)), paged_decode_blocks_kernel, dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)),
+                                PDEC_WARPS * 32, (cudaStream_t)stream, p);
 }
 
 extern "C" const char* gaac_status_string(int status) {

@@ -270,14 +270,14 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, KIND_V ? 7 : 8) decode_page_ke
     const uint8_t* __restrict__ sm, const uint8_t* __restrict__ codes, const int* __restrict__ flags, const int* __restrict__ tile_off,
     long tile_off_stride, const uint8_t* __restrict__ ovf, const int* __restrict__ head_start, const uint8_t* __restrict__ base3,
     const uint8_t* __restrict__ base4, const int* __restrict__ bidx, int n_kv, long S, long S_pad, uint16_t* __restrict__ out, int ntiles, int per_warp) {
-  __shared__ __align__(16) DecodeScratch scratch[ENC_WARPS];
+  __shared__ __align__(16) uint8_t scratch[ENC_WARPS * decode_scratch_bytes(TILE_MAX_ESC)];
   __shared__ __align__(16) DecodeTables tables;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long h = blockIdx.y;
-  DecodeScratch& ws = scratch[warp];
+  WarpScratch& ws = *reinterpret_cast<WarpScratch*>(scratch + warp * decode_scratch_bytes(TILE_MAX_ESC));
   griddep_wait();
   griddep_launch();
-  const int brow = bidx ? bidx[h] : (int)(h % n_kv);
+  const int brow = bidx ? bidx[h] : h < n_kv ? (int)h : (int)((unsigned)h % (unsigned)n_kv);
   const uint8_t* esc_head = ovf + (long)head_start[h];
   const int tile0 = blockIdx.x * (ENC_WARPS * per_warp) + warp;
   const int mine = tile0 + (lane >> 1) * ENC_WARPS + (lane & 1);                           // lanes 2i, 2i + 1: where the warp's i-th tile's escape bytes begin and end
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(ENC_WARPS * 32, KIND_V ? 7 : 8) decode_page_ke
     load_tile_words<KIND_V>(tw, sm + trow * D, codes + trow * CB, reinterpret_cast<const uint8_t*>(flags + trow), esc_head + from, tile + 1 < ntiles ? to - from : 0, lane);
   };
   if (tile0 < ntiles) ask(0);
-  const WarpView w = fill_decode_tables<KIND_V>(tables, base3 + (long)brow * D, base4 + (long)brow * D);
+  const u32 w = fill_decode_tables<KIND_V>(tables, base3 + (long)brow * D, base4 + (long)brow * D);
   __syncthreads();
 #pragma unroll 1
   for (int i = 0; i < per_warp; i++) {

@@ -46,10 +46,7 @@ __device__ __forceinline__ void tile_positions(u32 k0, u32 k1, u32 v0, u32 v1, u
 }
 
 // ---- group decoder
-constexpr int LUTX_BYTES = 2048, BASES_V = 256, BASES_BYTES = 512;      // escape-byte table; base words of K, of V behind them
-
-// Shared-memory addresses of the escape-byte table and of the base words (K, then V).
-struct WarpView { u32 lutx, bases; };
+constexpr int BASES_V = 256, BASES_BYTES = 512;      // base words of K, of V behind them
 
 __device__ __forceinline__ u32 lds_u8(u32 a) { u32 v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
 __device__ __forceinline__ u32 lds_u32(u32 a) { u32 v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
@@ -58,18 +55,18 @@ __device__ __forceinline__ u32x4 lds_u128(u32 a) { u32x4 v; asm volatile("ld.sha
 __device__ __forceinline__ void sts_u16(u32 a, u32 v) { asm volatile("{\n .reg .u16 t;\n cvt.u16.u32 t, %1;\n st.shared.u16 [%0], t;\n}" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts_u64(u32 a, u32 x, u32 y) { asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }
 __device__ __forceinline__ void sts_u128(u32 a, u32 x, u32 y, u32 z, u32 w) { asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory"); }
-// Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, pos = position of
-// the group's escape bytes, advanced past them.
-__device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& pos, const uint8_t* glob, const WarpView& w, const u32x4& bw, u32 out[4]) {
-  const u32 m1 = tg & 1u;                             // promoted (tags are 0, 1 or 3)
-  u32x2 x = lds_u64(w.lutx + 8u * (m1 ? (u32)glob[pos] : 0u));
-  if (tg & 2u) {
-    const uint8_t* p = glob + pos;
-    const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-    x = raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
-    pos += 4;
+// Rebuild one group (two sign/mantissa words) into four bf16x2 words; z as group_codes leaves it, tg = tag in the low bits, esc = where its escape bytes are (a shared-memory address,
+// which may be read in any case), advanced past them.  raws: some lane's group is raw (the same in all lanes).
+__device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& esc, bool raws, const u32x4& bw, u32 out[4]) {
+  const u32 m1 = tg & 1u, eb = lds_u8(esc) * m1;      // promoted (tags are 0, 1 or 3)
+  u32x2 x{spread_bit4(eb & 15u), spread_bit4(eb >> 4)};
+  if (raws) {
+    if (tg & 2u) {
+      x = raw_addends(lds_u32(esc & ~3u), lds_u32((esc & ~3u) + 4u), 8u * (esc & 3u), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
+      esc += 4u;
+    }
   }
-  pos += m1;
+  esc += m1;
   rebuild_group(sm_lo, sm_hi, z, m1, bw, x, out);
 }
 

@@ -130,11 +130,7 @@ GAAC_HD u32 spread_hi5(u32 u) {
 }
 // sign/mantissa bytes (4) + exponent bytes (4) -> bf16 pairs (elements 0,1) and (2,3)             gaac/kernel.py:34-36
 GAAC_HD void bf16x4(u32 sm4, u32 e4, u32& p01, u32& p23) {
-#if defined(__CUDA_ARCH__)
-  const u32 eh = __umulhi(e4, 0x80000000u);                          // e4 >> 1
-#else
   const u32 eh = e4 >> 1;
-#endif
   const u32 el = mad_k<128u>(e4, 0u);                                // e4 << 7
   const u32 h4 = bits_of(sm4, eh, 0x80808080u), l4 = bits_of(el, sm4, 0x80808080u);
   p01 = prmt(l4, h4, 0x5140); p23 = prmt(l4, h4, 0x7362);

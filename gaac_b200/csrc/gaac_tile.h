@@ -45,7 +45,7 @@ GAAC_HD int tag_esc_bytes(u32 tag) { return (int)(tag & 1u) + 2 * (int)(tag & 2u
 // ---- decode ----------------------------------------------------------------------------------------------------
 struct u32x4 { u32 x, y, z, w; };
 struct u32x2 { u32 x, y; };
-// Escape-byte table: lutx[b] = { spread_bit4(b & 15), spread_bit4(b >> 4) }, what escape byte b adds to the exponents of its group (2 KiB)
+// Escape-byte table, for the check of the decoder on the host (the device works an entry out): lutx[b] = { spread_bit4(b & 15), spread_bit4(b >> 4) }, what escape byte b adds to the exponents of its group
 GAAC_HD void fill_lutx(u32x2* lutx, int i) { lutx[i].x = spread_bit4((u32)i & 0xFu); lutx[i].y = spread_bit4((u32)i >> 4); }
 // The 24 code bits of a group, picked out of two neighbouring words by one byte permute that already puts codes 4..7 at the top:
 // bits 0..11 = codes 0..3, bits 20..31 = codes 4..7 (B = byte offset of the group in the lane's code string).

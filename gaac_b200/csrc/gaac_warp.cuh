@@ -9,19 +9,16 @@ namespace gaac {
 constexpr int XS_STRIDE = 136;                      // u16 per staged row: 272 B keeps 16-byte alignment and spreads banks
 constexpr unsigned FULL = 0xffffffffu;
 
-constexpr int ESC_STAGE = 256;                      // escape bytes of a tile that the decoder stages; longer tiles read theirs where they are
-
 // Per-warp scratch in shared memory.
 struct WarpScratch {
   uint16_t xs[T * XS_STRIDE];                        // staged tile, natural channel order
 };
-struct DecodeScratch : WarpScratch {
-  u32 esc[ESC_STAGE / 4 + 4];                        // the tile's escape bytes, from the 4-byte boundary at or below the first; the raw decoder may read one word behind them
-};
-// What the warps of a CTA that decodes tiles of one (kind, head) share: the escape-byte table and the base words.
+// A decoder's scratch: behind the rows room for the `most` escape bytes that a tile may have, from the 4-byte boundary at or below the first.  What follows them may be read: a
+// segment's four raw groups, and a word.
+__host__ __device__ constexpr int decode_scratch_bytes(int most) { return (int)sizeof(WarpScratch) + ((most + 3 + 20 + 8 + 15) & ~15); }
+// What the warps of a CTA that decodes tiles of one (kind, head) share: the base words.
 struct DecodeTables {
-  u32x2 lutx[256];
-  uint8_t bases[BASES_BYTES];
+  __align__(16) uint8_t bases[BASES_BYTES];
 };
 
 // Encoded tile held in registers, one lane's share.  8 groups per lane for both kinds, in runs of consecutive groups of one row (segments):
@@ -229,10 +226,9 @@ __device__ __forceinline__ void load_base_words(const uint8_t* b3row, const uint
 }
 // Fill the tables of a decoding CTA (any number of threads); the caller synchronises.
 template <int KIND_V>
-__device__ __forceinline__ WarpView fill_decode_tables(DecodeTables& t, const uint8_t* b3row, const uint8_t* b4row) {
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) fill_lutx(t.lutx, i);
+__device__ __forceinline__ u32 fill_decode_tables(DecodeTables& t, const uint8_t* b3row, const uint8_t* b4row) {
   if (threadIdx.x < 32) fill_bases<KIND_V != 0>(t.bases, b3row, b4row, threadIdx.x);
-  return WarpView{(u32)__cvta_generic_to_shared(t.lutx), (u32)__cvta_generic_to_shared(t.bases)};
+  return (u32)__cvta_generic_to_shared(t.bases);
 }
 template <bool TRANS> __device__ __forceinline__ void store_matrices(u32 at, int s, u32 w0, u32 w1, u32 w2, u32 w3) {       // the opposite of load_matrices
   if (!TRANS) asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(at + 32 * s), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
@@ -286,9 +282,12 @@ __device__ __forceinline__ void load_tile_words(TileWords<KIND_V>& tw, const uin
 }
 // Rebuild the tile into ws.xs (natural channel order, bf16 bits).  The escape bytes that did not come with the rest are fetched with one coalesced load as soon as the
 // tags say how many there are (a load per group waited for the one before it at every raw group's branch).  The fragments go to shared memory by
-// stmatrix.
+// stmatrix.  most: escape bytes that the scratch behind ws has room for; less than TILE_MAX_ESC only where no tile has more (tags that say otherwise make wrong values and nothing else).
+// All of a tile's escape bytes are staged, so that a group reads its own without asking whether it has one, and whether any lane's group is raw is asked once per tile: 771 -> 699 (K) and 788 -> 776
+// warp instructions per tile, most of them in branches and 64-bit addresses.  [8, 65536, 128] K and V 88.2 -> 85.7 us;  blocks of 32768 tokens 44.7 -> 43.3, of 512 3.5 -> 3.2.  A second copy of the
+// groups for escape bytes in global memory beside them spilled (93), and so did more than one tile per warp of the block decoder.  Without the rebuild, loads and stores alone, the pages take 80.
 template <int KIND_V>
-__device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, TileWords<KIND_V>& tw, const WarpView& w, int lane) {
+__device__ __forceinline__ void decode_tile_warp(WarpScratch& ws, TileWords<KIND_V>& tw, u32 bases, int lane, int most = TILE_MAX_ESC) {
   const int j = lane & 3, r = lane >> 2;
   constexpr int SEGS = TileWords<KIND_V>::SEGS;
   u32 tags, total, none, pos[SEGS];
@@ -308,28 +307,31 @@ __device__ __forceinline__ void decode_tile_warp(DecodeScratch& ws, TileWords<KI
     for (int t = 0; t < SEGS; t++) pos[t] = t & 1 ? vp[t >> 1] >> 16 : vp[t >> 1] & 0xFFFFu;
   }
   const int n = (int)((total & 0xFFFFu) + (total >> 16)), ofs = (int)(reinterpret_cast<uintptr_t>(esc_src) & 3);
-  const uint8_t* esc = esc_src;
   __syncwarp();                                      // the scratch is no longer in use
-  if (n <= ESC_STAGE) {
+  {
     const u32* g = reinterpret_cast<const u32*>(esc_src - ofs);
-    const int have = tw.n_esc > 0 ? (tw.n_esc + ofs + 3) >> 2 : 0;                           // words that came with the rest
-    if (lane < have) ws.esc[lane] = tw.esc;
-    for (int i = have + lane; 4 * i < (n > 0 ? n + ofs : 0); i += 32) ws.esc[i] = g[i];
-    esc = reinterpret_cast<const uint8_t*>(ws.esc) + ofs;
+    u32* const to = reinterpret_cast<u32*>(&ws + 1);
+    const int have = tw.n_esc > 0 ? (tw.n_esc + ofs + 3) >> 2 : 0;       // words that came with the rest
+    if (lane < have) to[lane] = tw.esc;
+    for (int i = have + lane; 4 * i < (n > 0 ? min(n, most) + ofs : 0); i += 32) to[i] = g[i];
   }
+  const u32 esc0 = (u32)__cvta_generic_to_shared(&ws + 1) + (u32)ofs;
+#pragma unroll
+  for (int i = 0; i < SEGS; i++) pos[i] = esc0 + min(pos[i], (u32)most);
+  const u32 raws = __reduce_or_sync(FULLM, tags & 0xAAAAu);
   __syncwarp();
   const u32 at = matrix_row_address(ws, lane);
 #pragma unroll
   for (int g = 0; g < (KIND_V ? 2 : 4); g++) {
     u32 f[SEGS][4];
-    const u32x4 bw = lds_u128(w.bases + (KIND_V ? BASES_V + 32 * r : 64 * j) + 16 * g);
+    const u32x4 bw = lds_u128(bases + (KIND_V ? BASES_V + 32 * r : 64 * j) + 16 * g);
 #pragma unroll
     for (int i = 0; i < SEGS; i++) {
       constexpr int PER = 8 / SEGS;                  // groups of a segment
       const int b = 3 * (PER * i + g);               // byte of the group's codes in the lane's 24
       const u32 z = b == 0 ? group_codes<0>(cd) : b == 3 ? group_codes<3>(cd) : b == 6 ? group_codes<6>(cd) : b == 9 ? group_codes<9>(cd) :
                     b == 12 ? group_codes<12>(cd) : b == 15 ? group_codes<15>(cd) : b == 18 ? group_codes<18>(cd) : group_codes<21>(cd);
-      decode_group_dev(sm[2 * (PER * i + g)], sm[2 * (PER * i + g) + 1], z, tags >> (2 * (PER * i + g)), pos[i], esc, w, bw, f[i]);
+      decode_group_dev(sm[2 * (PER * i + g)], sm[2 * (PER * i + g) + 1], z, tags >> (2 * (PER * i + g)), pos[i], (raws >> (2 * (PER * i + g)) & 2u) != 0u, bw, f[i]);
     }
     if (!KIND_V) {
 #pragma unroll
