@@ -159,11 +159,12 @@ GAAC_HD u32 pack_hi5(u32 e4) {
   return (f & 0x1Fu) | ((f >> 3) & 0x3E0u) | ((f >> 6) & 0x7C00u) | ((f >> 9) & 0xF8000u);
 }
 // the low three bits of every byte of lo (elements 0-3) and hi (4-7) -> 24 bits, element i at bit 3i; higher bits of the bytes are ignored
+// (bits 24 and above of the result are anything).  Fields are moved next to one another by multiplications, 7 of the 11 operations on the ALU, which the encoder keeps busiest; by shifts and selects all
+// 11 were: [8, 8192, 128] 9.13 (K) / 8.65 (V) -> 9.01 / 8.47 us, x 65536 45.4 / 44.1 -> 45.1 / 44.0.
 GAAC_HD u32 pack_codes8(u32 lo, u32 hi) {
-  const u32 yl = bits_of(lo, lo >> 5, 0x00070007u), yh = bits_of(hi, hi >> 5, 0x00070007u);      // two codes at bits 0-5 of bytes 0 and 2
-  u32 v = prmt(yl, yh, 0x6420) & 0x3F3F3F3Fu;
-  v = bits_of(v, v >> 2, 0x003F003Fu) & 0x0FFF0FFFu;
-  return bits_of(v, v >> 4, 0x00000FFFu);
+  const u32 yl = mad_k<33u>(lo & 0x07070707u, 0u), yh = mad_k<33u>(hi & 0x07070707u, 0u);                  // two codes side by side at bits 5-10 and at 21-26
+  const u32 zl = mad_k<1025u>(yl & 0x07E007E0u, 0u), zh = mad_k<1025u>(yh & 0x07E007E0u, 0u);              // four at bits 15-26
+  return bits_of(zl >> 15, zh >> 3, 0x00000FFFu);
 }
 
 // Encode one group of 8 stored positions given its exponent bytes (elements 0-3 in e_lo, 4-7 in e_hi) and the bases.
