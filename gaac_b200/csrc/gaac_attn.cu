@@ -616,12 +616,25 @@ __device__ __forceinline__ void fewer_ranges(int tiles, int at_once, int& ns, in
 }
 // How the rows are shared out.  GRID: (row, kv head) x splits;  SHARED: a balanced launch;  FLAT_LINE: above.  Instantiations of their own: the shares cost the others
 // registers that the main loop has none of, 1.5 % at 64K tokens.
-enum { GRID, SHARED, FLAT_LINE };
+enum { GRID, SHARED, FLAT_LINE, TEAM };
+// ---- teams: the ranges of a row as one cluster, at most eight CTAs (the portable size), whose partials meet in the shared memory of the first.  Through global memory they take a fence
+// until the partials have arrived there, an atomic, and a load of each back, 1.7 us of a launch of 7; through distributed shared memory 0.7: 8 heads x 500 tokens 7.2 -> 6.1 us in a graph.  The others
+// store into the first CTA and leave; it has said, ahead of its main loop, that the place is free, which is in the stages that a range of at most TEAM_TILES tiles does not reach.  Longer ranges, found out
+// only here where the caller goes by a bound, take the other way: both decide by the row's length, so the CTAs of a cluster agree.
+constexpr int TEAM_MOST = 8, TEAM_STAGE = 6, TEAM_TILES = TEAM_STAGE * TPS;
+static_assert((TEAM_MOST - 1) * 8 * 130 * 4 <= (NSTG - TEAM_STAGE) * STAGE_BYTES, "the partials lie in stages that so few tiles do not reach");
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ u32 cluster_address(u32 at, u32 rank) { u32 v; asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(v) : "r"(at), "r"(rank)); return v; }
+__device__ __forceinline__ void cluster_store(u32 at, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
+
 template <bool PAGED, bool DUMP, int NSET, int MODE>
 __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __grid_constant__ AttnParams p) {
-  constexpr bool SHARE = MODE == SHARED, FLAT = MODE == FLAT_LINE;
+  constexpr bool SHARE = MODE == SHARED, FLAT = MODE == FLAT_LINE, ROWS = MODE == GRID || MODE == TEAM;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int s_next, s_last, s_split, s_ns, s_tail, s_esc[6];        // (from s_split on: not needed inside the main loop, whose registers are all taken)
+  __shared__ int s_next, s_last, s_split, s_ns, s_tail, s_esc[6];
+  __shared__ int s_team;        // (from s_split on: not needed inside the main loop, whose registers are all taken)
   __shared__ FlatWalk s_flat;
   __shared__ int s_rows[FLAT ? 64 : 1];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -647,8 +660,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   };
   begin_ring(false);
   // What the grid's own numbering gives is worked out ahead of the wait: the divisions are a quarter of the time from there to the first copy.
-  int bh = blockIdx.x, b = bh / p.n_kv, kvh = bh - b * p.n_kv, chunk_all = MODE == GRID && !PAGED ? (((p.S_uniform + 15) >> 4) + p.nsplit - 1) / p.nsplit : 0;
-  if (MODE == GRID) asm volatile("" : "+r"(b), "+r"(kvh), "+r"(chunk_all));
+  int bh = blockIdx.x, b = bh / p.n_kv, kvh = bh - b * p.n_kv, chunk_all = ROWS && !PAGED ? (((p.S_uniform + 15) >> 4) + p.nsplit - 1) / p.nsplit : 0;
+  if (ROWS) asm volatile("" : "+r"(b), "+r"(kvh), "+r"(chunk_all));
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
 
@@ -704,7 +717,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (bh < 0) return;
     if (PAGED) S_paged = s_flat.tokens;
   }
-  if (MODE != GRID) { b = bh / p.n_kv; kvh = bh - b * p.n_kv; }
+  if (!ROWS) { b = bh / p.n_kv; kvh = bh - b * p.n_kv; }
 
   // ---- which cache head, how many tokens, this CTA's tile range [tlo, tlo + n)
   // (without a slot map row b reads slot b; without a length table every head holds S_uniform tokens: the two dependent
@@ -724,8 +737,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // compiler so, and the address arithmetic built on them stays in uniform registers.
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
   const int ntiles = (S + 15) >> 4;
-  int chunk = MODE == GRID && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
-  if (MODE == GRID && p.nsplit > 1) {
+  int chunk = ROWS && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
+  if (ROWS && p.nsplit > 1) {
     if (PAGED || p.seq_len) { fewer_ranges(ntiles, ATT_WARPS, ns0, chunk); if (split0 >= ns0) return; }
     if (tid == 0) s_ns = ns0;
   }
@@ -849,6 +862,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     for (int i = 0; i < 4; i++) { const uint4 w = q_place[32 * i]; Q.qa[2 * i][0] = w.x; Q.qa[2 * i][1] = w.y; Q.qa[2 * i + 1][0] = w.z; Q.qa[2 * i + 1][1] = w.w; }
     __syncthreads();
   }
+  if (MODE == TEAM) {
+    const bool team = ns0 > 1 && chunk <= TEAM_TILES;
+    if (tid == 0) s_team = team;
+    __syncwarp();
+    if (team) cluster_arrive();                      // (the places of the partials are free)
+  }
   if (filler && warp >= FIRST) {                     // (where all CTAs begin together, behind the warp's own first tile: any earlier, and these copies hold back the first stages')
     u32 flags;
     if (!FLAT) __all_sync(FULLM, mbar_wait_use(smem_s + TB_FULL + 8 * (warp / TPS), 0u, smem_s + TB_USE + 4 * warp, (u32)(warp / TPS) + 1u, flags));          // (one that runs out is met again in the main loop)
@@ -910,7 +929,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
     it = nx;
   }
-  const int split = SHARE || FLAT ? s_split : split0, NS = MODE == GRID && p.nsplit == 1 ? 1 : s_ns;
+  const int split = SHARE || FLAT ? s_split : split0, NS = ROWS && p.nsplit == 1 ? 1 : s_ns;
   if (FLAT) { bh = __shfl_sync(FULLM, s_flat.pair, 0); b = bh / p.n_kv; kvh = bh % p.n_kv; TL = __shfl_sync(FULLM, s_tail, 0); }
   // ---- slot layout: the raw BF16 tail belongs to the last split's last warp
   if (!PAGED && TL > 0 && split == NS - 1 && warp == ATT_WARPS - 1) {
@@ -960,12 +979,51 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     const int g = (tid >> 7) + 4 * i;
     if (g >= G) continue;
     merge_warps<ATT_WARPS>(smem + TB_RING, 1, 0, g, d, M[i], Lc[i], Ac[i]);
+    if (MODE == TEAM && s_team) continue;
     if (FLAT && NS == 1) deliver(g, M[i], Lc[i], Ac[i]);
     if (NS > 1) {
       const long pidx = FLAT ? (long)(blockIdx.x + bh) * G + g : SHARE ? ((long)blockIdx.x * p.units + blockIdx.y) * G + g : (qh0 + g) * p.nsplit + split;
       if (d == 0) { p.pm[pidx] = M[i]; p.pl[pidx] = Lc[i]; }
       p.pa[pidx * D + d] = Ac[i];
     }
+  }
+  if (MODE == TEAM && s_team) {
+    const float* const parts = reinterpret_cast<const float*>(smem + TB_RING + TEAM_STAGE * STAGE_BYTES);           // [split - 1][8][m, l, acc]
+    cluster_wait();
+    if (split) {
+      const u32 first = cluster_address(smem_s + TB_RING + TEAM_STAGE * STAGE_BYTES, 0u) + (u32)(split - 1) * (8 * 130 * 4);
+#pragma unroll
+      for (int i = 0; i < NSET; i++) {
+        const int g = (tid >> 7) + 4 * i;
+        if (g >= G) continue;
+        const u32 at = first + (u32)g * (130 * 4);
+        if (d == 0) { cluster_store(at, M[i]); cluster_store(at + 4, Lc[i]); }
+        cluster_store(at + 8 + 4 * d, Ac[i]);
+      }
+      __syncwarp();
+      cluster_arrive_release();
+      return;
+    }
+    cluster_arrive_release();
+    cluster_wait();
+#pragma unroll
+    for (int i = 0; i < NSET; i++) {
+      const int g = (tid >> 7) + 4 * i;
+      if (g >= G) continue;
+      float m[7], most = M[i];
+#pragma unroll
+      for (int s = 0; s < 7; s++) { m[s] = s + 1 < NS ? parts[(s * 8 + g) * 130] : -CUDART_INF_F; most = fmaxf(most, m[s]); }
+      const float keep = M[i] == -CUDART_INF_F ? 0.f : fast_exp2(M[i] - most);
+      float L = Lc[i] * keep, A2 = Ac[i] * keep;
+#pragma unroll
+      for (int s = 0; s < 7; s++)
+        if (s + 1 < NS && m[s] != -CUDART_INF_F) {
+          const float f = fast_exp2(m[s] - most);
+          L += parts[(s * 8 + g) * 130 + 1] * f; A2 += parts[(s * 8 + g) * 130 + 2 + d] * f;
+        }
+      deliver(g, most, L, A2);
+    }
+    return;
   }
   const bool last = NS == 1 || last_split(p.counters + bh, NS, &s_last);        // (of one split there is nothing to merge)
   if (!FLAT && !last) return;
@@ -1344,16 +1402,17 @@ static void launch_row_order(const int* seq_lens, int B, int2* order, cudaStream
 // Launch of an attention kernel, one CTA of ATT_THREADS per SM.  The permission for its shared memory is asked for once per kernel and device, not on every
 // launch; where a launch fails with the permission believed to be there (it goes with a device reset), it is asked for again.
 template <auto Kernel>
-static int launch_big(const AttnParams& p, dim3 grid, int smem_bytes, cudaStream_t st) {
+static int launch_big(const AttnParams& p, dim3 grid, int smem_bytes, cudaStream_t st, int team = 1) {
   static std::atomic<unsigned long long> allowed{0};                  // one bit per device
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = dim3(ATT_THREADS); cfg.dynamicSmemBytes = smem_bytes; cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
-  cfg.attrs = at; cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)team; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = team > 1 ? 2 : 1;
   bool asked = false;
   while (true) {
     if (asked || !(allowed.load(std::memory_order_relaxed) & bit)) {
@@ -1370,17 +1429,44 @@ static int launch_big(const AttnParams& p, dim3 grid, int smem_bytes, cudaStream
 template <bool PAGED, bool DUMP, int NSET, int MODE>
 static int launch_attn_as(const AttnParams& p, cudaStream_t st) {
   const dim3 grid = MODE == FLAT_LINE ? dim3((unsigned)p.flat) : MODE == SHARED ? dim3((unsigned)p.n_kv, (unsigned)p.units) : dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit);
-  return launch_big<decode_attn_kernel<PAGED, DUMP, NSET, MODE>>(p, grid, ATT_SMEM, st);
+  return launch_big<decode_attn_kernel<PAGED, DUMP, NSET, MODE>>(p, grid, ATT_SMEM, st, MODE == TEAM ? p.nsplit : 1);
 }
 template <int NSET>
 static int launch_attn256(const AttnParams& p, cudaStream_t st) {
   if (p.flat) return launch_big<paged256_attn_kernel<NSET, true>>(p, dim3((unsigned)p.flat), ATT256_SMEM, st);
   return launch_big<paged256_attn_kernel<NSET, false>>(p, dim3((unsigned)(p.B * p.n_kv), (unsigned)p.nsplit), ATT256_SMEM, st);
 }
+// Whether a launch may be made of teams: all of its clusters must fit the GPU at a time (15 of 8 or 7 CTAs, 22 of 6, 26 of 5, 33 of 4 on the one that this was measured on, since a cluster lies in one
+// group of SMs; 16 rows in 8 ranges each take 11.7 us as clusters, 8.7 without), and they gain only where ranges are short.
+template <bool PAGED, int NSET>
+static int team_room(int nsplit) {
+  static std::atomic<int> known[64][TEAM_MOST + 1];                   // clusters, and one
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
+  int n = known[dev][nsplit].load(std::memory_order_relaxed) - 1;
+  if (n < 0) {
+    const auto kernel = decode_attn_kernel<PAGED, false, NSET, TEAM>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(64, (unsigned)nsplit); cfg.blockDim = dim3(ATT_THREADS); cfg.dynamicSmemBytes = ATT_SMEM;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = (unsigned)nsplit; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 0) { cudaGetLastError(); n = 0; }
+    known[dev][nsplit].store(n + 1, std::memory_order_relaxed);
+  }
+  return n;
+}
+template <bool PAGED>
+static bool team_ok(const AttnParams& p) {
+  if (p.part || p.x_recv || p.row_order || p.nsplit < 2 || p.nsplit > TEAM_MOST) return false;
+  if (!PAGED && !p.seq_len && ((p.S_uniform + T - 1) / T + p.nsplit - 1) / p.nsplit > TEAM_TILES) return false;
+  return (int64_t)p.B * p.n_kv <= (p.G <= 4 ? team_room<PAGED, 1>(p.nsplit) : team_room<PAGED, 2>(p.nsplit));
+}
 template <bool PAGED, bool DUMP>
 static int launch_attn(const AttnParams& p, cudaStream_t st) {
   if (!DUMP && p.flat) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, FLAT_LINE>(p, st) : launch_attn_as<PAGED, false, 2, FLAT_LINE>(p, st);
   if (!DUMP && p.units) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, SHARED>(p, st) : launch_attn_as<PAGED, false, 2, SHARED>(p, st);
+  if (!DUMP && team_ok<PAGED>(p)) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, TEAM>(p, st) : launch_attn_as<PAGED, false, 2, TEAM>(p, st);
   return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1, GRID>(p, st) : launch_attn_as<PAGED, DUMP, 2, GRID>(p, st);
 }
 

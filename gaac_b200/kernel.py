@@ -82,7 +82,11 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     # faster; beyond, splits pay down to four tiles each until there are 16 (one per warp of the merge), more only with 16 tiles each.  Batch 1, 8
     # kv heads: 500 tokens 10.8 -> 8.4 us, 1000: 18.1 -> 8.3, 2000: 15.6 -> 8.8; 4 rows of 1000: 18.6 -> 9.9; 1 kv head, 8000 tokens: 16.3 in 15
     # splits, 13.3 in 32, 17.4 in 125.  A second wave costs more than it shortens (4 rows of 1000 in 6 splits: 15.3).
-    wave = sm_count // rows
+    # Up to eight ranges of a row are a team (clusters whose partials do not go through global memory), where all teams fit the GPU at a time; there three tiles are enough for a range, and ten tiles for
+    # a second one: batch 1, 8 kv heads, 200 tokens 6.6 -> 6.3, 500 7.2 -> 6.1, 1000 7.8 (15 splits) -> 6.8, 1500 8.2 -> 7.4, 2000 8.0 -> 8.05;  2 rows: 500 8.4 (8 splits) -> 7.2 (6), 1000 9.0 (9) -> 8.0.
+    wave, team = sm_count // rows, _team(rows)
+    if team > 1 and (8 if team >= 6 else ATT_WARPS) < ntiles <= 14 * team:         # (many rows of one CTA each: 32 x 1 of 200 tokens 8.4 -> 8.2 where they are that long, 5.3 -> 5.9 where that is a bound)
+        return min(team, ntiles // 3)
     if wave > 1 and 4 * most <= 3 * wave:
         return 1 if ntiles <= ATT_WARPS else min(wave, max(min(16, ntiles // 4), -(-ntiles // 16)))
     tile_us, tile_far_us, fixed_us, staged = 4.5, 5.2, 10.0, 512
@@ -95,6 +99,14 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
         if best_t is None or t < best_t * 0.985:                       # prefer fewer splits unless clearly better
             best, best_t = ns, t
     return best
+
+
+TEAMS = {8: 15, 6: 22, 5: 26, 4: 33, 3: 45, 2: 74}       # ranges of a team: how many teams a B200 has room for (the library asks, and does without them where there are fewer)
+
+
+def _team(rows: int) -> int:
+    """Most ranges that a row's team may have when all rows have one."""
+    return next((n for n in TEAMS if rows <= TEAMS[n]), 1)
 
 
 def _short_ranges(rows: int, ntiles: int, sm_count: int = SM_COUNT_B200) -> bool:
