@@ -1,12 +1,12 @@
 // Warp-level pieces of the fused decode attention: asynchronous copies, the rebuild of a compressed 16-token tile into tensor-core
 // fragments, the score and value products and the online softmax step.  Used by the kernels of gaac_attn.cu.
 //
-// What bounds them, measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens: 1052 warp instructions per (K tile + V tile) at 0.66 per cycle and scheduler (0.74 in the main loop), with
-// four warps to a scheduler; ALU pipe 61 %, the shared-memory pipe 282 cycles of the main loop's 345 per tile pair, DRAM 42 %.  A warp issues every 6 cycles and spends, of these, 1.2 waiting for a
-// result of fixed latency, 1.1 ready but not chosen, 0.9 on shared memory, 0.7 on a busy pipe (the ALU), 0.3 at barriers, 0.25 on global memory: instructions and cycles of shared memory
-// first, then latency, since a third of the issue slots finds no warp ready.  More warps do not help (gaac_attn.cu: 18 or 20 at 96 registers).  Timing-only builds of an earlier
-// form: without the raw groups 50 us of 57, without any of plan_tile 41.  What did not help: moving shifts from the ALU to the FMA pipe, fewer or longer chains at the same
-// count of instructions, warps of their own for plan_tile or for the copies.
+// What bounds them, measured on a B200 at batch 1, 32 query / 8 kv heads, 65536 tokens, 47.1 us: 950 warp instructions per (K tile + V tile) at 0.65 per cycle and scheduler, with
+// four warps to a scheduler; 430 of them on the ALU (59 % of its cycles), 279 wavefronts of shared memory, DRAM 44 %.  A warp issues every 6.1 cycles and spends, of these, 1.1 waiting for a
+// result of fixed latency, 1.1 ready but not chosen, 1.0 on shared memory, 0.7 on a busy pipe (the ALU), 0.3 at barriers, 0.3 on global memory: instructions first, then latency, since a
+// third of the issue slots finds no warp ready.  More warps do not help (gaac_attn.cu: 18 or 20 at 96 registers).  Timing-only builds of a form of 51 us: without the raw groups 47,
+// without any of plan_tile 39, with the payload read without bank conflicts 51, with no work on the tiles at all 34.  What did not help: moving shifts from the ALU to the FMA pipe, fewer
+// or longer chains at the same count of instructions, warps of their own for plan_tile or for the copies.
 //
 // Head columns.  The tensor-core tile has 8 columns.  Query heads are handled in sets of four (NSET = 1 for a GQA group of up to
 // 4, 2 for 5..8); lane j of a quad works for head 4 * set + j throughout:
@@ -16,7 +16,8 @@
 //           gets both channels of its own head.  16 products per tile, as many as a transposed form has for 8 heads
 //   values, two sets: the columns are the heads, as for the scores, and the words of two tokens are transposed by 32 byte permutes per tile.  The form
 //           above takes 32 products and 16 registers of weights where this takes 16 and 4, and was slower: group of 8, 8 kv heads, 65536
-//           tokens 67.1 us, now 64.4; paged 32768 40.1 -> 38.7; head_dim 256, 8 x 8000: 119 -> 111
+//           tokens 67.1 us, 64.4 with it; paged 32768 40.1 -> 38.7; head_dim 256, 8 x 8000: 119 -> 111.  Words of two tokens made by the rebuild itself, with its last
+//           permutes taking both: 64 x 32768 189.6 -> 189.4 and 32 bytes of spills, so not kept
 #pragma once
 #include <cuda_bf16.h>
 #include <math_constants.h>
@@ -262,7 +263,7 @@ __device__ __forceinline__ void scan_step16(u32& v, int d) {
 // Make the segment area of a tile pair.  Lane l has row l & 15 of K (l < 16) or of V.  live: the lane's side is compressed; fl, esc: shared-memory addresses of its
 // tag words and of its escape bytes, of which `avail` are staged.  Returned: bit 0 / 1: those of K / V are all staged (and the staged sides have no more than `room` raw
 // groups, which have their entries, 8 bytes each, behind the segment words; the other groups of raw_items need none).
-// Bound by its instructions, 282 of 1052 per tile pair before, about 235 now, and by its chain of latencies; hence a scan over 16 rows and not over 64 segments, and sizes from the tag words
+// Bound by its instructions, 282 of 1052 per tile pair before, about 200 of 950 now, and by its chain of latencies; hence a scan over 16 rows and not over 64 segments, and sizes from the tag words
 // while the segment table answers.  The scan counts the raw groups along with the escape bytes, so that a row knows its entries' places and takes its items without asking the
 // others.  The raw groups, 4 of 512, took half of it (147 instructions: 1.8 trips of a loop in which both kinds of item lay on either side of a branch; a timing-only build without that loop 51.3 -> 46.6 us).
 // Now each kind has a loop of its own, from the last item to the first, where the mask of what lies below an item also takes it off, and one vote asks whether everything is staged and

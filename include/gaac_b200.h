@@ -148,7 +148,8 @@ size_t gaac_attn_workspace_header_bytes(int B, int n_q);
 
 /* Fused decode attention over compressed K/V.  q [B, n_q, 128] bf16; batch row b reads cache head slot[b]*n_kv + kvh
  * (slot[b] < 0: padded row, output exactly 0); seq_len[cache head] compressed tokens; tail_len[cache head] raw tail tokens
- * (NULL when there is no tail).  nsplit >= 1 context splits per (row, kv head).  out [B, n_q, 128] bf16; when out_f32 is
+ * (NULL when there is no tail).  nsplit >= 1 context splits per (row, kv head), at most where lengths are read on the GPU: a row whose ranges would be shorter than
+ * a tile per warp takes fewer.  Ranges of up to 24 tiles of up to eight splits may run as a cluster, merged in its shared memory.  out [B, n_q, 128] bf16; when out_f32 is
  * non-NULL the un-rounded fp32 result is written there as well.  workspace: gaac_attn_workspace_bytes bytes with a zeroed
  * header (see above).  n_base_rows: rows of the base tables (cache head h uses row h % n_base_rows).  Here and in every other
  * attention call an infinite or NaN element of V makes its own output channel infinite or NaN and no other; the ranges that hold one
@@ -370,7 +371,7 @@ int gaac_paged_decode_attn_flat(const gaac_paged* st, const int32_t* bt, int64_t
  * bases, so the store, the block decoder and the bases all see 2 * (256-dim kv heads) half-heads: st->n_kv is that number of
  * HALF-heads (even), as for gaac_paged_store; the base tables have st->n_kv rows.  q [B, n_q, 256] bf16, out [B, n_q*256] bf16
  * (out_f32 optional), n_q a multiple of st->n_kv / 2 with group size 1..8.  workspace: gaac_attn_workspace_bytes(B, 2 * n_q,
- * nsplit) bytes.  Two launches (attention over warp pairs, then the split merge).  Replaces gaac_vpaged256_launch =
+ * nsplit) bytes.  Replaces gaac_vpaged256_launch =
  * gaac_vpaged256<G> + gaac_combine2 (gaac/vllm/paged_kernel256.py:40-283, 299-305). */
 int gaac_paged_decode_attn256(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                               int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes,
