@@ -1092,7 +1092,7 @@ constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;         
 static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 336 <= 232448, "one CTA per SM");
 
 static_assert(FLAT_SCRATCH <= ATT_WARPS * SEG256_BYTES, "planned in the segment areas");
-// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.1 -> 24.8 us, 20 x 8 of up to 3K 95 -> 73 (a grid, rows as they come).  Pieces of two tiles on short rows: of four
+// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.1 -> 24.8 us (22.5 now), 20 x 8 of up to 3K 95 -> 73 (a grid, rows as they come; 70 now).  Pieces of two tiles on short rows: of four
 // 0.5 us slower on 2 x 4 of 700.
 template <int NSET, bool FLAT>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
@@ -1140,7 +1140,23 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (bh < 0) return;
   }
   int b = bh / p.n_kv, kvh = bh % p.n_kv;
-  const int S = __shfl_sync(FULLM, FLAT ? s_flat.tokens : p.seq_len[b], 0);
+  // The loads that need no length, queries and bases, beside the first that are waited for: in a grid the length, in a flat launch, which has planned with it, the block table.  Then the table for the
+  // pair's first tile and for the tiles whose metadata is kept together, then both of their mode-table entries, so that the barrier waits for three loads behind one another.  (The first tile's chain, then
+  // queries, bases and the kept tiles' chain: five to six.)  us, with the return behind the merges: 8 x 4 rows of 1K-8K tokens 23.3 -> 22.5, 9 x 4 of 500-12000 41.7 -> 39.9, 6 x 2 of 4K-60K 66.1 ->
+  // 64.1, in a grid 8 x 4 of 510 11.2 -> 10.9.  The second tile of every pair asked for as soon as the first is there: 16.6 -> 16.2 where a pair has two or three, but its branch in the main loop
+  // costs a per cent where it has more.
+  const int tokens = FLAT ? s_flat.tokens : p.seq_len[b];
+  QFrag Q;
+  auto load_tables = [&] {
+    load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * (2 * D) + hf * D, 2 * D, G, lane);
+    if (warp >= 8 && warp < 12) {
+      const int h2 = warp & 1, row = (2 * kvh + h2) * D;
+      uint8_t* o = smem + T256_BASES + h2 * PAIR_BASES_BYTES;
+      if (lane < 16) { if (warp < 10) fill_pair_bases<false>(o, p.b3k + row, p.b4k + row, lane); else fill_pair_bases<true>(o, p.b3v + row, p.b4v + row, lane); }
+    }
+  };
+  if (!FLAT) load_tables();
+  const int S = __shfl_sync(FULLM, tokens, 0);
   const int ntiles = (S + 15) >> 4;
   int chunk = (ntiles + NS - 1) / NS;
   if (!FLAT) {
@@ -1167,19 +1183,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   };
   int it = pair;
   TileMeta cur{0, 0};
-  if (it < n) {
-    const int pc = slot_of(it) + 2 * hf;
-    cur = TileMeta{p.mt[pc], p.mt[pc + 1]};
-    if (lane == 0) issue(ring_s, cur);
-  }
-  QFrag Q;
-  load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * (2 * D) + hf * D, 2 * D, G, lane);
-  if (warp >= 8 && warp < 12) {
-    const int h2 = warp & 1, row = (2 * kvh + h2) * D;
-    uint8_t* o = smem + T256_BASES + h2 * PAIR_BASES_BYTES;
-    if (lane < 16) { if (warp < 10) fill_pair_bases<false>(o, p.b3k + row, p.b4k + row, lane); else fill_pair_bases<true>(o, p.b3v + row, p.b4v + row, lane); }
-  }
-  if (tid < min(n, META256_TILES)) { const int pc = slot_of(tid); reinterpret_cast<int4*>(smem + T256_META)[tid] = make_int4(p.mt[pc], p.mt[pc + 1], p.mt[pc + 2], p.mt[pc + 3]); }
+  const bool first = it < n, keeps = tid < min(n, META256_TILES);
+  const int pc = first ? slot_of(it) + 2 * hf : 0, pk = keeps ? slot_of(tid) : 0;
+  if (FLAT) load_tables();
+  int4 kept{0, 0, 0, 0};
+  if (first) cur = TileMeta{p.mt[pc], p.mt[pc + 1]};
+  if (keeps) kept = make_int4(p.mt[pk], p.mt[pk + 1], p.mt[pk + 2], p.mt[pk + 3]);
+  if (first && lane == 0) issue(ring_s, cur);
+  if (keeps) reinterpret_cast<int4*>(smem + T256_META)[tid] = kept;
   if (tid == 0) s_next = ATT_WARPS / 2;               // tiles 0 .. pairs - 1 of the range go to the pairs in order, the rest is handed out on demand
   WarpAcc<NSET> A;
   A.clear();
@@ -1278,7 +1289,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
       deliver(row0 + vg, Lv, Av);
     }
   }
-  if (FLAT) __syncthreads();                         // the shared memory is used again
+  if (FLAT) {
+    if (s_flat.share == 0) return;                   // (a plan of one piece per CTA: the walk would only find that out, 0.3 us later)
+    __syncthreads();                                 // the shared memory is used again
+  }
   } while (FLAT);
 }
 
