@@ -101,6 +101,8 @@ __device__ __forceinline__ void push_raw_tile(int* stack, int* top, int r) {
 
 // One warp: entry e, tile slot t = 2*kvh + kind.  Returns (lane 0) the raw tile that the store set free, or -1: it may go back on the stack once no
 // warp of the step pops any more.
+// Bound by its chain of loads: the entry, the mode table, rows and bases, then the encoder's work.  New rows and bases do not depend on the table and travel with its entry; behind one another
+// they cost most where no cache holds them: a step of 8 rows at head_dim 256, store and attention over two states in turn, 38.1 -> 34.5 us (58 MB of slots each); out of L2 nothing.
 template <int KIND_V>
 __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, int e, int t, int lane) {
   const gaac_paged& st = p.st;
@@ -116,17 +118,22 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   uint16_t* rawp = reinterpret_cast<uint16_t*>(st.raw);
   int fits = 0, r = r_old;
   if (full) {
-    // gather the tile: old rows from the raw tile (if any), new rows from this step's K/V
+    // gather the tile: old rows from the raw tile (if any), new rows from this step's K/V, which travel with the mode-table entry
+    uint4 v[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const int c = lane + 32 * k, row = c >> 4, col = (c & 15) * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (row >= off0) v = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
-      else if (have) v = *reinterpret_cast<const uint4*>(rawp + ((long)r_old * T + row) * D + col);
-      *reinterpret_cast<uint4*>(&ws.xs[row * XS_STRIDE + col]) = v;
+      v[k] = make_uint4(0, 0, 0, 0);
+      if (row >= off0) v[k] = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
     }
     u32 b3w[8], b4w[8];
     load_base_words<KIND_V>((KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D, lane, b3w, b4w);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int c = lane + 32 * k, row = c >> 4, col = (c & 15) * 8;
+      if (row < off0 && have) v[k] = *reinterpret_cast<const uint4*>(rawp + ((long)r_old * T + row) * D + col);
+      *reinterpret_cast<uint4*>(&ws.xs[row * XS_STRIDE + col]) = v[k];
+    }
     LaneTile lt;
     const int total = encode_tile_warp<KIND_V>(ws, T, b3w, b4w, lane, lt);
     fits = total <= st.ovf_slot;
@@ -137,9 +144,13 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
     }
   }
   if (!fits) {
+    const bool one = !full && lane < n * 16;         // the first row or two travel with the mode-table entry and the pop
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (one) v = *reinterpret_cast<const uint4*>(src + (long)(tok0 + (lane >> 4)) * sstride + (lane & 15) * 8);
     if (!have) r = pop_raw_tile(st, lane);
     // new rows, natural channel order, into raw tile r
-    for (int c = lane; c < (r < 0 ? 0 : n * 16); c += 32) {
+    if (one && r >= 0) *reinterpret_cast<uint4*>(rawp + ((long)r * T + off0 + (lane >> 4)) * D + (lane & 15) * 8) = v;
+    for (int c = full ? lane : lane + 32; c < (r < 0 ? 0 : n * 16); c += 32) {
       const int row = off0 + (c >> 4), col = (c & 15) * 8;
       *reinterpret_cast<uint4*>(rawp + ((long)r * T + row) * D + col) = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
     }
