@@ -17,20 +17,22 @@ struct AppendParams {
 
 // One CTA per (batch row, kv head): warp 0 appends K, warp 1 appends V; the shared counters are advanced once both are done
 // (the reference needs a second launch for that: gaac/kv_cache.py:72-73,87-96).
+// Bound by its chain of loads, from the slot number on; the new row travels with the slot number and the bases of a tile that fills with its rows (us, append and attention in a graph: 7 rows of up to
+// 3000 tokens 19.35 -> 19.2, 64 of 32768 188.5 -> 187.7).
 // First half: the new row goes into the tail; when that fills the tail, the 16 rows are encoded into registers.  Returns the
 // tile's escape bytes, or -1 when there is no tile to store (tail not full, or the head is at its token capacity).
 template <int KIND_V>
-__device__ __forceinline__ int append_encode(WarpScratch& ws, const gaac_store& st, const uint16_t* xrow, long h, int pos, int tile, long S_cap,
+__device__ __forceinline__ int append_encode(WarpScratch& ws, const gaac_store& st, uint2 row, long h, int pos, int tile, long S_cap,
                                              int n_base_rows, int lane, LaneTile& lt) {
   uint16_t* tail = reinterpret_cast<uint16_t*>(st.tail) + h * (T * D);
-  reinterpret_cast<uint2*>(tail + (long)pos * D)[lane] = reinterpret_cast<const uint2*>(xrow)[lane];       // 32 lanes x 8 B = one row
+  reinterpret_cast<uint2*>(tail + (long)pos * D)[lane] = row;                 // 32 lanes x 8 B
   if (pos + 1 != T) return -1;
   if ((long)tile * T + T > S_cap) return -1;          // cache full: never write past the head's capacity (callers check capacity at prefill)
-  __syncwarp();
-  stage_rows(ws, tail, D, T, lane);                   // rows written by this warp just now are visible to it after the barrier
   const int brow = (int)(h % n_base_rows);
   u32 b3w[8], b4w[8];
   load_base_words<KIND_V>(st.base3 + (long)brow * D, st.base4 + (long)brow * D, lane, b3w, b4w);
+  __syncwarp();
+  stage_rows(ws, tail, D, T, lane);                   // rows written by this warp just now are visible to it after the barrier
   return encode_tile_warp<KIND_V>(ws, T, b3w, b4w, lane, lt);
 }
 // Second half: the encoded tile goes to the head's streams, its escape bytes behind the bytes in use.
@@ -51,13 +53,14 @@ __global__ void __launch_bounds__(64) append_kv_kernel(const __grid_constant__ A
   griddep_wait();
   griddep_launch();                                   // the step's attention may set up its tables meanwhile
   const int sl = p.slot[i / p.n_kv];
+  const uint2 row = reinterpret_cast<const uint2*>((warp == 0 ? p.k_new : p.v_new) + (long)i * D)[lane];          // (travels with the slot number)
   if (sl < 0) return;
   const long h = (long)sl * p.n_kv + i % p.n_kv;
   const int pos = p.tail_len[h], tile = p.seq_len[h] / T;
   LaneTile lt;
   const gaac_store& st = warp == 0 ? p.K : p.V;
-  const int total = warp == 0 ? append_encode<0>(scratch[0], p.K, p.k_new + (long)i * D, h, pos, tile, p.S_cap, p.n_base_rows, lane, lt)
-                              : append_encode<1>(scratch[1], p.V, p.v_new + (long)i * D, h, pos, tile, p.S_cap, p.n_base_rows, lane, lt);
+  const int total = warp == 0 ? append_encode<0>(scratch[0], p.K, row, h, pos, tile, p.S_cap, p.n_base_rows, lane, lt)
+                              : append_encode<1>(scratch[1], p.V, row, h, pos, tile, p.S_cap, p.n_base_rows, lane, lt);
   // A tile whose escape bytes (plus the 8 bytes a reader may touch behind them) do not fit what is left of the head's escape
   // stream is not stored, for K and V alike: nothing is written outside the head's share, the counters stay, *err counts it.
   if (lane == 0) s_fit[warp] = total < 0 || (long)st.ovf_used[h] + total + 8 <= p.ovf_cap;
