@@ -645,8 +645,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // ---- programmatic dependent launch: the grid is launched with stream serialisation relaxed, so its CTAs can be made
   // resident while the previous kernel of the stream is still finishing (its split merge runs on a few SMs only).  What does not
   // depend on memory is set up before the wait; nothing is read before that kernel has completed; the next kernel of the stream may be
-  // staged behind this one right away (it cannot become resident before this grid's CTAs leave their SMs).  Both instructions are no-ops
-  // in a plain launch.
+  // staged behind this one as soon as all of this grid's CTAs are there, whatever they wait for (it waits in turn, and nobody needs the SMs that it takes any more): said ahead of the wait, layers
+  // back to back take 6.05 -> 5.8 us at 500 tokens and 47.3 -> 47.0 at 65536.  Both instructions are no-ops in a plain launch.
   if (tid < 256) fill_attn_tables(smem, tid);
   // Warp w fills stage w first, and clears the words of its tiles: a lane that publishes one has cleared it itself, so no other warp has to be waited for.
   auto begin_ring = [&](bool again) {
@@ -663,8 +663,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // What the grid's own numbering gives is worked out ahead of the wait: the divisions are a quarter of the time from there to the first copy.
   int bh = blockIdx.x, b = bh / p.n_kv, kvh = bh - b * p.n_kv, chunk_all = ROWS && !PAGED ? (((p.S_uniform + 15) >> 4) + p.nsplit - 1) / p.nsplit : 0;
   if (ROWS) asm volatile("" : "+r"(b), "+r"(kvh), "+r"(chunk_all));
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // Which (row, kv head, split) this CTA works on.  Normally the grid says so.  With a row order (ragged paged batches) the CTAs
   // are numbered in the order the hardware hands them out (x fastest) and that number walks the rows from the longest to the
@@ -1115,8 +1115,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     }
   };
   if (!FLAT) begin_ring();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   auto tokens_of = [&](int row) -> int { return p.seq_len[row]; };
   if (FLAT) {
     FlatWalk f;
