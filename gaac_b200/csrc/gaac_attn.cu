@@ -426,7 +426,7 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
 //  line    all pairs one behind the other, FLAT_EXTRA places in front of each, every CTA an equal share of the places: CTA c has [c * share, (c + 1) * share).  An
 //          empty pair (its output is zero) goes to the CTA that has its last place.  A CTA begins in the middle of a pair and pays for that piece: share + FLAT_EXTRA.
 //  single  no more pairs than CTAs: every pair in ceil(tiles / C) equal pieces (or in as many as every other, where they are about equally long), one piece per CTA, where
-//          the smallest C for which the CTAs suffice is no more than share.
+//          the smallest C for which the CTAs suffice is no more than share (and SLACK).
 //  whole   more pairs than CTAs: the pairs in order of length, longest first, dealt out forth and back.  Where the CTA that gets most has no more than the line's, it saves the
 //          pieces in the middle and the merges.  That is what short rows want, and a caller who has a table (or a capacity) much wider than its rows are long.
 // A piece has its partials at (CTA + pair) * G, which no two pieces share: pieces of a pair are those of consecutive CTAs, in order.
@@ -435,7 +435,11 @@ __device__ __forceinline__ void sum_exact(const AttnParams& p, uint8_t* area, in
 // The line alone, and now: 64 x 8 of 100-400 in a table of 8192 39.9 -> 32.0, 32 x 8 of 20-2000 49.1 -> 42.2, 24 x 8 of 64-600 23.9 -> 16.7, 512 x 1 of 50-600 48.4 -> 38.7, 8 x 8 of 200-3000
 // 18.4 -> 15.7, 37 x 4 of 8K 113.8 -> 108.0, 300 x 1 of 100-2000 67.3 -> 66.6;  head_dim 256: 32 x 8 of up to 1000 53.8 -> 40.1, 8 x 4 of 100-700 15.1 -> 13.2.
 // FLAT_EXTRA 24 / 36 / 48 (of the line): 16 x 8 421 / 422 / 424, 12 x 8 of 500-6000 - / 43.0 / 44.5, 64 x 1 - / 218 / 216.
-constexpr int FLAT_EXTRA = 36;
+// A tile of head_dim 256 is twice the work: with 18 there, 36 -> 18, 32 x 4 of 200-2000 43.4 -> 37.9, 16 x 8 of 1K-8K 125.0 -> 118.3, 20 x 8 of 200-3000 69.9 -> 63.1, 9 x 4 of 4K-30K 108.3 -> 106.5, 6 x 8
+// of 1K-16K (groups of 8) 81.3 -> 80.0, 8 x 4 of 1K-8K the same; 24 118 -> 120 and 63 -> 66, 14 up to 2.5 % slower in groups of 8.  FLAT_SLACK, what a piece of `single` may have beyond share, since the
+// line's pieces in the middle are dearer than share too: without it 16 x 8 of 2000 56.4 -> 58.7, with 18 12 x 4 of 2K-20K 104.4 -> 108.0.  At head_dim 128 42 in place of 36 and 21 for the slack: 64 x 1
+// slots 190.0 -> 187.7, 12 x 8 of 500-6000 38.8 -> 40.6, others the same: left.
+constexpr int FLAT_EXTRA = 36, FLAT_SLACK = 0, FLAT_EXTRA256 = 18, FLAT_SLACK256 = 9;
 constexpr int FLAT_ROWS = 2048, FLAT_SORT = ATT_THREADS, FLAT_WHOLE = 32;               // rows whose tiles are held while the plan is made; rows that are sorted; pairs of a CTA that are dealt out
 constexpr int FLAT_SCRATCH = 4 * (FLAT_ROWS + 2 * FLAT_SORT + 4 * ATT_WARPS);
 struct FlatWalk {
@@ -446,7 +450,7 @@ struct FlatWalk {
 __device__ __forceinline__ int tiles_in(int tokens) { return max((tokens + 15) >> 4, 0); }
 // Executed by the whole CTA; warp 0 gets the walk.  window: 64 words for flat_next;  scratch: FLAT_SCRATCH bytes that are free until the first piece begins;  least: tiles
 // of a piece of `single`, at least.
-template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B, int n_kv, int least, int* window, int* scratch, const F& tokens_of) {
+template <int EXTRA, int SLACK, class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B, int n_kv, int least, int* window, int* scratch, const F& tokens_of) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, ctas = gridDim.x, pairs = B * n_kv;
   int* const held = scratch;                          // the rows' tokens
   int* const order = held + FLAT_ROWS;
@@ -464,10 +468,10 @@ template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B,
   __syncthreads();
   const int w = lane & (ATT_WARPS - 1);
   sum = __reduce_add_sync(FULLM, lane < ATT_WARPS ? red[w] : 0u); longest = __reduce_max_sync(FULLM, red[ATT_WARPS + w]); shortest = __reduce_min_sync(FULLM, red[2 * ATT_WARPS + w]);
-  const u32 total = (u32)n_kv * (sum + (u32)(FLAT_EXTRA * B)), share = (total + ctas - 1) / ctas, most = share + FLAT_EXTRA;
+  const u32 total = (u32)n_kv * (sum + (u32)(EXTRA * B)), share = (total + ctas - 1) / ctas, most = share + EXTRA;
   f.row = f.kvh = f.at = f.tiles = f.tokens = 0; f.pair = -1;
   if (pairs <= ctas) {
-    const u32 lo = max((u32)least, ((u32)n_kv * sum + ctas - 1) / ctas), hi = max(lo, share), same = (u32)(ctas / pairs), even = (longest + same - 1) / same;
+    const u32 lo = max((u32)least, ((u32)n_kv * sum + ctas - 1) / ctas), hi = max(lo, share + SLACK), same = (u32)(ctas / pairs), even = (longest + same - 1) / same;
     f.share = 0;
     if (even <= min(hi, lo + 2 + lo / 16)) {           // rows of about one length, or so few tiles that nothing is left to gain: as many pieces of every pair
       if (warp != 0) return;
@@ -513,7 +517,7 @@ template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B,
     }
   } else {
     const int k = (pairs + ctas - 1) / ctas;
-    if (B <= FLAT_SORT && k <= FLAT_WHOLE && longest <= share && (u32)k * (FLAT_EXTRA + shortest) <= most && longest < 1u << 22) {
+    if (B <= FLAT_SORT && k <= FLAT_WHOLE && longest <= share && (u32)k * (EXTRA + shortest) <= most && longest < 1u << 22) {
       static_assert(FLAT_SORT <= 512, "nine bits of a key");
       const int mine = tid < B ? tiles_in(held[tid]) << 9 | (511 - tid) : -1;           // (no two alike)
       keys[tid] = mine;
@@ -530,7 +534,7 @@ template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B,
       for (int c = tid; c < ctas; c += ATT_THREADS) {
         u32 own = 0u;
         for (int i = 0; i < k; i++)
-          if (place(i, c) < pairs) own += FLAT_EXTRA + tiles_in(held[order[place(i, c) / n_kv]]);
+          if (place(i, c) < pairs) own += EXTRA + tiles_in(held[order[place(i, c) / n_kv]]);
         load = max(load, own);
       }
       load = __reduce_max_sync(FULLM, load);
@@ -554,7 +558,7 @@ template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B,
   u32 before = 0u;
   for (int r0 = 0; r0 < B && f.lo < f.hi; r0 += 32) {
     const int tokens = r0 + lane < B ? tokens_at(r0 + lane) : 0, t = tiles_in(tokens);
-    const u32 own = r0 + lane < B ? (u32)(n_kv * (FLAT_EXTRA + t)) : 0u;
+    const u32 own = r0 + lane < B ? (u32)(n_kv * (EXTRA + t)) : 0u;
     u32 inc = own;
     scan_step(inc, 1); scan_step(inc, 2); scan_step(inc, 4); scan_step(inc, 8); scan_step(inc, 16);
     const u32 past = __ballot_sync(FULLM, before + inc > (u32)f.lo);
@@ -562,8 +566,8 @@ template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B,
       const int l = __ffs((int)past) - 1;
       f.row = r0 + l; f.tiles = __shfl_sync(FULLM, t, l);
       const int row_at = (int)(before + __shfl_sync(FULLM, inc - own, l));
-      f.kvh = (f.lo - row_at) / (FLAT_EXTRA + f.tiles);
-      f.at = row_at + f.kvh * (FLAT_EXTRA + f.tiles);
+      f.kvh = (f.lo - row_at) / (EXTRA + f.tiles);
+      f.at = row_at + f.kvh * (EXTRA + f.tiles);
       window[lane] = tokens;
       __syncwarp();
       break;
@@ -572,7 +576,7 @@ template <class F> __device__ __forceinline__ void flat_plan(FlatWalk& f, int B,
   }
 }
 // The next piece, by the whole of warp 0.  On the line, window has the tokens of the 32 rows that the walk is among.
-template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int lane, int* window, const F& tokens_of) {
+template <int EXTRA, class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B, int n_kv, int lane, int* window, const F& tokens_of) {
   if (f.share <= 0) {
     if (f.at == 0) f.pair = -1;
     else if (--f.at, f.share < 0) { f.pair = window[f.at]; f.tokens = window[32 + f.at]; f.range[0] = 0; f.range[1] = tiles_in(f.tokens); f.split = 0; f.ns = 1; }
@@ -580,14 +584,14 @@ template <class F> __device__ __forceinline__ void flat_next(FlatWalk& f, int B,
   }
   f.pair = -1;
   while (f.row < B && f.pair < 0) {
-    const int first = f.at + FLAT_EXTRA - (f.tiles > 0 ? 0 : 1), last = first + max(f.tiles, 1) - 1;
+    const int first = f.at + EXTRA - (f.tiles > 0 ? 0 : 1), last = first + max(f.tiles, 1) - 1;
     if (first >= f.hi) return;
     if (last >= f.lo) {
       const int c0 = first / f.share;
       f.pair = f.row * n_kv + f.kvh; f.split = blockIdx.x - c0; f.ns = last / f.share - c0 + 1; f.tokens = window[f.row % 32];
       f.range[0] = f.tiles > 0 ? max(f.lo, first) - first : 0; f.range[1] = f.tiles > 0 ? min(f.hi - 1, last) - first + 1 - f.range[0] : 0;
     }
-    f.at += FLAT_EXTRA + f.tiles;
+    f.at += EXTRA + f.tiles;
     if (++f.kvh == n_kv) {
       f.kvh = 0;
       if (++f.row < B) {
@@ -701,7 +705,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   };
   if (FLAT) {
     FlatWalk f;
-    flat_plan(f, p.B, p.n_kv, 4, s_rows, reinterpret_cast<int*>(smem + TB_AREA), tokens_of);
+    flat_plan<FLAT_EXTRA, FLAT_SLACK>(f, p.B, p.n_kv, 4, s_rows, reinterpret_cast<int*>(smem + TB_AREA), tokens_of);
     if (tid == 0) s_flat = f;
     __syncwarp();
   }
@@ -710,7 +714,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     if (warp == 0) {
       FlatWalk f = s_flat;
       __syncwarp();
-      flat_next(f, p.B, p.n_kv, lane, s_rows, tokens_of);
+      flat_next<FLAT_EXTRA>(f, p.B, p.n_kv, lane, s_rows, tokens_of);
       if (lane == 0) { s_flat = f; s_split = f.split; s_ns = f.ns; }
     }
     __syncthreads();
@@ -1092,7 +1096,7 @@ constexpr int ATT256_SMEM = T256_RING + ATT_WARPS * WARP256_BYTES + 16;         
 static_assert(T256_BASES % 16 == 0 && T256_RING % 16 == 0 && T256_META % 16 == 0 && T256_CTL % 16 == 0 && ATT256_SMEM + 336 <= 232448, "one CTA per SM");
 
 static_assert(FLAT_SCRATCH <= ATT_WARPS * SEG256_BYTES, "planned in the segment areas");
-// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.1 -> 24.8 us (22.5 now), 20 x 8 of up to 3K 95 -> 73 (a grid, rows as they come; 70 now).  Pieces of two tiles on short rows: of four
+// FLAT: see FlatWalk; 8 rows x 4 kv heads of 1K-8K tokens 33.1 -> 24.8 us (22.5 now), 20 x 8 of up to 3K 95 -> 73 (a grid, rows as they come; 63 now).  Pieces of two tiles on short rows: of four
 // 0.5 us slower on 2 x 4 of 700.
 template <int NSET, bool FLAT>
 __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __grid_constant__ AttnParams p) {
@@ -1120,7 +1124,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   auto tokens_of = [&](int row) -> int { return p.seq_len[row]; };
   if (FLAT) {
     FlatWalk f;
-    flat_plan(f, p.B, p.n_kv, 2, s_rows, reinterpret_cast<int*>(smem + T256_SEG), tokens_of);
+    flat_plan<FLAT_EXTRA256, FLAT_SLACK256>(f, p.B, p.n_kv, 2, s_rows, reinterpret_cast<int*>(smem + T256_SEG), tokens_of);
     if (tid == 0) s_flat = f;
     __syncwarp();
   }
@@ -1130,7 +1134,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
     if (warp == 0) {
       FlatWalk f = s_flat;
       __syncwarp();
-      flat_next(f, p.B, p.n_kv, lane, s_rows, tokens_of);
+      flat_next<FLAT_EXTRA256>(f, p.B, p.n_kv, lane, s_rows, tokens_of);
       if (lane == 0) s_flat = f;
     }
     begin_ring();
