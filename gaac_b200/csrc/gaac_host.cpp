@@ -9,7 +9,8 @@
 //   gaac_store               an object with these fields (kv_cache._Store)
 //   gaac_paged               a tuple (buf, raw, mt, stack, top, err, b3k, b4k, b3v, b4v, n_kv, TS, ovf_slot)
 //   numbers                  as themselves
-// Nothing is kept between calls: every pointer is read from its tensor when the call is made.  The interpreter is let go for the duration of the library call, as ctypes does.
+// Nothing is kept between calls: every pointer is read from its tensor when the call is made.  The interpreter is let go for the duration of the library call, as ctypes does, and of an
+// allocation, as torch.empty does: either may wait for the GPU, whose queue may wait for what another thread has yet to launch.
 #include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
@@ -131,6 +132,13 @@ template <> struct Arg<const gaac_paged*> {
   operator const gaac_paged*() const { return &s; }
 };
 
+struct Released {                                    // the interpreter's lock, let go of, also by way of an exception
+  PyThreadState* const state = PyEval_SaveThread();
+  Released() = default;
+  ~Released() { PyEval_RestoreThread(state); }
+  Released(const Released&) = delete;
+};
+
 template <class F> PyObject* guarded(const F& f) {
   try { return f(); }
   catch (const Failed&) { return nullptr; }
@@ -141,11 +149,8 @@ template <class F> PyObject* guarded(const F& f) {
 template <class... A, size_t... I>
 PyObject* invoke(int (*fn)(A...), PyObject* const* args, std::index_sequence<I...>) {
   const std::tuple<Arg<A>...> a{Arg<A>(args[I])...};
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = fn(std::get<I>(a)...);
-  Py_END_ALLOW_THREADS
-  return PyLong_FromLong(rc);
+  const auto run = [&] { const Released released; return fn(std::get<I>(a)...); };
+  return PyLong_FromLong(run());
 }
 template <class... A>
 PyObject* call(int (*fn)(A...), const char* name, PyObject* const* args, Py_ssize_t n) {
@@ -180,7 +185,8 @@ PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
     int64_t size[4];
     for (Py_ssize_t i = 2; i < n; i++) size[i - 2] = whole(args[i]);
     auto options = at::TensorOptions().device(like.device()).dtype(kind == 0 ? at::kByte : kind == 1 ? at::kInt : kind == 2 ? at::kBFloat16 : like.scalar_type());
-    return THPVariable_Wrap(at::empty(at::IntArrayRef(size, (size_t)(n - 2)), options));
+    const auto make = [&] { const Released released; return at::empty(at::IntArrayRef(size, (size_t)(n - 2)), options); };
+    return THPVariable_Wrap(make());
   });
 }
 

@@ -1,5 +1,7 @@
 """The module that calls the library with tensors (csrc/gaac_host.cpp): the same answers as the ctypes binding to calls that the library refuses, and what its arguments may be.  Every call
 here is refused before memory is touched."""
+import sys
+import threading
 import types
 import pytest
 import torch
@@ -67,3 +69,30 @@ def test_empty():
     with pytest.raises(RuntimeError): H.empty(like, 0, -1)
     with pytest.raises(TypeError): H.empty(None, 0, 1)
     with pytest.raises(TypeError): H.empty(like, 0, 1, 1, 1, 1, 1)
+
+
+def test_other_threads_run_while_memory_is_allocated():
+    """The allocator may wait for a GPU, which may wait for another thread's launch.  With a switch interval that never ends a thread runs only where this one lets go of the interpreter."""
+    H, like = _lib.host(), torch.zeros(1)
+    ran, started, interval = [], threading.Event(), sys.getswitchinterval()
+    gate = threading.Lock()
+    gate.acquire()
+
+    def other():
+        started.set()
+        with gate: ran.append(1)
+
+    t = threading.Thread(target=other)
+    t.start()
+    started.wait()
+    sys.setswitchinterval(1000.0)
+    try:
+        gate.release()
+        kept = []                                    # (to free one lets go of the interpreter as well)
+        for _ in range(10000):
+            kept.append(H.empty(like, 0, 1 << 20))
+            if ran: break
+        assert ran
+    finally:
+        sys.setswitchinterval(interval)
+        t.join()
