@@ -144,7 +144,7 @@ class ContextSplitAttention:
                 if exchange == "p2p":
                     raise
         self.scale = scale if scale is not None else 128 ** -0.5
-        self.nsplit = nsplit or choose_nsplit_sm100(1, self.n_kv, max(kp.S, 1))
+        self.nsplit = nsplit or choose_nsplit_sm100(1, self.n_kv, max(kp.S, 1), teams=False)
         self.fused = fused and self.n_kv * self.nsplit <= SM_COUNT_B200
         self._part = torch.empty(n_q, 130, dtype=torch.float32, device=kp.sm.device)
 

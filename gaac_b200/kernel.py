@@ -50,7 +50,7 @@ def choose_nsplit(B: int, n_kv: int, S: int, target_ctas: int = 96, min_tok: int
 
 @functools.lru_cache(maxsize=4096)
 def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200, min_tiles_per_warp: int = 2, ragged: bool = False,
-                        total_tokens: int | None = None) -> int:
+                        total_tokens: int | None = None, teams: bool = True) -> int:
     """Splits per (row, kv head) for a B200.  The kernel runs one 16-warp CTA per SM.
 
     Equal lengths (S is every row's length): the split count minimises a cost model fitted to measurements,
@@ -84,7 +84,9 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     # splits, 13.3 in 32, 17.4 in 125.  A second wave costs more than it shortens (4 rows of 1000 in 6 splits: 15.3).
     # Up to eight ranges of a row are a team (clusters whose partials do not go through global memory), where all teams fit the GPU at a time; there three tiles are enough for a range, and ten tiles for
     # a second one: batch 1, 8 kv heads, 200 tokens 6.6 -> 6.3, 500 7.2 -> 6.1, 1000 7.8 (15 splits) -> 6.8, 1500 8.2 -> 7.4, 2000 8.0 -> 8.05;  2 rows: 500 8.4 (8 splits) -> 7.2 (6), 1000 9.0 (9) -> 8.0.
-    wave, team = sm_count // rows, _team(rows)
+    # teams=False: for launches that cannot be one, partials and exchanges.  There the ranges' partials go through global memory all the same: partials of 8 heads, 129 tokens 5.5 (one CTA), 7.1 in three
+    # ranges; 256 7.0 and 7.4 in five; 1500 7.6 in 16 and 8.2 in 8; 1700 7.6 and 8.8.
+    wave, team = sm_count // rows, _team(rows) if teams else 1
     if team > 1 and (8 if team >= 6 else ATT_WARPS) < ntiles <= 14 * team:         # (many rows of one CTA each: 32 x 1 of 200 tokens 8.4 -> 8.2 where they are that long, 5.3 -> 5.9 where that is a bound)
         return min(team, ntiles // 3)
     if wave > 1 and 4 * most <= 3 * wave:
@@ -193,7 +195,7 @@ def choose_nsplit256(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -
     tiles.  One wave of short ranges comes first; us, the counts made for 16 warps, or a flat launch, -> this, rows of hi / 8 to hi tokens (B x kv heads): 2 x 1 of 740 17.3 -> 8.9;  8 x 4 of 500 16.0 -> 10.8;
     5 x 8 of 740 20.9 -> 13.5;  2 x 4 of 4000 15.8 (flat) -> 13.7;  8 x 8 of 1100 20.8 (flat) -> 19.2;  1 x 1 of 300 10.2 -> 8.2.  Where ranges are longer a flat launch is as fast or faster (2 x 8 of
     4000, 28 tiles: 17.8 and 18;  8 x 4 of 2000, 31 tiles: 16.5 and 17)."""
-    return _splits256(B * n_kv, -(-S // 16), sm_count) or choose_nsplit_sm100(B, n_kv, S, ragged=True)
+    return _splits256(B * n_kv, -(-S // 16), sm_count) or choose_nsplit_sm100(B, n_kv, S, ragged=True, teams=False)
 
 
 def _flat_splits(B: int, n_kv: int, ctas: int) -> int:

@@ -78,3 +78,11 @@ def test_shard_heads():
         hs = [list(gd.shard_heads(n_kv, world, r)) for r in range(world)]
         assert sorted(h for x in hs for h in x) == list(range(n_kv))
         assert max(len(x) for x in hs) - min(len(x) for x in hs) <= 1
+
+
+@pytest.mark.parametrize("S,ranges", [(16, 1), (129, 1), (200, 1), (256, 1), (300, 4), (500, 8), (1000, 15), (1500, 16), (1700, 16), (2000, 16), (65536, 18)])
+def test_short_ranks_are_not_split_as_teams(S, ranges):
+    """Partials and exchanges go through global memory whatever the range count: 8 kv heads take the counts of launches without teams."""
+    import types
+    page = types.SimpleNamespace(H=8, S=S, sm=torch.zeros(1))
+    assert gd.ContextSplitAttention(page, page, 32).nsplit == ranges
