@@ -14,8 +14,7 @@ LIB = os.path.join(HERE, "libgaac_b200.so")
 SOURCES = ["gaac_encode.cu", "gaac_attn.cu", "gaac_cache.cu", "gaac_noalloc.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
-
-
+C_ABI = os.path.join(os.path.dirname(HERE), "include", "gaac_b200.h")
 HOST = os.path.join(HERE, "_host.so")
 
 
@@ -33,31 +32,49 @@ def _sources():
     return [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(HOST):
-        return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST))
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(os.path.dirname(HERE), "include", "gaac_b200.h")]
-    return any(os.path.getmtime(d) > t for d in deps)
+def _stale(made: str, sources) -> bool:
+    return not os.path.exists(made) or any(os.path.getmtime(d) > os.path.getmtime(made) for d in sources)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not _stale():
-        return LIB
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    objs = []
-    procs = [("gaac_host.cpp", subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True))]
-    for src in _sources():
-        obj = os.path.join("/tmp", "gaac_b200_" + os.path.basename(src) + ".o")
-        objs.append(obj)
-        procs.append((src, subprocess.Popen([nvcc, *NVCC_FLAGS, "-c", src, "-o", obj], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    for src, pr in procs:
+def _headers():
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))] + [C_ABI]
+
+
+def _start(name, command):
+    return name, subprocess.Popen(command, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
+def _finish(started, verbose: bool):
+    failed = None
+    for name, pr in started:
         out, _ = pr.communicate()
         if verbose or pr.returncode:
             print(out)
         if pr.returncode:
-            raise RuntimeError(f"the compiler failed on {src}")
-    subprocess.check_call([nvcc, "-shared", "-o", LIB, *objs, "-lcudart"])
+            failed = failed or name
+    if failed:
+        raise RuntimeError(f"the compiler failed on {failed}")
+
+
+def _start_host(force: bool):
+    """The module's compiler at work, or nothing: up to date, or there is no torch or no C++ compiler here.  The library, which callers of the C ABI need alone, does without either."""
+    if not force and not _stale(HOST, [os.path.join(CSRC, "gaac_host.cpp"), C_ABI]):
+        return []
+    try:
+        return [_start("gaac_host.cpp", _host_command())]
+    except (ImportError, FileNotFoundError) as e:
+        print(f"{os.path.basename(HOST)}, through which the Python package calls the library, is not built: {e}", file=sys.stderr)
+        return []
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    host = _start_host(force)
+    if force or _stale(LIB, [*_sources(), *_headers()]):
+        nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+        objs = [os.path.join("/tmp", "gaac_b200_" + os.path.basename(src) + ".o") for src in _sources()]
+        _finish([_start(src, [nvcc, *NVCC_FLAGS, "-c", src, "-o", obj]) for src, obj in zip(_sources(), objs)], verbose)
+        subprocess.check_call([nvcc, "-shared", "-o", LIB, *objs, "-lcudart"])
+    _finish(host, verbose)
     return LIB
 
 
