@@ -50,7 +50,7 @@ def choose_nsplit(B: int, n_kv: int, S: int, target_ctas: int = 96, min_tok: int
 
 @functools.lru_cache(maxsize=4096)
 def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200, min_tiles_per_warp: int = 2, ragged: bool = False,
-                        total_tokens: int | None = None, teams: bool = True) -> int:
+                        total_tokens: int | None = None, teams: bool = True, bound: bool = False) -> int:
     """Splits per (row, kv head) for a B200.  The kernel runs one 16-warp CTA per SM.
 
     Equal lengths (S is every row's length): the split count minimises a cost model fitted to measurements,
@@ -82,12 +82,16 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     # faster; beyond, splits pay down to four tiles each until there are 16 (one per warp of the merge), more only with 16 tiles each.  Batch 1, 8
     # kv heads: 500 tokens 10.8 -> 8.4 us, 1000: 18.1 -> 8.3, 2000: 15.6 -> 8.8; 4 rows of 1000: 18.6 -> 9.9; 1 kv head, 8000 tokens: 16.3 in 15
     # splits, 13.3 in 32, 17.4 in 125.  A second wave costs more than it shortens (4 rows of 1000 in 6 splits: 15.3).
-    # Up to eight ranges of a row are a team (clusters whose partials do not go through global memory), where all teams fit the GPU at a time; there three tiles are enough for a range, and ten tiles for
-    # a second one: batch 1, 8 kv heads, 200 tokens 6.6 -> 6.3, 500 7.2 -> 6.1, 1000 7.8 (15 splits) -> 6.8, 1500 8.2 -> 7.4, 2000 8.0 -> 8.05;  2 rows: 500 8.4 (8 splits) -> 7.2 (6), 1000 9.0 (9) -> 8.0.
+    # Up to eight ranges of a row are a team (clusters whose partials do not go through global memory), where all teams fit the GPU at a time; there three tiles are enough for a range, and 13 tiles for
+    # a second one: batch 1, 8 kv heads, 250 tokens 6.7 -> 6.1, 500 7.2 -> 6.1, 1000 7.8 (15 splits) -> 6.8, 1500 8.2 -> 7.4, 2000 8.0 -> 8.05;  2 rows: 500 8.4 (8 splits) -> 7.2 (6), 1000 9.0 (9) -> 8.0;
+    # ten tiles, in three ranges, 5.7 -> 6.2, and 6.8 -> 7.6 with groups of 8.
+    # bound=True: S is no more than a bound, the lengths are read on the GPU, where a row of up to 16 tiles takes one CTA whatever the count (fewer_ranges in gaac_attn.cu), and a cluster with
+    # nothing to merge costs 0.2 to 0.6 us: 8 kv heads, slots, 12 tiles 6.3 (one CTA), 6.8 (a team), paged 16 tiles 6.9 and 7.4.  The same is lost where the bound is longer and the rows are not (40 x 1
+    # of 7 tiles in a table of 28 5.9 -> 6.1), against 7.1 for 9.4 where they are.
     # teams=False: for launches that cannot be one, partials and exchanges.  There the ranges' partials go through global memory all the same: partials of 8 heads, 129 tokens 5.5 (one CTA), 7.1 in three
     # ranges; 256 7.0 and 7.4 in five; 1500 7.6 in 16 and 8.2 in 8; 1700 7.6 and 8.8.
     wave, team = sm_count // rows, _team(rows) if teams else 1
-    if team > 1 and (8 if team >= 6 else ATT_WARPS) < ntiles <= 14 * team:         # (many rows of one CTA each: 32 x 1 of 200 tokens 8.4 -> 8.2 where they are that long, 5.3 -> 5.9 where that is a bound)
+    if team > 1 and (ATT_WARPS if bound or team < 6 else 12) < ntiles <= 14 * team:         # (many rows of one CTA each: 32 x 1 of 200 tokens 8.4 -> 8.2 where they are that long, 5.3 -> 5.9 where that is a bound)
         return min(team, ntiles // 3)
     if wave > 1 and 4 * most <= 3 * wave:
         return 1 if ntiles <= ATT_WARPS else min(wave, max(min(16, ntiles // 4), -(-ntiles // 16)))

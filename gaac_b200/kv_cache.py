@@ -245,7 +245,7 @@ class CompressedKVCache:
         units = choose_units(B, self.n_kv, max_len or self.cap) if nsplit is None else 0
         flat = 0
         if nsplit is None:
-            if not units: nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap)
+            if not units: nsplit = choose_nsplit_sm100(B, self.n_kv, max_len or self.cap, bound=True)
             flat = choose_flat(B, self.n_kv, max_len or self.cap, nsplit or 0, units, q.shape[1] // self.n_kv, self.cap)
         K, V = self.k, self.v
         out = _ext().gaac_attn_launch(K.sm, K.codes, K.flags, K.tile_off, K.ovf, K.head_start, K.base3, K.base4,

@@ -31,7 +31,7 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     units = flat = 0
     if nsplit is None:
         units = choose_units(B, n_kv, bt.shape[1] * 16)
-        nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True)        # with units: what the workspace must have room for
+        nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True, bound=True)        # with units: what the workspace must have room for
         flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv, bt_stride * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)
     st = (buf, raw, mt, None, None, None, *bases, n_kv, TS, TS - 2880)

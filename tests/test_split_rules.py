@@ -1,0 +1,46 @@
+"""Split counts where the rows' lengths are known, and where the caller has no more than a bound on them: the rules, and what the calls hand to the library."""
+import types
+import pytest
+from gaac_b200.kernel import choose_nsplit_sm100
+
+
+class _Tensor:
+    """What the calls ask a tensor for before the library is called."""
+    def __init__(self, *shape): self.shape, self.device, self.is_cuda = shape, types.SimpleNamespace(type="cuda", index=0), True
+    def size(self, i): return self.shape[i]
+    def stride(self, i): return self.shape[-1] if i == 0 else 1
+    def numel(self): return 1 << 20
+    def data_ptr(self): return 0
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """The calls that reach the native module: (name, arguments)."""
+    from gaac_b200 import _lib, kernel
+    from gaac_b200.vllm import paged_kernel, paged_kernel256
+    made = []
+
+    class Recording:
+        def __getattr__(self, name): return lambda *a: made.append((name, a)) or 0
+    monkeypatch.setattr(_lib, "host", Recording)
+    monkeypatch.setattr(_lib, "stream_ptr", lambda dev: 0)
+    for module in (kernel, paged_kernel, paged_kernel256): monkeypatch.setattr(module, "workspace", lambda *a: _Tensor(1))
+    return made
+
+
+def _paged(calls, B, n_kv, G, blocks, wide=False, bases=(1, 2, 3, 4)):
+    from gaac_b200.vllm.paged_kernel import paged_attention
+    from gaac_b200.vllm.paged_kernel256 import paged_attention256
+    call = paged_attention256 if wide else paged_attention
+    call(_Tensor(B, n_kv * G, 256 if wide else 128), "out", "buf", "raw", "mt", _Tensor(B, blocks), "seq_lens", bases, 3008, n_kv * G, n_kv)
+    return calls.pop()
+
+
+@pytest.mark.parametrize("tiles", [1, 9, 10, 12, 13, 16, 17, 28])
+@pytest.mark.parametrize("B,n_kv", [(1, 1), (1, 8), (2, 8), (9, 2), (40, 1)])
+def test_rows_of_one_cta_are_no_teams(calls, B, n_kv, tiles):
+    """Up to 16 tiles a row takes one CTA wherever its length is read on the GPU: a count above one would only make a cluster of it."""
+    name, a = _paged(calls, B, n_kv, 4, tiles)
+    assert name == "gaac_paged_decode_attn" and (a[8] == 1) == (tiles <= 16)
+    assert (choose_nsplit_sm100(B, n_kv, 16 * tiles, bound=True) == 1) == (tiles <= 16)
+    if B * n_kv <= 22: assert (choose_nsplit_sm100(B, n_kv, 16 * tiles) == 1) == (tiles <= 12)              # lengths known
