@@ -609,12 +609,12 @@ template <int EXTRA, class F> __device__ __forceinline__ void flat_next(FlatWalk
 static_assert(FLAT_SCRATCH <= ATT_WARPS * AREA_BYTES, "planned in the segment areas");
 
 // Ranges of a row of a grid, where its length is only known here: the caller goes by a bound on the rows' lengths, the width of a block table or a capacity, and its split count (ns, the most there
-// may be) may be far too large for the rows that there are.  A row that fits the warps of one CTA (`at_once` tiles) is not split;  beyond, ranges go down to four tiles until there are 16 of them (24 at
-// head_dim 256, whose CTAs work on eight tiles at a time), then down to a tile per warp.  CTAs that get none leave before they load anything.  So the callers' rules may fill one wave: in a table of 2048
-// tokens 4 x 4 rows of 53 took 9.8 us in nine ranges each, 7.0 by shares of units and take 6.5 now;  in one of 8192 at head_dim 256 a row of 2000 17.5 in 128 ranges, now 10.1.
-__device__ __forceinline__ void fewer_ranges(int tiles, int at_once, int& ns, int& chunk) {
-  if (tiles <= at_once) { ns = 1; chunk = tiles; return; }
-  const int least = max(4, min(at_once, at_once == 16 ? (tiles + 15) >> 4 : tiles / 24));
+// may be) may be far too large for the rows that there are.  A row of up to `one` tiles is not split;  beyond, ranges go down to four tiles until there are 16 of them (24 at head_dim 256, whose CTAs
+// work on eight tiles at a time), then down to a tile per warp (`turn`: tiles that a CTA works on at a time).  CTAs that get none leave before they load anything.  So the callers' rules may fill one
+// wave: in a table of 2048 tokens 4 x 4 rows of 53 took 9.8 us in nine ranges each, 7.0 by shares of units and take 6.5 now;  in one of 8192 at head_dim 256 a row of 2000 17.5 in 128 ranges, now 10.1.
+__device__ __forceinline__ void fewer_ranges(int tiles, int one, int turn, int& ns, int& chunk) {
+  if (tiles <= one) { ns = 1; chunk = tiles; return; }
+  const int least = max(4, min(turn, turn == ATT_WARPS ? (tiles + 15) >> 4 : tiles / 24));
   if (chunk >= least) return;
   ns = (tiles + least - 1) / least;
   chunk = (tiles + ns - 1) / ns;                     // (as sum_exact takes it)
@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   const int ntiles = (S + 15) >> 4;
   int chunk = ROWS && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
   if (ROWS && p.nsplit > 1) {
-    if (PAGED || p.seq_len) { fewer_ranges(ntiles, ATT_WARPS, ns0, chunk); if (split0 >= ns0) return; }
+    if (PAGED || p.seq_len) { fewer_ranges(ntiles, ATT_WARPS, ATT_WARPS, ns0, chunk); if (split0 >= ns0) return; }
     if (tid == 0) s_ns = ns0;
   }
   const int tlo = FLAT ? min(__shfl_sync(FULLM, s_flat.range[0], 0), ntiles) : min(split0 * chunk, ntiles);
@@ -1164,7 +1164,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) paged256_attn_kernel(const __g
   const int ntiles = (S + 15) >> 4;
   int chunk = (ntiles + NS - 1) / NS;
   if (!FLAT) {
-    if (p.nsplit > 1) fewer_ranges(ntiles, ATT_WARPS / 2, NS, chunk);
+    // (the merge of groups of 5 to 8 is dearer: rows of 9 or 10 tiles, of a table of 36 or 40, 10.6 us in one CTA, 12.3 in ranges of four tiles;  two ranges pay from 24 tiles on)
+    if (p.nsplit > 1) fewer_ranges(ntiles, NSET == 1 ? ATT_WARPS / 2 : p.nsplit == 2 ? 24 : 16, ATT_WARPS / 2, NS, chunk);
     if (split >= NS) return;
     if (tid == 0) s_ns = NS;
   }

@@ -175,31 +175,36 @@ def choose_flat(B: int, n_kv: int, S: int, nsplit: int, units: int, group: int =
 
 
 @functools.lru_cache(maxsize=4096)
-def choose_flat256(B: int, n_kv: int, S: int, most: int = 0, sm_count: int = SM_COUNT_B200) -> int:
+def choose_flat256(B: int, n_kv: int, S: int, most: int = 0, sm_count: int = SM_COUNT_B200, group: int = 4) -> int:
     """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.1 -> 24.8;  20 x 8, up to 3K 95 -> 73;  32 x 2, up
     to 4K 56 -> 40;  6 x 2, up to 60K 124 -> 93;  8 x 4, 100-700 22.0 -> 13.2;  2 x 8 of 1000 30 -> 13;  9 x 4, up to 1500 23.8 -> 16.6;  30 x 4, up to 2K 55 -> 48;  32 x 4, up to 1000 30.7 -> 31.4,
     in a table of 8192 43 -> 31;  32 x 8 the same 53 -> 40, 65 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.3 -> 47.6;  so are a few very short ones: 4 x 4 of 50-300 in a
     table of 8192 9.4 -> 11.0;  one sequence has nothing to gain: 1 x 4 of 8K 17.9 -> 18.4.  More rows than SMs, 32 x 8: up to 500 22.1 -> 23.4, up to 740 35.5 -> 33.6, up to 1100 53.0 -> 44.4."""
     rows, tiles = B * n_kv, -(-S // 16)
-    if B <= 1 or not _flat_line(rows, max(S, most)) or _splits256(rows, tiles, sm_count):
+    if B <= 1 or not _flat_line(rows, max(S, most)) or _splits256(rows, tiles, group, sm_count):
         return 0
     return sm_count if tiles >= (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 64) else 0
 
 
-def _splits256(rows: int, tiles: int, sm_count: int = SM_COUNT_B200) -> int:
-    """Splits of one wave in which every row is split alike, where that leaves a CTA at most three tiles per pair of its warps, or 0."""
+def _splits256(rows: int, tiles: int, group: int = 4, sm_count: int = SM_COUNT_B200) -> int:
+    """Splits of one wave in which every row is split alike, where that leaves a CTA at most three tiles per pair of its warps, or 0.  Ranges of four tiles until there are 16 of them, then of
+    eight (a tile per pair) until there are 32: us, one row, groups of 4 and 8, by the number of ranges:  70 tiles 16: 9.9 and 13.7, 17: 10.4 and 14.3;  150 tiles 16: 12.5 and 16.3, 19: 11.5 and 15.1,
+    37: 11.5 and 15.6;  250 tiles 32: 12.2 and 16.0, 62: 12.5 and 16.2;  600 tiles 32: 17.0 and 21.1, 74: 18.8 and 25.6.  More than 16 want to save a turn of the pairs: 8 heads x 150 tiles 16: 13.1 and
+    16.7, 18: 13.3 and 17.3.  With groups of 5 to 8 the merge is dearer: 16 tiles stay in one CTA (27 x 2 of 10 tiles 11.3, in two ranges 12.8;  1 x 8 of 9 10.7, in three 12.4;  40 x 1 of 18 14.4
+    and 13.3), 24 where a row could only have two (27 x 2 of 18 tiles 14.4 and 15.5, of 28 17.9 and 16.5)."""
     wave = sm_count // rows if rows <= sm_count else 1
-    ns = min(wave, max(1, min(8, tiles // 3), tiles // 4))
+    ns = min(wave, max(1, min(8, tiles // 3), min(16, tiles // 4), min(32, -(-tiles // 8))))
+    if 16 < ns and 8 * ns < tiles <= 256: ns = 16
+    if tiles <= (8 if group <= 4 else 24 if ns == 2 else 16): ns = 1               # (as fewer_ranges in gaac_attn.cu)
     return ns if wave > 1 and tiles <= 24 * ns else 0
 
 
 @functools.lru_cache(maxsize=4096)
-def choose_nsplit256(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200) -> int:
+def choose_nsplit256(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200, group: int = 4) -> int:
     """Splits per (row, kv head) at head_dim 256, whose CTAs work on eight tiles at a time.  S may be a bound far above the rows' lengths: the kernel takes fewer ranges for a row of few
     tiles.  One wave of short ranges comes first; us, the counts made for 16 warps, or a flat launch, -> this, rows of hi / 8 to hi tokens (B x kv heads): 2 x 1 of 740 17.3 -> 8.9;  8 x 4 of 500 16.0 -> 10.8;
-    5 x 8 of 740 20.9 -> 13.5;  2 x 4 of 4000 15.8 (flat) -> 13.7;  8 x 8 of 1100 20.8 (flat) -> 19.2;  1 x 1 of 300 10.2 -> 8.2.  Where ranges are longer a flat launch is as fast or faster (2 x 8 of
-    4000, 28 tiles: 17.8 and 18;  8 x 4 of 2000, 31 tiles: 16.5 and 17)."""
-    return _splits256(B * n_kv, -(-S // 16), sm_count) or choose_nsplit_sm100(B, n_kv, S, ragged=True, teams=False)
+    5 x 8 of 740 20.9 -> 13.5;  2 x 4 of 4000 15.8 (flat) -> 13.7;  8 x 8 of 1100 20.8 (flat) -> 19.2;  1 x 1 of 300 10.2 -> 8.2."""
+    return _splits256(B * n_kv, -(-S // 16), group, sm_count) or choose_nsplit_sm100(B, n_kv, S, ragged=True, teams=False)
 
 
 def _flat_splits(B: int, n_kv: int, ctas: int) -> int:

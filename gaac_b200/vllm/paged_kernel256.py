@@ -9,7 +9,7 @@ dimensions of its half of V.
 from __future__ import annotations
 import torch
 from .. import _lib
-from ..kernel import workspace, choose_flat256, choose_nsplit256, _flat_splits
+from ..kernel import SM_COUNT_B200, workspace, choose_flat256, choose_nsplit256, _flat_splits
 
 
 def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, nsplit=None, scale=None, out_f32=None):
@@ -25,8 +25,8 @@ def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv,
     bt_stride = _lib.row_stride(bt)
     flat = 0
     if nsplit is None:
-        nsplit = choose_nsplit256(B, n_kv, bt.shape[1] * 16)
-        flat = choose_flat256(B, n_kv, bt.shape[1] * 16, bt_stride * 16)
+        nsplit = choose_nsplit256(B, n_kv, bt.shape[1] * 16, group=G)
+        flat = choose_flat256(B, n_kv, bt.shape[1] * 16, bt_stride * 16, SM_COUNT_B200, G)
         if flat: nsplit = _flat_splits(B, n_kv, flat)                                          # what the workspace must have room for
     st = (buf, raw, mt, None, None, None, *bases, 2 * n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)

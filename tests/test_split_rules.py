@@ -1,7 +1,7 @@
 """Split counts where the rows' lengths are known, and where the caller has no more than a bound on them: the rules, and what the calls hand to the library."""
 import types
 import pytest
-from gaac_b200.kernel import choose_nsplit_sm100
+from gaac_b200.kernel import choose_nsplit256, choose_nsplit_sm100
 
 
 class _Tensor:
@@ -44,3 +44,11 @@ def test_rows_of_one_cta_are_no_teams(calls, B, n_kv, tiles):
     assert name == "gaac_paged_decode_attn" and (a[8] == 1) == (tiles <= 16)
     assert (choose_nsplit_sm100(B, n_kv, 16 * tiles, bound=True) == 1) == (tiles <= 16)
     if B * n_kv <= 22: assert (choose_nsplit_sm100(B, n_kv, 16 * tiles) == 1) == (tiles <= 12)              # lengths known
+
+
+@pytest.mark.parametrize("B,n_kv,tiles,G,splits", [
+    (1, 8, 8, 4, 1), (1, 8, 9, 4, 3), (1, 8, 9, 8, 1), (1, 8, 16, 8, 1), (1, 8, 17, 8, 5), (27, 2, 18, 4, 2), (27, 2, 18, 8, 1), (27, 2, 25, 8, 2), (40, 1, 18, 8, 3),
+    (1, 1, 64, 4, 16), (1, 1, 70, 4, 16), (1, 1, 128, 4, 16), (1, 1, 150, 4, 19), (1, 8, 150, 4, 16), (1, 4, 250, 8, 32), (1, 8, 256, 8, 16), (1, 8, 400, 8, 18), (1, 2, 600, 4, 32), (1, 1, 5000, 4, 143)])
+def test_counts_of_head_dim_256(calls, B, n_kv, tiles, G, splits):
+    name, a = _paged(calls, B, n_kv, G, tiles, wide=True)
+    assert name == "gaac_paged_decode_attn256" and a[8] == splits == choose_nsplit256(B, n_kv, 16 * tiles, group=G)
