@@ -179,11 +179,16 @@ def choose_flat256(B: int, n_kv: int, S: int, most: int = 0, sm_count: int = SM_
     """The same for head_dim 256, whose grid hands the rows out as they come.  us, grid -> flat: 8 rows x 4 kv heads, 1K-8K tokens 33.1 -> 24.8;  20 x 8, up to 3K 95 -> 73;  32 x 2, up
     to 4K 56 -> 40;  6 x 2, up to 60K 124 -> 93;  8 x 4, 100-700 22.0 -> 13.2;  2 x 8 of 1000 30 -> 13;  9 x 4, up to 1500 23.8 -> 16.6;  30 x 4, up to 2K 55 -> 48;  32 x 4, up to 1000 30.7 -> 31.4,
     in a table of 8192 43 -> 31;  32 x 8 the same 53 -> 40, 65 -> 40.  A full wave of equal rows is the grid's: 12 x 4 of 4000 45.3 -> 47.6;  so are a few very short ones: 4 x 4 of 50-300 in a
-    table of 8192 9.4 -> 11.0;  one sequence has nothing to gain: 1 x 4 of 8K 17.9 -> 18.4.  More rows than SMs, 32 x 8: up to 500 22.1 -> 23.4, up to 740 35.5 -> 33.6, up to 1100 53.0 -> 44.4."""
+    table of 8192 9.4 -> 11.0;  one sequence has nothing to gain: 1 x 4 of 8K 17.9 -> 18.4.
+    More rows than SMs: from 160 tiles on, since rows much shorter than the table pay for the plan and for dearer pieces.  20 x 8 in a table of 72 tiles, rows of 18 23.1 -> 23.9 (groups of 8 26.9 ->
+    31.2), of 2-18 12.7 -> 14.6;  of 112, rows of 3-28 16.0 -> 17.9;  of 144, rows of 5-36 21.6 -> 20.8;  what rows as long as such a table would gain (70 tiles each 65 -> 47, 9-70 38.5 -> 34.5) is left.
+    A wave of equal ranges (_splits256) comes first where a CTA gets no more than 24 tiles, or 16 with groups of up to 4, whose ragged rows are better off by shares: 27 x 2 of 6-48 tiles, two ranges
+    each, 16.6, flat 15.2;  40 x 1 of 9-70 in three 16.5 and 15.3;  5 x 4 of 19-150 in seven 16.6 and 15.9;  groups of 8 20.1 and 19.9, 19.9 and 19.7, 20.4 and 20.5."""
     rows, tiles = B * n_kv, -(-S // 16)
-    if B <= 1 or not _flat_line(rows, max(S, most)) or _splits256(rows, tiles, group, sm_count):
+    if B <= 1 or not _flat_line(rows, max(S, most)) or tiles < (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 160):
         return 0
-    return sm_count if tiles >= (48 if 2 * rows <= sm_count else 96 if rows <= sm_count else 64) else 0
+    ns = _splits256(rows, tiles, group, sm_count)
+    return 0 if ns and tiles <= (16 if group <= 4 else 24) * ns else sm_count
 
 
 def _splits256(rows: int, tiles: int, group: int = 4, sm_count: int = SM_COUNT_B200) -> int:

@@ -1,7 +1,7 @@
 """Split counts where the rows' lengths are known, and where the caller has no more than a bound on them: the rules, and what the calls hand to the library."""
 import types
 import pytest
-from gaac_b200.kernel import choose_nsplit256, choose_nsplit_sm100
+from gaac_b200.kernel import choose_flat256, choose_nsplit256, choose_nsplit_sm100
 
 
 class _Tensor:
@@ -52,3 +52,10 @@ def test_rows_of_one_cta_are_no_teams(calls, B, n_kv, tiles):
 def test_counts_of_head_dim_256(calls, B, n_kv, tiles, G, splits):
     name, a = _paged(calls, B, n_kv, G, tiles, wide=True)
     assert name == "gaac_paged_decode_attn256" and a[8] == splits == choose_nsplit256(B, n_kv, 16 * tiles, group=G)
+
+
+@pytest.mark.parametrize("B,n_kv,tiles,G,flat", [(20, 8, 70, 4, False), (20, 8, 159, 8, False), (20, 8, 160, 4, True), (27, 2, 47, 4, False), (27, 2, 48, 4, True), (27, 2, 48, 8, False), (27, 2, 49, 8, True),
+                                                 (2, 1, 600, 4, True), (2, 1, 600, 8, False), (16, 2, 64, 4, False), (16, 2, 65, 4, True), (1, 8, 600, 4, False)])
+def test_flat_launches_of_head_dim_256(calls, B, n_kv, tiles, G, flat):
+    name, a = _paged(calls, B, n_kv, G, tiles, wide=True)
+    assert (name == "gaac_paged_decode_attn256_flat") == flat == (choose_flat256(B, n_kv, 16 * tiles, group=G) > 0)
