@@ -619,9 +619,10 @@ __device__ __forceinline__ void fewer_ranges(int tiles, int one, int turn, int& 
   ns = (tiles + least - 1) / least;
   chunk = (tiles + ns - 1) / ns;                     // (as sum_exact takes it)
 }
-// How the rows are shared out.  GRID: (row, kv head) x splits;  SHARED: a balanced launch;  FLAT_LINE: above.  Instantiations of their own: the shares cost the others
-// registers that the main loop has none of, 1.5 % at 64K tokens.
-enum { GRID, SHARED, FLAT_LINE, TEAM };
+// How the rows are shared out.  GRID: (row, kv head) x splits;  BOUND: the same with fewer_ranges;  TEAM: below;  SHARED: a balanced launch;  FLAT_LINE: above.  Instantiations of their own: the
+// shares cost the others registers that the main loop has none of, 1.5 % at 64K tokens, and fewer_ranges costs rows of one to five tiles in several waves, which have one range each, 0.08 us a wave
+// (paged 128 x 4 of 30-60 tokens 22.8 -> 22.4, 64 x 8 of 16-80 22.3 -> 21.9, 512 x 8 of 1-80 151 -> 149).
+enum { GRID, SHARED, FLAT_LINE, TEAM, BOUND };
 // ---- teams: the ranges of a row as one cluster, at most eight CTAs (the portable size), whose partials meet in the shared memory of the first.  Through global memory they take a fence
 // until the partials have arrived there, an atomic, and a load of each back, 1.7 us of a launch of 7; through distributed shared memory 0.7: 8 heads x 500 tokens 7.2 -> 6.1 us in a graph.  The others
 // store into the first CTA and leave; it has said, ahead of its main loop, that the place is free, which is in the stages that a range of at most TEAM_TILES tiles does not reach.  Longer ranges, found out
@@ -636,7 +637,7 @@ __device__ __forceinline__ void cluster_store(u32 at, float v) { asm volatile("s
 
 template <bool PAGED, bool DUMP, int NSET, int MODE>
 __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __grid_constant__ AttnParams p) {
-  constexpr bool SHARE = MODE == SHARED, FLAT = MODE == FLAT_LINE, ROWS = MODE == GRID || MODE == TEAM;
+  constexpr bool SHARE = MODE == SHARED, FLAT = MODE == FLAT_LINE, ROWS = MODE == GRID || MODE == TEAM || MODE == BOUND;
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_next, s_last, s_split, s_ns, s_tail, s_esc[6];
   __shared__ int s_team;        // (from s_split on: not needed inside the main loop, whose registers are all taken)
@@ -743,7 +744,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   S = __shfl_sync(FULLM, S, 0); ch = __shfl_sync(FULLM, ch, 0); TL = __shfl_sync(FULLM, TL, 0);
   const int ntiles = (S + 15) >> 4;
   int chunk = ROWS && !PAGED && !p.seq_len ? chunk_all : (ntiles + ns0 - 1) / ns0;
-  if (ROWS && p.nsplit > 1) {
+  if (MODE == TEAM || MODE == BOUND) {
     if (PAGED || p.seq_len) { fewer_ranges(ntiles, ATT_WARPS, ATT_WARPS, ns0, chunk); if (split0 >= ns0) return; }
     if (tid == 0) s_ns = ns0;
   }
@@ -934,7 +935,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
     }
     it = nx;
   }
-  const int split = SHARE || FLAT ? s_split : split0, NS = ROWS && p.nsplit == 1 ? 1 : s_ns;
+  const int split = SHARE || FLAT ? s_split : split0, NS = MODE == GRID ? p.nsplit : s_ns;
   if (FLAT) { bh = __shfl_sync(FULLM, s_flat.pair, 0); b = bh / p.n_kv; kvh = bh % p.n_kv; TL = __shfl_sync(FULLM, s_tail, 0); }
   // ---- slot layout: the raw BF16 tail belongs to the last split's last warp
   if (!PAGED && TL > 0 && split == NS - 1 && warp == ATT_WARPS - 1) {
@@ -1487,6 +1488,7 @@ static int launch_attn(const AttnParams& p, cudaStream_t st) {
   if (!DUMP && p.flat) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, FLAT_LINE>(p, st) : launch_attn_as<PAGED, false, 2, FLAT_LINE>(p, st);
   if (!DUMP && p.units) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, SHARED>(p, st) : launch_attn_as<PAGED, false, 2, SHARED>(p, st);
   if (!DUMP && team_ok<PAGED>(p)) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, TEAM>(p, st) : launch_attn_as<PAGED, false, 2, TEAM>(p, st);
+  if (!DUMP && p.nsplit > 1 && (PAGED || p.seq_len)) return p.G <= 4 ? launch_attn_as<PAGED, false, 1, BOUND>(p, st) : launch_attn_as<PAGED, false, 2, BOUND>(p, st);
   return p.G <= 4 ? launch_attn_as<PAGED, DUMP, 1, GRID>(p, st) : launch_attn_as<PAGED, DUMP, 2, GRID>(p, st);
 }
 
