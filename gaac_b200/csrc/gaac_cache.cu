@@ -209,9 +209,9 @@ __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restric
 
 // One warp per (entry, tile slot); the CTA's four entries have the slot index t = 2*kvh + kind in common, and with it the tables.
 // grid = (ceil(P / 4), 2*n_kv).
-// Bound by its chain of loads (entry, tile, escape bytes behind the tags, then the stores): the first two are asked for before the tables are made.  The tile's place in the block buffer is known
-// without the mode table, whose entry travels with it and says whether it counts (1500 tokens behind 6144: 18.6 -> 18.15 us in a graph; a raw tile's slot is read for nothing).  384
-// blocks of 16 tiles decoded and 1500 tokens stored: 24.7 -> 24.6 us.  128 bytes of the slot's escape bytes asked for with the tile: 19.0 -> 18.1 with everything in L2,
+// Bound by its chain of loads (entry, mode table, tile, escape bytes behind the tags, then the stores): the first three are asked for before the tables are made.  The tile's place is known without the
+// mode table, but asked for together with its entry a raw tile's slot is read for nothing: two states in turn, 384 blocks of 16 tiles 9.7 -> 9.4 us, with one block in ten raw 12.1 -> 12.3, all of them
+// 12.6 -> 17.4;  2048 blocks 43.0 -> 42.2, 47.7 -> 48.3 and 56.2 -> 66.2.  384 blocks decoded and 1500 tokens stored: 24.7 -> 24.6 us.  128 bytes of the slot's escape bytes asked for with the tile: 19.0 -> 18.1 with everything in L2,
 // but 24.4 and nothing gained from memory, where most of them are not the tile's.  9 CTAs per SM (56 registers, no spills): with 7 (72 registers) the chunk takes 20.9 us, now 20.0, and one behind 32768
 // tokens 57.7, now 54.4;  8 20.4 and 55.1;  10 (spills) 22.8 and 67.  All of these with the same blocks again and again, out of L2: where no earlier pass has touched them, the whole chunk (with
 // the overlapped launches 24.6 -> 20.4) gains about 1 %.
@@ -233,7 +233,7 @@ __device__ __forceinline__ void decode_blocks_cta(uint8_t* scratch, DecodeTables
     const long pt = (long)p.pairs[3 * e] * NT + t;
     const uint8_t* base = st.buf + pt * st.TS;
     m = st.mt[pt];
-    load_tile_words<KIND_V>(tw, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, base + SLOT_OVF_OFF, 0, lane);          // (its place does not depend on the mode table)
+    if (m >= 0) load_tile_words<KIND_V>(tw, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, base + SLOT_OVF_OFF, 0, lane);
   }
   const u32 w = fill_decode_tables<KIND_V>(tables, (KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D);
   __syncthreads();
