@@ -105,7 +105,8 @@ __device__ __forceinline__ void push_raw_tile(int* stack, int* top, int r) {
 // One warp: entry e, tile slot t = 2*kvh + kind.  Returns (lane 0) the raw tile that the store set free, or -1: it may go back on the stack once no
 // warp of the step pops any more.
 // Bound by its chain of loads: the entry, the mode table, rows and bases, then the encoder's work.  New rows and bases do not depend on the table and travel with its entry; behind one another
-// they cost most where no cache holds them: a step of 8 rows at head_dim 256, store and attention over two states in turn, 38.1 -> 34.5 us (58 MB of slots each); out of L2 nothing.
+// they cost most where no cache holds them: a step of 8 rows at head_dim 256, store and attention over two states in turn, 38.1 -> 34.5 us (58 MB of slots each); out of L2 32 x 8 blocks that fill
+// 9.2 -> 8.1, blocks that get one row the same.  A block that is new as a whole has no old rows to ask for: asked one by one whether they are there, 24 tiles took 4.8 us in place of 4.7 (now 4.6).
 template <int KIND_V>
 __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, int e, int t, int lane) {
   const gaac_paged& st = p.st;
@@ -121,7 +122,7 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   uint16_t* rawp = reinterpret_cast<uint16_t*>(st.raw);
   int fits = 0, r = r_old;
   if (full) {
-    // gather the tile: old rows from the raw tile (if any), new rows from this step's K/V, which travel with the mode-table entry
+    // gather the tile: new rows from this step's K/V, which travel with the mode-table entry, old rows from the raw tile (if any)
     uint4 v[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
@@ -131,10 +132,16 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
     }
     u32 b3w[8], b4w[8];
     load_base_words<KIND_V>((KIND_V ? st.b3v : st.b3k) + kvh * D, (KIND_V ? st.b4v : st.b4k) + kvh * D, lane, b3w, b4w);
+    if (off0 > 0 && have) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int c = lane + 32 * k, row = c >> 4, col = (c & 15) * 8;
+        if (row < off0) v[k] = *reinterpret_cast<const uint4*>(rawp + ((long)r_old * T + row) * D + col);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const int c = lane + 32 * k, row = c >> 4, col = (c & 15) * 8;
-      if (row < off0 && have) v[k] = *reinterpret_cast<const uint4*>(rawp + ((long)r_old * T + row) * D + col);
       *reinterpret_cast<uint4*>(&ws.xs[row * XS_STRIDE + col]) = v[k];
     }
     LaneTile lt;
