@@ -118,7 +118,10 @@ def host():
         try:
             from . import _host as module
         except ImportError as e:
-            raise RuntimeError(f"gaac_b200/_host.so is missing or does not fit this torch ({torch.__version__}): build it with `python -m gaac_b200.build --force`") from e
+            raise RuntimeError(f"gaac_b200's module _host is missing or does not fit this torch ({torch.__version__}): build it with `python -m gaac_b200.build`") from e
+        wanted = f"ABI {ABI_VERSION}, torch {torch.__version__}"                       # (it passes arguments as the header and torch's classes were when it was made)
+        if module.built_for != wanted:
+            raise RuntimeError(f"{module.__file__} was built for {module.built_for}, not for {wanted}: rebuild it with `python -m gaac_b200.build`")
         module.bind(handle)
         _host = module
     return _host

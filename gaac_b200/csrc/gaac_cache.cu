@@ -345,4 +345,4 @@ extern "C" const char* gaac_status_string(int status) {
   }
 }
 
-extern "C" int gaac_abi_version(void) { return 4; }
+extern "C" int gaac_abi_version(void) { return GAAC_ABI_VERSION; }

@@ -198,6 +198,14 @@ PyMethodDef methods[] = {
   {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
+#define TEXT(x) #x
+#define TEXT_OF(x) TEXT(x)
+const char built_for[] = "ABI " TEXT_OF(GAAC_ABI_VERSION) ", torch " TEXT_OF(GAAC_TORCH_VERSION);          // (checked before bind)
+
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+  PyObject* const made = PyModule_Create(&module);
+  if (made && PyModule_AddStringConstant(made, "built_for", built_for) < 0) { Py_DECREF(made); return nullptr; }
+  return made;
+}

@@ -30,7 +30,8 @@ enum {
 #define GAAC_TILE_MAX_ESC 1280   /* worst-case escape bytes of a 16-token tile; stride of the encoder's scratch slots */
 
 const char* gaac_status_string(int status);
-/* ABI version of this header (bumped on any signature change). */
+/* ABI version of this header (bumped on any signature change), and of a library. */
+#define GAAC_ABI_VERSION 4
 int gaac_abi_version(void);
 
 /* ---------------------------------------------------------------------------------------------- block encoder */
