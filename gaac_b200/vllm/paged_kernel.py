@@ -34,7 +34,7 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
         nsplit = -(-units // B) if units else choose_nsplit_sm100(B, n_kv, bt.shape[1] * 16, ragged=True, bound=True)        # with units: what the workspace must have room for
         flat = choose_flat(B, n_kv, bt.shape[1] * 16, nsplit, units, n_q // n_kv, bt_stride * 16)
         if flat: nsplit = _flat_splits(B, n_kv, flat)
-    st = (buf, raw, mt, None, None, None, *bases, n_kv, TS, TS - 2880)
+    st = (buf, raw, mt, None, None, None, bases[0], bases[1], bases[2], bases[3], n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, n_q, nsplit, stream)
     name = "gaac_paged_decode_attn_flat" if flat else "gaac_paged_decode_attn_balanced" if units else "gaac_paged_decode_attn"

@@ -28,7 +28,7 @@ def paged_attention256(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv,
         nsplit = choose_nsplit256(B, n_kv, bt.shape[1] * 16, group=G)
         flat = choose_flat256(B, n_kv, bt.shape[1] * 16, bt_stride * 16, SM_COUNT_B200, G)
         if flat: nsplit = _flat_splits(B, n_kv, flat)                                          # what the workspace must have room for
-    st = (buf, raw, mt, None, None, None, *bases, 2 * n_kv, TS, TS - 2880)
+    st = (buf, raw, mt, None, None, None, bases[0], bases[1], bases[2], bases[3], 2 * n_kv, TS, TS - 2880)
     stream = _lib.stream_ptr(q.device)
     ws = workspace(q.device, B, 2 * n_q, nsplit, stream)
     name = "gaac_paged_decode_attn256_flat" if flat else "gaac_paged_decode_attn256"
