@@ -161,26 +161,24 @@ class CompressedKVCache:
 
     def _prefill_launch(self, slot, L, k, v, scratch, status, copy_only: int):
         """status: the slot's four words as a tensor, or None where their address is enough (indexing costs a microsecond)."""
-        lib, dev = _lib.lib(), self.S.device
+        host, dev, K, V = _lib.host(), self.S.device, self.k, self.v
         stream = _lib.stream_ptr(dev)
-        if isinstance(self.k, _Store): calls, K, V = _lib.host(), self.k, self.v
-        else: calls, K, V = lib, self.k.c_store(), self.v.c_store()                                # (stores of another kind: by their descriptors)
         status = self._slot_status.data_ptr() + 16 * slot if status is None else status.data_ptr()
         rows = self.k.base3.shape[0]
         own = self.per_sequence_bases and L and not copy_only                                      # tables from the prompt itself
         if own and not _lib.capturing():
-            ws = _TABLES.of(self, dev, stream, lib.gaac_cache_tables_workspace_bytes(self.n_kv))
-            _lib.check(calls.gaac_cache_prefill_own(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(),
-                                                    self.cap, self.k.ovf_cap, rows, scratch.data_ptr(), scratch.numel(), status, ws.data_ptr(), ws.numel(), stream),
+            ws = _TABLES.of(self, dev, stream, _lib.lib().gaac_cache_tables_workspace_bytes(self.n_kv))
+            _lib.check(host.gaac_cache_prefill_own(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(),
+                                                   self.cap, self.k.ovf_cap, rows, scratch.data_ptr(), scratch.numel(), status, ws.data_ptr(), ws.numel(), stream),
                        "gaac_cache_prefill_own")
             return
         if own:                                      # a workspace made or cleared while a graph is captured would be so only when the graph runs
-            hist = torch.empty(lib.gaac_cache_calibrate_scratch_bytes(self.n_kv), dtype=torch.uint8, device=dev)
-            _lib.check(calls.gaac_cache_calibrate(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, rows, hist.data_ptr(), hist.numel(), stream),
+            hist = torch.empty(_lib.lib().gaac_cache_calibrate_scratch_bytes(self.n_kv), dtype=torch.uint8, device=dev)
+            _lib.check(host.gaac_cache_calibrate(K, V, k.data_ptr(), v.data_ptr(), L, _lib.row_stride(k), slot, self.n_kv, rows, hist.data_ptr(), hist.numel(), stream),
                        "gaac_cache_calibrate")
-        _lib.check(calls.gaac_cache_prefill(K, V, _lib.ptr(k), _lib.ptr(v), L, _lib.row_stride(k) if k is not None else self.n_kv * D,
-                                            slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(), self.cap, self.k.ovf_cap, rows,
-                                            scratch.data_ptr(), scratch.numel(), status, copy_only, stream), "gaac_cache_prefill")
+        _lib.check(host.gaac_cache_prefill(K, V, _lib.ptr(k), _lib.ptr(v), L, _lib.row_stride(k) if k is not None else self.n_kv * D,
+                                           slot, self.n_kv, self.tail_len.data_ptr(), self.S.data_ptr(), self.cap, self.k.ovf_cap, rows,
+                                           scratch.data_ptr(), scratch.numel(), status, copy_only, stream), "gaac_cache_prefill")
 
     def settle_prefills(self):
         """Host check of every prefill made with check=False: one read of their status words; the escape streams grow when one

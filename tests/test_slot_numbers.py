@@ -1,29 +1,40 @@
 """CompressedKVCache.prefill with the slot number as programs have it: an int, an element of an array, a tensor of one element."""
 import ctypes
+import types
 import numpy as np
 import pytest
 
 
 def _cache(monkeypatch, n_slots, own):
-    """A cache whose library records what it is handed (through the argument types of the real one)."""
+    """A cache whose native module records what it is handed (through the argument types of the real one)."""
     import torch
     import gaac_b200.kv_cache as kvc
     from gaac_b200 import _lib
     calls = []
 
+    class Sizes:
+        def __getattr__(self, name):
+            assert name.endswith("_bytes")
+            return lambda *a: 4096
+
     class Recording:
+        """The native module up to the library: what it is not handed as a number, an address or a store it would refuse."""
+        def empty(self, like, kind, *sizes): return torch.empty(sizes, dtype=torch.uint8)
+
         def __getattr__(self, name):
             res, args = _lib._SIGNATURES[name]
-            if name.endswith("_bytes"): return lambda *a: 4096
 
             def call(*a):
                 assert len(a) == len(args)
                 for value, kind in zip(a, args):
-                    kind.from_param(value)           # what ctypes would refuse
+                    if kind in (ctypes.POINTER(_lib.Store),):
+                        assert all(hasattr(value, f) for f in ("sm", "codes", "flags", "tile_off", "ovf", "ovf_used", "tail", "base3", "base4"))
+                    else: kind.from_param(value)
                 calls.append((name, a))
                 return 0
             return call
-    monkeypatch.setattr(kvc._lib, "lib", lambda: Recording())
+    monkeypatch.setattr(kvc._lib, "lib", Sizes)
+    monkeypatch.setattr(kvc._lib, "host", Recording)
     monkeypatch.setattr(kvc._lib, "stream_ptr", lambda dev: 0)
     monkeypatch.setattr(kvc._lib, "capturing", lambda: False)
     cache = object.__new__(kvc.CompressedKVCache)
@@ -32,7 +43,7 @@ def _cache(monkeypatch, n_slots, own):
     cache._slot_status, cache._pending, cache._pending_bytes, cache._scratch = torch.zeros(n_slots, 4, dtype=torch.int32), {}, 0, None
     cache.pending_scratch_limit = 1 << 30
     table = torch.zeros(2 * n_slots if own else 2, 128, dtype=torch.uint8)
-    cache.k = cache.v = type("Store", (), {"ovf_cap": 1 << 20, "base3": table, "c_store": lambda self: _lib.Store()})()
+    cache.k = cache.v = types.SimpleNamespace(ovf_cap=1 << 20, base3=table, base4=table, **{f: table for f in ("sm", "codes", "flags", "tile_off", "ovf", "ovf_used", "tail")})
     cache._token_rows = lambda x: x
     return cache, calls
 
