@@ -625,10 +625,12 @@ __device__ __forceinline__ void fewer_ranges(int tiles, int one, int turn, int& 
 enum { GRID, SHARED, FLAT_LINE, TEAM, BOUND };
 // ---- teams: the ranges of a row as one cluster, at most eight CTAs (the portable size), whose partials meet in the shared memory of the first.  Through global memory they take a fence
 // until the partials have arrived there, an atomic, and a load of each back, 1.7 us of a launch of 7; through distributed shared memory 0.7: 8 heads x 500 tokens 7.2 -> 6.1 us in a graph.  The others
-// store into the first CTA and leave; it has said, ahead of its main loop, that the place is free, which is in the stages that a range of at most TEAM_TILES tiles does not reach.  Longer ranges, found out
+// store into the first CTA and leave; it has said, ahead of its main loop, that the place is free, which is in the stages that a range of at most TEAM_TILES tiles does not reach and
+// that nobody has used before, the queries' way through the last of them included: so the word needs no release, which would take 0.4 us.  Longer ranges, found out
 // only here where the caller goes by a bound, take the other way: both decide by the row's length, so the CTAs of a cluster agree.
 constexpr int TEAM_MOST = 8, TEAM_STAGE = 6, TEAM_TILES = TEAM_STAGE * TPS;
-static_assert((TEAM_MOST - 1) * 8 * 130 * 4 <= (NSTG - TEAM_STAGE) * STAGE_BYTES, "the partials lie in stages that so few tiles do not reach");
+constexpr int Q_PLACE = TB_RING + NSTG * STAGE_BYTES - 2048;          // where one warp leaves the queries for the others: the end of the last stage
+static_assert(TEAM_STAGE * STAGE_BYTES + (TEAM_MOST - 1) * 8 * 130 * 4 <= Q_PLACE - TB_RING && Q_PLACE % 16 == 0, "the partials lie in stages that so few tiles do not reach, ahead of the queries");
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -834,7 +836,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) decode_attn_kernel(const __gri
   // The queries, by one warp for all, through the last stage's place, which is not filled before the second barrier.  Every warp on its own asked for them behind the first stages'
   // payload and had them 1.1 us later.  (Not in a flat launch, whose pieces begin at different times: 425 -> 433 us for 16 x 4096..65536.)
   static_assert(FIRST < NSTG && 2048 <= STAGE_BYTES, "the last stage is not one of the first");
-  uint4* const q_place = reinterpret_cast<uint4*>(smem + TB_RING + (NSTG - 1) * STAGE_BYTES) + lane;
+  uint4* const q_place = reinterpret_cast<uint4*>(smem + Q_PLACE) + lane;
   QFrag Q;
   if (!FLAT && warp == ATT_WARPS - 3) {
     load_q(Q, p.q + ((long)b * p.n_q + kvh * G) * D, D, G, lane);
