@@ -59,6 +59,7 @@ _SIGNATURES = {
     "gaac_decode_attn_exchange": (i32, [C.POINTER(Side), C.POINTER(Side), vp, vp, i32, i32, i32, vp, i64, f32, i32, vp, i32, i32, vp, sz, C.POINTER(Exchange), vp, vp, vp]),
     "gaac_debug_decode_attn_rebuild": (i32, [C.POINTER(Side), C.POINTER(Side), vp, vp, i32, i32, i32, vp, i64, i64, f32, i32, vp, i32, i32, vp, sz, vp, vp, vp, vp, i64, vp]),
     "gaac_debug_paged_decode_attn_rebuild": (i32, [C.POINTER(Paged), vp, i64, vp, vp, i32, i32, f32, i32, vp, sz, vp, vp, vp, vp, i64, vp]),
+    "gaac_debug_team_room": (i32, [i32, i32, i32]),
     "gaac_decode_attn": (i32, [C.POINTER(Side), C.POINTER(Side), vp, vp, i32, i32, i32, vp, i64, f32, i32, vp, i32, i32, vp, sz, vp, vp, vp]),
     "gaac_decode_attn_partial": (i32, [C.POINTER(Side), C.POINTER(Side), vp, vp, i32, i32, i32, vp, i64, f32, i32, vp, i32, i32, vp, sz, vp, vp]),
     "gaac_combine": (i32, [vp, vp, vp, i64, i32, vp, vp, vp]),

@@ -1474,7 +1474,10 @@ static int team_room(int nsplit) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = (unsigned)nsplit; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 0) { cudaGetLastError(); n = 0; }
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 0) {
+      cudaGetLastError();
+      return 0;                                      // (not known: asked again)
+    }
     known[dev][nsplit].store(n + 1, std::memory_order_relaxed);
   }
   return n;
@@ -1741,6 +1744,11 @@ extern "C" int gaac_debug_decode_attn_rebuild(const gaac_side* K, const gaac_sid
   if (!out_bf16 || !k_rebuilt || !v_rebuilt) return GAAC_E_ARG;
   SlotOut o; o.out = out_bf16; o.out_f32 = out_f32; o.dump_k = k_rebuilt; o.dump_v = v_rebuilt; o.dump_S = rebuilt_S;
   return slot_attn(K, V, q_bf16, slot, B, n_q, n_kv, seq_len, S_uniform, S_pad, scale, nsplit, tail_len, tail_cap, n_base_rows, workspace, workspace_bytes, o, stream);
+}
+
+extern "C" int gaac_debug_team_room(int paged, int group, int nsplit) {
+  if (nsplit < 2 || nsplit > TEAM_MOST || group < 1 || group > 8) return 0;
+  return paged ? (group <= 4 ? team_room<true, 1>(nsplit) : team_room<true, 2>(nsplit)) : group <= 4 ? team_room<false, 1>(nsplit) : team_room<false, 2>(nsplit);
 }
 
 extern "C" int gaac_debug_paged_decode_attn_rebuild(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,

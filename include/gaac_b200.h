@@ -398,6 +398,8 @@ int gaac_debug_decode_attn_rebuild(const gaac_side* K, const gaac_side* V, const
 int gaac_debug_paged_decode_attn_rebuild(const gaac_paged* st, const int32_t* bt, int64_t bt_stride, const int32_t* seq_lens, const void* q_bf16,
                                          int B, int n_q, float scale, int nsplit, void* workspace, size_t workspace_bytes, void* out_bf16,
                                          float* out_f32, void* k_rebuilt, void* v_rebuilt, int64_t rebuilt_S, void* stream);
+/* Rows (times kv heads) that the current GPU has room for as clusters of nsplit ranges each, for GQA groups of `group`: launches of no more run as such.  0: none, or not known. */
+int gaac_debug_team_room(int paged, int group, int nsplit);
 
 #ifdef __cplusplus
 }

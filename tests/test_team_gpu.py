@@ -16,6 +16,17 @@ def test_rules():
 
 
 @pytest.mark.gpu
+def test_the_gpu_has_the_room_that_the_rules_count_on():
+    """Otherwise the launches of this file would pass as grids."""
+    import torch
+    from gaac_b200 import _lib
+    from gaac_b200.kernel import TEAMS
+    room = _lib.lib().gaac_debug_team_room
+    assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or all(room(paged, G, n) >= TEAMS[n] for paged in (0, 1) for G in (1, 4, 5, 8) for n in TEAMS)
+    assert not any(room(0, G, n) for G, n in ((4, 1), (4, 9), (0, 4), (9, 4)))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("B,n_kv,G,S", [(1, 2, 4, 40), (1, 1, 8, 129), (2, 2, 4, 384), (1, 1, 5, 768), (1, 1, 1, 3072), (1, 1, 4, 3100), (3, 1, 6, 1000), (10, 2, 4, 300)])
 def test_pages(B, n_kv, G, S):
     import torch
