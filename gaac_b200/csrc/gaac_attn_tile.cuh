@@ -234,7 +234,7 @@ struct AttnView { u32 addends, segs, bases; };
 __device__ __forceinline__ void fill_attn_tables(uint8_t* at, int t) {
   const u32x2 x = pair_addends((u32)t), s = segment_entry((u32)t);
   reinterpret_cast<uint2*>(at + 16)[t] = make_uint2(x.x, x.y);
-  reinterpret_cast<uint2*>(at + ADDEND_BYTES)[t] = make_uint2((s.x & 0xFFFFu) | s.y << 16, s.x >> 16);           // (a permute takes the lower half of a selector)
+  reinterpret_cast<uint2*>(at + ADDEND_BYTES)[t] = make_uint2(s.x, s.y);
   if (t == 0) reinterpret_cast<uint2*>(at + 8)[0] = make_uint2(0u, 0u);
 }
 __device__ __forceinline__ AttnView attn_view(u32 tables, u32 bases) { return AttnView{tables + 16 - 256 * 8, tables + ADDEND_BYTES, bases}; }
@@ -310,7 +310,7 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
       u32 bit; asm("bfind.u32 %0, %1;" : "=r"(bit) : "r"(raws));
       const u32 below = ~(0xFFFFFFFFu << bit);
       raws &= below; index--;
-      const u32 pl = at + (u32)popc(fl & below & 0x55555555u) + 4u * (u32)popc(fl & below & 0xAAAAAAAAu);
+      const u32 pl = at + esc_below(fl, below);
       const u32x4 bw = lds_u128(side + 8u * bit + skew * (bit >> 3));
       const u32x2 x = pair_payload(__funnelshift_r(lds_u32(pl & ~3u), lds_u32((pl & ~3u) + 4u), 8u * pl), lds_u8(pl + 4u));
       const u32 m = index >> 8;
@@ -321,7 +321,7 @@ __device__ __forceinline__ int plan_tile(bool live, u32 fl_at, u32 esc, int avai
       u32 bit; asm("bfind.u32 %0, %1;" : "=r"(bit) : "r"(behind));
       const u32 below = ~(0xFFFFFFFFu << bit);
       behind &= below;
-      sts_u16(mine + bit, 256u + lds_u8(at + (u32)popc(fl & below & 0x55555555u) + 4u * (u32)popc(fl & below & 0xAAAAAAAAu)));
+      sts_u16(mine + bit, 256u + lds_u8(at + esc_below(fl, below)));
     }
   }
   __syncwarp();

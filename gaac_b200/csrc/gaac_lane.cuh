@@ -59,7 +59,7 @@ __device__ __forceinline__ void sts_u128(u32 a, u32 x, u32 y, u32 z, u32 w) { as
 // which may be read in any case), advanced past them.  raws: some lane's group is raw (the same in all lanes).
 __device__ __forceinline__ void decode_group_dev(u32 sm_lo, u32 sm_hi, u32 z, u32 tg, u32& esc, bool raws, const u32x4& bw, u32 out[4]) {
   const u32 m1 = tg & 1u, eb = lds_u8(esc) * m1;      // promoted (tags are 0, 1 or 3)
-  u32x2 x{spread_bit4(eb & 15u), spread_bit4(eb >> 4)};
+  u32x2 x = byte_addends(eb);
   if (raws) {
     if (tg & 2u) {
       x = raw_addends(lds_u32(esc & ~3u), lds_u32((esc & ~3u) + 4u), 8u * (esc & 3u), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));

@@ -110,6 +110,8 @@ template <int H, u32 K> GAAC_HD u32 mad_half(u32 a, u32 c) {
 // ---- tags -> escape byte counts --------------------------------------------------------------------------------
 // escape bytes of a row with tag word fl (tier 1 -> 1 byte, tier 2 -> 5 bytes)                  gaac/kernel.py:46
 GAAC_HD int row_esc_bytes(u32 fl) { return popc(fl & 0x55555555u) + 4 * popc(fl & 0xAAAAAAAAu); }
+// .. of the groups whose tag bits are in `below`
+GAAC_HD u32 esc_below(u32 fl, u32 below) { return (u32)popc(fl & below & 0x55555555u) + 4u * (u32)popc(fl & below & 0xAAAAAAAAu); }
 // escape bytes of the groups below bit position `bits` of the tag word                            gaac/kernel.py:29
 GAAC_HD int esc_prefix(u32 fl, int bits) {
   u32 low = bits >= 32 ? fl : (fl & ((1u << bits) - 1u));

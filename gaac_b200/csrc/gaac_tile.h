@@ -45,8 +45,8 @@ GAAC_HD int tag_esc_bytes(u32 tag) { return (int)(tag & 1u) + 2 * (int)(tag & 2u
 // ---- decode ----------------------------------------------------------------------------------------------------
 struct u32x4 { u32 x, y, z, w; };
 struct u32x2 { u32 x, y; };
-// Escape-byte table, for the check of the decoder on the host (the device works an entry out): lutx[b] = { spread_bit4(b & 15), spread_bit4(b >> 4) }, what escape byte b adds to the exponents of its group
-GAAC_HD void fill_lutx(u32x2* lutx, int i) { lutx[i].x = spread_bit4((u32)i & 0xFu); lutx[i].y = spread_bit4((u32)i >> 4); }
+// What escape byte b adds to the exponents of its group: of elements 0..3, 4..7
+GAAC_HD u32x2 byte_addends(u32 b) { return u32x2{spread_bit4(b & 15u), spread_bit4(b >> 4)}; }
 // The 24 code bits of a group, picked out of two neighbouring words by one byte permute that already puts codes 4..7 at the top:
 // bits 0..11 = codes 0..3, bits 20..31 = codes 4..7 (B = byte offset of the group in the lane's code string).
 template <int B> GAAC_HD u32 group_codes(const u32* cd) {
@@ -61,7 +61,7 @@ GAAC_HD u32x2 raw_addends(u32 w0, u32 w1, u32 sh, u32 blo, u32 bhi) {
   return u32x2{spread_hi5(lo & 0xFFFFFu) - blo, spread_hi5(funnel_r(lo, hi, 20) & 0xFFFFFu) - bhi};
 }
 // Rebuild one group (two sign/mantissa words) into four bf16x2 words: z as group_codes leaves it; m1 = 1 for a promoted group; bw = {3-bit-window base words of
-// the two half groups, what the 4-bit-window ones are above them}; x = the group's addends, from the escape-byte table or raw_addends.
+// the two half groups, what the 4-bit-window ones are above them}; x = the group's addends, of byte_addends or raw_addends.
 GAAC_HD void rebuild_group(u32 sm_lo, u32 sm_hi, u32 z, u32 m1, const u32x4& bw, const u32x2& x, u32 out[4]) {
   const u32 blo = mad(m1, bw.z, bw.x), bhi = mad(m1, bw.w, bw.y);
   // four 3-bit codes -> four bytes in two steps; each step moves the upper fields with a multiply-add: (t & M) * (2^k - 1) + t
@@ -120,9 +120,9 @@ GAAC_HD void rebuild_pairs(u32 sm_lo, u32 sm_hi, u32 u, u32 m, const u32x4& bw, 
   out[3] = bits_of(prmt(sm_lo, sm_hi, 0x7733), od >> 1, 0x807F807Fu);
 }
 // ---- escape bytes of four neighbouring groups of a row (a segment), by its tag byte t.  Segment words hold a 16-bit index per group: NO_ESC for a group without
-// escape byte, 256 + byte for a promoted one; entry `index` of the addend table is what to add, index >> 8 the m of rebuild_pairs.  {x: two selectors of 16
-// bits that pick the indexes of groups 0, 1 and of groups 2, 3 out of the segment's first four escape bytes and SEG_CONST; y: escape bytes of the segment}.
-// The selectors are right for the groups up to the segment's first raw one; raw_items are the others.
+// escape byte, 256 + byte for a promoted one; entry `index` of the addend table is what to add, index >> 8 the m of rebuild_pairs.  {x: selector of 16 bits that picks the
+// indexes of groups 0, 1 out of the segment's first four escape bytes and SEG_CONST, above it the segment's escape bytes; y: the selector of groups 2, 3}, since a permute takes the
+// lower half of a selector.  The selectors are right for the groups up to the segment's first raw one; raw_items are the others.
 constexpr u32 NO_ESC = 255u, SEG_CONST = 0x000100FFu;
 GAAC_HD u32x2 segment_entry(u32 t) {
   u32 sel = 0u, at = 0u;
@@ -131,7 +131,7 @@ GAAC_HD u32x2 segment_entry(u32 t) {
     sel |= (tag & 1u ? 0x60u | at : 0x54u) << (8 * g);
     at += tag & 1u;
   }
-  return u32x2{sel, seg_esc(t)};
+  return u32x2{(sel & 0xFFFFu) | seg_esc(t) << 16, sel >> 16};
 }
 // Groups of a row with tag word fl that the selectors leave out: the raw ones and the promoted ones behind a raw one of their segment, at their lower tag bits.
 GAAC_HD u32 raw_items(u32 fl) {

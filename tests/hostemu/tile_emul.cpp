@@ -76,17 +76,9 @@ extern "C" int emu_encode_tile(int kind_v, const uint16_t* x, int nvalid, const 
   return total;
 }
 
-// Rebuild.  PATCH false: the form that reads escape bytes where they are (decode_group_dev<false>); true: the form of staged tiles, where raw groups were
-// turned into table entries and the first payload byte of each into the entry's number (build_raw_patches, decode_group_dev<true>).  esc_in must be
-// readable to the end of the word behind its last byte.
-template <bool PATCH>
-static void decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in, const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
-  static u32x2 lutx[256]; static bool init = false;
-  if (!init) { for (int i = 0; i < 256; i++) fill_lutx(lutx, i); init = true; }
-  auto raw = [&](const uint8_t* p, u32 blo, u32 bhi) {
-    const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-    return raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(p) & 3), blo, bhi);
-  };
+// Rebuild as the decoders do it (decode_tile_warp, decode_group_dev): a lane goes along its segments' escape bytes, of which it reads one per group whether the group has it or not.
+// esc_in must be readable to the end of the word behind its last byte.
+extern "C" void emu_decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in, const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
   const int SEGS = kind_v ? 4 : 2, PER = 8 / SEGS;
   u32 base[32][2];                                   // {3-bit window, what the 4-bit one is above it} per half group
   for (int t = 0; t < 32; t++) {
@@ -101,13 +93,18 @@ static void decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, 
     const u32 z[8] = {group_codes<0>(cd), group_codes<3>(cd), group_codes<6>(cd), group_codes<9>(cd), group_codes<12>(cd), group_codes<15>(cd), group_codes<18>(cd), group_codes<21>(cd)};
     for (int s = 0; s < SEGS; s++) {
       const int row = kind_v ? v_tok(j, s) : 8 * s + r, first = kind_v ? 2 * r : 4 * j;
+      const uint8_t* esc = esc_in + esc_at(fl_in, row, first);
       for (int g = 0; g < PER; g++) {
         const int idx = PER * s + g, hg = kind_v ? 4 * r + 2 * g : 8 * j + 2 * g;
         const u32 tag = (fl_in[row] >> (2 * (first + g))) & 3u, m1 = tag & 1u;
         const u32x4 bw{base[hg][0], base[hg + 1][0], base[hg][1], base[hg + 1][1]};
-        const uint8_t* p = esc_in + esc_at(fl_in, row, first + g);
-        u32x2 x = lutx[tag == 1u ? *p : 0];
-        if (tag & 2u) x = PATCH ? raw(p, bw.x + bw.z, bw.y + bw.w) : raw(p, mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
+        u32x2 x = byte_addends(*esc * m1);
+        if (tag & 2u) {
+          const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(esc) & ~(uintptr_t)3);
+          x = raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(esc) & 3), mad(m1, bw.z, bw.x), mad(m1, bw.w, bw.y));
+          esc += 4;
+        }
+        esc += m1;
         u32 f[4];
         rebuild_group(sm[2 * idx], sm[2 * idx + 1], z[idx], m1, bw, x, f);
         for (int q = 0; q < 4; q++) {
@@ -120,17 +117,8 @@ static void decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, 
   }
 }
 
-extern "C" void emu_decode_tile(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in,
-                                const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
-  decode_tile<false>(kind_v, sm_in, cd_in, fl_in, esc_in, b3row, b4row, out);
-}
-extern "C" void emu_decode_tile_lut(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in,
-                                    const uint8_t* b3row, const uint8_t* b4row, uint16_t* out) {
-  decode_tile<true>(kind_v, sm_in, cd_in, fl_in, esc_in, b3row, b4row, out);
-}
-
-// Rebuild as the attention kernels do it: the tile's segments (four groups of a row) are expanded into indexes of the addend table, a raw group's index is that
-// of an entry of its own behind the table, and a word pairs elements that lie four apart.  first_patch: index of the first such entry.
+// Rebuild as the attention kernels do it (plan_tile, rebuild_pairs): the tile's segments (four groups of a row) are expanded into indexes of the addend table, a raw group's index is
+// that of an entry of its own behind the table, and a word pairs elements that lie four apart.  first_patch: index of the first such entry.
 extern "C" int emu_decode_tile_pairs(int kind_v, const uint8_t* sm_in, const uint8_t* cd_in, const uint32_t* fl_in, const uint8_t* esc_in,
                                      const uint8_t* b3row, const uint8_t* b4row, int first_patch, uint16_t* out) {
   static u32x2 addends[65536];
@@ -140,31 +128,38 @@ extern "C" int emu_decode_tile_pairs(int kind_v, const uint8_t* sm_in, const uin
   for (int t = 0; t < 16; t++) base[t] = kind_v ? pair_base_words<true>(b3row, b4row, t) : pair_base_words<false>(b3row, b4row, t);
   u32 words[16][4][2];                               // segment words of row, quarter
   int raws = 0;
-  for (int row = 0; row < 16; row++)
+  for (int row = 0; row < 16; row++) {               // a lane's row
+    const u32 fl = fl_in[row];
+    const uint8_t* const at = esc_in + esc_at(fl_in, row, 0);
+    const uint8_t* a = at;
     for (int q = 0; q < 4; q++) {
-      const u32 t = (fl_in[row] >> (8 * q)) & 0xFFu;
-      const u32x2 e = segment_entry(t);
-      const uint8_t* p = esc_in + esc_at(fl_in, row, 4 * q);
-      if (e.y != seg_esc(t)) return -1;
-      const u32 four = (u32)p[0] | (u32)p[1] << 8 | (u32)p[2] << 16 | (u32)p[3] << 24;
-      u32 (&w)[2] = words[row][q];
-      w[0] = prmt(four, SEG_CONST, e.x & 0xFFFFu); w[1] = prmt(four, SEG_CONST, e.x >> 16);
-      const u32 items = (raw_items(fl_in[row]) >> (8 * q)) & 0xFFu;
-      for (int g = 0; g < 4; g++)
-        if ((items >> (2 * g)) & 1u) {
-          const uint8_t* pl = p + seg_esc(t & ((1u << (2 * g)) - 1u));
-          u32 index = 256u + *pl;
-          if ((t >> (2 * g)) & 2u) {
-            const u32* a = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(pl) & ~(uintptr_t)3);
-            u32x2 x = pair_raw_addends(a[0], a[1], 8u * (u32)(reinterpret_cast<uintptr_t>(pl) & 3));
-            index = (u32)(first_patch + raws++);
-            const u32 m = index >> 8;
-            const u32x4& bw = base[4 * q + g];
-            addends[index] = u32x2{x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w};
-          }
-          w[g >> 1] = prmt(w[g >> 1], index, g & 1 ? 0x5410u : 0x3254u);
-        }
+      const u32x2 e = segment_entry((fl >> (8 * q)) & 0xFFu);
+      const u32 four = (u32)a[0] | (u32)a[1] << 8 | (u32)a[2] << 16 | (u32)a[3] << 24;
+      words[row][q][0] = prmt(four, SEG_CONST, e.x); words[row][q][1] = prmt(four, SEG_CONST, e.y);
+      a += e.x >> 16;
     }
+    if (a - at != row_esc_bytes(fl)) return -1;
+    uint16_t* const indexes = reinterpret_cast<uint16_t*>(words[row]);
+    u32 raw = (fl >> 1) & fl & 0x55555555u, behind = raw_items(fl) & ~raw;
+    raws += popc(raw);
+    u32 index = (u32)(first_patch + raws);           // behind the row's entries: from the last to the first
+    while (raw) {
+      const u32 bit = 31u - (u32)__builtin_clz(raw), below = ~(0xFFFFFFFFu << bit);
+      raw &= below; index--;
+      const uint8_t* const pl = at + esc_below(fl, below);
+      const u32* const w = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(pl) & ~(uintptr_t)3);
+      const u32x2 x = pair_payload(funnel_r(w[0], w[1], (int)(8 * (reinterpret_cast<uintptr_t>(pl) & 3))), pl[4]);
+      const u32 m = index >> 8;
+      const u32x4& bw = base[bit >> 1];
+      addends[index] = u32x2{x.x - bw.x - m * bw.z, x.y - bw.y - m * bw.w};
+      indexes[bit >> 1] = (uint16_t)index;
+    }
+    while (behind) {
+      const u32 bit = 31u - (u32)__builtin_clz(behind), below = ~(0xFFFFFFFFu << bit);
+      behind &= below;
+      indexes[bit >> 1] = (uint16_t)(256u + at[esc_below(fl, below)]);
+    }
+  }
   const int SEGS = kind_v ? 4 : 2, PER = 8 / SEGS;
   for (int lane = 0; lane < 32; lane++) {
     const int j = lane & 3, r = lane >> 2;
