@@ -285,7 +285,9 @@ __device__ __forceinline__ void load_tile_words(TileWords<KIND_V>& tw, const uin
 // stmatrix.  most: escape bytes that the scratch behind ws has room for; less than TILE_MAX_ESC only where no tile has more (tags that say otherwise make wrong values and nothing else).
 // All of a tile's escape bytes are staged, so that a group reads its own without asking whether it has one, and whether any lane's group is raw is asked once per tile: 771 -> 699 (K) and 788 -> 776
 // warp instructions per tile, most of them in branches and 64-bit addresses.  [8, 65536, 128] K and V 88.2 -> 85.7 us;  blocks of 32768 tokens 44.7 -> 43.3, of 512 3.5 -> 3.2.  A second copy of the
-// groups for escape bytes in global memory beside them spilled (93), and so did more than one tile per warp of the block decoder.  Without the rebuild, loads and stores alone, the pages take 80.
+// groups for escape bytes in global memory beside them spilled (93), and so did more than one tile per warp of the block decoder.  Tiles of many escape bytes have asynchronous copies of
+// them in flight together: by a load and a store per 128 bytes, one behind the other, values of random bits (1280 bytes a tile) took 80.6 us, [8, 32768, 128] K and V, read where they lie 59.4, now 59.2.
+// Without the rebuild, loads and stores alone, the pages of 65536 tokens take 80.
 template <int KIND_V>
 __device__ __forceinline__ void decode_tile_warp(WarpScratch& ws, TileWords<KIND_V>& tw, u32 bases, int lane, int most = TILE_MAX_ESC) {
   const int j = lane & 3, r = lane >> 2;
@@ -313,7 +315,15 @@ __device__ __forceinline__ void decode_tile_warp(WarpScratch& ws, TileWords<KIND
     u32* const to = reinterpret_cast<u32*>(&ws + 1);
     const int have = tw.n_esc > 0 ? (tw.n_esc + ofs + 3) >> 2 : 0;       // words that came with the rest
     if (lane < have) to[lane] = tw.esc;
-    for (int i = have + lane; 4 * i < (n > 0 ? min(n, most) + ofs : 0); i += 32) to[i] = g[i];
+    const int end = n > 0 ? min(n, most) + ofs : 0;
+    int i = have + lane;
+    if (4 * i < end) to[i] = g[i];
+    if (4 * (have + 32) < end) {                     // (the same in all lanes) many escape bytes: all of them on their way at once
+      const u32 at = (u32)__cvta_generic_to_shared(to);
+      for (i += 32; 4 * i < end; i += 32) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(at + 4u * (u32)i), "l"(g + i) : "memory");
+      async_commit();
+      async_wait<0>();
+    }
   }
   const u32 esc0 = (u32)__cvta_generic_to_shared(&ws + 1) + (u32)ofs;
 #pragma unroll
