@@ -16,18 +16,20 @@ inline int launch_status() { return cudaGetLastError() == cudaSuccess ? GAAC_OK 
 inline int g_launch_overlap = 1;      // see gaac_set_launch_overlap
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::); }
+// shared_bytes: dynamic shared memory;  carveout: per cent of an SM's memory that shared memory should have, the rest being L1 (0: as the driver has it).
 template <class... Params, class... Args>
-int launch_overlapped_with(int shared_bytes, void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
+int launch_overlapped_with(int shared_bytes, int carveout, void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = shared_bytes; cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = g_launch_overlap;
-  cfg.attrs = at; cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout; at[1].val.sharedMemCarveout = (unsigned)carveout;
+  cfg.attrs = at; cfg.numAttrs = carveout > 0 ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) != cudaSuccess) { cudaGetLastError(); return GAAC_E_LAUNCH; }
   return launch_status();
 }
 template <class... Params, class... Args>
 int launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, cudaStream_t stream, Args&&... args) {
-  return launch_overlapped_with(0, kernel, grid, threads, stream, std::forward<Args>(args)...);
+  return launch_overlapped_with(0, 0, kernel, grid, threads, stream, std::forward<Args>(args)...);
 }
 }  // namespace gaac

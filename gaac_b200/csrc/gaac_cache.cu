@@ -223,6 +223,9 @@ __global__ void __launch_bounds__(32) release_blocks_kernel(const int* __restric
 // tokens 57.7, now 54.4;  8 20.4 and 55.1;  10 (spills) 22.8 and 67.  All of these with the same blocks again and again, out of L2: where no earlier pass has touched them, the whole chunk (with
 // the overlapped launches 24.6 -> 20.4) gains about 1 %.
 constexpr int PDEC_WARPS = 4;
+// Shared memory's share: 196 KB of an SM's 256, which nine CTAs fit with slots of up to 768 escape bytes and eight with any.  Left to itself the driver makes room for nine, and with 28 KB of L1 the
+// codes, which are read 12 bytes apart, do not stay there: slots of 1280 bytes, 2048 blocks 51.0 us, now 44.3 (slots of 128 42.5 as before); with 85 in place of 80 slots of 832 to 960 are left out.
+constexpr int PDEC_SHARED = 80;
 struct PagedDecodeParams { gaac_paged st; const int* pairs; int P; uint16_t *sk, *sv; long row_stride; };
 
 template <int KIND_V>
@@ -329,7 +332,7 @@ extern "C" int gaac_paged_decode_blocks(const gaac_paged* st, const int32_t* pai
   if (!aligned16(sk) || !aligned16(sv) || row_stride % 8) return GAAC_E_ALIGN;
   if (P == 0) return GAAC_OK;
   PagedDecodeParams p{*st, pairs, P, (uint16_t*)sk, (uint16_t*)sv, row_stride};
-  return launch_overlapped_with(PDEC_WARPS * decode_scratch_bytes(std::min(st->ovf_slot, TILE_MAX_ESC)), paged_decode_blocks_kernel, dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)),
+  return launch_overlapped_with(PDEC_WARPS * decode_scratch_bytes(std::min(st->ovf_slot, TILE_MAX_ESC)), PDEC_SHARED, paged_decode_blocks_kernel, dim3((unsigned)((P + PDEC_WARPS - 1) / PDEC_WARPS), (unsigned)(2 * st->n_kv)),
                                 PDEC_WARPS * 32, (cudaStream_t)stream, p);
 }
 
