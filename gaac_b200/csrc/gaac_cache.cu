@@ -154,13 +154,9 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
     }
   }
   if (!fits) {
-    const bool one = !full && lane < n * 16;         // the first row or two travel with the mode-table entry and the pop
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (one) v = *reinterpret_cast<const uint4*>(src + (long)(tok0 + (lane >> 4)) * sstride + (lane & 15) * 8);
     if (!have) r = pop_raw_tile(st, lane);
     // new rows, natural channel order, into raw tile r
-    if (one && r >= 0) *reinterpret_cast<uint4*>(rawp + ((long)r * T + off0 + (lane >> 4)) * D + (lane & 15) * 8) = v;
-    for (int c = full ? lane : lane + 32; c < (r < 0 ? 0 : n * 16); c += 32) {
+    for (int c = lane; c < (r < 0 ? 0 : n * 16); c += 32) {
       const int row = off0 + (c >> 4), col = (c & 15) * 8;
       *reinterpret_cast<uint4*>(rawp + ((long)r * T + row) * D + col) = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
     }
