@@ -106,7 +106,8 @@ __device__ __forceinline__ void push_raw_tile(int* stack, int* top, int r) {
 // warp of the step pops any more.
 // Bound by its chain of loads: the entry, the mode table, rows and bases, then the encoder's work.  New rows and bases do not depend on the table and travel with its entry; behind one another
 // they cost most where no cache holds them: a step of 8 rows at head_dim 256, store and attention over two states in turn, 38.1 -> 34.5 us (58 MB of slots each); out of L2 32 x 8 blocks that fill
-// 9.2 -> 8.1, blocks that get one row the same.  A block that is new as a whole has no old rows to ask for: asked one by one whether they are there, 24 tiles took 4.8 us in place of 4.7 (now 4.6).
+// 9.2 -> 8.1.  (The rows of a block that stays raw wait for its tile: ahead of the entry they gained nothing.)  A block that is new as a whole has no old rows to ask for: asked one by one
+// whether they are there, 24 tiles took 4.8 us in place of 4.7 (now 4.6).
 template <int KIND_V>
 __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, int e, int t, int lane) {
   const gaac_paged& st = p.st;
@@ -165,7 +166,8 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   return fits && have ? r_old : -1;
 }
 
-__global__ void __launch_bounds__(32) paged_store_kernel(const __grid_constant__ PagedParams p) {
+// 28 CTAs per SM (72 registers, 16 bytes of spills): with the 80 that it would take, 25, a step of 475 x 8 tiles has a second wave, 8.2 -> 8.9 us;  512 x 16 17.2 and 16.8, 94 x 16 5.1 and 5.0.
+__global__ void __launch_bounds__(32, 28) paged_store_kernel(const __grid_constant__ PagedParams p) {
   __shared__ __align__(16) WarpScratch ws;
   const int e = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
   griddep_wait();

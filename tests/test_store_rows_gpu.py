@@ -1,4 +1,4 @@
-"""Rows of a store step, in one or two steps per block: the first two rows of a part of a block travel ahead of the mode-table entry, the others behind it; a block that
+"""Rows of a store step, in one or two steps per block: the new rows of a block that fills travel ahead of the mode-table entry, its old ones and those of a part of a block behind it; a block that
 fills is gathered from both; one whose escape bytes do not fit its slot stays raw.  What comes back out of the blocks is what went in, bit for bit, on both sides of the
 store's two forms (one cluster, two launches)."""
 import numpy as np
