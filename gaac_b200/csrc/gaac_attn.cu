@@ -1486,7 +1486,10 @@ template <bool PAGED>
 static bool team_ok(const AttnParams& p) {
   if (p.part || p.x_recv || p.row_order || p.nsplit < 2 || p.nsplit > TEAM_MOST) return false;
   if (!PAGED && !p.seq_len && ((p.S_uniform + T - 1) / T + p.nsplit - 1) / p.nsplit > TEAM_TILES) return false;
-  return (int64_t)p.B * p.n_kv <= (p.G <= 4 ? team_room<PAGED, 1>(p.nsplit) : team_room<PAGED, 2>(p.nsplit));
+  // Clusters of 3 and of 5 need room for two more: launches of 44 or 45 and of 25 or 26 of them behind one another take up to 1.4 times as long as grids (45 rows of 21 tiles in 3 ranges 11.9 us
+  // to 9.0; with another kernel between two of them 10.0 to 10.9), two fewer 0.9 times as long, as do the other sizes up to the last one.
+  const int64_t spare = p.nsplit == 3 || p.nsplit == 5 ? 2 : 0;
+  return (int64_t)p.B * p.n_kv + spare <= (p.G <= 4 ? team_room<PAGED, 1>(p.nsplit) : team_room<PAGED, 2>(p.nsplit));
 }
 template <bool PAGED, bool DUMP>
 static int launch_attn(const AttnParams& p, cudaStream_t st) {

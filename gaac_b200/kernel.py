@@ -90,7 +90,7 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
     # of 7 tiles in a table of 28 5.9 -> 6.1), against 7.1 for 9.4 where they are.
     # teams=False: for launches that cannot be one, partials and exchanges.  There the ranges' partials go through global memory all the same: partials of 8 heads, 129 tokens 5.5 (one CTA), 7.1 in three
     # ranges; 256 7.0 and 7.4 in five; 1500 7.6 in 16 and 8.2 in 8; 1700 7.6 and 8.8.
-    wave, team = sm_count // rows, _team(rows) if teams else 1
+    wave, team = sm_count // rows, _team(rows, True) if teams else 1
     if team > 1 and (ATT_WARPS if bound or team < 6 else 12) < ntiles <= 14 * team:         # (many rows of one CTA each: 32 x 1 of 200 tokens 8.4 -> 8.2 where they are that long, 5.3 -> 5.9 where that is a bound)
         return min(team, ntiles // 3)
     if wave > 1 and 4 * most <= 3 * wave:
@@ -110,9 +110,9 @@ def choose_nsplit_sm100(B: int, n_kv: int, S: int, sm_count: int = SM_COUNT_B200
 TEAMS = {8: 15, 6: 22, 5: 26, 4: 33, 3: 45, 2: 74}       # ranges of a team: how many teams a B200 has room for (the library asks, and does without them where there are fewer)
 
 
-def _team(rows: int) -> int:
-    """Most ranges that a row's team may have when all rows have one."""
-    return next((n for n in TEAMS if rows <= TEAMS[n]), 1)
+def _team(rows: int, spare: bool = False) -> int:
+    """Most ranges that a row's team may have when all rows have one.  spare: as the library takes it, which wants room for two more teams of 3 or 5 (see team_ok in gaac_attn.cu)."""
+    return next((n for n in TEAMS if rows + (2 if spare and n in (3, 5) else 0) <= TEAMS[n]), 1)
 
 
 def _short_ranges(rows: int, ntiles: int, sm_count: int = SM_COUNT_B200) -> bool:

@@ -46,6 +46,11 @@ def test_rows_of_one_cta_are_no_teams(calls, B, n_kv, tiles):
     if B * n_kv <= 22: assert (choose_nsplit_sm100(B, n_kv, 16 * tiles) == 1) == (tiles <= 12)              # lengths known
 
 
+@pytest.mark.parametrize("rows,most", [(15, 8), (16, 6), (22, 6), (23, 5), (24, 5), (25, 4), (26, 4), (33, 4), (34, 3), (43, 3), (44, 2), (45, 2), (74, 2), (75, 1)])
+def test_teams_of_three_and_five_are_not_packed_to_the_last(rows, most):
+    for bound in (False, True): assert choose_nsplit_sm100(rows, 1, 16 * 28, bound=bound) == (most if most > 1 else 1)
+
+
 @pytest.mark.parametrize("B,n_kv,tiles,G,splits", [
     (1, 8, 8, 4, 1), (1, 8, 9, 4, 3), (1, 8, 9, 8, 1), (1, 8, 16, 8, 1), (1, 8, 17, 8, 5), (27, 2, 18, 4, 2), (27, 2, 18, 8, 1), (27, 2, 25, 8, 2), (40, 1, 18, 8, 3),
     (1, 1, 64, 4, 16), (1, 1, 70, 4, 16), (1, 1, 128, 4, 16), (1, 1, 150, 4, 19), (1, 8, 150, 4, 16), (1, 4, 250, 8, 32), (1, 8, 256, 8, 16), (1, 8, 400, 8, 18), (1, 2, 600, 4, 32), (1, 1, 5000, 4, 143)])
