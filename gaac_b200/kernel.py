@@ -116,11 +116,12 @@ def _team(rows: int, spare: bool = False) -> int:
 
 
 def _short_ranges(rows: int, ntiles: int, sm_count: int = SM_COUNT_B200) -> bool:
-    """One wave of CTAs, every row split alike, leaves none of them more than about a tile per warp: then it hardly matters which row is the longest, and a plain grid, which plans nothing,
+    """One wave of CTAs, every row split alike, leaves none of them more than a tile per warp: then it hardly matters which row is the longest, and a plain grid, which plans nothing,
     is the faster launch.  us, shares of units -> this, rows of hi / 8 to hi tokens (B x kv heads):  paged 2 x 8 of 300 8.1 -> 7.0;  8 x 8 of 160 8.5 -> 6.1;  16 x 4 of 500 9.1 -> 8.7;  8 x 4 of
-    1100 9.4 -> 8.9;  slots 8 x 8 of 500 10.0 -> 9.0;  32 x 1 of 500 9.2 -> 7.9.  Longer ranges are as fast or faster by shares (3 x 8 of 2000, 21 tiles: 10.3 and 10.2; 16 x 1 of 4000, 28 tiles:
-    10.2 and 10.9)."""
-    return ntiles <= 17 * (sm_count // rows) + 1 and rows <= sm_count
+    1100 9.4 -> 8.9;  slots 8 x 8 of 500 10.0 -> 9.0;  32 x 1 of 500 9.2 -> 7.9.  With 17 tiles in the longest row's ranges a warp takes a second one: 2 x 8 of
+    2448 tokens 9.4 by shares, 10.4 as a grid, 8 x 2 of 2448 9.0 and 10.2, with one query head 8.2 and 9.8; of 2304 (16 tiles) 9.3 and 9.2,
+    9.1 and 9.0, 8.2 and 8.8.  Longer ranges are as fast or faster by shares (3 x 8 of 2000, 21 tiles: 10.3 and 10.2; 16 x 1 of 4000, 28 tiles: 10.2 and 10.9)."""
+    return ntiles <= ATT_WARPS * (sm_count // rows) and rows <= sm_count
 
 
 @functools.lru_cache(maxsize=4096)

@@ -51,6 +51,14 @@ def test_teams_of_three_and_five_are_not_packed_to_the_last(rows, most):
     for bound in (False, True): assert choose_nsplit_sm100(rows, 1, 16 * 28, bound=bound) == (most if most > 1 else 1)
 
 
+@pytest.mark.parametrize("B,n_kv", [(2, 8), (3, 4), (8, 2), (16, 1), (9, 4)])
+def test_equal_ranges_up_to_a_tile_per_warp(calls, B, n_kv):
+    wave = 148 // (B * n_kv)
+    for tiles, name in ((16 * wave, "gaac_paged_decode_attn"), (16 * wave + 1, "gaac_paged_decode_attn_balanced")):
+        made = _paged(calls, B, n_kv, 4, tiles)
+        assert made[0] == name and (name.endswith("balanced") or made[1][8] == wave)
+
+
 @pytest.mark.parametrize("B,n_kv,tiles,G,splits", [
     (1, 8, 8, 4, 1), (1, 8, 9, 4, 3), (1, 8, 9, 8, 1), (1, 8, 16, 8, 1), (1, 8, 17, 8, 5), (27, 2, 18, 4, 2), (27, 2, 18, 8, 1), (27, 2, 25, 8, 2), (40, 1, 18, 8, 3),
     (1, 1, 64, 4, 16), (1, 1, 70, 4, 16), (1, 1, 128, 4, 16), (1, 1, 150, 4, 19), (1, 8, 150, 4, 16), (1, 4, 250, 8, 32), (1, 8, 256, 8, 16), (1, 8, 400, 8, 18), (1, 2, 600, 4, 32), (1, 1, 5000, 4, 143)])
