@@ -136,15 +136,12 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
     if (off0 > 0 && have) {
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        const int c = lane + 32 * k, row = c >> 4, col = (c & 15) * 8;
-        if (row < off0) v[k] = *reinterpret_cast<const uint4*>(rawp + ((long)r_old * T + row) * D + col);
+        const int row = (lane >> 4) + 2 * k;
+        if (row < off0) v[k] = reinterpret_cast<const uint4*>(rawp + (long)r_old * T * D)[lane + 32 * k];
       }
     }
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int c = lane + 32 * k, row = c >> 4, col = (c & 15) * 8;
-      *reinterpret_cast<uint4*>(&ws.xs[row * XS_STRIDE + col]) = v[k];
-    }
+    for (int k = 0; k < 8; k++) *reinterpret_cast<uint4*>(&ws.xs[((lane >> 4) + 2 * k) * XS_STRIDE + (lane & 15) * 8]) = v[k];
     LaneTile lt;
     const int total = encode_tile_warp<KIND_V>(ws, T, b3w, b4w, lane, lt);
     fits = total <= st.ovf_slot;
@@ -166,7 +163,7 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   return fits && have ? r_old : -1;
 }
 
-// 28 CTAs per SM (72 registers, 16 bytes of spills): with the 80 that it would take, 25, a step of 475 x 8 tiles has a second wave, 8.2 -> 8.9 us;  512 x 16 17.2 and 16.8, 94 x 16 5.1 and 5.0.
+// 28 CTAs per SM (72 registers): with 80, 25 CTAs, a step of 475 x 8 tiles has a second wave, 7.9 -> 8.9 us.
 __global__ void __launch_bounds__(32, 28) paged_store_kernel(const __grid_constant__ PagedParams p) {
   __shared__ __align__(16) WarpScratch ws;
   const int e = blockIdx.x, t = blockIdx.y, lane = threadIdx.x;
