@@ -1,6 +1,6 @@
 // The calls of a decode step without the binding's cost: the library's functions as functions of a Python module that take tensors, and the objects that hold them, as they are.  A ctypes call
 // of 15 to 20 arguments takes 1.5 us, a descriptor built from ten data_ptr() calls 1.0 and torch.empty from Python 1.7, against 3 us for the launch itself, and a
-// step of short rows was bound by nothing else.  us, through ctypes -> here: attention over two Pages of 500 tokens 10.7 -> 7.3 (the kernel's time), append and attention of 7 rows 30.9 -> 22.8, paged
+// step of short rows was bound by nothing else.  us, through ctypes -> here: attention over two Pages of 500 tokens 10.7 -> 7.3 (5.8 in a graph), append and attention of 7 rows 30.9 -> 22.8, paged
 // store and attention of 5 rows 21.9 -> 16.4, an encode of [8, 1111, 128] 47.4 -> 41 with its copy, three prompts of 4001 tokens 117.7 -> 108.
 //
 // The module knows the functions' types from the C header and finds their addresses in the library that the package has loaded (bind).  What an argument may be:

@@ -289,7 +289,7 @@ def attention(q, kp, vp, scale=None, nsplit=None, out_f32=None, out=None):
     out (contiguous bf16 tensor of B*n_q*D elements) receives the result instead of a new tensor; out_f32 (fp32, same shape)
     additionally receives the result before its rounding to BF16.
     nsplit=None picks the B200 heuristic; an explicit nsplit is honoured as given.  us a call over 500 tokens, through ctypes and descriptors kept on the
-    Pages -> the native module, which reads the Pages: 10.7 -> 7.3, the kernel's own time."""
+    Pages -> the native module, which reads the Pages: 10.7 -> 7.3 (the launch takes 5.8 in a graph; what is left above it is this function)."""
     B, n_q, Dq = q.shape
     if Dq != 128:
         raise RuntimeError("head_dim must be 128")

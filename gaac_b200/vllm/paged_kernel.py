@@ -21,7 +21,7 @@ def paged_attention(q, out, buf, raw, mt, bt, seq_lens, bases, TS, n_q, n_kv, ns
     """q: [B, n_q, 128] bf16 contiguous; out: [B, n_q*128] bf16 (written); buf: uint8 flat block buffer; raw: [Pr,16,128] bf16;
     mt: int32 [num_blocks*2*n_kv]; bt: int32 [B, max_blocks]; seq_lens: int32 [B]; bases: (b3k,b4k,b3v,b4v) uint8 [n_kv,128].
     (gaac/vllm/paged_kernel.py:296-301; the softmax scale is 1/sqrt(128) as there.)  nsplit=None picks the B200 split count
-    for a ragged batch whose longest row fills the block table; an explicit nsplit is honoured as given."""
+    for a ragged batch whose longest row fills the block table; an explicit nsplit is the most that a row is split into (a short one takes fewer ranges)."""
     B = q.shape[0]; D = q.shape[-1]
     G = n_q // max(1, n_kv)
     if not (1 <= G <= 8): raise RuntimeError("G must be 1..8")
