@@ -122,7 +122,17 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
   const long sstride = KIND_V ? p.v_stride : p.k_stride;
   uint16_t* rawp = reinterpret_cast<uint16_t*>(st.raw);
   int fits = 0, r = r_old;
-  if (full) {
+  // The usual step of a row per block comes first in the code: behind the encoder it took 2.06 us in place of 2.01 (6 x 2 blocks of one row; 2 x 1 whole blocks 3.2 and 3.3).
+  const auto keep_raw = [&] {
+    if (!have) r = pop_raw_tile(st, lane);
+    // new rows, natural channel order, into raw tile r
+    for (int c = lane; c < (r < 0 ? 0 : n * 16); c += 32) {
+      const int row = off0 + (c >> 4), col = (c & 15) * 8;
+      *reinterpret_cast<uint4*>(rawp + ((long)r * T + row) * D + col) = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
+    }
+  };
+  if (!full) keep_raw();
+  else {
     // gather the tile: new rows from this step's K/V, which travel with the mode-table entry, old rows from the raw tile (if any)
     uint4 v[8];
 #pragma unroll
@@ -150,14 +160,7 @@ __device__ __forceinline__ int store_one(WarpScratch& ws, const PagedParams& p, 
       store_tile_payload<KIND_V>(lt, base, base + SLOT_CD_OFF, base + SLOT_FL_OFF, lane);
       store_tile_escapes<KIND_V>(ws, lt, base + SLOT_OVF_OFF, lane);
     }
-  }
-  if (!fits) {
-    if (!have) r = pop_raw_tile(st, lane);
-    // new rows, natural channel order, into raw tile r
-    for (int c = lane; c < (r < 0 ? 0 : n * 16); c += 32) {
-      const int row = off0 + (c >> 4), col = (c & 15) * 8;
-      *reinterpret_cast<uint4*>(rawp + ((long)r * T + row) * D + col) = *reinterpret_cast<const uint4*>(src + (long)(tok0 + row - off0) * sstride + col);
-    }
+    if (!fits) keep_raw();
   }
   if (lane == 0) st.mt[pt] = fits ? (int)pt : ~(r < 0 ? RAW_NONE : r);
   return fits && have ? r_old : -1;
