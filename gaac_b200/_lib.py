@@ -121,8 +121,9 @@ def host():
         except ImportError as e:
             raise RuntimeError(f"gaac_b200's module _host is missing or does not fit this torch ({torch.__version__}): build it with `python -m gaac_b200.build`") from e
         wanted = f"ABI {ABI_VERSION}, torch {torch.__version__}"                       # (it passes arguments as the header and torch's classes were when it was made)
-        if module.built_for != wanted:
-            raise RuntimeError(f"{module.__file__} was built for {module.built_for}, not for {wanted}: rebuild it with `python -m gaac_b200.build`")
+        found = getattr(module, "built_for", "nobody knows what")                      # (one from before it said so, under the name without an interpreter)
+        if found != wanted:
+            raise RuntimeError(f"{module.__file__} was built for {found}, not for {wanted}: rebuild it with `python -m gaac_b200.build`")
         module.bind(handle)
         _host = module
     return _host

@@ -58,13 +58,14 @@ def test_a_module_of_another_interpreter_is_not_found():
     assert build.HOST.endswith(sysconfig.get_config_var("EXT_SUFFIX")) and sysconfig.get_config_var("EXT_SUFFIX") in importlib.machinery.EXTENSION_SUFFIXES
 
 
-@pytest.mark.parametrize("built_for", ["ABI 3, torch %s", "ABI 4, torch 1.0"])
+@pytest.mark.parametrize("built_for", ["ABI 3, torch %s", "ABI 4, torch 1.0", None])
 def test_a_module_for_another_abi_or_torch_is_not_called(monkeypatch, built_for):
     import types
     import torch
     import gaac_b200
     from gaac_b200 import _lib
-    module = types.SimpleNamespace(built_for=built_for % torch.__version__ if "%s" in built_for else built_for, bind=lambda handle: pytest.fail("bound"), __file__="_host.so")
+    module = types.SimpleNamespace(bind=lambda handle: pytest.fail("bound"), __file__="_host.so")
+    if built_for: module.built_for = built_for % torch.__version__ if "%s" in built_for else built_for
     _lib.host()
     monkeypatch.setattr(gaac_b200, "_host", module); monkeypatch.setattr(_lib, "_host", None)
-    with pytest.raises(RuntimeError, match="was built for ABI"): _lib.host()
+    with pytest.raises(RuntimeError, match="was built for"): _lib.host()
